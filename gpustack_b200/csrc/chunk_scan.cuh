@@ -1,0 +1,449 @@
+// Matrix-state recurrences with one decay per head and token over prompt portions, all chunks of a sequence side by side.
+//
+// With a state S (dk x dv), rows t = 0 .. n-1 of a chunk of 64 and the weights that a recurrence's `Form` supplies:
+//     o_t = aq_t S_start^T q_t + sum_{s<=t} D(t, s) (k_s . q_t) v_s          S_end = a S_start + b sum_s w_s k_s v_s^T
+// Three launches:
+//   chunk_state   one CTA per (chunk, head, value tile): C = sum_s w_s k_s v_s^T into the workspace, [chunk][H][dk][dv]
+//   chunk_carry   one CTA per (32 x 32 piece of the state, head, sequence): walks a sequence's chunks, puts S_start in C's
+//                 place and leaves the sequence's final state in its slot
+//   chunk_output  one CTA per (chunk, head, value tile): k_s . q_t, then aq_t S_start^T q_t and the chunk's own rows
+// Why: the one-pass form (16 rows at a time, state in shared memory) is a serial chain of short phases on (sequences x heads x
+// dv / 32) CTAs -- 128 CTAs at 6 us per 16 rows for four prompts -- and idles the chip.  Chunks are independent but for the
+// elementwise carry, so a portion of any length fills the chip; the price is the chunks' states through L2 (dk dv 4 bytes per
+// 64 rows and head, written, carried and read once each).  Everything is fp32 FMAs as before; bound: the FMA rate
+// (4 dk dv + 64 (dk + dv) per row and head), which register tiles of packed pairs (fma.rn.f32x2) approach: a CTA of 256 threads
+// holds a 128 x 128 (state) or 64 x 128 (output) tile, one 16-byte shared-memory read feeds 8 to 16 FMAs.
+// 4 prompts of 2048 rows, 8 heads of 128 x 128 (5.6 GFLOP): 762 -> 246 us (linear attention), 717 -> 267 us (mLSTM), of which
+// state 65, carry 62, output 116 us.
+// Chunks of 64: with 32 the states double, with 128 the chunk's own rows cost more than the states save.
+// Sequences of at most kCsShort rows are left to the caller's one-pass kernel (their state would cross L2 three times for
+// a few rows of work).
+#pragma once
+#include "common.cuh"
+
+namespace b200 {
+
+constexpr int kCsRows = 64, kCsThreads = 256, kCsShort = 16, kCsAPitch = kCsRows + 4;
+
+typedef unsigned long long cs_f2;
+__device__ __forceinline__ cs_f2 cs_dup(float a) {
+  cs_f2 r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
+  return r;
+}
+__device__ __forceinline__ cs_f2 cs_pack(float a, float b) {
+  cs_f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 cs_split(cs_f2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ cs_f2 cs_fma(cs_f2 a, cs_f2 b, cs_f2 c) {
+  cs_f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ cs_f2 cs_mul(cs_f2 a, cs_f2 b) {
+  cs_f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+__device__ __forceinline__ float4 cs_ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 cs_ld4(const bf16* p) {
+  const uint2 r = *reinterpret_cast<const uint2*>(p);
+  return make_float4(bf16_lo(r.x), bf16_hi(r.x), bf16_lo(r.y), bf16_hi(r.y));
+}
+
+// What every recurrence shares: rows, sequences, state, outputs, workspace.
+struct ChunkScanArgs {
+  const void* x;                   // rows of TA
+  int64_t ld;
+  int q_col, k_col, v_col;
+  int H, G, dv;                    // head h reads query / key head h / (H / G)
+  const int32_t* cu_seq;
+  const int32_t* ctx_lens;
+  const int32_t* state_slots;
+  int n_seqs;
+  float* S;                        // [slots][H][dv][dk]
+  float* o;                        // [T][H dv]
+  float* ws;                       // [chunks][H][dk][dv]
+  float* ws_row;                   // [chunks][H][ws_row_width]: a recurrence's own carry (its Form says what)
+  int ws_row_width;                // dk + 4
+};
+
+__host__ __device__ __forceinline__ int cs_chunks(int rows) { return rows > kCsShort ? (rows + kCsRows - 1) / kCsRows : 0; }
+
+// Chunks that the sequences of a step can have at most: the launch's grid and the workspace are sized by this.
+inline int64_t cs_max_chunks(int64_t rows, int64_t n_seqs) {
+  const int64_t longs = rows / (kCsShort + 1);
+  return rows / kCsRows + (longs < n_seqs ? longs : n_seqs);
+}
+inline int64_t cs_workspace_floats(int64_t rows, int64_t n_seqs, int64_t H, int64_t dk, int64_t dv) {
+  return cs_max_chunks(rows, n_seqs) * H * (dk * dv + dk + 4);
+}
+
+// Sequence and place in it of chunk b (whole warp; seq -1: no such chunk), or with b < 0 the chunks before sequence `upto`.
+__device__ __forceinline__ void cs_find(const int32_t* cu, int n_seqs, int b, int upto, int& seq, int& local, int& before) {
+  const int lane = threadIdx.x & 31;
+  seq = -1;
+  local = 0;
+  before = 0;
+  for (int base = 0; base < n_seqs; base += 32) {
+    const int s = base + lane;
+    const int c = s < n_seqs ? cs_chunks(cu[s + 1] - cu[s]) : 0;
+    int incl = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    if (b >= 0) {
+      const uint32_t hit = __ballot_sync(0xffffffffu, before + incl > b);
+      if (hit) {
+        const int l = __ffs(hit) - 1;
+        seq = base + l;
+        local = b - before - (__shfl_sync(0xffffffffu, incl, l) - __shfl_sync(0xffffffffu, c, l));
+        return;
+      }
+    } else if (upto < base + 32) {
+      before += __shfl_sync(0xffffffffu, incl - c, upto - base);
+      return;
+    }
+    before += __shfl_sync(0xffffffffu, incl, 31);
+  }
+}
+
+// The chunk of a CTA of chunk_state / chunk_output.
+struct ChunkPlace {
+  int seq, first, rows, slot, local;
+};
+__device__ __forceinline__ ChunkPlace cs_place(const ChunkScanArgs& a, int* shared5) {
+  if (threadIdx.x < 32) {
+    int seq, local, before;
+    cs_find(a.cu_seq, a.n_seqs, (int)blockIdx.x, 0, seq, local, before);
+    if (threadIdx.x == 0) {
+      shared5[0] = seq;
+      if (seq >= 0) {
+        const int t0 = a.cu_seq[seq] + local * kCsRows;
+        shared5[1] = t0;
+        shared5[2] = min(kCsRows, a.cu_seq[seq + 1] - t0);
+        shared5[3] = a.state_slots[seq];
+        shared5[4] = local;
+      }
+    }
+  }
+  __syncthreads();
+  return {shared5[0], shared5[1], shared5[2], shared5[3], shared5[4]};
+}
+
+// rows x W values of column `col` on -> shared memory, rows beyond `n` zero.  width: columns that exist (a multiple of 4).
+template <int W, int PITCH, typename TA, typename F>
+__device__ __forceinline__ void cs_stage(const TA* x, int64_t ld, int first, int n, int col, int width, float* dst, F scale) {
+  constexpr int PER = W / 4, STEP = kCsThreads / PER, ITERS = kCsRows / STEP;
+  const int c = (threadIdx.x % PER) * 4, r0 = threadIdx.x / PER;
+  float4 v[ITERS];
+#pragma unroll
+  for (int i = 0; i < ITERS; ++i) {
+    const int r = r0 + i * STEP;
+    v[i] = (r < n && c < width) ? cs_ld4(x + (size_t)(first + r) * ld + col + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+#pragma unroll
+  for (int i = 0; i < ITERS; ++i) {
+    const int r = r0 + i * STEP;
+    const float m = scale(r);
+    *reinterpret_cast<float4*>(dst + r * PITCH + c) = make_float4(v[i].x * m, v[i].y * m, v[i].z * m, v[i].w * m);
+  }
+}
+
+template <int DK, int VT>
+struct ChunkSmem {
+  static constexpr int kState = kCsRows * (DK + VT);                                        // floats before the form's arrays
+  static constexpr int kB = kCsRows * (DK + 4 > VT ? DK + 4 : VT);
+  static constexpr int kOutput = kCsRows * (DK + 4) + kB + kCsRows * kCsAPitch;
+};
+
+// Form: `Scratch` (shared arrays of one chunk), `state_weights` (fills scratch, w(s) and row() for chunk_state), `output_weights`,
+// aq(t), D(t, s), finish() for chunk_output, and `carry` / `carry_row` for chunk_carry.
+template <int DK, int VT, typename TA, typename Form>
+__global__ void __launch_bounds__(kCsThreads, 2)
+chunk_state_kernel(const ChunkScanArgs a, const typename Form::Params p) {
+  extern __shared__ __align__(16) float smem[];
+  __shared__ typename Form::Scratch scratch;
+  __shared__ int shared5[5];
+  const ChunkPlace at = cs_place(a, shared5);
+  if (at.seq < 0 || at.slot < 0) return;
+  const int h = blockIdx.y, v0 = blockIdx.z * VT, tid = threadIdx.x;
+  float* ks = smem;                // [64][DK]
+  float* vs = smem + kCsRows * DK; // [64][VT], rows times w
+  Form::state_weights(p, a, scratch, h, at);
+  const TA* x = reinterpret_cast<const TA*>(a.x);
+  cs_stage<DK, DK>(x, a.ld, at.first, at.rows, a.k_col + h / (a.H / a.G) * DK, DK, ks, [](int) { return 1.0f; });
+  cs_stage<VT, VT>(x, a.ld, at.first, at.rows, a.v_col + h * a.dv + v0, a.dv - v0, vs, [&](int r) { return r < at.rows ? scratch.w[r] : 0.f; });
+  __syncthreads();
+  constexpr int KI = DK / 64, VJ = VT / 64;
+  const int vg = tid & 15, kg = tid >> 4;
+  cs_f2 acc[KI * 4][VJ * 2];
+#pragma unroll
+  for (int i = 0; i < KI * 4; ++i)
+#pragma unroll
+    for (int j = 0; j < VJ * 2; ++j) acc[i][j] = 0ull;
+  const int n = (at.rows + 3) & ~3;
+#pragma unroll 4
+  for (int s = 0; s < n; ++s) {
+    float4 kk[KI];
+    ulonglong2 vv[VJ];
+#pragma unroll
+    for (int i = 0; i < KI; ++i) kk[i] = *reinterpret_cast<const float4*>(ks + s * DK + 4 * kg + 64 * i);
+#pragma unroll
+    for (int j = 0; j < VJ; ++j) vv[j] = *reinterpret_cast<const ulonglong2*>(vs + s * VT + 4 * vg + 64 * j);
+#pragma unroll
+    for (int i = 0; i < KI; ++i) {
+      const cs_f2 d[4] = {cs_dup(kk[i].x), cs_dup(kk[i].y), cs_dup(kk[i].z), cs_dup(kk[i].w)};
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+#pragma unroll
+        for (int j = 0; j < VJ; ++j) {
+          acc[i * 4 + e][2 * j] = cs_fma(d[e], vv[j].x, acc[i * 4 + e][2 * j]);
+          acc[i * 4 + e][2 * j + 1] = cs_fma(d[e], vv[j].y, acc[i * 4 + e][2 * j + 1]);
+        }
+    }
+  }
+  float* out = a.ws + ((size_t)blockIdx.x * a.H + h) * DK * a.dv;
+#pragma unroll
+  for (int i = 0; i < KI * 4; ++i)
+#pragma unroll
+    for (int j = 0; j < VJ; ++j) {
+      const int k = 4 * kg + 64 * (i >> 2) + (i & 3), v = v0 + 4 * vg + 64 * j;
+      if (v < a.dv) *reinterpret_cast<ulonglong2*>(out + (size_t)k * a.dv + v) = make_ulonglong2(acc[i][2 * j], acc[i][2 * j + 1]);
+    }
+  if (blockIdx.z == 0) Form::template state_row<DK>(a, scratch, ks, h, at.rows);
+}
+
+// One 32 (keys) x 32 (values) piece of a head's state through a sequence's chunks.
+template <int DK, typename Form>
+__global__ void __launch_bounds__(kCsThreads)
+chunk_carry_kernel(const ChunkScanArgs a, const typename Form::Params p) {
+  __shared__ float tile[32][33];
+  __shared__ int base;
+  const int s = blockIdx.z, h = blockIdx.y, tid = threadIdx.x;
+  const int t0 = a.cu_seq[s], t1 = a.cu_seq[s + 1], nc = cs_chunks(t1 - t0), slot = a.state_slots[s];
+  if (nc == 0 || slot < 0) return;
+  if (tid < 32) {
+    int q, l, before;
+    cs_find(a.cu_seq, a.n_seqs, -1, s, q, l, before);
+    if (tid == 0) base = before;
+  }
+  const int k0 = (blockIdx.x % (DK / 32)) * 32, v0 = (blockIdx.x / (DK / 32)) * 32;
+  float* Sp = a.S + ((size_t)slot * a.H + h) * a.dv * DK;
+  const bool fresh = a.ctx_lens[s] == 0;
+  for (int i = tid; i < 1024; i += kCsThreads) {
+    const int v = i >> 5, k = i & 31;                // k fastest: the slot's layout
+    tile[v][k] = (!fresh && v0 + v < a.dv) ? Sp[(size_t)(v0 + v) * DK + k0 + k] : 0.f;
+  }
+  __syncthreads();
+  const int v = (tid & 7) * 4, k = tid >> 3;
+  float4 S = make_float4(tile[v][k], tile[v + 1][k], tile[v + 2][k], tile[v + 3][k]);
+  const bool live = v0 + v < a.dv;
+  const size_t step = (size_t)a.H * DK * a.dv;
+  float* C = a.ws + ((size_t)base * a.H + h) * DK * a.dv + (size_t)(k0 + k) * a.dv + v0 + v;
+  typename Form::Carry carry(p, a, s, h, base, fresh, slot);
+  constexpr int U = 4;                               // chunks in flight
+  for (int c0 = 0; c0 < nc; c0 += U) {
+    float4 in[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (live && c0 + u < nc) in[u] = *reinterpret_cast<const float4*>(C + (size_t)(c0 + u) * step);
+    carry.fetch(a, c0, nc);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (c0 + u >= nc) break;
+      float fa, fb;
+      carry.next(p, u, min(kCsRows, t1 - t0 - (c0 + u) * kCsRows), fa, fb);
+      if (live) {
+        *reinterpret_cast<float4*>(C + (size_t)(c0 + u) * step) = S;
+        S = make_float4(fmaf(fa, S.x, fb * in[u].x), fmaf(fa, S.y, fb * in[u].y), fmaf(fa, S.z, fb * in[u].z), fmaf(fa, S.w, fb * in[u].w));
+      }
+    }
+  }
+  __syncthreads();
+  tile[v][k] = S.x; tile[v + 1][k] = S.y; tile[v + 2][k] = S.z; tile[v + 3][k] = S.w;
+  __syncthreads();
+  for (int i = tid; i < 1024; i += kCsThreads) {
+    const int vv = i >> 5, kk = i & 31;
+    if (v0 + vv < a.dv) Sp[(size_t)(v0 + vv) * DK + k0 + kk] = tile[vv][kk];
+  }
+  if (blockIdx.x == 0) Form::template carry_row<DK>(p, a, s, h, base, nc, fresh, slot);
+}
+
+// acc[i][.] += sum over 4 rows of B: rows t = tg + 16 i of P (pitch `pp`, columns c .. c + 3), i >= I0.  DIAG >= 0: the rows of
+// B are the chunk's own rows 16 I0 + DIAG .. + 3, which the rows t of block I0 see only up to themselves -- the rest is left
+// out, not multiplied by zero, so that a value that is no number reaches no earlier row.
+template <int VT, int I0, int DIAG = -1>
+__device__ __forceinline__ void cs_outer(cs_f2 (&acc)[4][VT / 32], const float* P, int pp, const float* B, int tg, int vg) {
+  constexpr int VJ = VT / 64;
+  float4 pr[4];
+#pragma unroll
+  for (int i = I0; i < 4; ++i) pr[i] = *reinterpret_cast<const float4*>(P + (tg + 16 * i) * pp);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    ulonglong2 b[VJ];
+#pragma unroll
+    for (int j = 0; j < VJ; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(B + e * VT + 4 * vg + 64 * j);
+#pragma unroll
+    for (int i = I0; i < 4; ++i) {
+      if (DIAG >= 0 && i == I0 && DIAG + e > tg) continue;
+      const cs_f2 d = cs_dup(e == 0 ? pr[i].x : e == 1 ? pr[i].y : e == 2 ? pr[i].z : pr[i].w);
+#pragma unroll
+      for (int j = 0; j < VJ; ++j) {
+        acc[i][2 * j] = cs_fma(d, b[j].x, acc[i][2 * j]);
+        acc[i][2 * j + 1] = cs_fma(d, b[j].y, acc[i][2 * j + 1]);
+      }
+    }
+  }
+}
+
+// acc += A V over the chunk's own rows of block I0 (16 of them)
+template <int VT, int I0>
+__device__ __forceinline__ void cs_own_rows(cs_f2 (&acc)[4][VT / 32], const float* A, const float* V, int tg, int vg) {
+  cs_outer<VT, I0, 0>(acc, A + 16 * I0, kCsAPitch, V + 16 * I0 * VT, tg, vg);
+  cs_outer<VT, I0, 4>(acc, A + 16 * I0 + 4, kCsAPitch, V + (16 * I0 + 4) * VT, tg, vg);
+  cs_outer<VT, I0, 8>(acc, A + 16 * I0 + 8, kCsAPitch, V + (16 * I0 + 8) * VT, tg, vg);
+  cs_outer<VT, I0, 12>(acc, A + 16 * I0 + 12, kCsAPitch, V + (16 * I0 + 12) * VT, tg, vg);
+}
+
+template <int DK, int VT, typename TA, typename Form>
+__global__ void __launch_bounds__(kCsThreads, 2)
+chunk_output_kernel(const ChunkScanArgs a, const typename Form::Params p) {
+  extern __shared__ __align__(16) float smem[];
+  __shared__ typename Form::Scratch scratch;
+  __shared__ int shared5[5];
+  const ChunkPlace at = cs_place(a, shared5);
+  if (at.seq < 0 || at.slot < 0) return;
+  const int h = blockIdx.y, v0 = blockIdx.z * VT, tid = threadIdx.x, n = at.rows;
+  constexpr int QP = DK + 4, VJ = VT / 64;
+  float* qs = smem;                                  // [64][DK + 4]
+  float* B = qs + kCsRows * QP;                      // keys [64][DK + 4], then 64 state rows [64][VT], then values [64][VT]
+  float* A = B + ChunkSmem<DK, VT>::kB;              // [64][68]
+  const TA* x = reinterpret_cast<const TA*>(a.x);
+  const int hg = h / (a.H / a.G);
+  Form::output_weights(p, a, scratch, h, at);
+  cs_stage<DK, QP>(x, a.ld, at.first, n, a.q_col + hg * DK, DK, qs, [&](int) { return Form::q_scale(p); });
+  cs_stage<DK, QP>(x, a.ld, at.first, n, a.k_col + hg * DK, DK, B, [](int) { return 1.0f; });
+  __syncthreads();
+  const int tg = tid >> 4, vg = tid & 15;
+  {
+    // k_s . q_t: rows t = tg + 16 i, columns s = vg + 16 j, j <= i; even and odd entries summed apart
+    cs_f2 acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+#pragma unroll 2
+    for (int d = 0; d < DK; d += 4) {
+      ulonglong2 q[4], k[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        q[i] = *reinterpret_cast<const ulonglong2*>(qs + (tg + 16 * i) * QP + d);
+        k[i] = *reinterpret_cast<const ulonglong2*>(B + (vg + 16 * i) * QP + d);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j <= i; ++j) acc[i][j] = cs_fma(q[i].y, k[j].y, cs_fma(q[i].x, k[j].x, acc[i][j]));
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j <= i; ++j) {
+        const int t = tg + 16 * i, s = vg + 16 * j;
+        const float2 z = cs_split(acc[i][j]);
+        A[t * kCsAPitch + s] = (s <= t && t < n) ? Form::D(p, scratch, t, s) * (z.x + z.y) : 0.f;
+      }
+  }
+  cs_f2 acc[4][VT / 32];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < VT / 32; ++j) acc[i][j] = 0ull;
+  const bool zero_start = at.local == 0 && a.ctx_lens[at.seq] == 0;
+  if (!zero_start) {
+    const float* C = a.ws + ((size_t)blockIdx.x * a.H + h) * DK * a.dv;
+#pragma unroll 1
+    for (int k0 = 0; k0 < DK; k0 += 64) {
+      __syncthreads();                               // the keys / the state rows before are read
+      cs_stage<VT, VT>(C, a.dv, k0, 64, v0, a.dv - v0, B, [](int) { return 1.0f; });
+      __syncthreads();
+#pragma unroll 2
+      for (int d = 0; d < 64; d += 4) cs_outer<VT, 0>(acc, qs + k0 + d, QP, B + d * VT, tg, vg);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const cs_f2 f = cs_dup(Form::aq(scratch, tg + 16 * i));
+#pragma unroll
+      for (int j = 0; j < VT / 32; ++j) acc[i][j] = cs_mul(acc[i][j], f);
+    }
+  }
+  __syncthreads();
+  cs_stage<VT, VT>(x, a.ld, at.first, n, a.v_col + h * a.dv + v0, a.dv - v0, B, [](int) { return 1.0f; });
+  Form::template rows<DK>(p, a, scratch, qs, A, h, n, zero_start);
+  __syncthreads();
+  cs_own_rows<VT, 0>(acc, A, B, tg, vg);
+  cs_own_rows<VT, 1>(acc, A, B, tg, vg);
+  cs_own_rows<VT, 2>(acc, A, B, tg, vg);
+  cs_own_rows<VT, 3>(acc, A, B, tg, vg);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int t = tg + 16 * i;
+    if (t >= n) continue;
+#pragma unroll
+    for (int j = 0; j < VJ; ++j) {
+      const int v = v0 + 4 * vg + 64 * j;
+      if (v >= a.dv) continue;
+      const float2 lo = cs_split(acc[i][2 * j]), hi = cs_split(acc[i][2 * j + 1]);
+      const float4 own = *reinterpret_cast<const float4*>(B + t * VT + 4 * vg + 64 * j);
+      *reinterpret_cast<float4*>(a.o + (size_t)(at.first + t) * a.H * a.dv + h * a.dv + v) =
+          Form::finish(p, scratch, h, t, make_float4(lo.x, lo.y, hi.x, hi.y), own);
+    }
+  }
+}
+
+// Row layout and shapes that the three kernels take; everything else stays on the one-pass kernels.
+inline bool cs_covers(const void* x, int elem, int64_t ld, int q_col, int k_col, int v_col, int dk, int dv, const void* S, const void* o) {
+  const uintptr_t al = 4 * (uintptr_t)elem - 1;
+  return (dk == 64 || dk == 128) && dv % 4 == 0 && ld % 4 == 0 && q_col % 4 == 0 && k_col % 4 == 0 && v_col % 4 == 0 &&
+         ((uintptr_t)x & al) == 0 && ((uintptr_t)S & 15) == 0 && ((uintptr_t)o & 15) == 0;
+}
+
+template <int DK, int VT, typename TA, typename Form>
+int cs_launch_shape(const ChunkScanArgs& a, const typename Form::Params& p, int64_t rows, cudaStream_t s) {
+  const int64_t chunks = cs_max_chunks(rows, a.n_seqs);
+  const dim3 grid((unsigned)chunks, a.H, (a.dv + VT - 1) / VT);
+  const int sb = ChunkSmem<DK, VT>::kState * 4, ob = ChunkSmem<DK, VT>::kOutput * 4;
+  cudaError_t e = cudaFuncSetAttribute(chunk_state_kernel<DK, VT, TA, Form>, cudaFuncAttributeMaxDynamicSharedMemorySize, sb);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(chunk_output_kernel<DK, VT, TA, Form>, cudaFuncAttributeMaxDynamicSharedMemorySize, ob);
+  if (e != cudaSuccess) {
+    b200_set_error("chunk scan: %d bytes of shared memory: %s", ob, cudaGetErrorString(e));
+    return B200_ERR_CUDA;
+  }
+  chunk_state_kernel<DK, VT, TA, Form><<<grid, kCsThreads, sb, s>>>(a, p);
+  chunk_carry_kernel<DK, Form><<<dim3(DK / 32 * ((a.dv + 31) / 32), a.H, a.n_seqs), kCsThreads, 0, s>>>(a, p);
+  chunk_output_kernel<DK, VT, TA, Form><<<grid, kCsThreads, ob, s>>>(a, p);
+  return b200_check_launch(Form::kName);
+}
+
+template <typename TA, typename Form>
+int cs_launch(ChunkScanArgs a, const typename Form::Params& p, int dk, int64_t rows, float* ws, cudaStream_t s) {
+  const int64_t chunks = cs_max_chunks(rows, a.n_seqs);
+  if (chunks == 0) return B200_OK;
+  a.ws = ws;
+  a.ws_row = ws + chunks * a.H * dk * a.dv;
+  a.ws_row_width = dk + 4;
+  if (dk == 64) return a.dv <= 64 ? cs_launch_shape<64, 64, TA, Form>(a, p, rows, s) : cs_launch_shape<64, 128, TA, Form>(a, p, rows, s);
+  return a.dv <= 64 ? cs_launch_shape<128, 64, TA, Form>(a, p, rows, s) : cs_launch_shape<128, 128, TA, Form>(a, p, rows, s);
+}
+
+}  // namespace b200

@@ -19,9 +19,11 @@
 //                  Every power has a non-negative exponent (nothing is divided by a decay, so a small decay cannot
 //                  overflow); all products and sums are fp32 FMAs, only the grouping of the sums differs from the
 //                  serial form.  The CTA's 32 columns of S live in shared memory for the whole portion.
+// The same over chunks of 64 rows side by side (chunk_scan.cuh) when the caller brings a workspace.
 // `linattn_out`    closes the mixer: the heads' outputs over their root mean square -- per head without a weight, or
 //                  all heads together with a weight vector -- times sigmoid(g) or silu(g) of the gate columns of the
 //                  fused projection, rounded once to the activation type.
+#include "chunk_scan.cuh"
 #include "common.cuh"
 #include "runtime.h"
 #include "../../include/b200.h"
@@ -246,7 +248,7 @@ __global__ void __launch_bounds__(kLcThreads)
 linattn_chunk4_kernel(const float* __restrict__ x, int64_t ld, int q_col, int k_col, int v_col,
                       const float* __restrict__ decay, const int32_t* __restrict__ cu_seq,
                       const int32_t* __restrict__ ctx_lens, const int32_t* __restrict__ state_slots, float* S_state,
-                      float* __restrict__ o_raw, int H, int dk, int dv) {
+                      float* __restrict__ o_raw, int H, int dk, int dv, int most_rows) {
   extern __shared__ __align__(16) float smem[];
   const int kst = dk + 4;
   float* Ssm = smem;                                  // [dk][33]
@@ -260,7 +262,7 @@ linattn_chunk4_kernel(const float* __restrict__ x, int64_t ld, int q_col, int k_
   const int slot = state_slots[s];
   if (slot < 0) return;
   const int t0 = cu_seq[s], t1 = cu_seq[s + 1];
-  if (t1 <= t0) return;
+  if (t1 <= t0 || t1 - t0 > most_rows) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int c0 = z * 32;
   float* Sp = S_state + ((size_t)slot * H + h) * dv * dk;
@@ -362,6 +364,54 @@ linattn_chunk4_kernel(const float* __restrict__ x, int64_t ld, int q_col, int k_
   }
 }
 
+// The fixed decay in the chunk form of chunk_scan.cuh: every weight is a power of the head's decay with a non-negative
+// exponent, formed in fp64 by squaring (a decay of zero or below one's sign is as good as any) and rounded once.
+__device__ __forceinline__ float la_power(float d, int n) {
+  double r = 1.0, b = (double)d;
+#pragma unroll
+  for (int bit = 0; bit < 7; ++bit) {
+    if ((n >> bit) & 1) r *= b;
+    b *= b;
+  }
+  return (float)r;
+}
+
+struct LinearForm {
+  static constexpr const char* kName = "b200_linattn_scan(chunks)";
+  struct Params {
+    const float* decay;
+  };
+  struct Scratch {
+    float dp[kCsRows + 1], w[kCsRows];
+  };
+  static __device__ __forceinline__ void state_weights(const Params& p, const ChunkScanArgs&, Scratch& sc, int h, const ChunkPlace& at) {
+    if ((int)threadIdx.x < at.rows) sc.w[threadIdx.x] = la_power(p.decay[h], at.rows - 1 - (int)threadIdx.x);
+    __syncthreads();
+  }
+  template <int DK>
+  static __device__ __forceinline__ void state_row(const ChunkScanArgs&, const Scratch&, const float*, int, int) {}
+  struct Carry {
+    float d, full;
+    __device__ __forceinline__ Carry(const Params& p, const ChunkScanArgs&, int, int h, int, bool, int) : d(p.decay[h]), full(la_power(d, kCsRows)) {}
+    __device__ __forceinline__ void fetch(const ChunkScanArgs&, int, int) {}
+    __device__ __forceinline__ void next(const Params&, int, int rows, float& a, float& b) {
+      a = rows == kCsRows ? full : la_power(d, rows);
+      b = 1.0f;
+    }
+  };
+  template <int DK>
+  static __device__ __forceinline__ void carry_row(const Params&, const ChunkScanArgs&, int, int, int, int, bool, int) {}
+  static __device__ __forceinline__ void output_weights(const Params& p, const ChunkScanArgs&, Scratch& sc, int h, const ChunkPlace&) {
+    if (threadIdx.x <= kCsRows) sc.dp[threadIdx.x] = la_power(p.decay[h], threadIdx.x);
+  }
+  static __device__ __forceinline__ float q_scale(const Params&) { return 1.0f; }
+  static __device__ __forceinline__ float D(const Params&, const Scratch& sc, int t, int s) { return sc.dp[t - s]; }
+  static __device__ __forceinline__ float aq(const Scratch& sc, int t) { return sc.dp[t + 1]; }
+  template <int DK>
+  static __device__ __forceinline__ void rows(const Params&, const ChunkScanArgs&, Scratch&, const float*, const float*, int, int, bool) {}
+  static __device__ __forceinline__ float4 finish(const Params&, const Scratch&, int, int, float4 acc, float4) { return acc; }
+};
+
 // ------------------------------------------------------------------------------------------- out
 // One CTA per row.  all_heads: the H * dv outputs are normed together and multiplied by w; otherwise every head is
 // divided by its own root mean square (w optional, dv entries shared by the heads).  gate_act 0 sigmoid, 1 silu.
@@ -405,6 +455,18 @@ linattn_out_kernel(const float* __restrict__ o_raw, const TA* __restrict__ proj,
 
 using namespace b200;
 
+static int launch_chunk4(const float* x, int64_t ld, int q_col, int k_col, int v_col, const float* decay, const int32_t* cu_seq,
+                         const int32_t* ctx_lens, const int32_t* state_slots, float* S, float* o_raw, int n_seqs, int H, int dk, int dv,
+                         int most_rows, cudaStream_t s) {
+  const size_t smem4 = sizeof(float) * ((((size_t)dk * 33 + 3) & ~(size_t)3) + (size_t)dk * kL4QP + (size_t)kLcTok * (dk + 4) +
+                                        kLcTok * 32 + 4 * kLcTok * 32 + kLcTok * 17 + 32);
+  if (smem4 > 48 * 1024)
+    cudaFuncSetAttribute(linattn_chunk4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem4);
+  linattn_chunk4_kernel<<<dim3(n_seqs, H, (dv + kLaCols - 1) / kLaCols), kLcThreads, smem4, s>>>(
+      x, ld, q_col, k_col, v_col, decay, cu_seq, ctx_lens, state_slots, S, o_raw, H, dk, dv, most_rows);
+  return b200_check_launch("b200_linattn_scan(chunk4)");
+}
+
 extern "C" int b200_linattn_scan(const float* x, int64_t ld, int q_col, int k_col, int v_col, const float* decay,
                                  const int32_t* cu_seq, const int32_t* ctx_lens, const int32_t* state_slots, float* S,
                                  float* o_raw, int n_seqs, int H, int dk, int dv, int max_len, void* stream) {
@@ -416,13 +478,7 @@ extern "C" int b200_linattn_scan(const float* x, int64_t ld, int q_col, int k_co
   dim3 grid(n_seqs, H, Z);
   if (max_len > 2 && dk % 4 == 0) {
     // prompt portions: the chunk form (a single decode row riding in the same launch is a chunk of one)
-    const size_t smem4 = sizeof(float) * ((((size_t)dk * 33 + 3) & ~(size_t)3) + (size_t)dk * kL4QP + (size_t)kLcTok * (dk + 4) +
-                                          kLcTok * 32 + 4 * kLcTok * 32 + kLcTok * 17 + 32);
-    if (smem4 > 48 * 1024)
-      cudaFuncSetAttribute(linattn_chunk4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem4);
-    linattn_chunk4_kernel<<<grid, kLcThreads, smem4, s>>>(x, ld, q_col, k_col, v_col, decay, cu_seq, ctx_lens, state_slots, S,
-                                                          o_raw, H, dk, dv);
-    return b200_check_launch("b200_linattn_scan(chunk4)");
+    return launch_chunk4(x, ld, q_col, k_col, v_col, decay, cu_seq, ctx_lens, state_slots, S, o_raw, n_seqs, H, dk, dv, INT32_MAX, s);
   }
   if (max_len > 2) {
     // key widths that are not multiples of 4: the element-wise chunk kernel
@@ -443,6 +499,29 @@ extern "C" int b200_linattn_scan(const float* x, int64_t ld, int q_col, int k_co
   else B200_LA(8);
 #undef B200_LA
   return b200_check_launch("b200_linattn_scan");
+}
+
+// The same with a workspace of b200_chunk_scan_floats(rows, n_seqs, H, dk, dv) floats: sequences of more than 16 rows run with
+// all their chunks side by side, the others one-pass beside them.  Shapes and alignments that the chunk kernels do not take
+// run as b200_linattn_scan.
+extern "C" int b200_linattn_scan_chunked(const float* x, int64_t ld, int q_col, int k_col, int v_col, const float* decay,
+                                         const int32_t* cu_seq, const int32_t* ctx_lens, const int32_t* state_slots, float* S,
+                                         float* o_raw, int n_seqs, int H, int dk, int dv, int max_len, int rows, float* workspace,
+                                         int64_t workspace_floats, void* stream) {
+  if (workspace == nullptr || rows <= 0 || n_seqs <= 0 || H <= 0 || dv <= 0 || ((uintptr_t)workspace & 15) != 0 ||
+      !cs_covers(x, 4, ld, q_col, k_col, v_col, dk, dv, S, o_raw))
+    return b200_linattn_scan(x, ld, q_col, k_col, v_col, decay, cu_seq, ctx_lens, state_slots, S, o_raw, n_seqs, H, dk, dv, max_len,
+                             stream);
+  B200_REQUIRE(workspace_floats >= cs_workspace_floats(rows, n_seqs, H, dk, dv), "linattn_scan: workspace of %lld floats too small",
+               (long long)workspace_floats);
+  cudaStream_t s = (cudaStream_t)stream;
+  if (n_seqs > 1 || rows <= kCsShort) {
+    const int rc = launch_chunk4(x, ld, q_col, k_col, v_col, decay, cu_seq, ctx_lens, state_slots, S, o_raw, n_seqs, H, dk, dv,
+                                 kCsShort, s);
+    if (rc != B200_OK) return rc;
+  }
+  const ChunkScanArgs a{x, ld, q_col, k_col, v_col, H, H, dv, cu_seq, ctx_lens, state_slots, n_seqs, S, o_raw};
+  return cs_launch<float, LinearForm>(a, {decay}, dk, rows, workspace, s);
 }
 
 extern "C" int b200_linattn_out(const float* o_raw, const void* proj, int f32, int64_t ld, int gate_col, const void* w,

@@ -21,6 +21,7 @@
 //
 // `mlstm_out` then divides every head's o_t by its root mean square, multiplies by the norm
 // weight and the sigmoid output gate, and rounds to the activation type.
+#include "chunk_scan.cuh"
 #include "common.cuh"
 #include "runtime.h"
 #include "../../include/b200.h"
@@ -376,7 +377,8 @@ mlstm_chunk4_kernel(const TA* __restrict__ proj, int64_t ld, int q_col, int k_co
                     const float* __restrict__ gates, const bf16* __restrict__ gate_bias,
                     const int32_t* __restrict__ cu_seq, const int32_t* __restrict__ ctx_lens,
                     const int32_t* __restrict__ state_slots, float* S_state, float* n_state, float* m_state,
-                    float* __restrict__ o_raw, int H, int dk, int dv, float cap, float qscale) {
+                    float* __restrict__ o_raw, int H, int dk, int dv, float cap, float qscale,
+                    int most_rows) {
   extern __shared__ __align__(16) float smem[];
   const int dkp = dk + 4;
   float* qs = smem;                                   // [16][dk + 4]   (16-byte aligned rows)
@@ -398,7 +400,7 @@ mlstm_chunk4_kernel(const TA* __restrict__ proj, int64_t ld, int q_col, int k_co
   const int slot = state_slots[s];
   if (slot < 0) return;
   const int t0 = cu_seq[s], t1 = cu_seq[s + 1];
-  if (t1 <= t0) return;
+  if (t1 <= t0 || t1 - t0 > most_rows) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int c0 = z * 32;
   float* Sp = S_state + ((size_t)slot * H + h) * dv * dk;
@@ -587,7 +589,8 @@ template <typename TA>
 static int launch_chunk(const void* proj, int64_t ld, int q_col, int k_col, int v_col, const float* gates,
                         const void* gate_bias, const int32_t* cu_seq, const int32_t* ctx_lens,
                         const int32_t* state_slots, float* S_state, float* n_state, float* m_state, float* o_raw,
-                        int n_seq, int H, int dk, int dv, float cap, float qscale, cudaStream_t s) {
+                        int n_seq, int H, int dk, int dv, float cap, float qscale, cudaStream_t s,
+                        int most_rows = INT32_MAX) {
   dim3 grid(n_seq, H, (dv + 31) / 32);
   const size_t smem = sizeof(float) * ((size_t)dk * 33 + 2 * kChunkTok * (dk + 1) + kChunkTok * 32 + kChunkTok * 17 + dk +
                                        6 * kChunkTok);
@@ -602,7 +605,8 @@ static int launch_chunk(const void* proj, int64_t ld, int q_col, int k_col, int 
       cudaFuncSetAttribute(mlstm_chunk4_kernel<TA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem4);
     mlstm_chunk4_kernel<TA><<<grid, kChunkThreads, smem4, s>>>((const TA*)proj, ld, q_col, k_col, v_col, gates,
                                                               (const bf16*)gate_bias, cu_seq, ctx_lens, state_slots,
-                                                              S_state, n_state, m_state, o_raw, H, dk, dv, cap, qscale);
+                                                              S_state, n_state, m_state, o_raw, H, dk, dv, cap, qscale,
+                                                              most_rows);
     return b200_check_launch("b200_mlstm_scan(chunk4)");
   }
   if (smem > 48 * 1024)
@@ -612,6 +616,195 @@ static int launch_chunk(const void* proj, int64_t ld, int q_col, int k_col, int 
                                                           n_state, m_state, o_raw, H, dk, dv, cap, qscale);
   return b200_check_launch("b200_mlstm_scan(chunk)");
 }
+
+// The recurrence in the chunk form of chunk_scan.cuh.  Inside a chunk the log forget gates are summed in fp64 (64 of them, so
+// that differences of the sums keep an fp32 gate's precision); every exponent is <= 0 up to that rounding.  A chunk's own
+// contribution is stabilised by mloc = max_s (F_n - F_s + i_s); the carry turns that into the serial form's stabiliser
+// m = max(F_n + m_start, mloc).  The normaliser is one more value column of ones, carried beside the state; like the stabiliser
+// it is equal in all column slices, so slice 0 is read and all slices are written.
+//   ws_row of a chunk: [0, dk) the chunk's normaliser, then the one at its start; dk: F_n; dk + 1: mloc; dk + 2: m_start;
+//   dk + 3 (first chunk of a sequence): the stabiliser that the sequence came with
+struct MlstmForm {
+  static constexpr const char* kName = "b200_mlstm_scan(chunks)";
+  struct Params {
+    const float* gates;
+    const bf16* gate_bias;
+    float cap, qscale;
+    float* n_state;
+    float* m_state;
+    int Z;
+  };
+  struct Scratch {
+    double F[kCsRows];
+    float ii[kCsRows], w[kCsRows], m[kCsRows], aq[kCsRows], den[kCsRows];
+  };
+  // warp 0, two rows per lane: log gates of the chunk's rows, F their running sum, g the running maximum of i_s - F_s
+  static __device__ __forceinline__ void gate_sums(const Params& p, const ChunkScanArgs& a, int h, const ChunkPlace& at, double (&F)[2],
+                                                   double (&g)[2], float (&ii)[2]) {
+    const int lane = threadIdx.x & 31;
+    const float bi = __bfloat162float(p.gate_bias[h]), bf = __bfloat162float(p.gate_bias[a.H + h]);
+    double f[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int t = 2 * lane + e;
+      f[e] = 0.0;
+      ii[e] = 0.f;
+      if (t < at.rows) {
+        const float* gr = p.gates + (size_t)(at.first + t) * 2 * a.H;
+        ii[e] = p.cap * tanhf((gr[h] + bi) / p.cap);
+        f[e] = (double)log_sigmoid(p.cap * tanhf((gr[a.H + h] + bf) / p.cap));
+      }
+    }
+    double sum = f[0] + f[1];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double v = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += v;
+    }
+    F[1] = sum;
+    F[0] = sum - f[1];
+    constexpr double kNone = -1.0e300;
+    const double g0 = 2 * lane < at.rows ? (double)ii[0] - F[0] : kNone, g1 = 2 * lane + 1 < at.rows ? (double)ii[1] - F[1] : kNone;
+    double mx = fmax(g0, g1);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double v = __shfl_up_sync(0xffffffffu, mx, o);
+      if (lane >= o) mx = fmax(mx, v);
+    }
+    g[1] = mx;
+    const double up = __shfl_up_sync(0xffffffffu, mx, 1);
+    g[0] = lane ? fmax(up, g0) : g0;
+  }
+  static __device__ __forceinline__ float* row_of(const ChunkScanArgs& a, int chunk, int h, int dk) {
+    return a.ws_row + ((size_t)chunk * a.H + h) * (dk + 4);
+  }
+  static __device__ __forceinline__ void state_weights(const Params& p, const ChunkScanArgs& a, Scratch& sc, int h, const ChunkPlace& at) {
+    if (threadIdx.x < 32) {
+      double F[2], g[2];
+      float ii[2];
+      gate_sums(p, a, h, at, F, g, ii);
+      const int lane = threadIdx.x, last = (at.rows - 1) >> 1;
+      const double Fn = __shfl_sync(0xffffffffu, (at.rows & 1) ? F[0] : F[1], last);
+      const double gn = __shfl_sync(0xffffffffu, g[1], 31);
+#pragma unroll
+      for (int e = 0; e < 2; ++e) sc.w[2 * lane + e] = 2 * lane + e < at.rows ? expf((float)((double)ii[e] - F[e] - gn)) : 0.f;
+      if (lane == 0) {
+        sc.den[0] = (float)Fn;
+        sc.den[1] = (float)(Fn + gn);
+        sc.den[2] = at.local == 0 && a.ctx_lens[at.seq] != 0 ? p.m_state[((size_t)at.slot * a.H + h) * p.Z] : 0.f;
+      }
+    }
+    __syncthreads();
+  }
+  template <int DK>
+  static __device__ __forceinline__ void state_row(const ChunkScanArgs& a, const Scratch& sc, const float* ks, int h, int rows) {
+    float* row = row_of(a, blockIdx.x, h, DK);
+    const int k = threadIdx.x;
+    if (k < DK) {
+      float n = 0.f;
+      for (int s = 0; s < rows; ++s) n = fmaf(sc.w[s], ks[s * DK + k], n);
+      row[k] = n;
+    }
+    if (k == 0) {
+      row[DK] = sc.den[0];
+      row[DK + 1] = sc.den[1];
+      row[DK + 3] = sc.den[2];
+    }
+  }
+  struct Carry {
+    const float* row;
+    size_t step;
+    float m, F[4], ml[4];
+    int width;
+    __device__ __forceinline__ Carry(const Params&, const ChunkScanArgs& a, int, int h, int base, bool, int) {
+      width = (int)(a.ws_row_width);
+      row = a.ws_row + ((size_t)base * a.H + h) * width;
+      step = (size_t)a.H * width;
+      m = row[width - 1];
+    }
+    __device__ __forceinline__ void fetch(const ChunkScanArgs&, int c0, int nc) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (c0 + u < nc) {
+          F[u] = row[(c0 + u) * step + width - 4];
+          ml[u] = row[(c0 + u) * step + width - 3];
+        }
+    }
+    __device__ __forceinline__ void next(const Params&, int u, int, float& fa, float& fb) {
+      const float m_new = fmaxf(F[u] + m, ml[u]);
+      fa = expf(F[u] + m - m_new);
+      fb = expf(ml[u] - m_new);
+      m = m_new;
+    }
+  };
+  template <int DK>
+  static __device__ __forceinline__ void carry_row(const Params& p, const ChunkScanArgs& a, int, int h, int base, int nc, bool fresh, int slot) {
+    const int k = threadIdx.x;
+    if (k >= DK) return;
+    float* n_out = p.n_state + ((size_t)slot * a.H + h) * p.Z * DK;
+    float n = fresh ? 0.f : n_out[k];
+    float* row = row_of(a, base, h, DK);
+    float m = row[DK + 3];
+    for (int c = 0; c < nc; ++c, row += (size_t)a.H * (DK + 4)) {
+      const float own = row[k], F = row[DK], ml = row[DK + 1];
+      const float m_new = fmaxf(F + m, ml);
+      row[k] = n;
+      if (k == 0) row[DK + 2] = m;
+      n = fmaf(expf(F + m - m_new), n, expf(ml - m_new) * own);
+      m = m_new;
+    }
+    for (int z = 0; z < p.Z; ++z) n_out[z * DK + k] = n;
+    if (k < p.Z) p.m_state[((size_t)slot * a.H + h) * p.Z + k] = m;
+  }
+  static __device__ __forceinline__ void output_weights(const Params& p, const ChunkScanArgs& a, Scratch& sc, int h, const ChunkPlace& at) {
+    if (threadIdx.x < 32) {
+      double F[2], g[2];
+      float ii[2];
+      gate_sums(p, a, h, at, F, g, ii);
+      const double m0 = (double)a.ws_row[((size_t)blockIdx.x * a.H + h) * a.ws_row_width + a.ws_row_width - 2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int t = 2 * threadIdx.x + e;
+        const double gm = fmax(m0, g[e]);            // m_t - F_t
+        sc.F[t] = F[e];
+        sc.ii[t] = ii[e];
+        sc.m[t] = (float)(F[e] + gm);
+        sc.aq[t] = expf((float)(m0 - gm));
+      }
+    }
+  }
+  static __device__ __forceinline__ float q_scale(const Params& p) { return p.qscale; }
+  static __device__ __forceinline__ float D(const Params&, const Scratch& sc, int t, int s) {
+    return expf((float)((sc.F[t] - sc.F[s]) + (double)(sc.ii[s] - sc.m[t])));
+  }
+  static __device__ __forceinline__ float aq(const Scratch& sc, int t) { return sc.aq[t]; }
+  // den_t = max(|n_t . q_t|, exp(-m_t)) + 1e-6, four threads per row
+  template <int DK>
+  static __device__ __forceinline__ void rows(const Params&, const ChunkScanArgs& a, Scratch& sc, const float* qs, const float* A, int h, int n,
+                                              bool zero_start) {
+    const int t = threadIdx.x >> 2, part = threadIdx.x & 3;
+    float own = 0.f, old = 0.f;
+    for (int s = part * 4; s < kCsRows; s += 16) {
+      const float4 v = *reinterpret_cast<const float4*>(A + t * kCsAPitch + s);
+      if (s <= t) own += (v.x + v.y) + (v.z + v.w);
+    }
+    if (!zero_start) {
+      const float* row = row_of(a, blockIdx.x, h, DK);
+      for (int k = part * 4; k < DK; k += 16) {
+        const float4 u = *reinterpret_cast<const float4*>(row + k), q = *reinterpret_cast<const float4*>(qs + t * (DK + 4) + k);
+        old = fmaf(u.x, q.x, fmaf(u.y, q.y, fmaf(u.z, q.z, fmaf(u.w, q.w, old))));
+      }
+    }
+    own = fmaf(sc.aq[t], old, own);
+    own += __shfl_xor_sync(0xffffffffu, own, 1);
+    own += __shfl_xor_sync(0xffffffffu, own, 2);
+    if (part == 0) sc.den[t] = fmaxf(fabsf(own), expf(-sc.m[t])) + 1e-6f;
+  }
+  static __device__ __forceinline__ float4 finish(const Params&, const Scratch& sc, int, int t, float4 v, float4) {
+    const float d = sc.den[t];
+    return make_float4(v.x / d, v.y / d, v.z / d, v.w / d);
+  }
+};
 
 // one warp per (token, head), 8 warps per CTA: o / rms(o) * w * sigmoid(gate); the head is read once
 constexpr int kOutWarps = 8, kOutPer = 8;   // value width <= 256
@@ -703,6 +896,40 @@ extern "C" int b200_mlstm_scan(const void* proj, int f32, int64_t ld, int q_col,
                               n_state, m_state, o_raw, n_seq, H, dk, dv, cap, qscale, s);
   return launch_scan<bf16>(proj, ld, q_col, k_col, v_col, gates, gate_bias, cu_seq, ctx_lens, state_slots, S_state,
                            n_state, m_state, o_raw, n_seq, H, dk, dv, cap, qscale, s);
+}
+
+template <typename TA>
+static int launch_chunks(const void* proj, int64_t ld, int q_col, int k_col, int v_col, const float* gates, const void* gate_bias,
+                         const int32_t* cu_seq, const int32_t* ctx_lens, const int32_t* state_slots, float* S_state, float* n_state,
+                         float* m_state, float* o_raw, int n_seq, int H, int dk, int dv, float cap, float qscale, int rows,
+                         float* workspace, cudaStream_t s) {
+  if (n_seq > 1 || rows <= kCsShort) {
+    const int rc = launch_chunk<TA>(proj, ld, q_col, k_col, v_col, gates, gate_bias, cu_seq, ctx_lens, state_slots, S_state, n_state,
+                                    m_state, o_raw, n_seq, H, dk, dv, cap, qscale, s, kCsShort);
+    if (rc != B200_OK) return rc;
+  }
+  const ChunkScanArgs a{proj, ld, q_col, k_col, v_col, H, H, dv, cu_seq, ctx_lens, state_slots, n_seq, S_state, o_raw};
+  return cs_launch<TA, MlstmForm>(a, {gates, (const bf16*)gate_bias, cap, qscale, n_state, m_state, b200_mlstm_state_slices(dv)}, dk, rows,
+                                  workspace, s);
+}
+
+// The same with a workspace (chunk_scan.cuh): sequences of more than 16 rows run with all their chunks side by side, the others
+// one-pass beside them.  Shapes and alignments that the chunk kernels do not take run as b200_mlstm_scan.
+extern "C" int b200_mlstm_scan_chunked(const void* proj, int f32, int64_t ld, int q_col, int k_col, int v_col, const float* gates,
+                                       const void* gate_bias, const int32_t* cu_seq, const int32_t* ctx_lens,
+                                       const int32_t* state_slots, float* S_state, float* n_state, float* m_state, float* o_raw,
+                                       int n_seq, int H, int dk, int dv, float cap, float qscale, int max_len, int rows,
+                                       float* workspace, int64_t workspace_floats, void* stream) {
+  if (workspace == nullptr || rows <= 0 || n_seq <= 0 || H <= 0 || dv <= 0 || cap <= 0.f || ((uintptr_t)workspace & 15) != 0 ||
+      !cs_covers(proj, f32 ? 4 : 2, ld, q_col, k_col, v_col, dk, dv, S_state, o_raw))
+    return b200_mlstm_scan(proj, f32, ld, q_col, k_col, v_col, gates, gate_bias, cu_seq, ctx_lens, state_slots, S_state, n_state,
+                           m_state, o_raw, n_seq, H, dk, dv, cap, qscale, max_len, stream);
+  B200_REQUIRE(workspace_floats >= cs_workspace_floats(rows, n_seq, H, dk, dv), "mlstm_scan: workspace of %lld floats too small",
+               (long long)workspace_floats);
+  return f32 ? launch_chunks<float>(proj, ld, q_col, k_col, v_col, gates, gate_bias, cu_seq, ctx_lens, state_slots, S_state, n_state,
+                                    m_state, o_raw, n_seq, H, dk, dv, cap, qscale, rows, workspace, (cudaStream_t)stream)
+             : launch_chunks<bf16>(proj, ld, q_col, k_col, v_col, gates, gate_bias, cu_seq, ctx_lens, state_slots, S_state, n_state,
+                                   m_state, o_raw, n_seq, H, dk, dv, cap, qscale, rows, workspace, (cudaStream_t)stream);
 }
 
 extern "C" int b200_mlstm_out(const float* o_raw, const void* proj, int f32, int64_t ld, int gate_col,

@@ -95,6 +95,8 @@ SIGNATURES = {
     "b200_mlstm_state_slices": (_i32, [_i32]),
     "b200_mlstm_scan": (_i32, [_vp, _i32, _i64, _i32, _i32, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32,
                                _i32, _i32, _f32, _f32, _i32, _vp]),
+    "b200_mlstm_scan_chunked": (_i32, [_vp, _i32, _i64, _i32, _i32, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32,
+                                       _i32, _i32, _f32, _f32, _i32, _i32, _vp, _i64, _vp]),
     "b200_streams_step": (_i32, [_vp, _i32, _i64, _vp, _vp, _vp, _f32, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp]),
     "b200_embed_streams": (_i32, [_vp, _vp, _vp, _i32, _i32, _i32, _i32, _f32, _vp]),
     "b200_rms_rows": (_i32, [_vp, _i32, _i64, _vp, _vp, _i64, _i32, _i32, _f32, _vp]),
@@ -121,6 +123,8 @@ SIGNATURES = {
     "b200_rot_prep": (_i32, [_vp, _i32, _i64, _i32, _i32, _i32, _vp, _vp, _vp, _i64, _vp, _i64, _vp, _i64, _i32, _i32, _i32,
                              _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _vp, _i32, _f32, _f32, _f32, _vp]),
     "b200_linattn_scan": (_i32, [_vp, _i64, _i32, _i32, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _vp]),
+    "b200_linattn_scan_chunked": (_i32, [_vp, _i64, _i32, _i32, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32,
+                                         _vp, _i64, _vp]),
     "b200_linattn_out": (_i32, [_vp, _vp, _i32, _i64, _i32, _vp, _vp, _i64, _i32, _i32, _i32, _i32, _i32, _f32, _vp]),
     "b200_attn_sink_prefill_ex": (_i32, [_vp, _i32, _i64, _i32, _vp, _vp, _vp, _i32, _vp, _vp, _vp, _vp, _i32, _i32, _vp, _vp,
                                          _i64, _i32, _i32, _i32, _i32, _i32, _f32, _i64, _i32, _vp]),

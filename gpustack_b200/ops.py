@@ -620,15 +620,37 @@ def mlstm_state_slices(dv: int) -> int:
     return (dv + 31) // 32
 
 
+CHUNK_SCAN_MAX_BYTES = 1 << 30
+
+
+def _chunk_scan_workspace(rows: int, n_seqs: int, H: int, dk: int, dv: int, max_len: int, device):
+    """Workspace of the scans that run a prompt portion's chunks of 64 rows side by side, or None where the one-pass scans are
+    the better ones: key widths the chunk kernels do not take, and steps of short portions (three launches instead of one).
+    All rows beyond max_len are taken for single ones.  Measured, 8 heads of 128 x 128, L2 cold, one-pass -> chunks, linear
+    attention: one portion of 64 rows 34 -> 42 us, 128 rows 57 -> 42, 512 rows 199 -> 46, 2048 rows 762 -> 75; 4 of 64 rows
+    35 -> 48; 16 of 32 rows 55 -> 73, of 64 rows 92 -> 85, of 512 rows 621 -> 255; mLSTM within 10 us of these."""
+    if dk not in (64, 128) or dv % 4 or max_len < 128 or max_len < 96 * (n_seqs - max(0, rows - max_len)):
+        return None
+    n = (rows // 64 + min(n_seqs, rows // 17)) * H * (dk * dv + dk + 4)
+    return torch.empty(n, dtype=torch.float32, device=device) if 4 * n <= CHUNK_SCAN_MAX_BYTES else None
+
+
 def mlstm_scan(proj, q_col, k_col, v_col, gates, gate_bias, cu_seq, ctx_lens, state_slots, S, n, m, o_raw, H, dk, dv,
                cap: float, max_len: int = 1):
     """Runs every sequence's new rows through the matrix-memory recurrence (state slot in, state slot out).
     max_len: an upper bound of the new rows per sequence (prompt portions run in the chunk form)."""
     _cuda(proj, gates, gate_bias, cu_seq, ctx_lens, state_slots, S, n, m, o_raw)
     _req(gates, torch.float32, "gates"); _req(S, torch.float32, "S"); _req(o_raw, torch.float32, "o_raw")
+    n_seq = state_slots.shape[0]
+    ws = _chunk_scan_workspace(proj.shape[0], n_seq, H, dk, dv, max_len, proj.device)
+    if ws is not None:
+        check(load().b200_mlstm_scan_chunked(_p(proj), _is_f32(proj), proj.stride(0), q_col, k_col, v_col, _p(gates), _p(gate_bias),
+                                             _p(cu_seq), _p(ctx_lens), _p(state_slots), _p(S), _p(n), _p(m), _p(o_raw), n_seq, H, dk, dv,
+                                             cap, dk ** -0.5, int(max_len), proj.shape[0], _p(ws), ws.numel(), _stream()), "mlstm_scan")
+        return
     check(load().b200_mlstm_scan(_p(proj), _is_f32(proj), proj.stride(0), q_col, k_col, v_col, _p(gates), _p(gate_bias),
                                  _p(cu_seq), _p(ctx_lens), _p(state_slots), _p(S), _p(n), _p(m), _p(o_raw),
-                                 state_slots.shape[0], H, dk, dv, cap, dk ** -0.5, int(max_len), _stream()), "mlstm_scan")
+                                 n_seq, H, dk, dv, cap, dk ** -0.5, int(max_len), _stream()), "mlstm_scan")
 
 
 def mlstm_out(o_raw, proj, gate_col, norm_w, out, H, dv, eps):
@@ -682,8 +704,15 @@ def linattn_scan(x, q_col: int, k_col: int, v_col: int, decay, cu_seq, ctx_lens,
     _cuda(x, decay, cu_seq, ctx_lens, state_slots, S, o_raw)
     _req(x, torch.float32, "x"); _req(S, torch.float32, "S"); _req(o_raw, torch.float32, "o_raw")
     _req(decay, torch.float32, "decay")
+    n = state_slots.shape[0]
+    ws = _chunk_scan_workspace(x.shape[0], n, H, dk, dv, max_len, x.device)
+    if ws is not None:
+        check(load().b200_linattn_scan_chunked(_p(x), x.stride(0), q_col, k_col, v_col, _p(decay), _p(cu_seq), _p(ctx_lens),
+                                               _p(state_slots), _p(S), _p(o_raw), n, H, dk, dv, int(max_len), x.shape[0], _p(ws),
+                                               ws.numel(), _stream()), "linattn_scan")
+        return
     check(load().b200_linattn_scan(_p(x), x.stride(0), q_col, k_col, v_col, _p(decay), _p(cu_seq), _p(ctx_lens),
-                                   _p(state_slots), _p(S), _p(o_raw), state_slots.shape[0], H, dk, dv, int(max_len),
+                                   _p(state_slots), _p(S), _p(o_raw), n, H, dk, dv, int(max_len),
                                    _stream()), "linattn_scan")
 
 

@@ -308,6 +308,14 @@ int b200_mlstm_scan(const void* proj, int f32, int64_t ld, int q_col, int k_col,
                     const int32_t* ctx_lens, const int32_t* state_slots, float* S_state, float* n_state,
                     float* m_state, float* o_raw, int n_seq, int H, int dk, int dv, float cap, float qscale,
                     int max_len, void* stream);
+/* The same with a workspace: sequences of more than 16 rows run with all their chunks of 64 rows side by side.  rows: the rows
+ * of proj; workspace: 16-byte aligned, (rows / 64 + min(n_seq, rows / 17)) * H * (dk * dv + dk + 4) floats.  Widths other than
+ * dk 64 / 128 with dv % 4 == 0, unaligned rows or no workspace: as b200_mlstm_scan. */
+int b200_mlstm_scan_chunked(const void* proj, int f32, int64_t ld, int q_col, int k_col, int v_col, const float* gates,
+                            const void* gate_bias, const int32_t* cu_seq, const int32_t* ctx_lens, const int32_t* state_slots,
+                            float* S_state, float* n_state, float* m_state, float* o_raw, int n_seq, int H, int dk, int dv,
+                            float cap, float qscale, int max_len, int rows, float* workspace, int64_t workspace_floats,
+                            void* stream);
 /* out = o_raw / rms_head(o_raw) * norm_w * sigmoid(gate). */
 int b200_mlstm_out(const float* o_raw, const void* proj, int f32, int64_t ld, int gate_col,
                    const void* norm_w, void* out, int64_t ldo, int T, int H, int dv, float eps,
@@ -395,6 +403,13 @@ int b200_rot_prep(const void* proj, int src_f32, int64_t ld, int q_col, int k_co
 int b200_linattn_scan(const float* x, int64_t ld, int q_col, int k_col, int v_col, const float* decay,
                       const int32_t* cu_seq, const int32_t* ctx_lens, const int32_t* state_slots, float* S, float* o_raw,
                       int n_seqs, int H, int dk, int dv, int max_len, void* stream);
+/* The same with a workspace: sequences of more than 16 rows run with all their chunks of 64 rows side by side.  rows: the rows
+ * of x; workspace: 16-byte aligned, (rows / 64 + min(n_seqs, rows / 17)) * H * (dk * dv + dk + 4) floats.  Widths other than
+ * dk 64 / 128 with dv % 4 == 0, unaligned rows or no workspace: as b200_linattn_scan. */
+int b200_linattn_scan_chunked(const float* x, int64_t ld, int q_col, int k_col, int v_col, const float* decay,
+                              const int32_t* cu_seq, const int32_t* ctx_lens, const int32_t* state_slots, float* S,
+                              float* o_raw, int n_seqs, int H, int dk, int dv, int max_len, int rows, float* workspace,
+                              int64_t workspace_floats, void* stream);
 /* out = o_raw / rms * (w) * act(gate): all_heads: one RMS over the H*dv entries and w [H*dv]; else per head, w [dv] or
  * NULL.  gate = proj[t, gate_col : gate_col + H*dv]; gate_act 0 sigmoid, 1 silu. */
 int b200_linattn_out(const float* o_raw, const void* proj, int f32, int64_t ld, int gate_col, const void* w, void* out,

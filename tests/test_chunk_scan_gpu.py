@@ -1,0 +1,106 @@
+"""The recurrences with all chunks of a prompt portion side by side, against the recurrences themselves in fp64: chunk edges, short
+and single rows beside long portions, states carried in slots, value widths that fill no tile, a skipped sequence."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+F64 = torch.float64
+# rows of a step's sequences: one chunk, its edges, a remainder of one row, portions that stay one-pass beside long ones
+LENS = [[64], [65], [127], [17, 128, 16, 1, 300], [1, 1, 449], [63, 64, 65]]
+# fp32 sums of at most dk + 64 + (a chunk's share of the state) terms of one size, each rounded: |error| <= 300 * 2^-24 of the
+# terms' norm when all roundings point the same way; the outputs are sums of that kind without cancellation beyond a factor of 2
+TOL = 2 * 300 * 2.0 ** -24
+
+
+def _rel(a, b):
+    return float((a.cpu().to(F64) - b).norm() / b.norm())
+
+
+def _i32(v):
+    return torch.tensor(v, dtype=torch.int32, device="cuda")
+
+
+def _layout(lens):
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    ctx = [0 if i % 2 else 40 for i in range(len(lens))]
+    slots = list(range(len(lens)))[::-1]
+    return cu, ctx, slots
+
+
+@pytest.mark.parametrize("lens", LENS, ids=str)
+@pytest.mark.parametrize("H,dk,dv", [(2, 64, 64), (1, 128, 128), (2, 64, 132), (1, 128, 36)])
+def test_linear_chunks(lens, H, dk, dv):
+    from gpustack_b200 import ops
+
+    g = torch.Generator().manual_seed(sum(lens) + dk + dv)
+    cu, ctx, slots = _layout(lens)
+    T = cu[-1]
+    x = torch.randn(T, 2 * H * dk + H * dv, generator=g)
+    S = torch.randn(len(lens), H, dv, dk, generator=g)
+    decay = torch.tensor([0.98, 0.5][:H])
+    o, S_d = torch.zeros(T, H * dv, device="cuda"), S.cuda()
+    ops.linattn_scan(x.cuda(), 0, H * dk, 2 * H * dk, decay.cuda(), _i32(cu), _i32(ctx), _i32(slots), S_d, o, H, dk, dv, max_len=4096)
+    q, k = x[:, :H * dk].view(T, H, dk).to(F64), x[:, H * dk:2 * H * dk].view(T, H, dk).to(F64)
+    v = x[:, 2 * H * dk:].view(T, H, dv).to(F64)
+    want, S_want = torch.zeros(T, H, dv, dtype=F64), S.to(F64)
+    for i in range(len(lens)):
+        Z = S_want[slots[i]].clone() * (1.0 if ctx[i] else 0.0)
+        for t in range(cu[i], cu[i + 1]):
+            Z = decay.to(F64)[:, None, None] * Z + v[t][:, :, None] * k[t][:, None]
+            want[t] = torch.einsum("hvk,hk->hv", Z, q[t])
+        S_want[slots[i]] = Z
+    assert _rel(o, want.view(T, -1)) < TOL
+    assert _rel(S_d, S_want) < TOL
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("lens", LENS, ids=str)
+@pytest.mark.parametrize("H,dk,dv", [(2, 64, 64), (1, 128, 128), (2, 64, 132), (1, 128, 36)])
+def test_mlstm_chunks(lens, H, dk, dv, dtype):
+    from gpustack_b200 import ops
+    from oracle import vodavik_oracle as O
+
+    g = torch.Generator().manual_seed(sum(lens) + dk + dv)
+    cu, ctx, slots = _layout(lens)
+    T, n_seq, Z, cap = cu[-1], len(lens), ops.mlstm_state_slices(dv), 6.0
+    proj = torch.randn(T, 2 * H * dk + H * dv, generator=g).to(dtype)
+    gates = torch.randn(T, 2 * H, generator=g) * 3.0
+    bias = torch.cat([torch.randn(H, generator=g), 2 + torch.randn(H, generator=g)]).to(torch.bfloat16)
+    S = torch.randn(n_seq, H, dv, dk, generator=g)
+    n = torch.randn(n_seq, H, 1, dk, generator=g).expand(n_seq, H, Z, dk).contiguous()
+    m = torch.rand(n_seq, H, 1, generator=g).expand(n_seq, H, Z).contiguous()
+    o, S_d, n_d, m_d = torch.zeros(T, H * dv, device="cuda"), S.cuda(), n.cuda(), m.cuda()
+    ops.mlstm_scan(proj.cuda(), 0, H * dk, 2 * H * dk, gates.cuda(), bias.cuda(), _i32(cu), _i32(ctx), _i32(slots), S_d, n_d, m_d, o, H, dk,
+                   dv, cap, max_len=4096)
+    p = proj.to(F64)
+    q, k = p[:, :H * dk].view(T, H, dk) * dk ** -0.5, p[:, H * dk:2 * H * dk].view(T, H, dk)
+    v = p[:, 2 * H * dk:].view(T, H, dv)
+    a = cap * torch.tanh((gates.to(F64) + bias.to(F64)) / cap)
+    li, lf = a[:, :H], torch.nn.functional.logsigmoid(a[:, H:])
+    want = torch.zeros(T, H, dv, dtype=F64)
+    for i in range(n_seq):
+        rows, at = slice(cu[i], cu[i + 1]), slots[i]
+        state = (S[at].to(F64).transpose(1, 2), n[at, :, 0].to(F64), m[at, :, 0].to(F64)) if ctx[i] else None
+        want[rows], (Sw, nw, mw) = O.mlstm_scan(q[rows], k[rows], v[rows], li[rows], lf[rows], state)
+        assert _rel(S_d[at], Sw.transpose(1, 2)) < TOL
+        assert all(_rel(n_d[at, :, z], nw) < TOL for z in range(Z)) and all(_rel(m_d[at, :, z], mw) < TOL for z in range(Z))
+    # a denominator |n . q| cancels: its error is of the size of the terms, so rows are compared by the same norm as a whole
+    assert _rel(o, want.reshape(T, -1)) < 20 * TOL
+
+
+def test_no_row_reaches_an_earlier_one_and_negative_slots_are_skipped():
+    from gpustack_b200 import ops
+
+    H, dk, dv, T = 1, 64, 64, 200
+    x = torch.randn(T, 2 * dk + dv, generator=torch.Generator().manual_seed(5))
+    x[70, 2 * dk:] = float("nan")
+    x[130, dk:2 * dk] = float("inf")
+    S = torch.full((2, H, dv, dk), 3.0, device="cuda")
+    o = torch.full((T + 100, H * dv), 7.0, device="cuda")
+    xx = torch.cat([x, torch.randn(100, 2 * dk + dv, generator=torch.Generator().manual_seed(6))]).cuda()
+    ops.linattn_scan(xx, 0, dk, 2 * dk, torch.tensor([0.9]).cuda(), _i32([0, T, T + 100]), _i32([0, 5]), _i32([1, -1]), S, o, H, dk, dv, max_len=T)
+    assert bool(torch.isfinite(o[:70]).all()) and bool(torch.isnan(o[70:T]).all())
+    assert bool((o[T:] == 7.0).all()) and bool((S[0] == 3.0).all())
