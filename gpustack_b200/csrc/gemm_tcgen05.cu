@@ -234,12 +234,12 @@ __device__ __forceinline__ void epilogue_store_tile(uint32_t t_addr, const CUten
 //       tile, multicast into both CTAs' shared memory, so the activation bytes an SM has to ingest
 //       from L2 are halved (the measured limiter of decode-shaped tiles).  Stage release is a
 //       multicast tcgen05.commit: a slot is reused only after BOTH CTAs' MMAs have read it.
-template <int BLOCK_X, int EPI, int MC>
-__global__ void __launch_bounds__(kGemmThreads, 1)
-gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w,
-                         const __grid_constant__ CUtensorMap tmap_x,
-                         const __grid_constant__ CUtensorMap tmap_y, int M, int N, int K, int out_f32,
-                         int splits, int n_tiles, int m_tiles, int group_m, DirectOut dir) {
+// HEADS 1: `splits` independent products instead of K ranges of one: product h multiplies columns h * x_head ... of X with
+// weight rows h * N ... and stores output plane h (the output map's plane pitch is the distance of two heads' columns).
+template <int BLOCK_X, int EPI, int MC, int HEADS = 0>
+__device__ __forceinline__ void gemm_1sm_body(const CUtensorMap& tmap_w, const CUtensorMap& tmap_x, const CUtensorMap& tmap_y, int M,
+                                              int N, int K, int out_f32, int splits, int n_tiles, int m_tiles, int group_m,
+                                              DirectOut dir, int x_head = 0) {
   using Cfg = GemmCfg<BLOCK_X>;
   constexpr int STAGES = Cfg::kStages;
   extern __shared__ uint8_t smem_raw[];
@@ -284,7 +284,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w,
   // of the previous kernel; from here on we touch its outputs
   pdl_wait();
 
-  const int kb_per_split = (K / kBlockK) / splits;
+  const int kb_per_split = HEADS ? K / kBlockK : (K / kBlockK) / splits;
   // with MC == 2 a "unit" is a PAIR of adjacent weight tiles; this CTA takes tile 2*pair + crank
   const int n_units = (n_tiles + MC - 1) / MC;
   const int total_units = n_units * m_tiles * splits;
@@ -300,20 +300,21 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w,
       for (int u = first_unit; u < total_units; u += unit_stride) {
         const TileCoord c = decode_unit(u, n_units, m_tiles, splits, group_m);
         const int n_tile = c.n_tile * MC + (int)crank;
-        const int k0 = c.split * kb_per_split * kBlockK;
+        const int k0 = HEADS ? 0 : c.split * kb_per_split * kBlockK;
+        const int x0 = HEADS ? c.split * x_head : k0, w_row = n_tile * kBlockW + (HEADS ? c.split * N : 0);
         for (int kb = 0; kb < kb_per_split; ++kb) {
           mbar_wait_guarded(&empty_bar[stage], phase ^ 1);
           uint8_t* a = smem + stage * Cfg::kStageBytes;
           uint8_t* b = a + Cfg::kABytes;
           mbar_expect_tx(&full_bar[stage], Cfg::kStageBytes);
-          tma_load_2d(a, &tmap_w, &full_bar[stage], k0 + kb * kBlockK, n_tile * kBlockW, hint_w);
+          tma_load_2d(a, &tmap_w, &full_bar[stage], k0 + kb * kBlockK, w_row, hint_w);
           if constexpr (MC > 1) {
             constexpr int HALF = BLOCK_X / MC;  // rows of the activation tile this CTA fetches
             tma_load_2d_mc(b + crank * (HALF * kBlockK * 2), &tmap_x, &full_bar[stage],
                            k0 + kb * kBlockK, c.m_tile * BLOCK_X + (int)crank * HALF,
                            (uint16_t)((1u << MC) - 1), kEvictLast);
           } else {
-            tma_load_2d(b, &tmap_x, &full_bar[stage], k0 + kb * kBlockK, c.m_tile * BLOCK_X,
+            tma_load_2d(b, &tmap_x, &full_bar[stage], x0 + kb * kBlockK, c.m_tile * BLOCK_X,
                         kEvictLast);
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
@@ -383,6 +384,24 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w,
   }
 }
 
+template <int BLOCK_X, int EPI, int MC>
+__global__ void __launch_bounds__(kGemmThreads, 1)
+gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w,
+                         const __grid_constant__ CUtensorMap tmap_x,
+                         const __grid_constant__ CUtensorMap tmap_y, int M, int N, int K, int out_f32,
+                         int splits, int n_tiles, int m_tiles, int group_m, DirectOut dir) {
+  gemm_1sm_body<BLOCK_X, EPI, MC>(tmap_w, tmap_x, tmap_y, M, N, K, out_f32, splits, n_tiles, m_tiles, group_m, dir);
+}
+
+// One launch for the products of all heads (b200_gemm_bf16_heads).
+template <int BLOCK_X>
+__global__ void __launch_bounds__(kGemmThreads, 1)
+gemm_bf16_heads_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
+                       const __grid_constant__ CUtensorMap tmap_y, int M, int N, int K, int out_f32, int H, int n_tiles, int m_tiles,
+                       int group_m, int x_head) {
+  gemm_1sm_body<BLOCK_X, 0, 1, 1>(tmap_w, tmap_x, tmap_y, M, N, K, out_f32, H, n_tiles, m_tiles, group_m, DirectOut{nullptr, 0}, x_head);
+}
+
 // =================================================================================================
 // 2-SM variant (tcgen05.mma.cta_group::2): a CTA PAIR computes one 256 (weight rows) x BLOCK_X
 // (tokens) tile.  Each CTA stages its own 128 weight rows and HALF of the activation tile; the
@@ -413,9 +432,11 @@ struct Gemm2Cfg {
 // tile_expert[m] * N + n*128...  The number of m-tiles in use is read from device memory after the
 // dependency wait (no host round trip, graph capturable); `xscale`, when given, is the per-row
 // routing weight applied to the fp32 accumulator (MUL_ROUTED_WEIGHT of the reference's fused_moe).
+// GROUPED 2: the products of all heads, as HEADS of the 1-SM kernel (head = split index, x_head its first column of X).
 struct GroupInfo {
   const int32_t* tile_expert;   // [max m_tiles]
   const int32_t* num_m_tiles;   // device scalar
+  int x_head;
 };
 
 template <int BLOCK_X, int EPI, int FP8, int GROUPED = 0>
@@ -424,7 +445,7 @@ __device__ __forceinline__ void gemm_2sm_body(const CUtensorMap& tmap_w, const C
                                               int out_f32, int splits, int n_tiles, int m_tiles,
                                               int group_m, const float* __restrict__ xscale,
                                               const float* __restrict__ wscale, int wscale_stride,
-                                              DirectOut dir, GroupInfo grp = GroupInfo{nullptr, nullptr}) {
+                                              DirectOut dir, GroupInfo grp = GroupInfo{nullptr, nullptr, 0}) {
   using Cfg = Gemm2Cfg<BLOCK_X>;
   constexpr int kElemsK = FP8 ? 2 * kBlockK : kBlockK;   // elements per 128-byte k-block
   constexpr int STAGES = Cfg::kStages;
@@ -473,11 +494,11 @@ __device__ __forceinline__ void gemm_2sm_body(const CUtensorMap& tmap_w, const C
   const uint32_t tmem_base = *tmem_slot;
   pdl_wait();
 
-  if constexpr (GROUPED) {
+  if constexpr (GROUPED == 1) {
     const int used = *grp.num_m_tiles;   // written by the align kernel this grid depends on
     m_tiles = used < m_tiles ? used : m_tiles;
   }
-  const int kb_per_split = (K / kElemsK) / splits;
+  const int kb_per_split = GROUPED == 2 ? K / kElemsK : (K / kElemsK) / splits;
   const int n_units = (n_tiles + 1) / 2;  // a unit = a pair of adjacent weight tiles (256 rows)
   const int total_units = n_units * m_tiles * splits;
   const int first_unit = (int)(blockIdx.x / 2);
@@ -499,8 +520,10 @@ __device__ __forceinline__ void gemm_2sm_body(const CUtensorMap& tmap_w, const C
         const TileCoord c = decode_unit(u, n_units, m_tiles, splits, group_m);
         const int n_tile = c.n_tile * 2 + (int)crank;
         int w_row = n_tile * kBlockW;
-        if constexpr (GROUPED) w_row += grp.tile_expert[c.m_tile] * N;
-        const int k0 = c.split * kb_per_split * kElemsK;
+        if constexpr (GROUPED == 1) w_row += grp.tile_expert[c.m_tile] * N;
+        if constexpr (GROUPED == 2) w_row += c.split * N;
+        const int k0 = GROUPED == 2 ? 0 : c.split * kb_per_split * kElemsK;
+        const int x0 = GROUPED == 2 ? c.split * grp.x_head : k0;
         for (int kb = 0; kb < kb_per_split; ++kb) {
           mbar_wait_guarded(&empty_bar[stage], phase ^ 1);
           uint8_t* a = smem + stage * Cfg::kStageBytes;
@@ -508,7 +531,7 @@ __device__ __forceinline__ void gemm_2sm_body(const CUtensorMap& tmap_w, const C
           // this CTA's bytes are announced on the LEADER's barrier, where the TMAs complete
           mbar_expect_tx_cluster(mapa_u32(&full_bar[stage], 0), Cfg::kStageBytes);
           tma_load_2d_2sm(a, &tmap_w, &full_bar[stage], k0 + kb * kElemsK, w_row, hint_w);
-          tma_load_2d_2sm(b, &tmap_x, &full_bar[stage], k0 + kb * kElemsK,
+          tma_load_2d_2sm(b, &tmap_x, &full_bar[stage], x0 + kb * kElemsK,
                           c.m_tile * BLOCK_X + (int)crank * Cfg::kHalf, hint_x);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
@@ -566,7 +589,7 @@ __device__ __forceinline__ void gemm_2sm_body(const CUtensorMap& tmap_w, const C
         const float ws = n < N ? wscale[(size_t)n * wscale_stride] : 0.f;
         epilogue_store_tile<BLOCK_X, EPI, 1>(t_addr, &tmap_y, stg, which, n0, m_base, c.split, M, N, out_f32, lane,
                                              dir, xscale, ws);
-      } else if (GROUPED && xscale != nullptr) {
+      } else if (GROUPED == 1 && xscale != nullptr) {
         epilogue_store_tile<BLOCK_X, EPI, 1>(t_addr, &tmap_y, stg, which, n0, m_base, c.split, M, N, out_f32, lane,
                                              dir, xscale, 1.f);
       } else {
@@ -625,7 +648,16 @@ gemm_bf16_grouped_2sm_kernel(const __grid_constant__ CUtensorMap tmap_w,
                              const int32_t* __restrict__ tile_expert,
                              const int32_t* __restrict__ num_m_tiles, DirectOut dir, int out_flags) {
   gemm_2sm_body<BLOCK_X, EPI, 0, 1>(tmap_w, tmap_x, tmap_y, M, N, K, out_flags, 1, n_tiles, m_tiles, group_m,
-                                    row_scale, nullptr, 0, dir, GroupInfo{tile_expert, num_m_tiles});
+                                    row_scale, nullptr, 0, dir, GroupInfo{tile_expert, num_m_tiles, 0});
+}
+
+template <int BLOCK_X>
+__global__ void __launch_bounds__(kGemmThreads, 1)
+gemm_bf16_heads_2sm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
+                           const __grid_constant__ CUtensorMap tmap_y, int M, int N, int K, int out_f32, int H, int n_tiles,
+                           int m_tiles, int group_m, int x_head) {
+  gemm_2sm_body<BLOCK_X, 0, 0, 2>(tmap_w, tmap_x, tmap_y, M, N, K, out_f32, H, n_tiles, m_tiles, group_m, nullptr, nullptr, 0,
+                                  DirectOut{nullptr, 0}, GroupInfo{nullptr, nullptr, x_head});
 }
 
 // Tensor map of the output for the epilogue's TMA stores: [splits][M][N] (bf16, or fp32 when out_f32)
@@ -942,12 +974,74 @@ extern "C" int b200_gemm_bf16_silu_mul(const void* X, const void* W, void* Y, in
   }
 }
 
-// One GEMM per head over strided views of wider rows: Y[:, h * y_head : + N] = X[:, h * x_head : + K] W_h^T with W_h the
-// h-th contiguous [N, K] matrix.  The loop runs here so that a step pays one library call for all heads.
+// Y[:, h * y_head : + N] = X[:, h * x_head : + K] W_h^T for all heads in ONE launch, W_h the h-th contiguous [N, K] matrix: the
+// head is one more tile coordinate -- a column offset of X's tensor map, a row offset of W's, a plane of Y's.  One launch per
+// head encoded three maps each and left the chip to a few tiles: 16 heads, 8192 rows, 128 -> 512 columns 122 us, 512 -> 128
+// 157 us; together 48 and 40 us (L2 cold), bound by the epilogue's stores and the rows' reads.  Pairs of CTAs take 256 weight
+// rows when a head has them, single CTAs 128 otherwise.
+template <int BLOCK_X, bool PAIR>
+static int launch_heads(const void* X, const void* W, void* Y, int M, int N, int K, int64_t ldx, int64_t ldy, int H, int64_t x_head,
+                        int64_t y_head, int out_f32, cudaStream_t stream) {
+  const int smem = PAIR ? Gemm2Cfg<BLOCK_X>::kSmemBytes : GemmCfg<BLOCK_X>::kSmemBytes;
+  auto kernel = [] {
+    if constexpr (PAIR) return gemm_bf16_heads_2sm_kernel<BLOCK_X>;
+    else return gemm_bf16_heads_kernel<BLOCK_X>;
+  }();
+  static bool attr_set = false;
+  if (!attr_set) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) {
+      b200_set_error("gemm_heads: cudaFuncSetAttribute(smem=%d): %s", smem, cudaGetErrorString(e));
+      return B200_ERR_CUDA;
+    }
+    attr_set = true;
+  }
+  CUtensorMap tw, tx, ty;
+  int rc = make_tmap_bf16_2d(&tw, W, (uint64_t)H * N, (uint64_t)K, (uint64_t)K, kBlockW, kBlockK);
+  if (rc) return rc;
+  rc = make_tmap_bf16_2d(&tx, X, (uint64_t)M, (uint64_t)((H - 1) * x_head + K), (uint64_t)ldx, PAIR ? BLOCK_X / 2 : BLOCK_X, kBlockK);
+  if (rc) return rc;
+  rc = make_tmap_out_3d(&ty, Y, out_f32 ? 4 : 2, (uint64_t)N, (uint64_t)M, (uint64_t)H, (uint64_t)ldy, (uint64_t)y_head, 32,
+                        BLOCK_X >= 32 ? 32 : 16);
+  if (rc) return rc;
+  const int n_tiles = (N + kBlockW - 1) / kBlockW, m_tiles = (M + BLOCK_X - 1) / BLOCK_X;
+  const long long total = (long long)(PAIR ? (n_tiles + 1) / 2 : n_tiles) * m_tiles * H;
+  const int sms = device_info().sm_count > 0 ? device_info().sm_count : 148, cl = PAIR ? 2 : 1;
+  const int clusters = (int)(total < sms / cl ? total : sms / cl);
+  const int group_m = m_tiles < 8 ? m_tiles : 8;
+  cudaError_t e = launch_pdl(kernel, dim3(clusters * cl), dim3(kGemmThreads), (size_t)smem, stream, cl, tw, tx, ty, M, N, K, out_f32, H,
+                             n_tiles, m_tiles, group_m, (int)x_head);
+  if (e != cudaSuccess) {
+    b200_set_error("b200_gemm_bf16_heads: launch failed: %s", cudaGetErrorString(e));
+    (void)cudaGetLastError();
+    return B200_ERR_CUDA;
+  }
+  return b200_check_launch("b200_gemm_bf16_heads");
+}
+
 extern "C" int b200_gemm_bf16_heads(const void* X, const void* W, void* Y, int M, int N, int K, int64_t ldx,
                                     int64_t ldy, int H, int64_t x_head, int64_t y_head, int out_f32, void* stream) {
   B200_REQUIRE(H >= 1, "gemm_heads: bad head count %d", H);
   const size_t es = out_f32 ? 4 : 2;
+  out_f32 = out_f32 ? 1 : 0;
+  const DeviceInfo& d = device_info();
+  const int bx = plan_block_x(M, N, H);
+  const bool pair = N % (2 * kBlockW) == 0 && gemm_2sm_enabled();
+  // one launch: what three tensor maps can describe (a plane per head needs its pitch in whole 16 bytes, as rows do)
+  if (M > 0 && N > 0 && K > 0 && K % kBlockK == 0 && d.valid && d.cc_major == 10 && x_head >= 0 && y_head > 0 && ldx >= K && ldy >= N &&
+      (x_head * 2) % 16 == 0 && (ldx * 2) % 16 == 0 && ((size_t)y_head * es) % 16 == 0 && ((size_t)ldy * es) % 16 == 0 &&
+      (reinterpret_cast<uintptr_t>(X) & 15) == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0 &&
+      (reinterpret_cast<uintptr_t>(Y) & 15) == 0 && (H - 1) * x_head + K <= ldx && (int64_t)H * N <= INT32_MAX) {
+    cudaStream_t s = (cudaStream_t)stream;
+#define B200_HEADS(BX)                                                                                                    \
+  return pair ? launch_heads<BX, true>(X, W, Y, M, N, K, ldx, ldy, H, x_head, y_head, out_f32, s)                         \
+              : launch_heads<BX, false>(X, W, Y, M, N, K, ldx, ldy, H, x_head, y_head, out_f32, s)
+    if (bx <= 32) B200_HEADS(32);
+    if (bx == 64) B200_HEADS(64);
+    if (bx == 128) B200_HEADS(128);
+    B200_HEADS(256);
+#undef B200_HEADS
+  }
   for (int h = 0; h < H; ++h) {
     const int rc = b200_gemm_bf16_ex(reinterpret_cast<const bf16*>(X) + (size_t)h * x_head,
                                      reinterpret_cast<const bf16*>(W) + (size_t)h * N * K,
