@@ -33,6 +33,7 @@ SOURCES = [
     "streams.cu",
     "latent.cu",
     "latent_attention_mma.cu",
+    "latent_attention_tc.cu",
     "gemm_simt_grouped.cu",
     "moe_biased.cu",
     "prenorm.cu",
@@ -68,6 +69,7 @@ STREAMS_LATENT_SOURCES = [
     "streams.cu",
     "latent.cu",
     "latent_attention_mma.cu",
+    "latent_attention_tc.cu",
     "attention_sink.cu",
 ]
 ROUTED_SOURCES = ["moe.cu", "moe_biased.cu"]

@@ -134,6 +134,36 @@ static int make_tmap_2d(CUtensorMap* out, const void* base, uint64_t rows, uint6
   return B200_OK;
 }
 
+int make_tmap_bf16_nd(CUtensorMap* out, const void* base, int rank, const uint64_t* dims, const uint64_t* stride_bytes,
+                      const uint32_t* box) {
+  EncodeTiledFn fn = get_encode_fn();
+  if (!fn) {
+    b200_set_error("cuTensorMapEncodeTiled entry point not available");
+    return B200_ERR_CUDA;
+  }
+  bool ok = rank >= 2 && rank <= 5 && box[0] * 2 == 128 && (reinterpret_cast<uintptr_t>(base) & 15) == 0;
+  cuuint64_t d[5], st[4];
+  cuuint32_t b[5], estr[5];
+  for (int i = 0; ok && i < rank; ++i) {
+    d[i] = dims[i];
+    b[i] = box[i];
+    estr[i] = 1;
+    if (i + 1 < rank) ok = ((st[i] = stride_bytes[i]) & 15) == 0;
+  }
+  if (!ok) {
+    b200_set_error("TMA operand must be 16-byte aligned with a 128-byte inner box (base %p, rank %d)", base, rank);
+    return B200_ERR_INVALID;
+  }
+  const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(base), d, st, b, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    b200_set_error("cuTensorMapEncodeTiled failed: CUresult %d (rank %d)", (int)r, rank);
+    return B200_ERR_CUDA;
+  }
+  return B200_OK;
+}
+
 int make_tmap_out_3d(CUtensorMap* out, const void* base, int elem_bytes, uint64_t cols, uint64_t rows,
                      uint64_t planes, uint64_t ld_elems, uint64_t plane_elems, uint32_t box_cols,
                      uint32_t box_rows) {

@@ -24,6 +24,11 @@ int make_tmap_bf16_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_
 int make_tmap_u8_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld_elems,
                     uint32_t box_rows, uint32_t box_cols);
 
+// bf16 map of any rank with a 128-byte swizzle (box[0] 64 elements): dims and box innermost first, the strides of dims 1 .. rank - 1
+// in bytes, in any order of size (a row's column blocks may be a dimension of their own).
+int make_tmap_bf16_nd(CUtensorMap* out, const void* base, int rank, const uint64_t* dims, const uint64_t* stride_bytes,
+                      const uint32_t* box);
+
 // 3-D, un-swizzled map used by the GEMM epilogues' TMA STORES: tensor [planes][rows][cols] of
 // elem_bytes-wide elements (2 = bf16, 4 = fp32), row pitch ld_elems, plane pitch plane_elems
 // (split-K partial planes; 1 plane otherwise); box = box_cols x box_rows x 1.  The hardware clips

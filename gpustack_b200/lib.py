@@ -108,6 +108,8 @@ SIGNATURES = {
     "b200_latent_attn_covers": (_i32, [_i32, _i32, _i32]),
     "b200_latent_attn_prefill": (_i32, [_vp, _i64, _vp, _i32, _vp, _i32, _vp, _vp, _vp, _vp, _i32, _i32, _vp, _vp, _i64, _i32,
                                         _i32, _i32, _f32, _vp]),
+    "b200_latent_attn_prefill_rows": (_i32, [_vp, _i64, _i32, _vp, _i32, _i32, _vp, _i32, _vp, _vp, _vp, _vp, _i32, _i32, _vp, _vp,
+                                             _i64, _i32, _i32, _i32, _f32, _vp]),
     "b200_latent_attn_decode": (_i32, [_vp, _i64, _vp, _i32, _vp, _i32, _vp, _i32, _vp, _vp, _i64, _i32, _i32, _i32, _f32,
                                        _i32, _vp, _vp]),
     "b200_latent_attn_decode_splits": (_i32, [_i32, _i32, _i32]),

@@ -1037,10 +1037,10 @@ def latent_attn_prefill(qa, cache, block_table, cu_q, ctx_lens, tile_seq, tile_q
     kernel covers run there, everything else (fp32, odd widths) on the generic kernel with one shared key head."""
     _cuda(qa, cache, block_table, cu_q, ctx_lens, tile_seq, tile_q0, sink, out)
     if qa.dtype == torch.bfloat16 and latent_attn_covers(H, R, dr) and qa.stride(0) % 8 == 0 and qa.data_ptr() % 16 == 0:
-        check(load().b200_latent_attn_prefill(_p(qa), qa.stride(0), _p(cache), cache.shape[2], _p(block_table),
-                                              block_table.shape[1], _p(cu_q), _p(ctx_lens), _p(tile_seq), _p(tile_q0),
-                                              tile_seq.shape[0], tile_rows or attn_sink_prefill_tile(), _p(sink), _p(out),
-                                              out.stride(0), H, R, dr, scale, _stream()), "latent_attn_prefill")
+        check(load().b200_latent_attn_prefill_rows(_p(qa), qa.stride(0), qa.shape[0], _p(cache), cache.shape[0], cache.shape[2],
+                                                   _p(block_table), block_table.shape[1], _p(cu_q), _p(ctx_lens), _p(tile_seq),
+                                                   _p(tile_q0), tile_seq.shape[0], tile_rows or attn_sink_prefill_tile(), _p(sink),
+                                                   _p(out), out.stride(0), H, R, dr, scale, _stream()), "latent_attn_prefill")
         return out
     return attn_sink_prefill(qa, -1, cache, cache, block_table, cu_q, ctx_lens, tile_seq, tile_q0, sink, out, H, 1, R + dr, R,
                              scale, tile_rows=tile_rows, v_ld=R + dr)

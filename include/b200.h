@@ -350,6 +350,12 @@ int b200_latent_attn_prefill(const void* qa, int64_t ldq, const void* cache, int
                              int max_blocks, const int32_t* cu_q, const int32_t* ctx_lens, const int32_t* tile_seq,
                              const int32_t* tile_q0, int n_tiles, int tile_rows, const float* sink, void* out,
                              int64_t ldo, int H, int R, int dr, float scale, void* stream);
+/* The same with the number of query rows and cache pages: heads that divide 128 with R 512 + dr 64, 16-row pages, contiguous
+ * query rows and tile_rows * H a multiple of 256 run on CTA pairs with tcgen05 (csrc/latent_attention_tc.cu). */
+int b200_latent_attn_prefill_rows(const void* qa, int64_t ldq, int rows, const void* cache, int num_blocks, int page,
+                                  const int32_t* block_table, int max_blocks, const int32_t* cu_q, const int32_t* ctx_lens,
+                                  const int32_t* tile_seq, const int32_t* tile_q0, int n_tiles, int tile_rows,
+                                  const float* sink, void* out, int64_t ldo, int H, int R, int dr, float scale, void* stream);
 /* decode: nsplit > 1 cuts every row's keys into that many ranges (more CTAs for small batches of long sequences) and
  * merges them in a second launch; workspace of b200_latent_attn_decode_workspace_bytes(), contents irrelevant. */
 int b200_latent_attn_decode_splits(int B, int H, int max_len);

@@ -16,6 +16,66 @@ def _i32(v):
     return torch.tensor(v, dtype=torch.int32, device="cuda")
 
 
+# portions around the item (256 / H rows), page (16), value unit (32) and block (96) edges, new and continued, several in one step
+@pytest.mark.parametrize("H", [16, 32, 128])
+@pytest.mark.parametrize("lens,ctx", [([1], [0]), ([16], [0]), ([17], [47]), ([96], [0]), ([97], [96]), ([65, 1, 200], [0, 127, 64]),
+                                      ([33, 130], [300, 0])], ids=str)
+def test_prompt_portions(H, lens, ctx):
+    from gpustack_b200 import ops
+
+    g = torch.Generator().manual_seed(H + sum(lens))
+    T, total = sum(lens), [a + b for a, b in zip(lens, ctx)]
+    need = [(n + 15) // 16 for n in total]
+    order = torch.randperm(sum(need), generator=g).to(torch.int32)
+    table = torch.zeros(len(lens), max(need) + 2, dtype=torch.int32)
+    cache = torch.full((sum(need), 1, 16, R + DR), float("nan"), dtype=BF)      # what no sequence owns is no number
+    rows, at = [], 0
+    for i, n in enumerate(total):
+        table[i, :need[i]] = order[at:at + need[i]]
+        at += need[i]
+        rows.append(torch.randn(n, R + DR, generator=g).to(BF))
+        for j in range(n):
+            cache[table[i, j // 16], 0, j % 16] = rows[i][j]
+    q = torch.randn(T, H * (R + DR), generator=g).to(BF)
+    sink, scale = torch.randn(H, generator=g), 1.5 * (R + DR) ** -0.5
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    ts, tq = ops.build_prefill_tiles(lens, ops.attn_sink_prefill_tile(), ctx)
+    out = torch.zeros(T, H * R, dtype=BF, device="cuda")
+    ops.latent_attn_prefill(q.cuda(), cache.cuda(), table.cuda(), _i32(cu), _i32(ctx), _i32(ts), _i32(tq), sink.cuda(), out, H, R, DR, scale)
+    want = []
+    for i, n in enumerate(lens):
+        k = rows[i].to(F64)
+        s = torch.einsum("thd,nd->htn", q[cu[i]:cu[i + 1]].to(F64).view(n, H, R + DR), k) * scale
+        s.masked_fill_(torch.arange(total[i])[None] > ctx[i] + torch.arange(n)[:, None], -float("inf"))
+        p = torch.cat([s, sink.to(F64)[:, None, None].expand(H, n, 1)], -1).softmax(-1)[..., :-1]
+        want.append(torch.einsum("htn,nr->thr", p, k[:, :R]).reshape(n, -1))
+    # bf16 probabilities and outputs: 2^-9 each, rounded independently
+    assert _rel(out, torch.cat(want)) < 2 * 2.0 ** -9
+
+
+def test_a_growing_maximum_moves_the_reference():
+    """Scores that rise by far more than 2^8 from block to block: the accumulators are rescaled on the way."""
+    from gpustack_b200 import ops
+
+    H, n = 16, 520
+    g = torch.Generator().manual_seed(2)
+    C = torch.randn(n, R + DR, generator=g)
+    C[:, R] = torch.arange(n) // 100 * 40.0
+    q = torch.randn(1, H, R + DR, generator=g) * 0.02
+    q[..., R] = 1.0
+    C, q = C.to(BF), q.to(BF)
+    cache = torch.zeros((n + 15) // 16, 1, 16, R + DR, dtype=BF)
+    cache.view(-1, R + DR)[:n] = C
+    out = torch.zeros(1, H * R, dtype=BF, device="cuda")
+    ts, tq = ops.build_prefill_tiles([1], ops.attn_sink_prefill_tile(), [n - 1])
+    ops.latent_attn_prefill(q.view(1, -1).cuda(), cache.cuda(), torch.arange(cache.shape[0], dtype=torch.int32).view(1, -1).cuda(), _i32([0, 1]),
+                            _i32([n - 1]), _i32(ts), _i32(tq), None, out, H, R, DR, 1.0)
+    p = (q[0].to(F64) @ C.to(F64).T).softmax(-1)
+    assert _rel(out.view(H, R), p @ C[:, :R].to(F64)) < 2 * 2.0 ** -9
+
+
 @pytest.mark.parametrize("f32", [False, True])
 @pytest.mark.parametrize("M", [1, 33, 257, 700])
 @pytest.mark.parametrize("H,N,K,pad", [(16, 512, 128, 64), (5, 128, 512, 0), (3, 192, 64, 64), (2, 72, 128, 8)])
