@@ -13,8 +13,8 @@
 // 64 rows and head, written, carried and read once each).  Everything is fp32 FMAs as before; bound: the FMA rate
 // (4 dk dv + 64 (dk + dv) per row and head), which register tiles of packed pairs (fma.rn.f32x2) approach: a CTA of 256 threads
 // holds a 128 x 128 (state) or 64 x 128 (output) tile, one 16-byte shared-memory read feeds 8 to 16 FMAs.
-// 4 prompts of 2048 rows, 8 heads of 128 x 128 (5.6 GFLOP): 762 -> 246 us (linear attention), 717 -> 267 us (mLSTM), of which
-// state 65, carry 62, output 116 us.
+// 4 prompts of 2048 rows, 8 heads of 128 x 128 (5.6 GFLOP): one-pass 762 us, here 208 us (linear attention, L2 cold), of which
+// state 60, carry 45, output 100 us (without the copies behind the sums, and 32 x 32 pieces in the carry: 65, 62, 116).
 // Chunks of 64: with 32 the states double, with 128 the chunk's own rows cost more than the states save.
 // Sequences of at most kCsShort rows are left to the caller's one-pass kernel (their state would cross L2 three times for
 // a few rows of work).
@@ -50,12 +50,6 @@ __device__ __forceinline__ cs_f2 cs_mul(cs_f2 a, cs_f2 b) {
   cs_f2 r;
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
-}
-
-__device__ __forceinline__ float4 cs_ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-__device__ __forceinline__ float4 cs_ld4(const bf16* p) {
-  const uint2 r = *reinterpret_cast<const uint2*>(p);
-  return make_float4(bf16_lo(r.x), bf16_hi(r.x), bf16_lo(r.y), bf16_hi(r.y));
 }
 
 // What every recurrence shares: rows, sequences, state, outputs, workspace.
@@ -140,30 +134,50 @@ __device__ __forceinline__ ChunkPlace cs_place(const ChunkScanArgs& a, int* shar
   return {shared5[0], shared5[1], shared5[2], shared5[3], shared5[4]};
 }
 
-// rows x W values of column `col` on -> shared memory, rows beyond `n` zero.  width: columns that exist (a multiple of 4).
-template <int W, int PITCH, typename TA, typename F>
-__device__ __forceinline__ void cs_stage(const TA* x, int64_t ld, int first, int n, int col, int width, float* dst, F scale) {
-  constexpr int PER = W / 4, STEP = kCsThreads / PER, ITERS = kCsRows / STEP;
-  const int c = (threadIdx.x % PER) * 4, r0 = threadIdx.x / PER;
-  float4 v[ITERS];
+// ROWS x W values of column `col` on, on their way to shared memory (fp32, row pitch PITCH, rows from `n` and columns from
+// `width` on zero): fp32 rows by cp.async, bf16 rows through registers, converted when they land.
+template <typename TA, int ROWS, int W, int PITCH>
+struct ChunkTile {
+  static constexpr int PER = W / 4, STEP = kCsThreads / PER, ITERS = ROWS / STEP;
+  uint2 raw[ITERS];
+  __device__ __forceinline__ void issue(const TA* x, int64_t ld, int first, int n, int col, int width, float*) {
+    const int c = ((int)threadIdx.x % PER) * 4, r0 = (int)threadIdx.x / PER;
 #pragma unroll
-  for (int i = 0; i < ITERS; ++i) {
-    const int r = r0 + i * STEP;
-    v[i] = (r < n && c < width) ? cs_ld4(x + (size_t)(first + r) * ld + col + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = 0; i < ITERS; ++i) {
+      const int r = r0 + i * STEP;
+      raw[i] = make_uint2(0, 0);
+      if (r < n && c < width) raw[i] = *reinterpret_cast<const uint2*>(x + (size_t)(first + r) * ld + col + c);
+    }
   }
+  __device__ __forceinline__ void land(float* dst) const {
+    const int c = ((int)threadIdx.x % PER) * 4, r0 = (int)threadIdx.x / PER;
 #pragma unroll
-  for (int i = 0; i < ITERS; ++i) {
-    const int r = r0 + i * STEP;
-    const float m = scale(r);
-    *reinterpret_cast<float4*>(dst + r * PITCH + c) = make_float4(v[i].x * m, v[i].y * m, v[i].z * m, v[i].w * m);
+    for (int i = 0; i < ITERS; ++i)
+      *reinterpret_cast<float4*>(dst + (r0 + i * STEP) * PITCH + c) =
+          make_float4(bf16_lo(raw[i].x), bf16_hi(raw[i].x), bf16_lo(raw[i].y), bf16_hi(raw[i].y));
   }
-}
+};
+template <int ROWS, int W, int PITCH>
+struct ChunkTile<float, ROWS, W, PITCH> {
+  static constexpr int PER = W / 4, STEP = kCsThreads / PER, ITERS = ROWS / STEP;
+  __device__ __forceinline__ void issue(const float* x, int64_t ld, int first, int n, int col, int width, float* dst) {
+    const int c = ((int)threadIdx.x % PER) * 4, r0 = (int)threadIdx.x / PER;
+#pragma unroll
+    for (int i = 0; i < ITERS; ++i) {
+      const int r = r0 + i * STEP;
+      const bool in = r < n && c < width;
+      cp_async_16_zfill(dst + r * PITCH + c, in ? x + (size_t)(first + r) * ld + col + c : x, in);
+    }
+  }
+  __device__ __forceinline__ void land(float*) const {}
+};
 
 template <int DK, int VT>
 struct ChunkSmem {
-  static constexpr int kState = kCsRows * (DK + VT);                                        // floats before the form's arrays
-  static constexpr int kB = kCsRows * (DK + 4 > VT ? DK + 4 : VT);
-  static constexpr int kOutput = kCsRows * (DK + 4) + kB + kCsRows * kCsAPitch;
+  static constexpr int kState = kCsRows * (DK + VT);         // floats
+  static constexpr int kTile = 32 * VT;                      // a tile of 32 state or value rows
+  static constexpr int kB = kCsRows * (DK + 4) > 2 * kTile ? kCsRows * (DK + 4) : 2 * kTile;
+  static constexpr int kOutput = kCsRows * (DK + 4) + kB + kTile + kCsRows * kCsAPitch;
 };
 
 // Form: `Scratch` (shared arrays of one chunk), `state_weights` (fills scratch, w(s) and row() for chunk_state), `output_weights`,
@@ -178,12 +192,19 @@ chunk_state_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   if (at.seq < 0 || at.slot < 0) return;
   const int h = blockIdx.y, v0 = blockIdx.z * VT, tid = threadIdx.x;
   float* ks = smem;                // [64][DK]
-  float* vs = smem + kCsRows * DK; // [64][VT], rows times w
-  Form::state_weights(p, a, scratch, h, at);
+  float* vs = smem + kCsRows * DK; // [64][VT]
   const TA* x = reinterpret_cast<const TA*>(a.x);
-  cs_stage<DK, DK>(x, a.ld, at.first, at.rows, a.k_col + h / (a.H / a.G) * DK, DK, ks, [](int) { return 1.0f; });
-  cs_stage<VT, VT>(x, a.ld, at.first, at.rows, a.v_col + h * a.dv + v0, a.dv - v0, vs, [&](int r) { return r < at.rows ? scratch.w[r] : 0.f; });
-  __syncthreads();
+  const int kcol = a.k_col + h / (a.H / a.G) * DK, vcol = a.v_col + h * a.dv + v0;
+  // two halves of 32 rows: the second one is on its way while the first is summed
+  ChunkTile<TA, 32, DK, DK> kt[2];
+  ChunkTile<TA, 32, VT, VT> vt[2];
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    kt[e].issue(x, a.ld, at.first + 32 * e, at.rows - 32 * e, kcol, DK, ks + 32 * e * DK);
+    vt[e].issue(x, a.ld, at.first + 32 * e, at.rows - 32 * e, vcol, a.dv - v0, vs + 32 * e * VT);
+    cp_async_commit();
+  }
+  Form::state_weights(p, a, scratch, h, at);
   constexpr int KI = DK / 64, VJ = VT / 64;
   const int vg = tid & 15, kg = tid >> 4;
   cs_f2 acc[KI * 4][VJ * 2];
@@ -191,25 +212,35 @@ chunk_state_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   for (int i = 0; i < KI * 4; ++i)
 #pragma unroll
     for (int j = 0; j < VJ * 2; ++j) acc[i][j] = 0ull;
-  const int n = (at.rows + 3) & ~3;
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    kt[e].land(ks + 32 * e * DK);
+    vt[e].land(vs + 32 * e * VT);
+    if (e == 0) cp_async_wait<1>();
+    else cp_async_wait<0>();
+    __syncthreads();
+    const int n = min(at.rows - 32 * e, 32);
 #pragma unroll 4
-  for (int s = 0; s < n; ++s) {
-    float4 kk[KI];
-    ulonglong2 vv[VJ];
+    for (int r = 0; r < n; ++r) {
+      const int s = 32 * e + r;
+      const float w = scratch.w[s];
+      float4 kk[KI];
+      ulonglong2 vv[VJ];
 #pragma unroll
-    for (int i = 0; i < KI; ++i) kk[i] = *reinterpret_cast<const float4*>(ks + s * DK + 4 * kg + 64 * i);
+      for (int i = 0; i < KI; ++i) kk[i] = *reinterpret_cast<const float4*>(ks + s * DK + 4 * kg + 64 * i);
 #pragma unroll
-    for (int j = 0; j < VJ; ++j) vv[j] = *reinterpret_cast<const ulonglong2*>(vs + s * VT + 4 * vg + 64 * j);
+      for (int j = 0; j < VJ; ++j) vv[j] = *reinterpret_cast<const ulonglong2*>(vs + s * VT + 4 * vg + 64 * j);
 #pragma unroll
-    for (int i = 0; i < KI; ++i) {
-      const cs_f2 d[4] = {cs_dup(kk[i].x), cs_dup(kk[i].y), cs_dup(kk[i].z), cs_dup(kk[i].w)};
+      for (int i = 0; i < KI; ++i) {
+        const cs_f2 d[4] = {cs_dup(kk[i].x * w), cs_dup(kk[i].y * w), cs_dup(kk[i].z * w), cs_dup(kk[i].w * w)};
 #pragma unroll
-      for (int e = 0; e < 4; ++e)
+        for (int u = 0; u < 4; ++u)
 #pragma unroll
-        for (int j = 0; j < VJ; ++j) {
-          acc[i * 4 + e][2 * j] = cs_fma(d[e], vv[j].x, acc[i * 4 + e][2 * j]);
-          acc[i * 4 + e][2 * j + 1] = cs_fma(d[e], vv[j].y, acc[i * 4 + e][2 * j + 1]);
-        }
+          for (int j = 0; j < VJ; ++j) {
+            acc[i * 4 + u][2 * j] = cs_fma(d[u], vv[j].x, acc[i * 4 + u][2 * j]);
+            acc[i * 4 + u][2 * j + 1] = cs_fma(d[u], vv[j].y, acc[i * 4 + u][2 * j + 1]);
+          }
+      }
     }
   }
   float* out = a.ws + ((size_t)blockIdx.x * a.H + h) * DK * a.dv;
@@ -223,11 +254,14 @@ chunk_state_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   if (blockIdx.z == 0) Form::template state_row<DK>(a, scratch, ks, h, at.rows);
 }
 
-// One 32 (keys) x 32 (values) piece of a head's state through a sequence's chunks.
+// 8 keys x 128 values of a head's state through a sequence's chunks: a warp's row of a chunk is 512 contiguous bytes, eight
+// chunks are in flight.
+constexpr int kCsCarryKeys = 8, kCsCarryDepth = 8;
+
 template <int DK, typename Form>
 __global__ void __launch_bounds__(kCsThreads)
 chunk_carry_kernel(const ChunkScanArgs a, const typename Form::Params p) {
-  __shared__ float tile[32][33];
+  __shared__ float tile[128][kCsCarryKeys + 1];
   __shared__ int base;
   const int s = blockIdx.z, h = blockIdx.y, tid = threadIdx.x;
   const int t0 = a.cu_seq[s], t1 = a.cu_seq[s + 1], nc = cs_chunks(t1 - t0), slot = a.state_slots[s];
@@ -237,21 +271,21 @@ chunk_carry_kernel(const ChunkScanArgs a, const typename Form::Params p) {
     cs_find(a.cu_seq, a.n_seqs, -1, s, q, l, before);
     if (tid == 0) base = before;
   }
-  const int k0 = (blockIdx.x % (DK / 32)) * 32, v0 = (blockIdx.x / (DK / 32)) * 32;
+  const int k0 = (blockIdx.x % (DK / kCsCarryKeys)) * kCsCarryKeys, v0 = (blockIdx.x / (DK / kCsCarryKeys)) * 128;
   float* Sp = a.S + ((size_t)slot * a.H + h) * a.dv * DK;
   const bool fresh = a.ctx_lens[s] == 0;
-  for (int i = tid; i < 1024; i += kCsThreads) {
-    const int v = i >> 5, k = i & 31;                // k fastest: the slot's layout
+  for (int i = tid; i < 128 * kCsCarryKeys; i += kCsThreads) {
+    const int v = i / kCsCarryKeys, k = i % kCsCarryKeys;     // k fastest: the slot's layout, whole 32-byte sectors
     tile[v][k] = (!fresh && v0 + v < a.dv) ? Sp[(size_t)(v0 + v) * DK + k0 + k] : 0.f;
   }
   __syncthreads();
-  const int v = (tid & 7) * 4, k = tid >> 3;
+  const int v = (tid & 31) * 4, k = tid >> 5;
   float4 S = make_float4(tile[v][k], tile[v + 1][k], tile[v + 2][k], tile[v + 3][k]);
   const bool live = v0 + v < a.dv;
   const size_t step = (size_t)a.H * DK * a.dv;
   float* C = a.ws + ((size_t)base * a.H + h) * DK * a.dv + (size_t)(k0 + k) * a.dv + v0 + v;
   typename Form::Carry carry(p, a, s, h, base, fresh, slot);
-  constexpr int U = 4;                               // chunks in flight
+  constexpr int U = kCsCarryDepth;
   for (int c0 = 0; c0 < nc; c0 += U) {
     float4 in[U];
 #pragma unroll
@@ -272,8 +306,8 @@ chunk_carry_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   __syncthreads();
   tile[v][k] = S.x; tile[v + 1][k] = S.y; tile[v + 2][k] = S.z; tile[v + 3][k] = S.w;
   __syncthreads();
-  for (int i = tid; i < 1024; i += kCsThreads) {
-    const int vv = i >> 5, kk = i & 31;
+  for (int i = tid; i < 128 * kCsCarryKeys; i += kCsThreads) {
+    const int vv = i / kCsCarryKeys, kk = i % kCsCarryKeys;
     if (v0 + vv < a.dv) Sp[(size_t)(v0 + vv) * DK + k0 + kk] = tile[vv][kk];
   }
   if (blockIdx.x == 0) Form::template carry_row<DK>(p, a, s, h, base, nc, fresh, slot);
@@ -324,16 +358,43 @@ chunk_output_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   const ChunkPlace at = cs_place(a, shared5);
   if (at.seq < 0 || at.slot < 0) return;
   const int h = blockIdx.y, v0 = blockIdx.z * VT, tid = threadIdx.x, n = at.rows;
-  constexpr int QP = DK + 4, VJ = VT / 64;
+  constexpr int QP = DK + 4, VJ = VT / 64, TILE = ChunkSmem<DK, VT>::kTile;
   float* qs = smem;                                  // [64][DK + 4]
-  float* B = qs + kCsRows * QP;                      // keys [64][DK + 4], then 64 state rows [64][VT], then values [64][VT]
+  float* X = qs + kCsRows * QP;                      // ring of three tiles of 32 rows; the keys [64][DK + 4] first lie on tiles 1 and 2
+  float* B = X + TILE;
   float* A = B + ChunkSmem<DK, VT>::kB;              // [64][68]
   const TA* x = reinterpret_cast<const TA*>(a.x);
-  const int hg = h / (a.H / a.G);
-  Form::output_weights(p, a, scratch, h, at);
-  cs_stage<DK, QP>(x, a.ld, at.first, n, a.q_col + hg * DK, DK, qs, [&](int) { return Form::q_scale(p); });
-  cs_stage<DK, QP>(x, a.ld, at.first, n, a.k_col + hg * DK, DK, B, [](int) { return 1.0f; });
+  const int hg = h / (a.H / a.G), vcol = a.v_col + h * a.dv + v0;
+  const bool zero_start = at.local == 0 && a.ctx_lens[at.seq] == 0;
+  const float* C = a.ws + ((size_t)blockIdx.x * a.H + h) * DK * a.dv;
+  // tiles in the order of their use: the state's rows (none for a zero start), then the chunk's own values
+  const int n_state = zero_start ? 0 : DK / 32;
+  ChunkTile<TA, 32, VT, VT> own[2];
+  auto tile_at = [&](int i) { return X + (i % 3) * TILE; };
+  auto issue = [&](int i) {
+    if (i < n_state) {
+      ChunkTile<float, 32, VT, VT> t;
+      t.issue(C, a.dv, 32 * i, 32, v0, a.dv - v0, tile_at(i));
+    } else if (i == n_state) {
+      own[0].issue(x, a.ld, at.first, n, vcol, a.dv - v0, tile_at(i));
+    } else if (i == n_state + 1) {
+      own[1].issue(x, a.ld, at.first + 32, n - 32, vcol, a.dv - v0, tile_at(i));
+    }
+    cp_async_commit();
+  };
+  {
+    ChunkTile<TA, kCsRows, DK, QP> q, k;
+    q.issue(x, a.ld, at.first, n, a.q_col + hg * DK, DK, qs);
+    k.issue(x, a.ld, at.first, n, a.k_col + hg * DK, DK, B);
+    cp_async_commit();
+    issue(0);
+    Form::output_weights(p, a, scratch, h, at);
+    q.land(qs);
+    k.land(B);
+  }
+  cp_async_wait<1>();
   __syncthreads();
+  const float q_scale = Form::q_scale(p);
   const int tg = tid >> 4, vg = tid & 15;
   {
     // k_s . q_t: rows t = tg + 16 i, columns s = vg + 16 j, j <= i; even and odd entries summed apart
@@ -361,7 +422,7 @@ chunk_output_kernel(const ChunkScanArgs a, const typename Form::Params p) {
       for (int j = 0; j <= i; ++j) {
         const int t = tg + 16 * i, s = vg + 16 * j;
         const float2 z = cs_split(acc[i][j]);
-        A[t * kCsAPitch + s] = (s <= t && t < n) ? Form::D(p, scratch, t, s) * (z.x + z.y) : 0.f;
+        A[t * kCsAPitch + s] = (s <= t && t < n) ? Form::D(p, scratch, t, s) * ((z.x + z.y) * q_scale) : 0.f;
       }
   }
   cs_f2 acc[4][VT / 32];
@@ -369,32 +430,39 @@ chunk_output_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int j = 0; j < VT / 32; ++j) acc[i][j] = 0ull;
-  const bool zero_start = at.local == 0 && a.ctx_lens[at.seq] == 0;
-  if (!zero_start) {
-    const float* C = a.ws + ((size_t)blockIdx.x * a.H + h) * DK * a.dv;
+  // tile i: landed, and tile i - 1 used by every thread, so tile i + 2 may take its place (behind the first barrier the keys
+  // are used as well)
+  auto next_tile = [&](int i) {
+    if (i == n_state) own[0].land(tile_at(i));
+    if (i == n_state + 1) own[1].land(tile_at(i));
+    if (i == 0 || i == n_state + 1) cp_async_wait<0>();
+    else cp_async_wait<1>();
+    __syncthreads();
+    if (i == 0) issue(1);
+    if (i + 2 <= n_state + 1) issue(i + 2);
+    return tile_at(i);
+  };
 #pragma unroll 1
-    for (int k0 = 0; k0 < DK; k0 += 64) {
-      __syncthreads();                               // the keys / the state rows before are read
-      cs_stage<VT, VT>(C, a.dv, k0, 64, v0, a.dv - v0, B, [](int) { return 1.0f; });
-      __syncthreads();
+  for (int i = 0; i < n_state; ++i) {
+    const float* T = next_tile(i);
 #pragma unroll 2
-      for (int d = 0; d < 64; d += 4) cs_outer<VT, 0>(acc, qs + k0 + d, QP, B + d * VT, tg, vg);
-    }
+    for (int d = 0; d < 32; d += 4) cs_outer<VT, 0>(acc, qs + 32 * i + d, QP, T + d * VT, tg, vg);
+  }
+  if (!zero_start) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const cs_f2 f = cs_dup(Form::aq(scratch, tg + 16 * i));
+      const cs_f2 f = cs_dup(Form::aq(scratch, tg + 16 * i) * q_scale);
 #pragma unroll
       for (int j = 0; j < VT / 32; ++j) acc[i][j] = cs_mul(acc[i][j], f);
     }
   }
-  __syncthreads();
-  cs_stage<VT, VT>(x, a.ld, at.first, n, a.v_col + h * a.dv + v0, a.dv - v0, B, [](int) { return 1.0f; });
+  const float* V0 = next_tile(n_state);
   Form::template rows<DK>(p, a, scratch, qs, A, h, n, zero_start);
-  __syncthreads();
-  cs_own_rows<VT, 0>(acc, A, B, tg, vg);
-  cs_own_rows<VT, 1>(acc, A, B, tg, vg);
-  cs_own_rows<VT, 2>(acc, A, B, tg, vg);
-  cs_own_rows<VT, 3>(acc, A, B, tg, vg);
+  cs_own_rows<VT, 0>(acc, A, V0, tg, vg);
+  cs_own_rows<VT, 1>(acc, A, V0, tg, vg);
+  const float* V1 = next_tile(n_state + 1);
+  cs_own_rows<VT, 2>(acc, A, V1 - 32 * VT, tg, vg);
+  cs_own_rows<VT, 3>(acc, A, V1 - 32 * VT, tg, vg);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int t = tg + 16 * i;
@@ -404,9 +472,9 @@ chunk_output_kernel(const ChunkScanArgs a, const typename Form::Params p) {
       const int v = v0 + 4 * vg + 64 * j;
       if (v >= a.dv) continue;
       const float2 lo = cs_split(acc[i][2 * j]), hi = cs_split(acc[i][2 * j + 1]);
-      const float4 own = *reinterpret_cast<const float4*>(B + t * VT + 4 * vg + 64 * j);
+      const float4 mine = *reinterpret_cast<const float4*>((i < 2 ? V0 + t * VT : V1 + (t - 32) * VT) + 4 * vg + 64 * j);
       *reinterpret_cast<float4*>(a.o + (size_t)(at.first + t) * a.H * a.dv + h * a.dv + v) =
-          Form::finish(p, scratch, h, t, make_float4(lo.x, lo.y, hi.x, hi.y), own);
+          Form::finish(p, scratch, h, t, make_float4(lo.x, lo.y, hi.x, hi.y), mine);
     }
   }
 }
@@ -430,7 +498,7 @@ int cs_launch_shape(const ChunkScanArgs& a, const typename Form::Params& p, int6
     return B200_ERR_CUDA;
   }
   chunk_state_kernel<DK, VT, TA, Form><<<grid, kCsThreads, sb, s>>>(a, p);
-  chunk_carry_kernel<DK, Form><<<dim3(DK / 32 * ((a.dv + 31) / 32), a.H, a.n_seqs), kCsThreads, 0, s>>>(a, p);
+  chunk_carry_kernel<DK, Form><<<dim3(DK / kCsCarryKeys * ((a.dv + 127) / 128), a.H, a.n_seqs), kCsThreads, 0, s>>>(a, p);
   chunk_output_kernel<DK, VT, TA, Form><<<grid, kCsThreads, ob, s>>>(a, p);
   return b200_check_launch(Form::kName);
 }

@@ -714,7 +714,7 @@ struct MlstmForm {
   struct Carry {
     const float* row;
     size_t step;
-    float m, F[4], ml[4];
+    float m, F[kCsCarryDepth], ml[kCsCarryDepth];
     int width;
     __device__ __forceinline__ Carry(const Params&, const ChunkScanArgs& a, int, int h, int base, bool, int) {
       width = (int)(a.ws_row_width);
@@ -724,7 +724,7 @@ struct MlstmForm {
     }
     __device__ __forceinline__ void fetch(const ChunkScanArgs&, int c0, int nc) {
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
+      for (int u = 0; u < kCsCarryDepth; ++u)
         if (c0 + u < nc) {
           F[u] = row[(c0 + u) * step + width - 4];
           ml[u] = row[(c0 + u) * step + width - 3];
@@ -780,7 +780,7 @@ struct MlstmForm {
   static __device__ __forceinline__ float aq(const Scratch& sc, int t) { return sc.aq[t]; }
   // den_t = max(|n_t . q_t|, exp(-m_t)) + 1e-6, four threads per row
   template <int DK>
-  static __device__ __forceinline__ void rows(const Params&, const ChunkScanArgs& a, Scratch& sc, const float* qs, const float* A, int h, int n,
+  static __device__ __forceinline__ void rows(const Params& p, const ChunkScanArgs& a, Scratch& sc, const float* qs, const float* A, int h, int n,
                                               bool zero_start) {
     const int t = threadIdx.x >> 2, part = threadIdx.x & 3;
     float own = 0.f, old = 0.f;
@@ -795,7 +795,7 @@ struct MlstmForm {
         old = fmaf(u.x, q.x, fmaf(u.y, q.y, fmaf(u.z, q.z, fmaf(u.w, q.w, old))));
       }
     }
-    own = fmaf(sc.aq[t], old, own);
+    own = fmaf(sc.aq[t] * p.qscale, old, own);
     own += __shfl_xor_sync(0xffffffffu, own, 1);
     own += __shfl_xor_sync(0xffffffffu, own, 2);
     if (part == 0) sc.den[t] = fmaxf(fabsf(own), expf(-sc.m[t])) + 1e-6f;
