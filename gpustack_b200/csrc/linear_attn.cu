@@ -25,6 +25,7 @@
 //                  fused projection, rounded once to the activation type.
 #include "chunk_scan.cuh"
 #include "common.cuh"
+#include "head_out.cuh"
 #include "runtime.h"
 #include "../../include/b200.h"
 
@@ -531,6 +532,10 @@ extern "C" int b200_linattn_out(const float* o_raw, const void* proj, int f32, i
   B200_REQUIRE(!all_heads || w != nullptr, "linattn_out: the joint norm has a weight");
   if (T == 0) return B200_OK;
   cudaStream_t s = (cudaStream_t)stream;
+  // a norm per head keeps its heads in registers; the joint norm, and widths the other does not take, one CTA per row
+  if (!all_heads && (f32 ? head_out_launch<float>(o_raw, proj, ld, gate_col, w, 0, out, ldo, T, H, dv, gate_act, eps, s)
+                         : head_out_launch<bf16>(o_raw, proj, ld, gate_col, w, 0, out, ldo, T, H, dv, gate_act, eps, s)))
+    return b200_check_launch("b200_linattn_out(heads)");
   const size_t smem = sizeof(float) * H;
   if (f32)
     linattn_out_kernel<float><<<T, 256, smem, s>>>(o_raw, (const float*)proj, ld, gate_col, (const bf16*)w, (float*)out, ldo,

@@ -23,6 +23,7 @@
 // weight and the sigmoid output gate, and rounds to the activation type.
 #include "chunk_scan.cuh"
 #include "common.cuh"
+#include "head_out.cuh"
 #include "runtime.h"
 #include "../../include/b200.h"
 
@@ -938,6 +939,9 @@ extern "C" int b200_mlstm_out(const float* o_raw, const void* proj, int f32, int
   B200_REQUIRE(T >= 0 && H > 0 && dv > 0 && dv <= 32 * kOutPer, "mlstm_out: bad shape (value width <= %d)", 32 * kOutPer);
   if (T == 0) return B200_OK;
   cudaStream_t s = (cudaStream_t)stream;
+  if (f32 ? head_out_launch<float>(o_raw, proj, ld, gate_col, norm_w, dv, out, ldo, T, H, dv, 0, eps, s)
+          : head_out_launch<bf16>(o_raw, proj, ld, gate_col, norm_w, dv, out, ldo, T, H, dv, 0, eps, s))
+    return b200_check_launch("b200_mlstm_out(heads)");
   const int grid = (int)(((size_t)T * H + kOutWarps - 1) / kOutWarps);
   if (f32)
     mlstm_out_kernel<float><<<grid, kOutWarps * 32, 0, s>>>(o_raw, (const float*)proj, ld, gate_col, (const bf16*)norm_w,

@@ -142,40 +142,43 @@ rot_prep_kernel(RotPrepArgs a) {
   }
 }
 
-// The same steps with 16-byte accesses, one CTA per token: the token's cos / sin are computed ONCE (dims / 2 angles)
-// into shared memory and used by every head.  A head is cut into items of VEC = 16 bytes / sizeof(TA) entries: an
+// The same steps with 16-byte accesses, TOK tokens per CTA: a token's cos / sin are computed ONCE (dims / 2 angles)
+// into shared memory and used by every head.  A CTA of one token is one chain of latencies (position, angles, rows, stores);
+// four tokens share it, which is what a prompt's rows are bound by, and single rows keep a CTA each.  A head is cut into items of VEC = 16 bytes / sizeof(TA) entries: an
 // interleaved rotation turns the pairs inside an item; a half-split rotation makes an item of the piece [d, d + VEC)
 // and its partner [d + dims/2, ...); the unrotated rest are plain items.  LPH lanes (a power of two >= items per
 // head) share a head, a warp covers 32 / LPH head slots at a time, the sum of squares is reduced inside the group.
 constexpr int kRvThreads = 256;
 
-template <typename TA, typename TD>
+template <typename TA, typename TD, int TOK>
 __global__ void __launch_bounds__(kRvThreads)
-rot_prep_vec_kernel(RotPrepArgs a, int lph, int items_q, int items_v) {
+rot_prep_vec_kernel(RotPrepArgs a, int T, int lph, int items_q, int items_v) {
   constexpr int VEC = 16 / (int)sizeof(TA);
-  extern __shared__ float2 cs[];                      // [dims / 2] (cos, sin) of this token
-  const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  extern __shared__ float2 cs_all[];                  // [TOK][dims / 2] (cos, sin) of the tokens
+  const int tok0 = blockIdx.x * TOK, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int H = a.H, G = a.G, dk = a.dk, dv = a.dv, dims = a.dims, half = dims >> 1;
   if (dims > 0) {
-    const int pos = a.positions[t];
-    for (int j = threadIdx.x; j < half; j += kRvThreads) {
-      const double ang = (double)pos * a.freq[j];
+    for (int i = threadIdx.x; i < half * TOK; i += kRvThreads) {
+      const int e = TOK == 1 ? 0 : i / half, j = i - e * half;
+      if (tok0 + e >= T) break;
+      const double ang = (double)a.positions[tok0 + e] * a.freq[j];
       const float rem = (float)(ang - 6.283185307179586 * rint(ang * 0.15915494309189535));
       float sn, c;
       sincosf(rem, &sn, &c);
-      cs[j] = make_float2(c, sn);
+      cs_all[i] = make_float2(c, sn);
     }
     __syncthreads();
   }
   const bool has_v = a.v_col >= 0;
   const int n_slots = a.k_out == nullptr ? H : H + G + (has_v ? G : 0);    // no key destination: queries only
   const int per_warp = 32 / lph, sub = lane / lph, li = lane % lph;
-  const int slot = a.paged ? a.slots[t] : 0;
-  const TA* row = reinterpret_cast<const TA*>(a.proj) + (size_t)t * a.ld;
   const int n_rot = dims == 0 ? 0 : (a.half_layout ? half / VEC : dims / VEC);
-  for (int hs0 = warp * per_warp; hs0 < n_slots; hs0 += (kRvThreads / 32) * per_warp) {
-    const int hs = hs0 + sub;
-    const bool live = hs < n_slots;
+  for (int hs0 = warp * per_warp; hs0 < n_slots * TOK; hs0 += (kRvThreads / 32) * per_warp) {
+    const int e = TOK == 1 ? 0 : (hs0 + sub) / n_slots, hs = hs0 + sub - e * n_slots, t = tok0 + e;
+    const bool live = e < TOK && hs < n_slots && t < T;
+    const int slot = live && a.paged ? a.slots[t] : 0;
+    const TA* row = reinterpret_cast<const TA*>(a.proj) + (size_t)t * a.ld;
+    const float2* cs = cs_all + e * half;
     const bool is_q = live && hs < H, is_k = live && !is_q && hs < H + G, is_v = live && !is_q && !is_k;
     const int g = is_q ? hs : (is_k ? hs - H : hs - H - G);
     const bool act = live && li < (is_v ? items_v : items_q) && (is_q || !a.paged || slot >= 0);
@@ -325,10 +328,15 @@ extern "C" int b200_rot_prep_hm(const void* proj, int src_f32, int64_t ld, int q
     if (ok) {
       int lph = 1;
       while (lph < items) lph <<= 1;
+      // four tokens per CTA once that still leaves every SM eight CTAs (and their angles fit the default shared memory)
       const size_t smem = (size_t)(dims / 2) * sizeof(float2);
-      if (src_f32) rot_prep_vec_kernel<float, float><<<T, kRvThreads, smem, s>>>(a, lph, items_q, items_v);
-      else if (dst_f32) rot_prep_vec_kernel<bf16, float><<<T, kRvThreads, smem, s>>>(a, lph, items_q, items_v);
-      else rot_prep_vec_kernel<bf16, bf16><<<T, kRvThreads, smem, s>>>(a, lph, items_q, items_v);
+      if (T >= 4 * 8 * 148 && 4 * smem <= 40 * 1024) {
+        if (src_f32) rot_prep_vec_kernel<float, float, 4><<<(T + 3) / 4, kRvThreads, 4 * smem, s>>>(a, T, lph, items_q, items_v);
+        else if (dst_f32) rot_prep_vec_kernel<bf16, float, 4><<<(T + 3) / 4, kRvThreads, 4 * smem, s>>>(a, T, lph, items_q, items_v);
+        else rot_prep_vec_kernel<bf16, bf16, 4><<<(T + 3) / 4, kRvThreads, 4 * smem, s>>>(a, T, lph, items_q, items_v);
+      } else if (src_f32) rot_prep_vec_kernel<float, float, 1><<<T, kRvThreads, smem, s>>>(a, T, lph, items_q, items_v);
+      else if (dst_f32) rot_prep_vec_kernel<bf16, float, 1><<<T, kRvThreads, smem, s>>>(a, T, lph, items_q, items_v);
+      else rot_prep_vec_kernel<bf16, bf16, 1><<<T, kRvThreads, smem, s>>>(a, T, lph, items_q, items_v);
       return b200_check_launch("b200_rot_prep");
     }
   }
