@@ -172,16 +172,46 @@ struct ChunkTile<float, ROWS, W, PITCH> {
   __device__ __forceinline__ void land(float*) const {}
 };
 
-template <int DK, int VT>
+// Running sums of a chunk's logarithms per key channel, inclusive: F[t][k] = sum_(r <= t) lg(r, k), 256 threads, four runs of 16
+// rows each.  hi / lo: [64][DK + 4].  Ends with a barrier.
+template <int DK, typename LG>
+__device__ __forceinline__ void cs_channel_sums(float* hi, float* lo, double* run, LG lg) {
+  constexpr int RUNS = kCsThreads / DK, ROWS = kCsRows / RUNS, P = DK + 4;
+  const int k = (int)threadIdx.x % DK, r = (int)threadIdx.x / DK;
+  double sum = 0.0;
+#pragma unroll 4
+  for (int t = r * ROWS; t < (r + 1) * ROWS; ++t) sum += (double)lg(t, k);
+  run[r * DK + k] = sum;
+  __syncthreads();
+  double F = 0.0;
+  for (int i = 0; i < r; ++i) F += run[i * DK + k];
+#pragma unroll 4
+  for (int t = r * ROWS; t < (r + 1) * ROWS; ++t) {
+    F += (double)lg(t, k);
+    const float h = (float)F;
+    hi[t * P + k] = h;
+    lo[t * P + k] = (float)(F - (double)h);
+  }
+  __syncthreads();
+}
+// 2^(h + l) of a sum's two parts
+__device__ __forceinline__ float cs_exp2(float h, float l) { return ex2_approx(h) * fmaf(l, 0.6931471805599453f, 1.0f); }
+
+template <int DK, int VT, bool VECTOR = false>
 struct ChunkSmem {
-  static constexpr int kState = kCsRows * (DK + VT);         // floats
+  static constexpr int kSums = VECTOR ? 2 * kCsRows * (DK + 4) : 0;          // running sums, two parts
+  static constexpr int kState = kCsRows * (DK + VT) + kSums; // floats
   static constexpr int kTile = 32 * VT;                      // a tile of 32 state or value rows
   static constexpr int kB = kCsRows * (DK + 4) > 2 * kTile ? kCsRows * (DK + 4) : 2 * kTile;
-  static constexpr int kOutput = kCsRows * (DK + 4) + kB + kTile + kCsRows * kCsAPitch;
+  static constexpr int kOutput = kCsRows * (DK + 4) + kB + kTile + kCsRows * kCsAPitch + kSums;
 };
 
 // Form: `Scratch` (shared arrays of one chunk), `state_weights` (fills scratch, w(s) and row() for chunk_state), `output_weights`,
 // aq(t), D(t, s), finish() for chunk_output, and `carry` / `carry_row` for chunk_carry.
+// A Form with kVector has one decay per KEY CHANNEL instead: with the running sums F of a chunk's base-2 logarithms per channel
+// (summed in fp64, kept as two fp32 parts, so that a difference is as exact as an fp32 product of decays) the keys of the state
+// are weighted by 2^(F_n - F_s), the queries of the state's part by 2^F_t, and (k_s . q_t) is a sum of k q 2^(F_t - F_s) formed
+// term by term: 64 * 65 / 2 exponentials per channel, but none of a positive number, whatever the decays are.
 template <int DK, int VT, typename TA, typename Form>
 __global__ void __launch_bounds__(kCsThreads, 2)
 chunk_state_kernel(const ChunkScanArgs a, const typename Form::Params p) {
@@ -204,7 +234,10 @@ chunk_state_kernel(const ChunkScanArgs a, const typename Form::Params p) {
     vt[e].issue(x, a.ld, at.first + 32 * e, at.rows - 32 * e, vcol, a.dv - v0, vs + 32 * e * VT);
     cp_async_commit();
   }
-  Form::state_weights(p, a, scratch, h, at);
+  float* hi = vs + kCsRows * VT;   // [64][DK + 4] each, kVector only
+  float* lo = hi + kCsRows * (DK + 4);
+  if constexpr (Form::kVector) Form::template sums<DK>(p, a, scratch, h, at, hi, lo);
+  else Form::state_weights(p, a, scratch, h, at);
   constexpr int KI = DK / 64, VJ = VT / 64;
   const int vg = tid & 15, kg = tid >> 4;
   cs_f2 acc[KI * 4][VJ * 2];
@@ -220,10 +253,20 @@ chunk_state_kernel(const ChunkScanArgs a, const typename Form::Params p) {
     else cp_async_wait<0>();
     __syncthreads();
     const int n = min(at.rows - 32 * e, 32);
+    if constexpr (Form::kVector) {
+      const float* Fh = hi + (at.rows - 1) * (DK + 4);
+      const float* Fl = lo + (at.rows - 1) * (DK + 4);
+      for (int i = tid; i < n * DK; i += kCsThreads) {
+        const int s = 32 * e + i / DK, k = i % DK;
+        ks[s * DK + k] *= cs_exp2(Fh[k] - hi[s * (DK + 4) + k], Fl[k] - lo[s * (DK + 4) + k]);
+      }
+      __syncthreads();
+    }
 #pragma unroll 4
     for (int r = 0; r < n; ++r) {
       const int s = 32 * e + r;
-      const float w = scratch.w[s];
+      float w = 1.0f;
+      if constexpr (!Form::kVector) w = scratch.w[s];
       float4 kk[KI];
       ulonglong2 vv[VJ];
 #pragma unroll
@@ -251,7 +294,14 @@ chunk_state_kernel(const ChunkScanArgs a, const typename Form::Params p) {
       const int k = 4 * kg + 64 * (i >> 2) + (i & 3), v = v0 + 4 * vg + 64 * j;
       if (v < a.dv) *reinterpret_cast<ulonglong2*>(out + (size_t)k * a.dv + v) = make_ulonglong2(acc[i][2 * j], acc[i][2 * j + 1]);
     }
-  if (blockIdx.z == 0) Form::template state_row<DK>(a, scratch, ks, h, at.rows);
+  if constexpr (Form::kVector) {
+    if (blockIdx.z == 0 && tid < DK) {
+      const int i = (at.rows - 1) * (DK + 4) + tid;
+      a.ws_row[((size_t)blockIdx.x * a.H + h) * a.ws_row_width + tid] = cs_exp2(hi[i], lo[i]);
+    }
+  } else if (blockIdx.z == 0) {
+    Form::template state_row<DK>(a, scratch, ks, h, at.rows);
+  }
 }
 
 // 8 keys x 128 values of a head's state through a sequence's chunks: a warp's row of a chunk is 512 contiguous bytes, eight
@@ -284,7 +334,7 @@ chunk_carry_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   const bool live = v0 + v < a.dv;
   const size_t step = (size_t)a.H * DK * a.dv;
   float* C = a.ws + ((size_t)base * a.H + h) * DK * a.dv + (size_t)(k0 + k) * a.dv + v0 + v;
-  typename Form::Carry carry(p, a, s, h, base, fresh, slot);
+  typename Form::Carry carry(p, a, s, h, base, k0 + k);
   constexpr int U = kCsCarryDepth;
   for (int c0 = 0; c0 < nc; c0 += U) {
     float4 in[U];
@@ -363,6 +413,8 @@ chunk_output_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   float* X = qs + kCsRows * QP;                      // ring of three tiles of 32 rows; the keys [64][DK + 4] first lie on tiles 1 and 2
   float* B = X + TILE;
   float* A = B + ChunkSmem<DK, VT>::kB;              // [64][68]
+  float* hi = A + kCsRows * kCsAPitch;               // [64][DK + 4] each, kVector only
+  float* lo = hi + kCsRows * QP;
   const TA* x = reinterpret_cast<const TA*>(a.x);
   const int hg = h / (a.H / a.G), vcol = a.v_col + h * a.dv + v0;
   const bool zero_start = at.local == 0 && a.ctx_lens[at.seq] == 0;
@@ -388,7 +440,8 @@ chunk_output_kernel(const ChunkScanArgs a, const typename Form::Params p) {
     k.issue(x, a.ld, at.first, n, a.k_col + hg * DK, DK, B);
     cp_async_commit();
     issue(0);
-    Form::output_weights(p, a, scratch, h, at);
+    if constexpr (Form::kVector) Form::template sums<DK>(p, a, scratch, h, at, hi, lo);
+    else Form::output_weights(p, a, scratch, h, at);
     q.land(qs);
     k.land(B);
   }
@@ -396,7 +449,50 @@ chunk_output_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   __syncthreads();
   const float q_scale = Form::q_scale(p);
   const int tg = tid >> 4, vg = tid & 15;
-  {
+  if constexpr (Form::kVector) {
+    float acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+#pragma unroll 1
+    for (int d = 0; d < DK; d += 4) {
+      float4 k[4], kh[4], kl[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int at_ = (vg + 16 * j) * QP + d;
+        k[j] = *reinterpret_cast<const float4*>(B + at_);
+        kh[j] = *reinterpret_cast<const float4*>(hi + at_);
+        kl[j] = *reinterpret_cast<const float4*>(lo + at_);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int at_ = (tg + 16 * i) * QP + d;
+        const float4 q = *reinterpret_cast<const float4*>(qs + at_), qh = *reinterpret_cast<const float4*>(hi + at_),
+                     ql = *reinterpret_cast<const float4*>(lo + at_);
+#pragma unroll
+        for (int j = 0; j <= i; ++j) {
+          acc[i][j] = fmaf(q.x * k[j].x, ex2_approx((qh.x - kh[j].x) + (ql.x - kl[j].x)), acc[i][j]);
+          acc[i][j] = fmaf(q.y * k[j].y, ex2_approx((qh.y - kh[j].y) + (ql.y - kl[j].y)), acc[i][j]);
+          acc[i][j] = fmaf(q.z * k[j].z, ex2_approx((qh.z - kh[j].z) + (ql.z - kl[j].z)), acc[i][j]);
+          acc[i][j] = fmaf(q.w * k[j].w, ex2_approx((qh.w - kh[j].w) + (ql.w - kl[j].w)), acc[i][j]);
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j <= i; ++j) {
+        const int t = tg + 16 * i, s = vg + 16 * j;
+        A[t * kCsAPitch + s] = (s <= t && t < n) ? acc[i][j] * q_scale : 0.f;
+      }
+    __syncthreads();                                 // the queries as they came are used
+    if (!zero_start)
+      for (int i = tid; i < n * DK; i += kCsThreads) {
+        const int at_ = i / DK * QP + i % DK;
+        qs[at_] *= cs_exp2(hi[at_], lo[at_]);
+      }
+  } else {
     // k_s . q_t: rows t = tg + 16 i, columns s = vg + 16 j, j <= i; even and odd entries summed apart
     cs_f2 acc[4][4];
 #pragma unroll
@@ -490,7 +586,7 @@ template <int DK, int VT, typename TA, typename Form>
 int cs_launch_shape(const ChunkScanArgs& a, const typename Form::Params& p, int64_t rows, cudaStream_t s) {
   const int64_t chunks = cs_max_chunks(rows, a.n_seqs);
   const dim3 grid((unsigned)chunks, a.H, (a.dv + VT - 1) / VT);
-  const int sb = ChunkSmem<DK, VT>::kState * 4, ob = ChunkSmem<DK, VT>::kOutput * 4;
+  const int sb = ChunkSmem<DK, VT, Form::kVector>::kState * 4, ob = ChunkSmem<DK, VT, Form::kVector>::kOutput * 4;
   cudaError_t e = cudaFuncSetAttribute(chunk_state_kernel<DK, VT, TA, Form>, cudaFuncAttributeMaxDynamicSharedMemorySize, sb);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(chunk_output_kernel<DK, VT, TA, Form>, cudaFuncAttributeMaxDynamicSharedMemorySize, ob);
   if (e != cudaSuccess) {

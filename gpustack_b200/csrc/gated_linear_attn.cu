@@ -11,6 +11,7 @@
 // is then two FMAs per held element with the token's k, q and alpha broadcast from shared memory -- no shuffle; the
 // warps' partial sums of S^T q meet in shared memory once per 16 staged tokens and are added in warp order (a fixed
 // order, whatever the cut of the prompt).  A sequence's new rows run in order, 16 staged at a time.
+#include "chunk_scan.cuh"
 #include "common.cuh"
 #include "runtime.h"
 #include "../../include/b200.h"
@@ -42,7 +43,8 @@ template <int RPW>
 __global__ void __launch_bounds__(kGlWarps * 32)
 gla_scan_kernel(const float* __restrict__ x, int64_t ld, int q_col, int k_col, int v_col, const float* __restrict__ z,
                 int64_t ldz, float inv_tau, const int32_t* __restrict__ cu_seq, const int32_t* __restrict__ ctx_lens,
-                const int32_t* __restrict__ state_slots, float* S_state, float* __restrict__ o_raw, int H, int dk, int dv) {
+                const int32_t* __restrict__ state_slots, float* S_state, float* __restrict__ o_raw, int H, int dk, int dv,
+                int most_rows) {
   extern __shared__ __align__(16) float smem[];
   constexpr int DKP = RPW * kGlWarps;                 // key rows, padded to the warps' shares
   float* qs = smem;                                   // [16][DKP]
@@ -54,7 +56,7 @@ gla_scan_kernel(const float* __restrict__ x, int64_t ld, int q_col, int k_col, i
   const int slot = state_slots[s];
   if (slot < 0) return;
   const int t0 = cu_seq[s], t1 = cu_seq[s + 1];
-  if (t1 <= t0) return;
+  if (t1 <= t0 || t1 - t0 > most_rows) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int col = zc * kGlCols + lane, r0 = warp * RPW;
   float* Sp = S_state + ((size_t)slot * H + h) * dv * dk;
@@ -129,6 +131,59 @@ gla_scan_kernel(const float* __restrict__ x, int64_t ld, int q_col, int k_col, i
   for (int j = 0; j < RPW; ++j)
     if (r0 + j < dk && col < dv) Sp[(size_t)col * dk + r0 + j] = S[j];
 }
+
+// The decays of the chunk form: base-2 logarithms of sigmoid(z)^(1/tau) and their running sums per key channel.  What rounds to
+// zero as a decay (below 2^-10000) is cut there, so that sums stay finite; 2^ of them is zero all the same.
+struct GatedLinearForm {
+  static constexpr const char* kName = "b200_gla_scan(chunks)";
+  static constexpr bool kVector = true;
+  struct Params {
+    const float* z;
+    int64_t ldz;
+    float inv_tau;
+  };
+  struct Scratch {
+    double run[kCsThreads];
+  };
+  template <int DK>
+  static __device__ __forceinline__ void sums(const Params& p, const ChunkScanArgs&, Scratch& sc, int h, const ChunkPlace& at, float* hi, float* lo) {
+    for (int i = threadIdx.x; i < kCsRows * DK; i += kCsThreads) {
+      const int t = i / DK, k = i % DK;
+      float lg = 0.f;
+      if (t < at.rows) {
+        const float z = p.z[(size_t)(at.first + t) * p.ldz + h * DK + k];
+        lg = (fminf(z, 0.f) - log1pf(expf(-fabsf(z)))) * p.inv_tau * 1.4426950408889634f;
+        if (lg < -1.0e4f) lg = -1.0e4f;
+      }
+      lo[t * (DK + 4) + k] = lg;
+    }
+    __syncthreads();
+    cs_channel_sums<DK>(hi, lo, sc.run, [&](int t, int k) { return lo[t * (DK + 4) + k]; });
+  }
+  struct Carry {
+    const float* row;
+    size_t step;
+    float f[kCsCarryDepth];
+    __device__ __forceinline__ Carry(const Params&, const ChunkScanArgs& a, int, int h, int base, int k)
+        : row(a.ws_row + ((size_t)base * a.H + h) * a.ws_row_width + k), step((size_t)a.H * a.ws_row_width) {}
+    __device__ __forceinline__ void fetch(const ChunkScanArgs&, int c0, int nc) {
+#pragma unroll
+      for (int u = 0; u < kCsCarryDepth; ++u)
+        if (c0 + u < nc) f[u] = row[(c0 + u) * step];
+    }
+    __device__ __forceinline__ void next(const Params&, int u, int, float& a, float& b) {
+      a = f[u];
+      b = 1.0f;
+    }
+  };
+  template <int DK>
+  static __device__ __forceinline__ void carry_row(const Params&, const ChunkScanArgs&, int, int, int, int, bool, int) {}
+  static __device__ __forceinline__ float q_scale(const Params&) { return 1.0f; }
+  static __device__ __forceinline__ float aq(const Scratch&, int) { return 1.0f; }
+  template <int DK>
+  static __device__ __forceinline__ void rows(const Params&, const ChunkScanArgs&, Scratch&, const float*, const float*, int, int, bool) {}
+  static __device__ __forceinline__ float4 finish(const Params&, const Scratch&, int, int, float4 acc, float4) { return acc; }
+};
 
 // Single rows (a decode step): lane r holds the key rows r, r + 32, ... of its warp's 4 value columns, so the state is read
 // and written in whole lines; S^T q is a warp-shuffle reduction, which a step of one token can afford.
@@ -225,6 +280,41 @@ extern "C" int b200_gla_scan(const float* x, int64_t ld, int q_col, int k_col, i
                             0, stream);
 }
 
+static int launch_rows(const float* x, int64_t ld, int q_col, int k_col, int v_col, const float* z, int64_t ldz, float inv_tau,
+                       const int32_t* cu_seq, const int32_t* ctx_lens, const int32_t* state_slots, float* S, float* o_raw, int n_seqs,
+                       int H, int dk, int dv, int most_rows, cudaStream_t s) {
+  const dim3 grid(n_seqs, H, (dv + kGlCols - 1) / kGlCols);
+  const int rpw = dk <= 8 ? 1 : dk <= 16 ? 2 : dk <= 32 ? 4 : dk <= 64 ? 8 : dk <= 128 ? 16 : 32;   // key rows per warp
+  const size_t smem = sizeof(float) * (3 * (size_t)kGlTok * rpw * kGlWarps + kGlTok * kGlCols + kGlWarps * kGlTok * kGlCols);
+#define B200_GL(E)                                                                                                     \
+  do {                                                                                                                 \
+    if (smem > 48 * 1024) {                                                                                            \
+      static bool attr = false;                                                                                        \
+      if (!attr) {                                                                                                     \
+        const cudaError_t e_ = cudaFuncSetAttribute(gla_scan_kernel<E>, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
+                                                    (int)smem);                                                        \
+        if (e_ != cudaSuccess) {                                                                                       \
+          b200_set_error("gla_scan: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e_));                    \
+          return B200_ERR_CUDA;                                                                                        \
+        }                                                                                                              \
+        attr = true;                                                                                                   \
+      }                                                                                                                \
+    }                                                                                                                  \
+    gla_scan_kernel<E><<<grid, kGlWarps * 32, smem, s>>>(x, ld, q_col, k_col, v_col, z, ldz, inv_tau, cu_seq, ctx_lens, \
+                                                         state_slots, S, o_raw, H, dk, dv, most_rows);                 \
+  } while (0)
+  switch (rpw) {
+    case 1: B200_GL(1); break;
+    case 2: B200_GL(2); break;
+    case 4: B200_GL(4); break;
+    case 8: B200_GL(8); break;
+    case 16: B200_GL(16); break;
+    default: B200_GL(32); break;
+  }
+#undef B200_GL
+  return b200_check_launch("b200_gla_scan");
+}
+
 extern "C" int b200_gla_scan_rows(const float* x, int64_t ld, int q_col, int k_col, int v_col, const float* z, int64_t ldz,
                                   float inv_tau, const int32_t* cu_seq, const int32_t* ctx_lens, const int32_t* state_slots,
                                   float* S, float* o_raw, int n_seqs, int H, int dk, int dv, int max_len, void* stream) {
@@ -245,33 +335,27 @@ extern "C" int b200_gla_scan_rows(const float* x, int64_t ld, int q_col, int k_c
 #undef B200_GS
     return b200_check_launch("b200_gla_scan");
   }
-  const int rpw = dk <= 8 ? 1 : dk <= 16 ? 2 : dk <= 32 ? 4 : dk <= 64 ? 8 : dk <= 128 ? 16 : 32;   // key rows per warp
-  const size_t smem = sizeof(float) * (3 * (size_t)kGlTok * rpw * kGlWarps + kGlTok * kGlCols + kGlWarps * kGlTok * kGlCols);
-#define B200_GL(E)                                                                                                     \
-  do {                                                                                                                 \
-    if (smem > 48 * 1024) {                                                                                            \
-      static bool attr = false;                                                                                        \
-      if (!attr) {                                                                                                     \
-        const cudaError_t e_ = cudaFuncSetAttribute(gla_scan_kernel<E>, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
-                                                    (int)smem);                                                        \
-        if (e_ != cudaSuccess) {                                                                                       \
-          b200_set_error("gla_scan: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e_));                    \
-          return B200_ERR_CUDA;                                                                                        \
-        }                                                                                                              \
-        attr = true;                                                                                                   \
-      }                                                                                                                \
-    }                                                                                                                  \
-    gla_scan_kernel<E><<<grid, kGlWarps * 32, smem, s>>>(x, ld, q_col, k_col, v_col, z, ldz, inv_tau, cu_seq, ctx_lens, \
-                                                         state_slots, S, o_raw, H, dk, dv);                            \
-  } while (0)
-  switch (rpw) {
-    case 1: B200_GL(1); break;
-    case 2: B200_GL(2); break;
-    case 4: B200_GL(4); break;
-    case 8: B200_GL(8); break;
-    case 16: B200_GL(16); break;
-    default: B200_GL(32); break;
+  return launch_rows(x, ld, q_col, k_col, v_col, z, ldz, inv_tau, cu_seq, ctx_lens, state_slots, S, o_raw, n_seqs, H, dk, dv, INT32_MAX, s);
+}
+
+// The same with a workspace: portions of more than 16 rows over their chunks side by side, the others one-pass beside them.
+// Shapes and alignments that the chunk kernels do not take run as b200_gla_scan_rows.
+extern "C" int b200_gla_scan_chunked(const float* x, int64_t ld, int q_col, int k_col, int v_col, const float* z, int64_t ldz,
+                                     float inv_tau, const int32_t* cu_seq, const int32_t* ctx_lens, const int32_t* state_slots,
+                                     float* S, float* o_raw, int n_seqs, int H, int dk, int dv, int max_len, int rows,
+                                     float* workspace, int64_t workspace_floats, void* stream) {
+  if (workspace == nullptr || rows <= 0 || n_seqs <= 0 || H <= 0 || dv <= 0 || ((uintptr_t)workspace & 15) != 0 ||
+      !cs_covers(x, 4, ld, q_col, k_col, v_col, dk, dv, S, o_raw))
+    return b200_gla_scan_rows(x, ld, q_col, k_col, v_col, z, ldz, inv_tau, cu_seq, ctx_lens, state_slots, S, o_raw, n_seqs, H, dk, dv,
+                              max_len, stream);
+  B200_REQUIRE(workspace_floats >= cs_workspace_floats(rows, n_seqs, H, dk, dv), "gla_scan: workspace of %lld floats too small",
+               (long long)workspace_floats);
+  cudaStream_t s = (cudaStream_t)stream;
+  if (n_seqs > 1 || rows <= kCsShort) {
+    const int rc = launch_rows(x, ld, q_col, k_col, v_col, z, ldz, inv_tau, cu_seq, ctx_lens, state_slots, S, o_raw, n_seqs, H, dk, dv,
+                               kCsShort, s);
+    if (rc != B200_OK) return rc;
   }
-#undef B200_GL
-  return b200_check_launch("b200_gla_scan");
+  const ChunkScanArgs a{x, ld, q_col, k_col, v_col, H, H, dv, cu_seq, ctx_lens, state_slots, n_seqs, S, o_raw};
+  return cs_launch<float, GatedLinearForm>(a, {z, ldz, inv_tau}, dk, rows, workspace, s);
 }

@@ -17,6 +17,8 @@
 // per lane and serve its C columns: with one column that read, not the arithmetic, bounds the walk.  Keys, queries, values and gates are staged 16 or 32 tokens at a time by
 // cp.async into two buffers, so the walk never waits for memory; a column's sums do not depend on how a prompt was cut
 // beyond the order of the lanes' addends in S^T q.
+// The state-space recurrence over prompts, with a workspace, runs over chunks of 64 rows side by side instead (chunk_scan.cuh).
+#include "chunk_scan.cuh"
 #include "common.cuh"
 #include "runtime.h"
 #include "../../include/b200.h"
@@ -40,6 +42,7 @@ struct GatedScanArgs {
   float* S;
   float* o;                        // [T][H dv]
   int H, G, dkp, dv, dvp;
+  int most_rows;                   // sequences with more new rows are another kernel's
 };
 
 // two fp32 numbers in one 64-bit register pair: the packed fused multiply-add of sm_100
@@ -175,7 +178,7 @@ gated_scan_kernel(GatedScanArgs a) {
   const int slot = a.state_slots[s];
   if (slot < 0) return;
   const int t0 = a.cu_seq[s], t1 = a.cu_seq[s + 1];
-  if (t1 <= t0) return;
+  if (t1 <= t0 || t1 - t0 > a.most_rows) return;
   const int warp = tid >> 5, lane = tid & 31, l = lane % L;
   const int cw = warp * CPW + lane / L * C, col = z * COLS + cw;     // this lane's first column, in the CTA and in the head
   const int hk = h / (a.H / a.G);
@@ -410,6 +413,105 @@ int gated_scan_pick(const GatedScanArgs& a, int n_seqs, int max_len, cudaStream_
   return gated_scan_form<32, 4, 32, 4, DELTA>(a, n_seqs, max_len, s);
 }
 
+// The state-space recurrence in the chunk form: log decays of a chunk's rows summed in fp64, every exponent <= 0.
+//   ws_row[dk] of a chunk: its whole decay
+struct StateSpaceForm {
+  static constexpr const char* kName = "b200_gated_scan(chunks)";
+  static constexpr bool kVector = false;
+  struct Params {
+    const float* gates;
+    int64_t ld_g;
+    const float* rate;
+    const float* dt_bias;
+    const float* skip;
+  };
+  struct Scratch {
+    double F[kCsRows];
+    float beta[kCsRows], w[kCsRows], aq[kCsRows], all;
+  };
+  // warp 0, two rows per lane
+  static __device__ __forceinline__ void sums(const Params& p, int h, const ChunkPlace& at, double (&F)[2], float (&beta)[2]) {
+    const int lane = threadIdx.x & 31;
+    const float rate = p.rate[h], bias = p.dt_bias[h];
+    double f[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int t = 2 * lane + e;
+      f[e] = 0.0;
+      beta[e] = 0.f;
+      if (t < at.rows) {
+        beta[e] = gs_softplus(p.gates[(size_t)(at.first + t) * p.ld_g + h] + bias);
+        f[e] = (double)(-rate * beta[e]);
+      }
+    }
+    double sum = f[0] + f[1];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double v = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += v;
+    }
+    F[1] = sum;
+    F[0] = sum - f[1];
+  }
+  static __device__ __forceinline__ void state_weights(const Params& p, const ChunkScanArgs&, Scratch& sc, int h, const ChunkPlace& at) {
+    if (threadIdx.x < 32) {
+      double F[2];
+      float beta[2];
+      sums(p, h, at, F, beta);
+      const double Fn = __shfl_sync(0xffffffffu, F[1], 31);        // rows behind the last one decay by nothing
+#pragma unroll
+      for (int e = 0; e < 2; ++e) sc.w[2 * threadIdx.x + e] = expf((float)(Fn - F[e])) * beta[e];
+      if (threadIdx.x == 0) sc.all = expf((float)Fn);
+    }
+    __syncthreads();
+  }
+  template <int DK>
+  static __device__ __forceinline__ void state_row(const ChunkScanArgs& a, const Scratch& sc, const float*, int h, int) {
+    if (threadIdx.x == 0) a.ws_row[((size_t)blockIdx.x * a.H + h) * a.ws_row_width + DK] = sc.all;
+  }
+  struct Carry {
+    const float* row;
+    size_t step;
+    float f[kCsCarryDepth];
+    __device__ __forceinline__ Carry(const Params&, const ChunkScanArgs& a, int, int h, int base, int)
+        : row(a.ws_row + ((size_t)base * a.H + h) * a.ws_row_width + a.ws_row_width - 4), step((size_t)a.H * a.ws_row_width) {}
+    __device__ __forceinline__ void fetch(const ChunkScanArgs&, int c0, int nc) {
+#pragma unroll
+      for (int u = 0; u < kCsCarryDepth; ++u)
+        if (c0 + u < nc) f[u] = row[(c0 + u) * step];
+    }
+    __device__ __forceinline__ void next(const Params&, int u, int, float& a, float& b) {
+      a = f[u];
+      b = 1.0f;
+    }
+  };
+  template <int DK>
+  static __device__ __forceinline__ void carry_row(const Params&, const ChunkScanArgs&, int, int, int, int, bool, int) {}
+  static __device__ __forceinline__ void output_weights(const Params& p, const ChunkScanArgs&, Scratch& sc, int h, const ChunkPlace& at) {
+    if (threadIdx.x < 32) {
+      double F[2];
+      float beta[2];
+      sums(p, h, at, F, beta);
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int t = 2 * threadIdx.x + e;
+        sc.F[t] = F[e];
+        sc.beta[t] = beta[e];
+        sc.aq[t] = expf((float)F[e]);
+      }
+    }
+  }
+  static __device__ __forceinline__ float q_scale(const Params&) { return 1.0f; }
+  static __device__ __forceinline__ float D(const Params&, const Scratch& sc, int t, int s) { return expf((float)(sc.F[t] - sc.F[s])) * sc.beta[s]; }
+  static __device__ __forceinline__ float aq(const Scratch& sc, int t) { return sc.aq[t]; }
+  template <int DK>
+  static __device__ __forceinline__ void rows(const Params&, const ChunkScanArgs&, Scratch&, const float*, const float*, int, int, bool) {}
+  static __device__ __forceinline__ float4 finish(const Params& p, const Scratch&, int h, int, float4 v, float4 x) {
+    const float s = p.skip != nullptr ? p.skip[h] : 0.f;
+    return p.skip != nullptr ? make_float4(fmaf(s, x.x, v.x), fmaf(s, x.y, v.y), fmaf(s, x.z, v.z), fmaf(s, x.w, v.w)) : v;
+  }
+};
+
 // ------------------------------------------------------------------------------------------- out
 // out = RMSnorm over `parts` equal pieces of (y * silu(z)), times w[channel] -- the gate BEFORE the norm -- or, with the gate
 // AFTER it, RMSnorm of the pieces of y times w[place in the piece] (one weight vector for all pieces) times silu(z).  One CTA
@@ -548,9 +650,33 @@ extern "C" int b200_gated_scan(const float* x, int64_t ld, int q_col, int k_col,
                "gated_scan: rows, columns and state in whole 16-byte pieces");
   if (n_seqs == 0) return B200_OK;
   const GatedScanArgs a{x, ld, q_col, k_col, v_col, gates, ld_g, rate, dt_bias, skip, cu_seq, ctx_lens, state_slots, S, o_raw, H, G,
-                        (dk + 3) & ~3, dv, (dv + 3) & ~3};
+                        (dk + 3) & ~3, dv, (dv + 3) & ~3, INT32_MAX};
   cudaStream_t s = (cudaStream_t)stream;
   return delta ? gated_scan_pick<true>(a, n_seqs, max_len, s) : gated_scan_pick<false>(a, n_seqs, max_len, s);
+}
+
+// The state-space form with a workspace: portions of more than 16 rows over their chunks side by side, the others one-pass beside
+// them.  The delta rule, and shapes and alignments that the chunk kernels do not take, run as b200_gated_scan.
+extern "C" int b200_gated_scan_chunked(const float* x, int64_t ld, int q_col, int k_col, int v_col, const float* gates, int64_t ld_g,
+                                       const float* rate, const float* dt_bias, const float* skip, const int32_t* cu_seq,
+                                       const int32_t* ctx_lens, const int32_t* state_slots, float* S, float* o_raw, int n_seqs, int H,
+                                       int G, int dk, int dv, int delta, int max_len, int rows, float* workspace,
+                                       int64_t workspace_floats, void* stream) {
+  if (delta || workspace == nullptr || rows <= 0 || n_seqs <= 0 || H <= 0 || G <= 0 || H % G != 0 || dv <= 0 ||
+      ((uintptr_t)workspace & 15) != 0 || !cs_covers(x, 4, ld, q_col, k_col, v_col, dk, dv, S, o_raw))
+    return b200_gated_scan(x, ld, q_col, k_col, v_col, gates, ld_g, rate, dt_bias, skip, cu_seq, ctx_lens, state_slots, S, o_raw, n_seqs, H,
+                           G, dk, dv, delta, max_len, stream);
+  B200_REQUIRE(workspace_floats >= cs_workspace_floats(rows, n_seqs, H, dk, dv), "gated_scan: workspace of %lld floats too small",
+               (long long)workspace_floats);
+  cudaStream_t s = (cudaStream_t)stream;
+  if (n_seqs > 1 || rows <= kCsShort) {
+    const GatedScanArgs one{x, ld, q_col, k_col, v_col, gates, ld_g, rate, dt_bias, skip, cu_seq, ctx_lens, state_slots, S, o_raw, H, G,
+                            dk, dv, dv, kCsShort};
+    const int rc = gated_scan_pick<false>(one, n_seqs, kCsShort, s);
+    if (rc != B200_OK) return rc;
+  }
+  const ChunkScanArgs a{x, ld, q_col, k_col, v_col, H, G, dv, cu_seq, ctx_lens, state_slots, n_seqs, S, o_raw};
+  return cs_launch<float, StateSpaceForm>(a, {gates, ld_g, rate, dt_bias, skip}, dk, rows, workspace, s);
 }
 
 extern "C" int b200_gate_norm(const float* y, const void* proj, int f32, int64_t ld, int z_col, const void* w, void* out,

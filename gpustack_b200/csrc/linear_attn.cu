@@ -379,6 +379,7 @@ __device__ __forceinline__ float la_power(float d, int n) {
 
 struct LinearForm {
   static constexpr const char* kName = "b200_linattn_scan(chunks)";
+  static constexpr bool kVector = false;
   struct Params {
     const float* decay;
   };
@@ -393,7 +394,7 @@ struct LinearForm {
   static __device__ __forceinline__ void state_row(const ChunkScanArgs&, const Scratch&, const float*, int, int) {}
   struct Carry {
     float d, full;
-    __device__ __forceinline__ Carry(const Params& p, const ChunkScanArgs&, int, int h, int, bool, int) : d(p.decay[h]), full(la_power(d, kCsRows)) {}
+    __device__ __forceinline__ Carry(const Params& p, const ChunkScanArgs&, int, int h, int, int) : d(p.decay[h]), full(la_power(d, kCsRows)) {}
     __device__ __forceinline__ void fetch(const ChunkScanArgs&, int, int) {}
     __device__ __forceinline__ void next(const Params&, int, int rows, float& a, float& b) {
       a = rows == kCsRows ? full : la_power(d, rows);

@@ -627,6 +627,7 @@ static int launch_chunk(const void* proj, int64_t ld, int q_col, int k_col, int 
 //   dk + 3 (first chunk of a sequence): the stabiliser that the sequence came with
 struct MlstmForm {
   static constexpr const char* kName = "b200_mlstm_scan(chunks)";
+  static constexpr bool kVector = false;
   struct Params {
     const float* gates;
     const bf16* gate_bias;
@@ -717,7 +718,7 @@ struct MlstmForm {
     size_t step;
     float m, F[kCsCarryDepth], ml[kCsCarryDepth];
     int width;
-    __device__ __forceinline__ Carry(const Params&, const ChunkScanArgs& a, int, int h, int base, bool, int) {
+    __device__ __forceinline__ Carry(const Params&, const ChunkScanArgs& a, int, int h, int base, int) {
       width = (int)(a.ws_row_width);
       row = a.ws_row + ((size_t)base * a.H + h) * width;
       step = (size_t)a.H * width;

@@ -170,6 +170,8 @@ SIGNATURES = {
                                                   _i32, _i32, _f32, _i32, _i32, _vp, _i64, _vp]),
     "b200_gla_scan": (_i32, [_vp, _i64, _i32, _i32, _i32, _vp, _i64, _f32, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32,
                              _vp]),
+    "b200_gla_scan_chunked": (_i32, [_vp, _i64, _i32, _i32, _i32, _vp, _i64, _f32, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32,
+                                     _i32, _vp, _i64, _vp]),
     "b200_attn_sink_prefill_cap": (_i32, [_vp, _i32, _i64, _i32, _vp, _vp, _vp, _i32, _vp, _vp, _vp, _vp, _i32, _i32, _vp, _vp, _i64,
                    _i32, _i32, _i32, _i32, _i32, _f32, _i64, _i32, _i32, _vp, _vp, _vp, _i32, _i32, _f32, _vp]),
     "b200_attn_sink_decode_cap": (_i32, [_vp, _i32, _i64, _i32, _vp, _vp, _vp, _i32, _vp, _i32, _vp, _vp, _i64, _i32, _i32, _i32, _i32,
@@ -190,6 +192,8 @@ SIGNATURES = {
                                   _vp, _vp, _i64, _f32, _vp]),
     "b200_gated_scan": (_i32, [_vp, _i64, _i32, _i32, _i32, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32,
                                _i32, _i32, _i32, _vp]),
+    "b200_gated_scan_chunked": (_i32, [_vp, _i64, _i32, _i32, _i32, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32,
+                                       _i32, _i32, _i32, _i32, _i32, _vp, _i64, _vp]),
     "b200_gate_norm": (_i32, [_vp, _vp, _i32, _i64, _i32, _vp, _vp, _i64, _i32, _i32, _i32, _i32, _f32, _vp]),
     "b200_prenorm_join": (_i32, [_vp, _vp, _vp, _vp, _vp, _f32, _f32, _vp, _vp, _i32, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _f32,
                                  _f32, _vp]),

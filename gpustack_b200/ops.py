@@ -816,9 +816,15 @@ def gla_scan(x, q_col: int, k_col: int, v_col: int, z, inv_tau: float, cu_seq, c
     """Linear attention with the decay sigmoid(z)^inv_tau per key channel and token (csrc/gated_linear_attn.cu)."""
     _cuda(x, z, cu_seq, ctx_lens, state_slots, S, o_raw)
     _req(x, torch.float32, "x"); _req(z, torch.float32, "z"); _req(S, torch.float32, "S"); _req(o_raw, torch.float32, "o_raw")
+    n = state_slots.shape[0]
+    ws = _chunk_scan_workspace(x.shape[0], n, H, dk, dv, max_len, x.device)
+    if ws is not None:
+        check(load().b200_gla_scan_chunked(_p(x), x.stride(0), q_col, k_col, v_col, _p(z), z.stride(0), inv_tau, _p(cu_seq),
+                                           _p(ctx_lens), _p(state_slots), _p(S), _p(o_raw), n, H, dk, dv, int(max_len), x.shape[0],
+                                           _p(ws), ws.numel(), _stream()), "gla_scan")
+        return
     check(load().b200_gla_scan_rows(_p(x), x.stride(0), q_col, k_col, v_col, _p(z), z.stride(0), inv_tau, _p(cu_seq), _p(ctx_lens),
-                                    _p(state_slots), _p(S), _p(o_raw), state_slots.shape[0], H, dk, dv, int(max_len), _stream()),
-          "gla_scan")
+                                    _p(state_slots), _p(S), _p(o_raw), n, H, dk, dv, int(max_len), _stream()), "gla_scan")
 
 
 # ------------------------------------------- a norm on every sublayer's output, convolved q / k / v
@@ -936,8 +942,15 @@ def gated_scan(x, q_col: int, k_col: int, v_col: int, gates, rate, dt_bias, skip
             raise B200Error(f"gated_scan: {n_} is fp32")
     if tuple(S.shape[1:]) != (H, dv, -(-dk // 4) * 4) or not S.is_contiguous() or not o_raw.is_contiguous():
         raise B200Error("gated_scan: a contiguous state of [slots, heads, dv, dk rounded up to 4]")
+    n = state_slots.shape[0]
+    ws = None if delta else _chunk_scan_workspace(x.shape[0], n, H, dk, dv, max_len, x.device)
+    if ws is not None:
+        check(load().b200_gated_scan_chunked(_p(x), x.stride(0), q_col, k_col, v_col, _p(gates), gates.stride(0), _p(rate), _p(dt_bias),
+                                             _p(skip), _p(cu_seq), _p(ctx_lens), _p(state_slots), _p(S), _p(o_raw), n, H, G, dk, dv, 0,
+                                             int(max_len), x.shape[0], _p(ws), ws.numel(), _stream()), "gated_scan")
+        return
     check(load().b200_gated_scan(_p(x), x.stride(0), q_col, k_col, v_col, _p(gates), gates.stride(0), _p(rate), _p(dt_bias), _p(skip),
-                                 _p(cu_seq), _p(ctx_lens), _p(state_slots), _p(S), _p(o_raw), state_slots.shape[0], H, G, dk, dv,
+                                 _p(cu_seq), _p(ctx_lens), _p(state_slots), _p(S), _p(o_raw), n, H, G, dk, dv,
                                  1 if delta else 0, int(max_len), _stream()), "gated_scan")
 
 

@@ -559,6 +559,14 @@ int b200_gla_scan_rows(const float* x, int64_t ld, int q_col, int k_col, int v_c
                   const int32_t* cu_seq, const int32_t* ctx_lens, const int32_t* state_slots, float* S, float* o_raw,
                   int n_seqs, int H, int dk, int dv, int max_len, void* stream);
 
+/* ... with a workspace: sequences of more than 16 rows run with all their chunks of 64 rows side by side.  rows: the rows of x;
+ * workspace: 16-byte aligned, (rows / 64 + min(n_seqs, rows / 17)) * H * (dk * dv + dk + 4) floats.  Widths other than dk 64 /
+ * 128 with dv % 4 == 0, unaligned rows or no workspace: as b200_gla_scan_rows. */
+int b200_gla_scan_chunked(const float* x, int64_t ld, int q_col, int k_col, int v_col, const float* z, int64_t ldz, float inv_tau,
+                          const int32_t* cu_seq, const int32_t* ctx_lens, const int32_t* state_slots, float* S, float* o_raw,
+                          int n_seqs, int H, int dk, int dv, int max_len, int rows, float* workspace, int64_t workspace_floats,
+                          void* stream);
+
 /* ---- a norm on every sublayer's output; convolved q, k and v; capped scores and logits --------------------------- */
 /* z = x_in + LN(v; wb, bb) (layer norm with weight and bias); v is y [T][D], or (yp != NULL) the sum of the top_k rows
  * yp[pair_row[t top_k + j]] plus sigmoid(gate[t ld_gate]) * shared[t] (gate NULL: factor 1; shared NULL: none), or absent
@@ -606,6 +614,14 @@ int b200_gated_scan(const float* x, int64_t ld, int q_col, int k_col, int v_col,
                     const float* rate, const float* dt_bias, const float* skip, const int32_t* cu_seq, const int32_t* ctx_lens,
                     const int32_t* state_slots, float* S, float* o_raw, int n_seqs, int H, int G, int dk, int dv, int delta,
                     int max_len, void* stream);
+/* The state-space form with a workspace: sequences of more than 16 rows run with all their chunks of 64 rows side by side.  rows:
+ * the rows of x; workspace: 16-byte aligned, (rows / 64 + min(n_seqs, rows / 17)) * H * (dk * dv + dk + 4) floats.  The delta
+ * rule, widths other than dk 64 / 128 with dv % 4 == 0, or no workspace: as b200_gated_scan. */
+int b200_gated_scan_chunked(const float* x, int64_t ld, int q_col, int k_col, int v_col, const float* gates, int64_t ld_g,
+                            const float* rate, const float* dt_bias, const float* skip, const int32_t* cu_seq,
+                            const int32_t* ctx_lens, const int32_t* state_slots, float* S, float* o_raw, int n_seqs, int H, int G,
+                            int dk, int dv, int delta, int max_len, int rows, float* workspace, int64_t workspace_floats,
+                            void* stream);
 /* out = RMSnorm over `parts` equal pieces of (y * silu(z)) * w (the gate comes before the norm, one weight per channel), or
  * with gate_after RMSnorm of the pieces of y * w * silu(z) (one weight vector of a piece's width for all pieces). */
 int b200_gate_norm(const float* y, const void* proj, int f32, int64_t ld, int z_col, const void* w, void* out, int64_t ldo,

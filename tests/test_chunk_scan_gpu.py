@@ -91,6 +91,63 @@ def test_mlstm_chunks(lens, H, dk, dv, dtype):
     assert _rel(o, want.reshape(T, -1)) < 20 * TOL
 
 
+@pytest.mark.parametrize("lens", LENS, ids=str)
+@pytest.mark.parametrize("H,dk,dv", [(2, 64, 128), (1, 128, 64), (2, 64, 132)])
+def test_gated_linear_chunks(lens, H, dk, dv):
+    """Decays per key channel from nearly 1 to exactly 0 (a channel cleared in the middle of a chunk)."""
+    from gpustack_b200 import ops
+
+    g = torch.Generator().manual_seed(sum(lens) + dk + dv)
+    cu, ctx, slots = _layout(lens)
+    T = cu[-1]
+    x, z = torch.randn(T, 2 * H * dk + H * dv, generator=g), torch.randn(T, H * dk, generator=g) * 4 + 1
+    z[T // 2, ::3] = -1.0e5
+    S = torch.randn(len(lens), H, dv, dk, generator=g)
+    o, S_d = torch.zeros(T, H * dv, device="cuda"), S.cuda()
+    ops.gla_scan(x.cuda(), 0, H * dk, 2 * H * dk, z.cuda(), 1.0 / 16, _i32(cu), _i32(ctx), _i32(slots), S_d, o, H, dk, dv, max_len=4096)
+    q, k = x[:, :H * dk].view(T, H, dk).to(F64), x[:, H * dk:2 * H * dk].view(T, H, dk).to(F64)
+    v = x[:, 2 * H * dk:].view(T, H, dv).to(F64)
+    alpha = torch.exp(torch.nn.functional.logsigmoid(z.to(F64)) / 16).view(T, H, dk)
+    want, S_want = torch.zeros(T, H, dv, dtype=F64), S.to(F64)
+    for i in range(len(lens)):
+        Z = S_want[slots[i]].clone() * (1.0 if ctx[i] else 0.0)
+        for t in range(cu[i], cu[i + 1]):
+            Z = alpha[t][:, None] * Z + v[t][:, :, None] * k[t][:, None]
+            want[t] = torch.einsum("hvk,hk->hv", Z, q[t])
+        S_want[slots[i]] = Z
+    assert _rel(o, want.view(T, -1)) < TOL
+    assert _rel(S_d, S_want) < TOL
+
+
+@pytest.mark.parametrize("lens", LENS, ids=str)
+@pytest.mark.parametrize("H,G,dk,dv,skip", [(4, 2, 128, 64, True), (2, 1, 64, 128, False), (2, 2, 128, 36, True)])
+def test_state_space_chunks(lens, H, G, dk, dv, skip):
+    from gpustack_b200 import ops
+
+    g = torch.Generator().manual_seed(sum(lens) + dk + dv)
+    cu, ctx, slots = _layout(lens)
+    T = cu[-1]
+    x = torch.randn(T, 2 * G * dk + H * dv, generator=g)
+    gates, rate, dt = torch.randn(T, H, generator=g), torch.rand(H, generator=g), torch.randn(H, generator=g) - 2
+    D = torch.randn(H, generator=g) if skip else None
+    S = torch.randn(len(lens), H, dv, dk, generator=g)
+    o, S_d = torch.zeros(T, H * dv, device="cuda"), S.cuda()
+    ops.gated_scan(x.cuda(), 0, G * dk, 2 * G * dk, gates.cuda(), rate.cuda(), dt.cuda(), None if D is None else D.cuda(), _i32(cu), _i32(ctx),
+                   _i32(slots), S_d, o, H, G, dk, dv, False, max_len=4096)
+    q, k = (x[:, c:c + G * dk].view(T, G, dk).to(F64).repeat_interleave(H // G, 1) for c in (0, G * dk))
+    v = x[:, 2 * G * dk:].view(T, H, dv).to(F64)
+    step = torch.nn.functional.softplus(gates.to(F64) + dt.to(F64))
+    want, S_want = torch.zeros(T, H, dv, dtype=F64), S.to(F64)
+    for i in range(len(lens)):
+        Z = S_want[slots[i]].clone() * (1.0 if ctx[i] else 0.0)
+        for t in range(cu[i], cu[i + 1]):
+            Z = torch.exp(-rate.to(F64) * step[t])[:, None, None] * Z + (step[t][:, None] * v[t])[:, :, None] * k[t][:, None]
+            want[t] = torch.einsum("hvk,hk->hv", Z, q[t]) + (D.to(F64)[:, None] * v[t] if skip else 0.0)
+        S_want[slots[i]] = Z
+    assert _rel(o, want.view(T, -1)) < TOL
+    assert _rel(S_d, S_want) < TOL
+
+
 def test_no_row_reaches_an_earlier_one_and_negative_slots_are_skipped():
     from gpustack_b200 import ops
 
