@@ -67,6 +67,7 @@ struct ChunkScanArgs {
   float* ws;                       // [chunks][H][dk][dv]
   float* ws_row;                   // [chunks][H][ws_row_width]: a recurrence's own carry (its Form says what)
   int ws_row_width;                // dk + 4
+  float* ws_sums;                  // [chunks][H][2][64][dk]: kVector, the running sums' two parts
 };
 
 __host__ __device__ __forceinline__ int cs_chunks(int rows) { return rows > kCsShort ? (rows + kCsRows - 1) / kCsRows : 0; }
@@ -76,8 +77,8 @@ inline int64_t cs_max_chunks(int64_t rows, int64_t n_seqs) {
   const int64_t longs = rows / (kCsShort + 1);
   return rows / kCsRows + (longs < n_seqs ? longs : n_seqs);
 }
-inline int64_t cs_workspace_floats(int64_t rows, int64_t n_seqs, int64_t H, int64_t dk, int64_t dv) {
-  return cs_max_chunks(rows, n_seqs) * H * (dk * dv + dk + 4);
+inline int64_t cs_workspace_floats(int64_t rows, int64_t n_seqs, int64_t H, int64_t dk, int64_t dv, bool vector = false) {
+  return cs_max_chunks(rows, n_seqs) * H * (dk * dv + dk + 4 + (vector ? 2 * kCsRows * dk : 0));
 }
 
 // Sequence and place in it of chunk b (whole warp; seq -1: no such chunk), or with b < 0 the chunks before sequence `upto`.
@@ -199,11 +200,11 @@ __device__ __forceinline__ float cs_exp2(float h, float l) { return ex2_approx(h
 
 template <int DK, int VT, bool VECTOR = false>
 struct ChunkSmem {
-  static constexpr int kSums = VECTOR ? 2 * kCsRows * (DK + 4) : 0;          // running sums, two parts
-  static constexpr int kState = kCsRows * (DK + VT) + kSums; // floats
+  static constexpr int kSum = VECTOR ? kCsRows * (DK + 4) : 0;               // one part of the running sums
+  static constexpr int kState = kCsRows * (DK + VT) + 2 * kSum;              // floats
   static constexpr int kTile = 32 * VT;                      // a tile of 32 state or value rows
-  static constexpr int kB = kCsRows * (DK + 4) > 2 * kTile ? kCsRows * (DK + 4) : 2 * kTile;
-  static constexpr int kOutput = kCsRows * (DK + 4) + kB + kTile + kCsRows * kCsAPitch + kSums;
+  static constexpr int kB = kCsRows * (DK + 4) + kSum > 2 * kTile ? kCsRows * (DK + 4) + kSum : 2 * kTile;
+  static constexpr int kOutput = kCsRows * (DK + 4) + kB + kTile + kCsRows * kCsAPitch + kSum;
 };
 
 // Form: `Scratch` (shared arrays of one chunk), `state_weights` (fills scratch, w(s) and row() for chunk_state), `output_weights`,
@@ -295,9 +296,17 @@ chunk_state_kernel(const ChunkScanArgs a, const typename Form::Params p) {
       if (v < a.dv) *reinterpret_cast<ulonglong2*>(out + (size_t)k * a.dv + v) = make_ulonglong2(acc[i][2 * j], acc[i][2 * j + 1]);
     }
   if constexpr (Form::kVector) {
-    if (blockIdx.z == 0 && tid < DK) {
-      const int i = (at.rows - 1) * (DK + 4) + tid;
-      a.ws_row[((size_t)blockIdx.x * a.H + h) * a.ws_row_width + tid] = cs_exp2(hi[i], lo[i]);
+    if (blockIdx.z == 0) {
+      if (tid < DK) {
+        const int i = (at.rows - 1) * (DK + 4) + tid;
+        a.ws_row[((size_t)blockIdx.x * a.H + h) * a.ws_row_width + tid] = cs_exp2(hi[i], lo[i]);
+      }
+      float* sums = a.ws_sums + ((size_t)blockIdx.x * a.H + h) * (2 * kCsRows * DK);
+      for (int i = tid; i < kCsRows * DK / 4; i += kCsThreads) {
+        const int from = (4 * i / DK) * (DK + 4) + 4 * i % DK;
+        *reinterpret_cast<float4*>(sums + 4 * i) = *reinterpret_cast<const float4*>(hi + from);
+        *reinterpret_cast<float4*>(sums + kCsRows * DK + 4 * i) = *reinterpret_cast<const float4*>(lo + from);
+      }
     }
   } else if (blockIdx.z == 0) {
     Form::template state_row<DK>(a, scratch, ks, h, at.rows);
@@ -412,9 +421,9 @@ chunk_output_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   float* qs = smem;                                  // [64][DK + 4]
   float* X = qs + kCsRows * QP;                      // ring of three tiles of 32 rows; the keys [64][DK + 4] first lie on tiles 1 and 2
   float* B = X + TILE;
-  float* A = B + ChunkSmem<DK, VT>::kB;              // [64][68]
-  float* hi = A + kCsRows * kCsAPitch;               // [64][DK + 4] each, kVector only
-  float* lo = hi + kCsRows * QP;
+  float* A = B + ChunkSmem<DK, VT, Form::kVector>::kB;              // [64][68]
+  float* hi = A + kCsRows * kCsAPitch;               // [64][DK + 4] each, kVector only; lo behind the keys, until the ring takes the place
+  float* lo = B + kCsRows * QP;
   const TA* x = reinterpret_cast<const TA*>(a.x);
   const int hg = h / (a.H / a.G), vcol = a.v_col + h * a.dv + v0;
   const bool zero_start = at.local == 0 && a.ctx_lens[at.seq] == 0;
@@ -438,10 +447,15 @@ chunk_output_kernel(const ChunkScanArgs a, const typename Form::Params p) {
     ChunkTile<TA, kCsRows, DK, QP> q, k;
     q.issue(x, a.ld, at.first, n, a.q_col + hg * DK, DK, qs);
     k.issue(x, a.ld, at.first, n, a.k_col + hg * DK, DK, B);
+    if constexpr (Form::kVector) {                   // as chunk_state left them
+      const float* sums = a.ws_sums + ((size_t)blockIdx.x * a.H + h) * (2 * kCsRows * DK);
+      ChunkTile<float, kCsRows, DK, QP> f;
+      f.issue(sums, DK, 0, kCsRows, 0, DK, hi);
+      f.issue(sums, DK, kCsRows, kCsRows, 0, DK, lo);
+    }
     cp_async_commit();
     issue(0);
-    if constexpr (Form::kVector) Form::template sums<DK>(p, a, scratch, h, at, hi, lo);
-    else Form::output_weights(p, a, scratch, h, at);
+    if constexpr (!Form::kVector) Form::output_weights(p, a, scratch, h, at);
     q.land(qs);
     k.land(B);
   }
@@ -606,6 +620,7 @@ int cs_launch(ChunkScanArgs a, const typename Form::Params& p, int dk, int64_t r
   a.ws = ws;
   a.ws_row = ws + chunks * a.H * dk * a.dv;
   a.ws_row_width = dk + 4;
+  a.ws_sums = a.ws_row + chunks * a.H * (dk + 4);
   if (dk == 64) return a.dv <= 64 ? cs_launch_shape<64, 64, TA, Form>(a, p, rows, s) : cs_launch_shape<64, 128, TA, Form>(a, p, rows, s);
   return a.dv <= 64 ? cs_launch_shape<128, 64, TA, Form>(a, p, rows, s) : cs_launch_shape<128, 128, TA, Form>(a, p, rows, s);
 }

@@ -623,7 +623,7 @@ def mlstm_state_slices(dv: int) -> int:
 CHUNK_SCAN_MAX_BYTES = 1 << 30
 
 
-def _chunk_scan_workspace(rows: int, n_seqs: int, H: int, dk: int, dv: int, max_len: int, device):
+def _chunk_scan_workspace(rows: int, n_seqs: int, H: int, dk: int, dv: int, max_len: int, device, per_channel: bool = False):
     """Workspace of the scans that run a prompt portion's chunks of 64 rows side by side, or None where the one-pass scans are
     the better ones: key widths the chunk kernels do not take, and steps of short portions (three launches instead of one).
     All rows beyond max_len are taken for single ones.  Measured, 8 heads of 128 x 128, L2 cold, one-pass -> chunks, linear
@@ -631,7 +631,7 @@ def _chunk_scan_workspace(rows: int, n_seqs: int, H: int, dk: int, dv: int, max_
     35 -> 48; 16 of 32 rows 55 -> 73, of 64 rows 92 -> 85, of 512 rows 621 -> 255; mLSTM within 10 us of these."""
     if dk not in (64, 128) or dv % 4 or max_len < 128 or max_len < 96 * (n_seqs - max(0, rows - max_len)):
         return None
-    n = (rows // 64 + min(n_seqs, rows // 17)) * H * (dk * dv + dk + 4)
+    n = (rows // 64 + min(n_seqs, rows // 17)) * H * (dk * dv + dk + 4 + (128 * dk if per_channel else 0))
     return torch.empty(n, dtype=torch.float32, device=device) if 4 * n <= CHUNK_SCAN_MAX_BYTES else None
 
 
@@ -817,7 +817,7 @@ def gla_scan(x, q_col: int, k_col: int, v_col: int, z, inv_tau: float, cu_seq, c
     _cuda(x, z, cu_seq, ctx_lens, state_slots, S, o_raw)
     _req(x, torch.float32, "x"); _req(z, torch.float32, "z"); _req(S, torch.float32, "S"); _req(o_raw, torch.float32, "o_raw")
     n = state_slots.shape[0]
-    ws = _chunk_scan_workspace(x.shape[0], n, H, dk, dv, max_len, x.device)
+    ws = _chunk_scan_workspace(x.shape[0], n, H, dk, dv, max_len, x.device, per_channel=True)
     if ws is not None:
         check(load().b200_gla_scan_chunked(_p(x), x.stride(0), q_col, k_col, v_col, _p(z), z.stride(0), inv_tau, _p(cu_seq),
                                            _p(ctx_lens), _p(state_slots), _p(S), _p(o_raw), n, H, dk, dv, int(max_len), x.shape[0],

@@ -560,7 +560,7 @@ int b200_gla_scan_rows(const float* x, int64_t ld, int q_col, int k_col, int v_c
                   int n_seqs, int H, int dk, int dv, int max_len, void* stream);
 
 /* ... with a workspace: sequences of more than 16 rows run with all their chunks of 64 rows side by side.  rows: the rows of x;
- * workspace: 16-byte aligned, (rows / 64 + min(n_seqs, rows / 17)) * H * (dk * dv + dk + 4) floats.  Widths other than dk 64 /
+ * workspace: 16-byte aligned, (rows / 64 + min(n_seqs, rows / 17)) * H * (dk * dv + 129 * dk + 4) floats.  Widths other than dk 64 /
  * 128 with dv % 4 == 0, unaligned rows or no workspace: as b200_gla_scan_rows. */
 int b200_gla_scan_chunked(const float* x, int64_t ld, int q_col, int k_col, int v_col, const float* z, int64_t ldz, float inv_tau,
                           const int32_t* cu_seq, const int32_t* ctx_lens, const int32_t* state_slots, float* S, float* o_raw,
