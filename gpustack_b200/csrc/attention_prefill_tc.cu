@@ -7,9 +7,12 @@
 // share the kv-head times 128/G consecutive query tokens, so that S = Q K^T is a single UMMA M = 128
 // tile and every K/V byte staged in shared memory serves the whole GQA group.
 //
-//   warp 4    TMA producer: the Q tile once per work item, then K_j / V_j blocks of 64 tokens (4 KV pages of 16
-//             tokens, each page two 2 KB boxes of the 128-byte-swizzled layout) through a 4-slot
-//             mbarrier ring; pages past the end of the sequence are read from the all-zero null block;
+//   warp 4    TMA producer: the Q tile once per work item, then K_j / V_j blocks of 64 tokens through a 4-slot
+//             mbarrier ring; pages past the end of the sequence are read from the all-zero null block.  ONE copy per
+//             4 KB page (and one for the whole Q tile): the tensor maps split a row into its two 64-element halves and,
+//             for K, the tokens into groups of eight, in the order in which the operand descriptors step -- a copy
+//             costs the copy engine about 30 ns whatever its size (16 x 512 tokens, 32 / 8 heads: 73.9 us with a copy per
+//             2 KB, 71.6 us now);
 //   warp 5    MMA issuer (one elected thread): S_j = Q K_j^T into one of two 64-column TMEM buffers,
 //             O += P_j V_j into a 128-column TMEM accumulator.  S_{j+1} is issued BEFORE waiting for
 //             P_j, so the tensor pipe works on block j+1 while the softmax warps are busy with j;
@@ -47,8 +50,8 @@ constexpr int kFaD = 128;
 constexpr int kUmmaKBf16 = 16;                         // K elements per tcgen05.mma (kind::f16)
 constexpr int kFaKv = 64;                              // KV tokens per ring slot
 constexpr int kFaPage = 16;                            // tokens per KV page (vLLM block_size)
-constexpr int kFaSlotBytes = kFaKv * kFaD * 2;         // 16 KB = 2 d-halves x [64 tokens][128 B]
-constexpr int kFaHalfBytes = kFaKv * 128;              // 8 KB
+constexpr int kFaSlotBytes = kFaKv * kFaD * 2;         // 16 KB = 4 pages
+constexpr int kFaPageBytes = kFaPage * kFaD * 2;       // K: [2 groups][2 d-halves][8 tokens][128 B], V: [2 d-halves][16 tokens][128 B]
 constexpr int kFaSlots = 4;                            // K_j, V_j, K_j+1, V_j+1
 constexpr int kFaQBytes = 128 * kFaD * 2;              // 32 KB = 2 d-halves x [128 rows][128 B]
 constexpr int kFaQHalfBytes = 128 * 128;               // 16 KB
@@ -63,6 +66,23 @@ constexpr float kFaRescaleThreshold = 8.f;             // log2 units
 // a capped softmax whose scores stay within +-80 (base 2) runs against the reference 0: up to 2^80 per key, 2^24 keys and
 // values of 2^20 stay inside fp32, and 2^-80 is a normal number
 constexpr float kFaBoundedCap = 80.f;
+
+__device__ __forceinline__ void fa_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(
+                   smem_u32(dst)),
+               "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
+               : "memory");
+}
+__device__ __forceinline__ void fa_load_4d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2, int c3) {
+  asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(
+                   smem_u32(dst)),
+               "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+               : "memory");
+}
+// K-major, 128-byte swizzle, eight-row groups 2 KB apart (a page's groups hold both d-halves)
+__device__ __forceinline__ uint64_t fa_desc_k(uint32_t addr) {
+  return (uint64_t)((addr & 0x3FFFFu) >> 4) | (uint64_t)1 << 16 | (uint64_t)(2048 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)2 << 61;
+}
 
 // P_TMEM: P_j is written back into the first 32 columns of the TMEM buffer S_j came from (bf16 pairs
 // per 32-bit column, tcgen05.st) and the PV MMA reads its A operand from tensor memory: no shared-
@@ -185,13 +205,7 @@ paged_attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
       if (lane == 0) {
         if (it > 0) mbar_wait_guarded(q_empty, (it - 1) & 1);   // previous tile's Q K^T all retired
         mbar_expect_tx(q_full, kFaQBytes);
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h)
-            tma_load_2d(smem + h * kFaQHalfBytes + g * TPT * 128, &tmap_q, q_full, (m.kvh * G + g) * kFaD + h * 64,
-                        m.q_begin + m.q0, kEvictFirst);
-        }
+        fa_load_4d(smem, &tmap_q, q_full, 0, m.q_begin + m.q0, m.kvh * G, 0);      // [2 d-halves][G heads][tokens][128 B]
       }
       const int32_t* bt = block_table + (size_t)m.seq * max_blocks;
       int my_blk = 0;
@@ -212,10 +226,8 @@ paged_attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
             uint8_t* dst = smem + kFaOffKV + slot * kFaSlotBytes;
 #pragma unroll
             for (int p = 0; p < PPB; ++p) {
-#pragma unroll
-              for (int h = 0; h < 2; ++h)
-                tma_load_2d(dst + h * kFaHalfBytes + p * (kFaPage * 128), kv ? &tmap_v : &tmap_k, &kv_full[slot],
-                            h * 64, rows[p], kEvictNormal);
+              if (kv) fa_load_3d(dst + p * kFaPageBytes, &tmap_v, &kv_full[slot], 0, rows[p], 0);
+              else fa_load_4d(dst + p * kFaPageBytes, &tmap_k, &kv_full[slot], 0, 0, 0, rows[p] >> 3);
             }
             if (++slot == kFaSlots) { slot = 0; phase ^= 1; }
           }
@@ -243,8 +255,7 @@ paged_attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
 #pragma unroll
         for (int k = 0; k < kFaD / kUmmaKBf16; ++k) {   // 8 MMAs x 16 head-dim elements
           const uint32_t half = k >> 2, off = (k & 3) * 32;
-          umma_bf16(d, umma_desc_k_sw128(q_addr + half * kFaQHalfBytes + off),
-                    umma_desc_k_sw128(k_addr + half * kFaHalfBytes + off), idesc_s, k != 0);
+          umma_bf16(d, umma_desc_k_sw128(q_addr + half * kFaQHalfBytes + off), fa_desc_k(k_addr + half * 1024 + off), idesc_s, k != 0);
         }
         umma_commit(&kv_empty[slot]);     // K slot reusable once these MMAs retire
         umma_commit(&s_full[gb & 1]);     // S ready for the softmax warps
@@ -277,7 +288,7 @@ paged_attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
           const uint32_t v_addr = kv_addr + slot * kFaSlotBytes;
 #pragma unroll
           for (int k = 0; k < kFaKv / kUmmaKBf16; ++k) {   // 4 MMAs x 16 KV tokens
-            const uint64_t v_desc = umma_desc_mn_sw128(v_addr + k * (kUmmaKBf16 * 128), kFaHalfBytes, 1024);
+            const uint64_t v_desc = umma_desc_mn_sw128(v_addr + k * kFaPageBytes, kFaPage * 128, 1024);
             if constexpr (P_TMEM)   // A = P in TMEM: 16 bf16 of K = 8 columns per MMA
               umma_bf16_ts(tmem_base + 2 * kFaKv, tmem_base + (gb & 1) * kFaKv + k * 8, v_desc, idesc_o,
                            (j | k) != 0);
@@ -519,13 +530,23 @@ static int launch_prefill_tc(const void* q, int64_t q_stride, int num_tokens, co
     attr_set = true;
   }
   CUtensorMap tq, tk, tv;
-  int rc = make_tmap_bf16_2d(&tq, q, (uint64_t)num_tokens, (uint64_t)Hq * kFaD, (uint64_t)q_stride, 128 / G, 64);
-  if (rc) return rc;
-  const uint64_t kv_rows = (uint64_t)num_blocks * (uint64_t)Hkv * kFaPage;
-  rc = make_tmap_bf16_2d(&tk, k_cache, kv_rows, kFaD, kFaD, kFaPage, 64);
-  if (rc) return rc;
-  rc = make_tmap_bf16_2d(&tv, v_cache, kv_rows, kFaD, kFaD, kFaPage, 64);
-  if (rc) return rc;
+  int rc;
+  const uint64_t kv_rows = (uint64_t)num_blocks * (uint64_t)Hkv * kFaPage, row = kFaD * 2;
+  {
+    const uint64_t dims[4] = {64, (uint64_t)num_tokens, (uint64_t)Hq, 2}, st[3] = {(uint64_t)q_stride * 2, row, 128};
+    const uint32_t box[4] = {64, 128 / G, G, 2};
+    if ((rc = make_tmap_bf16_nd(&tq, q, 4, dims, st, box))) return rc;
+  }
+  {
+    const uint64_t dims[4] = {64, 8, 2, kv_rows / 8}, st[3] = {row, 128, 8 * row};
+    const uint32_t box[4] = {64, 8, 2, 2};
+    if ((rc = make_tmap_bf16_nd(&tk, k_cache, 4, dims, st, box))) return rc;
+  }
+  {
+    const uint64_t dims[3] = {64, kv_rows, 2}, st[2] = {row, 128};
+    const uint32_t box[3] = {64, kFaPage, 2};
+    if ((rc = make_tmap_bf16_nd(&tv, v_cache, 3, dims, st, box))) return rc;
+  }
   const float cap_log2 = softcap * 1.4426950408889634f;
   const float scale_log2 = (CAP ? 2.f * scale / softcap : scale) * 1.4426950408889634f;
   static int persist = -1;
