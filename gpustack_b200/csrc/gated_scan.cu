@@ -596,13 +596,13 @@ gate_norm_kernel(const float* __restrict__ y, const TA* __restrict__ proj, int64
   }
 }
 
-// Pieces of up to 128 channels (a head): W / 4 neighbouring lanes share one, a thread holds up to 8 of its row's 16-byte
-// groups in registers and all their loads are in flight together.
-template <typename TA, bool AFTER>
+// Pieces of up to 128 channels (a head): W / 4 neighbouring lanes share one, a thread holds up to N of its row's 16-byte
+// groups in registers and all their loads are in flight together.  Bound by bytes in flight: N 2 where it covers the row (the
+// registers of 8 leave 3 CTAs to an SM: 57 us for 8192 rows of 2048 channels, 38 us now).
+template <typename TA, bool AFTER, int N>
 __global__ void __launch_bounds__(kGnThreads)
 gate_norm_heads_kernel(const float* __restrict__ y, const TA* __restrict__ proj, int64_t ld, int z_col, const bf16* __restrict__ w, TA* out,
                        int64_t ldo, int C, int W, float eps) {
-  constexpr int N = 8;
   const int t = blockIdx.x, i0 = threadIdx.x * 4, step = kGnThreads * 4, lanes = W >> 2;
   const float* yr = y + (size_t)t * C;
   const TA* zr = proj + (size_t)t * ld + z_col;
@@ -690,10 +690,16 @@ extern "C" int b200_gate_norm(const float* y, const void* proj, int f32, int64_t
   const bool vec = (C / parts) % 4 == 0 && ld % 4 == 0 && ldo % 4 == 0 && z_col % 4 == 0 && al(y, 16) && al(proj, n) && al(out, n) && al(w, 8);
   const int W = C / parts, lanes = W / 4;
   if (vec && lanes <= 32 && (lanes & (lanes - 1)) == 0 && C <= kGnThreads * 4 * 8) {
-#define B200_GNH(TA, A) gate_norm_heads_kernel<TA, A><<<T, kGnThreads, 0, s>>>(y, (const TA*)proj, ld, z_col, (const bf16*)w, (TA*)out, ldo, C, W, eps)
+#define B200_GNHN(TA, A, N) gate_norm_heads_kernel<TA, A, N><<<T, kGnThreads, 0, s>>>(y, (const TA*)proj, ld, z_col, (const bf16*)w, (TA*)out, ldo, C, W, eps)
+#define B200_GNH(TA, A)                                            \
+  do {                                                             \
+    if (C <= 2 * kGnThreads * 4) B200_GNHN(TA, A, 2);              \
+    else B200_GNHN(TA, A, 8);                                      \
+  } while (0)
     if (f32) { if (gate_after) B200_GNH(float, true); else B200_GNH(float, false); }
     else { if (gate_after) B200_GNH(bf16, true); else B200_GNH(bf16, false); }
 #undef B200_GNH
+#undef B200_GNHN
     return b200_check_launch("b200_gate_norm");
   }
   B200_REQUIRE(smem <= 48 * 1024, "gate_norm: %d channels exceed the staged row (12288)", C);
