@@ -409,17 +409,15 @@ class LLMEngine:
                                 [e[3] for e in chunks], decode=(B, last, comp, bt) if B else None,
                                 state_slots=([e[1].state_slot for e in chunks] + dslots.tolist()) if self.state_slots else None)
             n_chunk_rows = sum(len(e[3]) for e in chunks)
-            lg = self.runner.last_logits(n_chunk_rows + B)
             parts, off = {}, 0
             for e in chunks:
-                parts[e[0]] = lg[off:off + len(e[3])]
+                parts[e[0]] = range(off, off + len(e[3]))
                 off += len(e[3])
             for j, e in enumerate(singles):
-                parts[e[0]] = lg[n_chunk_rows + j:n_chunk_rows + j + 1] if e[3] else lg[:0]
+                parts[e[0]] = range(n_chunk_rows + j, n_chunk_rows + j + (1 if e[3] else 0))
         else:
             self.runner.decode(B, last, comp, bt, state_slots=dslots if self.state_slots else None)
-            lg = self.runner.last_logits(B)
-            parts = {e[0]: (lg[j:j + 1] if e[3] else lg[:0]) for j, e in enumerate(singles)}
+            parts = {e[0]: range(j, j + (1 if e[3] else 0)) for j, e in enumerate(singles)}
         for _, r, toks, _ in chunks + singles:
             r.prompt_ids.extend(toks)
             r.num_computed += len(toks)
@@ -428,8 +426,7 @@ class LLMEngine:
             if r is not None:
                 s.replay_finish(r)
         self.counters["steps"] += 1
-        out = [parts[i] for i in range(len(entries))]
-        return (torch.cat(out, dim=0) if out else self.runner.logits[:0]).float().cpu().numpy()
+        return self.runner.host_logits([row for i in range(len(entries)) for row in parts[i]])
 
     def _apply_sampling(self, reqs, toks):
         """Plain temperature sampling happens in the sampler kernel (Gumbel-max, runner._sample); only

@@ -40,7 +40,8 @@ TIMER: Optional[KernelTimer] = None
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # the handle alone: a torch.cuda.Stream object costs more host time than the rest of a launch's arguments
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _p(t: Optional[torch.Tensor]) -> Optional[int]:

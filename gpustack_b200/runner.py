@@ -150,6 +150,7 @@ class ModelRunner:
         self.stage_np = self.stage_host.numpy()
         self.stage_dev = torch.zeros(self.stage_words, dtype=torch.int32, device=dev)
         self.out_host = torch.zeros(self.max_sample, dtype=torch.int32, pin_memory=True)
+        self.logits_host = torch.empty(1 << 20, dtype=torch.float32, pin_memory=True)
         # fixed decode layout inside the staging area
         S = self.max_seqs
         self.d_ids, self.d_pos, self.d_slots, self.d_lens = 0, S, 2 * S, 3 * S
@@ -747,6 +748,21 @@ class ModelRunner:
         return out
 
     # -------------------------------------------------------------------- test / debug hooks
+    def host_logits(self, rows: Sequence[int]) -> np.ndarray:
+        """fp32 logits [len(rows), V] of the given rows of the last _sample() call (local vocab shard).  Up to a few megabytes
+        pass a pinned buffer; neighbouring rows in order leave without a gather on the device."""
+        n = len(rows)
+        if n and rows[-1] - rows[0] == n - 1 and all(b == a + 1 for a, b in zip(rows, rows[1:])):
+            lg = self.logits[rows[0]:rows[0] + n]
+        else:
+            lg = self.logits[torch.tensor(rows, dtype=torch.long, device=self.device)]
+        if not 0 < lg.numel() <= self.logits_host.numel():
+            return lg.float().cpu().numpy()
+        host = self.logits_host[:lg.numel()].view(lg.shape)
+        host.copy_(lg, non_blocking=True)
+        torch.cuda.current_stream().synchronize()
+        return host.numpy().copy()
+
     def last_logits(self, n: int) -> torch.Tensor:
         """fp32 logits of the last _sample() call (local vocab shard), for parity tests."""
         return self.logits[:n].clone()
