@@ -303,29 +303,226 @@ latent_attn_mma_kernel(LaArgs a) {
   }
 }
 
+// Single rows of at most 16 heads: the kernel above would leave its second m-tile's warps idle and, with wide rows, every
+// fetch exposed (one buffer of 37 KB).  Here the 8 warps share one m-tile, the queries stay in registers, blocks of 32 keys pass
+// through a ring of five halves, and two CTAs share an SM:
+//   S:   warp w scores 16 keys (w & 1) over one quarter (w >> 1) of the row's width; the quarters meet in shared memory
+//   P:   warp w forms rows 2 w and 2 w + 1, a key per lane, and leaves probabilities and the accumulators' factor
+//   O:   warp w accumulates O[16][R / 8 columns from w R / 8].
+// Bound: instructions beside the cache's bytes; 64 sequences of 2048 rows of 576, 4 ranges, L2 cold: 67 us in the kernel above,
+// 51 here (57 with every warp forming all probabilities and two buffers, 64 with that and blocks of 16 keys).
+constexpr int kLdHalf = 16, kLdBufs = 5, kLdMaxW = 576, kLdSteps = kLdMaxW / 16 / 4;
+constexpr int kLdPitch = kLaKeys + 8;                  // floats per row of a partial score tile: conflict-free pairs
+
+template <int NT>   // n-tiles (8 columns) of the output per warp: R = 64 NT
+__global__ void __launch_bounds__(kLaWarps * 32, 2)
+latent_attn_step_kernel(LaArgs a) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  const int W = a.W, R = a.R, HB = a.HB;
+  const int pitch = W * 2 + 16, buf_bytes = kLdHalf * pitch;
+  uint8_t* k_s = smem;                                // [5][16][pitch]; the queries pass through the last buffer
+  float* s_s = reinterpret_cast<float*>(k_s + kLdBufs * buf_bytes);      // [4 quarters][16][kLdPitch]
+  uint8_t* p_s = reinterpret_cast<uint8_t*>(s_s + 4 * 16 * kLdPitch);    // [16][kLaPPitch]
+  float* f_s = reinterpret_cast<float*>(p_s + 16 * kLaPPitch);           // [3][16]: accumulators' factor; at the end maximum, sum
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int s = blockIdx.x, h0 = blockIdx.y * HB, kv_end = a.seq_lens[s];
+  if (kv_end <= 0) {                                   // a padding row of a captured batch: defined output, no keys
+    for (int i = threadIdx.x; i < HB * R; i += blockDim.x) {
+      const int h = h0 + i / R;
+      if (h < a.H) a.out[(size_t)s * a.ldo + (size_t)h * R + i % R] = __float2bfloat16_rn(0.f);
+    }
+    if (a.nsplit > 1 && threadIdx.x < HB && h0 + threadIdx.x < a.H) {       // an empty range for the merge kernel
+      float* w = a.ws + (((size_t)s * a.H + h0 + threadIdx.x) * a.nsplit + blockIdx.z) * (R + 2);
+      w[R] = -INFINITY;
+      w[R + 1] = 0.f;
+    }
+    return;
+  }
+  int blk_begin = 0, n_blk = (kv_end + kLaKeys - 1) / kLaKeys;
+  if (a.nsplit > 1) {                                  // this CTA's range of key blocks (it may be empty)
+    const int per = (n_blk + a.nsplit - 1) / a.nsplit;
+    blk_begin = min(n_blk, (int)blockIdx.z * per);
+    n_blk = min(n_blk, blk_begin + per);
+  }
+  const int n = n_blk - blk_begin, key_begin = blk_begin * kLaKeys;
+  const int32_t* bt = a.block_table + (size_t)s * a.max_blocks;
+  const int cpr = W / 8;
+  auto issue = [&](int half, int buf) {                // a warp copies two whole key rows
+    if (half < 2 * n) {
+#pragma unroll
+      for (int r = warp; r < kLdHalf; r += kLaWarps) {
+        const int key = key_begin + half * kLdHalf + r;
+        const bool live = key < kv_end;
+        const int kk = live ? key : 0;
+        const int pg = kk >> a.page_shift;
+        const bf16* src = a.cache + ((size_t)__ldg(bt + pg) * a.page + (kk - (pg << a.page_shift))) * W;
+        uint8_t* d = k_s + buf * buf_bytes + r * pitch;
+        for (int c = lane; c < cpr; c += 32) cp_async_16_zfill(d + c * 16, src + c * 8, live);
+      }
+    }
+    cp_async_commit();
+  };
+#pragma unroll
+  for (int i = 0; i < 3; ++i) issue(i, i);
+  const int t0 = lane >> 2, c0 = 2 * (lane & 3);
+  const int ai = lane >> 3, arr = lane & 7, a_row = arr + (ai & 1) * 8;
+  const int quarter = (W / 16 + 3) / 4, ks0 = (warp >> 1) * quarter, steps = min(W / 16 - ks0, quarter);
+  uint32_t q[kLdSteps][4];
+  {
+    uint8_t* q_s = k_s + (kLdBufs - 1) * buf_bytes;
+    for (int ci = threadIdx.x; ci < 16 * cpr; ci += blockDim.x) {
+      const int i = ci / cpr, c = ci - i * cpr;
+      uint4 v = make_uint4(0, 0, 0, 0);
+      if (i < HB && h0 + i < a.H) v = ld_v4(a.qa + (size_t)s * a.ldq + (size_t)(h0 + i) * W + c * 8);
+      *reinterpret_cast<uint4*>(q_s + i * pitch + c * 16) = v;
+    }
+    __syncthreads();
+    const uint32_t at = smem_u32(q_s) + a_row * pitch + ks0 * 32 + (ai >> 1) * 16;
+#pragma unroll
+    for (int i = 0; i < kLdSteps; ++i)
+      if (i < steps) ldsm_x4(at + i * 32, q[i][0], q[i][1], q[i][2], q[i][3]);
+  }
+
+  float o[NT][4];
+#pragma unroll
+  for (int t = 0; t < NT; ++t) o[t][0] = o[t][1] = o[t][2] = o[t][3] = 0.f;
+  float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};          // rows 2 warp, 2 warp + 1; the sums lane by lane
+  float* s_mine = s_s + ((warp >> 1) * 16 + t0) * kLdPitch + (warp & 1) * kLdHalf + c0;
+
+  int buf = 0;                                          // of the block's first half
+  for (int i = 0; i < n; ++i) {
+    const int buf1 = buf + 1 == kLdBufs ? 0 : buf + 1;
+    cp_async_wait<1>();
+    __syncthreads();                                    // block i visible; the block before (or the queries) is used
+    {
+      const int b3 = buf + 3 >= kLdBufs ? buf + 3 - kLdBufs : buf + 3, b4 = b3 + 1 == kLdBufs ? 0 : b3 + 1;
+      issue(2 * i + 3, b3);
+      issue(2 * i + 4, b4);
+    }
+    const uint32_t k0_base = smem_u32(k_s + buf * buf_bytes), k1_base = smem_u32(k_s + buf1 * buf_bytes);
+    float sa[4] = {0.f, 0.f, 0.f, 0.f}, sb[4] = {0.f, 0.f, 0.f, 0.f};
+    {
+      // one ldmatrix.x4 per step: keys 0-7 and 8-15, low and high half of the step's columns
+      const uint32_t kb_addr = ((warp & 1) ? k1_base : k0_base) + (arr + (ai >> 1) * 8) * pitch + ks0 * 32 + (ai & 1) * 16;
+#pragma unroll
+      for (int j = 0; j < kLdSteps; ++j) {
+        if (j >= steps) break;
+        uint32_t b0, b1, b2, b3;
+        ldsm_x4(kb_addr + j * 32, b0, b1, b2, b3);
+        mma_bf16_16816(sa, q[j], b0, b1);
+        mma_bf16_16816(sb, q[j], b2, b3);
+      }
+    }
+    *reinterpret_cast<float2*>(s_mine) = make_float2(sa[0], sa[1]);
+    *reinterpret_cast<float2*>(s_mine + 8) = make_float2(sb[0], sb[1]);
+    *reinterpret_cast<float2*>(s_mine + 8 * kLdPitch) = make_float2(sa[2], sa[3]);
+    *reinterpret_cast<float2*>(s_mine + 8 * kLdPitch + 8) = make_float2(sb[2], sb[3]);
+    __syncthreads();
+
+    const bool seen = key_begin + i * kLaKeys + lane < kv_end;
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const int row = 2 * warp + r;
+      const float* at = s_s + row * kLdPitch + lane;
+      float v = (at[0] + at[16 * kLdPitch]) + (at[32 * kLdPitch] + at[48 * kLdPitch]);     // (a quarter without steps: zeros)
+      v = seen ? v * a.scale_log2 : -INFINITY;
+      const float mn = fmaxf(m[r], warp_max(v));        // a block's first key is one that the row sees: finite
+      const float f = ex2_approx(m[r] - mn), p = ex2_approx(v - mn);
+      m[r] = mn;
+      l[r] = l[r] * f + p;
+      const bf16 pb = __float2bfloat16_rn(p);
+      *reinterpret_cast<bf16*>(p_s + row * kLaPPitch + lane * 2) = pb;
+      if (lane == 0) f_s[row] = f;
+    }
+    __syncthreads();
+
+    const float f0 = f_s[t0], f1 = f_s[t0 + 8];
+    if (__any_sync(0xffffffffu, f0 != 1.f || f1 != 1.f)) {         // no maximum moved in most blocks
+#pragma unroll
+      for (int t = 0; t < NT; ++t) { o[t][0] *= f0; o[t][1] *= f0; o[t][2] *= f1; o[t][3] *= f1; }
+    }
+#pragma unroll
+    for (int kk = 0; kk < 2; ++kk) {
+      uint32_t pa[4];
+      ldsm_x4(smem_u32(p_s) + a_row * kLaPPitch + (2 * kk + (ai >> 1)) * 16, pa[0], pa[1], pa[2], pa[3]);
+      const uint32_t v_addr = (kk ? k1_base : k0_base) + a_row * pitch + (warp * NT + (ai >> 1)) * 16;
+#pragma unroll
+      for (int c = 0; c < NT; c += 2) {
+        uint32_t b0, b1, b2, b3;
+        ldsm_x4_t(v_addr + c * 16, b0, b1, b2, b3);
+        mma_bf16_16816(o[c], pa, b0, b1);
+        mma_bf16_16816(o[c + 1], pa, b2, b3);
+      }
+    }
+    buf = buf1 + 1 == kLdBufs ? 0 : buf1 + 1;
+  }
+  cp_async_wait<0>();
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const float sum = warp_sum(l[r]);
+    if (lane == 0) {
+      f_s[16 + 2 * warp + r] = m[r];
+      f_s[32 + 2 * warp + r] = sum;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const int i = t0 + 8 * r, h = h0 + i, col = warp * NT * 8 + c0;
+    if (i >= HB || h >= a.H) continue;
+    const float m = f_s[16 + i];
+    float den = f_s[32 + i];
+    if (a.nsplit > 1) {                                 // park (O, m, l) of this key range; the merge kernel finishes
+      float* w = a.ws + (((size_t)s * a.H + h) * a.nsplit + blockIdx.z) * (R + 2);
+#pragma unroll
+      for (int t = 0; t < NT; ++t) { w[col + t * 8] = o[t][2 * r]; w[col + t * 8 + 1] = o[t][2 * r + 1]; }
+      if (warp == 0 && (lane & 3) == 0) { w[R] = m; w[R + 1] = den; }
+      continue;
+    }
+    if (a.sink != nullptr) den += exp2f(a.sink[h] * 1.4426950408889634f - m);
+    const float inv = den > 0.f ? 1.f / den : 0.f;
+#pragma unroll
+    for (int t = 0; t < NT; ++t)
+      *reinterpret_cast<uint32_t*>(a.out + (size_t)s * a.ldo + (size_t)h * R + col + t * 8) = pack_bf16(o[t][2 * r] * inv, o[t][2 * r + 1] * inv);
+  }
+}
+
 // out[b][h] = sum_s O_s 2^(m_s - M) / (sum_s l_s 2^(m_s - M) + 2^(sink_h log2 e - M)),  M = max_s m_s; empty ranges
 // (m_s = -inf) are skipped.
+// Lane s of every warp holds range s's maximum and sum (at most 16 ranges); a thread's loads of several ranges and columns are
+// in flight together.
 __global__ void __launch_bounds__(128)
 latent_attn_merge_kernel(const float* __restrict__ ws, const float* __restrict__ sink, bf16* out, int64_t ldo, int H,
                          int R, int nsplit) {
-  const int b = blockIdx.x, h = blockIdx.y;
+  const int b = blockIdx.x, h = blockIdx.y, lane = threadIdx.x & 31;
   const float* p = ws + ((size_t)b * H + h) * nsplit * (R + 2);
-  float M = -INFINITY;
-  for (int s = 0; s < nsplit; ++s) M = fmaxf(M, p[(size_t)s * (R + 2) + R]);
-  float den = 0.f;
-  for (int s = 0; s < nsplit; ++s) {
-    const float ms = p[(size_t)s * (R + 2) + R];
-    if (ms > -INFINITY) den += p[(size_t)s * (R + 2) + R + 1] * exp2f(ms - M);
-  }
+  float2 ml = make_float2(-INFINITY, 0.f);
+  if (lane < nsplit) ml = make_float2(p[(size_t)lane * (R + 2) + R], p[(size_t)lane * (R + 2) + R + 1]);
+  float M = ml.x;
+#pragma unroll
+  for (int w = 16; w > 0; w >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, w));
+  const float scale = ml.x > -INFINITY ? exp2f(ml.x - M) : 0.f;
+  float den = ml.x > -INFINITY ? ml.y * scale : 0.f;
+#pragma unroll
+  for (int w = 16; w > 0; w >>= 1) den += __shfl_xor_sync(0xffffffffu, den, w);
   if (sink != nullptr && M > -INFINITY) den += exp2f(sink[h] * 1.4426950408889634f - M);
   const float inv = den > 0.f ? 1.f / den : 0.f;
-  for (int d = threadIdx.x; d < R; d += blockDim.x) {
-    float acc = 0.f;
-    for (int s = 0; s < nsplit; ++s) {
-      const float ms = p[(size_t)s * (R + 2) + R];
-      if (ms > -INFINITY) acc += p[(size_t)s * (R + 2) + d] * exp2f(ms - M);
+  const unsigned live = __ballot_sync(0xffffffffu, ml.x > -INFINITY);
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};                 // R <= 512
+#pragma unroll 4
+  for (int s = 0; s < nsplit; ++s) {
+    const float f = __shfl_sync(0xffffffffu, scale, s);
+    if (!(live >> s & 1)) continue;                    // uniform
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int d = threadIdx.x + 128 * i;
+      if (d < R) acc[i] = fmaf(p[(size_t)s * (R + 2) + d], f, acc[i]);
     }
-    out[(size_t)b * ldo + (size_t)h * R + d] = __float2bfloat16_rn(acc * inv);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int d = threadIdx.x + 128 * i;
+    if (d < R) out[(size_t)b * ldo + (size_t)h * R + d] = __float2bfloat16_rn(acc[i] * inv);
   }
 }
 
@@ -363,6 +560,18 @@ static int la_launch(const LaArgs& a, dim3 grid, cudaStream_t s) {
   }
   latent_attn_mma_kernel<NT><<<grid, kLaWarps * 32, smem, s>>>(a);
   return b200_check_launch("b200_latent_attn");
+}
+
+template <int NT>
+static int ld_launch(const LaArgs& a, dim3 grid, cudaStream_t s) {
+  const size_t smem = (size_t)kLdBufs * kLdHalf * (a.W * 2 + 16) + (4 * 16 * kLdPitch + 3 * 16) * sizeof(float) + 16 * kLaPPitch;
+  const cudaError_t e = cudaFuncSetAttribute(latent_attn_step_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) {
+    b200_set_error("latent_attn_decode: cudaFuncSetAttribute(smem=%zu): %s", smem, cudaGetErrorString(e));
+    return B200_ERR_CUDA;
+  }
+  latent_attn_step_kernel<NT><<<grid, kLaWarps * 32, smem, s>>>(a);
+  return b200_check_launch("b200_latent_attn_decode");
 }
 
 static int la_dispatch(const LaArgs& a, dim3 grid, cudaStream_t s) {
@@ -446,7 +655,15 @@ extern "C" int b200_latent_attn_decode(const void* qa, int64_t ldq, const void* 
            sink, (bf16*)out, ldo, H, R + dr, R, hb, 1, scale * 1.4426950408889634f, la_log2(page), nsplit, (float*)workspace,
            la_nbuf(R + dr)};
   dim3 grid(B, (H + hb - 1) / hb, nsplit);
-  if (int rc = la_dispatch(a, grid, (cudaStream_t)stream)) return rc;
+  // one m-tile of heads, whole pairs of n-tiles per warp, and rows of which two CTAs' rings fit an SM: the step kernel
+  int rc;
+  const bool step = hb <= 16 && R % 128 == 0 && R + dr <= kLdMaxW;
+  if (step && R == 128) rc = ld_launch<2>(a, grid, (cudaStream_t)stream);
+  else if (step && R == 256) rc = ld_launch<4>(a, grid, (cudaStream_t)stream);
+  else if (step && R == 384) rc = ld_launch<6>(a, grid, (cudaStream_t)stream);
+  else if (step && R == 512) rc = ld_launch<8>(a, grid, (cudaStream_t)stream);
+  else rc = la_dispatch(a, grid, (cudaStream_t)stream);
+  if (rc) return rc;
   if (nsplit > 1) {
     latent_attn_merge_kernel<<<dim3(B, H), 128, 0, (cudaStream_t)stream>>>((const float*)workspace, sink, (bf16*)out, ldo, H, R,
                                                                           nsplit);

@@ -95,3 +95,39 @@ def test_products_of_all_heads(H, N, K, pad, M, f32):
     # fp32 sums of K exact products (K 2^-24 of the terms' norm at most), and one bf16 rounding
     assert float((got[..., :N].to(F64) - want).norm() / want.norm()) < (K * 2.0 ** -24 if f32 else 2.0 ** -8)
     assert bool((got[..., N:] == 9.0).all())                       # what lies between the heads is left alone
+
+
+@pytest.mark.parametrize("splits", [1, 2, 7])
+@pytest.mark.parametrize("H,R,dr", [(16, 512, 64), (9, 128, 16), (17, 384, 48), (1, 256, 0)])
+def test_single_rows_at_the_edges_of_key_blocks(H, R, dr, splits):
+    """One new row per sequence: lengths around the blocks of 32 keys and their halves, a row without keys, widths of an odd number of 16-column
+    steps, 1 to 16 heads per CTA.  bf16 probabilities and outputs: each rounds by at most 2^-9 of its value, so the norm of the
+    error stays below 2^-8 of the output's (values of one size, cancellation within a factor of 2)."""
+    from gpustack_b200 import ops
+
+    lens = [1, 15, 16, 17, 31, 32, 33, 97, 0, 513]
+    g = torch.Generator().manual_seed(H + R + dr)
+    pages = [-(-max(n, 1) // 16) for n in lens]
+    order = torch.randperm(sum(pages), generator=g).to(torch.int32)
+    cache = torch.randn(sum(pages), 1, 16, R + dr, generator=g).to(torch.bfloat16)
+    bt = torch.zeros(len(lens), max(pages), dtype=torch.int32)
+    q = torch.randn(len(lens), H * (R + dr), generator=g).to(torch.bfloat16)
+    scale, off, want = 1.3 / (R + dr) ** 0.5, 0, torch.zeros(len(lens), H, R, dtype=torch.float64)
+    for b, n in enumerate(lens):
+        bt[b, :pages[b]] = order[off:off + pages[b]]
+        off += pages[b]
+        if n:
+            k = cache[bt[b, :pages[b]].long()].reshape(-1, R + dr)[:n].double()
+            want[b] = torch.softmax(scale * q[b].view(H, -1).double() @ k.T, dim=-1) @ k[:, :R]
+    for b, n in enumerate(lens):                       # what lies behind a sequence's last key is no number
+        if n % 16:
+            cache[bt[b, pages[b] - 1].long(), 0, n % 16:] = float("nan")
+    out = torch.full((len(lens), H * R), 3.0, dtype=torch.bfloat16, device="cuda")
+    ws = ops.latent_attn_decode_workspace(len(lens), H, R, splits, "cuda")
+    ops.latent_attn_decode(q.cuda(), cache.cuda(), bt.cuda(), torch.tensor(lens, dtype=torch.int32, device="cuda"), None, out, H, R, dr, scale,
+                           num_splits=splits, workspace=ws)
+    got = out.view(len(lens), H, R).double().cpu()
+    assert bool((got[lens.index(0)] == 0).all())
+    for b, n in enumerate(lens):
+        if n:
+            assert float((got[b] - want[b]).norm() / want[b].norm()) < 2 * 2.0 ** -8, n
