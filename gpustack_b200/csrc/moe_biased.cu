@@ -28,21 +28,23 @@ constexpr int kRbMaxTop = 16;
 
 __device__ __forceinline__ float rb_f32(float v) { return v; }
 __device__ __forceinline__ float rb_f32(bf16 v) { return __bfloat162float(v); }
+__device__ __forceinline__ float4 rb_f32x4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 rb_f32x4(const bf16* p) {
+  const uint2 v = *reinterpret_cast<const uint2*>(p);
+  return make_float4(bf16_lo(v.x), bf16_hi(v.x), bf16_lo(v.y), bf16_hi(v.y));
+}
 
-// one warp per token, lane l holds outputs l, l + 32, ...
-__global__ void __launch_bounds__(128)
-moe_route_biased_kernel(const float* __restrict__ logits, int64_t ld, const float* __restrict__ correction,
-                        int32_t* __restrict__ topk_ids, float* __restrict__ topk_w, int T, int E, int K, float scale,
-                        int score_mode, int renormalize, int groups, int groups_keep) {
-  __shared__ float gc[4][32 * kRbPerLane], gbest[4][32 * kRbPerLane];    // choice scores, best of every group
-  const int t = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (t >= T) return;
+// A warp's token t: lane l holds outputs l, l + 32, ... of its logits; gc, gbest: this warp's choice scores, best of every group
+__device__ __forceinline__ void rb_route(const float* __restrict__ logits, const float* __restrict__ correction,
+                                         int32_t* __restrict__ topk_ids, float* __restrict__ topk_w, int t, int E, int K, float scale,
+                                         int score_mode, int renormalize, int groups, int groups_keep, float* gc, float* gbest) {
+  const int lane = threadIdx.x & 31;
   float s[kRbPerLane], c[kRbPerLane];
   float mx = -CUDART_INF_F;
 #pragma unroll
   for (int i = 0; i < kRbPerLane; ++i) {
     const int e = lane + 32 * i;
-    s[i] = e < E ? logits[(size_t)t * ld + e] : -CUDART_INF_F;
+    s[i] = e < E ? logits[e] : -CUDART_INF_F;
     mx = fmaxf(mx, s[i]);
   }
   mx = warp_max(mx);
@@ -81,8 +83,8 @@ moe_route_biased_kernel(const float* __restrict__ logits, int64_t ld, const floa
     }
   }
   if (groups > 1 && groups_keep < groups) {
-    float* cs = gc[threadIdx.x >> 5];
-    float* gs = gbest[threadIdx.x >> 5];
+    float* cs = gc;
+    float* gs = gbest;
     const int n = E / groups;
 #pragma unroll
     for (int i = 0; i < kRbPerLane; ++i)
@@ -139,23 +141,116 @@ moe_route_biased_kernel(const float* __restrict__ logits, int64_t ld, const floa
   }
 }
 
-template <typename TX, typename TP>
+__global__ void __launch_bounds__(128)
+moe_route_biased_kernel(const float* __restrict__ logits, int64_t ld, const float* __restrict__ correction,
+                        int32_t* __restrict__ topk_ids, float* __restrict__ topk_w, int T, int E, int K, float scale,
+                        int score_mode, int renormalize, int groups, int groups_keep) {
+  __shared__ float gc[4][32 * kRbPerLane], gbest[4][32 * kRbPerLane];
+  const int w = threadIdx.x >> 5, t = blockIdx.x * 4 + w;
+  if (t < T)
+    rb_route(logits + (size_t)t * ld, correction, topk_ids, topk_w, t, E, K, scale, score_mode, renormalize, groups, groups_keep, gc[w],
+             gbest[w]);
+}
+
+// The router's product and the choice in one launch, a cluster of eight CTAs per two tokens: each of its 64 warps sums the
+// products of two outputs at a time with both tokens in fp32, writes the logits and leaves them in the first CTA's shared
+// memory, whose first two warps choose.  A step of few tokens gives the tensor-core product one or two CTAs, a serial chain over
+// the whole width (with the choice, 2048 -> 128: 11.5 us for
+// 1 to 128 tokens; here 4.8 for one, 5.7 for 64, 7.3 for 128 and 12.4 for 256).  Bound: latency, then
+// the router's rows through L2 once per pair of tokens.
+constexpr int kRtWarps = 8, kRtCluster = 8, kRtRows = 2;
+
+__global__ void __launch_bounds__(kRtWarps * 32)
+moe_router_kernel(const bf16* __restrict__ x, int64_t ldx, const bf16* __restrict__ router, int64_t ldw, int N, int D, float* logits,
+                  int64_t ldl, const float* __restrict__ correction, int32_t* __restrict__ topk_ids, float* __restrict__ topk_w, int T,
+                  int E, int K, float scale, int score_mode, int renormalize, int groups, int groups_keep) {
+  __shared__ float z[2][32 * kRbPerLane], gc[2][32 * kRbPerLane], gbest[2][32 * kRbPerLane];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = (int)cluster_ctarank();
+  const int t0 = blockIdx.x / kRtCluster * 2;
+  const bool two = t0 + 1 < T;
+  const bf16* x0 = x + (size_t)t0 * ldx;
+  const bf16* x1 = two ? x0 + ldx : x0;
+  const uint32_t z0 = mapa_u32(z[0], 0);
+  for (int r0 = (rank * kRtWarps + warp) * kRtRows; r0 < N; r0 += kRtCluster * kRtWarps * kRtRows) {
+    float acc[kRtRows][2];
+#pragma unroll
+    for (int r = 0; r < kRtRows; ++r) acc[r][0] = acc[r][1] = 0.f;
+#pragma unroll 8
+    for (int d = lane * 8; d < D; d += 256) {
+      const uint4 u0 = ld_v4(x0 + d), u1 = ld_v4(x1 + d);
+      const uint32_t p[4] = {u0.x, u0.y, u0.z, u0.w}, q[4] = {u1.x, u1.y, u1.z, u1.w};
+#pragma unroll
+      for (int r = 0; r < kRtRows; ++r) {
+        const uint4 v = ld_v4(router + (size_t)min(r0 + r, N - 1) * ldw + d);
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          acc[r][0] = fmaf(bf16_lo(p[i]), bf16_lo(w[i]), acc[r][0]);
+          acc[r][1] = fmaf(bf16_lo(q[i]), bf16_lo(w[i]), acc[r][1]);
+          acc[r][0] = fmaf(bf16_hi(p[i]), bf16_hi(w[i]), acc[r][0]);
+          acc[r][1] = fmaf(bf16_hi(q[i]), bf16_hi(w[i]), acc[r][1]);
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < kRtRows; ++r)
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        const float sum = warp_sum(acc[r][t]);
+        if (lane != 0 || r0 + r >= N || (t == 1 && !two)) continue;
+        logits[(size_t)(t0 + t) * ldl + r0 + r] = sum;
+        if (r0 + r < E)
+          asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(z0 + (uint32_t)(t * 32 * kRbPerLane + r0 + r) * 4u), "f"(sum) : "memory");
+      }
+  }
+  cluster_sync_all();
+  if (rank == 0 && warp < (two ? 2 : 1))
+    rb_route(z[warp], correction, topk_ids, topk_w, t0 + warp, E, K, scale, score_mode, renormalize, groups, groups_keep, gc[warp], gbest[warp]);
+}
+
+// VEC: four neighbouring columns per thread (D % 4 == 0 and every row aligned for it)
+template <typename TX, typename TP, bool VEC>
 __global__ void __launch_bounds__(256)
 moe_combine_mixed_kernel(const TP* __restrict__ yp, int64_t ldp, const int32_t* __restrict__ pair_row,
                          const int32_t* __restrict__ topk_ids, const float* __restrict__ topk_w,
                          const TX* __restrict__ x, int64_t ldx, const TP* __restrict__ shared, int64_t lds,
                          float* __restrict__ out, int64_t ldo, int T, int D, int K, int n_real) {
-  const size_t total = (size_t)T * D;
+  pdl_launch_dependents();
+  pdl_wait();
+  constexpr int V = VEC ? 4 : 1;
+  const size_t total = (size_t)T * D / V;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-    const int t = (int)(i / D), d = (int)(i % D);
-    float acc = 0.f;
-    for (int j = 0; j < K; ++j) {
-      const int id = topk_ids[(size_t)t * K + j];
-      if (id < n_real) acc += rb_f32(yp[(size_t)pair_row[(size_t)t * K + j] * ldp + d]);
-      else acc += topk_w[(size_t)t * K + j] * rb_f32(x[(size_t)t * ldx + d]);
+    const int t = (int)(i / (D / V)), d = (int)(i % (D / V)) * V;
+    if constexpr (VEC) {
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int j = 0; j < K; ++j) {
+        const int id = topk_ids[(size_t)t * K + j];
+        if (id < n_real) {
+          const float4 v = rb_f32x4(yp + (size_t)pair_row[(size_t)t * K + j] * ldp + d);
+          acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+        } else {
+          const float w = topk_w[(size_t)t * K + j];
+          const float4 v = rb_f32x4(x + (size_t)t * ldx + d);
+          acc.x += w * v.x; acc.y += w * v.y; acc.z += w * v.z; acc.w += w * v.w;
+        }
+      }
+      if (shared != nullptr) {
+        const float4 v = rb_f32x4(shared + (size_t)t * lds + d);
+        acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+      }
+      *reinterpret_cast<float4*>(out + (size_t)t * ldo + d) = acc;
+    } else {
+      float acc = 0.f;
+      for (int j = 0; j < K; ++j) {
+        const int id = topk_ids[(size_t)t * K + j];
+        if (id < n_real) acc += rb_f32(yp[(size_t)pair_row[(size_t)t * K + j] * ldp + d]);
+        else acc += topk_w[(size_t)t * K + j] * rb_f32(x[(size_t)t * ldx + d]);
+      }
+      if (shared != nullptr) acc += rb_f32(shared[(size_t)t * lds + d]);
+      out[(size_t)t * ldo + d] = acc;
     }
-    if (shared != nullptr) acc += rb_f32(shared[(size_t)t * lds + d]);
-    out[(size_t)t * ldo + d] = acc;
   }
 }
 
@@ -163,19 +258,44 @@ moe_combine_mixed_kernel(const TP* __restrict__ yp, int64_t ldp, const int32_t* 
 
 using namespace b200;
 
-extern "C" int b200_moe_route_grouped(const float* logits, int64_t ld, const float* correction, int32_t* topk_ids,
-                                      float* topk_w, int T, int E, int K, float scale, int score_mode, int renormalize,
-                                      int groups, int groups_keep, void* stream) {
-  B200_REQUIRE(ld >= E, "moe_route_biased: row stride %lld < E=%d", (long long)ld, E);
+static int rb_check(int T, int E, int K, int score_mode, int groups, int groups_keep) {
   B200_REQUIRE(T >= 0 && E >= 1 && E <= 32 * kRbPerLane && K >= 1 && K <= kRbMaxTop && K <= E,
                "moe_route_biased: unsupported E=%d K=%d (E <= %d, K <= %d)", E, K, 32 * kRbPerLane, kRbMaxTop);
   B200_REQUIRE(score_mode >= 0 && score_mode <= 2, "moe_route_biased: unknown score form %d", score_mode);
   B200_REQUIRE(groups == 0 || (groups > 0 && E % groups == 0 && groups_keep >= 1 && groups_keep <= groups && K <= groups_keep * (E / groups)),
                "moe_route_biased: %d of %d groups of %d outputs, K=%d", groups_keep, groups, E, K);
+  return B200_OK;
+}
+
+extern "C" int b200_moe_route_grouped(const float* logits, int64_t ld, const float* correction, int32_t* topk_ids,
+                                      float* topk_w, int T, int E, int K, float scale, int score_mode, int renormalize,
+                                      int groups, int groups_keep, void* stream) {
+  B200_REQUIRE(ld >= E, "moe_route_biased: row stride %lld < E=%d", (long long)ld, E);
+  if (int rc = rb_check(T, E, K, score_mode, groups, groups_keep)) return rc;
   if (T == 0) return B200_OK;
   moe_route_biased_kernel<<<(T + 3) / 4, 128, 0, (cudaStream_t)stream>>>(logits, ld, correction, topk_ids, topk_w, T, E, K,
                                                                        scale, score_mode, renormalize, groups, groups_keep);
   return b200_check_launch("b200_moe_route_biased");
+}
+
+extern "C" int b200_moe_router(const void* x, int64_t ldx, const void* router, int64_t ldw, int N, int D, float* logits, int64_t ldl,
+                               const float* correction, int32_t* topk_ids, float* topk_w, int T, int E, int K, float scale, int score_mode,
+                               int renormalize, int groups, int groups_keep, void* stream) {
+  B200_REQUIRE(D > 0 && D % 8 == 0 && ldx >= D && ldw >= D && ldx % 8 == 0 && ldw % 8 == 0 &&
+                   ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(router)) & 15) == 0,
+               "moe_router: 16-byte aligned bf16 rows of a multiple of 8 columns required (D=%d)", D);
+  B200_REQUIRE(N >= E && ldl >= N, "moe_router: %d rows for %d outputs, logits of row stride %lld", N, E, (long long)ldl);
+  if (int rc = rb_check(T, E, K, score_mode, groups, groups_keep)) return rc;
+  if (T == 0) return B200_OK;
+  const cudaError_t e = launch_pdl_cls(kPdlMoe, moe_router_kernel, dim3((T + 1) / 2 * kRtCluster), dim3(kRtWarps * 32), 0, (cudaStream_t)stream,
+                                       kRtCluster, (const bf16*)x, ldx, (const bf16*)router, ldw, N, D, logits, ldl, correction, topk_ids,
+                                       topk_w, T, E, K, scale, score_mode, renormalize, groups, groups_keep);
+  if (e != cudaSuccess) {
+    b200_set_error("b200_moe_router: launch failed: %s", cudaGetErrorString(e));
+    (void)cudaGetLastError();
+    return B200_ERR_CUDA;
+  }
+  return b200_check_launch("b200_moe_router");
 }
 
 extern "C" int b200_moe_route_scored(const float* logits, int64_t ld, const float* correction, int32_t* topk_ids,
@@ -196,16 +316,25 @@ extern "C" int b200_moe_combine_mixed(const void* yp, int p_f32, int64_t ldp, co
   B200_REQUIRE(T >= 0 && D > 0 && K >= 1, "moe_combine_mixed: bad shape");
   if (T == 0) return B200_OK;
   cudaStream_t s = (cudaStream_t)stream;
-  size_t blocks = ((size_t)T * D + 255) / 256;
+  const uintptr_t xm = x_f32 ? 15 : 7, pm = p_f32 ? 15 : 7;
+  const bool vec = D % 4 == 0 && ldp % 4 == 0 && ldx % 4 == 0 && lds % 4 == 0 && ldo % 4 == 0 &&
+                   ((reinterpret_cast<uintptr_t>(yp) | reinterpret_cast<uintptr_t>(shared)) & pm) == 0 &&
+                   (reinterpret_cast<uintptr_t>(x) & xm) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+  size_t blocks = ((size_t)T * D / (vec ? 4 : 1) + 255) / 256;
   if (blocks > 8192) blocks = 8192;
-#define B200_CM(TX, TP)                                                                                             \
-  moe_combine_mixed_kernel<TX, TP><<<(int)blocks, 256, 0, s>>>((const TP*)yp, ldp, pair_row, topk_ids, topk_w,     \
-                                                               (const TX*)x, ldx, (const TP*)shared, lds, out, ldo, T, D, \
-                                                               K, n_real)
+#define B200_CMV(TX, TP, V)                                                                                          \
+  (void)launch_pdl_cls(kPdlMoe, moe_combine_mixed_kernel<TX, TP, V>, dim3((unsigned)blocks), dim3(256), 0, s, 1, (const TP*)yp, ldp, \
+                       pair_row, topk_ids, topk_w, (const TX*)x, ldx, (const TP*)shared, lds, out, ldo, T, D, K, n_real)
+#define B200_CM(TX, TP)                     \
+  do {                                      \
+    if (vec) B200_CMV(TX, TP, true);        \
+    else B200_CMV(TX, TP, false);           \
+  } while (0)
   if (x_f32 && p_f32) B200_CM(float, float);
   else if (x_f32) B200_CM(float, bf16);
   else if (p_f32) B200_CM(bf16, float);
   else B200_CM(bf16, bf16);
 #undef B200_CM
+#undef B200_CMV
   return b200_check_launch("b200_moe_combine_mixed");
 }

@@ -1184,6 +1184,17 @@ ROUTED_LAUNCHES = 6
 TC_GROUPED_ACTS = {"silu": 0, "gelu_tanh": 1, "clamped_swish": 2}
 
 
+# (token, router row) pairs up to which the router's product runs beside the choice on the CUDA cores: above, its rows cross L2
+# once per pair of tokens, and the tensor-core product has tiles enough (2048 -> 128: 7 us against 11 for 128 tokens, 12.4 against
+# 12.1 for 256; 4096 -> 256: 12.8 against 16.3 for 64, 18.6 against 16.5 for 128)
+ROUTER_FUSED_PAIRS = 128 * 128
+
+
+def _router_rows_ok(x, router, D: int) -> bool:
+    return (router.dtype == torch.bfloat16 and router.shape[1] == D and x.stride(-1) == 1 and router.stride(-1) == 1
+            and x.stride(0) % 8 == 0 and router.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and router.data_ptr() % 16 == 0)
+
+
 def routed_experts(x, router, correction, w13, w2, ws: RoutedWorkspace, out, n_real: int, n_identity: int, top_k: int,
                    scale: float, ff: int, limit: float, shared=None, sigmoid: bool = False, renormalize: bool = True,
                    weight_on: str = "output", act: str = "clamped_swish", score: Optional[str] = None, combine: bool = True,
@@ -1212,15 +1223,21 @@ def routed_experts(x, router, correction, w13, w2, ws: RoutedWorkspace, out, n_r
     if cap > ws.capacity:
         raise B200Error(f"routed_experts: {T} tokens exceed the workspace ({ws.capacity} rows)")
     L, st = load(), _stream()
-    lg = ws.logits[:T]
-    # fp32 logits; a router padded to whole weight tiles (weights.load_layer_list) takes the tensor-core GEMM in bf16
-    linear(x, router, lg, force_simt=router.shape[0] % 128 != 0)
     w_in = weight_on == "input"
     if w_in and n_identity:
         raise B200Error("routed_experts: identity experts with input weights are not defined")
-    check(L.b200_moe_route_grouped(_p(lg), lg.stride(0), _p(correction), _p(ws.topk_ids), _p(ws.topk_w), T, E, top_k, scale,
-                                   SCORE_MODES[score] if score else (1 if sigmoid else 0), 1 if renormalize else 0, groups,
-                                   groups_keep, st), "moe_route_grouped")
+    mode = SCORE_MODES[score] if score else (1 if sigmoid else 0)
+    lg, N = ws.logits[:T], router.shape[0]
+    if tc and T * N <= ROUTER_FUSED_PAIRS and N <= lg.shape[1] and _router_rows_ok(x, router, D):
+        _cuda(x, router)
+        check(L.b200_moe_router(_p(x), x.stride(0), _p(router), router.stride(0), N, D, _p(lg), lg.stride(0), _p(correction),
+                                _p(ws.topk_ids), _p(ws.topk_w), T, E, top_k, scale, mode, 1 if renormalize else 0, groups, groups_keep,
+                                st), "moe_router")
+    else:
+        # fp32 logits; a router padded to whole weight tiles (weights.load_layer_list) takes the tensor-core GEMM in bf16
+        linear(x, router, lg, force_simt=router.shape[0] % 128 != 0)
+        check(L.b200_moe_route_grouped(_p(lg), lg.stride(0), _p(correction), _p(ws.topk_ids), _p(ws.topk_w), T, E, top_k, scale, mode,
+                                       1 if renormalize else 0, groups, groups_keep, st), "moe_route_grouped")
     check(L.b200_moe_align(_p(ws.topk_ids), _p(ws.topk_w), n_pairs, E, bx, cap, _p(ws.pair_row), _p(ws.row_pair),
                            _p(ws.row_weight), _p(ws.tile_expert), _p(ws.num_tiles), st), "moe_align")
     act = ws.act[:cap * ff].view(cap, ff)

@@ -638,6 +638,11 @@ int b200_prenorm_join(const float* x_in, const float* y, const float* y2, const 
 int b200_moe_route_grouped(const float* logits, int64_t ld, const float* correction, int32_t* topk_ids, float* topk_w, int T,
                            int E, int K, float scale, int score_mode, int renormalize, int groups, int groups_keep,
                            void* stream);
+/* The router's product and b200_moe_route_grouped over its first E outputs in one launch: logits[t, n] = x[t] . router[n] for all
+ * N >= E rows, bf16 rows of D columns (a multiple of 8, rows 16-byte aligned), fp32 sums. */
+int b200_moe_router(const void* x, int64_t ldx, const void* router, int64_t ldw, int N, int D, float* logits, int64_t ldl,
+                    const float* correction, int32_t* topk_ids, float* topk_w, int T, int E, int K, float scale, int score_mode,
+                    int renormalize, int groups, int groups_keep, void* stream);
 /* The attention kernels with a soft cap on the scaled score, softcap * tanh(score / softcap) (0 = none). */
 int b200_attn_sink_prefill_cap(const void* proj, int f32, int64_t ld, int gate_col, const void* k_cache, const void* v_cache,
                                 const int32_t* block_table, int max_blocks, const int32_t* cu_q, const int32_t* ctx_lens,
