@@ -112,6 +112,35 @@ __device__ __forceinline__ float gated_pair(float g, float up, int gact, float l
   return round_bf16(g / (1.f + __expf(-g))) * up;
 }
 
+// gated_pair of N pairs, which wait for one another nowhere: with a division (and its branch) in each, an epilogue warp, alone on
+// its scheduler, took 370 clocks a pair, 25 us a tile of 256 x 256 beside a main loop of 17 (K 4096).  One check per chunk finds
+// the values that need the operator.  Gate-up products, L2 cold: 256 tokens, 4096 -> 28672 72 -> 57 us; 8192 tokens 1323 -> 1187
+// (1.62 PFLOP/s); 2048 -> 16384 619 -> 348; the experts' 64 tokens of 8 x (2048 -> 4096) 36 -> 27.
+template <int N>
+__device__ __forceinline__ void gated_pairs(const float (&g)[N], const float (&up)[N], int gact, float limit, float (&out)[N]) {
+  if (gact != 1) {
+    float a[N], e[N];
+    bool in_range = true;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      a[i] = gact == 2 ? fminf(g[i], limit) : round_bf16(g[i]);
+      e[i] = __expf(gact == 2 ? -1.702f * a[i] : -a[i]);
+      in_range = in_range && fabsf(a[i]) < kDivRange && e[i] < kDivRange;      // false for what is no number
+    }
+    if (__all_sync(0xffffffffu, in_range)) {
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        const float q = div_in_range(a[i], 1.0f + e[i]);
+        if (gact == 2) out[i] = q * (fminf(fmaxf(up[i], -limit), limit) + 1.0f);
+        else out[i] = round_bf16(q) * round_bf16(up[i]);
+      }
+      return;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < N; ++i) out[i] = gated_pair(g[i], up[i], gact, limit);
+}
+
 __host__ __device__ inline int gated_flags(int gact, float limit) {
 #ifdef __CUDA_ARCH__
   const uint32_t u = __float_as_uint(limit);
@@ -160,19 +189,28 @@ __device__ __forceinline__ void epilogue_store_tile(uint32_t t_addr, const CUten
         r[j] = __float_as_uint(v * v);
       }
     }
+    [[maybe_unused]] float gated[CH / 2];
+    if constexpr (EPI == 1) {
+      // lane pair (2p, 2p+1) = (gate, up) rows of output channel n0/2 + p: the even lane takes tokens j, the odd one tokens j + 1
+      const bool odd = lane & 1;
+      float g[CH / 2], up[CH / 2];
+#pragma unroll
+      for (int j = 0; j < CH; j += 2) {
+        const uint32_t send = odd ? r[j] : r[j + 1];
+        const uint32_t recv = __shfl_xor_sync(0xffffffffu, send, 1);
+        g[j >> 1] = __uint_as_float(odd ? recv : r[j]);
+        up[j >> 1] = __uint_as_float(odd ? r[j + 1] : recv);
+      }
+      gated_pairs(g, up, gact, glimit, gated);
+    }
     if (dir.ptr != nullptr) {   // warp-uniform
       const int n = n0 + lane;
       if constexpr (EPI == 1) {
         bf16* dst = reinterpret_cast<bf16*>(dir.ptr) + (size_t)(m_base + c0) * dir.ldy + (n >> 1);
-        const bool odd = lane & 1;
 #pragma unroll
         for (int j = 0; j < CH; j += 2) {
-          const uint32_t send = odd ? r[j] : r[j + 1];
-          const uint32_t recv = __shfl_xor_sync(0xffffffffu, send, 1);
-          const float g = __uint_as_float(odd ? recv : r[j]);
-          const float up = __uint_as_float(odd ? r[j + 1] : recv);
-          const int m = m_base + c0 + j + (odd ? 1 : 0);
-          if (n < N && m < M) dst[(size_t)(j + (odd ? 1 : 0)) * dir.ldy] = __float2bfloat16_rn(gated_pair(g, up, gact, glimit));
+          const int jj = j + (lane & 1);
+          if (n < N && m_base + c0 + jj < M) dst[(size_t)jj * dir.ldy] = __float2bfloat16_rn(gated[j >> 1]);
         }
       } else if (n < N) {
         const size_t off = ((size_t)split * M + (size_t)(m_base + c0)) * dir.ldy + n;
@@ -188,18 +226,11 @@ __device__ __forceinline__ void epilogue_store_tile(uint32_t t_addr, const CUten
     uint8_t* buf = stg + which * kStgBufBytes;
     const uint32_t sbuf = smem_u32(buf);
     if constexpr (EPI == 1) {
-      // lane pair (2p, 2p+1) = (gate, up) rows of output channel n0/2 + p; staging rows are 16 channels
-      const bool odd = lane & 1;
-      const uint32_t col = sbuf + (uint32_t)(lane >> 1) * 2u;
+      const uint32_t col = sbuf + (uint32_t)(lane >> 1) * 2u;       // staging rows are 16 channels
 #pragma unroll
       for (int j = 0; j < CH; j += 2) {
-        // even lane (gate row) computes token j, odd lane (up row) computes token j+1
-        const uint32_t send = odd ? r[j] : r[j + 1];
-        const uint32_t recv = __shfl_xor_sync(0xffffffffu, send, 1);
-        const float g = __uint_as_float(odd ? recv : r[j]);
-        const float up = __uint_as_float(odd ? r[j + 1] : recv);
-        const bf16 v = __float2bfloat16_rn(gated_pair(g, up, gact, glimit));
-        st_shared_u16(col + (uint32_t)(j + (odd ? 1 : 0)) * 32u, *reinterpret_cast<const uint16_t*>(&v));
+        const bf16 v = __float2bfloat16_rn(gated[j >> 1]);
+        st_shared_u16(col + (uint32_t)(j + (lane & 1)) * 32u, *reinterpret_cast<const uint16_t*>(&v));
       }
     } else if (out_f32) {
       const uint32_t col = sbuf + (uint32_t)lane * 4u;
