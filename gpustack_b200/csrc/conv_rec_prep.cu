@@ -100,11 +100,9 @@ conv_rec_prep_vec_kernel(CrpArgs a, int lph) {
 #pragma unroll
       for (int i = 0; i < V; ++i) y[i] = bias[i];
       conv_row<TA, TAPS, NB>(win, r, w, y);
+      logistic_all<true>(y, y);
 #pragma unroll
-      for (int i = 0; i < V; ++i) {
-        y[i] = crp_silu(y[i]);
-        ss = fmaf(y[i], y[i], ss);
-      }
+      for (int i = 0; i < V; ++i) ss = fmaf(y[i], y[i], ss);
     }
     for (int o = lph >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);    // all lanes take part
     if (!act) continue;

@@ -622,7 +622,11 @@ gate_norm_heads_kernel(const float* __restrict__ y, const TA* __restrict__ proj,
   for (int n = 0; n < N; ++n) {
     const int i = i0 + n * step;
     if (n * step >= C) break;
-    g[n] = make_float4(gs_silu(g[n].x), gs_silu(g[n].y), gs_silu(g[n].z), gs_silu(g[n].w));
+    {
+      float z[4] = {g[n].x, g[n].y, g[n].z, g[n].w};
+      logistic_all<true>(z, z);
+      g[n] = make_float4(z[0], z[1], z[2], z[3]);
+    }
     float4 x = v[n];
     if (!AFTER) { x.x *= g[n].x; x.y *= g[n].y; x.z *= g[n].z; x.w *= g[n].w; }
     float ss = fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, x.w * x.w)));

@@ -48,11 +48,10 @@ head_out_kernel(const float* __restrict__ o, const TA* __restrict__ proj, int64_
       }
       if (gate_col >= 0) {
         const float gv[4] = {g[u].x, g[u].y, g[u].z, g[u].w};
+        float sg[4];
+        logistic_all<false>(gv, sg);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float sg = 1.0f / (1.0f + expf(-gv[e]));
-          v[e] *= silu ? gv[e] * sg : sg;
-        }
+        for (int e = 0; e < 4; ++e) v[e] *= silu ? gv[e] * sg[e] : sg[e];
       }
       ho_st4(out + (size_t)t * ldo + h * DV + d, make_float4(v[0], v[1], v[2], v[3]));
     }

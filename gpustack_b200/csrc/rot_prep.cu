@@ -219,11 +219,8 @@ rot_prep_vec_kernel(RotPrepArgs a, int T, int lph, int items_q, int items_v) {
         }
       }
       if (a.feature == 1) {
-#pragma unroll
-        for (int i = 0; i < VEC; ++i) {
-          x0[i] = x0[i] / (1.0f + expf(-x0[i]));
-          if (d1 >= 0) x1[i] = x1[i] / (1.0f + expf(-x1[i]));
-        }
+        logistic_all<true>(x0, x0);
+        if (d1 >= 0) logistic_all<true>(x1, x1);
       }
       if (rot && a.half_layout) {
 #pragma unroll
