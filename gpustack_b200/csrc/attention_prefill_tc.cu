@@ -12,7 +12,7 @@
 //             4 KB page (and one for the whole Q tile): the tensor maps split a row into its two 64-element halves and,
 //             for K, the tokens into groups of eight, in the order in which the operand descriptors step -- a copy
 //             costs the copy engine about 30 ns whatever its size (16 x 512 tokens, 32 / 8 heads: 73.9 us with a copy per
-//             2 KB, 71.6 us now);
+//             2 KB, 71.6 us with these);
 //   warp 5    MMA issuer (one elected thread): S_j = Q K_j^T into one of two 64-column TMEM buffers,
 //             O += P_j V_j into a 128-column TMEM accumulator.  S_{j+1} is issued BEFORE waiting for
 //             P_j, so the tensor pipe works on block j+1 while the softmax warps are busy with j;
@@ -82,6 +82,29 @@ __device__ __forceinline__ void fa_load_4d(void* dst, const CUtensorMap* map, ui
 // K-major, 128-byte swizzle, eight-row groups 2 KB apart (a page's groups hold both d-halves)
 __device__ __forceinline__ uint64_t fa_desc_k(uint32_t addr) {
   return (uint64_t)((addr & 0x3FFFFu) >> 4) | (uint64_t)1 << 16 | (uint64_t)(2048 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)2 << 61;
+}
+
+// pairs of fp32 in one register pair
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 fa_pack2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 fa_unpack2(f32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ f32x2 fa_fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 fa_add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
 }
 
 // P_TMEM: P_j is written back into the first 32 columns of the TMEM buffer S_j came from (bf16 pairs
@@ -155,22 +178,37 @@ paged_attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
   const uint32_t tmem_base = *tmem_slot;
   pdl_wait();   // Q, the KV cache and the index buffers were written by preceding kernels / copies
 
-  // one work item = (tile, kv-head); tiles are listed heaviest first, the kv-heads of a tile are adjacent
+  // One work item = (tile, kv-head); tiles are listed heaviest first, the kv-heads of a tile are adjacent.  Its metadata are two
+  // loads deep, and a warp that forms an address or a difference waits for what it is formed from: the tile's entry is fetched
+  // two items ahead, the sequence's bounds one item ahead, and nothing is derived from them before the item begins (with it and
+  // two comparisons per masked score instead of five: 16 x 512 tokens 71.6 -> 69, 1 x 8192 tokens 477 -> 482 us).
+  struct Entry {
+    int seq, q0, kvh;
+  };
+  struct Raw {
+    int seq, q0, kvh, begin, end, ctx;
+  };
   struct Work {
     int seq, kvh, q0, q_begin, q_len, ctx, total_len, n_blocks, n_pages_seq;
     int j0;   // first KV block the tile reads: 0, or with a sliding window the block of its first row's first key
   };
   const int total_work = num_tiles * Hkv;
-  auto load_work = [&](int w) {
-    Work m;
+  auto fetch_entry = [&](int w) {
     if (w >= total_work) w = total_work - 1;               // prefetch past the end: harmless re-read
     const int tile = w / Hkv;
-    m.kvh = w - tile * Hkv;
-    m.seq = __ldg(tile_seq + tile);
-    m.q0 = __ldg(tile_q0 + tile);
-    m.q_begin = __ldg(cu_q + m.seq);
-    m.q_len = __ldg(cu_q + m.seq + 1) - m.q_begin;
-    m.ctx = __ldg(ctx_lens + m.seq);
+    return Entry{__ldg(tile_seq + tile), __ldg(tile_q0 + tile), w - tile * Hkv};
+  };
+  auto fetch_raw = [&](const Entry& e) {
+    return Raw{e.seq, e.q0, e.kvh, __ldg(cu_q + e.seq), __ldg(cu_q + e.seq + 1), __ldg(ctx_lens + e.seq)};
+  };
+  auto derive = [&](const Raw& r) {
+    Work m;
+    m.kvh = r.kvh;
+    m.seq = r.seq;
+    m.q0 = r.q0;
+    m.q_begin = r.begin;
+    m.q_len = r.end - r.begin;
+    m.ctx = r.ctx;
     m.total_len = m.ctx + m.q_len;
     const int kv_end = min(m.total_len, m.ctx + m.q0 + TPT);   // causal horizon of the tile (exclusive)
     m.n_blocks = (kv_end + kFaKv - 1) / kFaKv;                 // >= 1
@@ -197,10 +235,12 @@ paged_attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
     constexpr int PPB = kFaKv / kFaPage;   // pages per KV block
     int slot = 0;
     uint32_t phase = 0, it = 0;
-    Work nxt = load_work(work_of(0));
+    Raw nxt = fetch_raw(fetch_entry(work_of(0)));
+    Entry far = fetch_entry(work_of(1));
     for (int rd = 0; rd < n_rounds; ++rd) {
-      const Work m = nxt;
-      nxt = load_work(work_of(rd + 1));     // in flight while this tile streams
+      const Work m = derive(nxt);
+      nxt = fetch_raw(far);                 // in flight while this tile streams
+      far = fetch_entry(work_of(rd + 2));
       if (work_of(rd) >= total_work) break; // only in the last, partial round
       if (lane == 0) {
         if (it > 0) mbar_wait_guarded(q_empty, (it - 1) & 1);   // previous tile's Q K^T all retired
@@ -261,10 +301,13 @@ paged_attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
         umma_commit(&s_full[gb & 1]);     // S ready for the softmax warps
       };
       uint32_t gb = 0, it = 0;
-      Work nxt = load_work(work_of(0));
+      Raw nxt = fetch_raw(fetch_entry(work_of(0)));
+      Entry far = fetch_entry(work_of(1));
       for (int rd = 0; rd < n_rounds; ++rd) {
-        const int n_blocks = nxt.n_blocks - nxt.j0;   // blocks the tile reads (>= 1); j counts them from 0 here
-        nxt = load_work(work_of(rd + 1));
+        const Work m = derive(nxt);
+        const int n_blocks = m.n_blocks - m.j0;       // blocks the tile reads (>= 1); j counts them from 0 here
+        nxt = fetch_raw(far);
+        far = fetch_entry(work_of(rd + 2));
         if (work_of(rd) >= total_work) break;
         mbar_wait_guarded(q_full, it & 1);
         tc_fence_after();
@@ -311,20 +354,31 @@ paged_attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
     const uint32_t sw = (uint32_t)(row & 7);
     const bool wide = (reinterpret_cast<uintptr_t>(out) & 31u) == 0;   // 256-bit stores: one full sector per thread
     uint32_t gb = 0, it = 0;
-    Work nxt = load_work(work_of(0));
-    for (int rd = 0; rd < n_rounds; ++rd) {
-      const Work m = nxt;
-      nxt = load_work(work_of(rd + 1));
-      if (work_of(rd) >= total_work) break;
-      const int qi = m.q0 + tok;
-      const bool valid = qi < m.q_len;
-      const int qpos = m.ctx + qi;
+    Raw nxt = fetch_raw(fetch_entry(work_of(0)));
+    Entry far = fetch_entry(work_of(1));
+    // A tile's epilogue waits for its last PV product; the next tile's first scores are there before that, so their softmax
+    // goes first (with packed multiply-adds and sums of the scores: 16 x 512 tokens 69 -> 67 us, 1 x 8192 482 -> 473).  What the epilogue
+    // needs of its tile is kept beside; one round more than there are items ends with it.
+    struct {
+      int qi, q_begin, kvh, pending;
+      bool valid;
+      float m_used, l;
+    } past;
+    past.pending = 0;
+    for (int rd = 0; rd <= n_rounds; ++rd) {
+      const Work m = derive(nxt);
+      const bool more = rd < n_rounds && work_of(rd) < total_work;
+      if (!more && !past.pending) break;
+      nxt = fetch_raw(far);
+      far = fetch_entry(work_of(rd + 2));
+      const int qpos = m.ctx + m.q0 + tok;
       const int total_len = m.total_len;
       float m_used = (CAP && bounded) ? 0.f : -INFINITY, l = 0.f;
       const float sl = CAP ? 1.f : scale_log2;    // what a (masked) score is multiplied by on its way into the exponent
 
       const int row_lo = window > 0 ? qpos - window + 1 : 0;   // first key this row sees
-      for (int j = m.j0; j < m.n_blocks; ++j, ++gb) {
+      for (int j = m.j0; more ? j < m.n_blocks : j == m.j0; ++j) {
+       if (more) {
         const uint32_t s_col = (gb & 1) * kFaKv;
         mbar_wait_guarded(&s_full[gb & 1], (gb >> 1) & 1);
         tc_fence_after();
@@ -345,11 +399,19 @@ paged_attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
         const bool need_mask = (kv0 + kFaKv - 1 > m.ctx + m.q0) || (kv0 + kFaKv - 1 >= total_len) ||
                                (window > 0 && kv0 < m.ctx + m.q0 + TPT - window);
         if (need_mask) {   // ONE warp-uniform branch per block (the condition is tile-uniform), not one per column
+          const int last = min(qpos, total_len - 1) - kv0;   // the row's last visible column of the block
 #pragma unroll
           for (int c = 0; c < 32; ++c) {
-            const int ka = kv0 + c, kb = kv0 + 32 + c;
-            if (ka > qpos || ka >= total_len || ka < row_lo) s0[c] = 0xff800000u;   // -inf
-            if (kb > qpos || kb >= total_len || kb < row_lo) s1[c] = 0xff800000u;
+            if (c > last) s0[c] = 0xff800000u;               // -inf
+            if (c + 32 > last) s1[c] = 0xff800000u;
+          }
+          if (window > 0) {
+            const int first = row_lo - kv0;
+#pragma unroll
+            for (int c = 0; c < 32; ++c) {
+              if (c < first) s0[c] = 0xff800000u;
+              if (c + 32 < first) s1[c] = 0xff800000u;
+            }
           }
         }
         // row maximum on the raw scores (scale > 0 commutes with max); the scale itself is folded
@@ -371,20 +433,21 @@ paged_attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
           rescale = j > m.j0;
         }
         uint32_t pk[32];
-        float sum = 0.f;
+        f32x2 sum2 = 0ull;
         // a row whose window starts after this block has seen nothing yet (m_used = -inf): its probabilities are 0
         const float neg_m = m_used == -INFINITY ? 0.f : -m_used;
+        const f32x2 sl2 = fa_pack2(sl, sl), neg2 = fa_pack2(neg_m, neg_m);
 #pragma unroll
         for (int c = 0; c < 32; c += 2) {
-          const float p0 = ex2_approx(fmaf(__uint_as_float(s0[c]), sl, neg_m));
-          const float p1 = ex2_approx(fmaf(__uint_as_float(s0[c + 1]), sl, neg_m));
-          const float p2 = ex2_approx(fmaf(__uint_as_float(s1[c]), sl, neg_m));
-          const float p3 = ex2_approx(fmaf(__uint_as_float(s1[c + 1]), sl, neg_m));
-          sum += (p0 + p1) + (p2 + p3);
+          const float2 x = fa_unpack2(fa_fma2(fa_pack2(__uint_as_float(s0[c]), __uint_as_float(s0[c + 1])), sl2, neg2));
+          const float2 y = fa_unpack2(fa_fma2(fa_pack2(__uint_as_float(s1[c]), __uint_as_float(s1[c + 1])), sl2, neg2));
+          const float p0 = ex2_approx(x.x), p1 = ex2_approx(x.y), p2 = ex2_approx(y.x), p3 = ex2_approx(y.y);
+          sum2 = fa_add2(sum2, fa_add2(fa_pack2(p0, p1), fa_pack2(p2, p3)));
           pk[c >> 1] = pack_bf16(p0, p1);
           pk[16 + (c >> 1)] = pack_bf16(p2, p3);
         }
-        l += sum;
+        const float2 sums = fa_unpack2(sum2);
+        l += sums.x + sums.y;
         const bool any_rescale = __any_sync(0xffffffffu, rescale);
         // the previous block's PV (possibly the previous tile's last) must have retired before the
         // shared-memory P buffer is overwritten / before O is rescaled (any_rescale implies j > 0)
@@ -426,27 +489,34 @@ paged_attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive((gb & 1) ? p_full_b : p_full);
-      }
+        ++gb;
+       }
+       if (!past.pending) continue;
 
-      // ---- epilogue: O / l -> bf16 -> out[token, head, :]
-      mbar_wait_guarded(o_full, it & 1);
+      // ---- epilogue of the tile before: O / l -> bf16 -> out[token, head, :]
+      past.pending = 0;
+      mbar_wait_guarded(o_full, (it - 1) & 1);
       tc_fence_after();
+      const int qi = past.qi;
+      const bool valid = past.valid;
+      const float m_used = past.m_used;
+      float l = past.l;
       // softmax sink (mixers that have one): a learned per-head logit that joins the denominator only;
       // l is relative to the reference maximum m_used of the base-2 domain
-      if (sink != nullptr && m_used > -INFINITY) l += exp2f(sink[m.kvh * G + g] * 1.4426950408889634f - m_used);
+      if (sink != nullptr && m_used > -INFINITY) l += exp2f(sink[past.kvh * G + g] * 1.4426950408889634f - m_used);
       float inv = l > 0.f ? 1.f / l : 0.f;
       // the row's log-sum-exp (natural logarithm of the softmax denominator), for a caller that goes on with more keys
       if (lse_out != nullptr && valid)
-        lse_out[(size_t)(m.q_begin + qi) * Hq + (size_t)(m.kvh * G + g)] =
+        lse_out[(size_t)(past.q_begin + qi) * Hq + (size_t)(past.kvh * G + g)] =
             l > 0.f ? (m_used + log2f(l)) * 0.6931471805599453f : -INFINITY;
-      bf16* orow = out + ((size_t)(m.q_begin + qi) * Hq + (size_t)(m.kvh * G + g)) * kFaD;
+      bf16* orow = out + ((size_t)(past.q_begin + qi) * Hq + (size_t)(past.kvh * G + g)) * kFaD;
       // sigmoid output gate (mixers that have one): gate[token][head * D + column], same columns as the row -- or ONE
       // number per head, gate[token][head], which joins the row's normaliser
       const bf16* grow = (gate != nullptr && valid && !gate_per_head)
-                             ? gate + (size_t)(m.q_begin + qi) * gate_stride + (size_t)(m.kvh * G + g) * kFaD
+                             ? gate + (size_t)(past.q_begin + qi) * gate_stride + (size_t)(past.kvh * G + g) * kFaD
                              : nullptr;
       if (gate != nullptr && valid && gate_per_head) {
-        const float gv = __bfloat162float(gate[(size_t)(m.q_begin + qi) * gate_stride + (size_t)(m.kvh * G + g)]);
+        const float gv = __bfloat162float(gate[(size_t)(past.q_begin + qi) * gate_stride + (size_t)(past.kvh * G + g)]);
         inv *= 1.f / (1.f + __expf(-gv));
       }
       auto store32 = [&](const uint32_t (&o)[32], bf16* dst) {            // 32 fp32 columns -> 64 bytes of the row
@@ -498,6 +568,15 @@ paged_attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
           store32(o1, orow + c4 * 32 + 32);
         }
       }
+      }
+      past.qi = m.q0 + tok;
+      past.q_begin = m.q_begin;
+      past.kvh = m.kvh;
+      past.valid = past.qi < m.q_len;
+      past.m_used = m_used;
+      past.l = l;
+      past.pending = more;
+      if (!more) break;
       ++it;
     }
   }
