@@ -26,11 +26,12 @@ namespace b200 {
 constexpr int kRbPerLane = 8;        // E <= 256
 constexpr int kRbMaxTop = 16;
 
-__device__ __forceinline__ float rb_f32(float v) { return v; }
-__device__ __forceinline__ float rb_f32(bf16 v) { return __bfloat162float(v); }
-__device__ __forceinline__ float4 rb_f32x4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-__device__ __forceinline__ float4 rb_f32x4(const bf16* p) {
-  const uint2 v = *reinterpret_cast<const uint2*>(p);
+// (what the kernels before wrote is read past L1: a grid that became resident early has missed its invalidation)
+__device__ __forceinline__ float rb_cg(const float* p) { return __ldcg(p); }
+__device__ __forceinline__ float rb_cg(const bf16* p) { return __bfloat162float(__ldcg(p)); }
+__device__ __forceinline__ float4 rb_cg4(const float* p) { return __ldcg(reinterpret_cast<const float4*>(p)); }
+__device__ __forceinline__ float4 rb_cg4(const bf16* p) {
+  const uint2 v = __ldcg(reinterpret_cast<const uint2*>(p));
   return make_float4(bf16_lo(v.x), bf16_hi(v.x), bf16_lo(v.y), bf16_hi(v.y));
 }
 
@@ -179,7 +180,7 @@ moe_router_kernel(const bf16* __restrict__ x, int64_t ldx, const bf16* __restric
     for (int r = 0; r < kRtRows; ++r) acc[r][0] = acc[r][1] = 0.f;
 #pragma unroll 8
     for (int d = lane * 8; d < D; d += 256) {
-      const uint4 u0 = ld_v4(x0 + d), u1 = ld_v4(x1 + d);
+      const uint4 u0 = ld_cg_v4(x0 + d), u1 = ld_cg_v4(x1 + d);
       const uint32_t p[4] = {u0.x, u0.y, u0.z, u0.w}, q[4] = {u1.x, u1.y, u1.z, u1.w};
 #pragma unroll
       for (int r = 0; r < kRtRows; ++r) {
@@ -226,29 +227,29 @@ moe_combine_mixed_kernel(const TP* __restrict__ yp, int64_t ldp, const int32_t* 
     if constexpr (VEC) {
       float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
       for (int j = 0; j < K; ++j) {
-        const int id = topk_ids[(size_t)t * K + j];
+        const int id = __ldcg(topk_ids + (size_t)t * K + j);
         if (id < n_real) {
-          const float4 v = rb_f32x4(yp + (size_t)pair_row[(size_t)t * K + j] * ldp + d);
+          const float4 v = rb_cg4(yp + (size_t)__ldcg(pair_row + (size_t)t * K + j) * ldp + d);
           acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
         } else {
-          const float w = topk_w[(size_t)t * K + j];
-          const float4 v = rb_f32x4(x + (size_t)t * ldx + d);
+          const float w = __ldcg(topk_w + (size_t)t * K + j);
+          const float4 v = rb_cg4(x + (size_t)t * ldx + d);
           acc.x += w * v.x; acc.y += w * v.y; acc.z += w * v.z; acc.w += w * v.w;
         }
       }
       if (shared != nullptr) {
-        const float4 v = rb_f32x4(shared + (size_t)t * lds + d);
+        const float4 v = rb_cg4(shared + (size_t)t * lds + d);
         acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
       }
       *reinterpret_cast<float4*>(out + (size_t)t * ldo + d) = acc;
     } else {
       float acc = 0.f;
       for (int j = 0; j < K; ++j) {
-        const int id = topk_ids[(size_t)t * K + j];
-        if (id < n_real) acc += rb_f32(yp[(size_t)pair_row[(size_t)t * K + j] * ldp + d]);
-        else acc += topk_w[(size_t)t * K + j] * rb_f32(x[(size_t)t * ldx + d]);
+        const int id = __ldcg(topk_ids + (size_t)t * K + j);
+        if (id < n_real) acc += rb_cg(yp + (size_t)__ldcg(pair_row + (size_t)t * K + j) * ldp + d);
+        else acc += __ldcg(topk_w + (size_t)t * K + j) * rb_cg(x + (size_t)t * ldx + d);
       }
-      if (shared != nullptr) acc += rb_f32(shared[(size_t)t * lds + d]);
+      if (shared != nullptr) acc += rb_cg(shared + (size_t)t * lds + d);
       out[(size_t)t * ldo + d] = acc;
     }
   }
