@@ -105,6 +105,95 @@ latent_prep_kernel(const TA* __restrict__ proj, int64_t ld, int kv_col, const TA
   }
 }
 
+// The same for bf16 rows of 512 + 64 whose whole rotated part turns: a warp per token, nothing shared, no barrier.  Lane l holds
+// the latent's columns 8 l and 256 + 8 l (16 bytes each) and entries 2 l, 2 l + 1 of every 64-wide part; the token's loads are in
+// flight together.  Bound: latency, then HBM; the kernel above, a CTA per token with two-byte accesses, took 42 us for 8192 rows of
+// 16 heads and 10 us for 64, this one 10 and 4.4.
+constexpr int kLpHeads = 8;                            // heads in flight
+
+__global__ void __launch_bounds__(kLtWarps * 32)
+latent_prep_rows_kernel(const bf16* __restrict__ proj, int64_t ld, int kv_col, const bf16* __restrict__ q, int64_t ldq,
+                        const bf16* __restrict__ kv_norm_w, const int32_t* __restrict__ positions, const int32_t* __restrict__ slots,
+                        bf16* cache, bf16* qa, int64_t ldqa, int T, int H, int dn, int half_layout, const double* __restrict__ freq,
+                        float mag, float eps) {
+  constexpr int R = 512, DR = 64;
+  const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (t >= T) return;
+  const int pos = positions[t], slot = slots[t];
+  const bf16* kv = proj + (size_t)t * ld + kv_col;
+  const bf16* qr = q + (size_t)t * ldq + dn + 2 * lane;
+  uint4 lat[2], wn[2];
+  uint32_t part[kLpHeads + 1];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    lat[i] = ld_v4(kv + i * 256 + lane * 8);
+    wn[i] = ld_v4(kv_norm_w + i * 256 + lane * 8);
+  }
+  part[kLpHeads] = *reinterpret_cast<const uint32_t*>(kv + R + 2 * lane);
+#pragma unroll
+  for (int h = 0; h < kLpHeads; ++h) part[h] = h < H ? *reinterpret_cast<const uint32_t*>(qr + (size_t)h * (dn + DR)) : 0u;
+  // lane l: the angle of pair l, formed and reduced in fp64 as above
+  const double ang = (double)pos * freq[lane];
+  const double turns = rint(ang * 0.15915494309189535);
+  float sl, cl;
+  sincosf((float)fma(-turns, 6.283185307179586, ang), &sl, &cl);
+  cl *= mag;
+  sl *= mag;
+  // half layout: entry d turns with entry d ^ 32 by pair d % 32, so lanes 16 apart exchange; interleaved: a lane's own two entries
+  float c0 = cl, s0 = sl, c1 = cl, s1 = sl;
+  if (half_layout) {
+    const int i = (2 * lane) & 31;
+    c0 = __shfl_sync(0xffffffffu, cl, i);
+    s0 = __shfl_sync(0xffffffffu, sl, i);
+    c1 = __shfl_sync(0xffffffffu, cl, i + 1);
+    s1 = __shfl_sync(0xffffffffu, sl, i + 1);
+  }
+  const bool upper = lane >= 16;
+  auto turn = [&](uint32_t v) {
+    const float a = bf16_lo(v), b = bf16_hi(v);
+    if (!half_layout) return pack_bf16(a * c0 - b * s0, b * c0 + a * s0);
+    const uint32_t o = __shfl_xor_sync(0xffffffffu, v, 16);
+    const float oa = bf16_lo(o), ob = bf16_hi(o);
+    return upper ? pack_bf16(a * c0 + oa * s0, b * c1 + ob * s1) : pack_bf16(a * c0 - oa * s0, b * c1 - ob * s1);
+  };
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const uint32_t v[4] = {lat[i].x, lat[i].y, lat[i].z, lat[i].w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) ss = fmaf(bf16_hi(v[e]), bf16_hi(v[e]), fmaf(bf16_lo(v[e]), bf16_lo(v[e]), ss));
+  }
+  const float mul = 1.0f / sqrtf(warp_sum(ss) / (float)R + eps);
+  const uint32_t key = turn(part[kLpHeads]);
+  if (slot >= 0) {                                     // (a padding row has nothing to cache)
+    bf16* row = cache + (size_t)slot * (R + DR);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const uint32_t v[4] = {lat[i].x, lat[i].y, lat[i].z, lat[i].w}, w[4] = {wn[i].x, wn[i].y, wn[i].z, wn[i].w};
+      uint32_t o[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[e] = pack_bf16(bf16_lo(v[e]) * mul * bf16_lo(w[e]), bf16_hi(v[e]) * mul * bf16_hi(w[e]));
+      st_v4(row + i * 256 + lane * 8, make_uint4(o[0], o[1], o[2], o[3]));
+    }
+    *reinterpret_cast<uint32_t*>(row + R + 2 * lane) = key;
+  }
+  bf16* qd = qa + (size_t)t * ldqa + R + 2 * lane;
+  for (int h0 = 0; h0 < H; h0 += kLpHeads) {
+    uint32_t next[kLpHeads];
+#pragma unroll
+    for (int h = 0; h < kLpHeads; ++h) {
+      const int n = h0 + kLpHeads + h;
+      next[h] = n < H ? *reinterpret_cast<const uint32_t*>(qr + (size_t)n * (dn + DR)) : 0u;
+    }
+#pragma unroll
+    for (int h = 0; h < kLpHeads; ++h) {
+      const uint32_t v = turn(part[h]);
+      if (h0 + h < H) *reinterpret_cast<uint32_t*>(qd + (size_t)(h0 + h) * (R + DR)) = v;
+      part[h] = next[h];
+    }
+  }
+}
+
 }  // namespace b200
 
 using namespace b200;
@@ -129,6 +218,16 @@ extern "C" int b200_latent_prep(const void* proj, int f32, int64_t ld, int kv_co
                "latent_prep: bad shape H=%d dn=%d dr=%d R=%d dims=%d", H, dn, dr, R, dims);
   if (T == 0) return B200_OK;
   cudaStream_t s = (cudaStream_t)stream;
+  // four-byte pieces of the rotated parts, sixteen-byte ones of the latents
+  auto al = [](const void* p, int n) { return (reinterpret_cast<uintptr_t>(p) & (n - 1)) == 0; };
+  if (!f32 && R == 512 && dr == 64 && dims == 64 && ld % 8 == 0 && kv_col % 8 == 0 && ldq % 2 == 0 && dn % 2 == 0 && ldqa % 2 == 0 &&
+      al(proj, 16) && al(kv_norm_w, 16) && al(cache, 16) && al(q, 4) && al(qa, 4)) {
+    const int warps = T >= 4 * 148 ? kLtWarps : 1;     // few rows: a CTA each, over as many SMs
+    latent_prep_rows_kernel<<<(T + warps - 1) / warps, warps * 32, 0, s>>>((const bf16*)proj, ld, kv_col, (const bf16*)q, ldq,
+                                                                          (const bf16*)kv_norm_w, positions, slots, (bf16*)cache,
+                                                                          (bf16*)qa, ldqa, T, H, dn, half_layout, freq, mag, eps);
+    return b200_check_launch("b200_latent_prep");
+  }
   dim3 grid(T);
   const int threads = 32 * (H + 1 < kLtWarps ? H + 1 : kLtWarps);
   if (f32)

@@ -131,3 +131,43 @@ def test_single_rows_at_the_edges_of_key_blocks(H, R, dr, splits):
     for b, n in enumerate(lens):
         if n:
             assert float((got[b] - want[b]).norm() / want[b].norm()) < 2 * 2.0 ** -8, n
+
+
+@pytest.mark.parametrize("half", [True, False])
+@pytest.mark.parametrize("T,H", [(1, 1), (3, 8), (5, 17), (597, 16)])
+def test_preparation_of_rows(T, H, half):
+    """One warp per row: heads below, at and beyond a batch of eight, a remainder of rows in the last CTA, a padding row."""
+    from gpustack_b200 import ops
+
+    g = torch.Generator().manual_seed(T + H)
+    dn, kv_col, mag, eps = 6, 8, 1.25, 1e-5
+    proj, q = torch.randn(T, kv_col + R + DR + 8, generator=g).to(BF), torch.randn(T, H * (dn + DR), generator=g).to(BF)
+    w, pos = torch.randn(R, generator=g).to(BF), torch.randint(0, 100000, (T,), generator=g, dtype=torch.int32)
+    freq = 10000.0 ** (-torch.arange(DR // 2, dtype=F64) / 32)
+    slots = torch.randperm(T + 16, generator=g)[:T].to(torch.int32)
+    if T > 1:
+        slots[T // 2] = -1
+    pages = -(-(T + 16) // 16)
+    cache, qa = torch.full((pages, 1, 16, R + DR), 9.0, dtype=BF, device="cuda"), torch.full((T, H * (R + DR)), 9.0, dtype=BF, device="cuda")
+    ops.latent_prep(proj.cuda(), kv_col, q.cuda(), w.cuda(), pos.cuda(), slots.cuda(), cache, qa, H, dn, DR, R, DR, half, freq.cuda(), mag, eps)
+
+    def turn(x):                                       # [..., T, 64]
+        ang = pos.to(F64)[:, None] * freq
+        c, s = torch.cos(ang) * mag, torch.sin(ang) * mag
+        a, b = (x[..., :32], x[..., 32:]) if half else (x[..., ::2], x[..., 1::2])
+        u, v = a * c - b * s, b * c + a * s
+        return torch.cat([u, v], -1) if half else torch.stack([u, v], -1).flatten(-2)
+
+    lat = proj[:, kv_col:kv_col + R].to(F64)
+    want = torch.cat([lat / torch.sqrt((lat * lat).mean(-1, keepdim=True) + eps) * w.to(F64), turn(proj[:, kv_col + R:kv_col + R + DR].to(F64))], -1)
+    live = slots >= 0
+    got = cache.view(-1, R + DR)[slots[live].long().cuda()]
+    # one rounding to bf16 (2^-9 of each value; an angle's reduction and the fp32 products are far below)
+    assert float((got.cpu().to(F64) - want[live]).abs().max() / want.abs().max()) < 2.0 ** -8
+    assert _rel(got, want[live]) < 2.0 ** -9
+    rest = torch.ones(pages * 16, dtype=torch.bool)
+    rest[slots[live].long()] = False
+    assert bool((cache.view(-1, R + DR).cpu()[rest] == 9.0).all())
+    parts = turn(q.view(T, H, dn + DR)[..., dn:].to(F64).transpose(0, 1)).transpose(0, 1)
+    assert _rel(qa.view(T, H, R + DR)[..., R:], parts) < 2.0 ** -9
+    assert bool((qa.view(T, H, R + DR)[..., :R] == 9.0).all())
