@@ -101,8 +101,8 @@ def test_products_of_all_heads(H, N, K, pad, M, f32):
 @pytest.mark.parametrize("H,R,dr", [(16, 512, 64), (9, 128, 16), (17, 384, 48), (1, 256, 0)])
 def test_single_rows_at_the_edges_of_key_blocks(H, R, dr, splits):
     """One new row per sequence: lengths around the blocks of 32 keys and their halves, a row without keys, widths of an odd number of 16-column
-    steps, 1 to 16 heads per CTA.  bf16 probabilities and outputs: each rounds by at most 2^-9 of its value, so the norm of the
-    error stays below 2^-8 of the output's (values of one size, cancellation within a factor of 2)."""
+    steps, 1 to 16 heads per CTA.  bf16 probabilities and outputs: each rounds by at most 2^-8 of its value (half a unit in the
+    last of 8 bits), so the two together stay below 2 * 2^-8 of the output's norm."""
     from gpustack_b200 import ops
 
     lens = [1, 15, 16, 17, 31, 32, 33, 97, 0, 513]
