@@ -624,13 +624,17 @@ def mlstm_state_slices(dv: int) -> int:
 CHUNK_SCAN_MAX_BYTES = 1 << 30
 
 
-def _chunk_scan_workspace(rows: int, n_seqs: int, H: int, dk: int, dv: int, max_len: int, device, per_channel: bool = False):
+def _chunk_scan_workspace(rows: int, n_seqs: int, H: int, dk: int, dv: int, max_len: int, device, per_channel: bool = False,
+                          short: bool = False):
     """Workspace of the scans that run a prompt portion's chunks of 64 rows side by side, or None where the one-pass scans are
     the better ones: key widths the chunk kernels do not take, and steps of short portions (three launches instead of one).
-    All rows beyond max_len are taken for single ones.  Measured, 8 heads of 128 x 128, L2 cold, one-pass -> chunks, linear
-    attention: one portion of 64 rows 34 -> 42 us, 128 rows 57 -> 42, 512 rows 199 -> 46, 2048 rows 762 -> 75; 4 of 64 rows
-    35 -> 48; 16 of 32 rows 55 -> 73, of 64 rows 92 -> 85, of 512 rows 621 -> 255; mLSTM within 10 us of these."""
-    if dk not in (64, 128) or dv % 4 or max_len < 128 or max_len < 96 * (n_seqs - max(0, rows - max_len)):
+    All rows beyond max_len are taken for single ones.  Measured, 8 heads, L2 cold, one-pass -> chunks, linear attention of 128 x
+    128: one portion of 64 rows 33 -> 32 us, 128 rows 57 -> 38, 512 rows 197 -> 42, 2048 rows 758 -> 69; 4 of 64 rows 33 -> 38; 16
+    of 32 rows 54 -> 54, of 64 rows 92 -> 60, of 512 rows 621 -> 206; mLSTM alike.  short: scans whose one-pass form takes 0.15 us a
+    row (gated linear attention of 64 x 128: one portion of 128 rows 27 -> 48, 512 rows 83 -> 50, 2048 rows 303 -> 73; 16 of 128
+    rows 66 -> 77, of 512 rows 221 -> 212) start at 256 rows, and at 512 when there are more than one portion's."""
+    least = 128 if not short else 256 if rows < 2 * max_len else 512
+    if dk not in (64, 128) or dv % 4 or max_len < least or max_len < 96 * (n_seqs - max(0, rows - max_len)):
         return None
     n = (rows // 64 + min(n_seqs, rows // 17)) * H * (dk * dv + dk + 4 + (128 * dk if per_channel else 0))
     return torch.empty(n, dtype=torch.float32, device=device) if 4 * n <= CHUNK_SCAN_MAX_BYTES else None
@@ -818,7 +822,7 @@ def gla_scan(x, q_col: int, k_col: int, v_col: int, z, inv_tau: float, cu_seq, c
     _cuda(x, z, cu_seq, ctx_lens, state_slots, S, o_raw)
     _req(x, torch.float32, "x"); _req(z, torch.float32, "z"); _req(S, torch.float32, "S"); _req(o_raw, torch.float32, "o_raw")
     n = state_slots.shape[0]
-    ws = _chunk_scan_workspace(x.shape[0], n, H, dk, dv, max_len, x.device, per_channel=True)
+    ws = _chunk_scan_workspace(x.shape[0], n, H, dk, dv, max_len, x.device, per_channel=True, short=True)
     if ws is not None:
         check(load().b200_gla_scan_chunked(_p(x), x.stride(0), q_col, k_col, v_col, _p(z), z.stride(0), inv_tau, _p(cu_seq),
                                            _p(ctx_lens), _p(state_slots), _p(S), _p(o_raw), n, H, dk, dv, int(max_len), x.shape[0],
@@ -944,7 +948,7 @@ def gated_scan(x, q_col: int, k_col: int, v_col: int, gates, rate, dt_bias, skip
     if tuple(S.shape[1:]) != (H, dv, -(-dk // 4) * 4) or not S.is_contiguous() or not o_raw.is_contiguous():
         raise B200Error("gated_scan: a contiguous state of [slots, heads, dv, dk rounded up to 4]")
     n = state_slots.shape[0]
-    ws = None if delta else _chunk_scan_workspace(x.shape[0], n, H, dk, dv, max_len, x.device)
+    ws = None if delta else _chunk_scan_workspace(x.shape[0], n, H, dk, dv, max_len, x.device, short=True)
     if ws is not None:
         check(load().b200_gated_scan_chunked(_p(x), x.stride(0), q_col, k_col, v_col, _p(gates), gates.stride(0), _p(rate), _p(dt_bias),
                                              _p(skip), _p(cu_seq), _p(ctx_lens), _p(state_slots), _p(S), _p(o_raw), n, H, G, dk, dv, 0,
