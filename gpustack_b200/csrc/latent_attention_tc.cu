@@ -16,8 +16,11 @@
 //             and zeros behind it: probability zero times a stale page's content must not be no number;
 //   warp 5    MMA issuer (leading CTA): S = Q K^T (M 256, N 96), O += P V (M 256, N 256, P from tensor memory);
 //             S of block j + 1 is issued before P of block j is waited for;
-//   warps 0-3 softmax: thread = pair.  Base-2 online softmax with a lazily moved reference (by more than 2^8, as the other
-//             tensor-core attention kernels), P in bf16 over the score columns, O / (l + sink) at the end.
+//   warps 0-3 softmax: thread = pair.  Base-2 online softmax whose reference is the running maximum, so that a row's largest
+//             probability is exactly 1 in bf16, P in bf16 over the score columns, l the sum of P as it was rounded, O / (l + sink)
+//             at the end.  (A reference that moves by more than 2^8 only, as in the other tensor-core attention kernels, rounds the
+//             largest probability like any other: the error of P V over 512 to 2048 keys is 1.4 to 1.6 times as large.  The rescaling it
+//             saves, 25 us of the whole layer's 573 for 4 x 2048 rows of 16 heads, is not worth that.)
 // Persistent: one pair of CTAs per two SMs walks the heaviest-first (tile, sub-tile, half) list back and forth; barriers, tensor
 // memory and rings live for the whole kernel, so an item's epilogue overlaps the next one's loads and first scores.
 // Bound: the key ring's round trip (a unit's release to its refill crosses both CTAs and L2, with 54 KB in flight); leaving out
@@ -48,7 +51,6 @@ constexpr int kLtOffV = kLtOffK + kLtKSlots * kLtKUnit;
 constexpr int kLtOffBar = kLtOffV + kLtVUnits * kLtVUnit;     // 227,328
 constexpr int kLtSmemBytes = kLtOffBar + 256 + 1024;
 constexpr int kLtColS = 256, kLtColStep = 128;         // O: columns [0, 256), S0 from 256, S1 from 384
-constexpr float kLtRescale = 8.f;                      // log2 units
 
 __device__ __forceinline__ void umma_bf16_ts_2sm(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
                                                  uint32_t accumulate) {
@@ -387,7 +389,7 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         mx *= a.scale_log2;
         float alpha = 1.f;
         bool rescale = false;
-        if (mx > m_used + kLtRescale) {
+        if (mx > m_used) {
           alpha = ex2_approx(m_used - mx);
           m_used = mx;
           l *= alpha;
@@ -402,8 +404,9 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
           for (int i = 0; i < 32; i += 2) {
             const float p0 = ex2_approx(fmaf(__uint_as_float(s[c][i]), a.scale_log2, neg_m));
             const float p1 = ex2_approx(fmaf(__uint_as_float(s[c][i + 1]), a.scale_log2, neg_m));
-            sum += p0 + p1;
-            pk[c >> 1][(c & 1) * 16 + (i >> 1)] = pack_bf16(p0, p1);
+            const uint32_t both = pack_bf16(p0, p1);
+            sum += bf16_lo(both) + bf16_hi(both);
+            pk[c >> 1][(c & 1) * 16 + (i >> 1)] = both;
           }
         l += sum;
         if (__any_sync(0xffffffffu, rescale)) {        // (implies j > 0) the block before's product has retired

@@ -1,4 +1,6 @@
 """Latent attention of prompt portions on CTA pairs, and the products of all heads in one launch, against fp64."""
+import math
+
 import pytest
 import torch
 
@@ -74,6 +76,31 @@ def test_a_growing_maximum_moves_the_reference():
                             _i32([n - 1]), _i32(ts), _i32(tq), None, out, H, R, DR, 1.0)
     p = (q[0].to(F64) @ C.to(F64).T).softmax(-1)
     assert _rel(out.view(H, R), p @ C[:, :R].to(F64)) < 2 * 2.0 ** -9
+
+
+def test_the_largest_probability_is_exact():
+    """A key that outweighs an earlier block's by 4 (1 + 2^-8), halfway between two bf16 numbers: relative to the earlier block's
+    maximum its probability would be off by 2^-8, relative to its own it is 1."""
+    from gpustack_b200 import ops
+
+    H, n = 16, 200
+    delta = 2.0 + math.log2(1 + 2.0 ** -8)                       # base-2 distance of the two scores
+    C = torch.zeros(n, R + DR)
+    C[:, R] = -100.0                                             # every other key's weight is 2^-200
+    C[3, R], C[150, R] = 0.0, 1.0
+    C[150, :R] = torch.randn(R, generator=torch.Generator().manual_seed(5))
+    C = C.to(BF)
+    q = torch.zeros(1, H, R + DR, dtype=BF)
+    q[..., R] = 1.0
+    cache = torch.zeros((n + 15) // 16, 1, 16, R + DR, dtype=BF)
+    cache.view(-1, R + DR)[:n] = C
+    out = torch.zeros(1, H * R, dtype=BF, device="cuda")
+    ts, tq = ops.build_prefill_tiles([1], ops.attn_sink_prefill_tile(), [n - 1])
+    ops.latent_attn_prefill(q.view(1, -1).cuda(), cache.cuda(), torch.arange(cache.shape[0], dtype=torch.int32).view(1, -1).cuda(), _i32([0, 1]),
+                            _i32([n - 1]), _i32(ts), _i32(tq), None, out, H, R, DR, delta * math.log(2.0))
+    want = (C[150, :R].to(F64) * (2.0 ** delta / (1 + 2.0 ** delta))).expand(H, R)
+    # the output's rounding, at most 2^-9, and the smaller probability's, 2^-9 of a fifth of the weight
+    assert _rel(out.view(H, R), want) < 1.2 * 2.0 ** -9
 
 
 @pytest.mark.parametrize("f32", [False, True])
