@@ -260,14 +260,11 @@ __device__ __forceinline__ void epilogue_store_tile(uint32_t t_addr, const CUten
 //        values of an output channel sit in adjacent TMEM lanes = adjacent threads of one warp;
 //        a lane pair swaps halves with one shuffle per two tokens and writes
 //        act[m, i] = bf16(bf16(silu(bf16(g))) * bf16(u)) -- the same roundings as the unfused path.
-// MC 2: the kernel runs as clusters of two CTAs that own ADJACENT weight tiles of the same
-//       (m-tile, k-split).  Each CTA loads its own weight tile and HALF of the shared activation
-//       tile, multicast into both CTAs' shared memory, so the activation bytes an SM has to ingest
-//       from L2 are halved (the measured limiter of decode-shaped tiles).  Stage release is a
-//       multicast tcgen05.commit: a slot is reused only after BOTH CTAs' MMAs have read it.
+// Every CTA loads its own activation tile: 16 tokens, L2 cold, 4096 -> 4096 14.4 us, 14336 -> 4096 28.7, 8192 -> 2048 14.4, gate-up
+// 2048 -> 16384 20.5 (with pairs of CTAs that shared one: 16.4, 30.7, 16.4 and 22.4).
 // HEADS 1: `splits` independent products instead of K ranges of one: product h multiplies columns h * x_head ... of X with
 // weight rows h * N ... and stores output plane h (the output map's plane pitch is the distance of two heads' columns).
-template <int BLOCK_X, int EPI, int MC, int HEADS = 0>
+template <int BLOCK_X, int EPI, int HEADS = 0>
 __device__ __forceinline__ void gemm_1sm_body(const CUtensorMap& tmap_w, const CUtensorMap& tmap_x, const CUtensorMap& tmap_y, int M,
                                               int N, int K, int out_f32, int splits, int n_tiles, int m_tiles, int group_m,
                                               DirectOut dir, int x_head = 0) {
@@ -285,7 +282,6 @@ __device__ __forceinline__ void gemm_1sm_body(const CUtensorMap& tmap_w, const C
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const uint32_t crank = MC > 1 ? cluster_ctarank() : 0u;
   pdl_launch_dependents();  // the next kernel may start its prologue while this one runs
 
   if (threadIdx.x == 0) {
@@ -294,7 +290,7 @@ __device__ __forceinline__ void gemm_1sm_body(const CUtensorMap& tmap_w, const C
     tma_prefetch_desc(&tmap_y);
     for (int i = 0; i < STAGES; ++i) {
       mbar_init(&full_bar[i], 1);
-      mbar_init(&empty_bar[i], MC);  // one multicast commit per CTA of the cluster
+      mbar_init(&empty_bar[i], 1);
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&tmem_full[i], 1);
@@ -308,7 +304,6 @@ __device__ __forceinline__ void gemm_1sm_body(const CUtensorMap& tmap_w, const C
   }
   tc_fence_before();
   __syncthreads();
-  if constexpr (MC > 1) cluster_sync_all();  // peers' barriers are initialised before any remote arrive
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   // everything above (barrier init, TMEM allocation, descriptor prefetch) overlapped with the tail
@@ -316,11 +311,8 @@ __device__ __forceinline__ void gemm_1sm_body(const CUtensorMap& tmap_w, const C
   pdl_wait();
 
   const int kb_per_split = HEADS ? K / kBlockK : (K / kBlockK) / splits;
-  // with MC == 2 a "unit" is a PAIR of adjacent weight tiles; this CTA takes tile 2*pair + crank
-  const int n_units = (n_tiles + MC - 1) / MC;
-  const int total_units = n_units * m_tiles * splits;
-  const int first_unit = MC > 1 ? (int)(blockIdx.x / MC) : (int)blockIdx.x;
-  const int unit_stride = MC > 1 ? (int)(gridDim.x / MC) : (int)gridDim.x;
+  const int total_units = n_tiles * m_tiles * splits;
+  const int first_unit = (int)blockIdx.x, unit_stride = (int)gridDim.x;
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -329,25 +321,16 @@ __device__ __forceinline__ void gemm_1sm_body(const CUtensorMap& tmap_w, const C
       int stage = 0;
       uint32_t phase = 0;
       for (int u = first_unit; u < total_units; u += unit_stride) {
-        const TileCoord c = decode_unit(u, n_units, m_tiles, splits, group_m);
-        const int n_tile = c.n_tile * MC + (int)crank;
+        const TileCoord c = decode_unit(u, n_tiles, m_tiles, splits, group_m);
         const int k0 = HEADS ? 0 : c.split * kb_per_split * kBlockK;
-        const int x0 = HEADS ? c.split * x_head : k0, w_row = n_tile * kBlockW + (HEADS ? c.split * N : 0);
+        const int x0 = HEADS ? c.split * x_head : k0, w_row = c.n_tile * kBlockW + (HEADS ? c.split * N : 0);
         for (int kb = 0; kb < kb_per_split; ++kb) {
           mbar_wait_guarded(&empty_bar[stage], phase ^ 1);
           uint8_t* a = smem + stage * Cfg::kStageBytes;
           uint8_t* b = a + Cfg::kABytes;
           mbar_expect_tx(&full_bar[stage], Cfg::kStageBytes);
           tma_load_2d(a, &tmap_w, &full_bar[stage], k0 + kb * kBlockK, w_row, hint_w);
-          if constexpr (MC > 1) {
-            constexpr int HALF = BLOCK_X / MC;  // rows of the activation tile this CTA fetches
-            tma_load_2d_mc(b + crank * (HALF * kBlockK * 2), &tmap_x, &full_bar[stage],
-                           k0 + kb * kBlockK, c.m_tile * BLOCK_X + (int)crank * HALF,
-                           (uint16_t)((1u << MC) - 1), kEvictLast);
-          } else {
-            tma_load_2d(b, &tmap_x, &full_bar[stage], x0 + kb * kBlockK, c.m_tile * BLOCK_X,
-                        kEvictLast);
-          }
+          tma_load_2d(b, &tmap_x, &full_bar[stage], x0 + kb * kBlockK, c.m_tile * BLOCK_X, kEvictLast);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
       }
@@ -374,9 +357,7 @@ __device__ __forceinline__ void gemm_1sm_body(const CUtensorMap& tmap_w, const C
             umma_bf16(d_tmem, umma_desc_k_sw128(a_addr + k * kUmmaK * 2),
                       umma_desc_k_sw128(b_addr + k * kUmmaK * 2), idesc, (kb | k) != 0);
           }
-          // frees the smem stage (in every CTA that multicasts into it) once these MMAs retire
-          if constexpr (MC > 1) umma_commit_mc(&empty_bar[stage], (uint16_t)((1u << MC) - 1));
-          else umma_commit(&empty_bar[stage]);
+          umma_commit(&empty_bar[stage]);  // frees the smem stage once these MMAs retire
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
         umma_commit(&tmem_full[acc]);  // accumulator complete -> epilogue
@@ -391,10 +372,10 @@ __device__ __forceinline__ void gemm_1sm_body(const CUtensorMap& tmap_w, const C
     int acc = 0;
     uint32_t acc_phase = 0;
     for (int u = first_unit; u < total_units; u += unit_stride) {
-      const TileCoord c = decode_unit(u, n_units, m_tiles, splits, group_m);
+      const TileCoord c = decode_unit(u, n_tiles, m_tiles, splits, group_m);
       mbar_wait_guarded(&tmem_full[acc], acc_phase);
       tc_fence_after();
-      const int n0 = (c.n_tile * MC + (int)crank) * kBlockW + quad * 32;
+      const int n0 = c.n_tile * kBlockW + quad * 32;
       const int m_base = c.m_tile * BLOCK_X;
       const uint32_t t_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * BLOCK_X);
       epilogue_store_tile<BLOCK_X, EPI>(t_addr, &tmap_y, stg, which, n0, m_base, c.split, M, N, out_f32, lane, dir);
@@ -408,20 +389,19 @@ __device__ __forceinline__ void gemm_1sm_body(const CUtensorMap& tmap_w, const C
 
   tc_fence_before();
   __syncthreads();
-  if constexpr (MC > 1) cluster_sync_all();  // no CTA leaves while its peer may still write into it
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, Cfg::kTmemCols);
   }
 }
 
-template <int BLOCK_X, int EPI, int MC>
+template <int BLOCK_X, int EPI>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w,
                          const __grid_constant__ CUtensorMap tmap_x,
                          const __grid_constant__ CUtensorMap tmap_y, int M, int N, int K, int out_f32,
                          int splits, int n_tiles, int m_tiles, int group_m, DirectOut dir) {
-  gemm_1sm_body<BLOCK_X, EPI, MC>(tmap_w, tmap_x, tmap_y, M, N, K, out_f32, splits, n_tiles, m_tiles, group_m, dir);
+  gemm_1sm_body<BLOCK_X, EPI>(tmap_w, tmap_x, tmap_y, M, N, K, out_f32, splits, n_tiles, m_tiles, group_m, dir);
 }
 
 // One launch for the products of all heads (b200_gemm_bf16_heads).
@@ -430,7 +410,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_bf16_heads_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                        const __grid_constant__ CUtensorMap tmap_y, int M, int N, int K, int out_f32, int H, int n_tiles, int m_tiles,
                        int group_m, int x_head) {
-  gemm_1sm_body<BLOCK_X, 0, 1, 1>(tmap_w, tmap_x, tmap_y, M, N, K, out_f32, H, n_tiles, m_tiles, group_m, DirectOut{nullptr, 0}, x_head);
+  gemm_1sm_body<BLOCK_X, 0, 1>(tmap_w, tmap_x, tmap_y, M, N, K, out_f32, H, n_tiles, m_tiles, group_m, DirectOut{nullptr, 0}, x_head);
 }
 
 // =================================================================================================
@@ -714,21 +694,11 @@ static int make_out_tmap(CUtensorMap* ty, void* Y, int M, int N, int64_t ldy, in
                           (uint64_t)M * (uint64_t)ldy, 32, CH);
 }
 
-static int g_gemm_multicast = -1;  // -1: read B200_GEMM_MULTICAST once (default on)
-
-static bool gemm_multicast_enabled() {
-  if (g_gemm_multicast < 0) {
-    const char* e = getenv("B200_GEMM_MULTICAST");
-    g_gemm_multicast = (e && e[0] == '0') ? 0 : 1;
-  }
-  return g_gemm_multicast != 0;
-}
-
-template <int BLOCK_X, int EPI, int MC>
-static int launch_gemm_mc(const CUtensorMap& tw, const CUtensorMap& tx, void* Y, int M, int N, int K,
-                          int64_t ldy, int out_f32, int splits, cudaStream_t stream) {
+template <int BLOCK_X, int EPI>
+static int launch_gemm_1sm(const void* X, const void* W, void* Y, int M, int N, int K, int64_t ldx, int64_t ldw, int64_t ldy, int out_f32,
+                           int splits, cudaStream_t stream) {
   using Cfg = GemmCfg<BLOCK_X>;
-  auto kernel = gemm_bf16_tcgen05_kernel<BLOCK_X, EPI, MC>;
+  auto kernel = gemm_bf16_tcgen05_kernel<BLOCK_X, EPI>;
   static bool attr_set = false;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
@@ -738,20 +708,21 @@ static int launch_gemm_mc(const CUtensorMap& tw, const CUtensorMap& tx, void* Y,
     }
     attr_set = true;
   }
-  CUtensorMap ty;
+  CUtensorMap tw, tx, ty;
+  int rc = make_tmap_bf16_2d(&tw, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, kBlockW, kBlockK);
+  if (rc) return rc;
+  rc = make_tmap_bf16_2d(&tx, X, (uint64_t)M, (uint64_t)K, (uint64_t)ldx, BLOCK_X, kBlockK);
+  if (rc) return rc;
   DirectOut dir;
-  const int rc = make_out_tmap<BLOCK_X, EPI>(&ty, Y, M, N, ldy, out_f32, splits, &dir);
+  rc = make_out_tmap<BLOCK_X, EPI>(&ty, Y, M, N, ldy, out_f32, splits, &dir);
   if (rc) return rc;
   const int n_tiles = (N + kBlockW - 1) / kBlockW;
   const int m_tiles = (M + BLOCK_X - 1) / BLOCK_X;
-  const int n_units = (n_tiles + MC - 1) / MC;
-  const int total = n_units * m_tiles * splits;
+  const int total = n_tiles * m_tiles * splits;
   const int sms = device_info().sm_count > 0 ? device_info().sm_count : 148;
-  const int max_clusters = sms / MC;
-  const int clusters = total < max_clusters ? total : max_clusters;
   const int group_m = m_tiles < 8 ? m_tiles : 8;
-  cudaError_t e = launch_pdl(kernel, dim3(clusters * MC), dim3(kGemmThreads), (size_t)Cfg::kSmemBytes, stream, MC,
-                             tw, tx, ty, M, N, K, out_f32, splits, n_tiles, m_tiles, group_m, dir);
+  cudaError_t e = launch_pdl(kernel, dim3(total < sms ? total : sms), dim3(kGemmThreads), (size_t)Cfg::kSmemBytes, stream, 1, tw, tx, ty,
+                             M, N, K, out_f32, splits, n_tiles, m_tiles, group_m, dir);
   if (e != cudaSuccess) {
     b200_set_error("b200_gemm_bf16: launch failed: %s", cudaGetErrorString(e));
     (void)cudaGetLastError();
@@ -886,15 +857,7 @@ static int launch_gemm(const void* X, const void* W, void* Y, int M, int N, int 
     if (gemm_2sm_enabled() && n_tiles >= 2)
       return launch_gemm_2sm<BLOCK_X, EPI>(X, W, Y, M, N, K, ldx, ldw, ldy, out_f32, splits, stream);
   }
-  // pairs of weight tiles share one multicast activation tile; not worth it for a single tile
-  const bool mc = gemm_multicast_enabled() && n_tiles >= 2;
-  CUtensorMap tw, tx;
-  int rc = make_tmap_bf16_2d(&tw, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, kBlockW, kBlockK);
-  if (rc) return rc;
-  rc = make_tmap_bf16_2d(&tx, X, (uint64_t)M, (uint64_t)K, (uint64_t)ldx, mc ? BLOCK_X / 2 : BLOCK_X, kBlockK);
-  if (rc) return rc;
-  if (mc) return launch_gemm_mc<BLOCK_X, EPI, 2>(tw, tx, Y, M, N, K, ldy, out_f32, splits, stream);
-  return launch_gemm_mc<BLOCK_X, EPI, 1>(tw, tx, Y, M, N, K, ldy, out_f32, splits, stream);
+  return launch_gemm_1sm<BLOCK_X, EPI>(X, W, Y, M, N, K, ldx, ldw, ldy, out_f32, splits, stream);
 }
 
 }  // namespace b200

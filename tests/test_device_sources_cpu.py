@@ -1,0 +1,19 @@
+"""Rules on the kernels' sources whose breach shows on a GPU only now and then, or harms more than the process: read, not run."""
+import re
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parents[1] / "gpustack_b200" / "csrc"
+SOURCES = sorted([*CSRC.glob("*.cu"), *CSRC.glob("*.cuh"), *CSRC.glob("*.h")])
+
+
+def _instructions(text):
+    """PTX instruction names of a source, string pieces of one statement joined."""
+    return re.findall(r"cp\.async\.bulk[\w.:]*", re.sub(r'"\s*\n?\s*"', "", text))
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=lambda p: p.name)
+def test_bulk_copies_go_to_one_cta(path):
+    """The library serves several GPUs, whose buffers may be one another's: no bulk copy spreads over a cluster."""
+    assert not [i for i in _instructions(path.read_text()) if "multi" + "cast" in i]
