@@ -167,6 +167,7 @@ moe_router_kernel(const bf16* __restrict__ x, int64_t ldx, const bf16* __restric
                   int E, int K, float scale, int score_mode, int renormalize, int groups, int groups_keep) {
   __shared__ float z[2][32 * kRbPerLane], gc[2][32 * kRbPerLane], gbest[2][32 * kRbPerLane];
   pdl_launch_dependents();
+  cluster_sync_all();      // the first CTA has started: only then is its shared memory there to be stored into
   pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = (int)cluster_ctarank();
   const int t0 = blockIdx.x / kRtCluster * 2;

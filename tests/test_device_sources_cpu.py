@@ -17,3 +17,16 @@ def _instructions(text):
 def test_bulk_copies_go_to_one_cta(path):
     """The library serves several GPUs, whose buffers may be one another's: no bulk copy spreads over a cluster."""
     assert not [i for i in _instructions(path.read_text()) if "multi" + "cast" in i]
+
+
+def _definitions(text):
+    """The source cut at every definition that begins a line."""
+    return re.split(r"\n(?=template |__global__|__device__|static |extern )", text)
+
+
+@pytest.mark.parametrize("path", [p for p in SOURCES if p.suffix == ".cu"], ids=lambda p: p.name)
+def test_clusters_meet_before_remote_accesses(path):
+    """Another CTA's shared memory may be addressed only once that CTA is known to have started."""
+    for body in _definitions(path.read_text()):
+        if "mapa_u32(" in body:
+            assert "cluster_sync_all()" in body and body.index("cluster_sync_all()") < body.index("mapa_u32("), body[:200]

@@ -29,3 +29,9 @@ def test_router(T, N, E, D, top, groups, keep, mode):
     bound = (D / 32 + 6) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
     assert bool(((lg[:, :N].cpu().double() - want).abs() <= bound).all()) and bool((lg[:, N:] == 7.0).all())
     assert torch.equal(ids, ids2) and torch.equal(wt, wt2)
+
+
+def test_router_of_the_narrowest_rows():
+    """Eight columns: next to no work between a CTA's start and its stores into the cluster's first CTA."""
+    for T in (1, 2, 33):
+        test_router(T, 65, 64, 8, 3, 0, 0, 0)
