@@ -171,7 +171,7 @@ __device__ __forceinline__ void epilogue_store_tile(uint32_t t_addr, const CUten
     float xs_lane = 0.f;
     if constexpr (FP8) {
       const int m = m_base + c0 + lane;   // lane j holds the scale of column j of this chunk
-      xs_lane = (lane < CH && m < M) ? xs[m] : 0.f;
+      xs_lane = (lane < CH && m < M) ? __ldcg(xs + m) : 0.f;
     }
     // the store that read this buffer two chunks ago must have drained it before it is refilled
     if (lane == 0) bulk_wait_read<1>();
@@ -506,7 +506,7 @@ __device__ __forceinline__ void gemm_2sm_body(const CUtensorMap& tmap_w, const C
   pdl_wait();
 
   if constexpr (GROUPED == 1) {
-    const int used = *grp.num_m_tiles;   // written by the align kernel this grid depends on
+    const int used = __ldcg(grp.num_m_tiles);   // written by the align kernel this grid depends on
     m_tiles = used < m_tiles ? used : m_tiles;
   }
   const int kb_per_split = GROUPED == 2 ? K / kElemsK : (K / kElemsK) / splits;
@@ -531,7 +531,7 @@ __device__ __forceinline__ void gemm_2sm_body(const CUtensorMap& tmap_w, const C
         const TileCoord c = decode_unit(u, n_units, m_tiles, splits, group_m);
         const int n_tile = c.n_tile * 2 + (int)crank;
         int w_row = n_tile * kBlockW;
-        if constexpr (GROUPED == 1) w_row += grp.tile_expert[c.m_tile] * N;
+        if constexpr (GROUPED == 1) w_row += __ldcg(grp.tile_expert + c.m_tile) * N;
         if constexpr (GROUPED == 2) w_row += c.split * N;
         const int k0 = GROUPED == 2 ? 0 : c.split * kb_per_split * kElemsK;
         const int x0 = GROUPED == 2 ? c.split * grp.x_head : k0;

@@ -8,7 +8,8 @@
 // results of a token are summed back.  All bookkeeping stays on the device (no host sync), so the
 // whole layer is CUDA-graph capturable: tile counts are read by the GEMM from device memory.
 //
-// These kernels are index / byte movers: HBM- or latency-bound, no tensor cores.
+// These kernels are index / byte movers: HBM- or latency-bound, no tensor cores.  All are programmatic dependents: what the kernels
+// before wrote is read past L1 (a grid that became resident early has missed its invalidation).
 #include "common.cuh"
 #include "runtime.h"
 #include "../../include/b200.h"
@@ -30,7 +31,7 @@ moe_route_kernel(const bf16* __restrict__ logits, int64_t ld, int32_t* __restric
   float p[kMaxExperts];
   float mx = -INFINITY;
   for (int e = 0; e < E; ++e) {
-    p[e] = __bfloat162float(logits[(size_t)t * ld + e]);
+    p[e] = __bfloat162float(__ldcg(logits + (size_t)t * ld + e));
     mx = fmaxf(mx, p[e]);
   }
   float sum = 0.f;
@@ -78,7 +79,7 @@ moe_align_kernel(const int32_t* __restrict__ topk_ids, const float* __restrict__
   __shared__ int cursor[kMaxExperts];
   for (int e = threadIdx.x; e < E; e += blockDim.x) { count[e] = 0; cursor[e] = 0; }
   __syncthreads();
-  for (int i = threadIdx.x; i < n_pairs; i += blockDim.x) atomicAdd(&count[topk_ids[i]], 1);
+  for (int i = threadIdx.x; i < n_pairs; i += blockDim.x) atomicAdd(&count[__ldcg(topk_ids + i)], 1);
   __syncthreads();
   if (threadIdx.x == 0) {
     int r = 0, tile = 0;
@@ -102,11 +103,11 @@ moe_align_kernel(const int32_t* __restrict__ topk_ids, const float* __restrict__
   // rows inside an expert are assigned in pair order WITHIN a warp-stride pass only up to atomics:
   // the order does not matter, every output row depends on its own input row alone.
   for (int i = threadIdx.x; i < n_pairs; i += blockDim.x) {
-    const int e = topk_ids[i];
+    const int e = __ldcg(topk_ids + i);
     const int r = row0[e] + atomicAdd(&cursor[e], 1);
     pair_row[i] = r;
     row_pair[r] = i;
-    row_weight[r] = topk_w[i];
+    row_weight[r] = __ldcg(topk_w + i);
   }
   (void)used;
 }
@@ -119,19 +120,19 @@ moe_gather_kernel(const bf16* __restrict__ x, const int32_t* __restrict__ row_pa
                   const float* __restrict__ row_scale) {
   pdl_launch_dependents();
   pdl_wait();
-  const int rows = min(num_tiles[1], capacity_rows);
+  const int rows = min(__ldcg(num_tiles + 1), capacity_rows);
   const int vec_per_row = H >> 3;
   const size_t total = (size_t)rows * vec_per_row;
   for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
        idx += (size_t)gridDim.x * blockDim.x) {
     const size_t r = idx / vec_per_row;
     const int vi = (int)(idx % vec_per_row);
-    const int pair = row_pair[r];
+    const int pair = __ldcg(row_pair + r);
     uint4 v = make_uint4(0, 0, 0, 0);
     if (pair >= 0) {
-      v = ld_v4(x + (size_t)(pair / K) * H + (size_t)vi * 8);
+      v = ld_cg_v4(x + (size_t)(pair / K) * H + (size_t)vi * 8);
       if (row_scale != nullptr) {    // an expert that runs on weight * x: the row is scaled in fp32 and rounded once
-        const float w = row_scale[r];
+        const float w = __ldcg(row_scale + r);
         v.x = pack_bf16(bf16_lo(v.x) * w, bf16_hi(v.x) * w);
         v.y = pack_bf16(bf16_lo(v.y) * w, bf16_hi(v.y) * w);
         v.z = pack_bf16(bf16_lo(v.z) * w, bf16_hi(v.z) * w);
@@ -157,8 +158,8 @@ moe_combine_kernel(const bf16* __restrict__ yp, const int32_t* __restrict__ pair
     const int vi = (int)(idx % vec_per_row);
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     for (int j = 0; j < K; ++j) {
-      const int r = pair_row[t * K + j];
-      const uint4 a = ld_v4(yp + (size_t)r * H + (size_t)vi * 8);
+      const int r = __ldcg(pair_row + t * K + j);
+      const uint4 a = ld_cg_v4(yp + (size_t)r * H + (size_t)vi * 8);
       acc[0] += bf16_lo(a.x); acc[1] += bf16_hi(a.x);
       acc[2] += bf16_lo(a.y); acc[3] += bf16_hi(a.y);
       acc[4] += bf16_lo(a.z); acc[5] += bf16_hi(a.z);

@@ -30,3 +30,15 @@ def test_clusters_meet_before_remote_accesses(path):
     for body in _definitions(path.read_text()):
         if "mapa_u32(" in body:
             assert "cluster_sync_all()" in body and body.index("cluster_sync_all()") < body.index("mapa_u32("), body[:200]
+
+
+@pytest.mark.parametrize("name", ["moe.cu", "moe_biased.cu"])
+def test_routing_reads_earlier_outputs_past_l1(name):
+    """A grid that became resident early has missed the launch-time L1 invalidation: what the kernels before it wrote (all of the
+    routing kernels' inputs but the weights) is not read by plain loads."""
+    kernels = [d for d in _definitions((CSRC / name).read_text()) if "pdl_wait();" in d]
+    assert kernels
+    for body in kernels:
+        head, code = body.split("pdl_wait();", 1)
+        for arg in set(re.findall(r"const (?:\w+)\s*\*\s*(?:__restrict__\s+)?(\w+)", head)) - {"correction", "router"}:
+            assert not re.search(r"(?<![\w.])%s\[|[ (!]\*%s\b|(?<!_cg_)(?<!rb_)ld_v4\(%s\b" % (arg, arg, arg), code), (arg, body[:120])
