@@ -62,6 +62,7 @@ struct ChunkScanArgs {
   const int32_t* ctx_lens;
   const int32_t* state_slots;
   int n_seqs;
+  int short_rows;                  // sequences of at most so many rows are the one-pass kernel's (cs_short)
   float* S;                        // [slots][H][dv][dk]
   float* o;                        // [T][H dv]
   float* ws;                       // [chunks][H][dk][dv]
@@ -70,7 +71,10 @@ struct ChunkScanArgs {
   float* ws_sums;                  // [chunks][H][2][64][dk]: kVector, the running sums' two parts
 };
 
-__host__ __device__ __forceinline__ int cs_chunks(int rows) { return rows > kCsShort ? (rows + kCsRows - 1) / kCsRows : 0; }
+__host__ __device__ __forceinline__ int cs_chunks(int rows, int short_rows) { return rows > short_rows ? (rows + kCsRows - 1) / kCsRows : 0; }
+
+// A step of one sequence needs no one-pass launch beside the chunks: whatever the sequence's rows of a longer buffer, they are chunks.
+inline int cs_short(int64_t rows, int n_seqs) { return n_seqs > 1 || rows <= kCsShort ? kCsShort : 0; }
 
 // Chunks that the sequences of a step can have at most: the launch's grid and the workspace are sized by this.
 inline int64_t cs_max_chunks(int64_t rows, int64_t n_seqs) {
@@ -82,14 +86,14 @@ inline int64_t cs_workspace_floats(int64_t rows, int64_t n_seqs, int64_t H, int6
 }
 
 // Sequence and place in it of chunk b (whole warp; seq -1: no such chunk), or with b < 0 the chunks before sequence `upto`.
-__device__ __forceinline__ void cs_find(const int32_t* cu, int n_seqs, int b, int upto, int& seq, int& local, int& before) {
+__device__ __forceinline__ void cs_find(const int32_t* cu, int n_seqs, int short_rows, int b, int upto, int& seq, int& local, int& before) {
   const int lane = threadIdx.x & 31;
   seq = -1;
   local = 0;
   before = 0;
   for (int base = 0; base < n_seqs; base += 32) {
     const int s = base + lane;
-    const int c = s < n_seqs ? cs_chunks(cu[s + 1] - cu[s]) : 0;
+    const int c = s < n_seqs ? cs_chunks(cu[s + 1] - cu[s], short_rows) : 0;
     int incl = c;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -119,7 +123,7 @@ struct ChunkPlace {
 __device__ __forceinline__ ChunkPlace cs_place(const ChunkScanArgs& a, int* shared5) {
   if (threadIdx.x < 32) {
     int seq, local, before;
-    cs_find(a.cu_seq, a.n_seqs, (int)blockIdx.x, 0, seq, local, before);
+    cs_find(a.cu_seq, a.n_seqs, a.short_rows, (int)blockIdx.x, 0, seq, local, before);
     if (threadIdx.x == 0) {
       shared5[0] = seq;
       if (seq >= 0) {
@@ -323,11 +327,11 @@ chunk_carry_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   __shared__ float tile[128][kCsCarryKeys + 1];
   __shared__ int base;
   const int s = blockIdx.z, h = blockIdx.y, tid = threadIdx.x;
-  const int t0 = a.cu_seq[s], t1 = a.cu_seq[s + 1], nc = cs_chunks(t1 - t0), slot = a.state_slots[s];
+  const int t0 = a.cu_seq[s], t1 = a.cu_seq[s + 1], nc = cs_chunks(t1 - t0, a.short_rows), slot = a.state_slots[s];
   if (nc == 0 || slot < 0) return;
   if (tid < 32) {
     int q, l, before;
-    cs_find(a.cu_seq, a.n_seqs, -1, s, q, l, before);
+    cs_find(a.cu_seq, a.n_seqs, a.short_rows, -1, s, q, l, before);
     if (tid == 0) base = before;
   }
   const int k0 = (blockIdx.x % (DK / kCsCarryKeys)) * kCsCarryKeys, v0 = (blockIdx.x / (DK / kCsCarryKeys)) * 128;

@@ -354,11 +354,12 @@ extern "C" int b200_gla_scan_chunked(const float* x, int64_t ld, int q_col, int 
   B200_REQUIRE(workspace_floats >= cs_workspace_floats(rows, n_seqs, H, dk, dv, true), "gla_scan: workspace of %lld floats too small",
                (long long)workspace_floats);
   cudaStream_t s = (cudaStream_t)stream;
-  if (n_seqs > 1 || rows <= kCsShort) {
+  const int short_rows = cs_short(rows, n_seqs);
+  if (short_rows > 0) {
     const int rc = launch_rows(x, ld, q_col, k_col, v_col, z, ldz, inv_tau, cu_seq, ctx_lens, state_slots, S, o_raw, n_seqs, H, dk, dv,
-                               kCsShort, s);
+                               short_rows, s);
     if (rc != B200_OK) return rc;
   }
-  const ChunkScanArgs a{x, ld, q_col, k_col, v_col, H, H, dv, cu_seq, ctx_lens, state_slots, n_seqs, S, o_raw};
+  const ChunkScanArgs a{x, ld, q_col, k_col, v_col, H, H, dv, cu_seq, ctx_lens, state_slots, n_seqs, short_rows, S, o_raw};
   return cs_launch<float, GatedLinearForm>(a, {z, ldz, inv_tau}, dk, rows, workspace, s);
 }

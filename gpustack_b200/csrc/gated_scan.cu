@@ -673,13 +673,14 @@ extern "C" int b200_gated_scan_chunked(const float* x, int64_t ld, int q_col, in
   B200_REQUIRE(workspace_floats >= cs_workspace_floats(rows, n_seqs, H, dk, dv), "gated_scan: workspace of %lld floats too small",
                (long long)workspace_floats);
   cudaStream_t s = (cudaStream_t)stream;
-  if (n_seqs > 1 || rows <= kCsShort) {
+  const int short_rows = cs_short(rows, n_seqs);
+  if (short_rows > 0) {
     const GatedScanArgs one{x, ld, q_col, k_col, v_col, gates, ld_g, rate, dt_bias, skip, cu_seq, ctx_lens, state_slots, S, o_raw, H, G,
-                            dk, dv, dv, kCsShort};
-    const int rc = gated_scan_pick<false>(one, n_seqs, kCsShort, s);
+                            dk, dv, dv, short_rows};
+    const int rc = gated_scan_pick<false>(one, n_seqs, short_rows, s);
     if (rc != B200_OK) return rc;
   }
-  const ChunkScanArgs a{x, ld, q_col, k_col, v_col, H, G, dv, cu_seq, ctx_lens, state_slots, n_seqs, S, o_raw};
+  const ChunkScanArgs a{x, ld, q_col, k_col, v_col, H, G, dv, cu_seq, ctx_lens, state_slots, n_seqs, short_rows, S, o_raw};
   return cs_launch<float, StateSpaceForm>(a, {gates, ld_g, rate, dt_bias, skip}, dk, rows, workspace, s);
 }
 

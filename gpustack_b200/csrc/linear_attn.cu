@@ -517,12 +517,13 @@ extern "C" int b200_linattn_scan_chunked(const float* x, int64_t ld, int q_col, 
   B200_REQUIRE(workspace_floats >= cs_workspace_floats(rows, n_seqs, H, dk, dv), "linattn_scan: workspace of %lld floats too small",
                (long long)workspace_floats);
   cudaStream_t s = (cudaStream_t)stream;
-  if (n_seqs > 1 || rows <= kCsShort) {
+  const int short_rows = cs_short(rows, n_seqs);
+  if (short_rows > 0) {
     const int rc = launch_chunk4(x, ld, q_col, k_col, v_col, decay, cu_seq, ctx_lens, state_slots, S, o_raw, n_seqs, H, dk, dv,
-                                 kCsShort, s);
+                                 short_rows, s);
     if (rc != B200_OK) return rc;
   }
-  const ChunkScanArgs a{x, ld, q_col, k_col, v_col, H, H, dv, cu_seq, ctx_lens, state_slots, n_seqs, S, o_raw};
+  const ChunkScanArgs a{x, ld, q_col, k_col, v_col, H, H, dv, cu_seq, ctx_lens, state_slots, n_seqs, short_rows, S, o_raw};
   return cs_launch<float, LinearForm>(a, {decay}, dk, rows, workspace, s);
 }
 

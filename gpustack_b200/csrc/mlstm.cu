@@ -905,12 +905,13 @@ static int launch_chunks(const void* proj, int64_t ld, int q_col, int k_col, int
                          const int32_t* cu_seq, const int32_t* ctx_lens, const int32_t* state_slots, float* S_state, float* n_state,
                          float* m_state, float* o_raw, int n_seq, int H, int dk, int dv, float cap, float qscale, int rows,
                          float* workspace, cudaStream_t s) {
-  if (n_seq > 1 || rows <= kCsShort) {
+  const int short_rows = cs_short(rows, n_seq);
+  if (short_rows > 0) {
     const int rc = launch_chunk<TA>(proj, ld, q_col, k_col, v_col, gates, gate_bias, cu_seq, ctx_lens, state_slots, S_state, n_state,
-                                    m_state, o_raw, n_seq, H, dk, dv, cap, qscale, s, kCsShort);
+                                    m_state, o_raw, n_seq, H, dk, dv, cap, qscale, s, short_rows);
     if (rc != B200_OK) return rc;
   }
-  const ChunkScanArgs a{proj, ld, q_col, k_col, v_col, H, H, dv, cu_seq, ctx_lens, state_slots, n_seq, S_state, o_raw};
+  const ChunkScanArgs a{proj, ld, q_col, k_col, v_col, H, H, dv, cu_seq, ctx_lens, state_slots, n_seq, short_rows, S_state, o_raw};
   return cs_launch<TA, MlstmForm>(a, {gates, (const bf16*)gate_bias, cap, qscale, n_state, m_state, b200_mlstm_state_slices(dv)}, dk, rows,
                                   workspace, s);
 }

@@ -161,3 +161,48 @@ def test_no_row_reaches_an_earlier_one_and_negative_slots_are_skipped():
     ops.linattn_scan(xx, 0, dk, 2 * dk, torch.tensor([0.9]).cuda(), _i32([0, T, T + 100]), _i32([0, 5]), _i32([1, -1]), S, o, H, dk, dv, max_len=T)
     assert bool(torch.isfinite(o[:70]).all()) and bool(torch.isnan(o[70:T]).all())
     assert bool((o[T:] == 7.0).all()) and bool((S[0] == 3.0).all())
+
+
+def _scans(x, gates, z, cu, ctx, slots, H, dk, dv, max_len, n_seq=None):
+    """Every recurrence over the same rows; state slots start alike.  -> {name: (outputs, *states)}"""
+    from gpustack_b200 import ops
+
+    T, n, Z = x.shape[0], n_seq or len(slots), ops.mlstm_state_slices(dv)
+    cols, idx, out = (0, H * dk, 2 * H * dk), (_i32(cu), _i32(ctx), _i32(slots)), {}
+    g = torch.Generator().manual_seed(11)
+    S0, n0, m0 = torch.randn(n, H, dv, dk, generator=g), torch.randn(n, H, 1, dk, generator=g), torch.rand(n, H, 1, generator=g)
+    vec = lambda lo: torch.linspace(lo, lo + 0.3, H).cuda()   # noqa: E731
+    bias = torch.linspace(-1, 3, 2 * H).to(torch.bfloat16).cuda()
+    for name in ("linear", "mlstm", "gated_linear", "state_space"):
+        o, S = torch.full((T, H * dv), 7.0, device="cuda"), S0.cuda()
+        more = ()
+        if name == "linear":
+            ops.linattn_scan(x, *cols, vec(0.6), *idx, S, o, H, dk, dv, max_len=max_len)
+        elif name == "mlstm":
+            more = (n0.expand(n, H, Z, dk).contiguous().cuda(), m0.expand(n, H, Z).contiguous().cuda())
+            ops.mlstm_scan(x, *cols, gates, bias, *idx, S, *more, o, H, dk, dv, 6.0, max_len=max_len)
+        elif name == "gated_linear":
+            ops.gla_scan(x, *cols, z, 1.0 / 16, *idx, S, o, H, dk, dv, max_len=max_len)
+        else:
+            ops.gated_scan(x, *cols, gates[:, :H].contiguous(), vec(0.3), vec(-2.0), vec(0.5), *idx, S, o, H, H, dk, dv, False, max_len=max_len)
+        out[name] = (o, S) + more
+    return out
+
+
+def _rows(T, H, dk, dv, seed):
+    g = torch.Generator().manual_seed(seed)
+    return tuple(torch.randn(T, w, generator=g).cuda() for w in (2 * H * dk + H * dv, 2 * H, H * dk))
+
+
+@pytest.mark.parametrize("n", [1, 10, 16, 17, 70])
+def test_one_sequence_in_a_longer_buffer(n):
+    """The buffer's rows say nothing about the sequence's: a short one beside nothing is not left out."""
+    H, dk, dv, T = 2, 64, 64, 600
+    x, gates, z = _rows(T, H, dk, dv, n)
+    long = _scans(x, gates, z, [0, n], [5], [0], H, dk, dv, T)
+    alone = _scans(x[:n].contiguous(), gates[:n].contiguous(), z[:n].contiguous(), [0, n], [5], [0], H, dk, dv, n)
+    for name, got in long.items():
+        assert bool((got[0][n:] == 7.0).all())
+        assert _rel(got[0][:n], alone[name][0].cpu().to(F64)) < (20 if name == "mlstm" else 1) * TOL, name
+        for a, b in zip(got[1:], alone[name][1:]):
+            assert _rel(a, b.cpu().to(F64)) < TOL, name
