@@ -756,7 +756,7 @@ struct MlstmForm {
       m = m_new;
     }
     for (int z = 0; z < p.Z; ++z) n_out[z * DK + k] = n;
-    if (k < p.Z) p.m_state[((size_t)slot * a.H + h) * p.Z + k] = m;
+    for (int z = k; z < p.Z; z += DK) p.m_state[((size_t)slot * a.H + h) * p.Z + z] = m;
   }
   static __device__ __forceinline__ void output_weights(const Params& p, const ChunkScanArgs& a, Scratch& sc, int h, const ChunkPlace& at) {
     if (threadIdx.x < 32) {

@@ -206,3 +206,12 @@ def test_one_sequence_in_a_longer_buffer(n):
         assert _rel(got[0][:n], alone[name][0].cpu().to(F64)) < (20 if name == "mlstm" else 1) * TOL, name
         for a, b in zip(got[1:], alone[name][1:]):
             assert _rel(a, b.cpu().to(F64)) < TOL, name
+
+
+def test_mlstm_stabilisers_of_more_value_slices_than_keys():
+    """Every slice's copy of the stabiliser is written, also where there are more slices (value columns / 32) than key columns."""
+    H, dk, dv, T = 1, 64, 2084, 130
+    x, gates, z = _rows(T, H, dk, dv, 3)
+    for n in (T, 90):
+        m = _scans(x, gates, z, [0, n], [5], [0], H, dk, dv, T)["mlstm"][3]
+        assert bool((m == m[..., :1]).all())
