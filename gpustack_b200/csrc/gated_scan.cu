@@ -450,8 +450,9 @@ struct StateSpaceForm {
       const double v = __shfl_up_sync(0xffffffffu, sum, o);
       if (lane >= o) sum += v;
     }
+    const double before = __shfl_up_sync(0xffffffffu, sum, 1);
     F[1] = sum;
-    F[0] = sum - f[1];
+    F[0] = lane ? before + f[0] : f[0];               // (not sum - f[1]: what is no number in a row stays out of the one before)
   }
   static __device__ __forceinline__ void state_weights(const Params& p, const ChunkScanArgs&, Scratch& sc, int h, const ChunkPlace& at) {
     if (threadIdx.x < 32) {

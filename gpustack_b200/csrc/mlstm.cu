@@ -663,8 +663,9 @@ struct MlstmForm {
       const double v = __shfl_up_sync(0xffffffffu, sum, o);
       if (lane >= o) sum += v;
     }
+    const double before = __shfl_up_sync(0xffffffffu, sum, 1);
     F[1] = sum;
-    F[0] = sum - f[1];
+    F[0] = lane ? before + f[0] : f[0];               // (not sum - f[1]: what is no number in a row stays out of the one before)
     constexpr double kNone = -1.0e300;
     const double g0 = 2 * lane < at.rows ? (double)ii[0] - F[0] : kNone, g1 = 2 * lane + 1 < at.rows ? (double)ii[1] - F[1] : kNone;
     double mx = fmax(g0, g1);

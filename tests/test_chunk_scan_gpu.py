@@ -215,3 +215,20 @@ def test_mlstm_stabilisers_of_more_value_slices_than_keys():
     for n in (T, 90):
         m = _scans(x, gates, z, [0, n], [5], [0], H, dk, dv, T)["mlstm"][3]
         assert bool((m == m[..., :1]).all())
+
+
+@pytest.mark.parametrize("row", [70, 71])
+def test_what_is_no_number_reaches_no_earlier_row(row):
+    """A gate (or, without gates, a key) that is no number and an infinite value behind it: rows before stay as they are."""
+    H, dk, dv, T = 2, 64, 64, 400
+    x, gates, z = _rows(T, H, dk, dv, 7)
+    clean = _scans(x, gates, z, [0, T], [5], [0], H, dk, dv, 4096)
+    gates[row], z[row] = float("nan"), float("nan")
+    x[row + 60, 2 * H * dk:] = float("inf")
+    xk = x.clone()
+    xk[row, H * dk:2 * H * dk] = float("nan")
+    got = _scans(x, gates, z, [0, T], [5], [0], H, dk, dv, 4096)
+    got["linear"] = _scans(xk, gates, z, [0, T], [5], [0], H, dk, dv, 4096)["linear"]
+    for name, out in got.items():
+        assert torch.equal(out[0][:row], clean[name][0][:row]), name
+        assert bool(torch.isnan(out[0][row:]).all()) and bool(torch.isnan(out[1]).all()), name
