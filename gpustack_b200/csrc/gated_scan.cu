@@ -413,7 +413,8 @@ int gated_scan_pick(const GatedScanArgs& a, int n_seqs, int max_len, cudaStream_
   return gated_scan_form<32, 4, 32, 4, DELTA>(a, n_seqs, max_len, s);
 }
 
-// The state-space recurrence in the chunk form: log decays of a chunk's rows summed in fp64, every exponent <= 0.
+// The state-space recurrence in the chunk form: log decays of a chunk's rows summed in fp64, every exponent <= 0.  A decay of
+// less than e^-10000 is zero all the same and is cut there, so that sums and their differences stay finite.
 //   ws_row[dk] of a chunk: its whole decay
 struct StateSpaceForm {
   static constexpr const char* kName = "b200_gated_scan(chunks)";
@@ -441,7 +442,8 @@ struct StateSpaceForm {
       beta[e] = 0.f;
       if (t < at.rows) {
         beta[e] = gs_softplus(p.gates[(size_t)(at.first + t) * p.ld_g + h] + bias);
-        f[e] = (double)(-rate * beta[e]);
+        const float lg = -rate * beta[e];
+        f[e] = lg < -1.0e4f ? -1.0e4 : (double)lg;
       }
     }
     double sum = f[0] + f[1];

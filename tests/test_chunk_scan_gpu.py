@@ -232,3 +232,26 @@ def test_what_is_no_number_reaches_no_earlier_row(row):
     for name, out in got.items():
         assert torch.equal(out[0][:row], clean[name][0][:row]), name
         assert bool(torch.isnan(out[0][row:]).all()) and bool(torch.isnan(out[1]).all()), name
+
+
+def test_a_state_space_row_that_clears_the_state():
+    """A step whose rate times size overflows fp32 clears the state; what comes behind it knows only what came behind it."""
+    from gpustack_b200 import ops
+
+    dk, dv, T = 64, 64, 300
+    g = torch.Generator().manual_seed(9)
+    x, gates, S = torch.randn(T, 2 * dk + dv, generator=g), torch.randn(T, 1, generator=g) * 0.5 - 87.0, torch.randn(1, 1, dv, dk, generator=g)
+    gates[100] = 50.0
+    rate, dt = torch.tensor([1.0e38]), torch.zeros(1)
+    o, S_d = torch.zeros(T, dv, device="cuda"), S.cuda()
+    ops.gated_scan(x.cuda(), 0, dk, 2 * dk, gates.cuda(), rate.cuda(), dt.cuda(), None, _i32([0, T]), _i32([9]), _i32([0]), S_d, o, 1, 1, dk, dv,
+                   False, max_len=4096)
+    step, Z, want = torch.nn.functional.softplus(gates.to(F64))[:, 0], S[0, 0].to(F64), torch.zeros(T, dv, dtype=F64)
+    x = x.to(F64)
+    for t in range(T):
+        Z = torch.exp(-1.0e38 * step[t]) * Z + step[t] * x[t, 2 * dk:, None] * x[t, None, dk:2 * dk]
+        want[t] = Z @ x[t, :dk]
+    # the steps are formed from numbers of 2^-126, whose rounding is 2^-22 of them, and scaled by the rate in the exponent
+    for a, b in ((0, 100), (100, 104)):
+        assert _rel(o[a:b], want[a:b]) < TOL
+    assert bool(torch.isfinite(o).all()) and bool(torch.isfinite(S_d).all())
