@@ -6,6 +6,7 @@ eager/PyTorch fallback -- a missing library or a non-CUDA tensor raises.
 """
 from __future__ import annotations
 
+import collections
 import ctypes as C
 from typing import Optional, Sequence
 
@@ -623,21 +624,42 @@ def mlstm_state_slices(dv: int) -> int:
 
 CHUNK_SCAN_MAX_BYTES = 1 << 30
 
+# What the two forms of a recurrence cost, fitted to 148 measured steps each (4 to 32 heads, 1 to 201 sequences, 32 to 2048 rows, single
+# rows beside portions, L2 cold): the one-pass form takes fixed + max(row x longest portion, work x rows x heads), a serial chain or,
+# with CTAs enough, its throughput; the chunk form fixed + work x (rows + wasted x sequences) x heads.  us; work per 1000 rows and
+# heads of `width` = key x value columns; a sequence's first row, which is all of a single one, counts on neither side.  The form
+# taken is at most 11 % slower than the other in any of them.  One-pass -> chunks, 8 heads: linear attention of 64 rows 35 -> 40, of 128
+# 57 -> 42, of 2048 762 -> 71, 16 portions of 32 rows 55 -> 75, of 64 rows 92 -> 81; mLSTM of 128 rows 56 -> 54, of 2048 732 -> 87, 16 of 64
+# rows 114 -> 126, of 128 rows 201 -> 132; gated linear attention of 256 rows 47 -> 50, of 512 84 -> 52, 16 of 128 rows 70 -> 83, of
+# 1024 rows 433 -> 390, one of 2048 beside thirty of 16 449 -> 108; state space of 32 heads: 1024 rows 109 -> 87, 2048 rows
+# 207 -> 140, 16 of 512 rows 399 -> 532, one of 2048 beside thirty of 16 477 -> 195.
+ChunkCosts = collections.namedtuple("ChunkCosts", "width one_fixed one_row one_work chunk_fixed chunk_work wasted")
+CHUNK_COSTS = {"linear": ChunkCosts(128 * 128, 10.0, 0.37, 6.8, 36.0, 3.0, 0), "mlstm": ChunkCosts(128 * 128, 10.0, 0.36, 8.5, 60.0, 2.6, 32),
+               "gated_linear": ChunkCosts(64 * 128, 8.0, 0.146, 2.0, 44.0, 1.8, 0),
+               "state_space": ChunkCosts(128 * 64, 8.0, 0.097, 1.15, 32.0, 1.2, 0)}
 
-def _chunk_scan_workspace(rows: int, n_seqs: int, H: int, dk: int, dv: int, max_len: int, device, per_channel: bool = False,
-                          short: bool = False):
+
+def chunk_scan_pays(kind: str, rows: int, n_seqs: int, H: int, dk: int, dv: int, max_len: int) -> bool:
+    """Whether a step of `rows` rows in n_seqs sequences of at most max_len runs faster over chunks of 64 rows side by side.  A bound
+    of all rows of several sequences says nothing about one of them: they are taken for equal."""
+    if dk not in (64, 128) or dv % 4:
+        return False
+    c = CHUNK_COSTS[kind]
+    longest = -(-rows // n_seqs) if max_len == rows and n_seqs > 1 else max_len
+    if longest <= 32:                                   # half a chunk at most: one-pass is the better at every size measured
+        return False
+    heads = H * dk * dv / c.width / 1000.0
+    one = c.one_fixed + max(c.one_row * longest, c.one_work * (rows - n_seqs) * heads)
+    return c.chunk_fixed + c.chunk_work * (rows - n_seqs + c.wasted * min(n_seqs, rows // 17)) * heads < one
+
+
+def _chunk_scan_workspace(kind: str, rows: int, n_seqs: int, H: int, dk: int, dv: int, max_len: int, device):
     """Workspace of the scans that run a prompt portion's chunks of 64 rows side by side, or None where the one-pass scans are
-    the better ones: key widths the chunk kernels do not take, and steps of short portions (three launches instead of one).
-    All rows beyond max_len are taken for single ones.  Measured, 8 heads, L2 cold, one-pass -> chunks, linear attention of 128 x
-    128: one portion of 64 rows 33 -> 32 us, 128 rows 57 -> 38, 512 rows 197 -> 42, 2048 rows 758 -> 69; 4 of 64 rows 33 -> 38; 16
-    of 32 rows 54 -> 54, of 64 rows 92 -> 60, of 512 rows 621 -> 206; mLSTM alike.  short: scans whose one-pass form takes 0.15 us a
-    row (gated linear attention of 64 x 128: one portion of 128 rows 27 -> 48, 512 rows 83 -> 50, 2048 rows 303 -> 73; 16 of 128
-    rows 66 -> 77, of 512 rows 221 -> 212) start at 256 rows, and at 512 when there are more than one portion's."""
-    least = 128 if not short else 256 if rows < 2 * max_len else 512
-    if dk not in (64, 128) or dv % 4 or max_len < least or max_len < 96 * (n_seqs - max(0, rows - max_len)):
+    the better ones, or the only ones (key widths the chunk kernels do not take)."""
+    if not chunk_scan_pays(kind, rows, n_seqs, H, dk, dv, max_len):
         return None
-    n = (rows // 64 + min(n_seqs, rows // 17)) * H * (dk * dv + dk + 4 + (128 * dk if per_channel else 0))
-    return torch.empty(n, dtype=torch.float32, device=device) if 4 * n <= CHUNK_SCAN_MAX_BYTES else None
+    n = (rows // 64 + min(n_seqs, rows // 17)) * H * (dk * dv + dk + 4 + (128 * dk if kind == "gated_linear" else 0))
+    return torch.empty(n, dtype=torch.float32, device=device) if 0 < 4 * n <= CHUNK_SCAN_MAX_BYTES else None
 
 
 def mlstm_scan(proj, q_col, k_col, v_col, gates, gate_bias, cu_seq, ctx_lens, state_slots, S, n, m, o_raw, H, dk, dv,
@@ -647,7 +669,7 @@ def mlstm_scan(proj, q_col, k_col, v_col, gates, gate_bias, cu_seq, ctx_lens, st
     _cuda(proj, gates, gate_bias, cu_seq, ctx_lens, state_slots, S, n, m, o_raw)
     _req(gates, torch.float32, "gates"); _req(S, torch.float32, "S"); _req(o_raw, torch.float32, "o_raw")
     n_seq = state_slots.shape[0]
-    ws = _chunk_scan_workspace(proj.shape[0], n_seq, H, dk, dv, max_len, proj.device)
+    ws = _chunk_scan_workspace("mlstm", proj.shape[0], n_seq, H, dk, dv, max_len, proj.device)
     if ws is not None:
         check(load().b200_mlstm_scan_chunked(_p(proj), _is_f32(proj), proj.stride(0), q_col, k_col, v_col, _p(gates), _p(gate_bias),
                                              _p(cu_seq), _p(ctx_lens), _p(state_slots), _p(S), _p(n), _p(m), _p(o_raw), n_seq, H, dk, dv,
@@ -710,7 +732,7 @@ def linattn_scan(x, q_col: int, k_col: int, v_col: int, decay, cu_seq, ctx_lens,
     _req(x, torch.float32, "x"); _req(S, torch.float32, "S"); _req(o_raw, torch.float32, "o_raw")
     _req(decay, torch.float32, "decay")
     n = state_slots.shape[0]
-    ws = _chunk_scan_workspace(x.shape[0], n, H, dk, dv, max_len, x.device)
+    ws = _chunk_scan_workspace("linear", x.shape[0], n, H, dk, dv, max_len, x.device)
     if ws is not None:
         check(load().b200_linattn_scan_chunked(_p(x), x.stride(0), q_col, k_col, v_col, _p(decay), _p(cu_seq), _p(ctx_lens),
                                                _p(state_slots), _p(S), _p(o_raw), n, H, dk, dv, int(max_len), x.shape[0], _p(ws),
@@ -822,7 +844,7 @@ def gla_scan(x, q_col: int, k_col: int, v_col: int, z, inv_tau: float, cu_seq, c
     _cuda(x, z, cu_seq, ctx_lens, state_slots, S, o_raw)
     _req(x, torch.float32, "x"); _req(z, torch.float32, "z"); _req(S, torch.float32, "S"); _req(o_raw, torch.float32, "o_raw")
     n = state_slots.shape[0]
-    ws = _chunk_scan_workspace(x.shape[0], n, H, dk, dv, max_len, x.device, per_channel=True, short=True)
+    ws = _chunk_scan_workspace("gated_linear", x.shape[0], n, H, dk, dv, max_len, x.device)
     if ws is not None:
         check(load().b200_gla_scan_chunked(_p(x), x.stride(0), q_col, k_col, v_col, _p(z), z.stride(0), inv_tau, _p(cu_seq),
                                            _p(ctx_lens), _p(state_slots), _p(S), _p(o_raw), n, H, dk, dv, int(max_len), x.shape[0],
@@ -948,7 +970,7 @@ def gated_scan(x, q_col: int, k_col: int, v_col: int, gates, rate, dt_bias, skip
     if tuple(S.shape[1:]) != (H, dv, -(-dk // 4) * 4) or not S.is_contiguous() or not o_raw.is_contiguous():
         raise B200Error("gated_scan: a contiguous state of [slots, heads, dv, dk rounded up to 4]")
     n = state_slots.shape[0]
-    ws = None if delta else _chunk_scan_workspace(x.shape[0], n, H, dk, dv, max_len, x.device, short=True)
+    ws = None if delta else _chunk_scan_workspace("state_space", x.shape[0], n, H, dk, dv, max_len, x.device)
     if ws is not None:
         check(load().b200_gated_scan_chunked(_p(x), x.stride(0), q_col, k_col, v_col, _p(gates), gates.stride(0), _p(rate), _p(dt_bias),
                                              _p(skip), _p(cu_seq), _p(ctx_lens), _p(state_slots), _p(S), _p(o_raw), n, H, G, dk, dv, 0,

@@ -149,6 +149,7 @@ class ModelRunner:
         self.stage_host = torch.zeros(self.stage_words, dtype=torch.int32, pin_memory=True)
         self.stage_np = self.stage_host.numpy()
         self.stage_dev = torch.zeros(self.stage_words, dtype=torch.int32, device=dev)
+        self.longest_portion = 0                          # rows of the prompt step's longest portion
         self.out_host = torch.zeros(self.max_sample, dtype=torch.int32, pin_memory=True)
         self.logits_host = torch.empty(1 << 20, dtype=torch.float32, pin_memory=True)
         # fixed decode layout inside the staging area
@@ -605,6 +606,7 @@ class ModelRunner:
         o_cu = 3 * _align(T)
         o_ctx = o_cu + _align(S + 1)
         o_rows = o_ctx + _align(S)
+        self.longest_portion = max(lens, default=0)
         tile_seq, tile_q0 = ops.build_prefill_tiles(lens, self.prefill_tile, starts)
         nt = len(tile_seq)
         o_ts = o_rows + _align(NS)

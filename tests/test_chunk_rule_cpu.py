@@ -1,0 +1,46 @@
+"""The choice between a recurrence's one-pass and chunk forms, at steps whose times are known on both sides."""
+import pytest
+
+from gpustack_b200 import ops
+
+WIDTHS = {"linear": (128, 128), "mlstm": (128, 128), "gated_linear": (64, 128), "state_space": (128, 64)}
+
+
+# kind, heads, portions (rows), one-pass us, chunk us (L2 cold)
+@pytest.mark.parametrize("kind,H,lens,one,chunk", [
+    ("linear", 8, [64], 34.8, 40.0), ("linear", 8, [128], 57.3, 42.0), ("linear", 32, [2048], 761.9, 205.7),
+    ("linear", 8, [32] * 16, 55.3, 74.8), ("linear", 8, [64] * 16, 92.2, 80.9), ("linear", 8, [2048] + [16] * 30, 1252.4, 126.0),
+    ("linear", 8, [128] * 4 + [1] * 100, 198.7, 178.8), ("mlstm", 8, [64] * 16, 113.5, 126.0), ("mlstm", 8, [128] * 16, 200.7, 131.9),
+    ("mlstm", 16, [512] * 4 + [1] * 100, 845.8, 617.5), ("mlstm", 8, [2048] + [1] * 64, 840.5, 230.4),
+    ("gated_linear", 8, [256], 47.1, 50.2), ("gated_linear", 8, [512], 84.0, 52.2), ("gated_linear", 8, [128] * 16, 69.6, 82.9),
+    ("gated_linear", 8, [128] * 4 + [1] * 100, 96.2, 134.2), ("gated_linear", 8, [2048] + [16] * 30, 448.5, 107.5),
+    ("gated_linear", 16, [512] * 4, 118.8, 130.0), ("state_space", 32, [1024], 108.5, 87.0), ("state_space", 32, [512] * 4, 120.8, 148.5),
+    ("state_space", 32, [512] * 16, 399.4, 531.5), ("state_space", 32, [2048] + [16] * 30, 477.2, 195.3)], ids=str)
+def test_the_faster_form_is_chosen(kind, H, lens, one, chunk):
+    dk, dv = WIDTHS[kind]
+    pays = lambda longest: ops.chunk_scan_pays(kind, sum(lens), len(lens), H, dk, dv, longest)   # noqa: E731
+    assert pays(max(lens)) == (chunk < one)
+    if len(set(lens)) == 1:
+        assert pays(sum(lens)) == (chunk < one)                # all rows as the bound: portions are taken for equal
+
+
+@pytest.mark.parametrize("kind", sorted(WIDTHS))
+def test_single_rows_and_other_widths_stay_one_pass(kind):
+    dk, dv = WIDTHS[kind]
+    for n in (1, 7, 256, 4096):
+        assert not ops.chunk_scan_pays(kind, n, n, 128, dk, dv, 1)
+    assert ops.chunk_scan_pays(kind, 4096, 2, 8, dk, dv, 2048)
+    for a, b in ((96, dv), (dk, dv + 2), (256, dv)):
+        assert not ops.chunk_scan_pays(kind, 4096, 2, 8, a, b, 2048)
+
+
+def test_the_runner_states_the_longest_portion():
+    """A prompt step hands its scans the longest portion, not the sum of the portions."""
+    from pathlib import Path
+
+    root = Path(ops.__file__).parent
+    assert "self.longest_portion = max(lens" in (root / "runner.py").read_text()
+    text = (root / "layer_list_runner.py").read_text()
+    for scan in ("linattn_scan", "mlstm_scan", "gla_scan"):
+        call = text[text.index("ops." + scan):]
+        assert "max_len=self.longest_portion" in call[:call.index("ops.", 4)]
