@@ -445,6 +445,27 @@ def _up4(n: int) -> int:
     return -(-n // 4) * 4
 
 
+CHUNK_SCAN_MAX_BYTES = 1 << 30       # recurrences whose chunks would need more run one-pass
+
+
+def chunk_scan_floats(rows: int, n_seqs: int, heads: int, dk: int, dv: int, per_channel: bool = False) -> int:
+    """Workspace of a recurrence over chunks of 64 rows side by side (b200_chunk_scan_floats): every chunk's state and row of
+    factors, with a decay per key channel also its running sums."""
+    return (rows // 64 + min(n_seqs, rows // 17)) * heads * (dk * dv + dk + 4 + (128 * dk if per_channel else 0))
+
+
+def chunk_scan_workspace_floats(layers, rows: int, n_seqs: int) -> int:
+    """Workspace of steps of up to `rows` rows in up to n_seqs sequences for the layers' recurrences that have a chunk form."""
+    shapes = set()
+    for m in (l.mixer for l in layers):
+        if m.kind in ("mlstm", "linear_attention", "gated_linear_attention"):
+            shapes.add((m.heads, m.dim, m.vdim, m.kind == "gated_linear_attention"))
+        elif m.kind == "side_by_side" and m.right.kind == "state_space":
+            shapes.add((m.right.heads, m.right.state, m.right.vdim, False))
+    need = [chunk_scan_floats(rows, n_seqs, *s) for s in shapes if s[1] in (64, 128) and s[2] % 4 == 0]
+    return min(max(need, default=0), CHUNK_SCAN_MAX_BYTES // 4)
+
+
 @dataclass
 class SideBySideSpec:
     """Two mixers that read the same input; the mixer's output is left_scale * left + right_scale * right, with branch_norm

@@ -503,7 +503,7 @@ extern "C" int b200_linattn_scan(const float* x, int64_t ld, int q_col, int k_co
   return b200_check_launch("b200_linattn_scan");
 }
 
-// The same with a workspace of b200_chunk_scan_floats(rows, n_seqs, H, dk, dv) floats: sequences of more than 16 rows run with
+// The same with a workspace of b200_chunk_scan_floats(rows, n_seqs, H, dk, dv, 0) floats: sequences of more than 16 rows run with
 // all their chunks side by side, the others one-pass beside them.  Shapes and alignments that the chunk kernels do not take
 // run as b200_linattn_scan.
 extern "C" int b200_linattn_scan_chunked(const float* x, int64_t ld, int q_col, int k_col, int v_col, const float* decay,

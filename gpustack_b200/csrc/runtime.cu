@@ -1,5 +1,6 @@
 // Runtime glue of libb200.so: error reporting, device queries, TMA descriptor creation and
-// CUDA IPC handles.  No kernels here.
+// CUDA IPC handles, workspace sizes.  No kernels here.
+#include "chunk_scan.cuh"
 #include "common.cuh"
 #include "runtime.h"
 #include "../../include/b200.h"
@@ -269,3 +270,7 @@ int b200_ipc_close_handle(void* dev_ptr) {
 }
 
 }  // extern "C"
+
+extern "C" int64_t b200_chunk_scan_floats(int64_t rows, int64_t n_seqs, int H, int dk, int dv, int per_channel) {
+  return b200::cs_workspace_floats(rows, n_seqs, H, dk, dv, per_channel != 0);
+}

@@ -86,6 +86,7 @@ from typing import List, Optional
 import torch
 
 from . import ops
+from .config import chunk_scan_workspace_floats
 from .lib import B200Error
 from .runner import BF16, ModelRunner
 from .weights import pad_head_columns
@@ -199,6 +200,8 @@ class LayerListRunner(ModelRunner):
         gdr = [l.mixer.right.width for l in self.mcfg.layers
                if l.mixer.kind == "side_by_side" and l.mixer.right.kind == "gated_recurrence"]
         self.rec_ws = ops.gated_recurrence_workspace(T, self.max_seqs, max(gdr), dev) if gdr else None
+        n = chunk_scan_workspace_floats(self.mcfg.layers, T, self.max_seqs)
+        self.chunk_ws = e(n, dt=torch.float32) if n else None     # the recurrences' chunks, shared by all layers
         if self.sandwich or self.pre_norm:
             self.y2 = e(T, D, dt=torch.float32)           # the second output of a side-by-side mixer
         if self.sandwich:
@@ -510,7 +513,7 @@ class LayerListRunner(ModelRunner):
                 ops.linear(proj[:, ac:ac + m.decay_rank], lw.decay_up, z, bias=lw.decay_bias)
                 o_raw = self._view(self.o_raw, T, H * dv)
                 ops.gla_scan(x32, 0, kc, vc, z, 1.0 / m.tau, cu_all, ctx_all, slots_all, self.state[l][0], o_raw, H, dk, dv,
-                             max_len=self.longest_portion if Tp else 1)
+                             max_len=self.longest_portion if Tp else 1, workspace=self.chunk_ws)
                 ops.linattn_out(o_raw, proj, gc, lw.out_norm, out, H, dv, eps, False, "silu")
                 self.stats["kernel_launches"] += 5
             elif m.kind == "latent_attention":
@@ -551,7 +554,7 @@ class LayerListRunner(ModelRunner):
                              half_layout=m.rot is not None and m.rot.layout == "half", freq=lw.rot_freq, k_mul=m.k_scale)
                 o_raw = self._view(self.o_raw, T, H * dv)
                 ops.linattn_scan(x32, 0, kc, vc, lw.decay, cu_all, ctx_all, slots_all, self.state[l][0], o_raw, H, dk, dv,
-                                 max_len=self.longest_portion if Tp else 1)
+                                 max_len=self.longest_portion if Tp else 1, workspace=self.chunk_ws)
                 ops.linattn_out(o_raw, proj, vc + H * dv, lw.out_norm, out, H, dv, eps, m.out_norm == "all_heads", m.gate_act)
                 self.stats["kernel_launches"] += 4
             else:
@@ -561,7 +564,7 @@ class LayerListRunner(ModelRunner):
                 o_raw = self._view(self.o_raw, T, H * dv)
                 S, n, mm = self.state[l]
                 ops.mlstm_scan(proj, 0, H * dk, 2 * H * dk, gates, lw.gate_bias, cu_all, ctx_all, slots_all, S, n, mm,
-                               o_raw, H, dk, dv, m.gate_cap, max_len=self.longest_portion if Tp else 1)
+                               o_raw, H, dk, dv, m.gate_cap, max_len=self.longest_portion if Tp else 1, workspace=self.chunk_ws)
                 ops.mlstm_out(o_raw, proj, 2 * H * dk + H * dv, lw.out_norm, out, H, dv, eps)
                 self.stats["kernel_launches"] += 4
             ops.linear(out, wo if m.kind == "attention" else lw.o, self.y[:T])
@@ -665,7 +668,7 @@ class LayerListRunner(ModelRunner):
                           ((r.heads, r.vdim, None), (r.groups, r.state, None), (r.groups, r.state, None)), x32)
         b_col = r.row_width - 2 * r.groups * S.shape[3]
         ops.gated_scan(x32, b_col + r.groups * S.shape[3], b_col, 0, gates, lw.decay_rate, lw.dt_bias, lw.skip, cu_all, ctx_all,
-                       slots_all, S, o_raw, r.heads, r.groups, r.state, r.vdim, False, max_len=self.longest_portion if Tp else 1)
+                       slots_all, S, o_raw, r.heads, r.groups, r.state, r.vdim, False, max_len=self.longest_portion if Tp else 1, workspace=self.chunk_ws)
         ops.gate_norm(o_raw, proj, z_col, lw.out_norm, right, r.norm_groups, self.mcfg.norm_eps)
         ops.linear(right, lw.o2, self.y2[:T])
         self._pending = {"pair": (self.y[:T], self.y2[:T], lw.left_norm, lw.right_norm, m.left_scale, m.right_scale)}

@@ -95,6 +95,7 @@ SIGNATURES = {
     "b200_mlstm_state_slices": (_i32, [_i32]),
     "b200_mlstm_scan": (_i32, [_vp, _i32, _i64, _i32, _i32, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32,
                                _i32, _i32, _f32, _f32, _i32, _vp]),
+    "b200_chunk_scan_floats": (_i64, [_i64, _i64, _i32, _i32, _i32, _i32]),
     "b200_mlstm_scan_chunked": (_i32, [_vp, _i32, _i64, _i32, _i32, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32,
                                        _i32, _i32, _f32, _f32, _i32, _i32, _vp, _i64, _vp]),
     "b200_streams_step": (_i32, [_vp, _i32, _i64, _vp, _vp, _vp, _f32, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp]),

@@ -12,6 +12,7 @@ from typing import Optional, Sequence
 
 import torch
 
+from .config import CHUNK_SCAN_MAX_BYTES, chunk_scan_floats
 from .lib import B200Error, check, load
 
 BLOCK_SIZE = 16  # tokens per KV page (vLLM default block_size)
@@ -622,8 +623,6 @@ def mlstm_state_slices(dv: int) -> int:
     return (dv + 31) // 32
 
 
-CHUNK_SCAN_MAX_BYTES = 1 << 30
-
 # What the two forms of a recurrence cost, fitted to 148 measured steps each (4 to 32 heads, 1 to 201 sequences, 32 to 2048 rows, single
 # rows beside portions, L2 cold): the one-pass form takes fixed + max(row x longest portion, work x rows x heads), a serial chain or,
 # with CTAs enough, its throughput; the chunk form fixed + work x (rows + wasted x sequences) x heads.  us; work per 1000 rows and
@@ -653,23 +652,28 @@ def chunk_scan_pays(kind: str, rows: int, n_seqs: int, H: int, dk: int, dv: int,
     return c.chunk_fixed + c.chunk_work * (rows - n_seqs + c.wasted * min(n_seqs, rows // 17)) * heads < one
 
 
-def _chunk_scan_workspace(kind: str, rows: int, n_seqs: int, H: int, dk: int, dv: int, max_len: int, device):
-    """Workspace of the scans that run a prompt portion's chunks of 64 rows side by side, or None where the one-pass scans are
-    the better ones, or the only ones (key widths the chunk kernels do not take)."""
+def _chunk_scan_workspace(kind: str, rows: int, n_seqs: int, H: int, dk: int, dv: int, max_len: int, device, workspace=None):
+    """Workspace of the scans that run a prompt portion's chunks of 64 rows side by side (the caller's, where it brings one), or
+    None where the one-pass scans are the better ones, or the only ones (key widths the chunk kernels do not take, no room)."""
     if not chunk_scan_pays(kind, rows, n_seqs, H, dk, dv, max_len):
         return None
-    n = (rows // 64 + min(n_seqs, rows // 17)) * H * (dk * dv + dk + 4 + (128 * dk if kind == "gated_linear" else 0))
+    n = chunk_scan_floats(rows, n_seqs, H, dk, dv, kind == "gated_linear")
+    if workspace is not None:
+        _cuda(workspace)
+        _req(workspace, torch.float32, "workspace")
+        return workspace if workspace.numel() >= n else None
     return torch.empty(n, dtype=torch.float32, device=device) if 0 < 4 * n <= CHUNK_SCAN_MAX_BYTES else None
 
 
 def mlstm_scan(proj, q_col, k_col, v_col, gates, gate_bias, cu_seq, ctx_lens, state_slots, S, n, m, o_raw, H, dk, dv,
-               cap: float, max_len: int = 1):
+               cap: float, max_len: int = 1, workspace=None):
     """Runs every sequence's new rows through the matrix-memory recurrence (state slot in, state slot out).
-    max_len: an upper bound of the new rows per sequence (prompt portions run in the chunk form)."""
+    max_len: an upper bound of the new rows per sequence (prompt portions run in the chunk form).  workspace: room for the portions'
+    chunks that the caller keeps (config.chunk_scan_workspace_floats); without one it is allocated when it is used."""
     _cuda(proj, gates, gate_bias, cu_seq, ctx_lens, state_slots, S, n, m, o_raw)
     _req(gates, torch.float32, "gates"); _req(S, torch.float32, "S"); _req(o_raw, torch.float32, "o_raw")
     n_seq = state_slots.shape[0]
-    ws = _chunk_scan_workspace("mlstm", proj.shape[0], n_seq, H, dk, dv, max_len, proj.device)
+    ws = _chunk_scan_workspace("mlstm", proj.shape[0], n_seq, H, dk, dv, max_len, proj.device, workspace)
     if ws is not None:
         check(load().b200_mlstm_scan_chunked(_p(proj), _is_f32(proj), proj.stride(0), q_col, k_col, v_col, _p(gates), _p(gate_bias),
                                              _p(cu_seq), _p(ctx_lens), _p(state_slots), _p(S), _p(n), _p(m), _p(o_raw), n_seq, H, dk, dv,
@@ -725,14 +729,14 @@ def rot_prep(proj, q_col: int, k_col: int, v_col: int, positions, slots, q_out, 
 
 
 def linattn_scan(x, q_col: int, k_col: int, v_col: int, decay, cu_seq, ctx_lens, state_slots, S, o_raw, H, dk, dv,
-                 max_len: int = 1):
+                 max_len: int = 1, workspace=None):
     """Decayed linear attention over every sequence's new rows of the fp32 rows x (state slot in, state slot out).
-    max_len: an upper bound of the new rows per sequence (prompt portions run in the chunk form)."""
+    max_len: an upper bound of the new rows per sequence (prompt portions run in the chunk form).  workspace: as mlstm_scan's."""
     _cuda(x, decay, cu_seq, ctx_lens, state_slots, S, o_raw)
     _req(x, torch.float32, "x"); _req(S, torch.float32, "S"); _req(o_raw, torch.float32, "o_raw")
     _req(decay, torch.float32, "decay")
     n = state_slots.shape[0]
-    ws = _chunk_scan_workspace("linear", x.shape[0], n, H, dk, dv, max_len, x.device)
+    ws = _chunk_scan_workspace("linear", x.shape[0], n, H, dk, dv, max_len, x.device, workspace)
     if ws is not None:
         check(load().b200_linattn_scan_chunked(_p(x), x.stride(0), q_col, k_col, v_col, _p(decay), _p(cu_seq), _p(ctx_lens),
                                                _p(state_slots), _p(S), _p(o_raw), n, H, dk, dv, int(max_len), x.shape[0], _p(ws),
@@ -839,12 +843,13 @@ def gated_recurrence_scan(u, gates, gate_bias, lam, proj, y_col: int, y_bias, cu
 
 
 def gla_scan(x, q_col: int, k_col: int, v_col: int, z, inv_tau: float, cu_seq, ctx_lens, state_slots, S, o_raw, H, dk, dv,
-             max_len: int = 0):
-    """Linear attention with the decay sigmoid(z)^inv_tau per key channel and token (csrc/gated_linear_attn.cu)."""
+             max_len: int = 0, workspace=None):
+    """Linear attention with the decay sigmoid(z)^inv_tau per key channel and token (csrc/gated_linear_attn.cu).  max_len and
+    workspace: as mlstm_scan's."""
     _cuda(x, z, cu_seq, ctx_lens, state_slots, S, o_raw)
     _req(x, torch.float32, "x"); _req(z, torch.float32, "z"); _req(S, torch.float32, "S"); _req(o_raw, torch.float32, "o_raw")
     n = state_slots.shape[0]
-    ws = _chunk_scan_workspace("gated_linear", x.shape[0], n, H, dk, dv, max_len, x.device)
+    ws = _chunk_scan_workspace("gated_linear", x.shape[0], n, H, dk, dv, max_len, x.device, workspace)
     if ws is not None:
         check(load().b200_gla_scan_chunked(_p(x), x.stride(0), q_col, k_col, v_col, _p(z), z.stride(0), inv_tau, _p(cu_seq),
                                            _p(ctx_lens), _p(state_slots), _p(S), _p(o_raw), n, H, dk, dv, int(max_len), x.shape[0],
@@ -960,9 +965,10 @@ def conv_rec_prep(proj, conv_w, bias, ring, cu_seq, ctx_lens, state_slots, tile_
 
 
 def gated_scan(x, q_col: int, k_col: int, v_col: int, gates, rate, dt_bias, skip, cu_seq, ctx_lens, state_slots, S, o_raw, H, G, dk,
-               dv, delta: bool, max_len: int = 1):
+               dv, delta: bool, max_len: int = 1, workspace=None):
     """Delta rule (delta) or state-space recurrence over every sequence's new rows of the fp32 rows x (csrc/gated_scan.cu);
-    state S [slots, H, dv, dk rounded up to 4] in, state out.  max_len: an upper bound of the new rows per sequence."""
+    state S [slots, H, dv, dk rounded up to 4] in, state out.  max_len: an upper bound of the new rows per sequence;
+    workspace: as mlstm_scan's (the delta rule needs none)."""
     _cuda(x, gates, rate, dt_bias, skip, cu_seq, ctx_lens, state_slots, S, o_raw)
     for t_, n_ in ((x, "x"), (gates, "gates"), (rate, "rate"), (dt_bias, "dt_bias"), (S, "S"), (o_raw, "o_raw")):
         if t_.dtype != torch.float32:
@@ -970,7 +976,7 @@ def gated_scan(x, q_col: int, k_col: int, v_col: int, gates, rate, dt_bias, skip
     if tuple(S.shape[1:]) != (H, dv, -(-dk // 4) * 4) or not S.is_contiguous() or not o_raw.is_contiguous():
         raise B200Error("gated_scan: a contiguous state of [slots, heads, dv, dk rounded up to 4]")
     n = state_slots.shape[0]
-    ws = None if delta else _chunk_scan_workspace("state_space", x.shape[0], n, H, dk, dv, max_len, x.device)
+    ws = None if delta else _chunk_scan_workspace("state_space", x.shape[0], n, H, dk, dv, max_len, x.device, workspace)
     if ws is not None:
         check(load().b200_gated_scan_chunked(_p(x), x.stride(0), q_col, k_col, v_col, _p(gates), gates.stride(0), _p(rate), _p(dt_bias),
                                              _p(skip), _p(cu_seq), _p(ctx_lens), _p(state_slots), _p(S), _p(o_raw), n, H, G, dk, dv, 0,

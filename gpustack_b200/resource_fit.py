@@ -17,7 +17,7 @@ import math
 from dataclasses import asdict, dataclass
 from typing import Optional
 
-from .config import EngineConfig, ModelConfig
+from .config import EngineConfig, ModelConfig, chunk_scan_workspace_floats
 
 GiB = 1024 ** 3
 GRAPH_POOL_BYTES = 1 * GiB          # what ModelRunner.profile_num_blocks reserves for graphs / allocator slack
@@ -103,6 +103,7 @@ def _layer_list_workspace(m, e: EngineConfig) -> int:
     if m.residual == "sandwich":
         par = 8                                                                          # second output, normed input (fp32)
         routed += 8 * (T // 64 + S + 1) * max([x.mixer.right.width for x in m.layers if x.mixer.kind == "side_by_side"] or [0])
+    routed += 4 * chunk_scan_workspace_floats(m.layers, T, S)
     act = T * (D * (4 * getattr(m, "n_streams", 1) + a + 4 + par) + (proj + mix + ff + lat) * a + (gates + rec + lin) * 4) + routed
     max_len = e.max_model_len or m.max_position_embeddings
     staging = (3 * T + 10 * S + 3 * S_smp + S * math.ceil(max_len / e.block_size) + 2 * T) * 4

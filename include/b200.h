@@ -308,8 +308,11 @@ int b200_mlstm_scan(const void* proj, int f32, int64_t ld, int q_col, int k_col,
                     const int32_t* ctx_lens, const int32_t* state_slots, float* S_state, float* n_state,
                     float* m_state, float* o_raw, int n_seq, int H, int dk, int dv, float cap, float qscale,
                     int max_len, void* stream);
+/* Floats of the workspace of the recurrences' chunk forms for steps of up to `rows` rows in up to n_seqs sequences: (rows / 64 +
+ * min(n_seqs, rows / 17)) * H * (dk * dv + dk + 4), with a decay per key channel 128 * dk more per head. */
+int64_t b200_chunk_scan_floats(int64_t rows, int64_t n_seqs, int H, int dk, int dv, int per_channel);
 /* The same with a workspace: sequences of more than 16 rows run with all their chunks of 64 rows side by side.  rows: the rows
- * of proj; workspace: 16-byte aligned, (rows / 64 + min(n_seq, rows / 17)) * H * (dk * dv + dk + 4) floats.  Widths other than
+ * of proj, at least cu_seq[n_seq]; workspace: 16-byte aligned, b200_chunk_scan_floats(rows, n_seq, H, dk, dv, 0) floats.  Widths other than
  * dk 64 / 128 with dv % 4 == 0, unaligned rows or no workspace: as b200_mlstm_scan. */
 int b200_mlstm_scan_chunked(const void* proj, int f32, int64_t ld, int q_col, int k_col, int v_col, const float* gates,
                             const void* gate_bias, const int32_t* cu_seq, const int32_t* ctx_lens, const int32_t* state_slots,
@@ -410,7 +413,7 @@ int b200_linattn_scan(const float* x, int64_t ld, int q_col, int k_col, int v_co
                       const int32_t* cu_seq, const int32_t* ctx_lens, const int32_t* state_slots, float* S, float* o_raw,
                       int n_seqs, int H, int dk, int dv, int max_len, void* stream);
 /* The same with a workspace: sequences of more than 16 rows run with all their chunks of 64 rows side by side.  rows: the rows
- * of x; workspace: 16-byte aligned, (rows / 64 + min(n_seqs, rows / 17)) * H * (dk * dv + dk + 4) floats.  Widths other than
+ * of x; workspace: 16-byte aligned, b200_chunk_scan_floats(rows, n_seqs, H, dk, dv, 0) floats.  Widths other than
  * dk 64 / 128 with dv % 4 == 0, unaligned rows or no workspace: as b200_linattn_scan. */
 int b200_linattn_scan_chunked(const float* x, int64_t ld, int q_col, int k_col, int v_col, const float* decay,
                               const int32_t* cu_seq, const int32_t* ctx_lens, const int32_t* state_slots, float* S,
@@ -560,7 +563,7 @@ int b200_gla_scan_rows(const float* x, int64_t ld, int q_col, int k_col, int v_c
                   int n_seqs, int H, int dk, int dv, int max_len, void* stream);
 
 /* ... with a workspace: sequences of more than 16 rows run with all their chunks of 64 rows side by side.  rows: the rows of x;
- * workspace: 16-byte aligned, (rows / 64 + min(n_seqs, rows / 17)) * H * (dk * dv + 129 * dk + 4) floats.  Widths other than dk 64 /
+ * workspace: 16-byte aligned, b200_chunk_scan_floats(rows, n_seqs, H, dk, dv, 1) floats.  Widths other than dk 64 /
  * 128 with dv % 4 == 0, unaligned rows or no workspace: as b200_gla_scan_rows. */
 int b200_gla_scan_chunked(const float* x, int64_t ld, int q_col, int k_col, int v_col, const float* z, int64_t ldz, float inv_tau,
                           const int32_t* cu_seq, const int32_t* ctx_lens, const int32_t* state_slots, float* S, float* o_raw,
@@ -615,7 +618,7 @@ int b200_gated_scan(const float* x, int64_t ld, int q_col, int k_col, int v_col,
                     const int32_t* state_slots, float* S, float* o_raw, int n_seqs, int H, int G, int dk, int dv, int delta,
                     int max_len, void* stream);
 /* The state-space form with a workspace: sequences of more than 16 rows run with all their chunks of 64 rows side by side.  rows:
- * the rows of x; workspace: 16-byte aligned, (rows / 64 + min(n_seqs, rows / 17)) * H * (dk * dv + dk + 4) floats.  The delta
+ * the rows of x; workspace: 16-byte aligned, b200_chunk_scan_floats(rows, n_seqs, H, dk, dv, 0) floats.  The delta
  * rule, widths other than dk 64 / 128 with dv % 4 == 0, or no workspace: as b200_gated_scan. */
 int b200_gated_scan_chunked(const float* x, int64_t ld, int q_col, int k_col, int v_col, const float* gates, int64_t ld_g,
                             const float* rate, const float* dt_bias, const float* skip, const int32_t* cu_seq,

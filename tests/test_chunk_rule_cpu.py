@@ -1,7 +1,8 @@
 """The choice between a recurrence's one-pass and chunk forms, at steps whose times are known on both sides."""
 import pytest
 
-from gpustack_b200 import ops
+from gpustack_b200 import config, ops
+from gpustack_b200.lib import load
 
 WIDTHS = {"linear": (128, 128), "mlstm": (128, 128), "gated_linear": (64, 128), "state_space": (128, 64)}
 
@@ -44,3 +45,39 @@ def test_the_runner_states_the_longest_portion():
     for scan in ("linattn_scan", "mlstm_scan", "gla_scan"):
         call = text[text.index("ops." + scan):]
         assert "max_len=self.longest_portion" in call[:call.index("ops.", 4)]
+
+
+@pytest.mark.parametrize("rows,n", [(1, 1), (17, 3), (63, 1), (64, 64), (8192, 256), (100000, 5)])
+def test_the_workspace_has_one_size(rows, n):
+    for H, dk, dv, per_channel in ((1, 64, 36, False), (8, 64, 128, True), (32, 128, 64, False)):
+        assert config.chunk_scan_floats(rows, n, H, dk, dv, per_channel) == load().b200_chunk_scan_floats(rows, n, H, dk, dv, int(per_channel))
+
+
+def test_the_workspace_is_in_the_memory_estimate():
+    """The estimate of a model with such a recurrence counts what the runner allocates for the chunks."""
+    from gpustack_b200 import resource_fit
+    from gpustack_b200.config import EngineConfig, LinearAttentionSpec
+
+    class Layer:
+        mlp = None
+
+        def __init__(self, dim):
+            self.mixer = LinearAttentionSpec(heads=8, dim=dim, vdim=128, decay=(0.9,) * 8)
+
+    class Model:
+        family, hidden_size, vocab_size, residual, max_position_embeddings = "layer_list", 1024, 1000, "parallel", 4096
+        loop_times, n_streams = 1, 1
+
+        def __init__(self, dim):
+            self.layers = [Layer(dim)]
+
+        def state_bytes_per_seq(self):
+            return 0
+
+    e = EngineConfig(max_num_seqs=64, max_num_batched_tokens=8192)
+    with_chunks, without = (resource_fit._layer_list_workspace(Model(d), e) for d in (128, 96))
+    ws = 4 * config.chunk_scan_workspace_floats(Model(128).layers, 8192, 64)
+    assert ws == 4 * (128 + 64) * 8 * (128 * 128 + 132)
+    assert config.chunk_scan_workspace_floats(Model(96).layers, 8192, 64) == 0
+    assert with_chunks - without > ws
+    assert config.chunk_scan_workspace_floats(Model(128).layers, 10 ** 7, 256) * 4 == config.CHUNK_SCAN_MAX_BYTES
