@@ -255,3 +255,23 @@ def test_a_state_space_row_that_clears_the_state():
     for a, b in ((0, 100), (100, 104)):
         assert _rel(o[a:b], want[a:b]) < TOL
     assert bool(torch.isfinite(o).all()) and bool(torch.isfinite(S_d).all())
+
+
+# beyond the carry's eight chunks in flight, with its remainder and a second walk; more sequences than a warp looks up at once, long
+# ones before, between and behind single rows
+@pytest.mark.parametrize("lens", [[513], [577, 1100], [1] * 3 + [150] + [1] * 40 + [200, 17] + [1] * 20, [1] * 33 + [130]], ids=lambda v: str(len(v)))
+def test_long_portions_and_many_sequences(lens):
+    """The chunk form against the one-pass form, sequence by sequence (which the other tests hold against fp64)."""
+    H, dk, dv = 2, 64, 64
+    cu, ctx, slots = _layout(lens)
+    x, gates, z = _rows(cu[-1], H, dk, dv, len(lens))
+    got = _scans(x, gates, z, cu, ctx, slots, H, dk, dv, 4096)
+    for i, n in enumerate(lens):
+        a, b = cu[i], cu[i + 1]
+        want = _scans(x[a:b].contiguous(), gates[a:b].contiguous(), z[a:b].contiguous(), [0, n], [ctx[i]], [slots[i]], H, dk, dv, min(n, 30),
+                      n_seq=len(lens))
+        for name in got:
+            # both sides' sums are rounded, and an output's error is of the size of the sequence's outputs
+            assert _rel(got[name][0][a:b], want[name][0].cpu().to(F64)) < (40 if name == "mlstm" else 2) * TOL, (name, i)
+            for p, q in zip(got[name][1:], want[name][1:]):
+                assert _rel(p[slots[i]], q[slots[i]].cpu().to(F64)) < 2 * TOL, (name, i)

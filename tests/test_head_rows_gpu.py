@@ -54,3 +54,33 @@ def test_rotations_of_four_rows_per_cta(T, half):
         return x
 
     assert torch.equal(run(0, T), torch.cat([run(0, 2000), run(2000, 4000), run(4000, T)]))
+
+
+@pytest.mark.parametrize("src,dst", [(BF, BF), (torch.float32, torch.float32), (BF, torch.float32)])
+@pytest.mark.parametrize("half", [True, False])
+@pytest.mark.parametrize("T", [4737, 4739])
+def test_rotations_of_four_rows_per_cta_into_pages(T, half, src, dst):
+    """Every instance, paged, with a norm, factors, an unrotated rest, fewer key heads and rows that have no slot."""
+    from gpustack_b200 import ops
+
+    H, G, dk, dv, dims, page = 3, 2, 96, 64, 64, 16
+    kc, vc = H * dk, (H + G) * dk
+    g = torch.Generator().manual_seed(T + half)
+    proj = torch.randn(T, vc + G * dv, generator=g).to(src).cuda()
+    pos = torch.randint(0, 50000, (T,), generator=g, dtype=torch.int32).cuda()
+    slots = torch.randperm(T + 40, generator=g)[:T].to(torch.int32)
+    slots[::97] = -1
+    slots = slots.cuda()
+    freq = (10000.0 ** (-torch.arange(dims // 2, dtype=F64) / (dims // 2))).cuda()
+    mul = torch.rand(H, generator=g).cuda()
+
+    def run(cuts):
+        q = torch.full((T, H * dk), 7.0, dtype=dst, device="cuda")
+        k, v = (torch.full(((T + 40 + page - 1) // page, G, page, w), 7.0, dtype=dst, device="cuda") for w in (dk, dv))
+        for a, b in zip(cuts, cuts[1:]):
+            ops.rot_prep(proj[a:b], 0, kc, vc, pos[a:b], slots[a:b], q[a:b], k, v, H, G, dk, dv, paged=True, rot_dims=dims, half_layout=half,
+                         freq=freq, unit_norm=True, eps=1e-6, q_mul=0.5, k_mul=2.0, q_head_mul=mul)
+        return q, k, v
+
+    for a, b in zip(run([0, T]), run([0, 2000, 4000, T])):
+        assert torch.equal(a, b)
