@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 """bench.py -- the reference's headline metric on the hot path: output tok/s (+ p50 TTFT) of
 continuous-batched Llama-3-8B bf16 serving, 512-token prompts / 128 greedy output tokens
-(BASELINE.json configs[1]; TP = --gpus), random-init weights, synthetic token-id prompts.
+(TP = --gpus), random-init weights, synthetic token-id prompts.
 
   python bench.py --gpus 1 --steps K --warmup W                      (this engine)
   python -m torch.distributed.run --nnodes=1 --nproc-per-node N --master-addr 127.0.0.1 \
@@ -50,10 +50,10 @@ def parse_args():
     ap.add_argument("--output-len", type=int, default=128)
     ap.add_argument("--model", default="llama3-8b",
                     choices=["llama3-8b", "llama3-70b", "qwen2-0.5b", "tiny", "tiny128", "mixtral-8x7b", "tiny-mixtral"],
-                    help="llama3-8b is the BASELINE config; mixtral-8x7b is a side measurement of the MoE family")
+                    help="llama3-8b is the benchmark's model; mixtral-8x7b is a side measurement of the MoE family")
     ap.add_argument("--max-num-batched-tokens", type=int, default=8192, help="prefill token budget per engine step")
     ap.add_argument("--quantization", default=None, choices=[None, "fp8"],
-                    help="fp8 = W8A8 side measurement (NOT the BASELINE config, which is bf16)")
+                    help="fp8 = W8A8 side measurement (the benchmark itself is bf16)")
     ap.add_argument("--no-e2e", action="store_true", help="skip the HTTP end-to-end leg")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-parity-probe", action="store_true",
@@ -66,7 +66,7 @@ def parse_args():
     ap.add_argument("--cpu-sample-requests", type=int, default=2)
     ap.add_argument("--cpu-sample-output", type=int, default=16)
     ap.add_argument("--no-cpu-configs0", action="store_true",
-                    help="skip the BASELINE configs[0] CPU leg (Qwen2-0.5B shape, 32 requests on the host cores)")
+                    help="skip the CPU leg (Qwen2-0.5B shape, 32 requests on the host cores)")
     ap.add_argument("--family", default=None, choices=[None, "vodavik", "danipel", "resevik", "dotorax", "kerarax", "bovitar"],
                     help="side benchmark of another model family beside the closest Llama-class model of equal layer "
                          "sizes (prefill / decode tokens per second and per-kernel roofline fractions); prints its own "
@@ -243,7 +243,7 @@ PROBE_TOL = 2e-2   # relative to max|logit|: the engine-level tolerance of tests
 
 
 def parity_probe(a, rank, world):
-    """Correctness of the EXACT code path that is about to be timed, at BASELINE width: a 2-layer
+    """Correctness of the EXACT code path that is about to be timed, at the benchmark's width: a 2-layer
     Llama-3-8B-shaped model (H 4096, I 14336, 32/8 heads of 128, vocab 32768; the same tile shapes,
     split plans and -- under TP -- all-reduce paths as the benchmark model) generates 16 greedy
     tokens for 8 seeded prompts; the CPU oracle is teacher-forced on the engine's tokens and every
@@ -547,7 +547,7 @@ def run_ours(a):
     from gpustack_b200.engine import LLMEngine, TPWorker
     from gpustack_b200.scheduler import SamplingParams
 
-    # NCCL_DEBUG is left as the launcher set it (the communicator log is the driver's evidence of the
+    # NCCL_DEBUG is left as the launcher set it (the communicator log shows the
     # rank count); the JSON line is printed LAST, after the process group is gone.
     world = int(os.environ.get("WORLD_SIZE", "1"))
     rank = int(os.environ.get("RANK", "0"))
@@ -683,7 +683,7 @@ def run_ours(a):
                                "sample": f"{a.cpu_sample_requests} requests x {a.input_len} in / {a.cpu_sample_output} out, "
                                          f"sequential, {dt:.1f} s of CPU work (oracle/llama_oracle.py, fp32 math)"}
         if not a.no_cpu_configs0 and a.time_budget_s - (time.time() - _T0) > 420:
-            # BASELINE.json configs[0] (SURVEY section 8d): the reference's CPU-runnable case -- Qwen2-0.5B shape,
+            # the reference's CPU-runnable case -- Qwen2-0.5B shape,
             # the full 32 requests of the plumbing run, on this box's host cores, in this same run
             log("CPU baseline, configs[0]: Qwen2-0.5B shape x 32 requests ...")
             v0, t0_, dt0 = cpu_reference("qwen2-0.5b", 32, 64, 8)

@@ -1,5 +1,5 @@
-"""Reference-side binding for registering this engine as a FIRST-CLASS GPUStack backend (SURVEY.md
-section 8f-3) instead of a `-custom` backend: the file a GPUStack maintainer would add as
+"""Reference-side binding for registering this engine as a FIRST-CLASS GPUStack backend
+instead of a `-custom` backend: the file a GPUStack maintainer would add as
 `gpustack/worker/backends/b200_native.py`, plus the three one-line hooks listed at the bottom.
 
 It is written against the reference's own interfaces and imports them (gpustack.* and

@@ -4,7 +4,7 @@ request send to the FIRST SSE chunk (:74-81,120), usage read from the chunk that
 output tok/s = sum(completion_tokens) / total wall time and percentiles via numpy (:321-425).
 
 Differences, on purpose: token-id prompts through /v1/completions (token-exact lengths, seeded --
-the reference script's prompts are unseeded and tokenizer-dependent, SURVEY.md 8d) and raw aiohttp
+the reference script's prompts are unseeded and tokenizer-dependent) and raw aiohttp
 instead of the openai SDK (httpx_aiohttp is not installed offline).
 Run: python -m gpustack_b200.bench_client --url http://127.0.0.1:8000 --model m -n 256 -c 256 \
          --input-len 512 --output-len 128 --seed 0

@@ -203,11 +203,8 @@ def subset_lib(tag: str) -> Path:
     return CSRC / f"libb200_{tag}.so"
 
 
-def build(force: bool = False, verbose: bool = False, variant: str = "", sources=None, tag: str = "") -> Path:
-    """variant "" = the product library (dependents released after the kernel's own dependency wait);
-    "early" = libb200_early.so, the experimental build with the entry-time trigger
-    (-DB200_PDL_EARLY_TRIGGER), kept only to reproduce the hazard documented beside pdl_wait().
-    sources + tag: link only those files into libb200_<tag>.so (same ABI, fewer symbols) -- what a
+def build(force: bool = False, verbose: bool = False, sources=None, tag: str = "") -> Path:
+    """The product library, or with sources + tag: link only those files into libb200_<tag>.so (same ABI, fewer symbols) -- what a
     process that serves one model family needs on a fresh checkout.  Objects are cached per source
     file, so a later full build compiles only what is still missing."""
     names = list(SOURCES if sources is None else sources)
@@ -215,11 +212,10 @@ def build(force: bool = False, verbose: bool = False, variant: str = "", sources
     headers = sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.h")) + [CSRC.parent.parent / "include" / "b200.h"]
     if sources is not None and not tag:
         raise ValueError("a subset build needs a tag")
-    lib = (LIB if not tag else subset_lib(tag)) if not variant else CSRC / f"libb200_{variant}.so"
-    extra = {"": [], "early": ["-DB200_PDL_EARLY_TRIGGER=1"]}[variant]
-    objdir = CSRC / ("build" if not variant else f"build_{variant}")
+    lib = LIB if not tag else subset_lib(tag)
+    objdir = CSRC / "build"
     stamp = objdir / (f"stamp_{tag}" if tag else "stamp")
-    digests = {src: _file_digest(src, headers) + variant for src in srcs}
+    digests = {src: _file_digest(src, headers) for src in srcs}
     digest = hashlib.sha256("".join(f"{s.name}:{d};" for s, d in sorted(digests.items())).encode()).hexdigest()
     if not force and lib.exists() and stamp.exists() and stamp.read_text() == digest:
         return lib
@@ -231,7 +227,7 @@ def build(force: bool = False, verbose: bool = False, variant: str = "", sources
         mark = objdir / (src.stem + ".digest")
         if not force and obj.exists() and mark.exists() and mark.read_text() == digests[src]:
             return obj
-        cmd = [nvcc, *NVCC_FLAGS, *extra, "-c", str(src), "-o", str(obj)]
+        cmd = [nvcc, *NVCC_FLAGS, "-c", str(src), "-o", str(obj)]
         r = subprocess.run(cmd, capture_output=True, text=True)
         log = objdir / (src.stem + ".log")
         log.write_text(r.stdout + r.stderr)
@@ -266,4 +262,4 @@ def is_current(lib: Path = LIB) -> bool:
 
 
 if __name__ == "__main__":
-    print(build(force="--force" in sys.argv, verbose=True, variant="early" if "--early" in sys.argv else ""))
+    print(build(force="--force" in sys.argv, verbose=True))

@@ -633,7 +633,7 @@ gemm_bf16_tcgen05_2sm_kernel(const __grid_constant__ CUtensorMap tmap_w,
                                  group_m, nullptr, nullptr, 0, dir);
 }
 
-// W8A8 projection of the fp8 checkpoints GPUStack deploys (BASELINE config "Llama-3-70B fp8"):
+// W8A8 projection of the fp8 checkpoints GPUStack deploys (Llama-3-70B fp8):
 // Y[m,n] = (sum_k Xq[m,k] * Wq[n,k]) * xscale[m] * wscale[n * wscale_stride]
 // (reference operator: cutlass_scaled_mm behind Fp8LinearMethod.apply,
 // $VLLM/model_executor/layers/quantization/fp8.py:437-470).

@@ -1,4 +1,4 @@
-// Mixture-of-experts routing for the Mixtral family (BASELINE config "Mixtral-8x7B"; reference:
+// Mixture-of-experts routing for the Mixtral family (Mixtral-8x7B; reference:
 // MixtralMoE -> FusedMoE in $VLLM/model_executor/models/mixtral.py and
 // $VLLM/model_executor/layers/fused_moe/: topk_softmax, moe_align_block_size, moe_sum).
 //

@@ -41,7 +41,7 @@ int make_tmap_out_3d(CUtensorMap* out, const void* base, int elem_bytes, uint64_
 bool pdl_enabled();
 
 // Kernel classes whose launches can be taken out of programmatic dependent launch individually
-// (B200_PDL_OFF_CLASSES = bitmask, default 2): 1 = step-final sampler, 2 = MoE routing / grouped GEMMs.
+// (B200_PDL_OFF_CLASSES = bitmask, default 0): 1 = step-final sampler, 2 = MoE routing / grouped GEMMs.
 enum PdlClass { kPdlDefault = 0, kPdlSampler = 1, kPdlMoe = 2 };
 bool pdl_class_enabled(int cls);
 

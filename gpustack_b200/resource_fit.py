@@ -1,4 +1,4 @@
-"""Exact VRAM model of this engine, for GPUStack's placement (SURVEY.md section 8 f-3).
+"""Exact VRAM model of this engine, for GPUStack's placement.
 
 GPUStack places a custom backend with `VRAM = weight_file_bytes * 1.2 + 2 GiB`
 (gpustack/policies/utils.py:283-360; used by CustomBackendResourceFitSelector,

@@ -6,7 +6,7 @@ chunks of admitted / waiting prompts (with chunking of long prompts) -- ONE mixe
 running requests keep producing a token per step while new prompts are prefilled (the reference
 scheduler's unified token budget).  Steps without prompts to prefill are pure decode steps (CUDA-graph
 path); block allocation / prefix-cache reuse / preemption go through the BlockPool.
-`mixed_steps=False` restores the round-1 policy (prefill steps never carry decode tokens).
+`mixed_steps=False` restores the first policy (prefill steps never carry decode tokens).
 
 Running sequences live in a compact "persistent batch" of numpy arrays (rows 0..B-1) so that a
 decode step's inputs are produced by a handful of vectorised numpy ops instead of per-request

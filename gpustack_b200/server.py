@@ -1,6 +1,6 @@
 """OpenAI-compatible HTTP surface of the engine -- the drop-in boundary GPUStack talks to.
 
-Contract (SURVEY.md section 8b):
+Contract:
   * POST /v1/chat/completions, /v1/completions: stream = SSE `data: {json}\\n\\n` ... `data: [DONE]`;
     chunks validate as openai.types.chat.ChatCompletionChunk (parsed that way by
     gpustack/api/middlewares.py:219-262); final usage chunk when stream_options.include_usage

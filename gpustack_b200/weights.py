@@ -1,8 +1,8 @@
 """Weight loading: HF-format safetensors directory -> fused, tensor-parallel-sharded bf16 (or
 fp8 W8A8) tensors.
 
-Sharding follows the reference engine's Megatron layout (SURVEY.md section 8e;
-$VLLM/model_executor/models/llama.py:81-347): QKV and gate_up are column-parallel (each rank owns
+Sharding follows the reference engine's Megatron layout
+($VLLM/model_executor/models/llama.py:81-347): QKV and gate_up are column-parallel (each rank owns
 Hq/t query heads, Hkv/t kv heads and I/t MLP columns), O and down are row-parallel (in-dim / t),
 lm_head and the embedding table are vocab-parallel (rows [rank*ceil(V/t), ...)), the norms are replicated.
 

@@ -114,7 +114,7 @@ int b200_gemm_pick_block_x(int M, int N, int K);
 int b200_gemm_bf16_silu_mul(const void* X, const void* W, void* Y, int M, int N, int K, int64_t ldx,
                             int64_t ldw, int64_t ldy, void* stream);
 /* W8A8 fp8 (e4m3) projection -- the linear layers of the fp8 checkpoints GPUStack deploys
- * (BASELINE config "Llama-3-70B fp8"; reference operator: cutlass_scaled_mm behind
+ * (Llama-3-70B fp8; reference operator: cutlass_scaled_mm behind
  * Fp8LinearMethod.apply, $VLLM/model_executor/layers/quantization/fp8.py:437-470):
  *   Y[m,n] = (sum_k Xq[m,k] * Wq[n,k]) * xscale[m] * wscale[n * wscale_stride]
  * Xq [M,K], Wq [N,K] e4m3 bytes (K-major, K % 128 == 0, N > 128); xscale [M] fp32 dynamic

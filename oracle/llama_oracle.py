@@ -3,7 +3,7 @@
 Only tests/, __graft_entry__.smoke() and bench.py's cpu_baseline / --impl reference leg may import
 this module.  The engine (gpustack_b200/) never does: it has no CPU path.
 
-GPUStack itself contains no inference arithmetic (SURVEY.md section 0.1); the arithmetic of "the
+GPUStack itself contains no inference arithmetic; the arithmetic of "the
 reference's vLLM backend" lives in third-party vLLM (pinned vllm==0.10.1.1 in the reference's
 pyproject.toml:97, 0.22.0 installed here).  Each function below restates one operator of that
 engine in plain PyTorch-CPU fp32 with bf16 rounding at the points where the engine stores bf16,
@@ -13,7 +13,7 @@ Pinning: tests/golden/make_golden.py imports vLLM's own pure-PyTorch implementat
 (vllm.ir.ops.layernorm, RotaryEmbedding.forward_static, SiluAndMul.forward_native) and HF
 transformers' LlamaForCausalLM in the build container and commits their outputs as fixtures;
 tests/test_oracle_golden.py checks this oracle against them.  The reference publishes no golden
-vectors for inference (SURVEY.md section 8c), so those generated fixtures are the pin.
+vectors for inference, so those generated fixtures are the pin.
 """
 from __future__ import annotations
 

@@ -134,7 +134,7 @@ def tiny_llama_from_hf():
 
 
 def tiny_qwen2_from_hf():
-    """Qwen2 family: q/k/v bias + tied embeddings, GQA group of 7."""
+    """Qwen2 family (Qwen2-0.5B): q/k/v bias + tied embeddings, GQA group of 7."""
     from transformers import Qwen2Config, Qwen2ForCausalLM
 
     cfg = O.TINY_QWEN2
@@ -162,7 +162,7 @@ def tiny_qwen2_from_hf():
 
 
 def tiny_mixtral_from_hf():
-    """Mixtral family: 8 experts, top-2 routing with renormalisation.
+    """Mixtral family (Mixtral-8x7B): 8 experts, top-2 routing with renormalisation.
     transformers 5.x keeps the experts fused in memory (mlp.experts.gate_up_proj [E, 2I, H] = gate
     rows then up rows, mlp.experts.down_proj [E, H, I], router mlp.gate.weight); checkpoints -- and
     the oracle -- use the classic block_sparse_moe.experts.{e}.w1/w3/w2 names."""

@@ -1,5 +1,5 @@
 """End-to-end parity of the engine (scheduler + runner + kernels) against the CPU oracle on the
-seeded tiny Llama configs.  Stated tolerance (SURVEY.md 8c): last-position logits
+seeded tiny Llama configs.  Stated tolerance: last-position logits
 max-abs-diff <= 2e-2 * max|logit| (5e-2 for the mixture-of-experts family, 0.12 for fp8 W8A8 -- see
 the tests); greedy tokens teacher-forced: wherever the oracle's top-2 margin exceeds that tolerance
 the engine must pick the same token."""
@@ -202,7 +202,7 @@ FP8_TOL = 0.12
 @pytest.mark.parametrize("cfg_o", [O.TINY, O.TINY128, O.TINY_QWEN2], ids=["tiny64", "tiny128", "qwen2-bias-tied-g7"])
 def test_fp8_w8a8_engine_matches_fp8_oracle(cfg_o):
     """`--quantization fp8`: per-tensor e4m3 weights of the fused projections, dynamic per-token
-    e4m3 activations (BASELINE config "Llama-3-70B fp8" at a size the oracle runs in seconds).
+    e4m3 activations (Llama-3-70B fp8, at a size the oracle runs in seconds).
 
     Stated tolerance: last-position logits max-abs-diff <= 0.12 * max|logit| against the oracle run
     in the same W8A8 mode.  It is 6x the bf16 tolerance on purpose: an e4m3 quantiser turns a

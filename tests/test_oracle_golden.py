@@ -58,7 +58,7 @@ def test_whole_model_against_hf(hf_gold, name, cfg):
     logits = model.forward(0, g["prompt"])[-4:]
     ref32, ref16 = g["logits_fp32"], g["logits_bf16"]
     scale = float(ref32.abs().max())
-    # stated tolerance (SURVEY.md 8c): max-abs-diff <= 2e-2 * max|logit| for a bf16 pipeline
+    # stated tolerance: max-abs-diff <= 2e-2 * max|logit| for a bf16 pipeline
     assert float((logits - ref32).abs().max()) <= 2e-2 * scale
     assert float((logits - ref16).abs().max()) <= 3e-2 * scale
     # greedy tokens: exact wherever HF's own fp32 and bf16 runs agree (i.e. no near-tie)
@@ -84,7 +84,7 @@ def test_paged_gather_and_attention_shapes():
 
 
 def test_qwen2_family_against_hf():
-    """q/k/v bias, tied embeddings, GQA group of 7 (the Qwen2-0.5B family of BASELINE.json configs[0])."""
+    """q/k/v bias, tied embeddings, GQA group of 7 (the Qwen2-0.5B family)."""
     g = torch.load(GOLD / "tiny_qwen2_hf.pt", weights_only=False)
     model = O.OracleLlama(O.TINY_QWEN2, O.init_weights(O.TINY_QWEN2, seed=7))
     logits = model.forward(0, g["prompt"])[-4:]
@@ -129,7 +129,7 @@ def test_fp8_linear_is_the_dequantised_product():
 
 
 def test_mixtral_family_against_hf():
-    """8 experts, top-2 softmax routing with renormalisation (BASELINE.json configs[4] family)."""
+    """8 experts, top-2 softmax routing with renormalisation (the Mixtral-8x7B family)."""
     g = torch.load(GOLD / "tiny_mixtral_hf.pt", weights_only=False)
     model = O.OracleLlama(O.TINY_MIXTRAL, O.init_weights(O.TINY_MIXTRAL, seed=7))
     logits = model.forward(0, g["prompt"])[-4:]

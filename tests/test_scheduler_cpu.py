@@ -79,7 +79,7 @@ def test_mixed_steps_carry_decode_tokens_with_the_prefill_chunks():
     assert [r.req_id for r in s.rows] == ["r0", "r1"] and s.num_computed[:2].tolist() == [12, 40]
     d = s.schedule()
     assert isinstance(d, DecodePlan) and d.batch == 2            # nothing left to prefill: pure decode step
-    # the round-1 policy is still available
+    # the first policy is still available
     s2 = Scheduler(64, 16, 8, 32, 256, 2, mixed_steps=False)
     s2.add(req(0, 10, max_tokens=5, ignore_eos=True))
     drive(s2, s2.schedule())

@@ -265,7 +265,7 @@ def test_bench_client_against_the_frontend_process():
 
 
 def test_reference_benchmark_serving_runs_unmodified_against_the_frontend():
-    """BASELINE.json's harness, benchmarks/benchmark_serving.py of the reference, run UNMODIFIED
+    """The harness of the serving benchmark, benchmarks/benchmark_serving.py of the reference, run UNMODIFIED
     (tools/run_reference_harness.py: runpy + a stand-in for the missing httpx_aiohttp + a seed)
     against the real frontend process: chat completions, streaming, usage from the last chunk,
     TTFT on the first chunk -- every request must succeed and the token accounting must add up."""

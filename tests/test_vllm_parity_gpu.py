@@ -1,5 +1,4 @@
-"""Output parity against the LIVE reference engine (protocol iv; north star:
-"outputs match the reference's own vLLM backend on the same prompts and random-init weights"):
+"""Output parity against the LIVE reference engine ("outputs match the reference's own vLLM backend on the same prompts and random-init weights"):
 one seeded N(0, 0.02) safetensors checkpoint is served by this repo's engine and scored by vLLM
 (tools/vllm_parity.py, the version installed in the image) -- same directory, token-id prompts,
 greedy.  vLLM is teacher-forced on OUR tokens through `prompt_logprobs`; wherever its top-2

@@ -1,5 +1,5 @@
 """Weight sharding, checkpoint round trip and config parsing (CPU): the tensor-parallel shards must
-reassemble to exactly the un-sharded computation (SURVEY.md 8e: QKV/gate_up column-parallel,
+reassemble to exactly the un-sharded computation (QKV/gate_up column-parallel,
 O/down row-parallel + sum, vocab-parallel lm_head), and an HF-format directory written by
 save_checkpoint must load back bit-identically."""
 import json
@@ -93,7 +93,7 @@ def test_tp_divisibility_rule_matches_the_reference_scheduler():
 
 def test_config_parsing_and_byte_accounting():
     c = llama3_8b()
-    assert c.weight_bytes(1) == 15_009_849_344 and c.kv_bytes_per_token(1) == 131_072     # SURVEY.md 8d
+    assert c.weight_bytes(1) == 15_009_849_344 and c.kv_bytes_per_token(1) == 131_072
     assert c.kv_bytes_per_token(8) == 16_384
     hf = {"architectures": ["LlamaForCausalLM"], "vocab_size": 100, "hidden_size": 64, "intermediate_size": 128,
           "num_hidden_layers": 1, "num_attention_heads": 4, "rope_theta": 1e4, "eos_token_id": [7, 9]}
@@ -253,7 +253,7 @@ def test_mixtral_config_and_transformers5_fused_checkpoint_layout(tmp_path):
     back = ModelConfig.from_dict(d)
     assert back.num_local_experts == 8 and back.num_experts_per_tok == 2 and back.architecture == "MixtralForCausalLM"
     big = mixtral_8x7b()
-    # SURVEY.md 8: 46,702,792,704 parameters
+    # 46,702,792,704 parameters
     n = big.vocab_size * big.hidden_size * 2 + big.num_hidden_layers * (
         (big.q_size + 2 * big.kv_size) * big.hidden_size + big.q_size * big.hidden_size + 8 * 3 * big.intermediate_size * big.hidden_size
         + 8 * big.hidden_size + 2 * big.hidden_size) + big.hidden_size
@@ -282,7 +282,7 @@ def test_mixtral_config_and_transformers5_fused_checkpoint_layout(tmp_path):
         assert torch.equal(la.router, lb.router) and torch.equal(la.w13, lb.w13) and torch.equal(la.w2, lb.w2)
 
 
-# --------------------------------------------------------------------- VRAM model (SURVEY 8 f-3)
+# --------------------------------------------------------------------- VRAM model
 def _resident_bytes(w):
     """bytes the shard occupies once every tensor is its own device buffer (on the CPU the row
     slices are views of the full checkpoint tensors); a tied lm_head is a view of the embedding."""

@@ -1,4 +1,4 @@
-"""Extract the judged metrics from an .ncu-rep (read offline with `ncu -i ... --page raw --csv`)."""
+"""Extract the metrics of the profiles from an .ncu-rep (read offline with `ncu -i ... --page raw --csv`)."""
 import csv
 import io
 import subprocess

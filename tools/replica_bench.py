@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""BASELINE.json configs[2] / configs[4] topology as a declared stand-in: R independent
+"""The topology of 1,000 requests through a gateway, and of two replicas, as a declared stand-in: R independent
 `b200-engine serve` replicas (TP = --tp each, on disjoint GPUs) behind tools/rr_relay.py (the
 reference's RoundRobinStrategy + worker-proxy relay semantics), loaded by the reference's own
 benchmarks/benchmark_serving.py (unmodified) at a sweep of concurrencies -- the "QPS sweep".

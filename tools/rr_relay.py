@@ -1,8 +1,8 @@
 #!/usr/bin/env python
 """Declared STAND-IN for the part of GPUStack that sits in front of two engine replicas
-(BASELINE.json configs[2] / configs[4]: "through gpustack/gateway", "TP=4 x 2 replicas, gateway
-round-robin").  GPUStack itself (server + worker + Higress) cannot run offline (SURVEY.md section 0.2,
-Appendix C.1); this relay reproduces only the two behaviours that touch the request path:
+("through gpustack/gateway", "TP=4 x 2 replicas, gateway
+round-robin").  GPUStack itself (server + worker + Higress) cannot run offline;
+this relay reproduces only the two behaviours that touch the request path:
 
   * instance choice: `RoundRobinStrategy.select_instance` -- one `itertools.cycle` per model id,
     rebuilt when the list of running instances changes (gpustack/http_proxy/strategies.py:18-35,

@@ -10,7 +10,7 @@ baseline/_ref/benchmarks/benchmark_serving.py (an untracked, unmodified copy tha
 `__graft_entry__.build()` places there so that it travels to the GPU box; reference sources are
 never committed).  Two things it needs are supplied from outside, without touching it: the missing
 third-party `httpx_aiohttp` module (tools/shims/) and a seed for its unseeded `random` prompts
-(SURVEY.md section 8d: `random.seed(0)` via a wrapper).
+(`random.seed(0)` via a wrapper).
 """
 import os
 import random

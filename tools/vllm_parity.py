@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Live-engine parity, reference side (SURVEY.md section 8c protocol iv): the engine GPUStack's vLLM
+"""Live-engine parity, reference side (teacher-forced scores): the engine GPUStack's vLLM
 backend launches -- vLLM, whatever version is installed -- scores given token sequences from the SAME
 safetensors directory this repo's engine served.  For every sequence (prompt + the tokens OUR engine
 generated) vLLM returns, for each generated position, its top-k next-token log-probabilities given
