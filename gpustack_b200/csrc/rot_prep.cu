@@ -144,24 +144,29 @@ rot_prep_kernel(RotPrepArgs a) {
 
 // The same steps with 16-byte accesses, TOK tokens per CTA: a token's cos / sin are computed ONCE (dims / 2 angles)
 // into shared memory and used by every head.  A CTA of one token is one chain of latencies (position, angles, rows, stores);
-// four tokens share it, which is what a prompt's rows are bound by, and single rows keep a CTA each.  A head is cut into items of VEC = 16 bytes / sizeof(TA) entries: an
+// four tokens share it, which is what a prompt's rotated bf16 rows are bound by; fp32 rows, which are twice the bytes, rows without a
+// rotation, and steps of few tokens keep a CTA per token.  A head is cut into items of VEC = 16 bytes / sizeof(TA) entries: an
 // interleaved rotation turns the pairs inside an item; a half-split rotation makes an item of the piece [d, d + VEC)
 // and its partner [d + dims/2, ...); the unrotated rest are plain items.  LPH lanes (a power of two >= items per
 // head) share a head, a warp covers 32 / LPH head slots at a time, the sum of squares is reduced inside the group.
+// SILU is an instance of its own: its code, unused, cost the others 2 to 14 %.  Resident CTAs: five of bf16 rows (48 registers; without
+// the bound 58, 2048 rows 12.2 -> 14.1 us), fp32 rows as they compile.
 constexpr int kRvThreads = 256;
 
-template <typename TA, typename TD, int TOK>
-__global__ void __launch_bounds__(kRvThreads)
+template <typename TA, typename TD, int TOK, bool SILU>
+__global__ void __launch_bounds__(kRvThreads, sizeof(TA) == 2 ? 5 : SILU ? 6 : 1)
 rot_prep_vec_kernel(RotPrepArgs a, int T, int lph, int items_q, int items_v) {
   constexpr int VEC = 16 / (int)sizeof(TA);
   extern __shared__ float2 cs_all[];                  // [TOK][dims / 2] (cos, sin) of the tokens
   const int tok0 = blockIdx.x * TOK, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int H = a.H, G = a.G, dk = a.dk, dv = a.dv, dims = a.dims, half = dims >> 1;
+  const int slot0 = TOK == 1 && a.paged ? a.slots[tok0] : 0;
   if (dims > 0) {
+    const int pos0 = a.positions[tok0];
     for (int i = threadIdx.x; i < half * TOK; i += kRvThreads) {
       const int e = TOK == 1 ? 0 : i / half, j = i - e * half;
-      if (tok0 + e >= T) break;
-      const double ang = (double)a.positions[tok0 + e] * a.freq[j];
+      if (TOK > 1 && tok0 + e >= T) break;
+      const double ang = (double)(TOK == 1 ? pos0 : a.positions[tok0 + e]) * a.freq[j];
       const float rem = (float)(ang - 6.283185307179586 * rint(ang * 0.15915494309189535));
       float sn, c;
       sincosf(rem, &sn, &c);
@@ -175,8 +180,8 @@ rot_prep_vec_kernel(RotPrepArgs a, int T, int lph, int items_q, int items_v) {
   const int n_rot = dims == 0 ? 0 : (a.half_layout ? half / VEC : dims / VEC);
   for (int hs0 = warp * per_warp; hs0 < n_slots * TOK; hs0 += (kRvThreads / 32) * per_warp) {
     const int e = TOK == 1 ? 0 : (hs0 + sub) / n_slots, hs = hs0 + sub - e * n_slots, t = tok0 + e;
-    const bool live = e < TOK && hs < n_slots && t < T;
-    const int slot = live && a.paged ? a.slots[t] : 0;
+    const bool live = hs < n_slots && (TOK == 1 || (e < TOK && t < T));
+    const int slot = TOK == 1 ? slot0 : live && a.paged ? a.slots[t] : 0;
     const TA* row = reinterpret_cast<const TA*>(a.proj) + (size_t)t * a.ld;
     const float2* cs = cs_all + e * half;
     const bool is_q = live && hs < H, is_k = live && !is_q && hs < H + G, is_v = live && !is_q && !is_k;
@@ -218,7 +223,7 @@ rot_prep_vec_kernel(RotPrepArgs a, int T, int lph, int items_q, int items_v) {
           for (int i = 0; i < VEC; ++i) rp_store(vdst + d1 + i, x1[i]);
         }
       }
-      if (a.feature == 1) {
+      if constexpr (SILU) {
         logistic_all<true>(x0, x0);
         if (d1 >= 0) logistic_all<true>(x1, x1);
       }
@@ -325,15 +330,26 @@ extern "C" int b200_rot_prep_hm(const void* proj, int src_f32, int64_t ld, int q
     if (ok) {
       int lph = 1;
       while (lph < items) lph <<= 1;
-      // four tokens per CTA once that still leaves every SM eight CTAs (and their angles fit the default shared memory)
+      // four tokens per CTA of rotated bf16 rows once that still leaves every SM eight CTAs (and their angles fit the default shared
+      // memory): 8 + 8 + 8 heads of 128 into fp32 rows, warm, a CTA per token -> four: 4740 rows 25.3 -> 24.5 us, 8192 rows 49.0 ->
+      // 41.6; 16 + 4 + 4 heads into pages 31.1 -> 31.4 and 56.8 -> 50.7.  fp32 rows lose by it: 4800 rows 32.2 -> 38.0, 8192 rows 52.2 ->
+      // 57.0; rows without a rotation too: 18.9 -> 21.2 and 34.7 -> 34.7
       const size_t smem = (size_t)(dims / 2) * sizeof(float2);
-      if (T >= 4 * 8 * 148 && 4 * smem <= 40 * 1024) {
-        if (src_f32) rot_prep_vec_kernel<float, float, 4><<<(T + 3) / 4, kRvThreads, 4 * smem, s>>>(a, T, lph, items_q, items_v);
-        else if (dst_f32) rot_prep_vec_kernel<bf16, float, 4><<<(T + 3) / 4, kRvThreads, 4 * smem, s>>>(a, T, lph, items_q, items_v);
-        else rot_prep_vec_kernel<bf16, bf16, 4><<<(T + 3) / 4, kRvThreads, 4 * smem, s>>>(a, T, lph, items_q, items_v);
-      } else if (src_f32) rot_prep_vec_kernel<float, float, 1><<<T, kRvThreads, smem, s>>>(a, T, lph, items_q, items_v);
-      else if (dst_f32) rot_prep_vec_kernel<bf16, float, 1><<<T, kRvThreads, smem, s>>>(a, T, lph, items_q, items_v);
-      else rot_prep_vec_kernel<bf16, bf16, 1><<<T, kRvThreads, smem, s>>>(a, T, lph, items_q, items_v);
+      const bool four = !src_f32 && dims > 0 && T >= 4 * 8 * 148 && 4 * smem <= 40 * 1024;
+#define B200_RVS(TA, TD, TOK, S)                                                                                                  \
+  rot_prep_vec_kernel<TA, TD, TOK, S><<<(T + TOK - 1) / TOK, kRvThreads, TOK * smem, s>>>(a, T, lph, items_q, items_v)
+#define B200_RV(TA, TD, TOK)                        \
+  do {                                              \
+    if (feature == 1) B200_RVS(TA, TD, TOK, true);  \
+    else B200_RVS(TA, TD, TOK, false);              \
+  } while (0)
+      if (src_f32) B200_RV(float, float, 1);
+      else if (dst_f32 && four) B200_RV(bf16, float, 4);
+      else if (dst_f32) B200_RV(bf16, float, 1);
+      else if (four) B200_RV(bf16, bf16, 4);
+      else B200_RV(bf16, bf16, 1);
+#undef B200_RV
+#undef B200_RVS
       return b200_check_launch("b200_rot_prep");
     }
   }
