@@ -72,6 +72,71 @@ __device__ __forceinline__ bf16 finish_row(float num, float den, float mm, const
   return __float2bfloat16_rn(o);
 }
 
+// A group's ranges of keys, each parked by its CTA, into the final rows: the last CTA's work.
+// Every (maximum, sum) pair of the group is fetched at once and its factor formed once; then a thread adds up 16-byte pieces,
+// eight splits in flight.  (One value at a time, with the pairs read again for each, this was a chain of 2 x splits L2
+// latencies: a 3001-token row of 32 heads in 23 splits took 28 us, most of it here.)
+// A function of its own: inlined, it cost the rows that have one range 3 % (groups of 16 heads, 256 sequences of 100 rows: 17.1 -> 17.7 us).
+template <int D>
+__device__ __noinline__ void merge_splits(uint8_t* smem, const float* ws_o, const float* ws_ml, int num_splits, int G, size_t row0, int b,
+                                          int kvh, const float* sink, const bf16* gate, int64_t gate_stride, int gate_per_head, bf16* out,
+                                          float* lse_out) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float2* fac = reinterpret_cast<float2*>(smem);         // [G][num_splits] (maximum, sum), then (factor, factor * sum)
+  const bool al = (reinterpret_cast<uintptr_t>(ws_o) & 15) == 0;   // the caller's workspace need not be
+  for (int i = threadIdx.x; i < G * num_splits; i += blockDim.x) {
+    const float* ml = ws_ml + (row0 * num_splits + i) * 2;
+    fac[i] = make_float2(__ldcg(ml), __ldcg(ml + 1));
+  }
+  __syncthreads();
+  float* top = reinterpret_cast<float*>(fac + G * num_splits);     // [G][2] (maximum, denominator)
+  for (int g = warp; g < G; g += kDecWarps) {
+    float mm = -INFINITY;
+    for (int sp = lane; sp < num_splits; sp += 32) mm = fmaxf(mm, fac[g * num_splits + sp].x);
+    mm = warp_max(mm);
+    for (int sp = lane; sp < num_splits; sp += 32) {
+      float2& f = fac[g * num_splits + sp];
+      const float sc = f.x == -INFINITY ? 0.f : exp2f(f.x - mm);
+      f = make_float2(sc, sc * f.y);
+    }
+    __syncwarp();
+    if (lane == 0) {
+      float den = 0.f;
+      for (int sp = 0; sp < num_splits; ++sp) den += fac[g * num_splits + sp].y;
+      top[2 * g] = mm;
+      top[2 * g + 1] = den;
+    }
+  }
+  __syncthreads();
+  for (int idx = threadIdx.x; idx < G * (D / 4); idx += blockDim.x) {
+    const int g = idx / (D / 4), d = (idx % (D / 4)) * 4;
+    const size_t row = row0 + g;
+    const float* po_ = ws_o + row * num_splits * D + d;
+    const float2* f = fac + g * num_splits;
+    float num[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int s0 = 0; s0 < num_splits; s0 += 8) {
+      float4 v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (s0 + u < num_splits) {
+          const float* p = po_ + (size_t)(s0 + u) * D;
+          v[u] = al ? ld_cg_f4(p) : make_float4(__ldcg(p), __ldcg(p + 1), __ldcg(p + 2), __ldcg(p + 3));
+        }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        if (s0 + u >= num_splits || f[s0 + u].x == 0.f) continue;      // a split without keys: its sums are not read into the row
+        const float sc = f[s0 + u].x;
+        num[0] += sc * v[u].x; num[1] += sc * v[u].y; num[2] += sc * v[u].z; num[3] += sc * v[u].w;
+      }
+    }
+    const float mm = top[2 * g], den = top[2 * g + 1];
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      out[row * D + d + e] = finish_row(num[e], den, mm, sink, gate, gate_stride, b, kvh * G + g, D, d + e, gate_per_head);
+    if (lse_out != nullptr && d == 0) lse_out[row] = den > 0.f ? (mm + log2f(den)) * 0.6931471805599453f : -INFINITY;
+  }
+}
+
 // CAP: the scaled score passes cap * tanh(score / cap) before the mask; scale_log2 then holds 2 log2e scale / cap and
 // cap_log2 the cap in base-2 units.
 template <int D, bool CAP>
@@ -294,63 +359,7 @@ paged_attn_decode_kernel(const bf16* __restrict__ q, int64_t q_stride,
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  // Every (maximum, sum) pair of the group is fetched at once and its factor formed once; then a thread adds up 16-byte pieces,
-  // eight splits in flight.  (One value at a time, with the pairs read again for each, this was a chain of 2 x splits L2
-  // latencies: a 3001-token row of 32 heads in 23 splits took 28 us, most of it here.)
-  float2* fac = reinterpret_cast<float2*>(smem);         // [G][num_splits] (maximum, sum), then (factor, factor * sum)
-  const size_t row0 = (size_t)b * Hq + kvh * G;
-  const bool al = (reinterpret_cast<uintptr_t>(ws_o) & 15) == 0;   // the caller's workspace need not be
-  for (int i = threadIdx.x; i < G * num_splits; i += blockDim.x) {
-    const float* ml = ws_ml + (row0 * num_splits + i) * 2;
-    fac[i] = make_float2(__ldcg(ml), __ldcg(ml + 1));
-  }
-  __syncthreads();
-  float* top = reinterpret_cast<float*>(fac + G * num_splits);     // [G][2] (maximum, denominator)
-  for (int g = warp; g < G; g += kDecWarps) {
-    float mm = -INFINITY;
-    for (int sp = lane; sp < num_splits; sp += 32) mm = fmaxf(mm, fac[g * num_splits + sp].x);
-    mm = warp_max(mm);
-    for (int sp = lane; sp < num_splits; sp += 32) {
-      float2& f = fac[g * num_splits + sp];
-      const float sc = f.x == -INFINITY ? 0.f : exp2f(f.x - mm);
-      f = make_float2(sc, sc * f.y);
-    }
-    __syncwarp();
-    if (lane == 0) {
-      float den = 0.f;
-      for (int sp = 0; sp < num_splits; ++sp) den += fac[g * num_splits + sp].y;
-      top[2 * g] = mm;
-      top[2 * g + 1] = den;
-    }
-  }
-  __syncthreads();
-  for (int idx = threadIdx.x; idx < G * (D / 4); idx += blockDim.x) {
-    const int g = idx / (D / 4), d = (idx % (D / 4)) * 4;
-    const size_t row = row0 + g;
-    const float* po_ = ws_o + row * num_splits * D + d;
-    const float2* f = fac + g * num_splits;
-    float num[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int s0 = 0; s0 < num_splits; s0 += 8) {
-      float4 v[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u)
-        if (s0 + u < num_splits) {
-          const float* p = po_ + (size_t)(s0 + u) * D;
-          v[u] = al ? ld_cg_f4(p) : make_float4(__ldcg(p), __ldcg(p + 1), __ldcg(p + 2), __ldcg(p + 3));
-        }
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        if (s0 + u >= num_splits || f[s0 + u].x == 0.f) continue;      // a split without keys: its sums are not read into the row
-        const float sc = f[s0 + u].x;
-        num[0] += sc * v[u].x; num[1] += sc * v[u].y; num[2] += sc * v[u].z; num[3] += sc * v[u].w;
-      }
-    }
-    const float mm = top[2 * g], den = top[2 * g + 1];
-#pragma unroll
-    for (int e = 0; e < 4; ++e)
-      out[row * D + d + e] = finish_row(num[e], den, mm, sink, gate, gate_stride, b, kvh * G + g, D, d + e, gate_per_head);
-    if (lse_out != nullptr && d == 0) lse_out[row] = den > 0.f ? (mm + log2f(den)) * 0.6931471805599453f : -INFINITY;
-  }
+  merge_splits<D>(smem, ws_o, ws_ml, num_splits, G, (size_t)b * Hq + kvh * G, b, kvh, sink, gate, gate_stride, gate_per_head, out, lse_out);
 }
 
 // ----------------------------------------------------------------------------------- prefill

@@ -1,10 +1,11 @@
-// Matrix-state recurrences with one decay per head and token over prompt portions, all chunks of a sequence side by side.
+// Matrix-state recurrences with one decay per token and head, or per token and key channel, over prompt portions: all chunks of a
+// sequence side by side.
 //
 // With a state S (dk x dv), rows t = 0 .. n-1 of a chunk of 64 and the weights that a recurrence's `Form` supplies:
 //     o_t = aq_t S_start^T q_t + sum_{s<=t} D(t, s) (k_s . q_t) v_s          S_end = a S_start + b sum_s w_s k_s v_s^T
 // Three launches:
 //   chunk_state   one CTA per (chunk, head, value tile): C = sum_s w_s k_s v_s^T into the workspace, [chunk][H][dk][dv]
-//   chunk_carry   one CTA per (32 x 32 piece of the state, head, sequence): walks a sequence's chunks, puts S_start in C's
+//   chunk_carry   one CTA per (8 keys x 128 values of the state, head, sequence): walks a sequence's chunks, puts S_start in C's
 //                 place and leaves the sequence's final state in its slot
 //   chunk_output  one CTA per (chunk, head, value tile): k_s . q_t, then aq_t S_start^T q_t and the chunk's own rows
 // Why: the one-pass form (16 rows at a time, state in shared memory) is a serial chain of short phases on (sequences x heads x
@@ -177,8 +178,8 @@ struct ChunkTile<float, ROWS, W, PITCH> {
   __device__ __forceinline__ void land(float*) const {}
 };
 
-// Running sums of a chunk's logarithms per key channel, inclusive: F[t][k] = sum_(r <= t) lg(r, k), 256 threads, four runs of 16
-// rows each.  hi / lo: [64][DK + 4].  Ends with a barrier.
+// Running sums of a chunk's logarithms per key channel, inclusive: F[t][k] = sum_(r <= t) lg(r, k), 256 threads: four runs of 16
+// rows per channel, with 128 channels two of 32.  hi / lo: [64][DK + 4].  Ends with a barrier.
 template <int DK, typename LG>
 __device__ __forceinline__ void cs_channel_sums(float* hi, float* lo, double* run, LG lg) {
   constexpr int RUNS = kCsThreads / DK, ROWS = kCsRows / RUNS, P = DK + 4;

@@ -10,7 +10,8 @@
 // each of its 8 warps holds RPW = ceil(dk / 8) neighbouring key rows of those columns in registers.  A token's update
 // is then two FMAs per held element with the token's k, q and alpha broadcast from shared memory -- no shuffle; the
 // warps' partial sums of S^T q meet in shared memory once per 16 staged tokens and are added in warp order (a fixed
-// order, whatever the cut of the prompt).  A sequence's new rows run in order, 16 staged at a time.
+// order, whatever the cut of the prompt).  A sequence's new rows run in order, 16 staged at a time.  Long portions run over chunks
+// of 64 rows instead (chunk_scan.cuh), counted from the portion's first row: there the cut of a prompt moves the last bits.
 #include "chunk_scan.cuh"
 #include "common.cuh"
 #include "runtime.h"
