@@ -14,8 +14,8 @@
 // 64 rows and head, written, carried and read once each).  Everything is fp32 FMAs as before; bound: the FMA rate
 // (4 dk dv + 64 (dk + dv) per row and head), which register tiles of packed pairs (fma.rn.f32x2) approach: a CTA of 256 threads
 // holds a 128 x 128 (state) or 64 x 128 (output) tile, one 16-byte shared-memory read feeds 8 to 16 FMAs.
-// 4 prompts of 2048 rows, 8 heads of 128 x 128 (5.6 GFLOP): one-pass 762 us, here 208 us (linear attention, L2 cold), of which
-// state 60, carry 45, output 100 us (without the copies behind the sums, and 32 x 32 pieces in the carry: 65, 62, 116).
+// 4 prompts of 2048 rows, 8 heads of 128 x 128 (5.6 GFLOP): one-pass 762 us, here 210 us (linear attention, L2 cold), of which
+// state 62, carry 44, output 104 us (without the copies behind the sums, and pieces of 32 x 32 in the carry: 65, 62, 116).
 // Chunks of 64: with 32 the states double, with 128 the chunk's own rows cost more than the states save.
 // Sequences of at most kCsShort rows are left to the caller's one-pass kernel (their state would cross L2 three times for
 // a few rows of work).

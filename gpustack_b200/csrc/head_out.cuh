@@ -1,7 +1,7 @@
 // A recurrent mixer's closing step per (token, head): the head's fp32 output over its root mean square, times a weight, times the
 // gate's activation, rounded once.  A head of dv = 4 LPH values is held by LPH lanes as one 16-byte piece each, one head per group of
-// lanes: many small warps keep the bytes in flight.  Bound: launch and latency up to 1000 rows, then HBM, 4 bytes in, gate in and output
-// out per value.  8 heads of 128, bf16 gates, warm: 1.8 us for one row, 5.4 for 2048, 16.3 for 8192 (with four heads in flight per lane
+// lanes: many small warps keep the bytes in flight.  Bound: launch and latency up to 1000 rows, then instructions (3.1 per clock and SM,
+// 8192 rows at 4.1 TB/s).  8 heads of 128, bf16 gates, warm: 1.8 us for one row, 5.4 for 2048, 16.3 for 8192 (with four heads in flight per lane
 // 4.5, 7.0 and 19.5; a CTA or a warp per head, looping, 2.6, 7.4 and 22.9).
 #pragma once
 #include "common.cuh"
