@@ -47,6 +47,11 @@ __device__ __forceinline__ cs_f2 cs_fma(cs_f2 a, cs_f2 b, cs_f2 c) {
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;
 }
+__device__ __forceinline__ cs_f2 cs_sub(cs_f2 a, cs_f2 b) {
+  cs_f2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
 __device__ __forceinline__ cs_f2 cs_mul(cs_f2 a, cs_f2 b) {
   cs_f2 r;
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
@@ -70,6 +75,8 @@ struct ChunkScanArgs {
   float* ws_row;                   // [chunks][H][ws_row_width]: a recurrence's own carry (its Form says what)
   int ws_row_width;                // dk + 4
   float* ws_sums;                  // [chunks][H][2][64][dk]: kVector, the running sums' two parts
+  const void* v;                   // chunk_tc.cuh: rows of the values (x, or rows of their own) and their pitch
+  int64_t ld_v;
 };
 
 __host__ __device__ __forceinline__ int cs_chunks(int rows, int short_rows) { return rows > short_rows ? (rows + kCsRows - 1) / kCsRows : 0; }
@@ -82,8 +89,11 @@ inline int64_t cs_max_chunks(int64_t rows, int64_t n_seqs) {
   const int64_t longs = rows / (kCsShort + 1);
   return rows / kCsRows + (longs < n_seqs ? longs : n_seqs);
 }
+// (chunk_tc.cuh's chunks of 128 rows keep their first states in 6 bytes a number: room for the larger of the two)
 inline int64_t cs_workspace_floats(int64_t rows, int64_t n_seqs, int64_t H, int64_t dk, int64_t dv, bool vector = false) {
-  return cs_max_chunks(rows, n_seqs) * H * (dk * dv + dk + 4 + (vector ? 2 * kCsRows * dk : 0));
+  const int64_t longs = rows / (kCsShort + 1), n = longs < n_seqs ? longs : n_seqs;
+  const int64_t halves = 2 * (rows / kCsRows + n) > 3 * (rows / 128 + n) ? 2 * (rows / kCsRows + n) : 3 * (rows / 128 + n);
+  return (halves * H * (dk * dv + dk + 4 + (vector ? 2 * kCsRows * dk : 0)) + 1) / 2;
 }
 
 // Sequence and place in it of chunk b (whole warp; seq -1: no such chunk), or with b < 0 the chunks before sequence `upto`.

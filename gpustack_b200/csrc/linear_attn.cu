@@ -19,11 +19,11 @@
 //                  Every power has a non-negative exponent (nothing is divided by a decay, so a small decay cannot
 //                  overflow); all products and sums are fp32 FMAs, only the grouping of the sums differs from the
 //                  serial form.  The CTA's 32 columns of S live in shared memory for the whole portion.
-// The same over chunks of 64 rows side by side (chunk_scan.cuh) when the caller brings a workspace.
+// The same over chunks of 128 rows side by side (chunk_tc.cuh) when the caller brings a workspace.
 // `linattn_out`    closes the mixer: the heads' outputs over their root mean square -- per head without a weight, or
 //                  all heads together with a weight vector -- times sigmoid(g) or silu(g) of the gate columns of the
 //                  fused projection, rounded once to the activation type.
-#include "chunk_scan.cuh"
+#include "chunk_tc.cuh"
 #include "common.cuh"
 #include "head_out.cuh"
 #include "runtime.h"
@@ -365,12 +365,12 @@ linattn_chunk4_kernel(const float* __restrict__ x, int64_t ld, int q_col, int k_
   }
 }
 
-// The fixed decay in the chunk form of chunk_scan.cuh: every weight is a power of the head's decay with a non-negative
+// The fixed decay in the chunk form of chunk_tc.cuh: every weight is a power of the head's decay with a non-negative
 // exponent, formed in fp64 by squaring (a decay of zero or below one's sign is as good as any) and rounded once.
 __device__ __forceinline__ float la_power(float d, int n) {
   double r = 1.0, b = (double)d;
 #pragma unroll
-  for (int bit = 0; bit < 7; ++bit) {
+  for (int bit = 0; bit < 8; ++bit) {
     if ((n >> bit) & 1) r *= b;
     b *= b;
   }
@@ -379,39 +379,46 @@ __device__ __forceinline__ float la_power(float d, int n) {
 
 struct LinearForm {
   static constexpr const char* kName = "b200_linattn_scan(chunks)";
-  static constexpr bool kVector = false;
+  static constexpr bool kNorm = false;
   struct Params {
     const float* decay;
   };
   struct Scratch {
-    float dp[kCsRows + 1], w[kCsRows];
+    float dp[kCtRows + 1], w[kCtRows];
   };
-  static __device__ __forceinline__ void state_weights(const Params& p, const ChunkScanArgs&, Scratch& sc, int h, const ChunkPlace& at) {
-    if ((int)threadIdx.x < at.rows) sc.w[threadIdx.x] = la_power(p.decay[h], at.rows - 1 - (int)threadIdx.x);
-    __syncthreads();
+  static __device__ __forceinline__ void state_weights(const Params& p, const ChunkScanArgs&, Scratch& sc, int h, const ChunkPlace& at, int) {
+    const int t = ct_team_row();
+    sc.w[t] = t < at.rows ? la_power(p.decay[h], at.rows - 1 - t) : 0.f;
   }
-  template <int DK>
-  static __device__ __forceinline__ void state_row(const ChunkScanArgs&, const Scratch&, const float*, int, int) {}
+  static __device__ __forceinline__ void state_row(float*, const Scratch&) {}
   struct Carry {
-    float d, full;
-    __device__ __forceinline__ Carry(const Params& p, const ChunkScanArgs&, int, int h, int, int) : d(p.decay[h]), full(la_power(d, kCsRows)) {}
-    __device__ __forceinline__ void fetch(const ChunkScanArgs&, int, int) {}
-    __device__ __forceinline__ void next(const Params&, int, int rows, float& a, float& b) {
-      a = rows == kCsRows ? full : la_power(d, rows);
-      b = 1.0f;
+    float d;
+    __device__ __forceinline__ Carry(const Params& p, const ChunkScanArgs&, int h, int) : d(p.decay[h]) {}
+    __device__ __forceinline__ void factors(int c0, int, int rows, float2* table) const {
+      const int c = c0 + (threadIdx.x & 31);
+      table[threadIdx.x & 31] = make_float2(la_power(d, min(kCtRows, max(rows - c * kCtRows, 0))), 1.0f);
     }
   };
   template <int DK>
-  static __device__ __forceinline__ void carry_row(const Params&, const ChunkScanArgs&, int, int, int, int, bool, int) {}
-  static __device__ __forceinline__ void output_weights(const Params& p, const ChunkScanArgs&, Scratch& sc, int h, const ChunkPlace&) {
-    if (threadIdx.x <= kCsRows) sc.dp[threadIdx.x] = la_power(p.decay[h], threadIdx.x);
+  static __device__ __forceinline__ void carry_row(const Params&, const ChunkScanArgs&, int, int, int, bool, int) {}
+  static __device__ __forceinline__ void output_weights(const Params& p, const ChunkScanArgs&, Scratch& sc, int h, const ChunkPlace&, int) {
+    sc.dp[ct_team_row() + 1] = la_power(p.decay[h], ct_team_row() + 1);
+    if (ct_team_row() == 0) sc.dp[0] = 1.f;
   }
   static __device__ __forceinline__ float q_scale(const Params&) { return 1.0f; }
-  static __device__ __forceinline__ float D(const Params&, const Scratch& sc, int t, int s) { return sc.dp[t - s]; }
+  struct Row {};
+  static __device__ __forceinline__ Row row(const Params&, const Scratch&, int) { return {}; }
+  static __device__ __forceinline__ float D(const Params&, const Scratch& sc, const Row&, int t, int s) { return sc.dp[t - s]; }
+  // of sixteen rows from s0 on, all of them seen (`before`) or not
+  static __device__ __forceinline__ void weights(const Params&, const Scratch& sc, const Row&, int t, int s0, bool, float (&d)[16]) {
+#pragma unroll
+    for (int e = 0; e < 16; ++e) d[e] = sc.dp[max(t - s0 - e, 0)];
+  }
   static __device__ __forceinline__ float aq(const Scratch& sc, int t) { return sc.dp[t + 1]; }
-  template <int DK>
-  static __device__ __forceinline__ void rows(const Params&, const ChunkScanArgs&, Scratch&, const float*, const float*, int, int, bool) {}
-  static __device__ __forceinline__ float4 finish(const Params&, const Scratch&, int, int, float4 acc, float4) { return acc; }
+  struct Finish {
+    __device__ __forceinline__ Finish(const Params&, const ChunkScanArgs&, const Scratch&, int, int, const float*) {}
+    __device__ __forceinline__ void apply(float (&)[16], const void*, int) const {}
+  };
 };
 
 // ------------------------------------------------------------------------------------------- out
@@ -524,7 +531,7 @@ extern "C" int b200_linattn_scan_chunked(const float* x, int64_t ld, int q_col, 
     if (rc != B200_OK) return rc;
   }
   const ChunkScanArgs a{x, ld, q_col, k_col, v_col, H, H, dv, cu_seq, ctx_lens, state_slots, n_seqs, short_rows, S, o_raw};
-  return cs_launch<float, LinearForm>(a, {decay}, dk, rows, workspace, s);
+  return ct_launch<float, LinearForm>(a, {decay}, dk, rows, workspace, s);
 }
 
 extern "C" int b200_linattn_out(const float* o_raw, const void* proj, int f32, int64_t ld, int gate_col, const void* w,

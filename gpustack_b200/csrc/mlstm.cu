@@ -21,7 +21,7 @@
 //
 // `mlstm_out` then divides every head's o_t by its root mean square, multiplies by the norm
 // weight and the sigmoid output gate, and rounds to the activation type.
-#include "chunk_scan.cuh"
+#include "chunk_tc.cuh"
 #include "common.cuh"
 #include "head_out.cuh"
 #include "runtime.h"
@@ -618,195 +618,186 @@ static int launch_chunk(const void* proj, int64_t ld, int q_col, int k_col, int 
   return b200_check_launch("b200_mlstm_scan(chunk)");
 }
 
-// The recurrence in the chunk form of chunk_scan.cuh.  Inside a chunk the log forget gates are summed in fp64 (64 of them, so
-// that differences of the sums keep an fp32 gate's precision); every exponent is <= 0 up to that rounding.  A chunk's own
-// contribution is stabilised by mloc = max_s (F_n - F_s + i_s); the carry turns that into the serial form's stabiliser
-// m = max(F_n + m_start, mloc).  The normaliser is one more value column of ones, carried beside the state; like the stabiliser
-// it is equal in all column slices, so slice 0 is read and all slices are written.
-//   ws_row of a chunk: [0, dk) the chunk's normaliser, then the one at its start; dk: F_n; dk + 1: mloc; dk + 2: m_start;
-//   dk + 3 (first chunk of a sequence): the stabiliser that the sequence came with
+// The recurrence in the chunk form of chunk_tc.cuh.  Inside a chunk the log forget gates are summed in fp64 (128 of them, so
+// differences of the sums keep an fp32 gate's precision); with g_t = max(m_0, max_(s<=t) (i_s - F_s)) the serial stabiliser is
+// m_t = F_t + g_t, and every exponent is <= 0 as in the serial form.  A chunk's own contribution is stabilised without any state
+// before it; the carry moves it to the sequence's.  The normaliser is one more value column of ones, carried beside the state; like
+// the stabiliser it is equal in all column slices, so slice 0 is read and all slices are written.
+//   ws_row of a chunk: [0, dk) the chunk's normaliser, then the one at its start; dk: F of the whole chunk; dk + 1: its own stabiliser;
+//   dk + 2: m_start; dk + 3 (first chunk of a sequence): the stabiliser that the sequence came with
 struct MlstmForm {
   static constexpr const char* kName = "b200_mlstm_scan(chunks)";
-  static constexpr bool kVector = false;
+  static constexpr bool kNorm = true;
   struct Params {
     const float* gates;
     const bf16* gate_bias;
     float cap, qscale;
-    float* n_state;
-    float* m_state;
+    float *n_state, *m_state;
     int Z;
   };
   struct Scratch {
-    double F[kCsRows];
-    float ii[kCsRows], w[kCsRows], m[kCsRows], aq[kCsRows], den[kCsRows];
+    CtExp from[kCtRows], to[kCtRows];                // i_s - F_s, F_t - m_t
+    CtExp top[kCtRows / 16];                         // the largest i_s - F_s of sixteen rows
+    union {
+      float below[kCtRows];                          // exp(i_s - F_s - top)
+      float w[kCtRows];                              // (ct_state's)
+    };
+    float m[kCtRows], aq[kCtRows], row[4];
+    double parts[9];
   };
-  // warp 0, two rows per lane: log gates of the chunk's rows, F their running sum, g the running maximum of i_s - F_s
-  static __device__ __forceinline__ void gate_sums(const Params& p, const ChunkScanArgs& a, int h, const ChunkPlace& at, double (&F)[2],
-                                                   double (&g)[2], float (&ii)[2]) {
-    const int lane = threadIdx.x & 31;
+  // a row per thread: log gates, F their running sum, g the running maximum of i_s - F_s
+  static __device__ __forceinline__ void gate_sums(const Params& p, const ChunkScanArgs& a, Scratch& sc, int h, const ChunkPlace& at, double& F,
+                                                   double& g, float& ii) {
     const float bi = __bfloat162float(p.gate_bias[h]), bf = __bfloat162float(p.gate_bias[a.H + h]);
-    double f[2];
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int t = 2 * lane + e;
-      f[e] = 0.0;
-      ii[e] = 0.f;
-      if (t < at.rows) {
-        const float* gr = p.gates + (size_t)(at.first + t) * 2 * a.H;
-        ii[e] = p.cap * tanhf((gr[h] + bi) / p.cap);
-        f[e] = (double)log_sigmoid(p.cap * tanhf((gr[a.H + h] + bf) / p.cap));
-      }
+    const int t = ct_team_row();
+    F = 0.0;
+    ii = 0.f;
+    if (t < at.rows) {
+      const float* gr = p.gates + (size_t)(at.first + t) * 2 * a.H;
+      ii = p.cap * tanhf((gr[h] + bi) / p.cap);
+      F = (double)log_sigmoid(p.cap * tanhf((gr[a.H + h] + bf) / p.cap));
     }
-    double sum = f[0] + f[1];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const double v = __shfl_up_sync(0xffffffffu, sum, o);
-      if (lane >= o) sum += v;
-    }
-    const double before = __shfl_up_sync(0xffffffffu, sum, 1);
-    F[1] = sum;
-    F[0] = lane ? before + f[0] : f[0];               // (not sum - f[1]: what is no number in a row stays out of the one before)
-    constexpr double kNone = -1.0e300;
-    const double g0 = 2 * lane < at.rows ? (double)ii[0] - F[0] : kNone, g1 = 2 * lane + 1 < at.rows ? (double)ii[1] - F[1] : kNone;
-    double mx = fmax(g0, g1);
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const double v = __shfl_up_sync(0xffffffffu, mx, o);
-      if (lane >= o) mx = fmax(mx, v);
-    }
-    g[1] = mx;
-    const double up = __shfl_up_sync(0xffffffffu, mx, 1);
-    g[0] = lane ? fmax(up, g0) : g0;
+    F = ct_team_scan<false>(F, sc.parts);
+    g = ct_team_scan<true>(t < at.rows ? (double)ii - F : -1.0e300, sc.parts + 4);
   }
-  static __device__ __forceinline__ float* row_of(const ChunkScanArgs& a, int chunk, int h, int dk) {
-    return a.ws_row + ((size_t)chunk * a.H + h) * (dk + 4);
+  static __device__ __forceinline__ void state_weights(const Params& p, const ChunkScanArgs& a, Scratch& sc, int h, const ChunkPlace& at, int fresh) {
+    double F, g;
+    float ii;
+    gate_sums(p, a, sc, h, at, F, g, ii);
+    const int t = ct_team_row();
+    if (t == kCtRows - 1) {                          // rows behind the last one add nothing
+      sc.parts[8] = g;
+      sc.row[0] = (float)F;
+      sc.row[1] = (float)(F + g);
+      sc.row[3] = at.local == 0 && !fresh ? p.m_state[((size_t)at.slot * a.H + h) * p.Z] : 0.f;
+    }
+    ct_named_barrier(kCtBarTeam, kCtTeam);
+    sc.w[t] = t < at.rows ? expf((float)((double)ii - F - sc.parts[8])) : 0.f;
   }
-  static __device__ __forceinline__ void state_weights(const Params& p, const ChunkScanArgs& a, Scratch& sc, int h, const ChunkPlace& at) {
-    if (threadIdx.x < 32) {
-      double F[2], g[2];
-      float ii[2];
-      gate_sums(p, a, h, at, F, g, ii);
-      const int lane = threadIdx.x, last = (at.rows - 1) >> 1;
-      const double Fn = __shfl_sync(0xffffffffu, (at.rows & 1) ? F[0] : F[1], last);
-      const double gn = __shfl_sync(0xffffffffu, g[1], 31);
-#pragma unroll
-      for (int e = 0; e < 2; ++e) sc.w[2 * lane + e] = 2 * lane + e < at.rows ? expf((float)((double)ii[e] - F[e] - gn)) : 0.f;
-      if (lane == 0) {
-        sc.den[0] = (float)Fn;
-        sc.den[1] = (float)(Fn + gn);
-        sc.den[2] = at.local == 0 && a.ctx_lens[at.seq] != 0 ? p.m_state[((size_t)at.slot * a.H + h) * p.Z] : 0.f;
-      }
-    }
-    __syncthreads();
-  }
-  template <int DK>
-  static __device__ __forceinline__ void state_row(const ChunkScanArgs& a, const Scratch& sc, const float* ks, int h, int rows) {
-    float* row = row_of(a, blockIdx.x, h, DK);
-    const int k = threadIdx.x;
-    if (k < DK) {
-      float n = 0.f;
-      for (int s = 0; s < rows; ++s) n = fmaf(sc.w[s], ks[s * DK + k], n);
-      row[k] = n;
-    }
-    if (k == 0) {
-      row[DK] = sc.den[0];
-      row[DK + 1] = sc.den[1];
-      row[DK + 3] = sc.den[2];
-    }
+  static __device__ __forceinline__ void state_row(float* row, const Scratch& sc) {
+    row[0] = sc.row[0];
+    row[1] = sc.row[1];
+    row[3] = sc.row[3];
   }
   struct Carry {
     const float* row;
     size_t step;
-    float m, F[kCsCarryDepth], ml[kCsCarryDepth];
-    int width;
-    __device__ __forceinline__ Carry(const Params&, const ChunkScanArgs& a, int, int h, int base, int) {
-      width = (int)(a.ws_row_width);
-      row = a.ws_row + ((size_t)base * a.H + h) * width;
-      step = (size_t)a.H * width;
-      m = row[width - 1];
+    float m;
+    __device__ __forceinline__ Carry(const Params&, const ChunkScanArgs& a, int h, int base)
+        : row(a.ws_row + ((size_t)base * a.H + h) * a.ws_row_width + a.ws_row_width - 4), step((size_t)a.H * a.ws_row_width) {
+      m = row[3];
     }
-    __device__ __forceinline__ void fetch(const ChunkScanArgs&, int c0, int nc) {
-#pragma unroll
-      for (int u = 0; u < kCsCarryDepth; ++u)
-        if (c0 + u < nc) {
-          F[u] = row[(c0 + u) * step + width - 4];
-          ml[u] = row[(c0 + u) * step + width - 3];
-        }
-    }
-    __device__ __forceinline__ void next(const Params&, int u, int, float& fa, float& fb) {
-      const float m_new = fmaxf(F[u] + m, ml[u]);
-      fa = expf(F[u] + m - m_new);
-      fb = expf(ml[u] - m_new);
-      m = m_new;
+    // whole warp, a chunk per lane: m_c = max(F_c + m_(c-1), own_c) is a running maximum of own_c - (F's sum) -- formed one after the
+    // other, as the one-pass form does
+    __device__ __forceinline__ void factors(int c0, int nc, int, float2* table) {
+      const int lane = threadIdx.x & 31, c = c0 + lane;
+      const float F = c < nc ? row[c * step] : 0.f, ml = c < nc ? row[c * step + 1] : 0.f;
+      float before = m, after = m;
+      for (int l = 0; l < 32 && c0 + l < nc; ++l) {
+        const float f = __shfl_sync(0xffffffffu, F, l), o = __shfl_sync(0xffffffffu, ml, l);
+        if (lane == l) before = m;
+        m = fmaxf(f + m, o);
+        if (lane == l) after = m;
+      }
+      table[lane] = make_float2(expf(F + before - after), expf(ml - after));
     }
   };
   template <int DK>
-  static __device__ __forceinline__ void carry_row(const Params& p, const ChunkScanArgs& a, int, int h, int base, int nc, bool fresh, int slot) {
+  static __device__ __forceinline__ void carry_row(const Params& p, const ChunkScanArgs& a, int h, int base, int nc, bool fresh, int slot) {
     const int k = threadIdx.x;
     if (k >= DK) return;
     float* n_out = p.n_state + ((size_t)slot * a.H + h) * p.Z * DK;
     float n = fresh ? 0.f : n_out[k];
-    float* row = row_of(a, base, h, DK);
+    float* row = a.ws_row + ((size_t)base * a.H + h) * (DK + 4);
     float m = row[DK + 3];
-    for (int c = 0; c < nc; ++c, row += (size_t)a.H * (DK + 4)) {
-      const float own = row[k], F = row[DK], ml = row[DK + 1];
-      const float m_new = fmaxf(F + m, ml);
-      row[k] = n;
-      if (k == 0) row[DK + 2] = m;
-      n = fmaf(expf(F + m - m_new), n, expf(ml - m_new) * own);
-      m = m_new;
+    const size_t step = (size_t)a.H * (DK + 4);
+    for (int c0 = 0; c0 < nc; c0 += kCtDepth) {        // as many chunks' rows in flight as there are of the state
+      float own[kCtDepth], F[kCtDepth], ml[kCtDepth];
+#pragma unroll
+      for (int u = 0; u < kCtDepth; ++u)
+        if (c0 + u < nc) {
+          const float* at = row + (c0 + u) * step;
+          own[u] = at[k];
+          F[u] = at[DK];
+          ml[u] = at[DK + 1];
+        }
+#pragma unroll
+      for (int u = 0; u < kCtDepth; ++u) {
+        if (c0 + u >= nc) break;
+        float* at = row + (c0 + u) * step;
+        const float m_new = fmaxf(F[u] + m, ml[u]);
+        at[k] = n;
+        if (k == 0) at[DK + 2] = m;
+        n = fmaf(expf(F[u] + m - m_new), n, expf(ml[u] - m_new) * own[u]);
+        m = m_new;
+      }
     }
     for (int z = 0; z < p.Z; ++z) n_out[z * DK + k] = n;
     for (int z = k; z < p.Z; z += DK) p.m_state[((size_t)slot * a.H + h) * p.Z + z] = m;
   }
-  static __device__ __forceinline__ void output_weights(const Params& p, const ChunkScanArgs& a, Scratch& sc, int h, const ChunkPlace& at) {
-    if (threadIdx.x < 32) {
-      double F[2], g[2];
-      float ii[2];
-      gate_sums(p, a, h, at, F, g, ii);
-      const double m0 = (double)a.ws_row[((size_t)blockIdx.x * a.H + h) * a.ws_row_width + a.ws_row_width - 2];
+  static __device__ __forceinline__ void output_weights(const Params& p, const ChunkScanArgs& a, Scratch& sc, int h, const ChunkPlace& at, int chunk) {
+    double F, g;
+    float ii;
+    gate_sums(p, a, sc, h, at, F, g, ii);
+    const double m0 = (double)a.ws_row[((size_t)chunk * a.H + h) * a.ws_row_width + a.ws_row_width - 2];
+    const int t = ct_team_row();
+    const double gm = fmax(m0, g), from = (double)ii - F;            // m_t - F_t
+    const float m = (float)(F + gm);
+    sc.m[t] = m;
+    sc.from[t] = ct_exp(from);
+    sc.to[t] = ct_exp(F - (double)m);
+    sc.aq[t] = expf((float)(m0 - gm));
+    double top = from;
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int t = 2 * threadIdx.x + e;
-        const double gm = fmax(m0, g[e]);            // m_t - F_t
-        sc.F[t] = F[e];
-        sc.ii[t] = ii[e];
-        sc.m[t] = (float)(F[e] + gm);
-        sc.aq[t] = expf((float)(m0 - gm));
-      }
-    }
+    for (int o = 1; o < 16; o <<= 1) top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
+    sc.below[t] = expf((float)(from - top));
+    if ((t & 15) == 0) sc.top[t >> 4] = ct_exp(top);
   }
   static __device__ __forceinline__ float q_scale(const Params& p) { return p.qscale; }
-  static __device__ __forceinline__ float D(const Params&, const Scratch& sc, int t, int s) {
-    return expf((float)((sc.F[t] - sc.F[s]) + (double)(sc.ii[s] - sc.m[t])));
+  typedef CtExp Row;
+  static __device__ __forceinline__ Row row(const Params&, const Scratch& sc, int t) { return sc.to[t]; }
+  static __device__ __forceinline__ float D(const Params&, const Scratch& sc, const Row& r, int, int s) {
+    const CtExp f = sc.from[s];
+    return expf((r.h + f.h) + (r.l + f.l));
+  }
+  // of sixteen rows from s0 on; with all of them before row t (`before`) the exponent is cut at their largest, both parts of it <= 0
+  static __device__ __forceinline__ void weights(const Params& p, const Scratch& sc, const Row& r, int t, int s0, bool before, float (&d)[16]) {
+    if (before) {
+      const CtExp f = sc.top[s0 >> 4];
+      const float g = expf((r.h + f.h) + (r.l + f.l));
+#pragma unroll
+      for (int e = 0; e < 16; ++e) d[e] = g * sc.below[s0 + e];
+    } else {
+#pragma unroll
+      for (int e = 0; e < 16; ++e) d[e] = D(p, sc, r, t, s0 + e);
+    }
   }
   static __device__ __forceinline__ float aq(const Scratch& sc, int t) { return sc.aq[t]; }
-  // den_t = max(|n_t . q_t|, exp(-m_t)) + 1e-6, four threads per row
-  template <int DK>
-  static __device__ __forceinline__ void rows(const Params& p, const ChunkScanArgs& a, Scratch& sc, const float* qs, const float* A, int h, int n,
-                                              bool zero_start) {
-    const int t = threadIdx.x >> 2, part = threadIdx.x & 3;
-    float own = 0.f, old = 0.f;
-    for (int s = part * 4; s < kCsRows; s += 16) {
-      const float4 v = *reinterpret_cast<const float4*>(A + t * kCsAPitch + s);
-      if (s <= t) own += (v.x + v.y) + (v.z + v.w);
+  // o_t / den_t, den_t = max(|n_t . q_t|, exp(-m_t)) + 1e-6; den: the sums of a row's weighted scores in two halves, n_start . q_t
+  struct Finish {
+    float d, r;
+    __device__ __forceinline__ Finish(const Params& p, const ChunkScanArgs&, const Scratch& sc, int, int t, const float* den) {
+      const float nq = fmaf(sc.aq[t] * p.qscale, den[2 * kCtRows + t], den[t] + den[kCtRows + t]);
+      d = fmaxf(fabsf(nq), expf(-sc.m[t])) + 1e-6f;
+      r = 1.0f / d;
     }
-    if (!zero_start) {
-      const float* row = row_of(a, blockIdx.x, h, DK);
-      for (int k = part * 4; k < DK; k += 16) {
-        const float4 u = *reinterpret_cast<const float4*>(row + k), q = *reinterpret_cast<const float4*>(qs + t * (DK + 4) + k);
-        old = fmaf(u.x, q.x, fmaf(u.y, q.y, fmaf(u.z, q.z, fmaf(u.w, q.w, old))));
+    // a quotient by its reciprocal and its remainder (P. Markstein, 1990); out of the range in which both are normal, the operator's
+    __device__ __forceinline__ void apply(float (&f)[16], const void*, int) const {
+      bool in_range = d < kDivRange;
+#pragma unroll
+      for (int c = 0; c < 16; ++c) in_range = in_range && fabsf(f[c]) < kDivRange;
+      if (in_range) {
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+          const float q = f[c] * r;
+          f[c] = fmaf(fmaf(-d, q, f[c]), r, q);
+        }
+      } else {
+#pragma unroll
+        for (int c = 0; c < 16; ++c) f[c] = f[c] / d;
       }
     }
-    own = fmaf(sc.aq[t] * p.qscale, old, own);
-    own += __shfl_xor_sync(0xffffffffu, own, 1);
-    own += __shfl_xor_sync(0xffffffffu, own, 2);
-    if (part == 0) sc.den[t] = fmaxf(fabsf(own), expf(-sc.m[t])) + 1e-6f;
-  }
-  static __device__ __forceinline__ float4 finish(const Params&, const Scratch& sc, int, int t, float4 v, float4) {
-    const float d = sc.den[t];
-    return make_float4(v.x / d, v.y / d, v.z / d, v.w / d);
-  }
+  };
 };
 
 // one warp per (token, head), 8 warps per CTA: o / rms(o) * w * sigmoid(gate); the head is read once
@@ -913,11 +904,11 @@ static int launch_chunks(const void* proj, int64_t ld, int q_col, int k_col, int
     if (rc != B200_OK) return rc;
   }
   const ChunkScanArgs a{proj, ld, q_col, k_col, v_col, H, H, dv, cu_seq, ctx_lens, state_slots, n_seq, short_rows, S_state, o_raw};
-  return cs_launch<TA, MlstmForm>(a, {gates, (const bf16*)gate_bias, cap, qscale, n_state, m_state, b200_mlstm_state_slices(dv)}, dk, rows,
+  return ct_launch<TA, MlstmForm>(a, {gates, (const bf16*)gate_bias, cap, qscale, n_state, m_state, b200_mlstm_state_slices(dv)}, dk, rows,
                                   workspace, s);
 }
 
-// The same with a workspace (chunk_scan.cuh): sequences of more than 16 rows run with all their chunks side by side, the others
+// The same with a workspace (chunk_tc.cuh): sequences of more than 16 rows run with all their chunks side by side, the others
 // one-pass beside them.  Shapes and alignments that the chunk kernels do not take run as b200_mlstm_scan.
 extern "C" int b200_mlstm_scan_chunked(const void* proj, int f32, int64_t ld, int q_col, int k_col, int v_col, const float* gates,
                                        const void* gate_bias, const int32_t* cu_seq, const int32_t* ctx_lens,
