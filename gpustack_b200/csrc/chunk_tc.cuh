@@ -14,10 +14,10 @@
 // its full size.  Relative errors against 64 bits of 4 x 2048 rows of linear attention: state 2.3e-7 by fp32 FMAs, 1.3e-7 here; of
 // mLSTM over fp32 rows: outputs 2.1e-7 and 1.3e-7.
 // Why: the same sums by fp32 FMAs were bound by the FMA pipe and by shared-memory reads (mLSTM, 7 ragged prompts of 7919 rows, 8 heads of
-// 128 x 128: state 70, carry 68, output 135 us; here 26, 17 and 54 us.  Linear attention over fp32 rows, 4 x 2048: 62, 44, 104 us; here
-// 38, 12, 69).  Chunks of 128 rows are the matrix instructions' own height and halve the chunks' states.  What bounds it: the chain of
+// 128 x 128: state 70, carry 68, output 135 us; here 30, 18 and 52 us.  Linear attention over fp32 rows, 4 x 2048: 62, 44, 104 us; here
+// 35, 12, 66).  Chunks of 128 rows are the matrix instructions' own height and halve the chunks' states.  What bounds it: the chain of
 // an item -- keys converted, scores, the state's part, values converted, their part -- beside a few hundred cycles for every
-// conversion, copy and wait in it.
+// conversion, copy and wait in it (8 converting warps instead of 16, 16 columns of the output per store: 39, 12, 69 us).
 #pragma once
 #include <type_traits>
 
@@ -28,10 +28,10 @@
 namespace b200 {
 
 constexpr int kCtRows = 128, kCtHalf = 64;
-// one CTA per SM walks the items: 8 warps convert operands, 8 read tensor memory (and form the items' weights), one issues the
+// one CTA per SM walks the items: 16 warps convert operands, 8 read tensor memory (and form the items' weights), one issues the
 // products, one copies the chunks' first states, one finds the items
-constexpr int kCtConvWarps = 8, kCtReadWarps = 8, kCtConv = kCtConvWarps * 32, kCtMma = kCtConvWarps + kCtReadWarps, kCtCopy = kCtMma + 1,
-              kCtFind = kCtCopy + 1, kCtThreads = (kCtFind + 1) * 32;
+constexpr int kCtConvWarps = 16, kCtReadWarps = 8, kCtConv = kCtConvWarps * 32, kCtMma = kCtConvWarps + kCtReadWarps, kCtCopy = kCtMma + 1,
+              kCtFind = kCtCopy + 1, kCtThreads = (kCtFind + 2) * 32;
 constexpr int kCtCarryThreads = 256, kCtDepth = 8, kCtTable = 32;      // chunks in flight in the carry; chunks per table of factors
 
 // ------------------------------------------------------------------------------------------- operands
@@ -54,14 +54,14 @@ __device__ __forceinline__ bool ct_finite(float x) { return fabsf(x) < 3.38e38f;
 // another.  Blocks one below the other are a panel of more rows, blocks side by side more panels; the same bytes serve as a K-major
 // operand (rows x columns) and as an MN-major one (columns x rows).
 //
-// Two blocks on their way from global memory through a converting thread's registers: columns c .. c + 3 of rows r, r + 16, ...
+// Two blocks on their way from global memory through a converting thread's registers: columns c .. c + 3 of rows r and r + 32
 template <typename TA>
 struct CtBlocks {
   static constexpr bool kExact = sizeof(TA) == 2;
   typedef typename std::conditional<kExact, uint2, float4>::type Raw;
-  Raw raw[2][4];
+  Raw raw[2][2];
   __device__ __forceinline__ static int column() { return ((int)threadIdx.x & 15) * 4; }
-  __device__ __forceinline__ static int row() { return ((int)threadIdx.x >> 4) & 15; }
+  __device__ __forceinline__ static int row() { return ((int)threadIdx.x >> 4) & 31; }
   // block 1 begins `next` numbers behind block 0; rows and columns that are not there are zeros
   __device__ __forceinline__ void load(const TA* src, int64_t ld, int64_t next, int rows0, int rows1, int cols0, int cols1) {
     const TA* at = src + (int64_t)row() * ld + column();
@@ -69,9 +69,9 @@ struct CtBlocks {
     for (int u = 0; u < 2; ++u) {
       const int left = column() < (u ? cols1 : cols0) ? (u ? rows1 : rows0) - row() : 0;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+      for (int i = 0; i < 2; ++i) {
         raw[u][i] = Raw{};
-        if (16 * i < left) raw[u][i] = *reinterpret_cast<const Raw*>(at + u * next + (int64_t)(16 * i) * ld);
+        if (32 * i < left) raw[u][i] = *reinterpret_cast<const Raw*>(at + u * next + (int64_t)(32 * i) * ld);
       }
     }
   }
@@ -86,14 +86,14 @@ struct CtBlocks {
     } else {
       uint32_t low = 0;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float4 v = raw[i >> 2][i & 3];
+      for (int i = 0; i < 4; ++i) {
+        const float4 v = raw[i >> 1][i & 1];
         low |= __float_as_uint(v.x) | __float_as_uint(v.y) | __float_as_uint(v.z) | __float_as_uint(v.w);
       }
       return (low & 0xffffu) == 0;
     }
   }
-  // where this thread's part of a block lies (row + 16 is 2 KB on, the next block 8 KB)
+  // where this thread's part of a block lies (row + 32 is 4 KB on, the next block 8 KB)
   __device__ __forceinline__ static uint32_t place() {
     const int r = row(), c = column();
     return (uint32_t)(r * 128 + (((c >> 3) ^ (r & 7)) << 4) + ((c >> 2) & 1) * 8);
@@ -114,8 +114,8 @@ __device__ __forceinline__ void ct_store(const CtBlocks<TA>& b, int blocks, uint
   for (int u = 0; u < 2; ++u) {
     if (u >= blocks) break;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint32_t to = at + u * kCtBlock + i * 2048;
+    for (int i = 0; i < 2; ++i) {
+      const uint32_t to = at + u * kCtBlock + i * 4096;
       if constexpr (CtBlocks<TA>::kExact) ct_st8(to, b.raw[u][i].x, b.raw[u][i].y);
       else if (one_term) ct_st8(to, ct_high(b.raw[u][i].x, b.raw[u][i].y), ct_high(b.raw[u][i].z, b.raw[u][i].w));
       else ct_put(to, term_bytes, b.raw[u][i]);
@@ -234,6 +234,13 @@ __device__ __forceinline__ bool ct_named_all(int id, int threads, bool v) {
                : "memory");
   return r != 0;
 }
+// A warpgroup's share of the registers that the block was launched with (28 warps of 72): 16 converting warps of 64, 8 reading ones of 88,
+// 4 others of 72.
+template <int N>
+__device__ __forceinline__ void ct_more_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void ct_fewer_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+constexpr int kCtConvRegs = 64, kCtReadRegs = 88;
 constexpr int kCtBarConv = 1, kCtBarRead = 2, kCtBarTeam = 3, kCtBarTerms = 4;      // named barriers
 
 // The first four reading warps form an item's weights, a row each: inclusive sums and running maxima over the rows (`parts`: four
@@ -325,7 +332,7 @@ struct CtSmem {
   // state: two halves of 64 rows of keys and of weighted values.  With 64 keys the instruction's other 64 rows read on into what
   // follows and go nowhere.
   static constexpr int kStateK = kIn * DK * 128, kStateV = 3 * VT * 128, kStateHalf = kStateK + kStateV;
-  static constexpr int kSums = 16 * DK * 4;
+  static constexpr int kSums = 32 * DK * 4;
   static constexpr int kState = 2 * kStateHalf + kSums + 1024;
   // output: panels of 64 columns of Q and K, of S, halves of 64 rows of V.  Three terms: two regions of two stages that change roles
   // with every item, Q's and then V's, K's and then S's
@@ -384,6 +391,7 @@ ct_state_kernel(const ChunkScanArgs a, const typename Form::Params p, int items)
   }
   const uint32_t tmem = ct_tmem(&tmem_at, 4 * VT);
   if (warp < kCtConvWarps) {
+    ct_fewer_registers<kCtConvRegs>();
     float* sums = reinterpret_cast<float*>(ct_align(ct_raw) + 2 * L::kStateHalf);
     typedef CtBlocks<TA> Blocks;
     Blocks kt, vt;
@@ -413,20 +421,20 @@ ct_state_kernel(const ChunkScanArgs a, const typename Form::Params p, int items)
           if (tid == 0) one_term[e] = one;
           const uint32_t at = ks + Blocks::place();
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float w = one ? sc.w[kCtHalf * e + kt.row() + 16 * i] : 1.f;
+          for (int i = 0; i < 2; ++i) {
+            const float w = one ? sc.w[kCtHalf * e + kt.row() + 32 * i] : 1.f;
 #pragma unroll
             for (int u = 0; u < DK / 64; ++u) {
               float4 k = kt.value(u, i);
               k = make_float4(k.x * w, k.y * w, k.z * w, k.w * w);
-              ct_put(at + u * kCtBlock + i * 2048, DK * 128, k);
+              ct_put(at + u * kCtBlock + i * 4096, DK * 128, k);
             }
           }
         }
         if constexpr (Form::kNorm) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float w = sc.w[kCtHalf * e + kt.row() + 16 * i];
+          for (int i = 0; i < 2; ++i) {
+            const float w = sc.w[kCtHalf * e + kt.row() + 32 * i];
 #pragma unroll
             for (int u = 0; u < DK / 64; ++u) {
               const float4 k = kt.value(u, i);
@@ -441,13 +449,13 @@ ct_state_kernel(const ChunkScanArgs a, const typename Form::Params p, int items)
         } else {
           const uint32_t at = vs + Blocks::place();
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float w = sc.w[kCtHalf * e + vt.row() + 16 * i];
+          for (int i = 0; i < 2; ++i) {
+            const float w = sc.w[kCtHalf * e + vt.row() + 32 * i];
 #pragma unroll
             for (int u = 0; u < VT / 64; ++u) {
               float4 v = vt.value(u, i);
               v = make_float4(v.x * w, v.y * w, v.z * w, v.w * w);
-              ct_put(at + u * kCtBlock + i * 2048, VT * 128, v);
+              ct_put(at + u * kCtBlock + i * 4096, VT * 128, v);
             }
           }
         }
@@ -460,10 +468,10 @@ ct_state_kernel(const ChunkScanArgs a, const typename Form::Params p, int items)
           for (int u = 0; u < DK / 64; ++u) *reinterpret_cast<float4*>(sums + kt.row() * DK + 64 * u + kt.column()) = ksum[u];
           ct_named_barrier(kCtBarConv, kCtConv);
           if (tid < DK) {
-            float n = 0.f;
-#pragma unroll
-            for (int g = 0; g < 16; ++g) n += sums[g * DK + tid];
-            row[tid] = n;
+            double n = 0.0;                           // (fp32 sums of 32 groups are further off than the one-pass form's)
+#pragma unroll 8
+            for (int g = 0; g < 32; ++g) n += (double)sums[g * DK + tid];
+            row[tid] = (float)n;
           }
           ct_named_barrier(kCtBarConv, kCtConv);
         }
@@ -473,6 +481,7 @@ ct_state_kernel(const ChunkScanArgs a, const typename Form::Params p, int items)
       now = then;
     }
   } else if (warp < kCtConvWarps + kCtReadWarps) {
+    ct_more_registers<kCtReadRegs>();
     // lane = key, columns = values: a warp stores two 64-byte pieces of a row
     const int w = warp - kCtConvWarps, k = (w & 3) * 32 + lane;
     const size_t plane = ct_plane(DK, a.dv);
@@ -665,6 +674,7 @@ ct_output_kernel(const ChunkScanArgs a, const typename Form::Params p, int items
   const uint32_t t_s = ct_tmem(&tmem_at, 512), t_o = t_s + 256;      // two accumulators of scores, later the weights' terms; the state's part, the values'
   auto from_state = [](const CtItem& w) { return w.at.local > 0 || !w.fresh; };
   if (warp < kCtConvWarps) {
+    ct_fewer_registers<kCtConvRegs>();
     // an item's tiles in their order: NP panels of queries, NP of keys, two halves of values; one is on its way while another is stored
     typedef CtBlocks<TA> Blocks;
     constexpr int TILES = 2 * NP + 2;
@@ -683,7 +693,7 @@ ct_output_kernel(const ChunkScanArgs a, const typename Form::Params p, int items
     if (now.item < items) load(tiles[0], now, 0);
     for (int it = 0; now.item < items; ++it) {
       CtItem then{items};
-      float old[8];                                   // kNorm: n_start . q of a thread's rows
+      float old[4];                                   // kNorm: n_start . q of a thread's rows
 #pragma unroll 1
       for (int i0 = 0; i0 < TILES; i0 += 2) {
 #pragma unroll
@@ -704,16 +714,16 @@ ct_output_kernel(const ChunkScanArgs a, const typename Form::Params p, int items
               if (start)
                 n = *reinterpret_cast<const float4*>(a.ws_row + ((size_t)now.chunk * a.H + now.h) * a.ws_row_width + 64 * i + tile.column());
 #pragma unroll
-              for (int r = 0; r < 8; ++r) {
-                const float4 q = tile.value(r >> 2, r & 3);
+              for (int r = 0; r < 4; ++r) {
+                const float4 q = tile.value(r >> 1, r & 1);
                 old[r] = start ? fmaf(q.x, n.x, fmaf(q.y, n.y, fmaf(q.z, n.z, fmaf(q.w, n.w, i ? old[r] : 0.f)))) : 0.f;
               }
               if (i == NP - 1) {
 #pragma unroll
-                for (int r = 0; r < 8; ++r) {
+                for (int r = 0; r < 4; ++r) {
 #pragma unroll
                   for (int o = 8; o > 0; o >>= 1) old[r] += __shfl_xor_sync(0xffffffffu, old[r], o);
-                  if ((tid & 15) == 0) den_of[it & 1][2 * kCtRows + 64 * (r >> 2) + 16 * (r & 3) + tile.row()] = old[r];
+                  if ((tid & 15) == 0) den_of[it & 1][2 * kCtRows + 64 * (r >> 1) + 32 * (r & 1) + tile.row()] = old[r];
                 }
               }
             }
@@ -722,15 +732,15 @@ ct_output_kernel(const ChunkScanArgs a, const typename Form::Params p, int items
             const int e = i - 2 * NP;
             // values that are no finite bf16 number are left out (zero times one would reach the rows before) and noted
 #pragma unroll
-            for (int r = 0; r < 8; ++r) {
-              const float4 v = tile.value(r >> 2, r & 3);
+            for (int r = 0; r < 4; ++r) {
+              const float4 v = tile.value(r >> 1, r & 1);
               if (!(ct_finite(v.x) && ct_finite(v.y) && ct_finite(v.z) && ct_finite(v.w))) {
-                const int at = kCtHalf * e + tile.row() + 16 * (r & 3);
+                const int at = kCtHalf * e + tile.row() + 32 * (r & 1);
                 atomicOr(&special[it % kCtAhead][at >> 5], 1u << (at & 31));
                 const float4 f = make_float4(ct_finite(v.x) ? v.x : 0.f, ct_finite(v.y) ? v.y : 0.f, ct_finite(v.z) ? v.z : 0.f,
                                              ct_finite(v.w) ? v.w : 0.f);
-                if constexpr (Blocks::kExact) tile.raw[r >> 2][r & 3] = make_uint2(pack_bf16(f.x, f.y), pack_bf16(f.z, f.w));
-                else tile.raw[r >> 2][r & 3] = f;
+                if constexpr (Blocks::kExact) tile.raw[r >> 1][r & 1] = make_uint2(pack_bf16(f.x, f.y), pack_bf16(f.z, f.w));
+                else tile.raw[r >> 1][r & 1] = f;
               }
             }
             if (!L::kApart && e == 0) ct_wait(&state_done, it);        // the queries are used
@@ -746,18 +756,22 @@ ct_output_kernel(const ChunkScanArgs a, const typename Form::Params p, int items
       now = then;
     }
   } else if (warp < kCtConvWarps + kCtReadWarps) {
+    ct_more_registers<kCtReadRegs>();
     const int w0 = warp - kCtConvWarps, t = (w0 & 3) * 32 + lane, part = w0 >> 2;      // a thread's row and half of the columns
     const uint32_t lane_off = (uint32_t)((w0 & 3) * 32) << 16;
     const float q_scale = Form::q_scale(p);
-    float* turn = reinterpret_cast<float*>(ct_align(ct_raw) + L::kOperands + w0 * 2048);   // 16 columns of 32 rows on their way to whole lines
-    for (int it = 0;; ++it) {
-      const CtItem now = ct_item(queue, it);
-      if (now.item >= items) break;
-      typename Form::Scratch& sc = scratch[it & 1];
+    float* turn = reinterpret_cast<float*>(ct_align(ct_raw) + L::kOperands + w0 * 2048);   // 32 columns of 16 rows on their way to whole lines
+    // an item ahead, while the values' part of the one before is formed
+    auto weigh = [&](const CtItem& next, int it) {
+      if (w0 < kCtTeam / 32 && next.item < items) Form::output_weights(p, a, scratch[it & 1], next.h, next.at, next.chunk);
+    };
+    CtItem now = ct_item(queue, 0);
+    weigh(now, 0);
+    for (int it = 0; now.item < items; ++it) {
+      const typename Form::Scratch& sc = scratch[it & 1];
       const int n = now.at.rows, h = now.h;
       float* den = den_of[it & 1];
-      if (w0 < kCtTeam / 32) Form::output_weights(p, a, sc, h, now.at, now.chunk);
-      ct_named_barrier(kCtBarRead, kCtReadWarps * 32);
+      ct_named_barrier(kCtBarRead, kCtReadWarps * 32);                // the weights are there, the item before is behind every warp
       const typename Form::Row row = Form::row(p, sc, t);
       ct_wait(&score_done, it);
       // sixteen scores at a time become three terms of eight columns, in columns of their own that have been read
@@ -799,10 +813,13 @@ ct_output_kernel(const ChunkScanArgs a, const typename Form::Params p, int items
       if constexpr (Form::kNorm) den[part * kCtRows + t] = own;
       tmem_st_wait();
       tc_fence_before();
-      ct_arrive(&weight_full);
-      if constexpr (Form::kNorm) ct_named_barrier(kCtBarRead, kCtReadWarps * 32);      // both halves' sums
+      // (before the products of this item can end, behind which the next item's values arrive: what was noted about these is seen)
       mbar_wait_guarded(&value_full[0], it & 1);
       mbar_wait_guarded(&value_full[1], it & 1);
+      ct_arrive(&weight_full);
+      const CtItem then = ct_item(queue, it + 1);
+      weigh(then, it + 1);
+      if constexpr (Form::kNorm) ct_named_barrier(kCtBarRead, kCtReadWarps * 32);      // both halves' sums
       const uint32_t* sp = special[it % kCtAhead];
       const bool odd = (sp[0] | sp[1] | sp[2] | sp[3]) != 0, live = t < n, start = from_state(now);
       const float f = start ? Form::aq(sc, t) * q_scale : 0.f;
@@ -811,15 +828,18 @@ ct_output_kernel(const ChunkScanArgs a, const typename Form::Params p, int items
       const TA* my_v = vx + (size_t)(now.at.first + (live ? t : 0)) * a.ld_v + a.v_col + h * a.dv;
       ct_wait(&value_done, it);
 #pragma unroll 1
-      for (int c0 = 0; c0 < OC; c0 += 16) {
+      for (int c0 = 0; c0 < OC; c0 += 32) {
         const int v = now.v0 + part * OC + c0;
-        uint32_t r[16], r1[16];
-        tmem_ld_32x16(t_o + VT + lane_off + part * OC + c0, r);
-        tmem_ld_32x16(t_o + lane_off + part * OC + c0, r1);
-        tmem_ld_wait();
-        float o[16];
+        float o[32];
 #pragma unroll
-        for (int e = 0; e < 16; ++e) o[e] = start ? fmaf(__uint_as_float(r1[e]), f, __uint_as_float(r[e])) : __uint_as_float(r[e]);
+        for (int b = 0; b < 2; ++b) {
+          uint32_t r[16], r1[16];
+          tmem_ld_32x16(t_o + VT + lane_off + part * OC + c0 + 16 * b, r);
+          tmem_ld_32x16(t_o + lane_off + part * OC + c0 + 16 * b, r1);
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 16; ++e) o[16 * b + e] = start ? fmaf(__uint_as_float(r1[e]), f, __uint_as_float(r[e])) : __uint_as_float(r[e]);
+        }
         if (odd && live) {
           const int g = h / (a.H / a.G) * DK;
 #pragma unroll 1
@@ -829,29 +849,34 @@ ct_output_kernel(const ChunkScanArgs a, const typename Form::Params p, int items
             const float ps = Form::D(p, sc, row, t, s) *
                              (ct_dot(mine + a.q_col + g, x + (size_t)(now.at.first + s) * a.ld + a.k_col + g, DK) * q_scale);
 #pragma unroll
-            for (int e = 0; e < 16; ++e)
+            for (int e = 0; e < 32; ++e)
               if (v + e < a.dv && !ct_finite((float)vr[e])) o[e] = fmaf(ps, (float)vr[e], o[e]);
           }
         }
         if (live) finish.apply(o, my_v + v, a.dv - v);
-        // four lanes store 64 bytes of a row, eight rows at a time
-        __syncwarp();
+        // sixteen rows at a time: eight lanes store a line of a row
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
-          *reinterpret_cast<float4*>(turn + lane * 16 + ((e ^ (lane >> 1)) & 3) * 4) = make_float4(o[4 * e], o[4 * e + 1], o[4 * e + 2], o[4 * e + 3]);
-        __syncwarp();
-        const int col = v + 4 * (lane & 3);
-        float* out = a.o + (size_t)(now.at.first + (w0 & 3) * 32) * a.H * a.dv + h * a.dv + col;
+        for (int b = 0; b < 2; ++b) {
+          __syncwarp();
+          if (lane >> 4 == b)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int r_ = 8 * e + (lane >> 2);
-          if ((w0 & 3) * 32 + r_ < n && col < a.dv)
-            *reinterpret_cast<float4*>(out + (size_t)r_ * a.H * a.dv) = *reinterpret_cast<const float4*>(turn + r_ * 16 + ((lane ^ (r_ >> 1)) & 3) * 4);
+            for (int e = 0; e < 8; ++e)
+              *reinterpret_cast<float4*>(turn + (lane & 15) * 32 + ((e ^ lane) & 7) * 4) = make_float4(o[4 * e], o[4 * e + 1], o[4 * e + 2], o[4 * e + 3]);
+          __syncwarp();
+          const int col = v + 4 * (lane & 7);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int r_ = 4 * e + (lane >> 3), row_ = (w0 & 3) * 32 + 16 * b + r_;
+            if (row_ < n && col < a.dv)
+              *reinterpret_cast<float4*>(a.o + (size_t)(now.at.first + row_) * a.H * a.dv + h * a.dv + col) =
+                  *reinterpret_cast<const float4*>(turn + r_ * 32 + ((lane ^ r_) & 7) * 4);
+          }
         }
       }
       tc_fence_before();
       ct_arrive(&out_free);
       ct_arrive(&queue.free[it % kCtAhead]);
+      now = then;
     }
   } else if (warp == kCtMma) {
     if (lane == 0) {

@@ -782,19 +782,19 @@ struct MlstmForm {
       r = 1.0f / d;
     }
     // a quotient by its reciprocal and its remainder (P. Markstein, 1990); out of the range in which both are normal, the operator's
-    __device__ __forceinline__ void apply(float (&f)[16], const void*, int) const {
+    __device__ __forceinline__ void apply(float (&f)[32], const void*, int) const {
       bool in_range = d < kDivRange;
 #pragma unroll
-      for (int c = 0; c < 16; ++c) in_range = in_range && fabsf(f[c]) < kDivRange;
+      for (int c = 0; c < 32; ++c) in_range = in_range && fabsf(f[c]) < kDivRange;
       if (in_range) {
 #pragma unroll
-        for (int c = 0; c < 16; ++c) {
+        for (int c = 0; c < 32; ++c) {
           const float q = f[c] * r;
           f[c] = fmaf(fmaf(-d, q, f[c]), r, q);
         }
       } else {
 #pragma unroll
-        for (int c = 0; c < 16; ++c) f[c] = f[c] / d;
+        for (int c = 0; c < 32; ++c) f[c] = f[c] / d;
       }
     }
   };
