@@ -349,7 +349,7 @@ struct CtSmem {
   __device__ __forceinline__ static uint32_t v(int it, int i) { return kApart ? 4 * kStage + i * kStage : q(it, i); }
 };
 __device__ __forceinline__ uint8_t* ct_align(uint8_t* p) {
-  return reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(p) + 1023) & ~static_cast<uintptr_t>(1023));
+  return p + (-smem_u32(p) & 1023u);                  // (by an offset: the compiler still sees shared memory)
 }
 
 // ------------------------------------------------------------------------------------------- workspace
