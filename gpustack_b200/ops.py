@@ -632,6 +632,8 @@ def mlstm_state_slices(dv: int) -> int:
 # rows 114 -> 126, of 128 rows 201 -> 132; gated linear attention of 256 rows 47 -> 50, of 512 84 -> 52, 16 of 128 rows 70 -> 83, of
 # 1024 rows 433 -> 390, one of 2048 beside thirty of 16 449 -> 108; state space of 32 heads: 1024 rows 109 -> 87, 2048 rows
 # 207 -> 140, 16 of 512 rows 399 -> 532, one of 2048 beside thirty of 16 477 -> 195.
+# (Linear attention's and mLSTM's chunks were 64 rows by FMAs then; of 128 rows on the tensor cores since, they take no longer at any of
+# these steps -- linear attention of 128 rows 38 -> 36, mLSTM of 16 portions of 128 rows 101 -> 49 -- so a step that went to them still does.)
 ChunkCosts = collections.namedtuple("ChunkCosts", "width one_fixed one_row one_work chunk_fixed chunk_work wasted")
 CHUNK_COSTS = {"linear": ChunkCosts(128 * 128, 10.0, 0.37, 6.8, 36.0, 3.0, 0), "mlstm": ChunkCosts(128 * 128, 10.0, 0.36, 8.5, 60.0, 2.6, 32),
                "gated_linear": ChunkCosts(64 * 128, 8.0, 0.146, 2.0, 44.0, 1.8, 0),
@@ -639,7 +641,7 @@ CHUNK_COSTS = {"linear": ChunkCosts(128 * 128, 10.0, 0.37, 6.8, 36.0, 3.0, 0), "
 
 
 def chunk_scan_pays(kind: str, rows: int, n_seqs: int, H: int, dk: int, dv: int, max_len: int) -> bool:
-    """Whether a step of `rows` rows in n_seqs sequences of at most max_len runs faster over chunks of 64 rows side by side.  A bound
+    """Whether a step of `rows` rows in n_seqs sequences of at most max_len runs faster over chunks side by side.  A bound
     of all rows of several sequences says nothing about one of them: they are taken for equal."""
     if dk not in (64, 128) or dv % 4:
         return False
@@ -653,7 +655,7 @@ def chunk_scan_pays(kind: str, rows: int, n_seqs: int, H: int, dk: int, dv: int,
 
 
 def _chunk_scan_workspace(kind: str, rows: int, n_seqs: int, H: int, dk: int, dv: int, max_len: int, device, workspace=None):
-    """Workspace of the scans that run a prompt portion's chunks of 64 rows side by side (the caller's, where it brings one), or
+    """Workspace of the scans that run a prompt portion's chunks side by side (the caller's, where it brings one), or
     None where the one-pass scans are the better ones, or the only ones (key widths the chunk kernels do not take, no room)."""
     if not chunk_scan_pays(kind, rows, n_seqs, H, dk, dv, max_len):
         return None
