@@ -3,7 +3,8 @@
 //
 // With a state S (dk x dv), rows t = 0 .. n-1 of a chunk of 64 and the weights that a recurrence's `Form` supplies:
 //     o_t = aq_t S_start^T q_t + sum_{s<=t} D(t, s) (k_s . q_t) v_s          S_end = a S_start + b sum_s w_s k_s v_s^T
-// Three launches:
+// State space and, with a decay per key channel, gated linear attention; mLSTM and linear attention run on the tensor cores
+// (chunk_tc.cuh).  Three launches:
 //   chunk_state   one CTA per (chunk, head, value tile): C = sum_s w_s k_s v_s^T into the workspace, [chunk][H][dk][dv]
 //   chunk_carry   one CTA per (8 keys x 128 values of the state, head, sequence): walks a sequence's chunks, puts S_start in C's
 //                 place and leaves the sequence's final state in its slot
