@@ -462,8 +462,8 @@ ct_state_kernel(const ChunkScanArgs a, const typename Form::Params p, int items)
         ct_stored(&half_full[e]);
       }
       if (now.v0 == 0) {
-        float* row = a.ws_row + ((size_t)now.chunk * a.H + now.h) * a.ws_row_width;
         if constexpr (Form::kNorm) {                  // the keys' own sum: a thread's rows, then the row groups
+          float* row = a.ws_row + ((size_t)now.chunk * a.H + now.h) * a.ws_row_width;
 #pragma unroll
           for (int u = 0; u < DK / 64; ++u) *reinterpret_cast<float4*>(sums + kt.row() * DK + 64 * u + kt.column()) = ksum[u];
           ct_named_barrier(kCtBarConv, kCtConv);
@@ -475,7 +475,6 @@ ct_state_kernel(const ChunkScanArgs a, const typename Form::Params p, int items)
           }
           ct_named_barrier(kCtBarConv, kCtConv);
         }
-        if (tid == 0) Form::state_row(row + DK, sc);
       }
       ct_arrive(&queue.free[it % kCtAhead]);
       now = then;
@@ -485,10 +484,12 @@ ct_state_kernel(const ChunkScanArgs a, const typename Form::Params p, int items)
     // lane = key, columns = values: a warp stores two 64-byte pieces of a row
     const int w = warp - kCtConvWarps, k = (w & 3) * 32 + lane;
     const size_t plane = ct_plane(DK, a.dv);
-    // an item ahead: its buffer's last item is converted once its sums are complete
+    // an item ahead: the last item of its buffer has used its weights once its sums are complete (they are all that the converting
+    // warps read of it; the chunk's row of factors goes to the workspace from here)
     auto weigh = [&](const CtItem& next, int it) {
       if (w >= kCtTeam / 32 || next.item >= items) return;
-      Form::state_weights(p, a, scratch[it & 1], next.h, next.at, next.fresh);
+      float* row = a.ws_row + ((size_t)next.chunk * a.H + next.h) * a.ws_row_width + DK;
+      Form::state_weights(p, a, scratch[it & 1], next.h, next.at, next.fresh, next.v0 == 0 ? row : nullptr);
       ct_arrive(&weight_full[it & 1]);
     };
     CtItem now = ct_item(queue, 0);

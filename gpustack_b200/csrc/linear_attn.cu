@@ -386,11 +386,10 @@ struct LinearForm {
   struct Scratch {
     float dp[kCtRows + 1], w[kCtRows];
   };
-  static __device__ __forceinline__ void state_weights(const Params& p, const ChunkScanArgs&, Scratch& sc, int h, const ChunkPlace& at, int) {
+  static __device__ __forceinline__ void state_weights(const Params& p, const ChunkScanArgs&, Scratch& sc, int h, const ChunkPlace& at, int, float*) {
     const int t = ct_team_row();
     sc.w[t] = t < at.rows ? la_power(p.decay[h], at.rows - 1 - t) : 0.f;
   }
-  static __device__ __forceinline__ void state_row(float*, const Scratch&) {}
   struct Carry {
     float d;
     __device__ __forceinline__ Carry(const Params& p, const ChunkScanArgs&, int h, int) : d(p.decay[h]) {}

@@ -642,7 +642,7 @@ struct MlstmForm {
       float below[kCtRows];                          // exp(i_s - F_s - top)
       float w[kCtRows];                              // (ct_state's)
     };
-    float m[kCtRows], aq[kCtRows], row[4];
+    float m[kCtRows], aq[kCtRows];
     double parts[9];
   };
   // a row per thread: log gates, F their running sum, g the running maximum of i_s - F_s
@@ -660,24 +660,22 @@ struct MlstmForm {
     F = ct_team_scan<false>(F, sc.parts);
     g = ct_team_scan<true>(t < at.rows ? (double)ii - F : -1.0e300, sc.parts + 4);
   }
-  static __device__ __forceinline__ void state_weights(const Params& p, const ChunkScanArgs& a, Scratch& sc, int h, const ChunkPlace& at, int fresh) {
+  static __device__ __forceinline__ void state_weights(const Params& p, const ChunkScanArgs& a, Scratch& sc, int h, const ChunkPlace& at, int fresh,
+                                                       float* row) {
     double F, g;
     float ii;
     gate_sums(p, a, sc, h, at, F, g, ii);
     const int t = ct_team_row();
     if (t == kCtRows - 1) {                          // rows behind the last one add nothing
       sc.parts[8] = g;
-      sc.row[0] = (float)F;
-      sc.row[1] = (float)(F + g);
-      sc.row[3] = at.local == 0 && !fresh ? p.m_state[((size_t)at.slot * a.H + h) * p.Z] : 0.f;
+      if (row != nullptr) {
+        row[0] = (float)F;
+        row[1] = (float)(F + g);
+        row[3] = at.local == 0 && !fresh ? p.m_state[((size_t)at.slot * a.H + h) * p.Z] : 0.f;
+      }
     }
     ct_named_barrier(kCtBarTeam, kCtTeam);
     sc.w[t] = t < at.rows ? expf((float)((double)ii - F - sc.parts[8])) : 0.f;
-  }
-  static __device__ __forceinline__ void state_row(float* row, const Scratch& sc) {
-    row[0] = sc.row[0];
-    row[1] = sc.row[1];
-    row[3] = sc.row[3];
   }
   struct Carry {
     const float* row;

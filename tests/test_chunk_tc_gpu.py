@@ -1,5 +1,5 @@
-"""Linear attention over chunks of 128 rows on the tensor cores against the recurrence in fp64: chunk edges, values that are bf16 numbers in
-all, some or none of a chunk's halves (one term or three), and more items than CTAs."""
+"""Linear attention and mLSTM over chunks of 128 rows on the tensor cores against the recurrences in fp64: chunk edges, values that are
+bf16 numbers in all, some or none of a chunk's halves (one term or three), and many items per CTA."""
 import pytest
 import torch
 
@@ -35,3 +35,47 @@ def test_edges_and_terms(lens, H, exact, dk, dv):
             want[t] = torch.einsum("hvk,hk->hv", Z, q[t])
         assert float((S_d[i].cpu().to(F64) - Z).norm() / Z.norm()) < TOL
     assert float((o.cpu().to(F64) - want.view(T, -1)).norm() / want.norm()) < TOL
+
+
+# chunks of 128 rows, 1, 48, 64 and 65 rows at a sequence's end, more chunks of one than a table of the carry holds (32)
+MANY = [4400, 129, 300, 17, 193, 640, 1, 128]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_mlstm_beyond_the_second_item_of_a_cta(dtype):
+    """Buffers of a CTA's items are used again from its third item on: eight items per CTA (148 of them) and more."""
+    from gpustack_b200 import ops
+    from oracle import vodavik_oracle as O
+
+    H, dk, dv, cap, n = 24, 128, 128, 6.0, len(MANY)
+    cu = [sum(MANY[:i]) for i in range(n + 1)]
+    T, Z = cu[-1], ops.mlstm_state_slices(dv)
+    g = torch.Generator().manual_seed(3)
+    proj = torch.randn(T, 2 * H * dk + H * dv, generator=g)
+    proj[:T // 2, 2 * H * dk:] = proj[:T // 2, 2 * H * dk:].bfloat16().float()
+    proj, gates = proj.to(dtype).cuda(), (torch.randn(T, 2 * H, generator=g) * 3.0).cuda()
+    bias = torch.cat([torch.randn(H, generator=g), 2 + torch.randn(H, generator=g)]).bfloat16().cuda()
+    S, nn, m = (torch.randn(n, H, *w, generator=g).cuda() for w in ((dv, dk), (1, dk), (1,)))
+    nn, m = nn.expand(n, H, Z, dk).contiguous(), m.abs().expand(n, H, Z).contiguous()
+    o, S_d, n_d, m_d = torch.zeros(T, H * dv, device="cuda"), S.clone(), nn.clone(), m.clone()
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")   # noqa: E731
+    ctx = [i % 2 for i in range(n)]
+    ops.mlstm_scan(proj, 0, H * dk, 2 * H * dk, gates, bias, i32(cu), i32(ctx), i32(list(range(n))), S_d, n_d, m_d, o, H, dk, dv, cap,
+                   max_len=max(MANY))
+    p = proj.to(F64)
+    q, k, v = p[:, :H * dk].view(T, H, dk) * dk ** -0.5, p[:, H * dk:2 * H * dk].view(T, H, dk), p[:, 2 * H * dk:].view(T, H, dv)
+    a = cap * torch.tanh((gates.to(F64) + bias.to(F64)) / cap)
+    li, lf = a[:, :H], torch.nn.functional.logsigmoid(a[:, H:])
+    for i in range(n):
+        rows = slice(cu[i], cu[i + 1])
+        state = (S[i].to(F64).transpose(1, 2), nn[i, :, 0].to(F64), m[i, :, 0].to(F64)) if ctx[i] else None
+        with torch.device("cuda"):
+            want, (Sw, nw, mw) = O.mlstm_scan(q[rows], k[rows], v[rows], li[rows], lf[rows], state)
+        Sw = Sw.transpose(1, 2)
+        # per head: one chunk's wrong factors are not lost among the others.  A log gate up to 6 in fp32, twice in an exponent, is 12 x 2^-24
+        # of a weight; a denominator |n . q| cancels, its error is of the size of the terms
+        for got, ref, tol in ((S_d[i], Sw, 17 * 2.0 ** -24), (n_d[i, :, 0], nw, 17 * 2.0 ** -24),
+                              (o[rows].view(-1, H, dv).transpose(0, 1), want.transpose(0, 1), 20 * TOL)):
+            err = (got.to(F64) - ref).flatten(1).norm(dim=1) / ref.flatten(1).norm(dim=1)
+            assert float(err.max()) < tol, (i, MANY[i])
+        assert bool((m_d[i].to(F64) - mw[:, None]).abs().max() < 17 * 2.0 ** -24 * mw.abs().max().clamp(min=6.0))

@@ -42,3 +42,12 @@ def test_routing_reads_earlier_outputs_past_l1(name):
         head, code = body.split("pdl_wait();", 1)
         for arg in set(re.findall(r"const (?:\w+)\s*\*\s*(?:__restrict__\s+)?(\w+)", head)) - {"correction", "router"}:
             assert not re.search(r"(?<![\w.])%s\[|[ (!]\*%s\b|(?<!_cg_)(?<!rb_)ld_v4\(%s\b" % (arg, arg, arg), code), (arg, body[:120])
+
+
+def test_chunk_weights_are_read_before_their_buffer_is_free():
+    """The state's converting warps read an item's weights only before they hand its last half over: behind that, the weights of the item
+    after next take the buffer's place."""
+    kernel = next(d for d in _definitions((CSRC / "chunk_tc.cuh").read_text()) if "ct_state_kernel" in d)
+    converting = kernel[kernel.index("if (warp < kCtConvWarps)"):kernel.index("else if (warp < kCtConvWarps + kCtReadWarps)")]
+    before, behind = converting.split("ct_stored(&half_full[e]);")
+    assert re.search(r"\bsc\.w\[", before) and not re.search(r"\b(sc|scratch)\b", behind)
