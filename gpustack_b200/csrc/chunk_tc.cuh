@@ -123,6 +123,32 @@ __device__ __forceinline__ void ct_store(const CtBlocks<TA>& b, int blocks, uint
   }
 }
 
+// An infinite number (or one that rounds to one) has no three terms: every product with it is no number, where an fp32 FMA may give an
+// infinite one.  What comes out of the products neither finite nor zero is formed again by FMAs: its place is told by adding up
+// zero times the results, which is zero for finite ones alone.
+struct CtFinite {
+  cs_f2 sum = 0ull;
+  __device__ __forceinline__ void add(float a, float b) { sum = cs_fma(cs_pack(a, b), 0ull, sum); }
+  __device__ __forceinline__ bool all() const {
+    const float2 v = cs_split(sum);
+    return v.x + v.y == 0.f;
+  }
+};
+__device__ __forceinline__ bool ct_number(float x) { return fabsf(x) < INFINITY; }
+// k . q; sum of w_s k_s v_s over rows, until it is no number; q times a row of the state's terms
+template <typename TA>
+__device__ __noinline__ float ct_dot(const TA* q, const TA* k, int dk) {
+  float acc = 0.f;
+  for (int i = 0; i < dk; ++i) acc = fmaf((float)q[i], (float)k[i], acc);
+  return acc;
+}
+template <typename TA>
+__device__ __noinline__ float ct_rows_sum(const TA* k, int64_t ld, const TA* v, int64_t ld_v, const float* w, int rows) {
+  float acc = 0.f;
+  for (int s = 0; s < rows && acc == acc; ++s) acc = fmaf((float)k[s * ld] * w[s], (float)v[s * ld_v], acc);
+  return acc;
+}
+
 // One pair of terms over KS steps of 16, or all pairs (i, j) of 1 <= i + j <= 2, smallest first: the low words of the descriptors
 // and their steps in 16-byte units; A's terms in shared memory (A_TMEM: in tensor memory, a_step columns per step).  One thread.
 template <bool A_TMEM, int KS>
@@ -497,6 +523,7 @@ ct_state_kernel(const ChunkScanArgs a, const typename Form::Params p, int items)
     for (int it = 0; now.item < items; ++it) {
       const int buf = it & 1;
       const CtItem then = ct_item(queue, it + 1);
+      ct_named_barrier(kCtBarRead, kCtReadWarps * 32);                // the item before, whose weights these replace, is behind every warp
       weigh(then, it + 1);
       mbar_wait_guarded(&sum_full[buf], (it >> 1) & 1);
       tc_fence_after();
@@ -506,17 +533,30 @@ ct_state_kernel(const ChunkScanArgs a, const typename Form::Params p, int items)
       const uint32_t t0 = tmem + ((uint32_t)((w & 3) * 32) << 16) + buf * 2 * VT + (w >> 2) * PER;
       if ((w & 3) * 32 < DK) {
 #pragma unroll 1
-        for (int c0 = 0; c0 < PER; c0 += 32) {
-          uint32_t r[32], s[32];
-          tmem_ld_32x32(t0 + c0, r);
-          tmem_ld_32x32(t0 + VT + c0, s);
+        for (int c0 = 0; c0 < PER; c0 += 16) {
+          uint32_t r[16], s[16];
+          tmem_ld_32x16(t0 + c0, r);
+          tmem_ld_32x16(t0 + VT + c0, s);
           tmem_ld_wait();
           uint8_t* out = C + ((k >> 2) & 1) * plane + (size_t)((k >> 6) * a.dv + v0 + c0) * 128 + (k & 3) * 4;
           const int k8 = (k >> 3) & 7;                // (v0 + c0 is a multiple of 8)
+          CtFinite finite;
 #pragma unroll
-          for (int c = 0; c < 32; ++c)
-            if (v0 + c0 + c < a.dv)
-              *reinterpret_cast<float*>(out + c * 128 + ((k8 ^ (c & 7)) << 4)) = __uint_as_float(r[c]) + __uint_as_float(s[c]);
+          for (int c = 0; c < 16; ++c) r[c] = __float_as_uint(__uint_as_float(r[c]) + __uint_as_float(s[c]));
+#pragma unroll
+          for (int c = 0; c < 16; c += 2) finite.add(__uint_as_float(r[c]), __uint_as_float(r[c + 1]));
+#pragma unroll
+          for (int c = 0; c < 16; ++c)
+            if (v0 + c0 + c < a.dv) *reinterpret_cast<uint32_t*>(out + c * 128 + ((k8 ^ (c & 7)) << 4)) = r[c];
+          if (!finite.all()) {
+#pragma unroll 1
+            for (int c = 0; c < 16 && v0 + c0 + c < a.dv; ++c) {
+              float* C_kv = reinterpret_cast<float*>(out + c * 128 + ((k8 ^ (c & 7)) << 4));
+              if (!ct_number(*C_kv))
+                *C_kv = ct_rows_sum(x + (int64_t)now.at.first * a.ld + a.k_col + now.h / (a.H / a.G) * DK + k, a.ld,
+                                    vx + (int64_t)now.at.first * a.ld_v + a.v_col + now.h * a.dv + v0 + c0 + c, a.ld_v, scratch[buf].w, now.at.rows);
+            }
+          }
         }
       }
       tc_fence_before();
@@ -632,10 +672,18 @@ ct_carry_kernel(const ChunkScanArgs a, const typename Form::Params p) {
 // ------------------------------------------------------------------------------------------- output
 // Values that are no finite bf16 number are left out of the products (zero times one would reach the rows before) and join the rows
 // from their own on one by one.
+//
+// q . a value's row of the state's terms in the workspace, until it is no number
 template <typename TA>
-__device__ __noinline__ float ct_dot(const TA* q, const TA* k, int dk) {
+__device__ __noinline__ float ct_state_dot(const TA* q, const uint8_t* S, size_t plane, int v, int dk, int dv) {
   float acc = 0.f;
-  for (int i = 0; i < dk; ++i) acc = fmaf((float)q[i], (float)k[i], acc);
+  for (int k = 0; k < dk && acc == acc; ++k) {
+    const uint8_t* at = S + ct_in_plane(v, k >> 3, dv) + (k & 7) * 2;
+    float x = __bfloat162float(*reinterpret_cast<const bf16*>(at));
+    if (ct_number(x))                                 // (behind an infinite first term stand none)
+      x += __bfloat162float(*reinterpret_cast<const bf16*>(at + plane)) + __bfloat162float(*reinterpret_cast<const bf16*>(at + 2 * plane));
+    acc = fmaf((float)q[k], x, acc);
+  }
   return acc;
 }
 
@@ -811,7 +859,16 @@ ct_output_kernel(const ChunkScanArgs a, const typename Form::Params p, int items
         tmem_st_32x8(at + 8, term[1]);
         tmem_st_32x8(at + 128, term[2]);
       }
-      if constexpr (Form::kNorm) den[part * kCtRows + t] = own;
+      if constexpr (Form::kNorm) {
+        if (!ct_number(own) && t < n) {               // an infinite key or query: scores by FMAs
+          const TA* qk = x + (size_t)now.at.first * a.ld + h / (a.H / a.G) * DK;
+          own = 0.f;
+#pragma unroll 1
+          for (int s = 64 * part; s < min(64 * part + 64, t + 1) && own == own; ++s)
+            own += Form::D(p, sc, row, t, s) * (ct_dot(qk + (size_t)t * a.ld + a.q_col, qk + (size_t)s * a.ld + a.k_col, DK) * q_scale);
+        }
+        den[part * kCtRows + t] = own;
+      }
       tmem_st_wait();
       tc_fence_before();
       // (before the products of this item can end, behind which the next item's values arrive: what was noted about these is seen)
@@ -841,6 +898,10 @@ ct_output_kernel(const ChunkScanArgs a, const typename Form::Params p, int items
 #pragma unroll
           for (int e = 0; e < 16; ++e) o[16 * b + e] = start ? fmaf(__uint_as_float(r1[e]), f, __uint_as_float(r[e])) : __uint_as_float(r[e]);
         }
+        CtFinite finite;
+#pragma unroll
+        for (int e = 0; e < 32; e += 2) finite.add(o[e], o[e + 1]);
+        const bool bad = live && !finite.all();
         if (odd && live) {
           const int g = h / (a.H / a.G) * DK;
 #pragma unroll 1
@@ -871,6 +932,39 @@ ct_output_kernel(const ChunkScanArgs a, const typename Form::Params p, int items
             if (row_ < n && col < a.dv)
               *reinterpret_cast<float4*>(a.o + (size_t)(now.at.first + row_) * a.H * a.dv + h * a.dv + col) =
                   *reinterpret_cast<const float4*>(turn + r_ * 32 + ((lane ^ r_) & 7) * 4);
+          }
+        }
+        if (__any_sync(0xffffffffu, bad)) {
+          __syncwarp();                               // (a row is written by eight lanes)
+          if (bad) {
+            const int g = h / (a.H / a.G) * DK;
+            const size_t plane = ct_plane(DK, a.dv);
+            const uint8_t* S = reinterpret_cast<const uint8_t*>(a.ws) + ((size_t)now.chunk * a.H + h) * 3 * plane;
+            float* to = a.o + (size_t)(now.at.first + t) * a.H * a.dv + h * a.dv + v;
+            uint32_t again = 0;                       // columns that may yet be numbers
+#pragma unroll 1
+            for (int e = 0; e < 32 && v + e < a.dv; ++e) {
+              if (ct_number(to[e])) continue;
+              const float z = start ? ct_state_dot(mine + a.q_col + g, S, plane, v + e, DK, a.dv) * f : 0.f;
+              to[e] = z;
+              again |= z == z ? 1u << e : 0u;
+            }
+#pragma unroll 1
+            for (int s = 0; s <= t && again; ++s) {
+              const TA* vr = vx + (size_t)(now.at.first + s) * a.ld_v + a.v_col + h * a.dv + v;
+              const float ps = Form::D(p, sc, row, t, s) *
+                               (ct_dot(mine + a.q_col + g, x + (size_t)(now.at.first + s) * a.ld + a.k_col + g, DK) * q_scale);
+              for (uint32_t m = again; m; m &= m - 1) {
+                const int e = __ffs(m) - 1;
+                const float z = fmaf(ps, (float)vr[e], to[e]);
+                to[e] = z;
+                if (z != z) again &= ~(1u << e);
+              }
+            }
+            for (; again; again &= again - 1) {
+              float* z = to + __ffs(again) - 1;
+              *z = finish.one(*z);
+            }
           }
         }
       }

@@ -417,6 +417,7 @@ struct LinearForm {
   struct Finish {
     __device__ __forceinline__ Finish(const Params&, const ChunkScanArgs&, const Scratch&, int, int, const float*) {}
     __device__ __forceinline__ void apply(float (&)[32], const void*, int) const {}
+    __device__ __forceinline__ float one(float f) const { return f; }
   };
 };
 

@@ -779,6 +779,7 @@ struct MlstmForm {
       d = fmaxf(fabsf(nq), expf(-sc.m[t])) + 1e-6f;
       r = 1.0f / d;
     }
+    __device__ __forceinline__ float one(float f) const { return f / d; }
     // a quotient by its reciprocal and its remainder (P. Markstein, 1990); out of the range in which both are normal, the operator's
     __device__ __forceinline__ void apply(float (&f)[32], const void*, int) const {
       bool in_range = d < kDivRange;

@@ -79,3 +79,59 @@ def test_mlstm_beyond_the_second_item_of_a_cta(dtype):
             err = (got.to(F64) - ref).flatten(1).norm(dim=1) / ref.flatten(1).norm(dim=1)
             assert float(err.max()) < tol, (i, MANY[i])
         assert bool((m_d[i].to(F64) - mw[:, None]).abs().max() < 17 * 2.0 ** -24 * mw.abs().max().clamp(min=6.0))
+
+
+@pytest.mark.parametrize("where", ["query", "key", "value", "state", "largest key", "largest value"])
+@pytest.mark.parametrize("kind,dtype", [("linear", torch.float32), ("mlstm", torch.float32), ("mlstm", torch.bfloat16)])
+@pytest.mark.parametrize("dk,dv", [(128, 128), (64, 36)])
+def test_infinite_numbers(where, kind, dtype, dk, dv):
+    """An infinite number, and one that is infinite as a bf16 number only, gives what fp32 arithmetic gives.  Numbers of one sign in every
+    column: no sum has infinities of both."""
+    from gpustack_b200 import ops
+    from oracle import vodavik_oracle as O
+
+    H, T, cap = 2, 300, 6.0
+    g = torch.Generator().manual_seed(dk)
+    q, k, v = (0.1 + 0.8 * torch.rand(T, H, w, generator=g) for w in (dk, dk, dv))
+    sign = torch.tensor([1.0, -1.0]).repeat(dv)[:dv]
+    v, S = v * sign, (0.1 + torch.rand(H, dv, dk, generator=g)) * sign[:, None]
+    n, m = 0.1 + torch.rand(H, 1, dk, generator=g), torch.zeros(H, 1)
+    if where == "query":
+        q[70, 1, 3] = float("inf")
+    elif where == "key":
+        k[70, 1, 3] = float("inf")
+    elif where == "value":
+        v[200, 1, 5] = -float("inf")
+    elif where == "state":
+        S[1, 7, 9] = -float("inf")
+    elif where == "largest key":
+        k[70, 1, 3], q[:, 1, 3] = 3.395e38, 1e-3
+    else:
+        v[200, 1, 5], k[200, 1] = -3.395e38, 1e-3
+    x = torch.cat([t.reshape(T, -1) for t in (q, k, v)], 1).to(dtype)
+    i32 = lambda t: torch.tensor(t, dtype=torch.int32, device="cuda")   # noqa: E731
+    idx, o, S_d = (i32([0, T]), i32([9]), i32([0])), torch.zeros(T, H * dv, device="cuda"), S[None].cuda()
+    q, k, v = (x[:, a:b].view(T, H, -1).to(F64) for a, b in ((0, H * dk), (H * dk, 2 * H * dk), (2 * H * dk, x.shape[1])))
+    more = []
+    if kind == "linear":
+        decay = torch.tensor([0.5, 0.98])
+        ops.linattn_scan(x.cuda(), 0, H * dk, 2 * H * dk, decay.cuda(), *idx, S_d, o, H, dk, dv, max_len=T)
+        Z, want = S.to(F64), torch.zeros(T, H, dv, dtype=F64)
+        for t in range(T):
+            Z = decay.to(F64)[:, None, None] * Z + v[t][:, :, None] * k[t][:, None]
+            want[t] = torch.einsum("hvk,hk->hv", Z, q[t])
+    else:
+        slices = ops.mlstm_state_slices(dv)
+        gates, bias = torch.randn(T, 2 * H, generator=g), torch.tensor([0.0, 0.0, 3.0, 5.0]).bfloat16()
+        n_d, m_d = n.expand(H, slices, dk)[None].contiguous().cuda(), m.expand(H, slices)[None].contiguous().cuda()
+        ops.mlstm_scan(x.cuda(), 0, H * dk, 2 * H * dk, gates.cuda(), bias.cuda(), *idx, S_d, n_d, m_d, o, H, dk, dv, cap, max_len=T)
+        a = cap * torch.tanh((gates.to(F64) + bias.to(F64)) / cap)
+        want, (Z, nw, _) = O.mlstm_scan(q * dk ** -0.5, k, v, a[:, :H], torch.nn.functional.logsigmoid(a[:, H:]),
+                                        (S.to(F64).transpose(1, 2), n[:, 0].to(F64), m[:, 0].to(F64)))
+        Z, more = Z.transpose(1, 2), [(n_d[0, :, 0], nw)]
+    for got, ref in [(o, want.reshape(T, -1)), (S_d[0], Z)] + more:
+        got = got.cpu().to(F64)
+        assert torch.equal(got.isnan(), ref.isnan()) and torch.equal(got == float("inf"), ref == float("inf"))
+        assert torch.equal(got == -float("inf"), ref == -float("inf"))
+        a, b = (t[ref.isfinite()] for t in (got, ref))
+        assert bool(((a - b).abs() <= TOL * b.abs()).all())
