@@ -300,6 +300,16 @@ __device__ __forceinline__ CtExp ct_exp(double v) {
   return {h, (float)(v - (double)h)};
 }
 
+// The launches of a chain begin while the one before runs, on the SMs that it leaves free: set-up, places and, without a normaliser, the
+// first item's scores are behind them when it ends.  A grid that began early has missed the launch-time L1 invalidation: what the
+// chain's kernels write is read past L1.  Every CTA of the second and third launch waits, so that each launch's end is the end of
+// all before it.  Small steps are what it is for, whose code comes from DRAM three times over (L2 cold; launched one after the other
+// -> so; by FMAs over 64 rows): linear attention of 128 rows, 4 heads, 45 -> 30 (38) us, of 1024 rows, 8 heads, 46 -> 38 (44); mLSTM of 200
+// fp32 rows 51 -> 44 (51).  With a normaliser nothing can be formed before the carry's rows are there: the output is released at the
+// carry's end (its CTAs, apart from the start, take longer for 4 x 2048 fp32 rows of 32 heads: 476 -> 487; released at the end 479).
+__device__ __forceinline__ void ct_release_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void ct_wait_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // The items of a CTA, found ahead of their use (three loads deep).
 constexpr int kCtAhead = 4;
 constexpr int kCtUsers = kCtConvWarps + kCtReadWarps + 1;      // warps that release an item (the copying one is done before the products are)
@@ -404,6 +414,7 @@ ct_state_kernel(const ChunkScanArgs a, const typename Form::Params p, int items)
   const uint32_t smem = smem_u32(ct_align(ct_raw));
   const TA* x = reinterpret_cast<const TA*>(a.x);
   const TA* vx = reinterpret_cast<const TA*>(a.v);
+  ct_release_next();
   if (tid == 0) {
     ct_queue_init(queue);
     for (int i = 0; i < 2; ++i) {
@@ -616,7 +627,11 @@ ct_carry_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   __shared__ float2 table[kCtTable];                  // a chunk's factors: of the state so far, of the chunk's own part
   const int s = blockIdx.z, h = blockIdx.y, tid = threadIdx.x;
   const int t0 = a.cu_seq[s], t1 = a.cu_seq[s + 1], nc = ct_chunks(t1 - t0, a.short_rows), slot = a.state_slots[s];
-  if (nc == 0 || slot < 0) return;
+  if constexpr (!Form::kNorm) ct_release_next();
+  if (nc == 0 || slot < 0) {
+    ct_wait_before();
+    return;
+  }
   if (tid < 32) {
     int q, l, before;
     ct_find(a.cu_seq, a.n_seqs, a.short_rows, -1, s, q, l, before);
@@ -630,6 +645,7 @@ ct_carry_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   if (live && !fresh) { S[0] = Sp[0]; S[1] = Sp[1]; }
   const size_t plane = ct_plane(DK, a.dv), step = (size_t)a.H * 3 * plane;
   uint8_t* C = reinterpret_cast<uint8_t*>(a.ws) + ((size_t)base * a.H + h) * 3 * plane + ct_in_plane(i / DK, i % DK / 8, a.dv);
+  ct_wait_before();
   typename Form::Carry carry(p, a, h, base);
   for (int c0 = 0; c0 < nc; c0 += kCtDepth) {
     float4 in[kCtDepth][2];
@@ -637,8 +653,8 @@ ct_carry_kernel(const ChunkScanArgs a, const typename Form::Params p) {
     for (int u = 0; u < kCtDepth; ++u)
       if (live && c0 + u < nc) {
         const uint8_t* from = C + (size_t)(c0 + u) * step;
-        in[u][0] = *reinterpret_cast<const float4*>(from);
-        in[u][1] = *reinterpret_cast<const float4*>(from + plane);
+        in[u][0] = __ldcg(reinterpret_cast<const float4*>(from));
+        in[u][1] = __ldcg(reinterpret_cast<const float4*>(from + plane));
       }
     if (c0 % kCtTable == 0) {
       __syncthreads();
@@ -665,6 +681,7 @@ ct_carry_kernel(const ChunkScanArgs a, const typename Form::Params p) {
       }
     }
   }
+  if constexpr (Form::kNorm) ct_release_next();
   if (live) { Sp[0] = S[0]; Sp[1] = S[1]; }
   if (blockIdx.x == 0) Form::template carry_row<DK>(p, a, h, base, nc, fresh, slot);
 }
@@ -678,10 +695,10 @@ template <typename TA>
 __device__ __noinline__ float ct_state_dot(const TA* q, const uint8_t* S, size_t plane, int v, int dk, int dv) {
   float acc = 0.f;
   for (int k = 0; k < dk && acc == acc; ++k) {
-    const uint8_t* at = S + ct_in_plane(v, k >> 3, dv) + (k & 7) * 2;
-    float x = __bfloat162float(*reinterpret_cast<const bf16*>(at));
+    const unsigned short* at = reinterpret_cast<const unsigned short*>(S + ct_in_plane(v, k >> 3, dv)) + (k & 7);
+    float x = __uint_as_float((uint32_t)__ldcg(at) << 16);
     if (ct_number(x))                                 // (behind an infinite first term stand none)
-      x += __bfloat162float(*reinterpret_cast<const bf16*>(at + plane)) + __bfloat162float(*reinterpret_cast<const bf16*>(at + 2 * plane));
+      x += __uint_as_float((uint32_t)__ldcg(at + plane / 2) << 16) + __uint_as_float((uint32_t)__ldcg(at + plane) << 16);
     acc = fmaf((float)q[k], x, acc);
   }
   return acc;
@@ -740,6 +757,7 @@ ct_output_kernel(const ChunkScanArgs a, const typename Form::Params p, int items
     };
     CtItem now = ct_item(queue, 0);
     if (now.item < items) load(tiles[0], now, 0);
+    if constexpr (Form::kNorm) ct_wait_before();
     for (int it = 0; now.item < items; ++it) {
       CtItem then{items};
       float old[4];                                   // kNorm: n_start . q of a thread's rows
@@ -761,7 +779,7 @@ ct_output_kernel(const ChunkScanArgs a, const typename Form::Params p, int items
               const bool start = from_state(now);
               float4 n = make_float4(0.f, 0.f, 0.f, 0.f);
               if (start)
-                n = *reinterpret_cast<const float4*>(a.ws_row + ((size_t)now.chunk * a.H + now.h) * a.ws_row_width + 64 * i + tile.column());
+                n = __ldcg(reinterpret_cast<const float4*>(a.ws_row + ((size_t)now.chunk * a.H + now.h) * a.ws_row_width + 64 * i + tile.column()));
 #pragma unroll
               for (int r = 0; r < 4; ++r) {
                 const float4 q = tile.value(r >> 1, r & 1);
@@ -815,6 +833,7 @@ ct_output_kernel(const ChunkScanArgs a, const typename Form::Params p, int items
       if (w0 < kCtTeam / 32 && next.item < items) Form::output_weights(p, a, scratch[it & 1], next.h, next.at, next.chunk);
     };
     CtItem now = ct_item(queue, 0);
+    if constexpr (Form::kNorm) ct_wait_before();
     weigh(now, 0);
     for (int it = 0; now.item < items; ++it) {
       const typename Form::Scratch& sc = scratch[it & 1];
@@ -937,6 +956,7 @@ ct_output_kernel(const ChunkScanArgs a, const typename Form::Params p, int items
         if (__any_sync(0xffffffffu, bad)) {
           __syncwarp();                               // (a row is written by eight lanes)
           if (bad) {
+            ct_wait_before();                         // (long since true)
             const int g = h / (a.H / a.G) * DK;
             const size_t plane = ct_plane(DK, a.dv);
             const uint8_t* S = reinterpret_cast<const uint8_t*>(a.ws) + ((size_t)now.chunk * a.H + h) * 3 * plane;
@@ -1035,6 +1055,7 @@ ct_output_kernel(const ChunkScanArgs a, const typename Form::Params p, int items
   } else if (warp == kCtCopy) {
     if (lane == 0) {                                  // the state's panels, where the keys were
       const size_t plane = ct_plane(DK, a.dv);
+      ct_wait_before();
       for (int it = 0;; ++it) {
         const CtItem now = ct_item(queue, it);
         if (now.item >= items) break;
@@ -1095,8 +1116,9 @@ int ct_launch_shape(const ChunkScanArgs& a, const typename Form::Params& p, int6
   if (rc != B200_OK) return rc;
   const int grid = (int)(items < ct_sms() ? items : ct_sms());
   ct_state_kernel<DK, VT, TA, Form><<<grid, kCtThreads, sb, s>>>(a, p, (int)items);
-  ct_carry_kernel<DK, Form><<<dim3((DK * a.dv / 8 + kCtCarryThreads - 1) / kCtCarryThreads, a.H, a.n_seqs), kCtCarryThreads, 0, s>>>(a, p);
-  ct_output_kernel<DK, VT, TA, Form><<<grid, kCtThreads, ob, s>>>(a, p, (int)items);
+  const dim3 carry((DK * a.dv / 8 + kCtCarryThreads - 1) / kCtCarryThreads, a.H, a.n_seqs);
+  (void)launch_pdl(ct_carry_kernel<DK, Form>, carry, dim3(kCtCarryThreads), 0, s, 1, a, p);
+  (void)launch_pdl(ct_output_kernel<DK, VT, TA, Form>, dim3(grid), dim3(kCtThreads), (size_t)ob, s, 1, a, p, (int)items);
   return b200_check_launch(Form::kName);
 }
 

@@ -683,13 +683,13 @@ struct MlstmForm {
     float m;
     __device__ __forceinline__ Carry(const Params&, const ChunkScanArgs& a, int h, int base)
         : row(a.ws_row + ((size_t)base * a.H + h) * a.ws_row_width + a.ws_row_width - 4), step((size_t)a.H * a.ws_row_width) {
-      m = row[3];
+      m = __ldcg(row + 3);
     }
     // whole warp, a chunk per lane: m_c = max(F_c + m_(c-1), own_c) is a running maximum of own_c - (F's sum) -- formed one after the
     // other, as the one-pass form does
     __device__ __forceinline__ void factors(int c0, int nc, int, float2* table) {
       const int lane = threadIdx.x & 31, c = c0 + lane;
-      const float F = c < nc ? row[c * step] : 0.f, ml = c < nc ? row[c * step + 1] : 0.f;
+      const float F = c < nc ? __ldcg(row + c * step) : 0.f, ml = c < nc ? __ldcg(row + c * step + 1) : 0.f;
       float before = m, after = m;
       for (int l = 0; l < 32 && c0 + l < nc; ++l) {
         const float f = __shfl_sync(0xffffffffu, F, l), o = __shfl_sync(0xffffffffu, ml, l);
@@ -707,7 +707,7 @@ struct MlstmForm {
     float* n_out = p.n_state + ((size_t)slot * a.H + h) * p.Z * DK;
     float n = fresh ? 0.f : n_out[k];
     float* row = a.ws_row + ((size_t)base * a.H + h) * (DK + 4);
-    float m = row[DK + 3];
+    float m = __ldcg(row + DK + 3);
     const size_t step = (size_t)a.H * (DK + 4);
     for (int c0 = 0; c0 < nc; c0 += kCtDepth) {        // as many chunks' rows in flight as there are of the state
       float own[kCtDepth], F[kCtDepth], ml[kCtDepth];
@@ -715,9 +715,9 @@ struct MlstmForm {
       for (int u = 0; u < kCtDepth; ++u)
         if (c0 + u < nc) {
           const float* at = row + (c0 + u) * step;
-          own[u] = at[k];
-          F[u] = at[DK];
-          ml[u] = at[DK + 1];
+          own[u] = __ldcg(at + k);
+          F[u] = __ldcg(at + DK);
+          ml[u] = __ldcg(at + DK + 1);
         }
 #pragma unroll
       for (int u = 0; u < kCtDepth; ++u) {
@@ -737,7 +737,7 @@ struct MlstmForm {
     double F, g;
     float ii;
     gate_sums(p, a, sc, h, at, F, g, ii);
-    const double m0 = (double)a.ws_row[((size_t)chunk * a.H + h) * a.ws_row_width + a.ws_row_width - 2];
+    const double m0 = (double)__ldcg(a.ws_row + ((size_t)chunk * a.H + h) * a.ws_row_width + a.ws_row_width - 2);
     const int t = ct_team_row();
     const double gm = fmax(m0, g), from = (double)ii - F;            // m_t - F_t
     const float m = (float)(F + gm);

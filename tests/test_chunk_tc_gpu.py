@@ -135,3 +135,57 @@ def test_infinite_numbers(where, kind, dtype, dk, dv):
         assert torch.equal(got == -float("inf"), ref == -float("inf"))
         a, b = (t[ref.isfinite()] for t in (got, ref))
         assert bool(((a - b).abs() <= TOL * b.abs()).all())
+
+
+@pytest.mark.parametrize("kind,dtype", [("linear", torch.float32), ("mlstm", torch.float32), ("mlstm", torch.bfloat16)])
+@pytest.mark.parametrize("how", ["one after the other", "captured"])
+def test_launches_that_begin_early(kind, dtype, how):
+    """Steps of other lengths over one workspace with nothing between them, or in one captured graph, give what they give alone."""
+    from gpustack_b200 import config, ops
+
+    H, dk, dv = 3, 128, 128
+    steps = [[130], [700, 40], [64, 65, 1], [300], [2500], [129]] * 4
+    g = torch.Generator(device="cuda").manual_seed(1)
+    draw = lambda *s: torch.randn(*s, generator=g, device="cuda")   # noqa: E731
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")   # noqa: E731
+    ws = torch.empty(config.chunk_scan_floats(4096, 8, H, dk, dv), device="cuda")
+    calls, states = [], []
+    for lens in steps:
+        T, n, Z = sum(lens), len(lens), ops.mlstm_state_slices(dv)
+        x, o, gates = draw(T, 3 * H * dk).to(dtype), torch.zeros(T, H * dv, device="cuda"), draw(T, 2 * H)
+        idx = (i32([sum(lens[:i]) for i in range(n + 1)]), i32([9] * n), i32(list(range(n))))
+        S, more = draw(n, H, dv, dk), [draw(n, H, 1, dk).expand(n, H, Z, dk).contiguous(), torch.zeros(n, H, Z, device="cuda")]
+        decay, bias = torch.linspace(0.9, 0.999, H, device="cuda"), torch.linspace(-1, 3, 2 * H).bfloat16().cuda()
+        cols = (0, H * dk, 2 * H * dk)
+        if kind == "linear":
+            more = []
+            call = lambda x=x, i=idx, S=S, o=o, L=max(lens), d=decay: ops.linattn_scan(x, *cols, d, *i, S, o, H, dk, dv, max_len=L,   # noqa: E731
+                                                                                       workspace=ws)
+        else:
+            call = lambda x=x, i=idx, S=S, o=o, L=max(lens), m=more, b=bias, gt=gates: ops.mlstm_scan(   # noqa: E731
+                x, *cols, gt, b, *i, S, *m, o, H, dk, dv, 6.0, max_len=L, workspace=ws)
+        calls.append(call)
+        states.append([o, S] + more)
+    start = [[t.clone() for t in s] for s in states]
+    real, ops.chunk_scan_pays = ops.chunk_scan_pays, lambda *a: True
+    try:
+        want = []
+        for call, s, s0 in zip(calls, states, start):
+            call()
+            torch.cuda.synchronize()
+            want.append([t.clone() for t in s])
+            [a.copy_(b) for a, b in zip(s, s0)]
+        torch.cuda.synchronize()
+        if how == "captured":
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                for call in calls:
+                    call()
+            graph.replay()
+        else:
+            for call in calls:
+                call()
+        torch.cuda.synchronize()
+    finally:
+        ops.chunk_scan_pays = real
+    assert all(torch.equal(a, b) for s, w in zip(states, want) for a, b in zip(s, w))
