@@ -105,9 +105,9 @@ def test_infinite_numbers(where, kind, dtype, dk, dv):
     elif where == "state":
         S[1, 7, 9] = -float("inf")
     elif where == "largest key":
-        k[70, 1, 3], q[:, 1, 3] = 3.395e38, 1e-3
+        k[70, 1, 3], q[:, 1, 3] = 3.4e38, 1e-3
     else:
-        v[200, 1, 5], k[200, 1] = -3.395e38, 1e-3
+        v[200, 1, 5], k[200, 1] = -3.4e38, 1e-3
     x = torch.cat([t.reshape(T, -1) for t in (q, k, v)], 1).to(dtype)
     i32 = lambda t: torch.tensor(t, dtype=torch.int32, device="cuda")   # noqa: E731
     idx, o, S_d = (i32([0, T]), i32([9]), i32([0])), torch.zeros(T, H * dv, device="cuda"), S[None].cuda()
