@@ -11,8 +11,9 @@
 // Precision: an fp32 number is the sum of three bf16 numbers (8 + 8 + 8 bits), so a product of two is formed from the six pairs of terms
 // whose exponents matter, every pair exact and summed in fp32 by tcgen05.mma; what is a bf16 number is one term.  The instruction
 // cuts its accumulator to 24 bits (it does not round), so the small pairs come first and few instructions meet an accumulator at
-// its full size.  Relative errors against 64 bits of 4 x 2048 rows of linear attention: state 2.3e-7 by fp32 FMAs, 1.3e-7 here; of
-// mLSTM over fp32 rows: outputs 2.1e-7 and 1.3e-7.
+// its full size, and ct_uncut adds back what is lost on average.  Relative errors against 64 bits, by fp32 FMAs and here: states of
+// 4 x 2048 rows of linear attention 2.3e-7 and 1.1e-7; mLSTM over 4000 ragged fp32 rows, outputs 2.2e-7 and 1.4e-7, states 1.3e-7 and
+// 1.2e-7.
 // Why: the same sums by fp32 FMAs were bound by the FMA pipe and by shared-memory reads (mLSTM, 7 ragged prompts of 7919 rows, 8 heads of
 // 128 x 128: state 70, carry 68, output 135 us; here 30, 18 and 52 us.  Linear attention over fp32 rows, 4 x 2048: 62, 44, 104 us; here
 // 35, 12, 66).  Chunks of 128 rows are the matrix instructions' own height and halve the chunks' states.  What bounds it: the chain of
@@ -148,6 +149,11 @@ __device__ __noinline__ float ct_rows_sum(const TA* k, int64_t ld, const TA* v, 
   for (int s = 0; s < rows && acc == acc; ++s) acc = fmaf((float)k[s * ld] * w[s], (float)v[s * ld_v], acc);
   return acc;
 }
+
+// A sum that left the products is cut towards zero once per instruction; what that loses on average, sums of one sign and of both taken
+// together, is added back (measured, with and without: mean deviation of outputs -1.0e-7 to -2.3e-7 -> +-8e-8, of states -4e-8 to -8e-8
+// -> +-3e-8; their relative error to two thirds of that of fp32 FMAs, where rows of one sign stood at up to 1.9 times without).
+__device__ __forceinline__ float ct_uncut(float x) { return fmaf(x, 5.0e-8f, x); }
 
 // One pair of terms over KS steps of 16, or all pairs (i, j) of 1 <= i + j <= 2, smallest first: the low words of the descriptors
 // and their steps in 16-byte units; A's terms in shared memory (A_TMEM: in tensor memory, a_step columns per step).  One thread.
@@ -553,7 +559,7 @@ ct_state_kernel(const ChunkScanArgs a, const typename Form::Params p, int items)
           const int k8 = (k >> 3) & 7;                // (v0 + c0 is a multiple of 8)
           CtFinite finite;
 #pragma unroll
-          for (int c = 0; c < 16; ++c) r[c] = __float_as_uint(__uint_as_float(r[c]) + __uint_as_float(s[c]));
+          for (int c = 0; c < 16; ++c) r[c] = __float_as_uint(ct_uncut(__uint_as_float(r[c]) + __uint_as_float(s[c])));
 #pragma unroll
           for (int c = 0; c < 16; c += 2) finite.add(__uint_as_float(r[c]), __uint_as_float(r[c + 1]));
 #pragma unroll
@@ -858,7 +864,8 @@ ct_output_kernel(const ChunkScanArgs a, const typename Form::Params p, int items
           tmem_ld_wait();
 #pragma unroll
           for (int e = 0; e < 16; ++e) {
-            const float z = kTwo ? __uint_as_float(r[e]) + __uint_as_float(r1[e]) : __uint_as_float(r[e]);
+            float z = kTwo ? __uint_as_float(r[e]) + __uint_as_float(r1[e]) : __uint_as_float(r[e]);
+            if constexpr (!Form::kNorm) z = ct_uncut(z);        // (with a normaliser it divides out)
             const float w = (s0 + e <= t && t < n) ? d[e] * (z * q_scale) : 0.f;
             if (Form::kNorm) own += w;
             r[e] = __float_as_uint(w);
@@ -915,7 +922,7 @@ ct_output_kernel(const ChunkScanArgs a, const typename Form::Params p, int items
           tmem_ld_32x16(t_o + lane_off + part * OC + c0 + 16 * b, r1);
           tmem_ld_wait();
 #pragma unroll
-          for (int e = 0; e < 16; ++e) o[16 * b + e] = start ? fmaf(__uint_as_float(r1[e]), f, __uint_as_float(r[e])) : __uint_as_float(r[e]);
+          for (int e = 0; e < 16; ++e) o[16 * b + e] = ct_uncut(start ? fmaf(__uint_as_float(r1[e]), f, __uint_as_float(r[e])) : __uint_as_float(r[e]));
         }
         CtFinite finite;
 #pragma unroll

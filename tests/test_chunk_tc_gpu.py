@@ -189,3 +189,30 @@ def test_launches_that_begin_early(kind, dtype, how):
     finally:
         ops.chunk_scan_pays = real
     assert all(torch.equal(a, b) for s, w in zip(states, want) for a, b in zip(s, w))
+
+
+@pytest.mark.parametrize("dk,dv", [(128, 128), (64, 64)])
+def test_sums_of_one_sign(dk, dv):
+    """What the products cut from a sum does not add up: over rows of one sign the mean deviation of outputs and states is below half a
+    unit of fp32's last place (2^-24), and their error that of a few roundings."""
+    from gpustack_b200 import ops
+
+    H, lens = 2, [2048, 300]
+    T, cu = sum(lens), [0, lens[0], sum(lens)]
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn(T, H * (2 * dk + dv), generator=g, device="cuda").abs()
+    S, decay = torch.randn(2, H, dv, dk, generator=g, device="cuda").abs(), torch.tensor([0.9, 0.99], device="cuda")
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")   # noqa: E731
+    o, S_d = torch.zeros(T, H * dv, device="cuda"), S.clone()
+    ops.linattn_scan(x, 0, H * dk, 2 * H * dk, decay, i32(cu), i32([9, 9]), i32([0, 1]), S_d, o, H, dk, dv, max_len=lens[0])
+    q, k, v = (x[:, a:b].to(F64).view(T, H, -1).transpose(0, 1) for a, b in ((0, H * dk), (H * dk, 2 * H * dk), (2 * H * dk, x.shape[1])))
+    for i, n in enumerate(lens):
+        rows, t = slice(cu[i], cu[i + 1]), torch.arange(n, device="cuda", dtype=F64)
+        d, Z = decay.to(F64)[:, None, None], S[i].to(F64)
+        D = torch.where(t[:, None] >= t, d ** (t[:, None] - t).clamp(min=0), 0.0)
+        want_o = (q[:, rows] @ k[:, rows].mT * D) @ v[:, rows] + d ** (t[:, None] + 1) * (q[:, rows] @ Z.mT)
+        want_S = d ** n * Z + (d ** (n - 1 - t[:, None]) * v[:, rows]).mT @ k[:, rows]
+        for got, want in ((o[rows].view(n, H, dv).transpose(0, 1), want_o), (S_d[i], want_S)):
+            off = got.to(F64) - want
+            assert float((off.flatten(1).sum(1).abs() / want.flatten(1).sum(1)).max()) < 2.0 ** -24
+            assert float((off.flatten(1).norm(dim=1) / want.flatten(1).norm(dim=1)).max()) < 2.0 ** -23
