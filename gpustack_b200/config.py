@@ -449,11 +449,15 @@ CHUNK_SCAN_MAX_BYTES = 1 << 30       # recurrences whose chunks would need more 
 
 
 def chunk_scan_floats(rows: int, n_seqs: int, heads: int, dk: int, dv: int, per_channel: bool = False) -> int:
-    """Workspace of a recurrence over its chunks side by side (b200_chunk_scan_floats): every chunk's state and row of factors --
-    64 rows in fp32, or 128 rows in three bf16 terms -- with a decay per key channel also its running sums."""
-    n = min(n_seqs, rows // 17)
-    halves = max(2 * (rows // 64 + n), 3 * (rows // 128 + n))
-    return (halves * heads * (dk * dv + dk + 4 + (128 * dk if per_channel else 0)) + 1) // 2
+    """Workspace of a recurrence over chunks of 64 rows side by side (b200_chunk_scan_floats): every chunk's state and row of
+    factors, with a decay per key channel also its running sums."""
+    return (rows // 64 + min(n_seqs, rows // 17)) * heads * (dk * dv + dk + 4 + (128 * dk if per_channel else 0))
+
+
+def chunk_scan_whole_floats(rows: int, n_seqs: int, heads: int, dk: int, dv: int) -> int:
+    """Workspace with which linear attention and mLSTM, whose chunks of 128 rows are kept in 6 bytes a number, run all sequences at
+    once (a smaller one of chunk_scan_floats: in groups)."""
+    return (rows // 128 + min(n_seqs, rows // 17)) * heads * (-(-3 * dk * dv // 2) + dk + 4) + 4
 
 
 def chunk_scan_workspace_floats(layers, rows: int, n_seqs: int) -> int:

@@ -90,11 +90,8 @@ inline int64_t cs_max_chunks(int64_t rows, int64_t n_seqs) {
   const int64_t longs = rows / (kCsShort + 1);
   return rows / kCsRows + (longs < n_seqs ? longs : n_seqs);
 }
-// (chunk_tc.cuh's chunks of 128 rows keep their first states in 6 bytes a number: room for the larger of the two)
 inline int64_t cs_workspace_floats(int64_t rows, int64_t n_seqs, int64_t H, int64_t dk, int64_t dv, bool vector = false) {
-  const int64_t longs = rows / (kCsShort + 1), n = longs < n_seqs ? longs : n_seqs;
-  const int64_t halves = 2 * (rows / kCsRows + n) > 3 * (rows / 128 + n) ? 2 * (rows / kCsRows + n) : 3 * (rows / 128 + n);
-  return (halves * H * (dk * dv + dk + 4 + (vector ? 2 * kCsRows * dk : 0)) + 1) / 2;
+  return cs_max_chunks(rows, n_seqs) * H * (dk * dv + dk + 4 + (vector ? 2 * kCsRows * dk : 0));
 }
 
 // Sequence and place in it of chunk b (whole warp; seq -1: no such chunk), or with b < 0 the chunks before sequence `upto`.

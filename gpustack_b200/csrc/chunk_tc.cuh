@@ -1103,6 +1103,22 @@ ct_output_kernel(const ChunkScanArgs a, const typename Form::Params p, int items
   ct_end(t_s, 512);
 }
 
+// Its size for `chunks` chunks: the states, then every chunk's row of factors.  A workspace of cs_workspace_floats holds the chunks of
+// 64 rows in fp32, which is less than those of 128 rows need where portions are short (64 x 128 rows in 256 sequences: by a fifth);
+// then the sequences run in groups, one after the other, as many in each as it has room for.
+inline int64_t ct_state_floats(int64_t chunks, int64_t H, int64_t dk, int64_t dv) { return (chunks * H * dk * dv / 2 * 3 + 3) / 4 * 4; }
+inline int64_t ct_group(int64_t rows, int64_t n_seqs, int64_t H, int64_t dk, int64_t dv, int64_t floats) {
+  auto fits = [&](int64_t n) {
+    const int64_t chunks = ct_max_chunks(rows, n);
+    return ct_state_floats(chunks, H, dk, dv) + chunks * H * (dk + 4) <= floats;
+  };
+  if (fits(n_seqs)) return n_seqs;
+  int64_t n = 0;                                      // (sizes grow with n)
+  for (int64_t step = (int64_t)1 << 32; step > 0; step >>= 1)
+    if (n + step < n_seqs && fits(n + step)) n += step;
+  return n;
+}
+
 // ------------------------------------------------------------------------------------------- launch
 template <typename K>
 inline int ct_allow(K kernel, int bytes) {
@@ -1129,17 +1145,26 @@ int ct_launch_shape(const ChunkScanArgs& a, const typename Form::Params& p, int6
   return b200_check_launch(Form::kName);
 }
 
+// group: sequences per walk (ct_group)
 template <typename TA, typename Form>
-int ct_launch(ChunkScanArgs a, const typename Form::Params& p, int dk, int64_t rows, float* ws, cudaStream_t s) {
-  const int64_t chunks = ct_max_chunks(rows, a.n_seqs);
-  if (chunks == 0) return B200_OK;
+int ct_launch(ChunkScanArgs a, const typename Form::Params& p, int dk, int64_t rows, int group, float* ws, cudaStream_t s) {
   a.v = a.x;
   a.ld_v = a.ld;
   a.ws = ws;
-  a.ws_row = ws + (chunks * a.H * dk * a.dv / 2 * 3 + 3) / 4 * 4;
   a.ws_row_width = dk + 4;
-  if (dk == 64) return a.dv <= 64 ? ct_launch_shape<64, 64, TA, Form>(a, p, rows, s) : ct_launch_shape<64, 128, TA, Form>(a, p, rows, s);
-  return a.dv <= 64 ? ct_launch_shape<128, 64, TA, Form>(a, p, rows, s) : ct_launch_shape<128, 128, TA, Form>(a, p, rows, s);
+  int rc = B200_OK;
+  for (int left = a.n_seqs; left > 0 && rc == B200_OK; left -= group) {
+    a.n_seqs = left < group ? left : group;
+    const int64_t chunks = ct_max_chunks(rows, a.n_seqs);
+    if (chunks == 0) break;
+    a.ws_row = ws + ct_state_floats(chunks, a.H, dk, a.dv);
+    if (dk == 64) rc = a.dv <= 64 ? ct_launch_shape<64, 64, TA, Form>(a, p, rows, s) : ct_launch_shape<64, 128, TA, Form>(a, p, rows, s);
+    else rc = a.dv <= 64 ? ct_launch_shape<128, 64, TA, Form>(a, p, rows, s) : ct_launch_shape<128, 128, TA, Form>(a, p, rows, s);
+    a.cu_seq += group;
+    a.ctx_lens += group;
+    a.state_slots += group;
+  }
+  return rc;
 }
 
 }  // namespace b200

@@ -524,6 +524,10 @@ extern "C" int b200_linattn_scan_chunked(const float* x, int64_t ld, int q_col, 
   B200_REQUIRE(workspace_floats >= cs_workspace_floats(rows, n_seqs, H, dk, dv), "linattn_scan: workspace of %lld floats too small",
                (long long)workspace_floats);
   cudaStream_t s = (cudaStream_t)stream;
+  const int group = (int)ct_group(rows, n_seqs, H, dk, dv, workspace_floats);
+  if (group == 0)                                     // (fewer than 64 rows)
+    return b200_linattn_scan(x, ld, q_col, k_col, v_col, decay, cu_seq, ctx_lens, state_slots, S, o_raw, n_seqs, H, dk, dv, max_len,
+                             stream);
   const int short_rows = cs_short(rows, n_seqs);
   if (short_rows > 0) {
     const int rc = launch_chunk4(x, ld, q_col, k_col, v_col, decay, cu_seq, ctx_lens, state_slots, S, o_raw, n_seqs, H, dk, dv,
@@ -531,7 +535,7 @@ extern "C" int b200_linattn_scan_chunked(const float* x, int64_t ld, int q_col, 
     if (rc != B200_OK) return rc;
   }
   const ChunkScanArgs a{x, ld, q_col, k_col, v_col, H, H, dv, cu_seq, ctx_lens, state_slots, n_seqs, short_rows, S, o_raw};
-  return ct_launch<float, LinearForm>(a, {decay}, dk, rows, workspace, s);
+  return ct_launch<float, LinearForm>(a, {decay}, dk, rows, group, workspace, s);
 }
 
 extern "C" int b200_linattn_out(const float* o_raw, const void* proj, int f32, int64_t ld, int gate_col, const void* w,

@@ -895,7 +895,7 @@ template <typename TA>
 static int launch_chunks(const void* proj, int64_t ld, int q_col, int k_col, int v_col, const float* gates, const void* gate_bias,
                          const int32_t* cu_seq, const int32_t* ctx_lens, const int32_t* state_slots, float* S_state, float* n_state,
                          float* m_state, float* o_raw, int n_seq, int H, int dk, int dv, float cap, float qscale, int rows,
-                         float* workspace, cudaStream_t s) {
+                         int group, float* workspace, cudaStream_t s) {
   const int short_rows = cs_short(rows, n_seq);
   if (short_rows > 0) {
     const int rc = launch_chunk<TA>(proj, ld, q_col, k_col, v_col, gates, gate_bias, cu_seq, ctx_lens, state_slots, S_state, n_state,
@@ -904,7 +904,7 @@ static int launch_chunks(const void* proj, int64_t ld, int q_col, int k_col, int
   }
   const ChunkScanArgs a{proj, ld, q_col, k_col, v_col, H, H, dv, cu_seq, ctx_lens, state_slots, n_seq, short_rows, S_state, o_raw};
   return ct_launch<TA, MlstmForm>(a, {gates, (const bf16*)gate_bias, cap, qscale, n_state, m_state, b200_mlstm_state_slices(dv)}, dk, rows,
-                                  workspace, s);
+                                  group, workspace, s);
 }
 
 // The same with a workspace (chunk_tc.cuh): sequences of more than 16 rows run with all their chunks side by side, the others
@@ -914,16 +914,18 @@ extern "C" int b200_mlstm_scan_chunked(const void* proj, int f32, int64_t ld, in
                                        const int32_t* state_slots, float* S_state, float* n_state, float* m_state, float* o_raw,
                                        int n_seq, int H, int dk, int dv, float cap, float qscale, int max_len, int rows,
                                        float* workspace, int64_t workspace_floats, void* stream) {
-  if (workspace == nullptr || rows <= 0 || n_seq <= 0 || H <= 0 || dv <= 0 || cap <= 0.f || ((uintptr_t)workspace & 15) != 0 ||
-      !cs_covers(proj, f32 ? 4 : 2, ld, q_col, k_col, v_col, dk, dv, S_state, o_raw))
+  const bool chunks = workspace != nullptr && rows > 0 && n_seq > 0 && H > 0 && dv > 0 && cap > 0.f && ((uintptr_t)workspace & 15) == 0 &&
+                      cs_covers(proj, f32 ? 4 : 2, ld, q_col, k_col, v_col, dk, dv, S_state, o_raw);
+  B200_REQUIRE(!chunks || workspace_floats >= cs_workspace_floats(rows, n_seq, H, dk, dv), "mlstm_scan: workspace of %lld floats too small",
+               (long long)workspace_floats);
+  const int group = chunks ? (int)ct_group(rows, n_seq, H, dk, dv, workspace_floats) : 0;
+  if (group == 0)                                     // (with a workspace: fewer than 64 rows)
     return b200_mlstm_scan(proj, f32, ld, q_col, k_col, v_col, gates, gate_bias, cu_seq, ctx_lens, state_slots, S_state, n_state,
                            m_state, o_raw, n_seq, H, dk, dv, cap, qscale, max_len, stream);
-  B200_REQUIRE(workspace_floats >= cs_workspace_floats(rows, n_seq, H, dk, dv), "mlstm_scan: workspace of %lld floats too small",
-               (long long)workspace_floats);
   return f32 ? launch_chunks<float>(proj, ld, q_col, k_col, v_col, gates, gate_bias, cu_seq, ctx_lens, state_slots, S_state, n_state,
-                                    m_state, o_raw, n_seq, H, dk, dv, cap, qscale, rows, workspace, (cudaStream_t)stream)
+                                    m_state, o_raw, n_seq, H, dk, dv, cap, qscale, rows, group, workspace, (cudaStream_t)stream)
              : launch_chunks<bf16>(proj, ld, q_col, k_col, v_col, gates, gate_bias, cu_seq, ctx_lens, state_slots, S_state, n_state,
-                                   m_state, o_raw, n_seq, H, dk, dv, cap, qscale, rows, workspace, (cudaStream_t)stream);
+                                   m_state, o_raw, n_seq, H, dk, dv, cap, qscale, rows, group, workspace, (cudaStream_t)stream);
 }
 
 extern "C" int b200_mlstm_out(const float* o_raw, const void* proj, int f32, int64_t ld, int gate_col,

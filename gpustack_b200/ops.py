@@ -12,7 +12,7 @@ from typing import Optional, Sequence
 
 import torch
 
-from .config import CHUNK_SCAN_MAX_BYTES, chunk_scan_floats
+from .config import CHUNK_SCAN_MAX_BYTES, chunk_scan_floats, chunk_scan_whole_floats
 from .lib import B200Error, check, load
 
 BLOCK_SIZE = 16  # tokens per KV page (vLLM default block_size)
@@ -664,6 +664,9 @@ def _chunk_scan_workspace(kind: str, rows: int, n_seqs: int, H: int, dk: int, dv
         _cuda(workspace)
         _req(workspace, torch.float32, "workspace")
         return workspace if workspace.numel() >= n else None
+    if kind in ("linear", "mlstm"):
+        whole = chunk_scan_whole_floats(rows, n_seqs, H, dk, dv)
+        n = whole if n < whole <= CHUNK_SCAN_MAX_BYTES // 4 else n
     return torch.empty(n, dtype=torch.float32, device=device) if 0 < 4 * n <= CHUNK_SCAN_MAX_BYTES else None
 
 

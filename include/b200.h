@@ -312,8 +312,9 @@ int b200_mlstm_scan(const void* proj, int f32, int64_t ld, int q_col, int k_col,
  * min(n_seqs, rows / 17)) * H * (dk * dv + dk + 4), with a decay per key channel 128 * dk more per head. */
 int64_t b200_chunk_scan_floats(int64_t rows, int64_t n_seqs, int H, int dk, int dv, int per_channel);
 /* The same with a workspace: sequences of more than 16 rows run with all their chunks of 128 rows side by side.  rows: the rows
- * of proj, at least cu_seq[n_seq]; workspace: 16-byte aligned, b200_chunk_scan_floats(rows, n_seq, H, dk, dv, 0) floats.  Widths other than
- * dk 64 / 128 with dv % 4 == 0, unaligned rows or no workspace: as b200_mlstm_scan. */
+ * of proj, at least cu_seq[n_seq]; workspace: 16-byte aligned, b200_chunk_scan_floats(rows, n_seq, H, dk, dv, 0) floats or more (with
+ * fewer than (rows / 128 + min(n_seq, rows / 17)) * H * (1.5 * dk * dv + dk + 4) + 4 the sequences run in groups, one after the
+ * other).  Widths other than dk 64 / 128 with dv % 4 == 0, unaligned rows or no workspace: as b200_mlstm_scan. */
 int b200_mlstm_scan_chunked(const void* proj, int f32, int64_t ld, int q_col, int k_col, int v_col, const float* gates,
                             const void* gate_bias, const int32_t* cu_seq, const int32_t* ctx_lens, const int32_t* state_slots,
                             float* S_state, float* n_state, float* m_state, float* o_raw, int n_seq, int H, int dk, int dv,
@@ -413,8 +414,9 @@ int b200_linattn_scan(const float* x, int64_t ld, int q_col, int k_col, int v_co
                       const int32_t* cu_seq, const int32_t* ctx_lens, const int32_t* state_slots, float* S, float* o_raw,
                       int n_seqs, int H, int dk, int dv, int max_len, void* stream);
 /* The same with a workspace: sequences of more than 16 rows run with all their chunks of 128 rows side by side.  rows: the rows
- * of x; workspace: 16-byte aligned, b200_chunk_scan_floats(rows, n_seqs, H, dk, dv, 0) floats.  Widths other than
- * dk 64 / 128 with dv % 4 == 0, unaligned rows or no workspace: as b200_linattn_scan. */
+ * of x; workspace: 16-byte aligned, b200_chunk_scan_floats(rows, n_seqs, H, dk, dv, 0) floats or more (with fewer than those given at
+ * b200_mlstm_scan_chunked the sequences run in groups).  Widths other than dk 64 / 128 with dv % 4 == 0, unaligned rows or no
+ * workspace: as b200_linattn_scan. */
 int b200_linattn_scan_chunked(const float* x, int64_t ld, int q_col, int k_col, int v_col, const float* decay,
                               const int32_t* cu_seq, const int32_t* ctx_lens, const int32_t* state_slots, float* S,
                               float* o_raw, int n_seqs, int H, int dk, int dv, int max_len, int rows, float* workspace,

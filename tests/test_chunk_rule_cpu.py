@@ -50,7 +50,8 @@ def test_the_runner_states_the_longest_portion():
 @pytest.mark.parametrize("rows,n", [(1, 1), (17, 3), (63, 1), (64, 64), (8192, 256), (100000, 5)])
 def test_the_workspace_has_one_size(rows, n):
     for H, dk, dv, per_channel in ((1, 64, 36, False), (8, 64, 128, True), (32, 128, 64, False)):
-        assert config.chunk_scan_floats(rows, n, H, dk, dv, per_channel) == load().b200_chunk_scan_floats(rows, n, H, dk, dv, int(per_channel))
+        size = (rows // 64 + min(n, rows // 17)) * H * (dk * dv + dk + 4 + (128 * dk if per_channel else 0))    # as the header has it
+        assert config.chunk_scan_floats(rows, n, H, dk, dv, per_channel) == load().b200_chunk_scan_floats(rows, n, H, dk, dv, int(per_channel)) == size
 
 
 def test_the_workspace_is_in_the_memory_estimate():

@@ -216,3 +216,39 @@ def test_sums_of_one_sign(dk, dv):
             off = got.to(F64) - want
             assert float((off.flatten(1).sum(1).abs() / want.flatten(1).sum(1)).max()) < 2.0 ** -24
             assert float((off.flatten(1).norm(dim=1) / want.flatten(1).norm(dim=1)).max()) < 2.0 ** -23
+
+
+@pytest.mark.parametrize("kind", ["linear", "mlstm"])
+@pytest.mark.parametrize("lens,H", [([64] * 20 + [33] * 10, 2), ([17] * 70 + [200], 1), ([40], 1), ([40, 41], 1), ([1] * 30 + [130] * 3, 3)],
+                         ids=["short", "shortest", "one", "two", "singles"])
+def test_a_workspace_of_the_documented_size(kind, lens, H):
+    """Portions too short for all sequences' chunks to fit at once: in groups, within the workspace, with the same results."""
+    from gpustack_b200 import config, ops
+
+    dk = dv = 64
+    T, n, Z = sum(lens), len(lens), ops.mlstm_state_slices(dv)
+    floats = config.chunk_scan_floats(T, n, H, dk, dv)
+    g = torch.Generator(device="cuda").manual_seed(T)
+    draw = lambda *s: torch.randn(*s, generator=g, device="cuda")   # noqa: E731
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")   # noqa: E731
+    x, gates, S0, n0 = draw(T, 3 * H * dk), draw(T, 2 * H), draw(n, H, dv, dk), draw(n, H, 1, dk)
+    idx = (i32([sum(lens[:i]) for i in range(n + 1)]), i32([i % 3 for i in range(n)]), i32(list(range(n))[::-1]))
+    real, out = ops.chunk_scan_pays, []
+    for chunks in (True, False):
+        ws = torch.full((floats + 4096,), 7.0, device="cuda")
+        o, S, more = torch.zeros(T, H * dv, device="cuda"), S0.clone(), []
+        ops.chunk_scan_pays = lambda *a: chunks
+        try:
+            if kind == "linear":
+                ops.linattn_scan(x, 0, H * dk, 2 * H * dk, torch.linspace(0.9, 0.99, H, device="cuda"), *idx, S, o, H, dk, dv, max_len=max(lens),
+                                 workspace=ws[:floats])
+            else:
+                more = [n0.expand(n, H, Z, dk).contiguous(), torch.zeros(n, H, Z, device="cuda")]
+                ops.mlstm_scan(x, 0, H * dk, 2 * H * dk, gates, torch.linspace(-1, 3, 2 * H).bfloat16().cuda(), *idx, S, *more, o, H, dk, dv, 6.0,
+                               max_len=max(lens), workspace=ws[:floats])
+        finally:
+            ops.chunk_scan_pays = real
+        assert bool((ws[floats:] == 7.0).all()) and bool((ws[:floats] == 7.0).all()) == (not chunks or lens == [40])
+        out.append([o, S] + more)
+    for a, b in zip(*out):                              # two roundings' worth of either side's
+        assert float((a - b).norm() / b.norm().clamp(min=1.0)) < (40 if kind == "mlstm" else 2) * TOL
