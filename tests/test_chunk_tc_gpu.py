@@ -8,33 +8,47 @@ pytestmark = pytest.mark.gpu
 F64 = torch.float64
 # fp32 sums of at most 128 + 128 terms and a chunk's share of the state, every rounding the same way, terms without cancellation beyond 2
 TOL = 2 * 300 * 2.0 ** -24
+# ... as they come out, roundings of both signs: four per chunk and sum.  A product without its smallest terms (2^-17 of a number and
+# more) is ten times further off.
+CLOSE = 8 * 2.0 ** -24
 
 
-@pytest.mark.parametrize("lens,H", [([128], 1), ([129], 1), ([255, 257], 2), ([700], 40)], ids=str)
-@pytest.mark.parametrize("exact", ["all", "some", "none"])
+def _linear_exact(x, S, decay, dk, dv):
+    """Outputs [H, n, dv] and the state behind the rows of one sequence, in fp64, without chunks."""
+    n, H, t = x.shape[0], decay.shape[0], torch.arange(x.shape[0], device="cuda", dtype=F64)
+    q, k, v = (x[:, a:b].to(F64).view(n, H, -1).transpose(0, 1) for a, b in ((0, H * dk), (H * dk, 2 * H * dk), (2 * H * dk, x.shape[1])))
+    d, Z = decay.to(F64)[:, None, None], S.to(F64)
+    o, back = torch.empty(H, n, dv, device="cuda", dtype=F64), (t[:, None] - t).clamp(min=0)
+    for h in range(H):
+        D = torch.where(t[:, None] >= t, d[h] ** back, 0.0)
+        o[h] = (q[h] @ k[h].mT * D) @ v[h] + d[h] ** (t[:, None] + 1) * (q[h] @ Z[h].mT)
+    return o, d ** n * Z + (d ** (n - 1 - t[:, None]) * v).mT @ k
+
+
+# the last three: more than six items for each of 148 CTAs, and more chunks than a table of the carry holds
+@pytest.mark.parametrize("lens,H", [([128], 1), ([129], 1), ([255, 257], 2), ([700], 40), ([700, 65, 1400], 60), ([4400, 64], 3)], ids=str)
+@pytest.mark.parametrize("exact", ["all", "some", "nearly", "none"])
 @pytest.mark.parametrize("dk,dv", [(128, 128), (64, 64)])
 def test_edges_and_terms(lens, H, exact, dk, dv):
     from gpustack_b200 import ops
 
-    g = torch.Generator().manual_seed(sum(lens) + dk)
+    g = torch.Generator(device="cuda").manual_seed(sum(lens) + dk)
     T, n = sum(lens), len(lens)
-    x, S = torch.randn(T, 2 * H * dk + H * dv, generator=g), torch.randn(n, H, dv, dk, generator=g)
-    rows = {"all": T, "some": 70, "none": 0}[exact]
+    x, S = torch.randn(T, 2 * H * dk + H * dv, generator=g, device="cuda"), torch.randn(n, H, dv, dk, generator=g, device="cuda")
+    rows = {"all": T, "some": 70, "nearly": T, "none": 0}[exact]
     x[:rows, 2 * H * dk:] = x[:rows, 2 * H * dk:].to(torch.bfloat16).float()
+    if exact == "nearly":                               # bf16 numbers but for the last bits
+        x[:, 2 * H * dk:] = (x[:, 2 * H * dk:].view(torch.int32) | 0x3f).view(torch.float32)
     cu = [sum(lens[:i]) for i in range(n + 1)]
-    decay = torch.linspace(0.5, 0.999, H)
+    decay = torch.linspace(0.5, 0.999, H, device="cuda")
     i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")   # noqa: E731
-    o, S_d = torch.zeros(T, H * dv, device="cuda"), S.cuda()
-    ops.linattn_scan(x.cuda(), 0, H * dk, 2 * H * dk, decay.cuda(), i32(cu), i32([9] * n), i32(list(range(n))), S_d, o, H, dk, dv, max_len=max(lens))
-    q, k = x[:, :H * dk].view(T, H, dk).to(F64), x[:, H * dk:2 * H * dk].view(T, H, dk).to(F64)
-    v, want = x[:, 2 * H * dk:].view(T, H, dv).to(F64), torch.zeros(T, H, dv, dtype=F64)
+    o, S_d = torch.zeros(T, H * dv, device="cuda"), S.clone()
+    ops.linattn_scan(x, 0, H * dk, 2 * H * dk, decay, i32(cu), i32([9] * n), i32(list(range(n))), S_d, o, H, dk, dv, max_len=max(lens))
     for i in range(n):
-        Z = S[i].to(F64)
-        for t in range(cu[i], cu[i + 1]):
-            Z = decay.to(F64)[:, None, None] * Z + v[t][:, :, None] * k[t][:, None]
-            want[t] = torch.einsum("hvk,hk->hv", Z, q[t])
-        assert float((S_d[i].cpu().to(F64) - Z).norm() / Z.norm()) < TOL
-    assert float((o.cpu().to(F64) - want.view(T, -1)).norm() / want.norm()) < TOL
+        want, Z = _linear_exact(x[cu[i]:cu[i + 1]], S[i], decay, dk, dv)
+        got = o[cu[i]:cu[i + 1]].view(-1, H, dv).transpose(0, 1)
+        for a, b in ((got, want), (S_d[i], Z)):         # per head
+            assert float(((a.to(F64) - b).flatten(1).norm(dim=1) / b.flatten(1).norm(dim=1)).max()) < CLOSE
 
 
 # chunks of 128 rows, 1, 48, 64 and 65 rows at a sequence's end, more chunks of one than a table of the carry holds (32)
@@ -42,8 +56,10 @@ MANY = [4400, 129, 300, 17, 193, 640, 1, 128]
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-def test_mlstm_beyond_the_second_item_of_a_cta(dtype):
-    """Buffers of a CTA's items are used again from its third item on: eight items per CTA (148 of them) and more."""
+@pytest.mark.parametrize("sign", ["both", "one"])
+def test_mlstm_beyond_the_second_item_of_a_cta(dtype, sign):
+    """Buffers of a CTA's items are used again from its third item on: eight items per CTA (148 of them) and more.  With queries and keys
+    of one sign no denominator cancels, and the outputs are as close as the states."""
     from gpustack_b200 import ops
     from oracle import vodavik_oracle as O
 
@@ -52,10 +68,14 @@ def test_mlstm_beyond_the_second_item_of_a_cta(dtype):
     T, Z = cu[-1], ops.mlstm_state_slices(dv)
     g = torch.Generator().manual_seed(3)
     proj = torch.randn(T, 2 * H * dk + H * dv, generator=g)
+    if sign == "one":
+        proj[:, :2 * H * dk] = proj[:, :2 * H * dk].abs()
     proj[:T // 2, 2 * H * dk:] = proj[:T // 2, 2 * H * dk:].bfloat16().float()
     proj, gates = proj.to(dtype).cuda(), (torch.randn(T, 2 * H, generator=g) * 3.0).cuda()
     bias = torch.cat([torch.randn(H, generator=g), 2 + torch.randn(H, generator=g)]).bfloat16().cuda()
     S, nn, m = (torch.randn(n, H, *w, generator=g).cuda() for w in ((dv, dk), (1, dk), (1,)))
+    if sign == "one":
+        nn = nn.abs()
     nn, m = nn.expand(n, H, Z, dk).contiguous(), m.abs().expand(n, H, Z).contiguous()
     o, S_d, n_d, m_d = torch.zeros(T, H * dv, device="cuda"), S.clone(), nn.clone(), m.clone()
     i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")   # noqa: E731
@@ -75,7 +95,8 @@ def test_mlstm_beyond_the_second_item_of_a_cta(dtype):
         # per head: one chunk's wrong factors are not lost among the others.  A log gate up to 6 in fp32, twice in an exponent, is 12 x 2^-24
         # of a weight; a denominator |n . q| cancels, its error is of the size of the terms
         for got, ref, tol in ((S_d[i], Sw, 17 * 2.0 ** -24), (n_d[i, :, 0], nw, 17 * 2.0 ** -24),
-                              (o[rows].view(-1, H, dv).transpose(0, 1), want.transpose(0, 1), 20 * TOL)):
+                              (o[rows].view(-1, H, dv).transpose(0, 1), want.transpose(0, 1),
+                               17 * 2.0 ** -24 if sign == "one" else 20 * TOL)):
             err = (got.to(F64) - ref).flatten(1).norm(dim=1) / ref.flatten(1).norm(dim=1)
             assert float(err.max()) < tol, (i, MANY[i])
         assert bool((m_d[i].to(F64) - mw[:, None]).abs().max() < 17 * 2.0 ** -24 * mw.abs().max().clamp(min=6.0))
@@ -83,38 +104,38 @@ def test_mlstm_beyond_the_second_item_of_a_cta(dtype):
 
 @pytest.mark.parametrize("where", ["query", "key", "value", "state", "largest key", "largest value"])
 @pytest.mark.parametrize("kind,dtype", [("linear", torch.float32), ("mlstm", torch.float32), ("mlstm", torch.bfloat16)])
-@pytest.mark.parametrize("dk,dv", [(128, 128), (64, 36)])
-def test_infinite_numbers(where, kind, dtype, dk, dv):
+@pytest.mark.parametrize("H,dk,dv", [(2, 128, 128), (2, 64, 36), (160, 64, 36)])       # the last: in a CTA's second to fourth item
+def test_infinite_numbers(where, kind, dtype, H, dk, dv):
     """An infinite number, and one that is infinite as a bf16 number only, gives what fp32 arithmetic gives.  Numbers of one sign in every
     column: no sum has infinities of both."""
     from gpustack_b200 import ops
     from oracle import vodavik_oracle as O
 
-    H, T, cap = 2, 300, 6.0
+    T, cap = 300, 6.0
     g = torch.Generator().manual_seed(dk)
     q, k, v = (0.1 + 0.8 * torch.rand(T, H, w, generator=g) for w in (dk, dk, dv))
     sign = torch.tensor([1.0, -1.0]).repeat(dv)[:dv]
     v, S = v * sign, (0.1 + torch.rand(H, dv, dk, generator=g)) * sign[:, None]
     n, m = 0.1 + torch.rand(H, 1, dk, generator=g), torch.zeros(H, 1)
     if where == "query":
-        q[70, 1, 3] = float("inf")
+        q[70, -1, 3] = float("inf")
     elif where == "key":
-        k[70, 1, 3] = float("inf")
+        k[70, -1, 3] = float("inf")
     elif where == "value":
-        v[200, 1, 5] = -float("inf")
+        v[200, -1, 5] = -float("inf")
     elif where == "state":
-        S[1, 7, 9] = -float("inf")
+        S[-1, 7, 9] = -float("inf")
     elif where == "largest key":
-        k[70, 1, 3], q[:, 1, 3] = 3.4e38, 1e-3
+        k[70, -1, 3], q[:, -1, 3] = 3.4e38, 1e-3
     else:
-        v[200, 1, 5], k[200, 1] = -3.4e38, 1e-3
+        v[200, -1, 5], k[200, -1] = -3.4e38, 1e-3
     x = torch.cat([t.reshape(T, -1) for t in (q, k, v)], 1).to(dtype)
     i32 = lambda t: torch.tensor(t, dtype=torch.int32, device="cuda")   # noqa: E731
     idx, o, S_d = (i32([0, T]), i32([9]), i32([0])), torch.zeros(T, H * dv, device="cuda"), S[None].cuda()
     q, k, v = (x[:, a:b].view(T, H, -1).to(F64) for a, b in ((0, H * dk), (H * dk, 2 * H * dk), (2 * H * dk, x.shape[1])))
     more = []
     if kind == "linear":
-        decay = torch.tensor([0.5, 0.98])
+        decay = torch.linspace(0.5, 0.98, H)
         ops.linattn_scan(x.cuda(), 0, H * dk, 2 * H * dk, decay.cuda(), *idx, S_d, o, H, dk, dv, max_len=T)
         Z, want = S.to(F64), torch.zeros(T, H, dv, dtype=F64)
         for t in range(T):
@@ -122,7 +143,7 @@ def test_infinite_numbers(where, kind, dtype, dk, dv):
             want[t] = torch.einsum("hvk,hk->hv", Z, q[t])
     else:
         slices = ops.mlstm_state_slices(dv)
-        gates, bias = torch.randn(T, 2 * H, generator=g), torch.tensor([0.0, 0.0, 3.0, 5.0]).bfloat16()
+        gates, bias = torch.randn(T, 2 * H, generator=g), torch.cat([torch.zeros(H), torch.linspace(3, 5, H)]).bfloat16()
         n_d, m_d = n.expand(H, slices, dk)[None].contiguous().cuda(), m.expand(H, slices)[None].contiguous().cuda()
         ops.mlstm_scan(x.cuda(), 0, H * dk, 2 * H * dk, gates.cuda(), bias.cuda(), *idx, S_d, n_d, m_d, o, H, dk, dv, cap, max_len=T)
         a = cap * torch.tanh((gates.to(F64) + bias.to(F64)) / cap)
@@ -205,13 +226,9 @@ def test_sums_of_one_sign(dk, dv):
     i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")   # noqa: E731
     o, S_d = torch.zeros(T, H * dv, device="cuda"), S.clone()
     ops.linattn_scan(x, 0, H * dk, 2 * H * dk, decay, i32(cu), i32([9, 9]), i32([0, 1]), S_d, o, H, dk, dv, max_len=lens[0])
-    q, k, v = (x[:, a:b].to(F64).view(T, H, -1).transpose(0, 1) for a, b in ((0, H * dk), (H * dk, 2 * H * dk), (2 * H * dk, x.shape[1])))
     for i, n in enumerate(lens):
-        rows, t = slice(cu[i], cu[i + 1]), torch.arange(n, device="cuda", dtype=F64)
-        d, Z = decay.to(F64)[:, None, None], S[i].to(F64)
-        D = torch.where(t[:, None] >= t, d ** (t[:, None] - t).clamp(min=0), 0.0)
-        want_o = (q[:, rows] @ k[:, rows].mT * D) @ v[:, rows] + d ** (t[:, None] + 1) * (q[:, rows] @ Z.mT)
-        want_S = d ** n * Z + (d ** (n - 1 - t[:, None]) * v[:, rows]).mT @ k[:, rows]
+        rows = slice(cu[i], cu[i + 1])
+        want_o, want_S = _linear_exact(x[rows], S[i], decay, dk, dv)
         for got, want in ((o[rows].view(n, H, dv).transpose(0, 1), want_o), (S_d[i], want_S)):
             off = got.to(F64) - want
             assert float((off.flatten(1).sum(1).abs() / want.flatten(1).sum(1)).max()) < 2.0 ** -24
