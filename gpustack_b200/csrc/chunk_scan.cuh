@@ -2,7 +2,7 @@
 // sequence side by side.
 //
 // With a state S (dk x dv), rows t = 0 .. n-1 of a chunk of 64 and the weights that a recurrence's `Form` supplies:
-//     o_t = aq_t S_start^T q_t + sum_{s<=t} D(t, s) (k_s . q_t) v_s          S_end = a S_start + b sum_s w_s k_s v_s^T
+//     o_t = aq_t S_start^T q_t + sum_{s<=t} D(t, s) (k_s . q_t) v_s          S_end = a S_start + sum_s w_s k_s v_s^T
 // State space and, with a decay per key channel, gated linear attention; mLSTM and linear attention run on the tensor cores
 // (chunk_tc.cuh).  Three launches:
 //   chunk_state   one CTA per (chunk, head, value tile): C = sum_s w_s k_s v_s^T into the workspace, [chunk][H][dk][dv]
@@ -76,11 +76,10 @@ struct ChunkScanArgs {
   float* ws_row;                   // [chunks][H][ws_row_width]: a recurrence's own carry (its Form says what)
   int ws_row_width;                // dk + 4
   float* ws_sums;                  // [chunks][H][2][64][dk]: kVector, the running sums' two parts
-  const void* v;                   // chunk_tc.cuh: rows of the values (x, or rows of their own) and their pitch
-  int64_t ld_v;
 };
 
-__host__ __device__ __forceinline__ int cs_chunks(int rows, int short_rows) { return rows > short_rows ? (rows + kCsRows - 1) / kCsRows : 0; }
+template <int ROWS>
+__host__ __device__ __forceinline__ int cs_chunks(int rows, int short_rows) { return rows > short_rows ? (rows + ROWS - 1) / ROWS : 0; }
 
 // A step of one sequence needs no one-pass launch beside the chunks: whatever the sequence's rows of a longer buffer, they are chunks.
 inline int cs_short(int64_t rows, int n_seqs) { return n_seqs > 1 || rows <= kCsShort ? kCsShort : 0; }
@@ -94,7 +93,8 @@ inline int64_t cs_workspace_floats(int64_t rows, int64_t n_seqs, int64_t H, int6
   return cs_max_chunks(rows, n_seqs) * H * (dk * dv + dk + 4 + (vector ? 2 * kCsRows * dk : 0));
 }
 
-// Sequence and place in it of chunk b (whole warp; seq -1: no such chunk), or with b < 0 the chunks before sequence `upto`.
+// Sequence and place in it of chunk b of ROWS rows (whole warp; seq -1: no such chunk), or with b < 0 the chunks before sequence `upto`.
+template <int ROWS>
 __device__ __forceinline__ void cs_find(const int32_t* cu, int n_seqs, int short_rows, int b, int upto, int& seq, int& local, int& before) {
   const int lane = threadIdx.x & 31;
   seq = -1;
@@ -102,7 +102,7 @@ __device__ __forceinline__ void cs_find(const int32_t* cu, int n_seqs, int short
   before = 0;
   for (int base = 0; base < n_seqs; base += 32) {
     const int s = base + lane;
-    const int c = s < n_seqs ? cs_chunks(cu[s + 1] - cu[s], short_rows) : 0;
+    const int c = s < n_seqs ? cs_chunks<ROWS>(cu[s + 1] - cu[s], short_rows) : 0;
     int incl = c;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -132,7 +132,7 @@ struct ChunkPlace {
 __device__ __forceinline__ ChunkPlace cs_place(const ChunkScanArgs& a, int* shared5) {
   if (threadIdx.x < 32) {
     int seq, local, before;
-    cs_find(a.cu_seq, a.n_seqs, a.short_rows, (int)blockIdx.x, 0, seq, local, before);
+    cs_find<kCsRows>(a.cu_seq, a.n_seqs, a.short_rows, (int)blockIdx.x, 0, seq, local, before);
     if (threadIdx.x == 0) {
       shared5[0] = seq;
       if (seq >= 0) {
@@ -148,43 +148,19 @@ __device__ __forceinline__ ChunkPlace cs_place(const ChunkScanArgs& a, int* shar
   return {shared5[0], shared5[1], shared5[2], shared5[3], shared5[4]};
 }
 
-// ROWS x W values of column `col` on, on their way to shared memory (fp32, row pitch PITCH, rows from `n` and columns from
-// `width` on zero): fp32 rows by cp.async, bf16 rows through registers, converted when they land.
-template <typename TA, int ROWS, int W, int PITCH>
-struct ChunkTile {
-  static constexpr int PER = W / 4, STEP = kCsThreads / PER, ITERS = ROWS / STEP;
-  uint2 raw[ITERS];
-  __device__ __forceinline__ void issue(const TA* x, int64_t ld, int first, int n, int col, int width, float*) {
-    const int c = ((int)threadIdx.x % PER) * 4, r0 = (int)threadIdx.x / PER;
-#pragma unroll
-    for (int i = 0; i < ITERS; ++i) {
-      const int r = r0 + i * STEP;
-      raw[i] = make_uint2(0, 0);
-      if (r < n && c < width) raw[i] = *reinterpret_cast<const uint2*>(x + (size_t)(first + r) * ld + col + c);
-    }
-  }
-  __device__ __forceinline__ void land(float* dst) const {
-    const int c = ((int)threadIdx.x % PER) * 4, r0 = (int)threadIdx.x / PER;
-#pragma unroll
-    for (int i = 0; i < ITERS; ++i)
-      *reinterpret_cast<float4*>(dst + (r0 + i * STEP) * PITCH + c) =
-          make_float4(bf16_lo(raw[i].x), bf16_hi(raw[i].x), bf16_lo(raw[i].y), bf16_hi(raw[i].y));
-  }
-};
+// ROWS x W values of column `col` on, on their way to shared memory by cp.async (row pitch PITCH, rows from `n` and columns from
+// `width` on zero).
 template <int ROWS, int W, int PITCH>
-struct ChunkTile<float, ROWS, W, PITCH> {
-  static constexpr int PER = W / 4, STEP = kCsThreads / PER, ITERS = ROWS / STEP;
-  __device__ __forceinline__ void issue(const float* x, int64_t ld, int first, int n, int col, int width, float* dst) {
-    const int c = ((int)threadIdx.x % PER) * 4, r0 = (int)threadIdx.x / PER;
+__device__ __forceinline__ void cs_issue(const float* x, int64_t ld, int first, int n, int col, int width, float* dst) {
+  constexpr int PER = W / 4, STEP = kCsThreads / PER, ITERS = ROWS / STEP;
+  const int c = ((int)threadIdx.x % PER) * 4, r0 = (int)threadIdx.x / PER;
 #pragma unroll
-    for (int i = 0; i < ITERS; ++i) {
-      const int r = r0 + i * STEP;
-      const bool in = r < n && c < width;
-      cp_async_16_zfill(dst + r * PITCH + c, in ? x + (size_t)(first + r) * ld + col + c : x, in);
-    }
+  for (int i = 0; i < ITERS; ++i) {
+    const int r = r0 + i * STEP;
+    const bool in = r < n && c < width;
+    cp_async_16_zfill(dst + r * PITCH + c, in ? x + (size_t)(first + r) * ld + col + c : x, in);
   }
-  __device__ __forceinline__ void land(float*) const {}
-};
+}
 
 // Running sums of a chunk's logarithms per key channel, inclusive: F[t][k] = sum_(r <= t) lg(r, k), 256 threads: four runs of 16
 // rows per channel, with 128 channels two of 32.  hi / lo: [64][DK + 4].  Ends with a barrier.
@@ -220,13 +196,13 @@ struct ChunkSmem {
   static constexpr int kOutput = kCsRows * (DK + 4) + kB + kTile + kCsRows * kCsAPitch + kSum;
 };
 
-// Form: `Scratch` (shared arrays of one chunk), `state_weights` (fills scratch, w(s) and row() for chunk_state), `output_weights`,
-// aq(t), D(t, s), finish() for chunk_output, and `carry` / `carry_row` for chunk_carry.
+// Form: `Scratch` (shared arrays of one chunk), `state_weights` and `state_row` for chunk_state, `output_weights`, aq(t), D(t, s) and
+// finish() for chunk_output, `Carry` (the chunks' decays) for chunk_carry.
 // A Form with kVector has one decay per KEY CHANNEL instead: with the running sums F of a chunk's base-2 logarithms per channel
 // (summed in fp64, kept as two fp32 parts, so that a difference is as exact as an fp32 product of decays) the keys of the state
 // are weighted by 2^(F_n - F_s), the queries of the state's part by 2^F_t, and (k_s . q_t) is a sum of k q 2^(F_t - F_s) formed
 // term by term: 64 * 65 / 2 exponentials per channel, but none of a positive number, whatever the decays are.
-template <int DK, int VT, typename TA, typename Form>
+template <int DK, int VT, typename Form>
 __global__ void __launch_bounds__(kCsThreads, 2)
 chunk_state_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   extern __shared__ __align__(16) float smem[];
@@ -237,15 +213,13 @@ chunk_state_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   const int h = blockIdx.y, v0 = blockIdx.z * VT, tid = threadIdx.x;
   float* ks = smem;                // [64][DK]
   float* vs = smem + kCsRows * DK; // [64][VT]
-  const TA* x = reinterpret_cast<const TA*>(a.x);
+  const float* x = reinterpret_cast<const float*>(a.x);
   const int kcol = a.k_col + h / (a.H / a.G) * DK, vcol = a.v_col + h * a.dv + v0;
   // two halves of 32 rows: the second one is on its way while the first is summed
-  ChunkTile<TA, 32, DK, DK> kt[2];
-  ChunkTile<TA, 32, VT, VT> vt[2];
 #pragma unroll
   for (int e = 0; e < 2; ++e) {
-    kt[e].issue(x, a.ld, at.first + 32 * e, at.rows - 32 * e, kcol, DK, ks + 32 * e * DK);
-    vt[e].issue(x, a.ld, at.first + 32 * e, at.rows - 32 * e, vcol, a.dv - v0, vs + 32 * e * VT);
+    cs_issue<32, DK, DK>(x, a.ld, at.first + 32 * e, at.rows - 32 * e, kcol, DK, ks + 32 * e * DK);
+    cs_issue<32, VT, VT>(x, a.ld, at.first + 32 * e, at.rows - 32 * e, vcol, a.dv - v0, vs + 32 * e * VT);
     cp_async_commit();
   }
   float* hi = vs + kCsRows * VT;   // [64][DK + 4] each, kVector only
@@ -261,8 +235,6 @@ chunk_state_kernel(const ChunkScanArgs a, const typename Form::Params p) {
     for (int j = 0; j < VJ * 2; ++j) acc[i][j] = 0ull;
 #pragma unroll
   for (int e = 0; e < 2; ++e) {
-    kt[e].land(ks + 32 * e * DK);
-    vt[e].land(vs + 32 * e * VT);
     if (e == 0) cp_async_wait<1>();
     else cp_async_wait<0>();
     __syncthreads();
@@ -322,7 +294,7 @@ chunk_state_kernel(const ChunkScanArgs a, const typename Form::Params p) {
       }
     }
   } else if (blockIdx.z == 0) {
-    Form::template state_row<DK>(a, scratch, ks, h, at.rows);
+    Form::template state_row<DK>(a, scratch, h);
   }
 }
 
@@ -336,11 +308,11 @@ chunk_carry_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   __shared__ float tile[128][kCsCarryKeys + 1];
   __shared__ int base;
   const int s = blockIdx.z, h = blockIdx.y, tid = threadIdx.x;
-  const int t0 = a.cu_seq[s], t1 = a.cu_seq[s + 1], nc = cs_chunks(t1 - t0, a.short_rows), slot = a.state_slots[s];
+  const int t0 = a.cu_seq[s], t1 = a.cu_seq[s + 1], nc = cs_chunks<kCsRows>(t1 - t0, a.short_rows), slot = a.state_slots[s];
   if (nc == 0 || slot < 0) return;
   if (tid < 32) {
     int q, l, before;
-    cs_find(a.cu_seq, a.n_seqs, a.short_rows, -1, s, q, l, before);
+    cs_find<kCsRows>(a.cu_seq, a.n_seqs, a.short_rows, -1, s, q, l, before);
     if (tid == 0) base = before;
   }
   const int k0 = (blockIdx.x % (DK / kCsCarryKeys)) * kCsCarryKeys, v0 = (blockIdx.x / (DK / kCsCarryKeys)) * 128;
@@ -356,22 +328,21 @@ chunk_carry_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   const bool live = v0 + v < a.dv;
   const size_t step = (size_t)a.H * DK * a.dv;
   float* C = a.ws + ((size_t)base * a.H + h) * DK * a.dv + (size_t)(k0 + k) * a.dv + v0 + v;
-  typename Form::Carry carry(p, a, s, h, base, k0 + k);
+  typename Form::Carry carry(a, h, base, k0 + k);
   constexpr int U = kCsCarryDepth;
   for (int c0 = 0; c0 < nc; c0 += U) {
     float4 in[U];
 #pragma unroll
     for (int u = 0; u < U; ++u)
       if (live && c0 + u < nc) in[u] = *reinterpret_cast<const float4*>(C + (size_t)(c0 + u) * step);
-    carry.fetch(a, c0, nc);
+    carry.fetch(c0, nc);
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       if (c0 + u >= nc) break;
-      float fa, fb;
-      carry.next(p, u, min(kCsRows, t1 - t0 - (c0 + u) * kCsRows), fa, fb);
+      const float f = carry.f[u];
       if (live) {
         *reinterpret_cast<float4*>(C + (size_t)(c0 + u) * step) = S;
-        S = make_float4(fmaf(fa, S.x, fb * in[u].x), fmaf(fa, S.y, fb * in[u].y), fmaf(fa, S.z, fb * in[u].z), fmaf(fa, S.w, fb * in[u].w));
+        S = make_float4(fmaf(f, S.x, in[u].x), fmaf(f, S.y, in[u].y), fmaf(f, S.z, in[u].z), fmaf(f, S.w, in[u].w));
       }
     }
   }
@@ -382,7 +353,6 @@ chunk_carry_kernel(const ChunkScanArgs a, const typename Form::Params p) {
     const int vv = i / kCsCarryKeys, kk = i % kCsCarryKeys;
     if (v0 + vv < a.dv) Sp[(size_t)(v0 + vv) * DK + k0 + kk] = tile[vv][kk];
   }
-  if (blockIdx.x == 0) Form::template carry_row<DK>(p, a, s, h, base, nc, fresh, slot);
 }
 
 // acc[i][.] += sum over 4 rows of B: rows t = tg + 16 i of P (pitch `pp`, columns c .. c + 3), i >= I0.  DIAG >= 0: the rows of
@@ -421,7 +391,7 @@ __device__ __forceinline__ void cs_own_rows(cs_f2 (&acc)[4][VT / 32], const floa
   cs_outer<VT, I0, 12>(acc, A + 16 * I0 + 12, kCsAPitch, V + (16 * I0 + 12) * VT, tg, vg);
 }
 
-template <int DK, int VT, typename TA, typename Form>
+template <int DK, int VT, typename Form>
 __global__ void __launch_bounds__(kCsThreads, 2)
 chunk_output_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   extern __shared__ __align__(16) float smem[];
@@ -437,44 +407,37 @@ chunk_output_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   float* A = B + ChunkSmem<DK, VT, Form::kVector>::kB;              // [64][68]
   float* hi = A + kCsRows * kCsAPitch;               // [64][DK + 4] each, kVector only; lo behind the keys, until the ring takes the place
   float* lo = B + kCsRows * QP;
-  const TA* x = reinterpret_cast<const TA*>(a.x);
+  const float* x = reinterpret_cast<const float*>(a.x);
   const int hg = h / (a.H / a.G), vcol = a.v_col + h * a.dv + v0;
   const bool zero_start = at.local == 0 && a.ctx_lens[at.seq] == 0;
   const float* C = a.ws + ((size_t)blockIdx.x * a.H + h) * DK * a.dv;
   // tiles in the order of their use: the state's rows (none for a zero start), then the chunk's own values
   const int n_state = zero_start ? 0 : DK / 32;
-  ChunkTile<TA, 32, VT, VT> own[2];
   auto tile_at = [&](int i) { return X + (i % 3) * TILE; };
   auto issue = [&](int i) {
     if (i < n_state) {
-      ChunkTile<float, 32, VT, VT> t;
-      t.issue(C, a.dv, 32 * i, 32, v0, a.dv - v0, tile_at(i));
+      cs_issue<32, VT, VT>(C, a.dv, 32 * i, 32, v0, a.dv - v0, tile_at(i));
     } else if (i == n_state) {
-      own[0].issue(x, a.ld, at.first, n, vcol, a.dv - v0, tile_at(i));
+      cs_issue<32, VT, VT>(x, a.ld, at.first, n, vcol, a.dv - v0, tile_at(i));
     } else if (i == n_state + 1) {
-      own[1].issue(x, a.ld, at.first + 32, n - 32, vcol, a.dv - v0, tile_at(i));
+      cs_issue<32, VT, VT>(x, a.ld, at.first + 32, n - 32, vcol, a.dv - v0, tile_at(i));
     }
     cp_async_commit();
   };
   {
-    ChunkTile<TA, kCsRows, DK, QP> q, k;
-    q.issue(x, a.ld, at.first, n, a.q_col + hg * DK, DK, qs);
-    k.issue(x, a.ld, at.first, n, a.k_col + hg * DK, DK, B);
+    cs_issue<kCsRows, DK, QP>(x, a.ld, at.first, n, a.q_col + hg * DK, DK, qs);
+    cs_issue<kCsRows, DK, QP>(x, a.ld, at.first, n, a.k_col + hg * DK, DK, B);
     if constexpr (Form::kVector) {                   // as chunk_state left them
       const float* sums = a.ws_sums + ((size_t)blockIdx.x * a.H + h) * (2 * kCsRows * DK);
-      ChunkTile<float, kCsRows, DK, QP> f;
-      f.issue(sums, DK, 0, kCsRows, 0, DK, hi);
-      f.issue(sums, DK, kCsRows, kCsRows, 0, DK, lo);
+      cs_issue<kCsRows, DK, QP>(sums, DK, 0, kCsRows, 0, DK, hi);
+      cs_issue<kCsRows, DK, QP>(sums, DK, kCsRows, kCsRows, 0, DK, lo);
     }
     cp_async_commit();
     issue(0);
     if constexpr (!Form::kVector) Form::output_weights(p, a, scratch, h, at);
-    q.land(qs);
-    k.land(B);
   }
   cp_async_wait<1>();
   __syncthreads();
-  const float q_scale = Form::q_scale(p);
   const int tg = tid >> 4, vg = tid & 15;
   if constexpr (Form::kVector) {
     float acc[4][4];
@@ -511,7 +474,7 @@ chunk_output_kernel(const ChunkScanArgs a, const typename Form::Params p) {
 #pragma unroll
       for (int j = 0; j <= i; ++j) {
         const int t = tg + 16 * i, s = vg + 16 * j;
-        A[t * kCsAPitch + s] = (s <= t && t < n) ? acc[i][j] * q_scale : 0.f;
+        A[t * kCsAPitch + s] = (s <= t && t < n) ? acc[i][j] : 0.f;
       }
     __syncthreads();                                 // the queries as they came are used
     if (!zero_start)
@@ -545,7 +508,7 @@ chunk_output_kernel(const ChunkScanArgs a, const typename Form::Params p) {
       for (int j = 0; j <= i; ++j) {
         const int t = tg + 16 * i, s = vg + 16 * j;
         const float2 z = cs_split(acc[i][j]);
-        A[t * kCsAPitch + s] = (s <= t && t < n) ? Form::D(p, scratch, t, s) * ((z.x + z.y) * q_scale) : 0.f;
+        A[t * kCsAPitch + s] = (s <= t && t < n) ? Form::D(p, scratch, t, s) * (z.x + z.y) : 0.f;
       }
   }
   cs_f2 acc[4][VT / 32];
@@ -556,8 +519,6 @@ chunk_output_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   // tile i: landed, and tile i - 1 used by every thread, so tile i + 2 may take its place (behind the first barrier the keys
   // are used as well)
   auto next_tile = [&](int i) {
-    if (i == n_state) own[0].land(tile_at(i));
-    if (i == n_state + 1) own[1].land(tile_at(i));
     if (i == 0 || i == n_state + 1) cp_async_wait<0>();
     else cp_async_wait<1>();
     __syncthreads();
@@ -574,13 +535,12 @@ chunk_output_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   if (!zero_start) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const cs_f2 f = cs_dup(Form::aq(scratch, tg + 16 * i) * q_scale);
+      const cs_f2 f = cs_dup(Form::aq(scratch, tg + 16 * i));
 #pragma unroll
       for (int j = 0; j < VT / 32; ++j) acc[i][j] = cs_mul(acc[i][j], f);
     }
   }
   const float* V0 = next_tile(n_state);
-  Form::template rows<DK>(p, a, scratch, qs, A, h, n, zero_start);
   cs_own_rows<VT, 0>(acc, A, V0, tg, vg);
   cs_own_rows<VT, 1>(acc, A, V0, tg, vg);
   const float* V1 = next_tile(n_state + 1);
@@ -609,24 +569,24 @@ inline bool cs_covers(const void* x, int elem, int64_t ld, int q_col, int k_col,
          ((uintptr_t)x & al) == 0 && ((uintptr_t)S & 15) == 0 && ((uintptr_t)o & 15) == 0;
 }
 
-template <int DK, int VT, typename TA, typename Form>
+template <int DK, int VT, typename Form>
 int cs_launch_shape(const ChunkScanArgs& a, const typename Form::Params& p, int64_t rows, cudaStream_t s) {
   const int64_t chunks = cs_max_chunks(rows, a.n_seqs);
   const dim3 grid((unsigned)chunks, a.H, (a.dv + VT - 1) / VT);
   const int sb = ChunkSmem<DK, VT, Form::kVector>::kState * 4, ob = ChunkSmem<DK, VT, Form::kVector>::kOutput * 4;
-  cudaError_t e = cudaFuncSetAttribute(chunk_state_kernel<DK, VT, TA, Form>, cudaFuncAttributeMaxDynamicSharedMemorySize, sb);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(chunk_output_kernel<DK, VT, TA, Form>, cudaFuncAttributeMaxDynamicSharedMemorySize, ob);
+  cudaError_t e = cudaFuncSetAttribute(chunk_state_kernel<DK, VT, Form>, cudaFuncAttributeMaxDynamicSharedMemorySize, sb);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(chunk_output_kernel<DK, VT, Form>, cudaFuncAttributeMaxDynamicSharedMemorySize, ob);
   if (e != cudaSuccess) {
     b200_set_error("chunk scan: %d bytes of shared memory: %s", ob, cudaGetErrorString(e));
     return B200_ERR_CUDA;
   }
-  chunk_state_kernel<DK, VT, TA, Form><<<grid, kCsThreads, sb, s>>>(a, p);
+  chunk_state_kernel<DK, VT, Form><<<grid, kCsThreads, sb, s>>>(a, p);
   chunk_carry_kernel<DK, Form><<<dim3(DK / kCsCarryKeys * ((a.dv + 127) / 128), a.H, a.n_seqs), kCsThreads, 0, s>>>(a, p);
-  chunk_output_kernel<DK, VT, TA, Form><<<grid, kCsThreads, ob, s>>>(a, p);
+  chunk_output_kernel<DK, VT, Form><<<grid, kCsThreads, ob, s>>>(a, p);
   return b200_check_launch(Form::kName);
 }
 
-template <typename TA, typename Form>
+template <typename Form>
 int cs_launch(ChunkScanArgs a, const typename Form::Params& p, int dk, int64_t rows, float* ws, cudaStream_t s) {
   const int64_t chunks = cs_max_chunks(rows, a.n_seqs);
   if (chunks == 0) return B200_OK;
@@ -634,8 +594,8 @@ int cs_launch(ChunkScanArgs a, const typename Form::Params& p, int dk, int64_t r
   a.ws_row = ws + chunks * a.H * dk * a.dv;
   a.ws_row_width = dk + 4;
   a.ws_sums = a.ws_row + chunks * a.H * (dk + 4);
-  if (dk == 64) return a.dv <= 64 ? cs_launch_shape<64, 64, TA, Form>(a, p, rows, s) : cs_launch_shape<64, 128, TA, Form>(a, p, rows, s);
-  return a.dv <= 64 ? cs_launch_shape<128, 64, TA, Form>(a, p, rows, s) : cs_launch_shape<128, 128, TA, Form>(a, p, rows, s);
+  if (dk == 64) return a.dv <= 64 ? cs_launch_shape<64, 64, Form>(a, p, rows, s) : cs_launch_shape<64, 128, Form>(a, p, rows, s);
+  return a.dv <= 64 ? cs_launch_shape<128, 64, Form>(a, p, rows, s) : cs_launch_shape<128, 128, Form>(a, p, rows, s);
 }
 
 }  // namespace b200

@@ -184,41 +184,9 @@ __device__ __forceinline__ void ct_copy(uint32_t to, const void* from, uint32_t 
 constexpr uint32_t kCtAmn = 1u << 15, kCtBmn = 1u << 16;      // instruction descriptor: operand is MN-major
 
 // ------------------------------------------------------------------------------------------- places
-__host__ __device__ __forceinline__ int ct_chunks(int rows, int short_rows) { return rows > short_rows ? (rows + kCtRows - 1) / kCtRows : 0; }
 inline int64_t ct_max_chunks(int64_t rows, int64_t n_seqs) {
   const int64_t longs = rows / (kCsShort + 1);
   return rows / kCtRows + (longs < n_seqs ? longs : n_seqs);
-}
-
-// Sequence and place in it of chunk b (whole warp; seq -1: no such chunk), or with b < 0 the chunks before sequence `upto`.
-__device__ __forceinline__ void ct_find(const int32_t* cu, int n_seqs, int short_rows, int b, int upto, int& seq, int& local, int& before) {
-  const int lane = threadIdx.x & 31;
-  seq = -1;
-  local = 0;
-  before = 0;
-  for (int base = 0; base < n_seqs; base += 32) {
-    const int s = base + lane;
-    const int c = s < n_seqs ? ct_chunks(cu[s + 1] - cu[s], short_rows) : 0;
-    int incl = c;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += v;
-    }
-    if (b >= 0) {
-      const uint32_t hit = __ballot_sync(0xffffffffu, before + incl > b);
-      if (hit) {
-        const int l = __ffs(hit) - 1;
-        seq = base + l;
-        local = b - before - (__shfl_sync(0xffffffffu, incl, l) - __shfl_sync(0xffffffffu, c, l));
-        return;
-      }
-    } else if (upto < base + 32) {
-      before += __shfl_sync(0xffffffffu, incl - c, upto - base);
-      return;
-    }
-    before += __shfl_sync(0xffffffffu, incl, 31);
-  }
 }
 
 // The items of a CTA that walks (chunk, head, value tile) triples `step` apart: the next one from `item` on that there is (items:
@@ -234,7 +202,7 @@ __device__ __forceinline__ CtItem ct_next(const ChunkScanArgs& a, int items, int
   CtItem r{items};
   for (; item < items; item += step) {
     int seq, local, before;
-    ct_find(a.cu_seq, a.n_seqs, a.short_rows, item / per, 0, seq, local, before);
+    cs_find<kCtRows>(a.cu_seq, a.n_seqs, a.short_rows, item / per, 0, seq, local, before);
     if (seq < 0) break;                               // the chunks that there are come first
     const int slot = a.state_slots[seq];
     if (slot < 0) continue;
@@ -419,7 +387,6 @@ ct_state_kernel(const ChunkScanArgs a, const typename Form::Params p, int items)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t smem = smem_u32(ct_align(ct_raw));
   const TA* x = reinterpret_cast<const TA*>(a.x);
-  const TA* vx = reinterpret_cast<const TA*>(a.v);
   ct_release_next();
   if (tid == 0) {
     ct_queue_init(queue);
@@ -440,7 +407,7 @@ ct_state_kernel(const ChunkScanArgs a, const typename Form::Params p, int items)
     Blocks kt, vt;
     auto load_k = [&](const CtItem& w, int e) {
       const int n = w.at.rows - kCtHalf * e;
-      kt.load(x + (int64_t)(w.at.first + kCtHalf * e) * a.ld + a.k_col + w.h / (a.H / a.G) * DK, a.ld, 64, n, DK == 128 ? n : 0, 64, 64);
+      kt.load(x + (int64_t)(w.at.first + kCtHalf * e) * a.ld + a.k_col + w.h * DK, a.ld, 64, n, DK == 128 ? n : 0, 64, 64);
     };
     CtItem now = ct_item(queue, 0);
     if (now.item < items) load_k(now, 0);
@@ -452,7 +419,7 @@ ct_state_kernel(const ChunkScanArgs a, const typename Form::Params p, int items)
       for (int e = 0; e < 2; ++e) {
         const uint32_t ks = smem + e * L::kStateHalf, vs = ks + L::kStateK;
         const int n = now.at.rows - kCtHalf * e, width = a.dv - now.v0;
-        vt.load(vx + (int64_t)(now.at.first + kCtHalf * e) * a.ld_v + a.v_col + now.h * a.dv + now.v0, a.ld_v, 64, n, VT == 128 ? n : 0, width,
+        vt.load(x + (int64_t)(now.at.first + kCtHalf * e) * a.ld + a.v_col + now.h * a.dv + now.v0, a.ld, 64, n, VT == 128 ? n : 0, width,
                 width - 64);
         if (it) ct_wait(&half_done[e], it - 1);       // the item before has used this half
         if (e == 0) mbar_wait_guarded(&weight_full[it & 1], (it >> 1) & 1);
@@ -570,8 +537,8 @@ ct_state_kernel(const ChunkScanArgs a, const typename Form::Params p, int items)
             for (int c = 0; c < 16 && v0 + c0 + c < a.dv; ++c) {
               float* C_kv = reinterpret_cast<float*>(out + c * 128 + ((k8 ^ (c & 7)) << 4));
               if (!ct_number(*C_kv))
-                *C_kv = ct_rows_sum(x + (int64_t)now.at.first * a.ld + a.k_col + now.h / (a.H / a.G) * DK + k, a.ld,
-                                    vx + (int64_t)now.at.first * a.ld_v + a.v_col + now.h * a.dv + v0 + c0 + c, a.ld_v, scratch[buf].w, now.at.rows);
+                *C_kv = ct_rows_sum(x + (int64_t)now.at.first * a.ld + a.k_col + now.h * DK + k, a.ld,
+                                    x + (int64_t)now.at.first * a.ld + a.v_col + now.h * a.dv + v0 + c0 + c, a.ld, scratch[buf].w, now.at.rows);
             }
           }
         }
@@ -617,8 +584,8 @@ ct_state_kernel(const ChunkScanArgs a, const typename Form::Params p, int items)
       ct_arrive(&queue.full[buf]);
       if (next.item >= items) break;
       const int w = min(VT, a.dv - next.v0) * (int)sizeof(TA);
-      ct_prefetch(x + (int64_t)next.at.first * a.ld + a.k_col + next.h / (a.H / a.G) * DK, a.ld * sizeof(TA), next.at.rows, DK * (int)sizeof(TA));
-      ct_prefetch(vx + (int64_t)next.at.first * a.ld_v + a.v_col + next.h * a.dv + next.v0, a.ld_v * sizeof(TA), next.at.rows, w);
+      ct_prefetch(x + (int64_t)next.at.first * a.ld + a.k_col + next.h * DK, a.ld * sizeof(TA), next.at.rows, DK * (int)sizeof(TA));
+      ct_prefetch(x + (int64_t)next.at.first * a.ld + a.v_col + next.h * a.dv + next.v0, a.ld * sizeof(TA), next.at.rows, w);
       item = next.item + (int)gridDim.x;
     }
   }
@@ -632,7 +599,7 @@ ct_carry_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   __shared__ int base;
   __shared__ float2 table[kCtTable];                  // a chunk's factors: of the state so far, of the chunk's own part
   const int s = blockIdx.z, h = blockIdx.y, tid = threadIdx.x;
-  const int t0 = a.cu_seq[s], t1 = a.cu_seq[s + 1], nc = ct_chunks(t1 - t0, a.short_rows), slot = a.state_slots[s];
+  const int t0 = a.cu_seq[s], t1 = a.cu_seq[s + 1], nc = cs_chunks<kCtRows>(t1 - t0, a.short_rows), slot = a.state_slots[s];
   if constexpr (!Form::kNorm) ct_release_next();
   if (nc == 0 || slot < 0) {
     ct_wait_before();
@@ -640,7 +607,7 @@ ct_carry_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   }
   if (tid < 32) {
     int q, l, before;
-    ct_find(a.cu_seq, a.n_seqs, a.short_rows, -1, s, q, l, before);
+    cs_find<kCtRows>(a.cu_seq, a.n_seqs, a.short_rows, -1, s, q, l, before);
     if (tid == 0) base = before;
   }
   __syncthreads();
@@ -727,7 +694,6 @@ ct_output_kernel(const ChunkScanArgs a, const typename Form::Params p, int items
   constexpr bool kTwo = NP == 2 || L::kIn == 3;       // the scores have a second accumulator
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const TA* x = reinterpret_cast<const TA*>(a.x);
-  const TA* vx = reinterpret_cast<const TA*>(a.v);
   const uint32_t smem = smem_u32(ct_align(ct_raw));
   if (tid == 0) {
     ct_queue_init(queue);
@@ -753,11 +719,11 @@ ct_output_kernel(const ChunkScanArgs a, const typename Form::Params p, int items
     Blocks tiles[2];
     auto load = [&](Blocks& b, const CtItem& w, int i) {
       if (i < 2 * NP) {
-        const int col = (i < NP ? a.q_col : a.k_col) + w.h / (a.H / a.G) * DK + 64 * (i % NP);
+        const int col = (i < NP ? a.q_col : a.k_col) + w.h * DK + 64 * (i % NP);
         b.load(x + (int64_t)w.at.first * a.ld + col, a.ld, 64 * a.ld, w.at.rows, w.at.rows - 64, 64, 64);
       } else {
         const int n = w.at.rows - kCtHalf * (i - 2 * NP), width = a.dv - w.v0;
-        b.load(vx + (int64_t)(w.at.first + kCtHalf * (i - 2 * NP)) * a.ld_v + a.v_col + w.h * a.dv + w.v0, a.ld_v, 64, n, VT == 128 ? n : 0,
+        b.load(x + (int64_t)(w.at.first + kCtHalf * (i - 2 * NP)) * a.ld + a.v_col + w.h * a.dv + w.v0, a.ld, 64, n, VT == 128 ? n : 0,
                width, width - 64);
       }
     };
@@ -887,7 +853,7 @@ ct_output_kernel(const ChunkScanArgs a, const typename Form::Params p, int items
       }
       if constexpr (Form::kNorm) {
         if (!ct_number(own) && t < n) {               // an infinite key or query: scores by FMAs
-          const TA* qk = x + (size_t)now.at.first * a.ld + h / (a.H / a.G) * DK;
+          const TA* qk = x + (size_t)now.at.first * a.ld + h * DK;
           own = 0.f;
 #pragma unroll 1
           for (int s = 64 * part; s < min(64 * part + 64, t + 1) && own == own; ++s)
@@ -909,7 +875,6 @@ ct_output_kernel(const ChunkScanArgs a, const typename Form::Params p, int items
       const float f = start ? Form::aq(sc, t) * q_scale : 0.f;
       const typename Form::Finish finish(p, a, sc, h, t, den);
       const TA* mine = x + (size_t)(now.at.first + (live ? t : 0)) * a.ld;
-      const TA* my_v = vx + (size_t)(now.at.first + (live ? t : 0)) * a.ld_v + a.v_col + h * a.dv;
       ct_wait(&value_done, it);
 #pragma unroll 1
       for (int c0 = 0; c0 < OC; c0 += 32) {
@@ -929,11 +894,11 @@ ct_output_kernel(const ChunkScanArgs a, const typename Form::Params p, int items
         for (int e = 0; e < 32; e += 2) finite.add(o[e], o[e + 1]);
         const bool bad = live && !finite.all();
         if (odd && live) {
-          const int g = h / (a.H / a.G) * DK;
+          const int g = h * DK;
 #pragma unroll 1
           for (int s = 0; s <= t; ++s) {
             if (!((sp[s >> 5] >> (s & 31)) & 1)) continue;
-            const TA* vr = vx + (size_t)(now.at.first + s) * a.ld_v + a.v_col + h * a.dv + v;
+            const TA* vr = x + (size_t)(now.at.first + s) * a.ld + a.v_col + h * a.dv + v;
             const float ps = Form::D(p, sc, row, t, s) *
                              (ct_dot(mine + a.q_col + g, x + (size_t)(now.at.first + s) * a.ld + a.k_col + g, DK) * q_scale);
 #pragma unroll
@@ -941,7 +906,7 @@ ct_output_kernel(const ChunkScanArgs a, const typename Form::Params p, int items
               if (v + e < a.dv && !ct_finite((float)vr[e])) o[e] = fmaf(ps, (float)vr[e], o[e]);
           }
         }
-        if (live) finish.apply(o, my_v + v, a.dv - v);
+        if (live) finish.apply(o);
         // sixteen rows at a time: eight lanes store a line of a row
 #pragma unroll
         for (int b = 0; b < 2; ++b) {
@@ -964,7 +929,7 @@ ct_output_kernel(const ChunkScanArgs a, const typename Form::Params p, int items
           __syncwarp();                               // (a row is written by eight lanes)
           if (bad) {
             ct_wait_before();                         // (long since true)
-            const int g = h / (a.H / a.G) * DK;
+            const int g = h * DK;
             const size_t plane = ct_plane(DK, a.dv);
             const uint8_t* S = reinterpret_cast<const uint8_t*>(a.ws) + ((size_t)now.chunk * a.H + h) * 3 * plane;
             float* to = a.o + (size_t)(now.at.first + t) * a.H * a.dv + h * a.dv + v;
@@ -978,7 +943,7 @@ ct_output_kernel(const ChunkScanArgs a, const typename Form::Params p, int items
             }
 #pragma unroll 1
             for (int s = 0; s <= t && again; ++s) {
-              const TA* vr = vx + (size_t)(now.at.first + s) * a.ld_v + a.v_col + h * a.dv + v;
+              const TA* vr = x + (size_t)(now.at.first + s) * a.ld + a.v_col + h * a.dv + v;
               const float ps = Form::D(p, sc, row, t, s) *
                                (ct_dot(mine + a.q_col + g, x + (size_t)(now.at.first + s) * a.ld + a.k_col + g, DK) * q_scale);
               for (uint32_t m = again; m; m &= m - 1) {
@@ -1093,10 +1058,10 @@ ct_output_kernel(const ChunkScanArgs a, const typename Form::Params p, int items
       ct_arrive(&queue.full[buf]);
       if (next.item >= items) break;
       const TA* row = x + (int64_t)next.at.first * a.ld;
-      const int g = next.h / (a.H / a.G) * DK, w = min(VT, a.dv - next.v0) * (int)sizeof(TA);
+      const int g = next.h * DK, w = min(VT, a.dv - next.v0) * (int)sizeof(TA);
       ct_prefetch(row + a.q_col + g, a.ld * sizeof(TA), next.at.rows, DK * (int)sizeof(TA));
       ct_prefetch(row + a.k_col + g, a.ld * sizeof(TA), next.at.rows, DK * (int)sizeof(TA));
-      ct_prefetch(vx + (int64_t)next.at.first * a.ld_v + a.v_col + next.h * a.dv + next.v0, a.ld_v * sizeof(TA), next.at.rows, w);
+      ct_prefetch(x + (int64_t)next.at.first * a.ld + a.v_col + next.h * a.dv + next.v0, a.ld * sizeof(TA), next.at.rows, w);
       item = next.item + (int)gridDim.x;
     }
   }
@@ -1148,8 +1113,6 @@ int ct_launch_shape(const ChunkScanArgs& a, const typename Form::Params& p, int6
 // group: sequences per walk (ct_group)
 template <typename TA, typename Form>
 int ct_launch(ChunkScanArgs a, const typename Form::Params& p, int dk, int64_t rows, int group, float* ws, cudaStream_t s) {
-  a.v = a.x;
-  a.ld_v = a.ld;
   a.ws = ws;
   a.ws_row_width = dk + 4;
   int rc = B200_OK;

@@ -168,24 +168,15 @@ struct GatedLinearForm {
     const float* row;
     size_t step;
     float f[kCsCarryDepth];
-    __device__ __forceinline__ Carry(const Params&, const ChunkScanArgs& a, int, int h, int base, int k)
+    __device__ __forceinline__ Carry(const ChunkScanArgs& a, int h, int base, int k)
         : row(a.ws_row + ((size_t)base * a.H + h) * a.ws_row_width + k), step((size_t)a.H * a.ws_row_width) {}
-    __device__ __forceinline__ void fetch(const ChunkScanArgs&, int c0, int nc) {
+    __device__ __forceinline__ void fetch(int c0, int nc) {
 #pragma unroll
       for (int u = 0; u < kCsCarryDepth; ++u)
         if (c0 + u < nc) f[u] = row[(c0 + u) * step];
     }
-    __device__ __forceinline__ void next(const Params&, int u, int, float& a, float& b) {
-      a = f[u];
-      b = 1.0f;
-    }
   };
-  template <int DK>
-  static __device__ __forceinline__ void carry_row(const Params&, const ChunkScanArgs&, int, int, int, int, bool, int) {}
-  static __device__ __forceinline__ float q_scale(const Params&) { return 1.0f; }
   static __device__ __forceinline__ float aq(const Scratch&, int) { return 1.0f; }
-  template <int DK>
-  static __device__ __forceinline__ void rows(const Params&, const ChunkScanArgs&, Scratch&, const float*, const float*, int, int, bool) {}
   static __device__ __forceinline__ float4 finish(const Params&, const Scratch&, int, int, float4 acc, float4) { return acc; }
 };
 
@@ -362,5 +353,5 @@ extern "C" int b200_gla_scan_chunked(const float* x, int64_t ld, int q_col, int 
     if (rc != B200_OK) return rc;
   }
   const ChunkScanArgs a{x, ld, q_col, k_col, v_col, H, H, dv, cu_seq, ctx_lens, state_slots, n_seqs, short_rows, S, o_raw};
-  return cs_launch<float, GatedLinearForm>(a, {z, ldz, inv_tau}, dk, rows, workspace, s);
+  return cs_launch<GatedLinearForm>(a, {z, ldz, inv_tau}, dk, rows, workspace, s);
 }

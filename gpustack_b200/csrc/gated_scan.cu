@@ -469,27 +469,21 @@ struct StateSpaceForm {
     __syncthreads();
   }
   template <int DK>
-  static __device__ __forceinline__ void state_row(const ChunkScanArgs& a, const Scratch& sc, const float*, int h, int) {
+  static __device__ __forceinline__ void state_row(const ChunkScanArgs& a, const Scratch& sc, int h) {
     if (threadIdx.x == 0) a.ws_row[((size_t)blockIdx.x * a.H + h) * a.ws_row_width + DK] = sc.all;
   }
   struct Carry {
     const float* row;
     size_t step;
     float f[kCsCarryDepth];
-    __device__ __forceinline__ Carry(const Params&, const ChunkScanArgs& a, int, int h, int base, int)
+    __device__ __forceinline__ Carry(const ChunkScanArgs& a, int h, int base, int)
         : row(a.ws_row + ((size_t)base * a.H + h) * a.ws_row_width + a.ws_row_width - 4), step((size_t)a.H * a.ws_row_width) {}
-    __device__ __forceinline__ void fetch(const ChunkScanArgs&, int c0, int nc) {
+    __device__ __forceinline__ void fetch(int c0, int nc) {
 #pragma unroll
       for (int u = 0; u < kCsCarryDepth; ++u)
         if (c0 + u < nc) f[u] = row[(c0 + u) * step];
     }
-    __device__ __forceinline__ void next(const Params&, int u, int, float& a, float& b) {
-      a = f[u];
-      b = 1.0f;
-    }
   };
-  template <int DK>
-  static __device__ __forceinline__ void carry_row(const Params&, const ChunkScanArgs&, int, int, int, int, bool, int) {}
   static __device__ __forceinline__ void output_weights(const Params& p, const ChunkScanArgs&, Scratch& sc, int h, const ChunkPlace& at) {
     if (threadIdx.x < 32) {
       double F[2];
@@ -504,11 +498,8 @@ struct StateSpaceForm {
       }
     }
   }
-  static __device__ __forceinline__ float q_scale(const Params&) { return 1.0f; }
   static __device__ __forceinline__ float D(const Params&, const Scratch& sc, int t, int s) { return expf((float)(sc.F[t] - sc.F[s])) * sc.beta[s]; }
   static __device__ __forceinline__ float aq(const Scratch& sc, int t) { return sc.aq[t]; }
-  template <int DK>
-  static __device__ __forceinline__ void rows(const Params&, const ChunkScanArgs&, Scratch&, const float*, const float*, int, int, bool) {}
   static __device__ __forceinline__ float4 finish(const Params& p, const Scratch&, int h, int, float4 v, float4 x) {
     const float s = p.skip != nullptr ? p.skip[h] : 0.f;
     return p.skip != nullptr ? make_float4(fmaf(s, x.x, v.x), fmaf(s, x.y, v.y), fmaf(s, x.z, v.z), fmaf(s, x.w, v.w)) : v;
@@ -684,7 +675,7 @@ extern "C" int b200_gated_scan_chunked(const float* x, int64_t ld, int q_col, in
     if (rc != B200_OK) return rc;
   }
   const ChunkScanArgs a{x, ld, q_col, k_col, v_col, H, G, dv, cu_seq, ctx_lens, state_slots, n_seqs, short_rows, S, o_raw};
-  return cs_launch<float, StateSpaceForm>(a, {gates, ld_g, rate, dt_bias, skip}, dk, rows, workspace, s);
+  return cs_launch<StateSpaceForm>(a, {gates, ld_g, rate, dt_bias, skip}, dk, rows, workspace, s);
 }
 
 extern "C" int b200_gate_norm(const float* y, const void* proj, int f32, int64_t ld, int z_col, const void* w, void* out,

@@ -416,7 +416,7 @@ struct LinearForm {
   static __device__ __forceinline__ float aq(const Scratch& sc, int t) { return sc.dp[t + 1]; }
   struct Finish {
     __device__ __forceinline__ Finish(const Params&, const ChunkScanArgs&, const Scratch&, int, int, const float*) {}
-    __device__ __forceinline__ void apply(float (&)[32], const void*, int) const {}
+    __device__ __forceinline__ void apply(float (&)[32]) const {}
     __device__ __forceinline__ float one(float f) const { return f; }
   };
 };

@@ -781,7 +781,7 @@ struct MlstmForm {
     }
     __device__ __forceinline__ float one(float f) const { return f / d; }
     // a quotient by its reciprocal and its remainder (P. Markstein, 1990); out of the range in which both are normal, the operator's
-    __device__ __forceinline__ void apply(float (&f)[32], const void*, int) const {
+    __device__ __forceinline__ void apply(float (&f)[32]) const {
       bool in_range = d < kDivRange;
 #pragma unroll
       for (int c = 0; c < 32; ++c) in_range = in_range && fabsf(f[c]) < kDivRange;
