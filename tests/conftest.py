@@ -31,7 +31,5 @@ def pytest_collection_modifyitems(config, items):
 
 
 @pytest.fixture(scope="session")
-def out_dir():
-    d = ROOT / "gpurun_out"
-    d.mkdir(exist_ok=True)
-    return d
+def out_dir(tmp_path_factory):
+    return tmp_path_factory.mktemp("out")

@@ -3,7 +3,7 @@ Llama-3-8B engine.  Meant to run under ncu with --profile-from-start off: only t
 cudaProfilerStart/Stop is captured.
 
   ncu --profile-from-start off --metrics gpu__time_duration.sum --clock-control none --csv \
-      --log-file gpurun_out/launches.csv python tools/profile_step.py
+      --log-file launches.csv python tools/profile_step.py
 """
 import sys
 from pathlib import Path

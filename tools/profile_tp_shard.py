@@ -1,7 +1,7 @@
 """Single-GPU stand-in for ONE rank of a TP=t Llama-3-8B decode step (same per-rank shapes, no
 communication): shows where a tensor-parallel decode step spends its GPU time.
   ncu --profile-from-start off --metrics gpu__time_duration.sum --clock-control none --csv \
-      --log-file gpurun_out/launches_tp8shard.csv python tools/profile_tp_shard.py 8"""
+      --log-file launches_tp8shard.csv python tools/profile_tp_shard.py 8"""
 import os
 import sys
 import time
