@@ -15,10 +15,12 @@
 // 4 x 2048 rows of linear attention 2.3e-7 and 1.1e-7; mLSTM over 4000 ragged fp32 rows, outputs 2.2e-7 and 1.4e-7, states 1.3e-7 and
 // 1.2e-7.
 // Why: the same sums by fp32 FMAs were bound by the FMA pipe and by shared-memory reads (mLSTM, 7 ragged prompts of 7919 rows, 8 heads of
-// 128 x 128: state 70, carry 68, output 135 us; here 30, 18 and 52 us.  Linear attention over fp32 rows, 4 x 2048: 62, 44, 104 us; here
-// 35, 12, 66).  Chunks of 128 rows are the matrix instructions' own height and halve the chunks' states.  What bounds it: the chain of
-// an item -- keys converted, scores, the state's part, values converted, their part -- beside a few hundred cycles for every
-// conversion, copy and wait in it (8 converting warps instead of 16, 16 columns of the output per store: 39, 12, 69 us).
+// 128 x 128: state 70, carry 68, output 135 us; here, one launch after the other, 26, 17 and 52 us.  Linear attention over fp32 rows,
+// 4 x 2048: 62, 44, 104 us; here 32, 11, 63; with each launch begun while the one before runs, the chain takes 2 to 5 us less).
+// Chunks of 128 rows are the matrix instructions' own height and halve the chunks' states.  What bounds it: the chain of an item --
+// keys converted, scores, the state's part, values converted, their part -- beside a few hundred cycles for every conversion, copy and
+// wait in it: tensor pipe 13 (state) to 28 % (output) active, issue slots 41 to 47 %, DRAM 15 to 33 %, waits on memory and at barriers
+// first among the stalls (8 converting warps instead of 16, 16 columns of the output per store: 39, 12, 69 us).
 #pragma once
 #include <type_traits>
 
@@ -204,15 +206,15 @@ __device__ __forceinline__ CtItem ct_next(const ChunkScanArgs& a, int items, int
     int seq, local, before;
     cs_find<kCtRows>(a.cu_seq, a.n_seqs, a.short_rows, item / per, 0, seq, local, before);
     if (seq < 0) break;                               // the chunks that there are come first
-    const int slot = a.state_slots[seq];
+    const int slot = a.state_slots[seq], first = a.cu_seq[seq], end = a.cu_seq[seq + 1], ctx = a.ctx_lens[seq];      // (one wait)
     if (slot < 0) continue;
-    const int t0 = a.cu_seq[seq] + local * kCtRows;
+    const int t0 = first + local * kCtRows;
     r.item = item;
     r.chunk = item / per;
     r.h = item % per / tiles;
     r.v0 = item % tiles * VT;
-    r.at = {seq, t0, min(kCtRows, a.cu_seq[seq + 1] - t0), slot, local};
-    r.fresh = a.ctx_lens[seq] == 0;
+    r.at = {seq, t0, min(kCtRows, end - t0), slot, local};
+    r.fresh = ctx == 0;
     break;
   }
   return r;
@@ -279,8 +281,9 @@ __device__ __forceinline__ CtExp ct_exp(double v) {
 // chain's kernels write is read past L1.  Every CTA of the second and third launch waits, so that each launch's end is the end of
 // all before it.  Small steps are what it is for, whose code comes from DRAM three times over (L2 cold; launched one after the other
 // -> so; by FMAs over 64 rows): linear attention of 128 rows, 4 heads, 45 -> 30 (38) us, of 1024 rows, 8 heads, 46 -> 38 (44); mLSTM of 200
-// fp32 rows 51 -> 44 (51).  With a normaliser nothing can be formed before the carry's rows are there: the output is released at the
-// carry's end (its CTAs, apart from the start, take longer for 4 x 2048 fp32 rows of 32 heads: 476 -> 487; released at the end 479).
+// fp32 rows 51 -> 44 (51).  With a normaliser nothing can be formed before the carry's rows are there, and a step of more than an
+// item per SM releases the output at the carry's end (its CTAs, apart from the start, take longer for 4 x 2048 fp32 rows of 32 heads:
+// 476 -> 487; released at the end 479).
 __device__ __forceinline__ void ct_release_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void ct_wait_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -595,12 +598,12 @@ ct_state_kernel(const ChunkScanArgs a, const typename Form::Params p, int items)
 // ------------------------------------------------------------------------------------------- carry
 template <int DK, typename Form>
 __global__ void __launch_bounds__(kCtCarryThreads)
-ct_carry_kernel(const ChunkScanArgs a, const typename Form::Params p) {
+ct_carry_kernel(const ChunkScanArgs a, const typename Form::Params p, bool early) {
   __shared__ int base;
   __shared__ float2 table[kCtTable];                  // a chunk's factors: of the state so far, of the chunk's own part
   const int s = blockIdx.z, h = blockIdx.y, tid = threadIdx.x;
   const int t0 = a.cu_seq[s], t1 = a.cu_seq[s + 1], nc = cs_chunks<kCtRows>(t1 - t0, a.short_rows), slot = a.state_slots[s];
-  if constexpr (!Form::kNorm) ct_release_next();
+  if (early) ct_release_next();
   if (nc == 0 || slot < 0) {
     ct_wait_before();
     return;
@@ -654,7 +657,7 @@ ct_carry_kernel(const ChunkScanArgs a, const typename Form::Params p) {
       }
     }
   }
-  if constexpr (Form::kNorm) ct_release_next();
+  if (!early) ct_release_next();
   if (live) { Sp[0] = S[0]; Sp[1] = S[1]; }
   if (blockIdx.x == 0) Form::template carry_row<DK>(p, a, h, base, nc, fresh, slot);
 }
@@ -1105,7 +1108,8 @@ int ct_launch_shape(const ChunkScanArgs& a, const typename Form::Params& p, int6
   const int grid = (int)(items < ct_sms() ? items : ct_sms());
   ct_state_kernel<DK, VT, TA, Form><<<grid, kCtThreads, sb, s>>>(a, p, (int)items);
   const dim3 carry((DK * a.dv / 8 + kCtCarryThreads - 1) / kCtCarryThreads, a.H, a.n_seqs);
-  (void)launch_pdl(ct_carry_kernel<DK, Form>, carry, dim3(kCtCarryThreads), 0, s, 1, a, p);
+  const bool early = !Form::kNorm || items <= ct_sms();
+  (void)launch_pdl(ct_carry_kernel<DK, Form>, carry, dim3(kCtCarryThreads), 0, s, 1, a, p, early);
   (void)launch_pdl(ct_output_kernel<DK, VT, TA, Form>, dim3(grid), dim3(kCtThreads), (size_t)ob, s, 1, a, p, (int)items);
   return b200_check_launch(Form::kName);
 }

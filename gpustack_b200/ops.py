@@ -627,13 +627,15 @@ def mlstm_state_slices(dv: int) -> int:
 # rows beside portions, L2 cold): the one-pass form takes fixed + max(row x longest portion, work x rows x heads), a serial chain or,
 # with CTAs enough, its throughput; the chunk form fixed + work x (rows + wasted x sequences) x heads.  us; work per 1000 rows and
 # heads of `width` = key x value columns; a sequence's first row, which is all of a single one, counts on neither side.  The form
-# taken is at most 11 % slower than the other in any of them.  One-pass -> chunks, 8 heads: linear attention of 64 rows 35 -> 40, of 128
-# 57 -> 42, of 2048 762 -> 71, 16 portions of 32 rows 55 -> 75, of 64 rows 92 -> 81; mLSTM of 128 rows 56 -> 54, of 2048 732 -> 87, 16 of 64
-# rows 114 -> 126, of 128 rows 201 -> 132; gated linear attention of 256 rows 47 -> 50, of 512 84 -> 52, 16 of 128 rows 70 -> 83, of
-# 1024 rows 433 -> 390, one of 2048 beside thirty of 16 449 -> 108; state space of 32 heads: 1024 rows 109 -> 87, 2048 rows
-# 207 -> 140, 16 of 512 rows 399 -> 532, one of 2048 beside thirty of 16 477 -> 195.
-# (Linear attention's and mLSTM's chunks were 64 rows by FMAs then; of 128 rows on the tensor cores since, they take no longer at any of
-# these steps -- linear attention of 128 rows 38 -> 36, mLSTM of 16 portions of 128 rows 101 -> 49 -- so a step that went to them still does.)
+# taken was at most 11 % slower than the other in any of them.  One-pass -> chunks, 8 heads: gated linear attention of 256 rows 47 -> 50,
+# of 512 84 -> 52, 16 of 128 rows 70 -> 83, of 1024 rows 433 -> 390, one of 2048 beside thirty of 16 449 -> 108; state space of 32
+# heads: 1024 rows 109 -> 87, 2048 rows 207 -> 140, 16 of 512 rows 399 -> 532, one of 2048 beside thirty of 16 477 -> 195.
+# Linear attention's and mLSTM's lines lie where their chunks of 64 rows by FMAs crossed the one-pass form.  Of 128 rows on the tensor
+# cores, measured at 432 steps of 1 to 201 sequences of 33 to 2048 rows and 4 to 32 heads: the 294 that go to chunks are faster than
+# one-pass, all of them, and no slower than by FMAs (one by 2 %); of the 138 that stay one-pass 68 would be more than 11 % faster over
+# chunks, up to 2.1 times.  One-pass -> chunks, 8 heads: linear attention of 64 rows 33 -> 28 (stays one-pass), of 128 57 -> 30, of
+# 2048 760 -> 46, 16 portions of 32 rows 53 -> 46 (stays), of 64 92 -> 46; mLSTM over bf16 rows of 128 rows 53 -> 40 (stays), of 2048
+# 712 -> 50, 16 of 64 rows 103 -> 50 (stays), of 128 rows 187 -> 54.
 ChunkCosts = collections.namedtuple("ChunkCosts", "width one_fixed one_row one_work chunk_fixed chunk_work wasted")
 CHUNK_COSTS = {"linear": ChunkCosts(128 * 128, 10.0, 0.37, 6.8, 36.0, 3.0, 0), "mlstm": ChunkCosts(128 * 128, 10.0, 0.36, 8.5, 60.0, 2.6, 32),
                "gated_linear": ChunkCosts(64 * 128, 8.0, 0.146, 2.0, 44.0, 1.8, 0),
@@ -641,13 +643,13 @@ CHUNK_COSTS = {"linear": ChunkCosts(128 * 128, 10.0, 0.37, 6.8, 36.0, 3.0, 0), "
 
 
 def chunk_scan_pays(kind: str, rows: int, n_seqs: int, H: int, dk: int, dv: int, max_len: int) -> bool:
-    """Whether a step of `rows` rows in n_seqs sequences of at most max_len runs faster over chunks side by side.  A bound
-    of all rows of several sequences says nothing about one of them: they are taken for equal."""
+    """Whether a step of `rows` rows in n_seqs sequences of at most max_len runs over chunks side by side: where they are the faster
+    form by CHUNK_COSTS.  A bound of all rows of several sequences says nothing about one of them: they are taken for equal."""
     if dk not in (64, 128) or dv % 4:
         return False
     c = CHUNK_COSTS[kind]
     longest = -(-rows // n_seqs) if max_len == rows and n_seqs > 1 else max_len
-    if longest <= 32:                                   # half a chunk at most: one-pass is the better at every size measured
+    if longest <= 32:                                   # half a chunk of 64 rows at most: over those one-pass was always the better
         return False
     heads = H * dk * dv / c.width / 1000.0
     one = c.one_fixed + max(c.one_row * longest, c.one_work * (rows - n_seqs) * heads)
