@@ -591,6 +591,7 @@ ct_state_kernel(const ChunkScanArgs a, const typename Form::Params p, int items)
       ct_prefetch(x + (int64_t)next.at.first * a.ld + a.v_col + next.h * a.dv + next.v0, a.ld * sizeof(TA), next.at.rows, w);
       item = next.item + (int)gridDim.x;
     }
+    ct_wait_before();                                 // (the short sequences' one-pass kernel, beside which this one runs)
   }
   ct_end(tmem, 4 * VT);
 }
@@ -1098,7 +1099,7 @@ inline int ct_allow(K kernel, int bytes) {
 inline int ct_sms() { return device_info().sm_count > 0 ? device_info().sm_count : 148; }
 
 template <int DK, int VT, typename TA, typename Form>
-int ct_launch_shape(const ChunkScanArgs& a, const typename Form::Params& p, int64_t rows, cudaStream_t s) {
+int ct_launch_shape(const ChunkScanArgs& a, const typename Form::Params& p, int64_t rows, bool beside, cudaStream_t s) {
   const int64_t items = ct_max_chunks(rows, a.n_seqs) * a.H * ((a.dv + VT - 1) / VT);
   constexpr int sb = CtSmem<DK, VT, TA>::kState, ob = CtSmem<DK, VT, TA>::kOutput;
   B200_REQUIRE(items < INT32_MAX - 65536, "chunk scan: too many chunks");
@@ -1106,7 +1107,8 @@ int ct_launch_shape(const ChunkScanArgs& a, const typename Form::Params& p, int6
   if (rc == B200_OK) rc = ct_allow(ct_output_kernel<DK, VT, TA, Form>, ob);
   if (rc != B200_OK) return rc;
   const int grid = (int)(items < ct_sms() ? items : ct_sms());
-  ct_state_kernel<DK, VT, TA, Form><<<grid, kCtThreads, sb, s>>>(a, p, (int)items);
+  if (beside) (void)launch_pdl(ct_state_kernel<DK, VT, TA, Form>, dim3(grid), dim3(kCtThreads), (size_t)sb, s, 1, a, p, (int)items);
+  else ct_state_kernel<DK, VT, TA, Form><<<grid, kCtThreads, sb, s>>>(a, p, (int)items);
   const dim3 carry((DK * a.dv / 8 + kCtCarryThreads - 1) / kCtCarryThreads, a.H, a.n_seqs);
   const bool early = !Form::kNorm || items <= ct_sms();
   (void)launch_pdl(ct_carry_kernel<DK, Form>, carry, dim3(kCtCarryThreads), 0, s, 1, a, p, early);
@@ -1114,19 +1116,24 @@ int ct_launch_shape(const ChunkScanArgs& a, const typename Form::Params& p, int6
   return b200_check_launch(Form::kName);
 }
 
-// group: sequences per walk (ct_group)
+// group: sequences per walk (ct_group).  The sequences of at most a.short_rows rows are in a one-pass kernel launched just before: it writes
+// other slots and rows than the chunks.  Where sequences of 48 rows or fewer on average say that there are such, the chunks begin
+// beside it (one portion of 2048 rows beside 64 single ones, mLSTM, 2 heads of 64 x 64: 62.5 -> 52.7 us, by FMAs 59.4; four of 512
+// without any, 8 heads of 128 x 128, would take 58.3 instead of 56.3).
 template <typename TA, typename Form>
 int ct_launch(ChunkScanArgs a, const typename Form::Params& p, int dk, int64_t rows, int group, float* ws, cudaStream_t s) {
   a.ws = ws;
   a.ws_row_width = dk + 4;
   int rc = B200_OK;
+  bool beside = a.short_rows > 0 && rows <= 48 * (int64_t)a.n_seqs;
   for (int left = a.n_seqs; left > 0 && rc == B200_OK; left -= group) {
     a.n_seqs = left < group ? left : group;
     const int64_t chunks = ct_max_chunks(rows, a.n_seqs);
     if (chunks == 0) break;
     a.ws_row = ws + ct_state_floats(chunks, a.H, dk, a.dv);
-    if (dk == 64) rc = a.dv <= 64 ? ct_launch_shape<64, 64, TA, Form>(a, p, rows, s) : ct_launch_shape<64, 128, TA, Form>(a, p, rows, s);
-    else rc = a.dv <= 64 ? ct_launch_shape<128, 64, TA, Form>(a, p, rows, s) : ct_launch_shape<128, 128, TA, Form>(a, p, rows, s);
+    if (dk == 64) rc = a.dv <= 64 ? ct_launch_shape<64, 64, TA, Form>(a, p, rows, beside, s) : ct_launch_shape<64, 128, TA, Form>(a, p, rows, beside, s);
+    else rc = a.dv <= 64 ? ct_launch_shape<128, 64, TA, Form>(a, p, rows, beside, s) : ct_launch_shape<128, 128, TA, Form>(a, p, rows, beside, s);
+    beside = false;
     a.cu_seq += group;
     a.ctx_lens += group;
     a.state_slots += group;

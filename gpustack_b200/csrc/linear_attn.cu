@@ -250,6 +250,7 @@ linattn_chunk4_kernel(const float* __restrict__ x, int64_t ld, int q_col, int k_
                       const float* __restrict__ decay, const int32_t* __restrict__ cu_seq,
                       const int32_t* __restrict__ ctx_lens, const int32_t* __restrict__ state_slots, float* S_state,
                       float* __restrict__ o_raw, int H, int dk, int dv, int most_rows) {
+  if (most_rows != INT32_MAX) ct_release_next();      // the other sequences' chunks, which touch nothing of these
   extern __shared__ __align__(16) float smem[];
   const int kst = dk + 4;
   float* Ssm = smem;                                  // [dk][33]

@@ -401,6 +401,7 @@ mlstm_chunk4_kernel(const TA* __restrict__ proj, int64_t ld, int q_col, int k_co
   const int slot = state_slots[s];
   if (slot < 0) return;
   const int t0 = cu_seq[s], t1 = cu_seq[s + 1];
+  if (most_rows != INT32_MAX) ct_release_next();      // the other sequences' chunks, which touch nothing of these
   if (t1 <= t0 || t1 - t0 > most_rows) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int c0 = z * 32;

@@ -165,11 +165,11 @@ def test_launches_that_begin_early(kind, dtype, how):
     from gpustack_b200 import config, ops
 
     H, dk, dv = 3, 128, 128
-    steps = [[130], [700, 40], [64, 65, 1], [300], [2500], [129]] * 4
+    steps = [[130], [700, 40], [64, 65, 1], [300] + [1] * 20, [2500], [129]] * 4       # chunks also beside a one-pass kernel
     g = torch.Generator(device="cuda").manual_seed(1)
     draw = lambda *s: torch.randn(*s, generator=g, device="cuda")   # noqa: E731
     i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")   # noqa: E731
-    ws = torch.empty(config.chunk_scan_floats(4096, 8, H, dk, dv), device="cuda")
+    ws = torch.empty(config.chunk_scan_floats(4096, 32, H, dk, dv), device="cuda")
     calls, states = [], []
     for lens in steps:
         T, n, Z = sum(lens), len(lens), ops.mlstm_state_slices(dv)
