@@ -127,8 +127,9 @@ __device__ __forceinline__ void ct_store(const CtBlocks<TA>& b, int blocks, uint
 }
 
 // An infinite number (or one that rounds to one) has no three terms: every product with it is no number, where an fp32 FMA may give an
-// infinite one.  What comes out of the products neither finite nor zero is formed again by FMAs: its place is told by adding up
-// zero times the results, which is zero for finite ones alone.
+// infinite one.  What comes out of the products not finite is formed again by FMAs, in its place; that there is such is told by adding up
+// zero times the results, which is zero for finite ones alone.  (With every value of 4 x 2048 rows
+// infinite, 8 heads of 128 x 128: 51 ms; with every key no number, which ends a sum, 4 ms.)
 struct CtFinite {
   cs_f2 sum = 0ull;
   __device__ __forceinline__ void add(float a, float b) { sum = cs_fma(cs_pack(a, b), 0ull, sum); }
@@ -138,7 +139,7 @@ struct CtFinite {
   }
 };
 __device__ __forceinline__ bool ct_number(float x) { return fabsf(x) < INFINITY; }
-// k . q; sum of w_s k_s v_s over rows, until it is no number; q times a row of the state's terms
+// k . q; sum of w_s k_s v_s over rows, until it is no number
 template <typename TA>
 __device__ __noinline__ float ct_dot(const TA* q, const TA* k, int dk) {
   float acc = 0.f;
