@@ -11,12 +11,20 @@
 //
 // Every value column of S is a recurrence of its own, so columns are the unit of work: L lanes share C neighbouring columns,
 // lane l holds the key entries 4 (i L + l) .. + 3 (i < R4) of each in registers, and a warp walks its C 32 / L columns
-// through the sequence's new rows one token after the other.  Per token: S^T k (a butterfly over the L lanes; delta rule
-// only), the update, and the lane's share of S^T q.  Those shares stay in registers for 8 tokens and are then summed over the
-// lanes in one transposing exchange (about 2 shuffles a token).  A token's keys and queries are read from shared memory once
-// per lane and serve its C columns: with one column that read, not the arithmetic, bounds the walk.  Keys, queries, values and gates are staged 16 or 32 tokens at a time by
-// cp.async into two buffers, so the walk never waits for memory; a column's sums do not depend on how a prompt was cut
-// beyond the order of the lanes' addends in S^T q.
+// through the sequence's new rows in blocks of four tokens.  Of a block, with G_j the product of its decays up to token j and D_ij
+// of those behind token i up to j:
+//   u_j = beta_j v_j - beta_j G_j S^T k_j - sum_(i < j) beta_j D_ij (k_i . k_j) u_i       (state space: beta_j v_j)
+//   o_j = G_j S^T q_j + sum_(i <= j) D_ij (k_i . q_j) u_i,      S <- G_3 S + sum_i D_i3 k_i u_i^T
+// so S^T k and S^T q of all four tokens come from the state before the block: their sums over the lanes travel together, and the
+// state is scaled once for four tokens.  Token by token, as this was, each token waits for a sum over the lanes: 680 us for the delta
+// rule over 4 x 2048 rows of 16 heads of 128 x 128 where blocks take 467 (fp32 pipe some 55 % busy), 453 -> 343 for the state space of
+// 32 heads of 128 x 64.  Errors against 64 bits are no larger (delta rule 4 x 600 rows: outputs 1.23e-7 -> 1.17e-7, states 1.61e-7 -> 1.50e-7;
+// state space 1.38e-7 -> 1.35e-7, 1.61e-7 -> 1.49e-7; rows of one sign 5.86e-8 -> 5.86e-8 and 1.43e-7 -> 1.45e-7, states 6 % less).
+// What bounds it is one warp's issue: the products of a token go column by column in turn so that four chains cover an FMA's latency,
+// and a token's sum over the lanes goes on a level per product that follows.  Of no use: eight warps of half the columns each (+6 %),
+// key rows held over the block instead of read twice, queries a block ahead (+10 %, registers).
+// Beside the four warps that walk, four warps stage rows by cp.async (16 tokens a stage), form a block's factors each, ahead of the
+// walk, and write the outputs: the walk itself reads neither gates nor global memory.
 // The state-space recurrence over prompts, with a workspace, runs over chunks of 64 rows side by side instead (chunk_scan.cuh).
 #include "chunk_scan.cuh"
 #include "common.cuh"
@@ -24,8 +32,6 @@
 #include "../../include/b200.h"
 
 namespace b200 {
-
-constexpr int kGsWarps = 8;
 
 struct GatedScanArgs {
   const float* x;
@@ -82,10 +88,6 @@ __device__ __forceinline__ float2 gs_gate(float a, float b, float rate, float bi
   return make_float2(expf(-rate * sp), DELTA ? 1.0f / (1.0f + expf(-b)) : sp);
 }
 
-__device__ __forceinline__ void cp16(float* dst, const float* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-
 template <int L>
 __device__ __forceinline__ float lanes_sum(float v) {
 #pragma unroll
@@ -93,64 +95,29 @@ __device__ __forceinline__ float lanes_sum(float v) {
   return v;
 }
 
-// the lane's shares of S^T x for C columns
+// the lane's shares of S^T x for C columns, a column's entries in turn with the others'
 template <int R2, int C>
 __device__ __forceinline__ void gs_dot(const f32x2 (&S)[C][R2], const f32x2 (&x)[R2], float (&o)[C]) {
+  f32x2 p[C];
 #pragma unroll
-  for (int c = 0; c < C; ++c) {
-    f32x2 p0 = mul2(S[c][0], x[0]), p1 = mul2(S[c][1], x[1]);
+  for (int c = 0; c < C; ++c) p[c] = mul2(S[c][0], x[0]);
 #pragma unroll
-    for (int i = 2; i < R2; i += 2) {
-      p0 = fma2(S[c][i], x[i], p0);
-      p1 = fma2(S[c][i + 1], x[i + 1], p1);
-    }
-    o[c] = sum2(add2(p0, p1));
-  }
+  for (int i = 1; i < R2; ++i)
+#pragma unroll
+    for (int c = 0; c < C; ++c) p[c] = fma2(S[c][i], x[i], p[c]);
+#pragma unroll
+  for (int c = 0; c < C; ++c) o[c] = sum2(p[c]);
 }
-
-// sums over the L lanes of a group, in every lane.  Two columns: the lanes' halves take one each and exchange the sums.
-template <int L, int C>
-__device__ __forceinline__ void gs_lanes_sum(float (&p)[C]) {
-  if constexpr (C == 2 && L > 8) {
-    const bool hi = threadIdx.x & (L / 2);
-    float mine = (hi ? p[1] : p[0]) + __shfl_xor_sync(0xffffffffu, hi ? p[0] : p[1], L / 2);
+// ... for one column, in two chains
+template <int R2>
+__device__ __forceinline__ float gs_dot1(const f32x2 (&S)[R2], const f32x2 (&x)[R2]) {
+  f32x2 p0 = mul2(S[0], x[0]), p1 = mul2(S[1], x[1]);
 #pragma unroll
-    for (int w = L / 4; w > 0; w >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, w);
-    const float other = __shfl_xor_sync(0xffffffffu, mine, L / 2);
-    p[0] = hi ? other : mine;
-    p[1] = hi ? mine : other;
-  } else {
-#pragma unroll
-    for (int w = L / 2; w > 0; w >>= 1)
-#pragma unroll
-      for (int c = 0; c < C; ++c) p[c] += __shfl_xor_sync(0xffffffffu, p[c], w);
+  for (int i = 2; i < R2; i += 2) {
+    p0 = fma2(S[i], x[i], p0);
+    p1 = fma2(S[i + 1], x[i + 1], p1);
   }
-}
-
-// One token of C columns: S <- g S + k u^T with u = beta v, or beta (v - g S^T k) for the delta rule.  The read-out of the
-// token BEFORE (o, from q; none for a block's first token) and the decay of S need no other lane: they run while the
-// butterfly's shuffles are in flight.
-template <int L, int R2, int C, bool DELTA, bool READ>
-__device__ __forceinline__ void gs_token(f32x2 (&S)[C][R2], const f32x2 (&k)[R2], const f32x2 (&q)[R2], const float (&v)[C], float2 gb,
-                                         float (&o)[C]) {
-  float p[C];
-  if (DELTA) {
-    gs_dot<R2, C>(S, k, p);
-    gs_lanes_sum<L, C>(p);
-  }
-  if (READ) gs_dot<R2, C>(S, q, o);
-  const f32x2 g2 = pack2(gb.x, gb.x);
-#pragma unroll
-  for (int c = 0; c < C; ++c)
-#pragma unroll
-    for (int i = 0; i < R2; ++i) S[c][i] = mul2(g2, S[c][i]);
-#pragma unroll
-  for (int c = 0; c < C; ++c) {
-    const float u = DELTA ? gb.y * (v[c] - gb.x * p[c]) : gb.y * v[c];
-    const f32x2 u2 = pack2(u, u);
-#pragma unroll
-    for (int i = 0; i < R2; ++i) S[c][i] = fma2(k[i], u2, S[c][i]);
-  }
+  return sum2(add2(p0, p1));
 }
 
 // 4 R4 entries of a row of key entries: lane l of L takes entries 4 (i L + l) .. + 3
@@ -164,172 +131,376 @@ __device__ __forceinline__ void gs_row(const float* __restrict__ row, int l, f32
   }
 }
 
-template <int L, int R4, int C, int TOK, bool DELTA>
-__global__ void __launch_bounds__(kGsWarps * 32, C * R4 <= 4 ? 2 : 1)
+// 16 bytes of global memory -> shared memory, or zeros
+__device__ __forceinline__ void gs_copy(float* to, const float* from, bool there) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(to)), "l"(from), "r"(there ? 16 : 0) : "memory");
+}
+// what rounding left of sum = a + b
+__device__ __forceinline__ float gs_left(float a, float b, float sum) {
+  const float t = sum - a;
+  return (a - (sum - t)) + (b - t);
+}
+
+// Shares p[column][token] of the L lanes that hold the same columns -> lane l's column 0, summed over them, a level at a time: first
+// l ^ 1, .. l ^ (C - 1) exchange columns, then all add.  A lane counts its columns from its own: number c is column c ^ (l % C),
+// so what a lane keeps and what it gives away have the same numbers in every lane.
+template <int C>
+__device__ __forceinline__ void gs_level(float (&p)[C][4], int j, int level) {
+  const int w = C >> (level + 1);
+  if (w > 0) {
+#pragma unroll
+    for (int c = 0; c < w; ++c) p[c][j] += __shfl_xor_sync(0xffffffffu, p[c + w][j], w);
+  } else {
+    p[0][j] += __shfl_xor_sync(0xffffffffu, p[0][j], (C << level) / C);
+  }
+}
+constexpr int gs_log2(int n) { return n <= 1 ? 0 : 1 + gs_log2(n / 2); }
+
+constexpr int kGsWarps = 4;                            // warps that walk columns
+constexpr int kGsStepWarps = 8;                        // of the single rows' kernel
+constexpr int kGsSms = 148;
+constexpr int kGsTile = 4;                             // tokens of a block
+constexpr int kGsHelpers = 4;                          // warps that stage rows and form the factors of a block each: blocks of a stage
+constexpr int kGsStage = kGsHelpers * kGsTile;
+// A block's factors in shared memory, floats: beta_j | D_03 D_13 D_23 G_3 | G_j | what rounding left of G_j | D_ij k_i.k_j (i < j) |
+// D_ij k_i.q_j (row j, i <= j).  An error of theirs is one of every column and entry, which nothing averages out: decays and the last sums of
+// the products are formed in 64 bits and rounded once, and an output's last sum takes along what its rounding leaves (fp32 throughout:
+// outputs 3 to 8 % further off than token by token, 19 % over rows of one sign; all of it in 64 bits: the walk waits for it, 328 -> 379 us
+// for the state space of 4 x 2048 rows).
+constexpr int kGsBeta = 0, kGsD3 = 4, kGsG = 8, kGsGl = 12, kGsA = 16, kGsB = 24, kGsFactors = 40;
+
+template <int L, int R4, int C>
+struct GsShape {
+  static constexpr int DKP = 4 * R4 * L, CPW = C * 32 / L, BUFS = DKP <= 256 ? 4 : 2;
+  // stages that factors are ahead of outputs: one holds up a walk of few entries per lane (state space, one sequence of 2048 rows: 207 us,
+  // with two 184), with two a short portion of many takes longer (8 of 8 rows 12.2 and 14.3)
+  static constexpr int AHEAD = C * R4 <= 4 ? 2 : 1;
+  static constexpr int VW = kGsWarps * CPW;
+  static constexpr int OUT = 4 * (L / C + 1);         // of a column and block: what the steps u are, and its lanes' shares of the read-outs
+  static constexpr int kFloats = kGsHelpers * (BUFS * (kGsTile * (2 * DKP + VW) + kGsFactors) + (AHEAD + 1) * VW * OUT);
+  static constexpr size_t kBytes = sizeof(float) * kFloats + 2 * BUFS * sizeof(uint64_t);
+};
+
+template <int L, int R4, int C, bool DELTA>
+__global__ void __launch_bounds__((kGsWarps + kGsHelpers) * 32, C * R4 <= 8 ? 2 : 1)
 gated_scan_kernel(GatedScanArgs a) {
   extern __shared__ __align__(16) float smem[];
-  constexpr int R2 = 2 * R4, DKP = 4 * R4 * L, CPW = C * 32 / L, COLS = kGsWarps * CPW, OP = COLS + 8;
-  float* ks = smem;                                   // [2][TOK][DKP]
-  float* qs = ks + 2 * TOK * DKP;                  // [2][TOK][DKP]
-  float* vs = qs + 2 * TOK * DKP;                  // [2][TOK][COLS]
-  float2* gb = reinterpret_cast<float2*>(vs + 2 * TOK * COLS);   // [2][TOK]
-  float* os = reinterpret_cast<float*>(gb + 2 * TOK);            // [TOK][OP]
-  const int s = blockIdx.x, h = blockIdx.y, z = blockIdx.z, tid = threadIdx.x;
-  const int slot = a.state_slots[s];
-  if (slot < 0) return;
-  const int t0 = a.cu_seq[s], t1 = a.cu_seq[s + 1];
-  if (t1 <= t0 || t1 - t0 > a.most_rows) return;
-  const int warp = tid >> 5, lane = tid & 31, l = lane % L;
-  const int cw = warp * CPW + lane / L * C, col = z * COLS + cw;     // this lane's first column, in the CTA and in the head
-  const int hk = h / (a.H / a.G);
-  const int dkp = a.dkp;
-  float* Sp = a.S + (((size_t)slot * a.H + h) * a.dv + col) * dkp;
-  const bool fresh = a.ctx_lens[s] == 0;
-  f32x2 S[C][R2];
-#pragma unroll
-  for (int c = 0; c < C; ++c)
-#pragma unroll
-    for (int i = 0; i < R4; ++i) {
-      ulonglong2 t = make_ulonglong2(0, 0);
-      if (!fresh && col + c < a.dv && 4 * (i * L + l) < dkp) t = *reinterpret_cast<const ulonglong2*>(Sp + c * dkp + 4 * (i * L + l));
-      S[c][2 * i] = t.x;
-      S[c][2 * i + 1] = t.y;
+  using Sh = GsShape<L, R4, C>;
+  constexpr int R2 = 2 * R4, DKP = Sh::DKP, CPW = Sh::CPW, BUFS = Sh::BUFS, VW = Sh::VW, BLOCKS = kGsHelpers, AHEAD = Sh::AHEAD;
+  float* ks = smem;                                   // [BUFS][kGsStage][DKP]
+  float* qs = ks + BUFS * kGsStage * DKP;             // [BUFS][kGsStage][DKP]
+  float* vs = qs + BUFS * kGsStage * DKP;             // [BUFS][kGsStage][VW]
+  float* fs = vs + BUFS * kGsStage * VW;              // [BUFS][BLOCKS][kGsFactors]
+  float* os = fs + BUFS * BLOCKS * kGsFactors;        // [AHEAD + 1][BLOCKS][L / C + 1][VW][4]
+  uint64_t* factors_full = reinterpret_cast<uint64_t*>(os + (AHEAD + 1) * BLOCKS * VW * Sh::OUT);     // [BUFS] each
+  uint64_t* empty = factors_full + BUFS;
+  const int s = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int col0 = blockIdx.z * VW;
+  const int slot = a.state_slots[s], t0 = a.cu_seq[s], t1 = a.cu_seq[s + 1], ctx = a.ctx_lens[s];      // (one wait)
+  if (slot < 0 || t1 <= t0 || t1 - t0 > a.most_rows) return;
+  const int dkp = a.dkp, rows = t1 - t0, blocks = (rows + kGsTile - 1) / kGsTile, stages = (blocks + BLOCKS - 1) / BLOCKS;
+  if (tid == 0) {
+    for (int i = 0; i < BUFS; ++i) {
+      mbar_init(&factors_full[i], kGsHelpers);
+      mbar_init(&empty[i], kGsWarps);
     }
-  // key entries behind dkp: zeros in both buffers, written once
+    fence_mbar_init();
+  }
+  // key entries behind dkp: zeros in all buffers, written once
   if (dkp < DKP) {
     const int pad = DKP - dkp;
-    for (int i = tid; i < 2 * TOK * pad; i += kGsWarps * 32) {
+    for (int i = tid; i < BUFS * kGsStage * pad; i += (kGsWarps + kGsHelpers) * 32) {
       const int r = i / pad, d = dkp + i % pad;
       ks[r * DKP + d] = 0.f;
       qs[r * DKP + d] = 0.f;
     }
   }
-  const float rate = a.rate[h], bias = a.dt_bias[h];
-  const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-  // this thread's share of the staging: entries d0 .. d0 + 3 of rows tt0, tt0 + per_pass, ... (dkp <= 512: at least one pass)
-  const int dk4 = dkp >> 2, per_pass = kGsWarps * 32 / dk4, d0 = tid % dk4 * 4;
-  const int tt0 = tid / dk4 < per_pass ? tid / dk4 : TOK;
-  const float* src = a.x + hk * dkp + d0;
-  auto stage = [&](int ch, int buf) {                 // rows ch .. ch + TOK - 1; rows behind the portion are zeros
-    const int nt = min(TOK, t1 - ch);
-    for (int tt = tt0; tt < TOK; tt += per_pass) {
-      const int to = (buf * TOK + tt) * DKP + d0;
-      if (tt < nt) {
-        const float* row = src + (size_t)(ch + tt) * a.ld;
-        cp16(ks + to, row + a.k_col);
-        cp16(qs + to, row + a.q_col);
-      } else {
-        *reinterpret_cast<float4*>(ks + to) = zero4;
-        *reinterpret_cast<float4*>(qs + to) = zero4;
+  // the lane's columns are group .. group + C - 1, counted from its own: number c is column group + (c ^ l % C)
+  const int l = lane % L, group = warp * CPW + lane / L * C, mine = group + l % C;
+  float* Sp = a.S + (((size_t)slot * a.H + h) * a.dv + col0) * dkp;
+  f32x2 S[C][R2];
+  if (warp < kGsWarps) {                               // (on its way beside the first rows)
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+#pragma unroll
+      for (int i = 0; i < R4; ++i) {
+        ulonglong2 t = make_ulonglong2(0, 0);
+        const int col = group + (c ^ l % C);
+        if (ctx != 0 && col0 + col < a.dv && 4 * (i * L + l) < dkp) t = *reinterpret_cast<const ulonglong2*>(Sp + (size_t)col * dkp + 4 * (i * L + l));
+        S[c][2 * i] = t.x;
+        S[c][2 * i + 1] = t.y;
       }
-    }
-    for (int i = tid; i < TOK * (COLS / 4); i += kGsWarps * 32) {
-      const int tt = i / (COLS / 4), c = (i - tt * (COLS / 4)) * 4;
-      float* to = vs + (buf * TOK + tt) * COLS + c;
-      if (tt < nt && z * COLS + c < a.dvp) cp16(to, a.x + (size_t)(ch + tt) * a.ld + a.v_col + h * a.dvp + z * COLS + c);
-      else *reinterpret_cast<float4*>(to) = zero4;
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  float ra = 0.f, rb = 0.f;
-  auto raw_gates = [&](int ch) {
-    if (tid < TOK && ch + tid < t1) {
-      const float* g = a.gates + (size_t)(ch + tid) * a.ld_g;
-      ra = DELTA ? g[a.H + h] : g[h];
-      if (DELTA) rb = g[h];
-    }
-  };
-  auto put_gates = [&](int ch, int buf) {             // rows behind the portion: decay 1, step 0 (the state stays)
-    if (tid < TOK) gb[buf * TOK + tid] = ch + tid < t1 ? gs_gate<DELTA>(ra, rb, rate, bias) : make_float2(1.f, 0.f);
-  };
-  stage(t0, 0);
-  raw_gates(t0);
-  put_gates(t0, 0);
-  int buf = 0;
-  for (int ch = t0; ch < t1; ch += TOK, buf ^= 1) {
-    const int nt = min(TOK, t1 - ch), next = ch + TOK;
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();                                  // this chunk is staged; the last one's outputs have left os
-    if (next < t1) {
-      stage(next, buf ^ 1);
-      raw_gates(next);
-    }
+  }
+  __syncthreads();
+
+  if (warp >= kGsWarps) {
+    // ------------------------------------------------------------------ staging, and a block's factors per warp and stage
+    const int helper = warp - kGsWarps, n = lane & 15, j = n & 3, lo = min(n >> 2, j), hi = max(n >> 2, j);
+    const bool upper = j > n >> 2;                    // lane n: the pair (row n / 4, column n % 4); above the diagonal keys with keys
+    const int hk = h / (a.H / a.G), v4 = min(VW, a.dvp - col0) >> 2;
+    const float rate = a.rate[h], bias = a.dt_bias[h];
+    const float* x = a.x + (size_t)t0 * a.ld + lane * 4;
+    const int kc = a.k_col + hk * dkp, qc = a.q_col + hk * dkp, vc = a.v_col + h * a.dvp + col0;
+    auto stage = [&](int st) {                        // the rows of this warp's block; those behind the portion are zeros
+      const int from = (st * BLOCKS + helper) * kGsTile, to = (st % BUFS * BLOCKS + helper) * kGsTile;
+#pragma unroll
+      for (int r = 0; r < kGsTile; ++r) {
+        const bool there = from + r < rows;
+        const float* row = x + (size_t)min(from + r, rows - 1) * a.ld;
+#pragma unroll
+        for (int d = 0; d < DKP; d += 128)
+          if (d + lane * 4 < dkp) {
+            gs_copy(ks + (to + r) * DKP + d + lane * 4, row + kc + d, there);
+            gs_copy(qs + (to + r) * DKP + d + lane * 4, row + qc + d, there);
+          }
+        if (lane < v4) gs_copy(vs + (to + r) * VW + lane * 4, row + vc, there);
+      }
+    };
+    float ra = 0.f, rb = 0.f;
+    auto raw_gates = [&](int st) {
+      const int t = (st * BLOCKS + helper) * kGsTile + j;
+      if (t < rows) {
+        const float* g = a.gates + (size_t)(t0 + t) * a.ld_g;
+        ra = DELTA ? g[a.H + h] : g[h];
+        if (DELTA) rb = g[h];
+      }
+    };
+    // outputs of this warp's block: the read-out of the state before it and what its own tokens add
+    const float skip = a.skip != nullptr ? a.skip[h] : 0.f;
+    auto put = [&](int st) {
+      mbar_wait_guarded(&empty[st % BUFS], (st / BUFS) & 1);
+      const int b = st * BLOCKS + helper, at = st % BUFS * BLOCKS + helper;
+      const float* f = fs + at * kGsFactors;
+      const float* ob = os + (st % (AHEAD + 1) * BLOCKS + helper) * VW * Sh::OUT;
+      float G[4], Gl[4], B[10];
+#pragma unroll
+      for (int i = 0, n = 0; i < 4; ++i) {
+        G[i] = f[kGsG + i];
+        Gl[i] = f[kGsGl + i];
+#pragma unroll
+        for (int e = 0; e <= i; ++e) B[n++] = f[kGsB + 4 * i + e];
+      }
+      for (int c = lane; c < VW && col0 + c < a.dv; c += 32) {
+        const float4 uf = *reinterpret_cast<const float4*>(ob + c * 4);
+        const float u[4] = {uf.x, uf.y, uf.z, uf.w};
+        float r[2][4];                                 // two halves of the lanes' shares
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) r[e][i] = 0.f;
+#pragma unroll
+        for (int i = 0; i < L / C; ++i) {
+          const float4 m = *reinterpret_cast<const float4*>(ob + ((i + 1) * VW + c) * 4);
+          float (&h2)[4] = r[2 * i >= L / C && L > C];
+          h2[0] += m.x; h2[1] += m.y; h2[2] += m.z; h2[3] += m.w;
+        }
+        const float* v = vs + at * kGsTile * VW + c;
+        float* out = a.o + (size_t)(t0 + b * kGsTile) * a.H * a.dv + h * a.dv + col0 + c;
+#pragma unroll
+        for (int i = 0, n = 0; i < 4; ++i) {
+          float y = B[n] * u[0], low = DELTA ? fmaf(B[n], u[0], -y) : 0.f;
+          ++n;
+#pragma unroll
+          for (int e = 1; e <= i; ++e, ++n) {
+            if (DELTA) {                               // (whose steps take values back: what their sum's rounding leaves counts too)
+              const float m = B[n] * u[e], z = y + m;
+              low += gs_left(y, m, z) + fmaf(B[n], u[e], -m);
+              y = z;
+            } else {
+              y = fmaf(B[n], u[e], y);
+            }
+          }
+          y = fmaf(skip, v[i * VW], y);
+          const float R = r[0][i] + r[1][i], left = gs_left(r[0][i], r[1][i], R), P = G[i] * R, sum = P + y;
+          low += gs_left(P, y, sum) + fmaf(Gl[i], R, fmaf(G[i], left, fmaf(G[i], R, -P)));
+          y = fabsf(sum) < INFINITY ? sum + low : sum;
+          if (b * kGsTile + i < rows) out[(size_t)i * a.H * a.dv] = y;
+        }
+      }
+    };
+    auto factors = [&](int st) {
+      const int b = st * BLOCKS + helper, at = st % BUFS * BLOCKS + helper;
+      const float2 gb = b * kGsTile + j < rows ? gs_gate<DELTA>(ra, rb, rate, bias) : make_float2(1.f, 0.f);   // (behind the portion the state stays)
+      if (st + 1 < stages) raw_gates(st + 1);
+      const float g0 = __shfl_sync(0xffffffffu, gb.x, 0), g1 = __shfl_sync(0xffffffffu, gb.x, 1), g2 = __shfl_sync(0xffffffffu, gb.x, 2),
+                  g3 = __shfl_sync(0xffffffffu, gb.x, 3);
+      double decay = 1.0;                             // from token lo to token hi
+      if (lo < 1 && hi >= 1) decay = g1;
+      if (lo < 2 && hi >= 2) decay *= g2;
+      if (lo < 3 && hi >= 3) decay *= g3;
+      asm volatile("cp.async.wait_group %0;" ::"n"(BUFS - AHEAD - 1) : "memory");
+      __syncwarp();
+      float dot[16];
+      {
+        f32x2 d2[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) d2[i] = 0;
+        const float* kb = ks + at * kGsTile * DKP;
+        const float* qb = qs + at * kGsTile * DKP;
 #pragma unroll 1
-    for (int tb = 0; tb < nt; tb += 8) {
-      float o[8][C];
-      f32x2 k[2][R2], q[2][R2];      // this token's and the next one's keys; the last token's and this one's queries
-      const float* kr = ks + (buf * TOK + tb) * DKP;
-      const float* qr = qs + (buf * TOK + tb) * DKP;
-      const float* vr = vs + (buf * TOK + tb) * COLS + cw;
-      const float2* gr = gb + buf * TOK + tb;
-      gs_row<L, R4>(kr, l, k[0]);
+        for (int d = lane * 4; d < DKP; d += 128) {
+          ulonglong2 k[4], q[4];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        float v[C];
+          for (int i = 0; i < 4; ++i) {
+            k[i] = *reinterpret_cast<const ulonglong2*>(kb + i * DKP + d);
+            q[i] = *reinterpret_cast<const ulonglong2*>(qb + i * DKP + d);
+          }
 #pragma unroll
-        for (int c = 0; c < C; ++c) v[c] = vr[j * COLS + c];
-        if (j < 7) gs_row<L, R4>(kr + (j + 1) * DKP, l, k[(j + 1) & 1]);
-        gs_row<L, R4>(qr + j * DKP, l, q[j & 1]);
-        if (j == 0) gs_token<L, R2, C, DELTA, false>(S, k[0], q[1], v, gr[0], o[0]);
-        else gs_token<L, R2, C, DELTA, true>(S, k[j & 1], q[(j + 1) & 1], v, gr[j], o[j - 1]);
+          for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              if (c <= r) d2[r * 4 + c] = fma2(k[c].y, q[r].y, fma2(k[c].x, q[r].x, d2[r * 4 + c]));
+              else if (DELTA) d2[r * 4 + c] = fma2(k[c].y, k[r].y, fma2(k[c].x, k[r].x, d2[r * 4 + c]));
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) dot[i] = sum2(d2[i]);
       }
-      gs_dot<R2, C>(S, q[1], o[7]);
-      // lane l ends with token tb + (l & 7), summed over the columns' lanes
-      const bool b4 = l & 4, b2 = l & 2, b1 = l & 1;
-      float sum[C];
+#pragma unroll
+      for (int w = 8; w > 2; w >>= 1) {                // lanes n and n + 16 end with pair n
+        const bool up = n & w;
+#pragma unroll
+        for (int i = 0; i < w; ++i) {
+          const float own = up ? dot[i + w] : dot[i], other = up ? dot[i] : dot[i + w];
+          dot[i] = own + __shfl_xor_sync(0xffffffffu, other, w);
+        }
+      }
+      double sum[4] = {dot[0], dot[1], dot[2], dot[3]};
+#pragma unroll
+      for (int w = 2; w > 0; w >>= 1) {
+        const bool up = n & w;
+#pragma unroll
+        for (int i = 0; i < w; ++i) {
+          const double own = up ? sum[i + w] : sum[i], other = up ? sum[i] : sum[i + w];
+          sum[i] = own + __shfl_xor_sync(0xffffffffu, other, w);
+        }
+      }
+      sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], 16);
+      float* f = fs + at * kGsFactors;
+      if (lane < 16) {
+        f[upper ? kGsA + hi * (hi - 1) / 2 + lo : kGsB + n] = (float)(decay * sum[0]);
+      } else if (lane < 20) {
+        double G = g0, D3 = 1.0;
+        if (n >= 1) G *= g1;
+        if (n >= 2) G *= g2;
+        if (n >= 3) G *= g3;
+        if (n < 1) D3 = g1;
+        if (n < 2) D3 *= g2;
+        if (n < 3) D3 *= g3;
+        const float high = (float)G;
+        f[kGsBeta + n] = gb.y;
+        f[kGsG + n] = high;
+        f[kGsGl + n] = (float)(G - high);
+        f[kGsD3 + n] = n == 3 ? high : (float)D3;
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&factors_full[st % BUFS]);
+    };
+    raw_gates(0);
+    // a stage's factors, the outputs of the one AHEAD before it, then the rows of the next one for its buffer: none of the walk's
+    // stages waits for outputs or copies.  A warp copies, reads and writes out its own block only.
+    for (int st = AHEAD - BUFS; st < stages + AHEAD; ++st) {
+      if (st >= 0 && st < stages) factors(st);
+      if (st >= AHEAD) put(st - AHEAD);
+      if (st - AHEAD + BUFS < stages) stage(st - AHEAD + BUFS);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    return;
+  }
+
+  // -------------------------------------------------------------------- the walk
+  constexpr int LV = gs_log2(L), LC = gs_log2(C);
+  mbar_wait_guarded(&factors_full[0], 0);             // (a stage's rows have landed when its factors are there)
+#pragma unroll 1
+  for (int b = 0; b < blocks; ++b) {
+    const int at = b % (BUFS * BLOCKS);
+    const float* vr = vs + at * kGsTile * VW + mine;
+    const float* f = fs + at * kGsFactors;
+    float* ob = os + b % ((AHEAD + 1) * BLOCKS) * VW * Sh::OUT;
+    if ((b + 1) % BLOCKS == 0 && b + 1 < blocks) {
+      const int st = (b + 1) / BLOCKS;
+      mbar_wait_guarded(&factors_full[st % BUFS], (st / BUFS) & 1);
+    }
+    float v[4], p[C][4], r[C][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = vr[j * VW];
+    const float4 beta = *reinterpret_cast<const float4*>(f + kGsBeta), d3 = *reinterpret_cast<const float4*>(f + kGsD3);
+    // S^T k of the block's tokens, then S^T q; a token's sum over the lanes goes on a level for each product that follows.  A row's
+    // successor in the next block is on its way as soon as the row is used (behind the last block: read, not used).
+    constexpr int FIRST = DELTA ? 0 : 4;
+#pragma unroll
+    for (int t = FIRST; t < 8 || (DELTA && t < 4 + LV); ++t) {
+      if (t < 8) {
+        float d[C];
+        f32x2 q[R2];
+        gs_row<L, R4>((t < 4 ? ks : qs) + (at * kGsTile + (t & 3)) * DKP, l, q);
+        gs_dot<R2, C>(S, q, d);
+#pragma unroll
+        for (int c = 0; c < C; ++c) (t < 4 ? p : r)[c][t & 3] = d[c];
+      }
+      if (DELTA) {
+#pragma unroll
+        for (int lv = 0; lv < LV; ++lv)
+          if (t - 1 - lv >= 0 && t - 1 - lv < 4) gs_level<C>(p, t - 1 - lv, lv);
+      }
+    }
+    const f32x2 g4 = pack2(d3.w, d3.w);
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+#pragma unroll
+      for (int i = 0; i < R2; ++i) S[c][i] = mul2(g4, S[c][i]);
+    float u[4];
+    if (DELTA) {
+      const float4 G = *reinterpret_cast<const float4*>(f + kGsG), Gl = *reinterpret_cast<const float4*>(f + kGsGl),
+                   a0 = *reinterpret_cast<const float4*>(f + kGsA);
+      const float2 a1 = *reinterpret_cast<const float2*>(f + kGsA + 4);
+      u[0] = beta.x * fmaf(-Gl.x, p[0][0], fmaf(-G.x, p[0][0], v[0]));
+      u[1] = beta.y * fmaf(-a0.x, u[0], fmaf(-Gl.y, p[0][1], fmaf(-G.y, p[0][1], v[1])));
+      u[2] = beta.z * fmaf(-a0.z, u[1], fmaf(-a0.y, u[0], fmaf(-Gl.z, p[0][2], fmaf(-G.z, p[0][2], v[2]))));
+      u[3] = beta.w * fmaf(-a1.y, u[2], fmaf(-a1.x, u[1], fmaf(-a0.w, u[0], fmaf(-Gl.w, p[0][3], fmaf(-G.w, p[0][3], v[3])))));
+    } else {
+      u[0] = beta.x * v[0];
+      u[1] = beta.y * v[1];
+      u[2] = beta.z * v[2];
+      u[3] = beta.w * v[3];
+    }
+    const float w[4] = {d3.x * u[0], d3.y * u[1], d3.z * u[2], u[3]};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      f32x2 k[R2];
+      gs_row<L, R4>(ks + (at * kGsTile + j) * DKP, l, k);
 #pragma unroll
       for (int c = 0; c < C; ++c) {
+        const float x = c ? __shfl_xor_sync(0xffffffffu, w[j], c) : w[j];
+        const f32x2 x2 = pack2(x, x);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float mine = b4 ? o[j + 4][c] : o[j][c], other = b4 ? o[j][c] : o[j + 4][c];
-          o[j][c] = mine + __shfl_xor_sync(0xffffffffu, other, 4);
-        }
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const float mine = b2 ? o[j + 2][c] : o[j][c], other = b2 ? o[j][c] : o[j + 2][c];
-          o[j][c] = mine + __shfl_xor_sync(0xffffffffu, other, 2);
-        }
-        const float mine = b1 ? o[1][c] : o[0][c], other = b1 ? o[0][c] : o[1][c];
-        sum[c] = mine + __shfl_xor_sync(0xffffffffu, other, 1);
+        for (int i = 0; i < R2; ++i) S[c][i] = fma2(k[i], x2, S[c][i]);
       }
-      if constexpr (C == 2 && L > 8) {                 // the lanes' halves of 8 take one column each
-        const bool hi = l & 8;
-        float one = (hi ? sum[1] : sum[0]) + __shfl_xor_sync(0xffffffffu, hi ? sum[0] : sum[1], 8);
+      if (j < LC) {
 #pragma unroll
-        for (int w = 16; w < L; w <<= 1) one += __shfl_xor_sync(0xffffffffu, one, w);
-        if (l < 16) os[(tb + (l & 7)) * OP + cw + (hi ? 1 : 0)] = one;
-      } else {
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-#pragma unroll
-          for (int w = 8; w < L; w <<= 1) sum[c] += __shfl_xor_sync(0xffffffffu, sum[c], w);
-          if (l < 8) os[(tb + l) * OP + cw + c] = sum[c];
-        }
+        for (int i = 0; i < 4; ++i) gs_level<C>(r, i, j);
       }
     }
-    if (next < t1) put_gates(next, buf ^ 1);
-    __syncthreads();
-    const float sk = a.skip != nullptr ? a.skip[h] : 0.f;
-    for (int i = tid; i < nt * COLS; i += kGsWarps * 32) {
-      const int tt = i / COLS, c = i - tt * COLS;
-      if (z * COLS + c < a.dv)
-        a.o[(size_t)(ch + tt) * a.H * a.dv + h * a.dv + z * COLS + c] =
-            fmaf(sk, vs[(buf * TOK + tt) * COLS + c], os[tt * OP + c]);
+    if (l < C) *reinterpret_cast<float4*>(ob + mine * 4) = make_float4(u[0], u[1], u[2], u[3]);
+    *reinterpret_cast<float4*>(ob + ((l / C + 1) * VW + mine) * 4) = make_float4(r[0][0], r[0][1], r[0][2], r[0][3]);
+    if ((b + 1) % BLOCKS == 0 || b + 1 == blocks) {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[b / BLOCKS % BUFS]);
     }
   }
 #pragma unroll
   for (int c = 0; c < C; ++c)
 #pragma unroll
     for (int i = 0; i < R4; ++i)
-      if (col + c < a.dv && 4 * (i * L + l) < dkp)
-        *reinterpret_cast<ulonglong2*>(Sp + c * dkp + 4 * (i * L + l)) = make_ulonglong2(S[c][2 * i], S[c][2 * i + 1]);
+      if (col0 + group + (c ^ l % C) < a.dv && 4 * (i * L + l) < dkp)
+        *reinterpret_cast<ulonglong2*>(Sp + (size_t)(group + (c ^ l % C)) * dkp + 4 * (i * L + l)) = make_ulonglong2(S[c][2 * i], S[c][2 * i + 1]);
 }
 
 // Single rows (a decode step): the state, the token's rows and its gates are in flight together; no staging, no barrier.
 template <int L, int R4, bool DELTA>
-__global__ void __launch_bounds__(kGsWarps * 32, 4)
+__global__ void __launch_bounds__(kGsStepWarps * 32, 4)
 gated_step_kernel(GatedScanArgs a) {
-  constexpr int R2 = 2 * R4, CPW = 32 / L, COLS = kGsWarps * CPW;
+  constexpr int R2 = 2 * R4, CPW = 32 / L, COLS = kGsStepWarps * CPW;
   const int s = blockIdx.x, h = blockIdx.y, z = blockIdx.z;
   const int slot = a.state_slots[s];
   if (slot < 0) return;
@@ -340,7 +511,7 @@ gated_step_kernel(GatedScanArgs a) {
   const bool live = col < a.dv, fresh = a.ctx_lens[s] == 0;
   float* Sp = a.S + (((size_t)slot * a.H + h) * a.dv + col) * dkp;
   const float* row = a.x + (size_t)t * a.ld;
-  f32x2 S[1][R2], k[R2], q[R2];
+  f32x2 S[R2], k[R2], q[R2];
 #pragma unroll
   for (int i = 0; i < R4; ++i) {
     const int d = 4 * (i * L + l);
@@ -350,67 +521,79 @@ gated_step_kernel(GatedScanArgs a) {
       tk = *reinterpret_cast<const ulonglong2*>(row + a.k_col + hk * dkp + d);
       tq = *reinterpret_cast<const ulonglong2*>(row + a.q_col + hk * dkp + d);
     }
-    S[0][2 * i] = ts.x; S[0][2 * i + 1] = ts.y;
+    S[2 * i] = ts.x; S[2 * i + 1] = ts.y;
     k[2 * i] = tk.x; k[2 * i + 1] = tk.y;
     q[2 * i] = tq.x; q[2 * i + 1] = tq.y;
   }
-  const float v[1] = {live ? row[a.v_col + h * a.dvp + col] : 0.f};
+  const float v = live ? row[a.v_col + h * a.dvp + col] : 0.f;
   const float* g = a.gates + (size_t)t * a.ld_g;
   const float2 gb = gs_gate<DELTA>(DELTA ? g[a.H + h] : g[h], DELTA ? g[h] : 0.f, a.rate[h], a.dt_bias[h]);
-  float o[1];
-  gs_token<L, R2, 1, DELTA, false>(S, k, q, v, gb, o);
-  gs_dot<R2, 1>(S, q, o);
-  o[0] = lanes_sum<L>(o[0]);
+  float u = gb.y * v;
+  if (DELTA) u = gb.y * (v - gb.x * lanes_sum<L>(gs_dot1<R2>(S, k)));
+  const f32x2 g2 = pack2(gb.x, gb.x), u2 = pack2(u, u);
+#pragma unroll
+  for (int i = 0; i < R2; ++i) S[i] = fma2(k[i], u2, mul2(g2, S[i]));
+  const float o = lanes_sum<L>(gs_dot1<R2>(S, q));
   if (!live) return;
 #pragma unroll
   for (int i = 0; i < R4; ++i) {
     const int d = 4 * (i * L + l);
-    if (d < dkp) *reinterpret_cast<ulonglong2*>(Sp + d) = make_ulonglong2(S[0][2 * i], S[0][2 * i + 1]);
+    if (d < dkp) *reinterpret_cast<ulonglong2*>(Sp + d) = make_ulonglong2(S[2 * i], S[2 * i + 1]);
   }
-  if (l == 0) a.o[(size_t)t * a.H * a.dv + h * a.dv + col] = a.skip != nullptr ? fmaf(a.skip[h], v[0], o[0]) : o[0];
+  if (l == 0) a.o[(size_t)t * a.H * a.dv + h * a.dv + col] = a.skip != nullptr ? fmaf(a.skip[h], v, o) : o;
 }
 
 template <int L, int R4, int C, bool DELTA>
 int gated_scan_launch(const GatedScanArgs& a, int n_seqs, cudaStream_t s) {
-  constexpr int COLS = kGsWarps * C * (32 / L), DKP = 4 * R4 * L;
-  constexpr int TOK = DKP <= 128 ? 32 : 16;
-  const dim3 grid(n_seqs, a.H, (a.dv + COLS - 1) / COLS);
-  constexpr size_t smem = sizeof(float) * (4 * (size_t)TOK * DKP + 2 * TOK * COLS + 4 * TOK + TOK * (COLS + 8));
-  if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(gated_scan_kernel<L, R4, C, TOK, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) {
-      b200_set_error("gated_scan: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
-      return B200_ERR_CUDA;
-    }
+  using Sh = GsShape<L, R4, C>;
+  const cudaError_t e = cudaFuncSetAttribute(gated_scan_kernel<L, R4, C, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::kBytes);
+  if (e != cudaSuccess) {
+    b200_set_error("gated_scan: %zu bytes of shared memory: %s", Sh::kBytes, cudaGetErrorString(e));
+    return B200_ERR_CUDA;
   }
-  gated_scan_kernel<L, R4, C, TOK, DELTA><<<grid, kGsWarps * 32, smem, s>>>(a);
+  gated_scan_kernel<L, R4, C, DELTA><<<dim3(n_seqs, a.H, (a.dv + Sh::VW - 1) / Sh::VW), (kGsWarps + kGsHelpers) * 32, Sh::kBytes, s>>>(a);
   return b200_check_launch("b200_gated_scan");
 }
 
-// L, R4: single rows; PL, PR4: prompt portions (fewer entries of two columns per lane: the same registers, half the reads)
-template <int L, int R4, int PL, int PR4, bool DELTA>
-int gated_scan_form(const GatedScanArgs& a, int n_seqs, int max_len, cudaStream_t s) {
-  if (max_len == 1) {
-    constexpr int COLS = kGsWarps * (32 / L);
-    gated_step_kernel<L, R4, DELTA><<<dim3(n_seqs, a.H, (a.dv + COLS - 1) / COLS), kGsWarps * 32, 0, s>>>(a);
-    return b200_check_launch("b200_gated_scan(step)");
-  }
-  // too few CTAs to fill the GPU: the widest spread of a column over lanes, the shortest walk per token
-  if constexpr (PL == 16 && PR4 == 2) {
-    constexpr int COLS = kGsWarps * 2 * (32 / PL);
-    if (n_seqs * a.H * ((a.dv + COLS - 1) / COLS) < 148) return gated_scan_launch<32, 1, 2, DELTA>(a, n_seqs, s);
-  }
-  return gated_scan_launch<PL, PR4, 2, DELTA>(a, n_seqs, s);
+template <int L, int R4, bool DELTA>
+int gated_step_launch(const GatedScanArgs& a, int n_seqs, cudaStream_t s) {
+  constexpr int COLS = kGsStepWarps * (32 / L);
+  gated_step_kernel<L, R4, DELTA><<<dim3(n_seqs, a.H, (a.dv + COLS - 1) / COLS), kGsStepWarps * 32, 0, s>>>(a);
+  return b200_check_launch("b200_gated_scan(step)");
 }
 
+// Single rows have a kernel of their own.  Portions: the more columns a warp walks the fewer instructions a column costs, the fewer
+// it walks the shorter a block takes, so the widest form whose CTAs still find an SM each: us for 1, 2, 3 and 4 sequences of the delta
+// rule with 16 heads of 128 x 128 (2048, 1024, 1024 and 2048 rows), in CTAs of 64 columns 471, 241, 242, 472, of 32 columns 336, 174, 285, 558,
+// of 16 columns 283, 225, 348, 860.  CTAs of 32 columns share an SM in pairs, which covers the start and the end of short portions: 16
+// of 16 rows 34.5 in CTAs of 64 columns, 31.0 of 32, but 8 of 1024 rows 476 and 551.  A bound on the rows per portion is often that of all
+// of them, so pairs are for sequences enough to fill the GPU three times (16 of 512 rows: 480 either way) or a bound that is short.
+template <int L, int R4>
+bool gs_fits(const GatedScanArgs& a, int n_seqs) {
+  constexpr int cols = GsShape<L, R4, 4>::VW;
+  return (int64_t)n_seqs * a.H * ((a.dv + cols - 1) / cols) <= kGsSms;
+}
 template <bool DELTA>
 int gated_scan_pick(const GatedScanArgs& a, int n_seqs, int max_len, cudaStream_t s) {
-  if (a.dkp <= 32) return gated_scan_form<8, 1, 8, 1, DELTA>(a, n_seqs, max_len, s);
-  if (a.dkp <= 64) return gated_scan_form<8, 2, 16, 1, DELTA>(a, n_seqs, max_len, s);
-  if (a.dkp <= 96) return gated_scan_form<8, 3, 8, 3, DELTA>(a, n_seqs, max_len, s);
-  if (a.dkp <= 128) return gated_scan_form<8, 4, 16, 2, DELTA>(a, n_seqs, max_len, s);
-  if (a.dkp <= 256) return gated_scan_form<16, 4, 32, 2, DELTA>(a, n_seqs, max_len, s);
-  return gated_scan_form<32, 4, 32, 4, DELTA>(a, n_seqs, max_len, s);
+  if (max_len == 1) {
+    if (a.dkp <= 32) return gated_step_launch<8, 1, DELTA>(a, n_seqs, s);
+    if (a.dkp <= 64) return gated_step_launch<8, 2, DELTA>(a, n_seqs, s);
+    if (a.dkp <= 96) return gated_step_launch<8, 3, DELTA>(a, n_seqs, s);
+    if (a.dkp <= 128) return gated_step_launch<8, 4, DELTA>(a, n_seqs, s);
+    if (a.dkp <= 256) return gated_step_launch<16, 4, DELTA>(a, n_seqs, s);
+    return gated_step_launch<32, 4, DELTA>(a, n_seqs, s);
+  }
+  if (a.dkp <= 16) return gated_scan_launch<4, 1, 4, DELTA>(a, n_seqs, s);
+  if (a.dkp <= 32) return gated_scan_launch<8, 1, 4, DELTA>(a, n_seqs, s);
+  if (a.dkp <= 64) return gs_fits<16, 1>(a, n_seqs) ? gated_scan_launch<16, 1, 4, DELTA>(a, n_seqs, s) : gated_scan_launch<8, 2, 4, DELTA>(a, n_seqs, s);
+  if (a.dkp <= 96) return gated_scan_launch<8, 3, 4, DELTA>(a, n_seqs, s);
+  if (a.dkp <= 128) {
+    if (gs_fits<32, 1>(a, n_seqs)) return gated_scan_launch<32, 1, 4, DELTA>(a, n_seqs, s);
+    const bool pairs = gs_fits<16, 2>(a, n_seqs) || max_len <= 64 || !gs_fits<8, 4>(a, (n_seqs + 2) / 3);
+    return pairs ? gated_scan_launch<16, 2, 4, DELTA>(a, n_seqs, s) : gated_scan_launch<8, 4, 4, DELTA>(a, n_seqs, s);
+  }
+  if (a.dkp <= 256) return gs_fits<32, 2>(a, n_seqs) ? gated_scan_launch<32, 2, 4, DELTA>(a, n_seqs, s) : gated_scan_launch<16, 4, 4, DELTA>(a, n_seqs, s);
+  return gated_scan_launch<32, 4, 4, DELTA>(a, n_seqs, s);
 }
 
 // The state-space recurrence in the chunk form: log decays of a chunk's rows summed in fp64, every exponent <= 0.  A decay of

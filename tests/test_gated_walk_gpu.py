@@ -1,0 +1,95 @@
+"""Delta rule and state space over portions in blocks of four tokens (csrc/gated_scan.cu): every width of a warp's columns, portions that
+end inside a block, a stage of four blocks and the ring of four stages, against a token-by-token walk in 64 bits."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+F64 = torch.float64
+LENS = [1, 3, 4, 5, 15, 16, 17, 48, 63, 64, 65, 131]
+
+
+def _i32(v):
+    return torch.tensor(v, dtype=torch.int32, device="cuda")
+
+
+def _inputs(lens, H, G, dk, dv, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")   # noqa: E731
+    T, n, kp, vp = sum(lens), len(lens), -(-dk // 4) * 4, -(-dv // 4) * 4
+    q, k, v = r(T, G, dk), r(T, G, dk), r(T, H, dv)
+    k /= k.norm(dim=-1, keepdim=True)
+    x = torch.zeros(T, 2 * G * kp + H * vp, device="cuda")
+    x[:, :G * kp].view(T, G, kp)[..., :dk], x[:, G * kp:2 * G * kp].view(T, G, kp)[..., :dk] = q, k
+    x[:, 2 * G * kp:].view(T, H, vp)[..., :dv] = v
+    S = torch.zeros(n, H, dv, kp, device="cuda")
+    S[..., :dk] = r(n, H, dv, dk)
+    return x, q, k, v, r(T, 2 * H), S, torch.linspace(0.1, 1.0, H, device="cuda"), torch.linspace(-2.5, -1.5, H, device="cuda")
+
+
+def _scan(x, gates, rate, bias, skip, lens, ctx, S, H, G, dk, dv, delta):
+    from gpustack_b200 import ops
+
+    kp, n = -(-dk // 4) * 4, len(lens)
+    cu = [sum(lens[:i]) for i in range(n + 1)]
+    out = torch.full((x.shape[0], H * dv), 7.0, device="cuda")
+    ops.gated_scan(x, 0, G * kp, 2 * G * kp, gates if delta else gates[:, :H].contiguous(), rate, bias, skip, _i32(cu), _i32(ctx),
+                   _i32(list(range(n))[::-1]), S, out, H, G, dk, dv, delta, max_len=max(2, max(lens)))
+    return out
+
+
+def _walk(q, k, v, gates, rate, bias, skip, lens, ctx, S, H, G, dk, delta):
+    q, k = (t.to(F64).repeat_interleave(H // G, 1) for t in (q, k))
+    v, gates, S = v.to(F64), gates.to(F64), S.to(F64)
+    sp = torch.nn.functional.softplus((gates[:, H:] if delta else gates[:, :H]) + bias.to(F64))
+    decay, step = torch.exp(-rate.to(F64) * sp), torch.sigmoid(gates[:, :H]) if delta else sp
+    n, out, at = len(lens), torch.empty_like(v), 0
+    first = torch.tensor([sum(lens[:i]) for i in range(n)], device="cuda")
+    live = torch.tensor(lens, device="cuda")
+    Z = torch.stack([S[n - 1 - i, ..., :dk] * (1.0 if ctx[i] else 0.0) for i in range(n)])
+    for at in range(max(lens)):                        # token `at` of every sequence that has one
+        i = (live > at).nonzero()[:, 0]
+        t = first[i] + at
+        z = Z[i] * decay[t][..., None, None]
+        u = v[t] - torch.einsum("nhvk,nhk->nhv", z, k[t]) if delta else v[t]
+        z = z + (step[t][..., None] * u)[..., None] * k[t][:, :, None]
+        Z[i], out[t] = z, torch.einsum("nhvk,nhk->nhv", z, q[t]) + (0.0 if skip is None else skip.to(F64)[:, None] * v[t])
+    return out.flatten(1), Z
+
+
+def _rel(a, b):
+    return float((a.to(F64) - b).norm() / b.norm())
+
+
+# heads and copies of the portions so that each of the widths that a number of CTAs chooses runs: (16, 64), (32, 128), (32, 256)
+@pytest.mark.parametrize("H,G,dk,dv,copies", [(2, 1, 14, 17, 1), (2, 2, 32, 64, 1), (2, 1, 64, 33, 1), (4, 2, 52, 64, 6), (2, 1, 90, 70, 1),
+                                              (1, 1, 128, 64, 1), (4, 2, 128, 60, 1), (8, 4, 124, 64, 2), (8, 4, 128, 128, 2), (1, 1, 256, 20, 1),
+                                              (4, 4, 200, 128, 2), (1, 1, 400, 40, 1)])
+@pytest.mark.parametrize("delta", [True, False])
+def test_blocks_of_four(H, G, dk, dv, copies, delta):
+    lens = LENS * copies
+    ctx = [9 * (i % 3) for i in range(len(lens))]
+    x, q, k, v, gates, S, rate, bias = _inputs(lens, H, G, dk, dv, dk + dv)
+    skip = None if delta else torch.linspace(-1.0, 1.0, H, device="cuda")
+    want, Z = _walk(q, k, v, gates, rate, bias, skip, lens, ctx, S, H, G, dk, delta)
+    out = _scan(x, gates, rate, bias, skip, lens, ctx, S, H, G, dk, dv, delta)
+    # fp32 sums of dk products and 131 steps; the state-space rows gain no more than their own size per step
+    assert _rel(out, want) < 5e-6
+    for i in range(len(lens)):
+        assert _rel(S[len(lens) - 1 - i, ..., :dk], Z[i]) < 5e-6, lens[i]
+    assert not S[..., dk:].any()
+
+
+@pytest.mark.parametrize("row", [4, 5, 6, 7])
+@pytest.mark.parametrize("delta", [True, False])
+def test_what_is_no_number_stays_behind_its_row(row, delta):
+    """... also from the rows of its own block, each of them."""
+    H, G, dk, dv, lens = 2, 1, 128, 64, [40]
+    x, q, k, v, gates, S, rate, bias = _inputs(lens, H, G, dk, dv, 3)
+    clean = _scan(x, gates, rate, bias, None, lens, [5], S.clone(), H, G, dk, dv, delta)
+    bad = x.clone()
+    bad[row, 2 * G * dk:] = float("nan")
+    bad[row + 9, G * dk:2 * G * dk] = float("inf")
+    out = _scan(bad, gates, rate, bias, None, lens, [5], S, H, G, dk, dv, delta)
+    assert torch.equal(out[:row], clean[:row])
+    assert bool(torch.isnan(out[row:]).all()) and bool(torch.isnan(S).all())
