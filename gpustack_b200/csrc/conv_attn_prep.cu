@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(kCapWarps * 32, 2)
 conv_attn_prep_vec_kernel(CapArgs a, int lph) {
   constexpr int V = 16 / (int)sizeof(TA), R = TAPS - 1, NB = kCapRows;
   static_assert(R <= NB, "a sequence's first piece holds every row that reads the ring");
-  const CapWork m = cap_work<kCapRows>(a);
+  const CapWork m = cap_work(a, kCapRows);
   if (m.n <= 0) return;
   const int lane = threadIdx.x & 31, per_warp = 32 / lph;
   const int hs = (blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5)) * per_warp + lane / lph;
@@ -161,7 +161,7 @@ template <typename TA>
 __global__ void __launch_bounds__(kCapWarps * 32)
 conv_attn_prep_kernel(CapArgs a) {
   constexpr int kPer = 16;                             // columns per lane: widths up to 512
-  const CapWork m = cap_work<kCapRows>(a);
+  const CapWork m = cap_work(a, kCapRows);
   const int hs = blockIdx.y * kCapWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (m.n <= 0 || hs >= a.H + 2 * a.G) return;
   const bool is_q = hs < a.H, is_k = !is_q && hs < a.H + a.G;
@@ -248,7 +248,7 @@ conv_attn_prep_joint_vec_kernel(CapArgs a, int lph) {
   static_assert(R + 2 + 3 <= kCapSlots, "a step's rows, the ones before and the ones in flight have slots of their own");
   extern __shared__ __align__(16) uint4 raw[];         // [8][threads]
   __shared__ float head_ss[2][2][kCapJointWarps * 32]; // [step parity][row][head slot]
-  const CapWork m = cap_work<kCapRun>(a);
+  const CapWork m = cap_work(a, kCapRun);
   if (m.n <= 0) return;
   const int lane = threadIdx.x & 31, per_warp = 32 / lph, li = lane % lph, d = li * V, half = a.dims >> 1;
   const int hs = (threadIdx.x >> 5) * per_warp + lane / lph;
@@ -440,7 +440,7 @@ conv_attn_prep_joint_kernel(CapArgs a) {
   constexpr int NB = kCapRows;
   extern __shared__ __align__(16) float heads[];       // a head per warp
   __shared__ float red[kCapWarps][2][NB], mul[2][NB];
-  const CapWork m = cap_work<NB>(a);
+  const CapWork m = cap_work(a, NB);
   if (m.n <= 0) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = a.dims >> 1, n_slots = a.H + 2 * a.G, R = a.taps - 1;
   const int C = (a.H + a.G) * a.dk + a.G * a.dv, wmax = a.dk > a.dv ? a.dk : a.dv;

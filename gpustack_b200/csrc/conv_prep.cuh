@@ -19,52 +19,61 @@ __device__ __forceinline__ void ca_store(bf16* p, float v) { *p = __float2bfloat
 struct CapWork {
   int row0, q0, n, qlen, ctx, slot;
 };
-template <int ROWS, typename Args>
-__device__ __forceinline__ CapWork cap_work(const Args& a) {
+template <typename Args>
+__device__ __forceinline__ CapWork cap_work(const Args& a, int rows) {
   CapWork m;
   int s, q0 = 0;
   if ((int)blockIdx.x < a.n_pieces) {
     const int tile = blockIdx.x / a.per_tile;
     s = a.tile_seq[tile];
-    q0 = a.tile_q0[tile] + ROWS * (blockIdx.x - tile * a.per_tile);
+    q0 = a.tile_q0[tile] + rows * ((int)blockIdx.x - tile * a.per_tile);
   } else {
     s = a.n_prompt + (int)blockIdx.x - a.n_pieces;
   }
   m.row0 = a.cu_seq[s];
   m.q0 = q0;
   m.qlen = a.cu_seq[s + 1] - m.row0;
-  m.n = min(ROWS, m.qlen - q0);
+  m.n = min(rows, m.qlen - q0);
   m.ctx = a.ctx_lens[s];
   m.slot = a.ring != nullptr ? a.state_slots[s] : -1;
   return m;
 }
 
-// One 16-byte piece (V channels from channel c on) of a work item's rows and of the TAPS - 1 rows before them, as loaded:
-// win[R + i] is row q0 + i, win[R - 1 - b] the input b + 1 positions before row q0 -- from this step's rows, else from the
-// sequence's ring (a ring entry is an input, so it fits the element type exactly), else zero.  src: row 0 of the sequence.
-template <typename TA, int TAPS, int NB>
-__device__ __forceinline__ void conv_window(uint4 (&win)[TAPS - 1 + NB], const CapWork& m, const TA* src, int64_t ld,
-                                            const float* ring, int c, int C) {
+// One 16-byte piece (V channels from channel c on) of the TAPS - 1 rows before a work item's, as loaded: old[b] is the input b + 1
+// positions before row q0 -- from this step's rows, else from the sequence's ring (a ring entry is an input, so it fits the
+// element type exactly), else zero.  src: row 0 of the sequence.
+template <typename TA, int TAPS>
+__device__ __forceinline__ void conv_before(uint4 (&old)[TAPS > 1 ? TAPS - 1 : 1], const CapWork& m, const TA* src, int64_t ld, const float* ring,
+                                            int c, int C) {
   constexpr int V = 16 / (int)sizeof(TA), R = TAPS - 1, RR = R > 0 ? R : 1;
-  static_assert(R <= NB, "a sequence's first piece holds every row that reads the ring");
-  const uint4 zero4 = make_uint4(0, 0, 0, 0);
-#pragma unroll
-  for (int i = 0; i < NB; ++i)
-    win[R + i] = i < m.n ? *reinterpret_cast<const uint4*>(src + (int64_t)(m.q0 + i) * ld) : zero4;
-  if constexpr (R > 0)
 #pragma unroll
   for (int b = 0; b < R; ++b) {
     const int q = m.q0 - 1 - b, p = m.ctx + q;
-    win[R - 1 - b] = zero4;
+    old[b] = make_uint4(0, 0, 0, 0);
     if (q >= 0) {
-      win[R - 1 - b] = *reinterpret_cast<const uint4*>(src + (int64_t)q * ld);
+      old[b] = *reinterpret_cast<const uint4*>(src + (int64_t)q * ld);
     } else if (p >= 0 && m.slot >= 0) {
       const float* rp = ring + ((size_t)m.slot * R + p % RR) * C + c;
-      TA* w = reinterpret_cast<TA*>(&win[R - 1 - b]);
+      TA* w = reinterpret_cast<TA*>(&old[b]);
 #pragma unroll
       for (int i = 0; i < V; ++i) ca_store(w + i, rp[i]);
     }
   }
+}
+
+// ... and of its rows too: win[R + i] is row q0 + i, win[R - 1 - b] the input b + 1 positions before row q0
+template <typename TA, int TAPS, int NB>
+__device__ __forceinline__ void conv_window(uint4 (&win)[TAPS - 1 + NB], const CapWork& m, const TA* src, int64_t ld,
+                                            const float* ring, int c, int C) {
+  constexpr int R = TAPS - 1;
+  static_assert(R <= NB, "a sequence's first piece holds every row that reads the ring");
+#pragma unroll
+  for (int i = 0; i < NB; ++i)
+    win[R + i] = i < m.n ? *reinterpret_cast<const uint4*>(src + (int64_t)(m.q0 + i) * ld) : make_uint4(0, 0, 0, 0);
+  uint4 old[R > 0 ? R : 1];
+  conv_before<TA, TAPS>(old, m, src, ld, ring, c, C);
+#pragma unroll
+  for (int b = 0; b < R; ++b) win[R - 1 - b] = old[b];
 }
 
 // The step's last inputs of the piece's channels go to the ring: called by the threads of a sequence's FIRST piece after

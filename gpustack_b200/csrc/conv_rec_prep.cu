@@ -64,12 +64,26 @@ __device__ __forceinline__ CrpHead crp_head(const CrpArgs& a, int hs) {
 
 __device__ __forceinline__ float crp_silu(float y) { return y / (1.0f + expf(-y)); }
 
-// LPH lanes share a head, each owns one 16-byte piece of it in NB rows.
-template <typename TA, int TAPS, int NB>
-__global__ void __launch_bounds__(kCapWarps * 32)
-conv_rec_prep_vec_kernel(CrpArgs a, int lph) {
-  constexpr int V = 16 / (int)sizeof(TA), R = TAPS - 1;
-  const CapWork m = cap_work<NB>(a);
+// two entries of a 16-byte piece as fp32 numbers
+__device__ __forceinline__ void crp_pairs(const uint4& raw, f32x2 (&x)[4], bf16) {
+  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) x[i] = pack2(bf16_lo(w[i]), bf16_hi(w[i]));
+}
+__device__ __forceinline__ void crp_pairs(const uint4& raw, f32x2 (&x)[2], float) {
+  x[0] = pack2(__uint_as_float(raw.x), __uint_as_float(raw.y));
+  x[1] = pack2(__uint_as_float(raw.z), __uint_as_float(raw.w));
+}
+
+// LPH lanes share a head, each owns one 16-byte piece of it and walks the work item's rows: a row is loaded and made fp32 once, four rows
+// before it is used, and serves the outputs of TAPS rows from registers.  Bound by instructions (some 25 per output value: a logistic of 11,
+// the taps in pairs): 8192 rows of 4096 channels 75 us with four rows per item, all of a window's rows made fp32 for every tap and the
+// logistic of 19, 57 now; 2048 rows 24.2 -> 22.2.
+template <typename TA, int TAPS>
+__global__ void __launch_bounds__(kCapWarps * 32, sizeof(TA) == 4 ? 3 : 2)
+conv_rec_prep_vec_kernel(CrpArgs a, int lph, int rows) {
+  constexpr int V = 16 / (int)sizeof(TA), P = V / 2, R = TAPS - 1;
+  const CapWork m = cap_work(a, rows);
   if (m.n <= 0) return;
   const int lane = threadIdx.x & 31, per_warp = 32 / lph;
   const int hs = (blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5)) * per_warp + lane / lph;
@@ -80,36 +94,83 @@ conv_rec_prep_vec_kernel(CrpArgs a, int lph) {
   const bool act = live && d < h.width;
   const int c = h.c + d;
   const TA* src = reinterpret_cast<const TA*>(a.proj) + (size_t)m.row0 * a.ld + c;
-  uint4 win[R + NB];
-  float w[TAPS][V], bias[V];
-  if (act) {
-    conv_window<TA, TAPS, NB>(win, m, src, a.ld, a.ring, c, a.C);
-    conv_weights<TAPS, V>(w, a.conv_w, c, a.C);
+  const TA* at = src + (size_t)m.q0 * a.ld;
+  uint4 raw[4];                                        // rows that are on their way: row r in raw[r % 4]
+  f32x2 x[4][P], w[TAPS][P], bias[P];                  // row r in x[r % 4]
 #pragma unroll
-    for (int i = 0; i < V; ++i) bias[i] = a.bias != nullptr ? a.bias[c + i] : 0.f;
+  for (int i = 0; i < 4; ++i) raw[i] = make_uint4(0, 0, 0, 0);
+#pragma unroll
+  for (int i = 0; i < P; ++i) {
+    bias[i] = 0;
+#pragma unroll
+    for (int b = 0; b < TAPS; ++b) w[b][i] = 0;
+#pragma unroll
+    for (int b = 0; b < 4; ++b) x[b][i] = 0;
+  }
+  if (act) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (i < m.n) raw[i] = *reinterpret_cast<const uint4*>(at + (int64_t)i * a.ld);
+    uint4 old[R > 0 ? R : 1];
+    conv_before<TA, TAPS>(old, m, src, a.ld, a.ring, c, a.C);
+#pragma unroll
+    for (int b = 0; b < R; ++b) crp_pairs(old[b], x[3 - b], TA());
+    float f[TAPS][V];
+    conv_weights<TAPS, V>(f, a.conv_w, c, a.C);
+#pragma unroll
+    for (int b = 0; b < TAPS; ++b)
+#pragma unroll
+      for (int i = 0; i < P; ++i) w[b][i] = pack2(f[b][2 * i], f[b][2 * i + 1]);
+    if (a.bias != nullptr)
+#pragma unroll
+      for (int i = 0; i < P; ++i) bias[i] = pack2(a.bias[c + 2 * i], a.bias[c + 2 * i + 1]);
     conv_ring_put<TA, TAPS>(m, src, a.ld, a.ring, c, a.C);
   }
   float* dst = a.out + (size_t)(m.row0 + m.q0) * a.ldo + h.o + d;
+  const bool unit = __any_sync(0xffffffffu, act && sg.unit);
+#pragma unroll 1
+  for (int r0 = 0; r0 < m.n; r0 += 4) {
 #pragma unroll
-  for (int r = 0; r < NB; ++r) {
-    if (r >= m.n) break;
-    float y[V], ss = 0.f;
+    for (int i = 0; i < 4; i += 2) {                   // two rows at a time: one alone waits for itself
+      const int r = r0 + i;
+      if (r >= m.n) break;
+      float y[2][V], ss[2] = {0.f, 0.f};
 #pragma unroll
-    for (int i = 0; i < V; ++i) y[i] = 0.f;
-    if (act) {
+      for (int k = 0; k < 2; ++k) {
+        crp_pairs(raw[i + k], x[i + k], TA());
+        if (act && r + k + 4 < m.n) raw[i + k] = *reinterpret_cast<const uint4*>(at + (int64_t)(r + k + 4) * a.ld);
 #pragma unroll
-      for (int i = 0; i < V; ++i) y[i] = bias[i];
-      conv_row<TA, TAPS, NB>(win, r, w, y);
-      logistic_all<true>(y, y);
+        for (int e = 0; e < P; ++e) {
+          f32x2 s = bias[e];
 #pragma unroll
-      for (int i = 0; i < V; ++i) ss = fmaf(y[i], y[i], ss);
+          for (int b = 0; b < TAPS; ++b) s = fma2(w[b][e], x[(i + k - b) & 3][e], s);
+          const float2 v = unpack2(s);
+          y[k][2 * e] = v.x;
+          y[k][2 * e + 1] = v.y;
+        }
+      }
+      logistic_both<true>(y);
+      if (unit) {                                      // (of the warp: all lanes take part)
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+          for (int e = 0; e < V; ++e) ss[k] = fmaf(y[k][e], y[k][e], ss[k]);
+        for (int o = lph >> 1; o > 0; o >>= 1) {
+#pragma unroll
+          for (int k = 0; k < 2; ++k) ss[k] += __shfl_xor_sync(0xffffffffu, ss[k], o);
+        }
+      }
+      if (!act) continue;
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        if (r + k >= m.n) break;
+        const float mul = sg.unit ? sg.mul * inv_sqrt(ss[k] + a.eps) : sg.mul;
+#pragma unroll
+        for (int e = 0; e < V; e += 4)
+          *reinterpret_cast<float4*>(dst + (size_t)(r + k) * a.ldo + e) =
+              make_float4(y[k][e] * mul, y[k][e + 1] * mul, y[k][e + 2] * mul, y[k][e + 3] * mul);
+      }
     }
-    for (int o = lph >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);    // all lanes take part
-    if (!act) continue;
-    const float mul = sg.unit ? sg.mul / sqrtf(ss + a.eps) : sg.mul;
-#pragma unroll
-    for (int i = 0; i < V; i += 4)
-      *reinterpret_cast<float4*>(dst + (size_t)r * a.ldo + i) = make_float4(y[i] * mul, y[i + 1] * mul, y[i + 2] * mul, y[i + 3] * mul);
   }
 }
 
@@ -118,7 +179,7 @@ template <typename TA>
 __global__ void __launch_bounds__(kCapWarps * 32)
 conv_rec_prep_kernel(CrpArgs a) {
   constexpr int kPer = 16;                             // columns per lane: widths up to 512
-  const CapWork m = cap_work<kCapRows>(a);
+  const CapWork m = cap_work(a, kCapRows);
   const int hs = blockIdx.y * kCapWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (m.n <= 0 || hs >= a.n_heads) return;
   const CrpHead h = crp_head(a, hs);
@@ -192,7 +253,12 @@ extern "C" int b200_conv_rec_prep(const void* proj, int f32, int64_t ld, const f
   auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   const bool fast = whole && al(proj) && al(conv_w) && al(out) && al(a.ring) && taps <= 4 && ld % vec == 0 && ldo % 4 == 0 && a.C % 4 == 0 &&
                     (!unit || wmax / vec <= 32);
-  const int rows = fast ? 4 : kCapRows;
+  // rows per item: the more the fewer loads of weights and of rows before it, but items enough to fill the GPU (two CTAs per SM,
+  // three of fp32 rows) four times; tiles are whole multiples
+  int rows = fast ? 4 : kCapRows;
+  if (fast)
+    while (rows < 32 && tile_rows % (2 * rows) == 0 && (int64_t)n_tiles * (tile_rows / (2 * rows)) * ((a.C / vec + kCapWarps * 32 - 1) / (kCapWarps * 32)) >= 4 * (f32 ? 3 : 2) * 148)
+      rows *= 2;
   a.per_tile = n_tiles > 0 ? tile_rows / rows : 1;
   a.n_pieces = n_tiles * a.per_tile;
   const int n_x = a.n_pieces + n_single;
@@ -210,7 +276,7 @@ extern "C" int b200_conv_rec_prep(const void* proj, int f32, int64_t ld, const f
     const int all_warps = (a.n_heads + 32 / lph - 1) / (32 / lph), ny = (all_warps + kCapWarps - 1) / kCapWarps;
     const int warps = (all_warps + ny - 1) / ny;
     const dim3 grid(n_x, ny);
-#define B200_CRP(TA, N) conv_rec_prep_vec_kernel<TA, N, 4><<<grid, warps * 32, 0, s>>>(a, lph)
+#define B200_CRP(TA, N) conv_rec_prep_vec_kernel<TA, N><<<grid, warps * 32, 0, s>>>(a, lph, rows)
 #define B200_CRPT(TA)                        \
   switch (taps) {                            \
     case 1: B200_CRP(TA, 1); break;          \

@@ -51,34 +51,6 @@ struct GatedScanArgs {
   int most_rows;                   // sequences with more new rows are another kernel's
 };
 
-// two fp32 numbers in one 64-bit register pair: the packed fused multiply-add of sm_100
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pack2(float a, float b) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ float sum2(f32x2 v) {
-  float a, b;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-  return a + b;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-
 __device__ __forceinline__ float gs_softplus(float z) { return z > 20.f ? z : log1pf(expf(z)); }
 
 // (decay, step) of a token from the raw gates
@@ -775,12 +747,14 @@ gate_norm_kernel(const float* __restrict__ y, const TA* __restrict__ proj, int64
 
 // Pieces of up to 128 channels (a head): W / 4 neighbouring lanes share one, a thread holds up to N of its row's 16-byte
 // groups in registers and all their loads are in flight together.  Bound by bytes in flight: N 2 where it covers the row (the
-// registers of 8 leave 3 CTAs to an SM: 57 us for 8192 rows of 2048 channels, 38 us now).
+// registers of 8 leave 3 CTAs to an SM: 57 us for 8192 rows of 2048 channels, 38 of 2), and by instructions (325 a thread where the
+// logistic and the root of common.cuh took 455: 31 us now; weights in registers over several rows, the next row's loads in flight: 32).
 template <typename TA, bool AFTER, int N>
 __global__ void __launch_bounds__(kGnThreads)
 gate_norm_heads_kernel(const float* __restrict__ y, const TA* __restrict__ proj, int64_t ld, int z_col, const bf16* __restrict__ w, TA* out,
                        int64_t ldo, int C, int W, float eps) {
   const int t = blockIdx.x, i0 = threadIdx.x * 4, step = kGnThreads * 4, lanes = W >> 2;
+  const float over = 1.0f / (float)W;                  // (a power of two)
   const float* yr = y + (size_t)t * C;
   const TA* zr = proj + (size_t)t * ld + z_col;
   TA* o = out + (size_t)t * ldo;
@@ -807,10 +781,12 @@ gate_norm_heads_kernel(const float* __restrict__ y, const TA* __restrict__ proj,
     float4 x = v[n];
     if (!AFTER) { x.x *= g[n].x; x.y *= g[n].y; x.z *= g[n].z; x.w *= g[n].w; }
     float ss = fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, x.w * x.w)));
-    for (int w_ = lanes >> 1; w_ > 0; w_ >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, w_);
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1)
+      if (s < lanes) ss += __shfl_xor_sync(0xffffffffu, ss, s);
     if (i >= C) continue;
-    const float rstd = 1.0f / sqrtf(ss / (float)W + eps);
-    const float4 c = gs_ld4<bf16>(w + (AFTER ? i % W : i));
+    const float rstd = inv_sqrt(ss * over + eps);
+    const float4 c = gs_ld4<bf16>(w + (AFTER ? i & (W - 1) : i));
     x = make_float4(x.x * rstd * c.x, x.y * rstd * c.y, x.z * rstd * c.z, x.w * rstd * c.w);
     if (AFTER) { x.x *= g[n].x; x.y *= g[n].y; x.z *= g[n].z; x.w *= g[n].w; }
     gs_st4(o + i, x);

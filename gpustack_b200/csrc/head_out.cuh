@@ -1,14 +1,14 @@
 // A recurrent mixer's closing step per (token, head): the head's fp32 output over its root mean square, times a weight, times the
 // gate's activation, rounded once.  A head of dv = 4 LPH values is held by LPH lanes as one 16-byte piece each, one head per group of
-// lanes: many small warps keep the bytes in flight.  Bound: launch and latency up to 1000 rows, then instructions (3.1 per clock and SM,
-// 8192 rows at 4.1 TB/s).  8 heads of 128, bf16 gates, warm: 1.8 us for one row, 5.4 for 2048, 16.3 for 8192 (with four heads in flight per lane
-// 4.5, 7.0 and 19.5; a CTA or a warp per head, looping, 2.6, 7.4 and 22.9).
+// lanes; a group goes through the heads of one number (its weight stays in registers, a step is an addition per pointer), the next
+// head's loads in flight.  Bound: launch and latency up to 1000 rows, then instructions.  8 heads of 128, bf16 gates, 8192 rows:
+// a head per group, its place divided out, 18.9 us (205 instructions a thread), 17.1 now (155 a head).
 #pragma once
 #include "common.cuh"
 
 namespace b200 {
 
-constexpr int kHoThreads = 256;
+constexpr int kHoThreads = 256, kHoCtas = 5;           // CTAs per SM
 
 __device__ __forceinline__ float4 ho_ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ float4 ho_ld4(const bf16* p) {
@@ -19,36 +19,52 @@ __device__ __forceinline__ void ho_st4(float* p, float4 v) { *reinterpret_cast<f
 __device__ __forceinline__ void ho_st4(bf16* p, float4 v) { *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w)); }
 
 template <typename TA, int LPH>
-__global__ void __launch_bounds__(kHoThreads)
+__global__ void __launch_bounds__(kHoThreads, kHoCtas)
 head_out_kernel(const float* __restrict__ o, const TA* __restrict__ proj, int64_t ld, int gate_col, const bf16* __restrict__ w, int w_head,
-                TA* out, int64_t ldo, int items, int H, int silu, float eps) {
+                TA* out, int64_t ldo, int items, int H, int step, int silu, float eps) {
   constexpr int DV = 4 * LPH;
-  const int lane = threadIdx.x & 31, i = (blockIdx.x * (kHoThreads / 32) + (threadIdx.x >> 5)) * (32 / LPH) + lane / LPH, d = (lane % LPH) * 4;
-  const int t = i / H, h = i - t * H;
-  const bool live = i < items;
-  float4 x = make_float4(0.f, 0.f, 0.f, 0.f), g = x;
-  if (live) {
-    x = ho_ld4(o + (size_t)i * DV + d);
-    if (gate_col >= 0) g = ho_ld4(proj + (size_t)t * ld + gate_col + h * DV + d);
+  const int lane = threadIdx.x & 31, d = (lane % LPH) * 4;
+  const int first = (blockIdx.x * (kHoThreads / 32) + (threadIdx.x >> 5)) * (32 / LPH), i0 = first + lane / LPH;
+  if (first >= step) return;                           // (step: a multiple of H)
+  const int t0 = i0 / H, h = i0 - t0 * H, rows = step / H;
+  const bool mine = i0 < step;
+  const float* op = o + (size_t)i0 * DV + d;
+  const TA* gp = gate_col >= 0 ? proj + (size_t)t0 * ld + gate_col + h * DV + d : nullptr;
+  TA* to = out + (size_t)t0 * ldo + h * DV + d;
+  float4 ww = make_float4(1.f, 1.f, 1.f, 1.f);
+  if (mine && w != nullptr) ww = ho_ld4(w + h * w_head + d);
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 x = zero, g = zero;
+  if (mine && i0 < items) {
+    x = ho_ld4(op);
+    if (gate_col >= 0) g = ho_ld4(gp);
   }
-  float ss = fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, x.w * x.w)));
+  for (int at = first, i = i0; at < items; at += step, i += step) {
+    const bool live = mine && i < items;
+    float4 xn = zero, gn = zero;
+    op += (size_t)step * DV;
+    if (mine && i < items - step) {
+      xn = ho_ld4(op);
+      if (gate_col >= 0) gn = ho_ld4(gp += (size_t)rows * ld);
+    }
+    float ss = fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, x.w * x.w)));
 #pragma unroll
-  for (int off = LPH / 2; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
-  if (!live) return;
-  const float mul = 1.0f / sqrtf(ss / (float)DV + eps);
-  float v[4] = {x.x * mul, x.y * mul, x.z * mul, x.w * mul};
-  if (w != nullptr) {
-    const float4 ww = ho_ld4(w + h * w_head + d);
+    for (int off = LPH / 2; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+    const float mul = inv_sqrt(ss * (1.0f / DV) + eps);
+    float v[4] = {x.x * mul, x.y * mul, x.z * mul, x.w * mul};
     v[0] *= ww.x; v[1] *= ww.y; v[2] *= ww.z; v[3] *= ww.w;
-  }
-  if (gate_col >= 0) {
-    const float gv[4] = {g.x, g.y, g.z, g.w};
-    float sg[4];
-    logistic_all<false>(gv, sg);
+    if (gate_col >= 0) {
+      const float gv[4] = {g.x, g.y, g.z, g.w};
+      float sg[4];
+      logistic_all<false>(gv, sg);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) v[e] *= silu ? gv[e] * sg[e] : sg[e];
+      for (int e = 0; e < 4; ++e) v[e] *= silu ? gv[e] * sg[e] : sg[e];
+    }
+    if (live) ho_st4(to, make_float4(v[0], v[1], v[2], v[3]));
+    to += (size_t)rows * ldo;
+    x = xn;
+    g = gn;
   }
-  ho_st4(out + (size_t)t * ldo + h * DV + d, make_float4(v[0], v[1], v[2], v[3]));
 }
 
 // Heads of 32, 64 or 128 values with aligned 4-value pieces on every side; false: the caller's general kernel.
@@ -60,9 +76,13 @@ bool head_out_launch(const float* o, const void* proj, int64_t ld, int gate_col,
       (int64_t)T * H > INT32_MAX / 2)
     return false;
   if (gate_col >= 0 && (ld % 4 != 0 || gate_col % 4 != 0 || ((uintptr_t)proj & al))) return false;
-  const int items = T * H, per = kHoThreads / 32 * (128 / dv), grid = (items + per - 1) / per;
+  const int items = T * H, per = kHoThreads / 32 * (128 / dv);      // groups per CTA
+  // groups in whole multiples of the heads; no more CTAs than are resident
+  int step = items;
+  if (items > kHoCtas * 148 * per && H <= kHoCtas * 148 * per) step = kHoCtas * 148 * per / H * H;
+  const int grid = (step + per - 1) / per;
 #define B200_HO(L)                                                                                                                 \
-  head_out_kernel<TA, L><<<grid, kHoThreads, 0, s>>>(o, (const TA*)proj, ld, gate_col, (const bf16*)w, w_head, (TA*)out, ldo, items, H, \
+  head_out_kernel<TA, L><<<grid, kHoThreads, 0, s>>>(o, (const TA*)proj, ld, gate_col, (const bf16*)w, w_head, (TA*)out, ldo, items, H, step, \
                                                      silu, eps)
   if (dv == 32) B200_HO(8);
   else if (dv == 64) B200_HO(16);

@@ -147,15 +147,17 @@ rot_prep_kernel(RotPrepArgs a) {
 // four tokens share it, which is what a prompt's rotated bf16 rows are bound by; fp32 rows, which are twice the bytes, rows without a
 // rotation, and steps of few tokens keep a CTA per token.  A head is cut into items of VEC = 16 bytes / sizeof(TA) entries: an
 // interleaved rotation turns the pairs inside an item; a half-split rotation makes an item of the piece [d, d + VEC)
-// and its partner [d + dims/2, ...); the unrotated rest are plain items.  LPH lanes (a power of two >= items per
-// head) share a head, a warp covers 32 / LPH head slots at a time, the sum of squares is reduced inside the group.
+// and its partner [d + dims/2, ...), and of a value head's pieces [d, d + VEC) and [d + dv/2, ...) (v_half: with plain items half
+// of the lanes idle on queries and keys: 8 + 8 + 8 heads of 128 into fp32 rows, 8192 rows 43.4 -> 35.0 us, 16 + 4 + 4 into pages
+// 45.4 -> 28.2); the unrotated rest are plain items.  LPH lanes (a power of two >= items per head) share a head, a warp covers
+// 32 / LPH head slots at a time, the sum of squares is reduced inside the group.
 // SILU is an instance of its own: its code, unused, cost the others 2 to 14 %.  Resident CTAs: five of bf16 rows (48 registers; without
 // the bound 58, 2048 rows 12.2 -> 14.1 us), fp32 rows as they compile.
 constexpr int kRvThreads = 256;
 
 template <typename TA, typename TD, int TOK, bool SILU>
 __global__ void __launch_bounds__(kRvThreads, sizeof(TA) == 2 ? 5 : SILU ? 6 : 1)
-rot_prep_vec_kernel(RotPrepArgs a, int T, int lph, int items_q, int items_v) {
+rot_prep_vec_kernel(RotPrepArgs a, int T, int lph, int items_q, int items_v, int v_half) {
   constexpr int VEC = 16 / (int)sizeof(TA);
   extern __shared__ float2 cs_all[];                  // [TOK][dims / 2] (cos, sin) of the tokens
   const int tok0 = blockIdx.x * TOK, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -202,6 +204,7 @@ rot_prep_vec_kernel(RotPrepArgs a, int T, int lph, int items_q, int items_v) {
       const bool rot = !is_v && li < n_rot;
       d0 = is_v ? li * VEC : (rot ? li * VEC : dims + (li - n_rot) * VEC);
       if (rot && a.half_layout) d1 = d0 + half;
+      if (is_v && v_half) d1 = d0 + v_half;
       {
         const uint4 raw = *reinterpret_cast<const uint4*>(src + d0);
         const TA* rv = reinterpret_cast<const TA*>(&raw);
@@ -244,15 +247,16 @@ rot_prep_vec_kernel(RotPrepArgs a, int T, int lph, int items_q, int items_v) {
           x0[i + 1] = v * c.x + u * c.y;
         }
       }
-#pragma unroll
-      for (int i = 0; i < VEC; ++i) {
-        ss = fmaf(x0[i], x0[i], ss);
-        if (d1 >= 0) ss = fmaf(x1[i], x1[i], ss);
-      }
     }
     float mul = is_q ? a.q_mul : a.k_mul;
     if (is_q && a.q_head_mul != nullptr) mul *= a.q_head_mul[g];
-    if (a.unit_norm) {                                 // every lane takes part in the shuffles
+    if (a.unit_norm) {                                 // every lane takes part in the shuffles (what it does not hold is zero)
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) ss = fmaf(x0[i], x0[i], ss);
+      if (d1 >= 0) {
+#pragma unroll
+        for (int i = 0; i < VEC; ++i) ss = fmaf(x1[i], x1[i], ss);
+      }
       for (int o = lph >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
       mul *= 1.0f / sqrtf(ss / (float)dk + a.eps);
     }
@@ -277,6 +281,58 @@ rot_prep_vec_kernel(RotPrepArgs a, int T, int lph, int items_q, int items_v) {
       }
       *reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(dst) + d0) = *reinterpret_cast<uint4*>(w0);
       if (d1 >= 0) *reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(dst) + d1) = *reinterpret_cast<uint4*>(w1);
+    }
+  }
+}
+
+// Rows without a rotation, a norm or a feature map: every column of the queries, keys and values times its factor, a thread's columns in
+// ROWS rows, all their loads in flight together.  Bound by memory: 8 + 8 heads of 64 and 8 of 128 into fp32 rows, 8192 rows 36.3 -> 24.2 us
+// (101 MB), 2048 rows 11.9 -> 7.6, one row 5.3 -> 4.0.
+template <typename TA, typename TD, int ROWS>
+__global__ void __launch_bounds__(kRvThreads)
+rot_plain_kernel(RotPrepArgs a, int T) {
+  constexpr int VEC = 16 / (int)sizeof(TA);
+  const int t0 = blockIdx.y * ROWS, nq = a.H * a.dk, nk = a.G * a.dk;
+  int c = (blockIdx.x * kRvThreads + threadIdx.x) * VEC;
+  if (c >= nq + nk + a.G * a.dv) return;
+  int col = a.q_col;
+  int64_t ld = a.ldq;
+  TD* dst = reinterpret_cast<TD*>(a.q_out);
+  float mul = a.q_mul;
+  if (c >= nq) {
+    c -= nq;
+    col = a.k_col;
+    ld = a.ldk;
+    dst = reinterpret_cast<TD*>(a.k_out);
+    mul = a.k_mul;
+    if (c >= nk) {
+      c -= nk;
+      col = a.v_col;
+      ld = a.ldv;
+      dst = reinterpret_cast<TD*>(a.v_out);
+      mul = 1.f;
+    }
+  }
+  const TA* src = reinterpret_cast<const TA*>(a.proj) + (size_t)t0 * a.ld + col + c;
+  dst += (size_t)t0 * ld + c;
+  uint4 raw[ROWS];
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r)
+    if (t0 + r < T) raw[r] = *reinterpret_cast<const uint4*>(src + (size_t)r * a.ld);
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) {
+    if (t0 + r >= T) break;
+    const TA* x = reinterpret_cast<const TA*>(&raw[r]);
+    TD* to = dst + (size_t)r * ld;
+    if constexpr (sizeof(TD) == 4) {
+#pragma unroll
+      for (int i = 0; i < VEC; i += 4)
+        *reinterpret_cast<float4*>(to + i) = make_float4(rp_f32(x[i]) * mul, rp_f32(x[i + 1]) * mul, rp_f32(x[i + 2]) * mul, rp_f32(x[i + 3]) * mul);
+    } else {
+      uint32_t w[VEC / 2];
+#pragma unroll
+      for (int i = 0; i < VEC; i += 2) w[i / 2] = pack_bf16(rp_f32(x[i]) * mul, rp_f32(x[i + 1]) * mul);
+      *reinterpret_cast<uint4*>(to) = *reinterpret_cast<uint4*>(w);
     }
   }
 }
@@ -321,23 +377,40 @@ extern "C" int b200_rot_prep_hm(const void* proj, int src_f32, int64_t ld, int q
     auto al = [](const void* p_) { return (reinterpret_cast<uintptr_t>(p_) & 15) == 0; };
     const bool has_v = v_col >= 0;
     const int rot_items = dims == 0 ? 0 : (half_layout ? (dims / 2) / vec : dims / vec);
-    const int items_q = rot_items + (dk - dims) / vec, items_v = dv / vec;
+    const int v_half = half_layout && dims > 0 && has_v && dv % (2 * vec) == 0 ? dv / 2 : 0;
+    const int items_q = rot_items + (dk - dims) / vec, items_v = (v_half ? v_half : dv) / vec;
     const int items = items_q > items_v ? items_q : items_v;
     bool ok = dk % vec == 0 && dv % vec == 0 && dims % vec == 0 && (!half_layout || (dims / 2) % vec == 0) && items <= 32 &&
               ld % vec == 0 && q_col % vec == 0 && k_col % vec == 0 && (!has_v || v_col % vec == 0) && al(proj) && al(q_out) &&
               al(k_out) && al(v_out) && (ldq * dsz) % 16 == 0 && (paged || ((ldk * dsz) % 16 == 0 && (ldv * dsz) % 16 == 0)) &&
               (size_t)(dims / 2) * sizeof(float2) <= 40 * 1024 && !(src_f32 && !dst_f32);
+    if (ok && dims == 0 && !unit_norm && feature == 0 && !paged && has_v && k_out != nullptr && q_head_mul == nullptr && q_out != proj) {
+      const int cols = H * dk + G * dk + G * dv, nx = (cols / vec + kRvThreads - 1) / kRvThreads;
+      const bool four = (int64_t)T * nx >= 4 * 4 * 148 && T <= 65535 * 4;
+#define B200_RP(TA, TD)                                                                                          \
+  do {                                                                                                           \
+    if (four) rot_plain_kernel<TA, TD, 4><<<dim3(nx, (T + 3) / 4), kRvThreads, 0, s>>>(a, T);                     \
+    else rot_plain_kernel<TA, TD, 1><<<dim3(nx, T), kRvThreads, 0, s>>>(a, T);                                    \
+  } while (0)
+      if (T <= 65535 || four) {
+        if (src_f32) B200_RP(float, float);
+        else if (dst_f32) B200_RP(bf16, float);
+        else B200_RP(bf16, bf16);
+#undef B200_RP
+        return b200_check_launch("b200_rot_prep");
+      }
+    }
     if (ok) {
       int lph = 1;
       while (lph < items) lph <<= 1;
       // four tokens per CTA of rotated bf16 rows once that still leaves every SM eight CTAs (and their angles fit the default shared
       // memory): 8 + 8 + 8 heads of 128 into fp32 rows, warm, a CTA per token -> four: 4740 rows 25.3 -> 24.5 us, 8192 rows 49.0 ->
       // 41.6; 16 + 4 + 4 heads into pages 31.1 -> 31.4 and 56.8 -> 50.7.  fp32 rows lose by it: 4800 rows 32.2 -> 38.0, 8192 rows 52.2 ->
-      // 57.0; rows without a rotation too: 18.9 -> 21.2 and 34.7 -> 34.7
+      // 57.0 (all before values went in pairs of pieces)
       const size_t smem = (size_t)(dims / 2) * sizeof(float2);
       const bool four = !src_f32 && dims > 0 && T >= 4 * 8 * 148 && 4 * smem <= 40 * 1024;
 #define B200_RVS(TA, TD, TOK, S)                                                                                                  \
-  rot_prep_vec_kernel<TA, TD, TOK, S><<<(T + TOK - 1) / TOK, kRvThreads, TOK * smem, s>>>(a, T, lph, items_q, items_v)
+  rot_prep_vec_kernel<TA, TD, TOK, S><<<(T + TOK - 1) / TOK, kRvThreads, TOK * smem, s>>>(a, T, lph, items_q, items_v, v_half)
 #define B200_RV(TA, TD, TOK)                        \
   do {                                              \
     if (feature == 1) B200_RVS(TA, TD, TOK, true);  \
