@@ -312,15 +312,25 @@ latent_attn_mma_kernel(LaArgs a) {
 // Bound: instructions beside the cache's bytes; 64 sequences of 2048 rows of 576, 4 ranges, L2 cold: 67 us in the kernel above,
 // 51 here (57 with every warp forming all probabilities and two buffers, 64 with that and blocks of 16 keys).
 constexpr int kLdHalf = 16, kLdBufs = 5, kLdMaxW = 576, kLdSteps = kLdMaxW / 16 / 4;
+// a page's 16 rows of all slabs
+__device__ __forceinline__ void ld_rows(void* dst, const CUtensorMap* map, uint64_t* bar, int row) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %3}], [%2];" ::"r"(smem_u32(dst)),
+               "l"(map), "r"(smem_u32(bar)), "r"(0), "r"(row)
+               : "memory");
+}
 constexpr int kLdPitch = kLaKeys + 8;                  // floats per row of a partial score tile: conflict-free pairs
 
-template <int NT>   // n-tiles (8 columns) of the output per warp: R = 64 NT
+// TMA: pages of 16 rows, each as one copy [W / 64 slabs][16 rows][128 bytes], the eight 16-byte pieces of a row's slab exchanged by the row (the
+// 128-byte swizzle); else rows by cp.async, padded to `pitch`.
+template <int NT, bool TMA>   // n-tiles (8 columns) of the output per warp: R = 64 NT
 __global__ void __launch_bounds__(kLaWarps * 32, 2)
-latent_attn_step_kernel(LaArgs a) {
-  extern __shared__ __align__(16) uint8_t smem[];
+latent_attn_step_kernel(const __grid_constant__ CUtensorMap rows_map, LaArgs a) {
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  __shared__ uint64_t full[kLdBufs];
+  uint8_t* smem = TMA ? reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023)) : smem_raw;
   const int W = a.W, R = a.R, HB = a.HB;
-  const int pitch = W * 2 + 16, buf_bytes = kLdHalf * pitch;
-  uint8_t* k_s = smem;                                // [5][16][pitch]; the queries pass through the last buffer
+  const int pitch = W * 2 + 16, buf_bytes = kLdHalf * (TMA ? W * 2 : pitch);
+  uint8_t* k_s = smem;                                // [5][16 rows]; the queries pass through the last two buffers, padded
   float* s_s = reinterpret_cast<float*>(k_s + kLdBufs * buf_bytes);      // [4 quarters][16][kLdPitch]
   uint8_t* p_s = reinterpret_cast<uint8_t*>(s_s + 4 * 16 * kLdPitch);    // [16][kLaPPitch]
   float* f_s = reinterpret_cast<float*>(p_s + 16 * kLaPPitch);           // [3][16]: accumulators' factor; at the end maximum, sum
@@ -347,7 +357,20 @@ latent_attn_step_kernel(LaArgs a) {
   const int n = n_blk - blk_begin, key_begin = blk_begin * kLaKeys;
   const int32_t* bt = a.block_table + (size_t)s * a.max_blocks;
   const int cpr = W / 8;
-  auto issue = [&](int half, int buf) {                // a warp copies two whole key rows
+  if (TMA && threadIdx.x == 0) {
+    tma_prefetch_desc(&rows_map);
+    for (int i = 0; i < kLdBufs; ++i) mbar_init(&full[i], 1);
+    fence_mbar_init();
+  }
+  const int pages = (kv_end + kLdHalf - 1) / kLdHalf - key_begin / kLdHalf;      // of this range and those behind it
+  auto issue = [&](int half, int buf) {                // a page by one copy, or two whole key rows per warp
+    if constexpr (TMA) {
+      if (threadIdx.x == 0 && half < 2 * n && half < pages) {
+        mbar_expect_tx(&full[buf], buf_bytes);
+        ld_rows(k_s + buf * buf_bytes, &rows_map, &full[buf], __ldg(bt + key_begin / kLdHalf + half) * kLdHalf);
+      }
+      return;
+    }
     if (half < 2 * n) {
 #pragma unroll
       for (int r = warp; r < kLdHalf; r += kLaWarps) {
@@ -362,6 +385,7 @@ latent_attn_step_kernel(LaArgs a) {
     }
     cp_async_commit();
   };
+  if (TMA) __syncthreads();
 #pragma unroll
   for (int i = 0; i < 3; ++i) issue(i, i);
   const int t0 = lane >> 2, c0 = 2 * (lane & 3);
@@ -369,7 +393,7 @@ latent_attn_step_kernel(LaArgs a) {
   const int quarter = (W / 16 + 3) / 4, ks0 = (warp >> 1) * quarter, steps = min(W / 16 - ks0, quarter);
   uint32_t q[kLdSteps][4];
   {
-    uint8_t* q_s = k_s + (kLdBufs - 1) * buf_bytes;
+    uint8_t* q_s = k_s + (kLdBufs - (TMA ? 2 : 1)) * buf_bytes;
     for (int ci = threadIdx.x; ci < 16 * cpr; ci += blockDim.x) {
       const int i = ci / cpr, c = ci - i * cpr;
       uint4 v = make_uint4(0, 0, 0, 0);
@@ -392,7 +416,23 @@ latent_attn_step_kernel(LaArgs a) {
   int buf = 0;                                          // of the block's first half
   for (int i = 0; i < n; ++i) {
     const int buf1 = buf + 1 == kLdBufs ? 0 : buf + 1;
-    cp_async_wait<1>();
+    if constexpr (TMA) {
+      // half h of the range passes through buffer h % 5 for the (h / 5)-th time
+      mbar_wait_guarded(&full[buf], (2 * i / kLdBufs) & 1);
+      const bool both = 2 * i + 1 < pages;              // (the last page of an odd number: rows of zeros beside it)
+      if (both) mbar_wait_guarded(&full[buf1], ((2 * i + 1) / kLdBufs) & 1);
+      const int rest = kv_end - (key_begin + i * kLaKeys);
+      if (rest < kLaKeys) {                             // behind the sequence: whatever the page holds times zero must be no number
+        for (int e = threadIdx.x; e < (kLaKeys - rest) * cpr; e += kLaWarps * 32) {
+          const int r = rest + e / cpr, c = e % cpr;
+          *reinterpret_cast<uint4*>(k_s + (r < kLdHalf ? buf : buf1) * buf_bytes + (c >> 3) * (kLdHalf * 128) + (r & 15) * 128 + (c & 7) * 16) =
+              make_uint4(0, 0, 0, 0);
+        }
+      }
+      if (i == 0) fence_proxy_async();                  // the queries' buffers are a copy's next
+    } else {
+      cp_async_wait<1>();
+    }
     __syncthreads();                                    // block i visible; the block before (or the queries) is used
     {
       const int b3 = buf + 3 >= kLdBufs ? buf + 3 - kLdBufs : buf + 3, b4 = b3 + 1 == kLdBufs ? 0 : b3 + 1;
@@ -403,12 +443,14 @@ latent_attn_step_kernel(LaArgs a) {
     float sa[4] = {0.f, 0.f, 0.f, 0.f}, sb[4] = {0.f, 0.f, 0.f, 0.f};
     {
       // one ldmatrix.x4 per step: keys 0-7 and 8-15, low and high half of the step's columns
-      const uint32_t kb_addr = ((warp & 1) ? k1_base : k0_base) + (arr + (ai >> 1) * 8) * pitch + ks0 * 32 + (ai & 1) * 16;
+      const uint32_t kb = (warp & 1) ? k1_base : k0_base;
+      const uint32_t kb_addr = kb + (arr + (ai >> 1) * 8) * (TMA ? 128 : pitch) + (TMA ? 0 : ks0 * 32 + (ai & 1) * 16);
 #pragma unroll
       for (int j = 0; j < kLdSteps; ++j) {
         if (j >= steps) break;
         uint32_t b0, b1, b2, b3;
-        ldsm_x4(kb_addr + j * 32, b0, b1, b2, b3);
+        const int chunk = 2 * (ks0 + j) + (ai & 1);     // the row's 16-byte piece
+        ldsm_x4(TMA ? kb_addr + (chunk >> 3) * (kLdHalf * 128) + ((chunk & 7) ^ arr) * 16 : kb_addr + j * 32, b0, b1, b2, b3);
         mma_bf16_16816(sa, q[j], b0, b1);
         mma_bf16_16816(sb, q[j], b2, b3);
       }
@@ -445,18 +487,19 @@ latent_attn_step_kernel(LaArgs a) {
     for (int kk = 0; kk < 2; ++kk) {
       uint32_t pa[4];
       ldsm_x4(smem_u32(p_s) + a_row * kLaPPitch + (2 * kk + (ai >> 1)) * 16, pa[0], pa[1], pa[2], pa[3]);
-      const uint32_t v_addr = (kk ? k1_base : k0_base) + a_row * pitch + (warp * NT + (ai >> 1)) * 16;
+      const uint32_t v_base = kk ? k1_base : k0_base, v_addr = v_base + a_row * pitch + (warp * NT + (ai >> 1)) * 16;
 #pragma unroll
       for (int c = 0; c < NT; c += 2) {
         uint32_t b0, b1, b2, b3;
-        ldsm_x4_t(v_addr + c * 16, b0, b1, b2, b3);
+        const int chunk = warp * NT + (ai >> 1) + c;
+        ldsm_x4_t(TMA ? v_base + (chunk >> 3) * (kLdHalf * 128) + a_row * 128 + ((chunk & 7) ^ arr) * 16 : v_addr + c * 16, b0, b1, b2, b3);
         mma_bf16_16816(o[c], pa, b0, b1);
         mma_bf16_16816(o[c + 1], pa, b2, b3);
       }
     }
     buf = buf1 + 1 == kLdBufs ? 0 : buf1 + 1;
   }
-  cp_async_wait<0>();
+  if (!TMA) cp_async_wait<0>();
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
     const float sum = warp_sum(l[r]);
@@ -562,16 +605,28 @@ static int la_launch(const LaArgs& a, dim3 grid, cudaStream_t s) {
   return b200_check_launch("b200_latent_attn");
 }
 
-template <int NT>
-static int ld_launch(const LaArgs& a, dim3 grid, cudaStream_t s) {
-  const size_t smem = (size_t)kLdBufs * kLdHalf * (a.W * 2 + 16) + (4 * 16 * kLdPitch + 3 * 16) * sizeof(float) + 16 * kLaPPitch;
-  const cudaError_t e = cudaFuncSetAttribute(latent_attn_step_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+template <int NT, bool TMA>
+static int ld_launch_form(const CUtensorMap& map, const LaArgs& a, dim3 grid, cudaStream_t s) {
+  const size_t smem = (size_t)kLdBufs * kLdHalf * (TMA ? a.W * 2 : a.W * 2 + 16) + (TMA ? 1024 : 0) + (4 * 16 * kLdPitch + 3 * 16) * sizeof(float) +
+                      16 * kLaPPitch;
+  const cudaError_t e = cudaFuncSetAttribute(latent_attn_step_kernel<NT, TMA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) {
     b200_set_error("latent_attn_decode: cudaFuncSetAttribute(smem=%zu): %s", smem, cudaGetErrorString(e));
     return B200_ERR_CUDA;
   }
-  latent_attn_step_kernel<NT><<<grid, kLaWarps * 32, smem, s>>>(a);
+  latent_attn_step_kernel<NT, TMA><<<grid, kLaWarps * 32, smem, s>>>(map, a);
   return b200_check_launch("b200_latent_attn_decode");
+}
+
+template <int NT>
+static int ld_launch(const LaArgs& a, dim3 grid, cudaStream_t s) {
+  CUtensorMap map = {};
+  if (a.page != kLdHalf || a.W % 64 != 0) return ld_launch_form<NT, false>(map, a, grid, s);
+  // (the number of pages is not known here; the block table's are)
+  const uint64_t dims[3] = {64, (uint64_t)1 << 31, (uint64_t)a.W / 64}, strides[2] = {(uint64_t)a.W * 2, 128};
+  const uint32_t box[3] = {64, kLdHalf, (uint32_t)a.W / 64};
+  if (const int rc = make_tmap_bf16_nd(&map, a.cache, 3, dims, strides, box)) return rc;
+  return ld_launch_form<NT, true>(map, a, grid, s);
 }
 
 static int la_dispatch(const LaArgs& a, dim3 grid, cudaStream_t s) {
