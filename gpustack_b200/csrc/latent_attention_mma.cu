@@ -312,6 +312,12 @@ latent_attn_mma_kernel(LaArgs a) {
 // Bound: instructions beside the cache's bytes; 64 sequences of 2048 rows of 576, 4 ranges, L2 cold: 67 us in the kernel above,
 // 51 here (57 with every warp forming all probabilities and two buffers, 64 with that and blocks of 16 keys).
 constexpr int kLdHalf = 16, kLdBufs = 5, kLdMaxW = 576, kLdSteps = kLdMaxW / 16 / 4;
+// the largest of a warp's values, in one instruction
+__device__ __forceinline__ float warp_max_redux(float v) {
+  float r;
+  asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
 // a page's 16 rows of all slabs
 __device__ __forceinline__ void ld_rows(void* dst, const CUtensorMap* map, uint64_t* bar, int row) {
   asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %3}], [%2];" ::"r"(smem_u32(dst)),
@@ -462,19 +468,25 @@ latent_attn_step_kernel(const __grid_constant__ CUtensorMap rows_map, LaArgs a) 
     __syncthreads();
 
     const bool seen = key_begin + i * kLaKeys + lane < kv_end;
+    float v[2], mn[2];
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
-      const int row = 2 * warp + r;
-      const float* at = s_s + row * kLdPitch + lane;
-      float v = (at[0] + at[16 * kLdPitch]) + (at[32 * kLdPitch] + at[48 * kLdPitch]);     // (a quarter without steps: zeros)
-      v = seen ? v * a.scale_log2 : -INFINITY;
-      const float mn = fmaxf(m[r], warp_max(v));        // a block's first key is one that the row sees: finite
-      const float f = ex2_approx(m[r] - mn), p = ex2_approx(v - mn);
-      m[r] = mn;
+      const float* at = s_s + (2 * warp + r) * kLdPitch + lane;
+      v[r] = (at[0] + at[16 * kLdPitch]) + (at[32 * kLdPitch] + at[48 * kLdPitch]);        // (a quarter without steps: zeros)
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      v[r] = seen ? v[r] * a.scale_log2 : -INFINITY;
+      mn[r] = warp_max_redux(v[r]);
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      mn[r] = fmaxf(m[r], mn[r]);                       // a block's first key is one that the row sees: finite
+      const float f = ex2_approx(m[r] - mn[r]), p = ex2_approx(v[r] - mn[r]);
+      m[r] = mn[r];
       l[r] = l[r] * f + p;
-      const bf16 pb = __float2bfloat16_rn(p);
-      *reinterpret_cast<bf16*>(p_s + row * kLaPPitch + lane * 2) = pb;
-      if (lane == 0) f_s[row] = f;
+      *reinterpret_cast<bf16*>(p_s + (2 * warp + r) * kLaPPitch + lane * 2) = __float2bfloat16_rn(p);
+      if (lane == 0) f_s[2 * warp + r] = f;
     }
     __syncthreads();
 
