@@ -15,7 +15,7 @@
 // 64 rows and head, written, carried and read once each).  Everything is fp32 FMAs as before; bound: the FMA rate
 // (4 dk dv + 64 (dk + dv) per row and head), which register tiles of packed pairs (fma.rn.f32x2) approach: a CTA of 256 threads
 // holds a 128 x 128 (state) or 64 x 128 (output) tile, one 16-byte shared-memory read feeds 8 to 16 FMAs.
-// Gated linear attention, 5 ragged prompts of 6007 rows, 8 heads of 64 x 128: state 57, carry 12, output 85 us (one-pass, the layer
+// Gated linear attention, 5 ragged prompts of 6007 rows, 8 heads of 64 x 128: state 44, carry 12, output 85 us (one-pass, the layer
 // 501 us, so 224).  State space, one prompt of 2048 rows, 32 heads of 128 x 64: 37, 14, 82 us (one-pass 207).  The copies behind the
 // sums and the carry's whole lines are worth a tenth (measured over linear attention's 4 x 2048 rows before it left: 62, 44, 104 us,
 // without them 65, 62, 116).  Chunks of 64: with 32 the states double, with 128 the chunk's own rows cost more FMAs than the states save.
