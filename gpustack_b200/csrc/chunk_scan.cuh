@@ -13,12 +13,16 @@
 // dv / 32) CTAs -- 128 CTAs at 6 us per 16 rows for four prompts -- and idles the chip.  Chunks are independent but for the
 // elementwise carry, so a portion of any length fills the chip; the price is the chunks' states through L2 (dk dv 4 bytes per
 // 64 rows and head, written, carried and read once each).  Everything is fp32 FMAs as before; bound: the FMA rate
-// (4 dk dv + 64 (dk + dv) per row and head), which register tiles of packed pairs (fma.rn.f32x2) approach: a CTA of 256 threads
-// holds a 128 x 128 (state) or 64 x 128 (output) tile, one 16-byte shared-memory read feeds 8 to 16 FMAs.
-// Gated linear attention, 5 ragged prompts of 6007 rows, 8 heads of 64 x 128: state 44, carry 12, output 85 us (one-pass, the layer
-// 501 us, so 224).  State space, one prompt of 2048 rows, 32 heads of 128 x 64: 37, 14, 82 us (one-pass 207).  The copies behind the
-// sums and the carry's whole lines are worth a tenth (measured over linear attention's 4 x 2048 rows before it left: 62, 44, 104 us,
-// without them 65, 62, 116).  Chunks of 64: with 32 the states double, with 128 the chunk's own rows cost more FMAs than the states save.
+// (4 dk dv + 64 (dk + dv) per row and head) and, next to it, shared memory: a 16-byte read takes it four cycles for a warp of many
+// addresses and two for a warp of one, a packed FMA (fma.rn.f32x2) a scheduler two.  So a CTA of 256 threads holds a 128 x 128 (state)
+// or 64 x 128 (output) tile in which a warp shares its keys or rows and its lanes the 128 values: per key or row of 8 x 128, two reads
+// of one address and one of many feed 16 packed FMAs, 64 cycles of either for the eight warps (4 x 8 tiles, two sets of keys or
+// rows to a warp: 96 of reads).
+// Gated linear attention, 5 ragged prompts of 6007 rows, 8 heads of 64 x 128: state 42, carry 12, output 67 us (with 4 x 8 tiles and
+// the weights pair by pair 44, 12, 85; one-pass, the layer 501 us, so 177).  State space, one prompt of 2048 rows, 32 heads of
+// 128 x 64: 36, 14, 79 us (one-pass 191).  The copies behind the sums and the carry's whole lines are worth a tenth (measured over
+// linear attention's 4 x 2048 rows before it left: 62, 44, 104 us, without them 65, 62, 116).  Chunks of 64: with 32 the states double,
+// with 128 the chunk's own rows cost more FMAs than the states save.
 // Sequences of at most kCsShort rows are left to the caller's one-pass kernel (their state would cross L2 three times for
 // a few rows of work).
 #pragma once
@@ -227,13 +231,14 @@ chunk_state_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   float* lo = hi + kCsRows * (DK + 4);
   if constexpr (Form::kVector) Form::template sums<DK>(p, a, scratch, h, at, hi, lo);
   else Form::state_weights(p, a, scratch, h, at);
-  constexpr int KI = DK / 64, VJ = VT / 64;
-  const int vg = tid & 15, kg = tid >> 4;
-  cs_f2 acc[KI * 4][VJ * 2];
+  // a thread: KR keys (in pairs) x 4 values; the lanes of a group share the keys
+  constexpr int LANES = VT / 4, KR = DK / (kCsThreads / LANES);
+  const int vl = tid % LANES, kg = tid / LANES;
+  cs_f2 acc[KR / 2][4];
 #pragma unroll
-  for (int i = 0; i < KI * 4; ++i)
+  for (int i = 0; i < KR / 2; ++i)
 #pragma unroll
-    for (int j = 0; j < VJ * 2; ++j) acc[i][j] = 0ull;
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
 #pragma unroll
   for (int e = 0; e < 2; ++e) {
     if (e == 0) cp_async_wait<1>();
@@ -241,46 +246,42 @@ chunk_state_kernel(const ChunkScanArgs a, const typename Form::Params p) {
     __syncthreads();
     const int n = min(at.rows - 32 * e, 32);
     if constexpr (Form::kVector) {
-      const float* Fh = hi + (at.rows - 1) * (DK + 4);
-      const float* Fl = lo + (at.rows - 1) * (DK + 4);
-      for (int i = tid; i < n * DK; i += kCsThreads) {
-        const int s = 32 * e + i / DK, k = i % DK;
-        ks[s * DK + k] *= cs_exp2(Fh[k] - hi[s * (DK + 4) + k], Fl[k] - lo[s * (DK + 4) + k]);
-      }
+      const int k = tid % DK;
+      const float Fh = hi[(at.rows - 1) * (DK + 4) + k], Fl = lo[(at.rows - 1) * (DK + 4) + k];
+#pragma unroll 4
+      for (int s = 32 * e + tid / DK; s < 32 * e + n; s += kCsThreads / DK)
+        ks[s * DK + k] *= cs_exp2(Fh - hi[s * (DK + 4) + k], Fl - lo[s * (DK + 4) + k]);
       __syncthreads();
     }
 #pragma unroll 4
     for (int r = 0; r < n; ++r) {
       const int s = 32 * e + r;
-      float w = 1.0f;
-      if constexpr (!Form::kVector) w = scratch.w[s];
-      float4 kk[KI];
-      ulonglong2 vv[VJ];
+      float4 v = *reinterpret_cast<const float4*>(vs + s * VT + 4 * vl);
+      if constexpr (!Form::kVector) {
+        const float w = scratch.w[s];
+        v = make_float4(v.x * w, v.y * w, v.z * w, v.w * w);
+      }
+      const cs_f2 d[4] = {cs_dup(v.x), cs_dup(v.y), cs_dup(v.z), cs_dup(v.w)};
 #pragma unroll
-      for (int i = 0; i < KI; ++i) kk[i] = *reinterpret_cast<const float4*>(ks + s * DK + 4 * kg + 64 * i);
+      for (int i = 0; i < KR / 4; ++i) {
+        const ulonglong2 kk = *reinterpret_cast<const ulonglong2*>(ks + s * DK + KR * kg + 4 * i);
 #pragma unroll
-      for (int j = 0; j < VJ; ++j) vv[j] = *reinterpret_cast<const ulonglong2*>(vs + s * VT + 4 * vg + 64 * j);
-#pragma unroll
-      for (int i = 0; i < KI; ++i) {
-        const cs_f2 d[4] = {cs_dup(kk[i].x * w), cs_dup(kk[i].y * w), cs_dup(kk[i].z * w), cs_dup(kk[i].w * w)};
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-          for (int j = 0; j < VJ; ++j) {
-            acc[i * 4 + u][2 * j] = cs_fma(d[u], vv[j].x, acc[i * 4 + u][2 * j]);
-            acc[i * 4 + u][2 * j + 1] = cs_fma(d[u], vv[j].y, acc[i * 4 + u][2 * j + 1]);
-          }
+        for (int j = 0; j < 4; ++j) {
+          acc[2 * i][j] = cs_fma(kk.x, d[j], acc[2 * i][j]);
+          acc[2 * i + 1][j] = cs_fma(kk.y, d[j], acc[2 * i + 1][j]);
+        }
       }
     }
   }
-  float* out = a.ws + ((size_t)blockIdx.x * a.H + h) * DK * a.dv;
+  float* out = a.ws + (((size_t)blockIdx.x * a.H + h) * DK + KR * kg) * a.dv + v0 + 4 * vl;
+  if (v0 + 4 * vl < a.dv) {
 #pragma unroll
-  for (int i = 0; i < KI * 4; ++i)
-#pragma unroll
-    for (int j = 0; j < VJ; ++j) {
-      const int k = 4 * kg + 64 * (i >> 2) + (i & 3), v = v0 + 4 * vg + 64 * j;
-      if (v < a.dv) *reinterpret_cast<ulonglong2*>(out + (size_t)k * a.dv + v) = make_ulonglong2(acc[i][2 * j], acc[i][2 * j + 1]);
+    for (int i = 0; i < KR / 2; ++i) {
+      const float2 u[4] = {cs_split(acc[i][0]), cs_split(acc[i][1]), cs_split(acc[i][2]), cs_split(acc[i][3])};
+      *reinterpret_cast<float4*>(out + (size_t)(2 * i) * a.dv) = make_float4(u[0].x, u[1].x, u[2].x, u[3].x);
+      *reinterpret_cast<float4*>(out + (size_t)(2 * i + 1) * a.dv) = make_float4(u[0].y, u[1].y, u[2].y, u[3].y);
     }
+  }
   if constexpr (Form::kVector) {
     if (blockIdx.z == 0) {
       if (tid < DK) {
@@ -356,40 +357,208 @@ chunk_carry_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   }
 }
 
-// acc[i][.] += sum over 4 rows of B: rows t = tg + 16 i of P (pitch `pp`, columns c .. c + 3), i >= I0.  DIAG >= 0: the rows of
-// B are the chunk's own rows 16 I0 + DIAG .. + 3, which the rows t of block I0 see only up to themselves -- the rest is left
-// out, not multiplied by zero, so that a value that is no number reaches no earlier row.
-template <int VT, int I0, int DIAG = -1>
-__device__ __forceinline__ void cs_outer(cs_f2 (&acc)[4][VT / 32], const float* P, int pp, const float* B, int tg, int vg) {
-  constexpr int VJ = VT / 64;
-  float4 pr[4];
+// How chunk_output's threads share the 64 rows x VT values: VT / 4 lanes side by side are a group, a thread has 4 values of the
+// group's rows, which lie in pairs (2 g, 2 g + 1) + i * BLOCK.  Queries and weights lie transposed, [key or row][64], a
+// group's rows side by side, so that one read serves a whole group (half the price of one with addresses of its own) and its pairs
+// are the operands of packed FMAs.
+template <int VT>
+struct CsRows {
+  static constexpr int kLanes = VT / 4, kGroups = kCsThreads / kLanes, kRows = kCsRows / kGroups, kPairs = kRows / 2, kBlock = 2 * kGroups;
+  static __device__ __forceinline__ int place(int t) { return t % kBlock / 2 * kRows + t / kBlock * 2 + (t & 1); }
+};
+
+// a group's rows of one key or row: its pairs
+template <int VT>
+__device__ __forceinline__ void cs_pairs(const float* p, cs_f2 (&out)[CsRows<VT>::kPairs]) {
 #pragma unroll
-  for (int i = I0; i < 4; ++i) pr[i] = *reinterpret_cast<const float4*>(P + (tg + 16 * i) * pp);
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    ulonglong2 b[VJ];
-#pragma unroll
-    for (int j = 0; j < VJ; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(B + e * VT + 4 * vg + 64 * j);
-#pragma unroll
-    for (int i = I0; i < 4; ++i) {
-      if (DIAG >= 0 && i == I0 && DIAG + e > tg) continue;
-      const cs_f2 d = cs_dup(e == 0 ? pr[i].x : e == 1 ? pr[i].y : e == 2 ? pr[i].z : pr[i].w);
-#pragma unroll
-      for (int j = 0; j < VJ; ++j) {
-        acc[i][2 * j] = cs_fma(d, b[j].x, acc[i][2 * j]);
-        acc[i][2 * j + 1] = cs_fma(d, b[j].y, acc[i][2 * j + 1]);
-      }
-    }
+  for (int i = 0; i < CsRows<VT>::kPairs; i += 2) {
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p + 2 * i);
+    out[i] = v.x;
+    out[i + 1] = v.y;
   }
 }
 
-// acc += A V over the chunk's own rows of block I0 (16 of them)
+// acc += weights^T V over the chunk's own rows of block I0.  A row sees those up to itself -- the rest is left out, not multiplied by
+// zero, so that a value that is no number reaches no earlier row.
 template <int VT, int I0>
-__device__ __forceinline__ void cs_own_rows(cs_f2 (&acc)[4][VT / 32], const float* A, const float* V, int tg, int vg) {
-  cs_outer<VT, I0, 0>(acc, A + 16 * I0, kCsAPitch, V + 16 * I0 * VT, tg, vg);
-  cs_outer<VT, I0, 4>(acc, A + 16 * I0 + 4, kCsAPitch, V + (16 * I0 + 4) * VT, tg, vg);
-  cs_outer<VT, I0, 8>(acc, A + 16 * I0 + 8, kCsAPitch, V + (16 * I0 + 8) * VT, tg, vg);
-  cs_outer<VT, I0, 12>(acc, A + 16 * I0 + 12, kCsAPitch, V + (16 * I0 + 12) * VT, tg, vg);
+__device__ __forceinline__ void cs_own_rows(cs_f2 (&acc)[CsRows<VT>::kPairs][4], const float* A, const float* V, int g, int vl) {
+  using R = CsRows<VT>;
+#pragma unroll 4
+  for (int r = 0; r < R::kBlock; ++r) {
+    const int s = R::kBlock * I0 + r;
+    const float4 v = *reinterpret_cast<const float4*>(V + s * VT + 4 * vl);
+    const cs_f2 d[4] = {cs_dup(v.x), cs_dup(v.y), cs_dup(v.z), cs_dup(v.w)};
+    cs_f2 w[R::kPairs];
+    cs_pairs<VT>(A + s * kCsAPitch + R::kRows * g, w);
+    if (r <= 2 * g) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[I0][j] = cs_fma(w[I0], d[j], acc[I0][j]);
+    } else if (r == 2 * g + 1) {
+      const float u = cs_split(w[I0]).y, vv[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 o = cs_split(acc[I0][j]);
+        acc[I0][j] = cs_pack(o.x, fmaf(u, vv[j], o.y));
+      }
+    }
+#pragma unroll
+    for (int i = I0 + 1; i < R::kPairs; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = cs_fma(w[i], d[j], acc[i][j]);
+  }
+}
+
+// The weights k_s . q_t of a recurrence with a decay per key channel, transposed into A, and the queries' part of the state into qs
+// ([key][64] in the order of `place`, times 2^F_t).  Rows are taken in 16 blocks of four.  Within a block the sums are formed term by
+// term, with the decay between the two rows.  Between two blocks the decay comes in three factors, from s to the end of its
+// block, from there to the end of the one before t's, and on to t: no exponent is positive, only the middle one
+// belongs to a pair of blocks, and 4 x 4 sums share it.  (With an exponential for each of the 2080 pairs of rows and each channel,
+// and both rows and their sums read for it, these weights alone kept shared memory busy for 12.3k of the kernel's 31k cycles.)
+// On entry the queries in qs, the keys in B, the sums in hi / lo, all [64][DK + 4]; hi and lo are used up.
+template <int DK, int VT>
+__device__ __forceinline__ void cs_vector_weights(float* qs, float* B, float* hi, float* lo, float* A, bool zero_start) {
+  using R = CsRows<VT>;
+  constexpr int P = DK + 4, QUADS = DK / 4;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  {
+    // the blocks' own weights: 16 lanes share the channels of a block
+    const int b = tid >> 4, c = tid & 15;
+    float sum[10];
+#pragma unroll
+    for (int i = 0; i < 10; ++i) sum[i] = 0.f;
+#pragma unroll
+    for (int e = 0; e < QUADS / 16; ++e) {
+      float q[4][4], k[4][4], h[4][4], l[4][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int from = (4 * b + i) * P + 4 * (c + 16 * e);
+        *reinterpret_cast<float4*>(q[i]) = *reinterpret_cast<const float4*>(qs + from);
+        *reinterpret_cast<float4*>(k[i]) = *reinterpret_cast<const float4*>(B + from);
+        *reinterpret_cast<float4*>(h[i]) = *reinterpret_cast<const float4*>(hi + from);
+        *reinterpret_cast<float4*>(l[i]) = *reinterpret_cast<const float4*>(lo + from);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j <= i; ++j)
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            sum[i * (i + 1) / 2 + j] = fmaf(q[i][u] * k[j][u], ex2_approx((h[i][u] - h[j][u]) + (l[i][u] - l[j][u])), sum[i * (i + 1) / 2 + j]);
+    }
+    float mine = 0.f;
+    int to = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j <= i; ++j) {
+        float v = sum[i * (i + 1) / 2 + j];
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (c == i * (i + 1) / 2 + j) {
+          mine = v;
+          to = (4 * b + j) * kCsAPitch + R::place(4 * b + i);
+        }
+      }
+    if (c < 10) A[to] = mine;
+  }
+  __syncthreads();
+  // a lane has two rows (one of each half), a warp every eighth quad of channels: rows of pitch DK + 4 are read without conflicts
+  constexpr int ITEMS = QUADS / 8 * 2;
+  float qe[ITEMS][4], qt[ITEMS][4];
+#pragma unroll
+  for (int e = 0; e < ITEMS; ++e) {
+    const int t = lane + 32 * (e & 1), k0 = 4 * (warp + 8 * (e >> 1)), from = t * P + k0, end = (t | 3) * P + k0, start = ((t & ~3) - 1) * P + k0;
+    float q[4], k[4], h[4], l[4], eh[4], el[4], sh[4] = {0.f, 0.f, 0.f, 0.f}, sl[4] = {0.f, 0.f, 0.f, 0.f};
+    *reinterpret_cast<float4*>(q) = *reinterpret_cast<const float4*>(qs + from);
+    *reinterpret_cast<float4*>(k) = *reinterpret_cast<const float4*>(B + from);
+    *reinterpret_cast<float4*>(h) = *reinterpret_cast<const float4*>(hi + from);
+    *reinterpret_cast<float4*>(l) = *reinterpret_cast<const float4*>(lo + from);
+    *reinterpret_cast<float4*>(eh) = *reinterpret_cast<const float4*>(hi + end);
+    *reinterpret_cast<float4*>(el) = *reinterpret_cast<const float4*>(lo + end);
+    if (t >= 4) {
+      *reinterpret_cast<float4*>(sh) = *reinterpret_cast<const float4*>(hi + start);
+      *reinterpret_cast<float4*>(sl) = *reinterpret_cast<const float4*>(lo + start);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      k[u] *= cs_exp2(eh[u] - h[u], el[u] - l[u]);
+      qe[e][u] = q[u] * cs_exp2(h[u] - sh[u], l[u] - sl[u]);
+      qt[e][u] = zero_start ? 0.f : q[u] * cs_exp2(h[u], l[u]);
+    }
+    *reinterpret_cast<float4*>(B + from) = *reinterpret_cast<const float4*>(k);
+  }
+  // the sums at the blocks' ends: a warp has two of them
+  constexpr int EK = DK / 32;                        // a lane's channels of a row
+  float e_h[2][EK], e_l[2][EK];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int u = 0; u < EK; ++u) {
+      e_h[i][u] = hi[(4 * (2 * warp + i) + 3) * P + lane + 32 * u];
+      e_l[i][u] = lo[(4 * (2 * warp + i) + 3) * P + lane + 32 * u];
+    }
+  __syncthreads();
+  float* Eh = lo;                                    // [16][DK + 4] each
+  float* El = lo + 16 * P;
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int u = 0; u < EK; ++u) {
+      Eh[(2 * warp + i) * P + lane + 32 * u] = e_h[i][u];
+      El[(2 * warp + i) * P + lane + 32 * u] = e_l[i][u];
+    }
+#pragma unroll
+  for (int e = 0; e < ITEMS; ++e) {
+    const int t = lane + 32 * (e & 1), k0 = 4 * (warp + 8 * (e >> 1));
+    *reinterpret_cast<float4*>(hi + t * P + k0) = *reinterpret_cast<const float4*>(qe[e]);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) qs[(k0 + u) * kCsRows + R::place(t)] = qt[e][u];
+  }
+  __syncthreads();
+  {
+    // 120 pairs of blocks; two lanes share a pair's channels, and start at different ones where their rows lie in the same banks
+    const int half = tid & 1, u = min(tid >> 1, 119);
+    int bt = 1;
+    while (bt * (bt + 1) / 2 <= u) ++bt;
+    const int bs = u - bt * (bt - 1) / 2;
+    cs_f2 acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+#pragma unroll 1
+    for (int d = 0; d < QUADS / 2; ++d) {
+      const int c = 4 * (2 * ((d + (bs >> 1)) & (QUADS / 2 - 1)) + half);
+      const float4 sh = *reinterpret_cast<const float4*>(Eh + (bt - 1) * P + c), sl = *reinterpret_cast<const float4*>(El + (bt - 1) * P + c),
+                   eh = *reinterpret_cast<const float4*>(Eh + bs * P + c), el = *reinterpret_cast<const float4*>(El + bs * P + c);
+      const cs_f2 m0 = cs_pack(ex2_approx((sh.x - eh.x) + (sl.x - el.x)), ex2_approx((sh.y - eh.y) + (sl.y - el.y))),
+                  m1 = cs_pack(ex2_approx((sh.z - eh.z) + (sl.z - el.z)), ex2_approx((sh.w - eh.w) + (sl.w - el.w)));
+      ulonglong2 k[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) k[j] = *reinterpret_cast<const ulonglong2*>(B + (4 * bs + j) * P + c);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        ulonglong2 q = *reinterpret_cast<const ulonglong2*>(hi + (4 * bt + i) * P + c);
+        q.x = cs_mul(q.x, m0);
+        q.y = cs_mul(q.y, m1);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = cs_fma(q.y, k[j].y, cs_fma(q.x, k[j].x, acc[i][j]));
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 z = cs_split(acc[i][j]);
+        v[i] = z.x + z.y;
+      }
+      const float a0 = __shfl_xor_sync(0xffffffffu, half ? v[0] : v[2], 1), a1 = __shfl_xor_sync(0xffffffffu, half ? v[1] : v[3], 1);
+      if (tid < 240)
+        *reinterpret_cast<float2*>(A + (4 * bs + j) * kCsAPitch + R::place(4 * bt + 2 * half)) =
+            half ? make_float2(v[2] + a0, v[3] + a1) : make_float2(v[0] + a0, v[1] + a1);
+    }
+  }
 }
 
 template <int DK, int VT, typename Form>
@@ -401,11 +570,12 @@ chunk_output_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   const ChunkPlace at = cs_place(a, shared5);
   if (at.seq < 0 || at.slot < 0) return;
   const int h = blockIdx.y, v0 = blockIdx.z * VT, tid = threadIdx.x, n = at.rows;
-  constexpr int QP = DK + 4, VJ = VT / 64, TILE = ChunkSmem<DK, VT>::kTile;
+  using R = CsRows<VT>;
+  constexpr int QP = DK + 4, TILE = ChunkSmem<DK, VT>::kTile;
   float* qs = smem;                                  // [64][DK + 4]
   float* X = qs + kCsRows * QP;                      // ring of three tiles of 32 rows; the keys [64][DK + 4] first lie on tiles 1 and 2
   float* B = X + TILE;
-  float* A = B + ChunkSmem<DK, VT, Form::kVector>::kB;              // [64][68]
+  float* A = B + ChunkSmem<DK, VT, Form::kVector>::kB;              // [64][68], a row for each s
   float* hi = A + kCsRows * kCsAPitch;               // [64][DK + 4] each, kVector only; lo behind the keys, until the ring takes the place
   float* lo = B + kCsRows * QP;
   const float* x = reinterpret_cast<const float*>(a.x);
@@ -439,51 +609,10 @@ chunk_output_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   }
   cp_async_wait<1>();
   __syncthreads();
-  const int tg = tid >> 4, vg = tid & 15;
   if constexpr (Form::kVector) {
-    float acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-#pragma unroll 1
-    for (int d = 0; d < DK; d += 4) {
-      float4 k[4], kh[4], kl[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int at_ = (vg + 16 * j) * QP + d;
-        k[j] = *reinterpret_cast<const float4*>(B + at_);
-        kh[j] = *reinterpret_cast<const float4*>(hi + at_);
-        kl[j] = *reinterpret_cast<const float4*>(lo + at_);
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int at_ = (tg + 16 * i) * QP + d;
-        const float4 q = *reinterpret_cast<const float4*>(qs + at_), qh = *reinterpret_cast<const float4*>(hi + at_),
-                     ql = *reinterpret_cast<const float4*>(lo + at_);
-#pragma unroll
-        for (int j = 0; j <= i; ++j) {
-          acc[i][j] = fmaf(q.x * k[j].x, ex2_approx((qh.x - kh[j].x) + (ql.x - kl[j].x)), acc[i][j]);
-          acc[i][j] = fmaf(q.y * k[j].y, ex2_approx((qh.y - kh[j].y) + (ql.y - kl[j].y)), acc[i][j]);
-          acc[i][j] = fmaf(q.z * k[j].z, ex2_approx((qh.z - kh[j].z) + (ql.z - kl[j].z)), acc[i][j]);
-          acc[i][j] = fmaf(q.w * k[j].w, ex2_approx((qh.w - kh[j].w) + (ql.w - kl[j].w)), acc[i][j]);
-        }
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j <= i; ++j) {
-        const int t = tg + 16 * i, s = vg + 16 * j;
-        A[t * kCsAPitch + s] = (s <= t && t < n) ? acc[i][j] : 0.f;
-      }
-    __syncthreads();                                 // the queries as they came are used
-    if (!zero_start)
-      for (int i = tid; i < n * DK; i += kCsThreads) {
-        const int at_ = i / DK * QP + i % DK;
-        qs[at_] *= cs_exp2(hi[at_], lo[at_]);
-      }
+    cs_vector_weights<DK, VT>(qs, B, hi, lo, A, zero_start);
   } else {
+    const int tg = tid >> 4, vg = tid & 15;
     // k_s . q_t: rows t = tg + 16 i, columns s = vg + 16 j, j <= i; even and odd entries summed apart
     cs_f2 acc[4][4];
 #pragma unroll
@@ -509,14 +638,31 @@ chunk_output_kernel(const ChunkScanArgs a, const typename Form::Params p) {
       for (int j = 0; j <= i; ++j) {
         const int t = tg + 16 * i, s = vg + 16 * j;
         const float2 z = cs_split(acc[i][j]);
-        A[t * kCsAPitch + s] = (s <= t && t < n) ? Form::D(p, scratch, t, s) * (z.x + z.y) : 0.f;
+        A[s * kCsAPitch + R::place(t)] = (s <= t && t < n) ? Form::D(p, scratch, t, s) * (z.x + z.y) : 0.f;
       }
+    if (!zero_start) {                               // the queries, [key][64]
+      constexpr int ITEMS = DK / 32 * 2;
+      const int warp = tid >> 5, lane = tid & 31;
+      float4 v[ITEMS];
+#pragma unroll
+      for (int e = 0; e < ITEMS; ++e) v[e] = *reinterpret_cast<const float4*>(qs + (lane + 32 * (e & 1)) * QP + 4 * (warp + 8 * (e >> 1)));
+      __syncthreads();
+#pragma unroll
+      for (int e = 0; e < ITEMS; ++e) {
+        float* to = qs + 4 * (warp + 8 * (e >> 1)) * kCsRows + R::place(lane + 32 * (e & 1));
+        to[0] = v[e].x;
+        to[kCsRows] = v[e].y;
+        to[2 * kCsRows] = v[e].z;
+        to[3 * kCsRows] = v[e].w;
+      }
+    }
   }
-  cs_f2 acc[4][VT / 32];
+  const int g = tid / R::kLanes, vl = tid % R::kLanes;
+  cs_f2 acc[R::kPairs][4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < R::kPairs; ++i)
 #pragma unroll
-    for (int j = 0; j < VT / 32; ++j) acc[i][j] = 0ull;
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
   // tile i: landed, and tile i - 1 used by every thread, so tile i + 2 may take its place (behind the first barrier the keys
   // are used as well)
   auto next_tile = [&](int i) {
@@ -530,35 +676,46 @@ chunk_output_kernel(const ChunkScanArgs a, const typename Form::Params p) {
 #pragma unroll 1
   for (int i = 0; i < n_state; ++i) {
     const float* T = next_tile(i);
-#pragma unroll 2
-    for (int d = 0; d < 32; d += 4) cs_outer<VT, 0>(acc, qs + 32 * i + d, QP, T + d * VT, tg, vg);
+#pragma unroll 4
+    for (int d = 0; d < 32; ++d) {
+      cs_f2 q[R::kPairs];
+      cs_pairs<VT>(qs + (32 * i + d) * kCsRows + R::kRows * g, q);
+      const float4 v = *reinterpret_cast<const float4*>(T + d * VT + 4 * vl);
+      const cs_f2 b[4] = {cs_dup(v.x), cs_dup(v.y), cs_dup(v.z), cs_dup(v.w)};
+#pragma unroll
+      for (int u = 0; u < R::kPairs; ++u)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[u][j] = cs_fma(q[u], b[j], acc[u][j]);
+    }
   }
   if (!zero_start) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const cs_f2 f = cs_dup(Form::aq(scratch, tg + 16 * i));
+    for (int i = 0; i < R::kPairs; ++i) {
+      const int t = R::kBlock * i + 2 * g;
+      const cs_f2 f = cs_pack(Form::aq(scratch, t), Form::aq(scratch, t + 1));
 #pragma unroll
-      for (int j = 0; j < VT / 32; ++j) acc[i][j] = cs_mul(acc[i][j], f);
+      for (int j = 0; j < 4; ++j) acc[i][j] = cs_mul(acc[i][j], f);
     }
   }
+  constexpr int HALF = R::kPairs / 2;                // blocks in each half of the rows
   const float* V0 = next_tile(n_state);
-  cs_own_rows<VT, 0>(acc, A, V0, tg, vg);
-  cs_own_rows<VT, 1>(acc, A, V0, tg, vg);
-  const float* V1 = next_tile(n_state + 1);
-  cs_own_rows<VT, 2>(acc, A, V1 - 32 * VT, tg, vg);
-  cs_own_rows<VT, 3>(acc, A, V1 - 32 * VT, tg, vg);
+  cs_own_rows<VT, 0>(acc, A, V0, g, vl);
+  if constexpr (HALF == 2) cs_own_rows<VT, 1>(acc, A, V0, g, vl);
+  const float* V1 = next_tile(n_state + 1) - 32 * VT;
+  cs_own_rows<VT, HALF>(acc, A, V1, g, vl);
+  if constexpr (HALF == 2) cs_own_rows<VT, 3>(acc, A, V1, g, vl);
+  const int v = v0 + 4 * vl;
+  if (v >= a.dv) return;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int t = tg + 16 * i;
-    if (t >= n) continue;
+  for (int i = 0; i < R::kPairs; ++i) {
+    const float2 u[4] = {cs_split(acc[i][0]), cs_split(acc[i][1]), cs_split(acc[i][2]), cs_split(acc[i][3])};
 #pragma unroll
-    for (int j = 0; j < VJ; ++j) {
-      const int v = v0 + 4 * vg + 64 * j;
-      if (v >= a.dv) continue;
-      const float2 lo = cs_split(acc[i][2 * j]), hi = cs_split(acc[i][2 * j + 1]);
-      const float4 mine = *reinterpret_cast<const float4*>((i < 2 ? V0 + t * VT : V1 + (t - 32) * VT) + 4 * vg + 64 * j);
-      *reinterpret_cast<float4*>(a.o + (size_t)(at.first + t) * a.H * a.dv + h * a.dv + v) =
-          Form::finish(p, scratch, h, t, make_float4(lo.x, lo.y, hi.x, hi.y), mine);
+    for (int e = 0; e < 2; ++e) {
+      const int t = R::kBlock * i + 2 * g + e;
+      if (t >= n) continue;
+      const float4 mine = *reinterpret_cast<const float4*>((i < HALF ? V0 : V1) + t * VT + 4 * vl);
+      const float4 sum = e ? make_float4(u[0].y, u[1].y, u[2].y, u[3].y) : make_float4(u[0].x, u[1].x, u[2].x, u[3].x);
+      *reinterpret_cast<float4*>(a.o + (size_t)(at.first + t) * a.H * a.dv + h * a.dv + v) = Form::finish(p, scratch, h, t, sum, mine);
     }
   }
 }
