@@ -386,7 +386,7 @@ class LLMEngine:
             toks = [int(t) for t in toks]
             if not toks:
                 raise ValueError(f"request {rid}: an entry without tokens")
-            if any(t < 0 or t >= self.mcfg.vocab_size for t in toks):
+            if min(toks) < 0 or max(toks) >= self.mcfg.vocab_size:
                 raise ValueError("token id out of range")
             r = self.requests.get(rid)
             if r is None:
@@ -404,10 +404,14 @@ class LLMEngine:
         for j, e in enumerate(singles):
             bt[j, :len(e[1].blocks)] = e[1].blocks
         dslots = np.asarray([e[1].state_slot for e in singles], dtype=np.int32)
+        # nothing reads the sampled tokens, and the copy of the logits waits for the stream: a wait of the step's own and the
+        # bookkeeping behind it would only keep that copy from following at once (3 rows, graph of 132 us: a step 252 -> 214 us)
+        wait = not any(want for _, _, _, want in chunks + singles)
         if chunks:
             self.runner.prefill([e[2] for e in chunks], [e[1].num_computed for e in chunks], [e[1].blocks for e in chunks],
                                 [e[3] for e in chunks], decode=(B, last, comp, bt) if B else None,
-                                state_slots=([e[1].state_slot for e in chunks] + dslots.tolist()) if self.state_slots else None)
+                                state_slots=([e[1].state_slot for e in chunks] + dslots.tolist()) if self.state_slots else None,
+                                wait=wait)
             n_chunk_rows = sum(len(e[3]) for e in chunks)
             parts, off = {}, 0
             for e in chunks:
@@ -416,7 +420,7 @@ class LLMEngine:
             for j, e in enumerate(singles):
                 parts[e[0]] = range(n_chunk_rows + j, n_chunk_rows + j + (1 if e[3] else 0))
         else:
-            self.runner.decode(B, last, comp, bt, state_slots=dslots if self.state_slots else None)
+            self.runner.decode(B, last, comp, bt, state_slots=dslots if self.state_slots else None, wait=wait)
             parts = {e[0]: range(j, j + (1 if e[3] else 0)) for j, e in enumerate(singles)}
         for _, r, toks, _ in chunks + singles:
             r.prompt_ids.extend(toks)

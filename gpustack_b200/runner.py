@@ -523,9 +523,10 @@ class ModelRunner:
 
     def decode(self, B: int, last_token: np.ndarray, num_computed: np.ndarray, block_table: np.ndarray,
                temps: Optional[np.ndarray] = None, seeds: Optional[np.ndarray] = None,
-               state_slots: Optional[np.ndarray] = None) -> np.ndarray:
+               state_slots: Optional[np.ndarray] = None, wait: bool = True) -> Optional[np.ndarray]:
         """One decode step for rows 0..B-1 of the scheduler's persistent batch.  temps (fp32) / seeds
-        (uint32, already mixed with the position) per row drive the in-kernel sampler; None = greedy."""
+        (uint32, already mixed with the position) per row drive the in-kernel sampler; None = greedy.
+        wait=False: the tokens stay on the device and the caller waits for the stream before it stages another step."""
         S, bs = self.max_seqs, self.block_size
         Bp = B
         if self.graphs:
@@ -562,19 +563,23 @@ class ModelRunner:
             self.stats["kernel_launches"] += self.launches_per_decode
         else:
             self._decode_forward(Bp)
-        self.out_host[:B].copy_(self.out_ids[:B], non_blocking=True)
-        torch.cuda.current_stream().synchronize()
-        self.stats["decode_gpu_s"] = self.stats.get("decode_gpu_s", 0.0) + time.perf_counter() - t_gpu
+        if wait:
+            self.out_host[:B].copy_(self.out_ids[:B], non_blocking=True)
+            torch.cuda.current_stream().synchronize()
+            self.stats["decode_gpu_s"] = self.stats.get("decode_gpu_s", 0.0) + time.perf_counter() - t_gpu
+            self.stats["d2h_bytes"] += B * 4
         self.stats["decode_steps"] += 1
         self.stats["h2d_bytes"] += n * 4
-        self.stats["d2h_bytes"] += B * 4
         self.stats["decode_kv_tokens"] += int(pos.sum()) + B
+        if not wait:
+            return None
         return self.out_host[:B].numpy()
 
     # ------------------------------------------------------------------------------ prefill
     def prefill(self, token_chunks: Sequence[Sequence[int]], starts: Sequence[int], block_tables: Sequence[Sequence[int]],
                 sample: Sequence[bool], decode=None, sample_temps: Optional[Sequence[float]] = None,
-                sample_seeds: Optional[Sequence[int]] = None, state_slots: Optional[Sequence[int]] = None) -> np.ndarray:
+                sample_seeds: Optional[Sequence[int]] = None, state_slots: Optional[Sequence[int]] = None,
+                wait: bool = True) -> Optional[np.ndarray]:
         """Runs one (chunked) prefill step.  token_chunks[s] are the ids of chunk s, which occupies
         positions [starts[s], starts[s]+len).  sample[s] is the number of TRAILING rows of chunk s whose
         next token is sampled (False/0: none, True/1: the last row = a completed prompt, 1 + k: every row
@@ -585,7 +590,7 @@ class ModelRunner:
         both); their B tokens follow the prefill tokens in the returned array.
         sample[s] may also be a LIST of row offsets inside chunk s (a replayed step asks for the logits of
         chosen rows).  state_slots: recurrent-state slot of every chunk, then of every riding decode row
-        (models with recurrent mixers; None = no state)."""
+        (models with recurrent mixers; None = no state).  wait=False: as for decode()."""
         S = len(token_chunks)
         lens = [len(c) for c in token_chunks]
         Tp = sum(lens)
@@ -673,12 +678,14 @@ class ModelRunner:
         self.stats["prefill_steps"] += 1
         self.stats["mixed_steps"] = self.stats.get("mixed_steps", 0) + (1 if Bd else 0)
         self.stats["h2d_bytes"] += end * 4
-        self.stats["d2h_bytes"] += ns * 4
+        self.stats["d2h_bytes"] += ns * 4 if wait else 0
         self.stats["prefill_tokens"] += Tp
         if ns == 0:
             torch.cuda.current_stream().synchronize()
             return np.zeros(0, dtype=np.int32)
         self._sample(ns, sd[o_rows:o_rows + ns], sd[o_st:o_st + ns].view(torch.float32), sd[o_ss:o_ss + ns])
+        if not wait:
+            return None
         self.out_host[:ns].copy_(self.out_ids[:ns], non_blocking=True)
         torch.cuda.current_stream().synchronize()
         return self.out_host[:ns].numpy().copy()
