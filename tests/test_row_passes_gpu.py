@@ -113,3 +113,24 @@ def test_gates_out_of_range_and_no_numbers():
     # four units in the last place; below x = -88.73 the exponential is infinite in fp32 and the result zero, where it is x e^x: at most
     # 88.73 * 2^-128 < 2^-121
     assert bool(((out.to(F64) - want).abs() <= 4 * 2.0 ** -23 * want.abs() + 2.0 ** -121)[~bad].all())
+
+
+# pieces of whole warps: one, several and an odd number of 128s, rows that end inside a pass of the block, the widest in registers and
+# the next
+@pytest.mark.parametrize("C,parts", [(256, 1), (2048, 2), (2048, 1), (1152, 3), (1792, 1), (2176, 1)])
+@pytest.mark.parametrize("dtype", [F32, BF])
+@pytest.mark.parametrize("after", [False, True])
+def test_norm_of_wide_pieces(C, parts, dtype, after):
+    from gpustack_b200 import ops
+
+    T, W = 7, C // parts
+    y, p, w = _rnd(T, C, seed=1), _rnd(T, C + 8, seed=2, dtype=dtype), (1 + _rnd(W if after else C, seed=3) * 0.1).to(BF)
+    y[:, :W] *= 40.0                                                   # pieces of very different size
+    p[:, 8::7] *= 40.0                                                 # gates beyond +-64 beside others
+    out = torch.zeros(T, C + 4, dtype=dtype, device="cuda")
+    ops.gate_norm(y, p, 8, w, out[:, :C], parts, 1e-5, gate_after=after)
+    g, x = torch.nn.functional.silu(p[:, 8:].to(F64)), y.to(F64)
+    x = (x if after else x * g).view(T, parts, W)
+    x = (x / (x.square().mean(-1, keepdim=True) + 1e-5).sqrt() * w.to(F64).view(1 if after else parts, W)).flatten(1)
+    assert _rel(out[:, :C], x * g if after else x) < (1e-6 if dtype == F32 else 4e-3)
+    assert not out[:, C:].any()
