@@ -518,10 +518,12 @@ gated_step_kernel(GatedScanArgs a) {
 template <int L, int R4, int C, bool DELTA>
 int gated_scan_launch(const GatedScanArgs& a, int n_seqs, cudaStream_t s) {
   using Sh = GsShape<L, R4, C>;
-  const cudaError_t e = cudaFuncSetAttribute(gated_scan_kernel<L, R4, C, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::kBytes);
-  if (e != cudaSuccess) {
-    b200_set_error("gated_scan: %zu bytes of shared memory: %s", Sh::kBytes, cudaGetErrorString(e));
-    return B200_ERR_CUDA;
+  if constexpr (Sh::kBytes > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(gated_scan_kernel<L, R4, C, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::kBytes);
+    if (e != cudaSuccess) {
+      b200_set_error("gated_scan: %zu bytes of shared memory: %s", Sh::kBytes, cudaGetErrorString(e));
+      return B200_ERR_CUDA;
+    }
   }
   gated_scan_kernel<L, R4, C, DELTA><<<dim3(n_seqs, a.H, (a.dv + Sh::VW - 1) / Sh::VW), (kGsWarps + kGsHelpers) * 32, Sh::kBytes, s>>>(a);
   return b200_check_launch("b200_gated_scan");
