@@ -310,7 +310,8 @@ latent_attn_mma_kernel(LaArgs a) {
 //   P:   warp w forms rows 2 w and 2 w + 1, a key per lane, and leaves probabilities and the accumulators' factor
 //   O:   warp w accumulates O[16][R / 8 columns from w R / 8].
 // Bound: instructions beside the cache's bytes; 64 sequences of 2048 rows of 576, 4 ranges, L2 cold: 67 us in the kernel above,
-// 51 here (57 with every warp forming all probabilities and two buffers, 64 with that and blocks of 16 keys).
+// 45 here (51 with rows copied by cp.async and maxima by shuffles; before that 57 with every warp forming all probabilities and two
+// buffers, 64 with that and blocks of 16 keys).
 constexpr int kLdHalf = 16, kLdBufs = 5, kLdMaxW = 576, kLdSteps = kLdMaxW / 16 / 4;
 // the largest of a warp's values, in one instruction
 __device__ __forceinline__ float warp_max_redux(float v) {

@@ -23,10 +23,13 @@
 //             saves, 25 us of the whole layer's 573 for 4 x 2048 rows of 16 heads, is not worth that.)
 // Persistent: one pair of CTAs per two SMs walks the heaviest-first (tile, sub-tile, half) list back and forth; barriers, tensor
 // memory and rings live for the whole kernel, so an item's epilogue overlaps the next one's loads and first scores.
-// Bound: the key ring's round trip (a unit's release to its refill crosses both CTAs and L2, with 54 KB in flight); leaving out
-// the exponentials or either product's MMAs changed nothing.  So bytes in flight and few copies decide: blocks of 128 keys in
-// nine slabs of 8 KB, 52 copies of 2 KB each per block, took 458 us for 4 x 2048 rows of 16 heads where these took 430.  Now, with the
-// reference that moves at every new maximum, 421 us with L2 cold, the tensor pipe 53 % active (mma.sync kernel: 1940 us).
+// Bound: the products' reads of shared memory.  With both operands there, S of a block (36 instructions of 256 x 96 x 16) takes 3700
+// cycles of the block's 5000, where the tensor pipe needs 1730 for it: the 256 query rows of every instruction leave shared memory
+// at about 64 bytes a cycle.  (The same queries held in tensor memory: 2270 cycles; but they fill what a second score buffer and the
+// accumulators need, and two of nine slabs there, in turns with the scores, cost more in waits than they save, 498 -> 528 us.)  Rings of
+// three to six units take the same time; few copies matter: blocks of 128 keys in nine slabs of 8 KB, 52 copies of 2 KB each per
+// block, took 458 us for 4 x 2048 rows of 16 heads where these took 430.  Now, with the reference that moves at every new maximum, 421
+// us with L2 cold, the tensor pipe 53 % active (mma.sync kernel: 1940 us).
 #include "common.cuh"
 #include "runtime.h"
 #include "../../include/b200.h"
