@@ -19,7 +19,7 @@
 // of one address and one of many feed 16 packed FMAs, 64 cycles of either for the eight warps (4 x 8 tiles, two sets of keys or
 // rows to a warp: 96 of reads).
 // Gated linear attention, 5 ragged prompts of 6007 rows, 8 heads of 64 x 128: state 42, carry 12, output 67 us (with 4 x 8 tiles and
-// the weights pair by pair 44, 12, 85; one-pass, the layer 501 us, so 177).  State space, one prompt of 2048 rows, 32 heads of
+// the weights pair by pair 44, 12, 85; one-pass, the layer 501 us, so 171).  State space, one prompt of 2048 rows, 32 heads of
 // 128 x 64: 36, 14, 79 us (one-pass 191).  The copies behind the sums and the carry's whole lines are worth a tenth (measured over
 // linear attention's 4 x 2048 rows before it left: 62, 44, 104 us, without them 65, 62, 116).  Chunks of 64: with 32 the states double,
 // with 128 the chunk's own rows cost more FMAs than the states save.
