@@ -82,6 +82,7 @@ __device__ __forceinline__ void crp_pairs(const uint4& raw, f32x2 (&x)[2], float
 template <typename TA, int TAPS>
 __global__ void __launch_bounds__(kCapWarps * 32, sizeof(TA) == 4 ? 3 : 2)
 conv_rec_prep_vec_kernel(CrpArgs a, int lph, int rows) {
+  pdl_wait();
   constexpr int V = 16 / (int)sizeof(TA), P = V / 2, R = TAPS - 1;
   const CapWork m = cap_work(a, rows);
   if (m.n <= 0) return;
@@ -276,7 +277,7 @@ extern "C" int b200_conv_rec_prep(const void* proj, int f32, int64_t ld, const f
     const int all_warps = (a.n_heads + 32 / lph - 1) / (32 / lph), ny = (all_warps + kCapWarps - 1) / kCapWarps;
     const int warps = (all_warps + ny - 1) / ny;
     const dim3 grid(n_x, ny);
-#define B200_CRP(TA, N) conv_rec_prep_vec_kernel<TA, N><<<grid, warps * 32, 0, s>>>(a, lph, rows)
+#define B200_CRP(TA, N) (void)launch_pdl(conv_rec_prep_vec_kernel<TA, N>, dim3(grid), dim3(warps * 32), 0, s, 1, a, lph, rows)
 #define B200_CRPT(TA)                        \
   switch (taps) {                            \
     case 1: B200_CRP(TA, 1); break;          \

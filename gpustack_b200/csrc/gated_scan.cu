@@ -156,6 +156,7 @@ struct GsShape {
 template <int L, int R4, int C, bool DELTA>
 __global__ void __launch_bounds__((kGsWarps + kGsHelpers) * 32, C * R4 <= 8 ? 2 : 1)
 gated_scan_kernel(GatedScanArgs a) {
+  pdl_wait();
   extern __shared__ __align__(16) float smem[];
   using Sh = GsShape<L, R4, C>;
   constexpr int R2 = 2 * R4, DKP = Sh::DKP, CPW = Sh::CPW, BUFS = Sh::BUFS, VW = Sh::VW, BLOCKS = kGsHelpers, AHEAD = Sh::AHEAD;
@@ -472,6 +473,7 @@ gated_scan_kernel(GatedScanArgs a) {
 template <int L, int R4, bool DELTA>
 __global__ void __launch_bounds__(kGsStepWarps * 32, 4)
 gated_step_kernel(GatedScanArgs a) {
+  pdl_wait();
   constexpr int R2 = 2 * R4, CPW = 32 / L, COLS = kGsStepWarps * CPW;
   const int s = blockIdx.x, h = blockIdx.y, z = blockIdx.z;
   const int slot = a.state_slots[s];
@@ -525,14 +527,15 @@ int gated_scan_launch(const GatedScanArgs& a, int n_seqs, cudaStream_t s) {
       return B200_ERR_CUDA;
     }
   }
-  gated_scan_kernel<L, R4, C, DELTA><<<dim3(n_seqs, a.H, (a.dv + Sh::VW - 1) / Sh::VW), (kGsWarps + kGsHelpers) * 32, Sh::kBytes, s>>>(a);
+  (void)launch_pdl(gated_scan_kernel<L, R4, C, DELTA>, dim3(n_seqs, a.H, (a.dv + Sh::VW - 1) / Sh::VW), dim3((kGsWarps + kGsHelpers) * 32),
+                   Sh::kBytes, s, 1, a);
   return b200_check_launch("b200_gated_scan");
 }
 
 template <int L, int R4, bool DELTA>
 int gated_step_launch(const GatedScanArgs& a, int n_seqs, cudaStream_t s) {
   constexpr int COLS = kGsStepWarps * (32 / L);
-  gated_step_kernel<L, R4, DELTA><<<dim3(n_seqs, a.H, (a.dv + COLS - 1) / COLS), kGsStepWarps * 32, 0, s>>>(a);
+  (void)launch_pdl(gated_step_kernel<L, R4, DELTA>, dim3(n_seqs, a.H, (a.dv + COLS - 1) / COLS), dim3(kGsStepWarps * 32), 0, s, 1, a);
   return b200_check_launch("b200_gated_scan(step)");
 }
 
@@ -690,6 +693,7 @@ template <typename TA, bool VEC, bool AFTER>
 __global__ void __launch_bounds__(kGnThreads)
 gate_norm_kernel(const float* __restrict__ y, const TA* __restrict__ proj, int64_t ld, int z_col, const bf16* __restrict__ w,
                  TA* out, int64_t ldo, int C, int parts, float eps) {
+  pdl_wait();
   extern __shared__ __align__(16) float row[];        // [C], then the warps' partial sums
   __shared__ float sums[kGnThreads / 32];
   const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -755,6 +759,7 @@ template <typename TA, bool AFTER, int N>
 __global__ void __launch_bounds__(kGnThreads)
 gate_norm_heads_kernel(const float* __restrict__ y, const TA* __restrict__ proj, int64_t ld, int z_col, const bf16* __restrict__ w, TA* out,
                        int64_t ldo, int C, int W, float eps) {
+  pdl_wait();
   const int t = blockIdx.x, i0 = threadIdx.x * 4, step = kGnThreads * 4, lanes = W >> 2;
   const float over = 1.0f / (float)W;                  // (a power of two)
   const float* yr = y + (size_t)t * C;
@@ -803,6 +808,7 @@ template <typename TA, bool AFTER>
 __global__ void __launch_bounds__(kGnThreads)
 gate_norm_parts_kernel(const float* __restrict__ y, const TA* __restrict__ proj, int64_t ld, int z_col, const bf16* __restrict__ w, TA* out,
                        int64_t ldo, int C, int W, float eps) {
+  pdl_wait();
   constexpr int NW = kGnThreads / 32, N = 2;
   __shared__ float sums[N * NW];                       // of the row's groups of 128 channels
   const int t = blockIdx.x, i0 = threadIdx.x * 4, step = kGnThreads * 4, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, per = W / 128;
@@ -900,7 +906,9 @@ extern "C" int b200_gate_norm(const float* y, const void* proj, int f32, int64_t
   const bool vec = (C / parts) % 4 == 0 && ld % 4 == 0 && ldo % 4 == 0 && z_col % 4 == 0 && al(y, 16) && al(proj, n) && al(out, n) && al(w, 8);
   const int W = C / parts, lanes = W / 4;
   if (vec && lanes <= 32 && (lanes & (lanes - 1)) == 0 && C <= kGnThreads * 4 * 8) {
-#define B200_GNHN(TA, A, N) gate_norm_heads_kernel<TA, A, N><<<T, kGnThreads, 0, s>>>(y, (const TA*)proj, ld, z_col, (const bf16*)w, (TA*)out, ldo, C, W, eps)
+#define B200_GNHN(TA, A, N) \
+  (void)launch_pdl(gate_norm_heads_kernel<TA, A, N>, dim3(T), dim3(kGnThreads), 0, s, 1, y, (const TA*)proj, ld, z_col, (const bf16*)w, (TA*)out, \
+                   ldo, C, W, eps)
 #define B200_GNH(TA, A)                                            \
   do {                                                             \
     if (C <= 2 * kGnThreads * 4) B200_GNHN(TA, A, 2);              \
@@ -913,7 +921,9 @@ extern "C" int b200_gate_norm(const float* y, const void* proj, int f32, int64_t
     return b200_check_launch("b200_gate_norm");
   }
   if (vec && W % 128 == 0 && C <= kGnThreads * 8) {      // (two groups per thread; with four of 4096 channels 84 us where the staged row takes 71)
-#define B200_GNP(TA, A) gate_norm_parts_kernel<TA, A><<<T, kGnThreads, 0, s>>>(y, (const TA*)proj, ld, z_col, (const bf16*)w, (TA*)out, ldo, C, W, eps)
+#define B200_GNP(TA, A) \
+  (void)launch_pdl(gate_norm_parts_kernel<TA, A>, dim3(T), dim3(kGnThreads), 0, s, 1, y, (const TA*)proj, ld, z_col, (const bf16*)w, (TA*)out, ldo, \
+                   C, W, eps)
     if (f32) { if (gate_after) B200_GNP(float, true); else B200_GNP(float, false); }
     else { if (gate_after) B200_GNP(bf16, true); else B200_GNP(bf16, false); }
 #undef B200_GNP
@@ -921,7 +931,8 @@ extern "C" int b200_gate_norm(const float* y, const void* proj, int f32, int64_t
   }
   B200_REQUIRE(smem <= 48 * 1024, "gate_norm: %d channels exceed the staged row (12288)", C);
 #define B200_GN(TA, V, A) \
-  gate_norm_kernel<TA, V, A><<<T, kGnThreads, smem, s>>>(y, (const TA*)proj, ld, z_col, (const bf16*)w, (TA*)out, ldo, C, parts, eps)
+  (void)launch_pdl(gate_norm_kernel<TA, V, A>, dim3(T), dim3(kGnThreads), smem, s, 1, y, (const TA*)proj, ld, z_col, (const bf16*)w, (TA*)out, ldo, C, \
+                   parts, eps)
 #define B200_GN2(TA)                                                                                     \
   do {                                                                                                   \
     if (gate_after) { if (vec) B200_GN(TA, true, true); else B200_GN(TA, false, true); }                 \

@@ -28,6 +28,7 @@ template <typename TX, typename TY>
 __global__ void __launch_bounds__(256)
 gemm_simt_kernel(const TX* __restrict__ X, const bf16* __restrict__ W, const bf16* __restrict__ bias,
                  TY* __restrict__ Y, int M, int N, int K, int64_t ldx, int64_t ldw, int64_t ldy) {
+  pdl_wait();
   __shared__ __align__(16) float Xs[kSimtBK][kSimtBM + 4];
   __shared__ __align__(16) float Ws[kSimtBK][kSimtBN + 4];
   const int tid = threadIdx.x;
@@ -101,8 +102,7 @@ template <typename TX, typename TY>
 static int launch_simt(const void* X, const void* W, const void* bias, void* Y, int M, int N, int K, int64_t ldx,
                        int64_t ldw, int64_t ldy, cudaStream_t s) {
   dim3 grid((N + kSimtBN - 1) / kSimtBN, (M + kSimtBM - 1) / kSimtBM);
-  gemm_simt_kernel<TX, TY><<<grid, 256, 0, s>>>((const TX*)X, (const bf16*)W, (const bf16*)bias, (TY*)Y, M, N, K,
-                                                ldx, ldw, ldy);
+  (void)launch_pdl(gemm_simt_kernel<TX, TY>, grid, dim3(256), 0, s, 1, (const TX*)X, (const bf16*)W, (const bf16*)bias, (TY*)Y, M, N, K, ldx, ldw, ldy);
   return b200_check_launch("b200_linear_simt");
 }
 

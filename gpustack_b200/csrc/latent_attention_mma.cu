@@ -332,6 +332,7 @@ constexpr int kLdPitch = kLaKeys + 8;                  // floats per row of a pa
 template <int NT, bool TMA>   // n-tiles (8 columns) of the output per warp: R = 64 NT
 __global__ void __launch_bounds__(kLaWarps * 32, 2)
 latent_attn_step_kernel(const __grid_constant__ CUtensorMap rows_map, LaArgs a) {
+  pdl_wait();
   extern __shared__ __align__(16) uint8_t smem_raw[];
   __shared__ uint64_t full[kLdBufs];
   uint8_t* smem = TMA ? reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023)) : smem_raw;
@@ -550,6 +551,7 @@ latent_attn_step_kernel(const __grid_constant__ CUtensorMap rows_map, LaArgs a) 
 __global__ void __launch_bounds__(128)
 latent_attn_merge_kernel(const float* __restrict__ ws, const float* __restrict__ sink, bf16* out, int64_t ldo, int H,
                          int R, int nsplit) {
+  pdl_wait();
   const int b = blockIdx.x, h = blockIdx.y, lane = threadIdx.x & 31;
   const float* p = ws + ((size_t)b * H + h) * nsplit * (R + 2);
   float2 ml = make_float2(-INFINITY, 0.f);
@@ -627,7 +629,7 @@ static int ld_launch_form(const CUtensorMap& map, const LaArgs& a, dim3 grid, cu
     b200_set_error("latent_attn_decode: cudaFuncSetAttribute(smem=%zu): %s", smem, cudaGetErrorString(e));
     return B200_ERR_CUDA;
   }
-  latent_attn_step_kernel<NT, TMA><<<grid, kLaWarps * 32, smem, s>>>(map, a);
+  (void)launch_pdl(latent_attn_step_kernel<NT, TMA>, grid, dim3(kLaWarps * 32), smem, s, 1, map, a);
   return b200_check_launch("b200_latent_attn_decode");
 }
 
@@ -733,8 +735,8 @@ extern "C" int b200_latent_attn_decode(const void* qa, int64_t ldq, const void* 
   else rc = la_dispatch(a, grid, (cudaStream_t)stream);
   if (rc) return rc;
   if (nsplit > 1) {
-    latent_attn_merge_kernel<<<dim3(B, H), 128, 0, (cudaStream_t)stream>>>((const float*)workspace, sink, (bf16*)out, ldo, H, R,
-                                                                          nsplit);
+    (void)launch_pdl(latent_attn_merge_kernel, dim3(B, H), dim3(128), 0, (cudaStream_t)stream, 1, (const float*)workspace, sink, (bf16*)out,
+                     ldo, H, R, nsplit);
     return b200_check_launch("b200_latent_attn_decode(merge)");
   }
   return B200_OK;

@@ -158,6 +158,7 @@ constexpr int kRvThreads = 256;
 template <typename TA, typename TD, int TOK, bool SILU>
 __global__ void __launch_bounds__(kRvThreads, sizeof(TA) == 2 ? 5 : SILU ? 6 : 1)
 rot_prep_vec_kernel(RotPrepArgs a, int T, int lph, int items_q, int items_v, int v_half) {
+  pdl_wait_in_place();
   constexpr int VEC = 16 / (int)sizeof(TA);
   extern __shared__ float2 cs_all[];                  // [TOK][dims / 2] (cos, sin) of the tokens
   const int tok0 = blockIdx.x * TOK, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -291,6 +292,7 @@ rot_prep_vec_kernel(RotPrepArgs a, int T, int lph, int items_q, int items_v, int
 template <typename TA, typename TD, int ROWS>
 __global__ void __launch_bounds__(kRvThreads)
 rot_plain_kernel(RotPrepArgs a, int T) {
+  pdl_wait_in_place();
   constexpr int VEC = 16 / (int)sizeof(TA);
   const int t0 = blockIdx.y * ROWS, nq = a.H * a.dk, nk = a.G * a.dk;
   int c = (blockIdx.x * kRvThreads + threadIdx.x) * VEC;
@@ -389,8 +391,8 @@ extern "C" int b200_rot_prep_hm(const void* proj, int src_f32, int64_t ld, int q
       const bool four = (int64_t)T * nx >= 4 * 4 * 148 && T <= 65535 * 4;
 #define B200_RP(TA, TD)                                                                                          \
   do {                                                                                                           \
-    if (four) rot_plain_kernel<TA, TD, 4><<<dim3(nx, (T + 3) / 4), kRvThreads, 0, s>>>(a, T);                     \
-    else rot_plain_kernel<TA, TD, 1><<<dim3(nx, T), kRvThreads, 0, s>>>(a, T);                                    \
+    if (four) (void)launch_pdl(rot_plain_kernel<TA, TD, 4>, dim3(nx, (T + 3) / 4), dim3(kRvThreads), 0, s, 1, a, T); \
+    else (void)launch_pdl(rot_plain_kernel<TA, TD, 1>, dim3(nx, T), dim3(kRvThreads), 0, s, 1, a, T);             \
   } while (0)
       if (T <= 65535 || four) {
         if (src_f32) B200_RP(float, float);
@@ -410,7 +412,8 @@ extern "C" int b200_rot_prep_hm(const void* proj, int src_f32, int64_t ld, int q
       const size_t smem = (size_t)(dims / 2) * sizeof(float2);
       const bool four = !src_f32 && dims > 0 && T >= 4 * 8 * 148 && 4 * smem <= 40 * 1024;
 #define B200_RVS(TA, TD, TOK, S)                                                                                                  \
-  rot_prep_vec_kernel<TA, TD, TOK, S><<<(T + TOK - 1) / TOK, kRvThreads, TOK * smem, s>>>(a, T, lph, items_q, items_v, v_half)
+  (void)launch_pdl(rot_prep_vec_kernel<TA, TD, TOK, S>, dim3((unsigned)((T + TOK - 1) / TOK)), dim3(kRvThreads), TOK * smem, s, 1, a, T, lph, \
+                   items_q, items_v, v_half)
 #define B200_RV(TA, TD, TOK)                        \
   do {                                              \
     if (feature == 1) B200_RVS(TA, TD, TOK, true);  \
