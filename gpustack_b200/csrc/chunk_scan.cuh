@@ -19,7 +19,7 @@
 // of one address and one of many feed 16 packed FMAs, 64 cycles of either for the eight warps (4 x 8 tiles, two sets of keys or
 // rows to a warp: 96 of reads).
 // Gated linear attention, 5 ragged prompts of 6007 rows, 8 heads of 64 x 128: state 42, carry 12, output 67 us (with 4 x 8 tiles and
-// the weights pair by pair 44, 12, 85; one-pass, the layer 501 us, so 162).  State space, one prompt of 2048 rows, 32 heads of
+// the weights pair by pair 44, 12, 85; one-pass, the layer 501 us, so 155).  State space, one prompt of 2048 rows, 32 heads of
 // 128 x 64: 36, 14, 79 us (one-pass 191).  The copies behind the sums and the carry's whole lines are worth a tenth (measured over
 // linear attention's 4 x 2048 rows before it left: 62, 44, 104 us, without them 65, 62, 116).  Chunks of 64: with 32 the states double,
 // with 128 the chunk's own rows cost more FMAs than the states save.
@@ -209,7 +209,7 @@ struct ChunkSmem {
 // are weighted by 2^(F_n - F_s), the queries of the state's part by 2^F_t, and (k_s . q_t) is a sum of k q 2^(F_t - F_s) formed
 // term by term: 64 * 65 / 2 exponentials per channel, but none of a positive number, whatever the decays are.
 // The carry and the output begin while the launch before runs (programmatic launches): a carry's CTAs load their slots' states, an
-// output's their queries and keys, before they wait for it (gated linear attention of 6007 rows, the layer 171 -> 162 us; of 256 to
+// output's their queries and keys, before they wait for it (gated linear attention of 6007 rows, the layer 171 -> 162 us, with the states' own launch and those before it 155; of 256 to
 // 2048 rows 2 to 4 us less).
 __device__ __forceinline__ void cs_release_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void cs_wait_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -217,7 +217,7 @@ __device__ __forceinline__ void cs_wait_before() { asm volatile("griddepcontrol.
 template <int DK, int VT, typename Form>
 __global__ void __launch_bounds__(kCsThreads, 2)
 chunk_state_kernel(const ChunkScanArgs a, const typename Form::Params p) {
-  cs_release_next();
+  pdl_wait();
   extern __shared__ __align__(16) float smem[];
   __shared__ typename Form::Scratch scratch;
   __shared__ int shared5[5];
@@ -749,7 +749,7 @@ int cs_launch_shape(const ChunkScanArgs& a, const typename Form::Params& p, int6
     b200_set_error("chunk scan: %d bytes of shared memory: %s", ob, cudaGetErrorString(e));
     return B200_ERR_CUDA;
   }
-  chunk_state_kernel<DK, VT, Form><<<grid, kCsThreads, sb, s>>>(a, p);
+  (void)launch_pdl(chunk_state_kernel<DK, VT, Form>, grid, dim3(kCsThreads), (size_t)sb, s, 1, a, p);
   (void)launch_pdl(chunk_carry_kernel<DK, Form>, dim3(DK / kCsCarryKeys * ((a.dv + 127) / 128), a.H, a.n_seqs), dim3(kCsThreads), 0, s, 1, a, p);
   (void)launch_pdl(chunk_output_kernel<DK, VT, Form>, grid, dim3(kCsThreads), (size_t)ob, s, 1, a, p);
   return b200_check_launch(Form::kName);

@@ -46,6 +46,7 @@ gla_scan_kernel(const float* __restrict__ x, int64_t ld, int q_col, int k_col, i
                 int64_t ldz, float inv_tau, const int32_t* __restrict__ cu_seq, const int32_t* __restrict__ ctx_lens,
                 const int32_t* __restrict__ state_slots, float* S_state, float* __restrict__ o_raw, int H, int dk, int dv,
                 int most_rows) {
+  pdl_wait();
   extern __shared__ __align__(16) float smem[];
   constexpr int DKP = RPW * kGlWarps;                 // key rows, padded to the warps' shares
   float* qs = smem;                                   // [16][DKP]
@@ -196,6 +197,7 @@ __global__ void __launch_bounds__(kGlWarps * 32)
 gla_step_kernel(const float* __restrict__ x, int64_t ld, int q_col, int k_col, int v_col, const float* __restrict__ z,
                 int64_t ldz, float inv_tau, const int32_t* __restrict__ cu_seq, const int32_t* __restrict__ ctx_lens,
                 const int32_t* __restrict__ state_slots, float* S_state, float* __restrict__ o_raw, int H, int dk, int dv) {
+  pdl_wait();
   extern __shared__ float smem[];
   float* qs = smem;                                   // [16][dk]
   float* ks = qs + kGlTok * dk;                       // [16][dk]
@@ -302,8 +304,8 @@ static int launch_rows(const float* x, int64_t ld, int q_col, int k_col, int v_c
         attr = true;                                                                                                   \
       }                                                                                                                \
     }                                                                                                                  \
-    gla_scan_kernel<E><<<grid, kGlWarps * 32, smem, s>>>(x, ld, q_col, k_col, v_col, z, ldz, inv_tau, cu_seq, ctx_lens, \
-                                                         state_slots, S, o_raw, H, dk, dv, most_rows);                 \
+    (void)launch_pdl(gla_scan_kernel<E>, grid, dim3(kGlWarps * 32), smem, s, 1, x, ld, q_col, k_col, v_col, z, ldz,     \
+                     inv_tau, cu_seq, ctx_lens, state_slots, S, o_raw, H, dk, dv, most_rows);                          \
   } while (0)
   switch (rpw) {
     case 1: B200_GL(1); break;
@@ -328,7 +330,7 @@ extern "C" int b200_gla_scan_rows(const float* x, int64_t ld, int q_col, int k_c
   const size_t smem1 = sizeof(float) * (3 * (size_t)kGlTok * dk + kGlTok * kGlCols);
   if (max_len == 1 && smem1 <= 48 * 1024) {       // no sequence brings more than one row
 #define B200_GS(E)                                                                                                      \
-  gla_step_kernel<E><<<grid, kGlWarps * 32, smem1, s>>>(x, ld, q_col, k_col, v_col, z, ldz, inv_tau, cu_seq, ctx_lens, \
+  (void)launch_pdl(gla_step_kernel<E>, grid, dim3(kGlWarps * 32), smem1, s, 1, x, ld, q_col, k_col, v_col, z, ldz, inv_tau, cu_seq, ctx_lens, \
                                                         state_slots, S, o_raw, H, dk, dv)
     if (dk <= 32) B200_GS(1);
     else if (dk <= 64) B200_GS(2);
