@@ -206,11 +206,12 @@ struct ChunkSmem {
 // finish() for chunk_output, `Carry` (the chunks' decays) for chunk_carry.
 // A Form with kVector has one decay per KEY CHANNEL instead: with the running sums F of a chunk's base-2 logarithms per channel
 // (summed in fp64, kept as two fp32 parts, so that a difference is as exact as an fp32 product of decays) the keys of the state
-// are weighted by 2^(F_n - F_s), the queries of the state's part by 2^F_t, and (k_s . q_t) is a sum of k q 2^(F_t - F_s) formed
-// term by term: 64 * 65 / 2 exponentials per channel, but none of a positive number, whatever the decays are.
+// are weighted by 2^(F_n - F_s), the queries of the state's part by 2^F_t, and (k_s . q_t) is a sum of k q 2^(F_t - F_s), whose
+// exponents cs_vector_weights forms in parts: none of a positive number, whatever the decays are.
 // The carry and the output begin while the launch before runs (programmatic launches): a carry's CTAs load their slots' states, an
-// output's their queries and keys, before they wait for it (gated linear attention of 6007 rows, the layer 171 -> 162 us, with the states' own launch and those before it 155; of 256 to
-// 2048 rows 2 to 4 us less).
+// output's their queries and keys, before they wait for it (gated linear attention of 6007 rows, the layer 171 -> 162 us, with the
+// states' own launch and those before it 155; of 256 to 2048 rows 2 to 4 us less).  Every CTA of chunk_state waits first and only then
+// lets a carry start, so that one whose CTAs have nothing to do still comes after the one-pass kernel before the chunks.
 __device__ __forceinline__ void cs_release_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void cs_wait_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
