@@ -375,6 +375,7 @@ gated_scan_kernel(GatedScanArgs a) {
     for (int st = AHEAD - BUFS; st < stages + AHEAD; ++st) {
       if (st >= 0 && st < stages) factors(st);
       if (st >= AHEAD) put(st - AHEAD);
+      __syncwarp();                                   // a lane copies columns that others read in put(), each in as many turns as it has columns
       if (st - AHEAD + BUFS < stages) stage(st - AHEAD + BUFS);
       asm volatile("cp.async.commit_group;" ::: "memory");
     }

@@ -51,3 +51,12 @@ def test_chunk_weights_are_read_before_their_buffer_is_free():
     converting = kernel[kernel.index("if (warp < kCtConvWarps)"):kernel.index("else if (warp < kCtConvWarps + kCtReadWarps)")]
     before, behind = converting.split("ct_stored(&half_full[e]);")
     assert re.search(r"\bsc\.w\[", before) and not re.search(r"\b(sc|scratch)\b", behind)
+
+
+def test_rows_are_copied_once_every_lane_has_read_the_ones_before():
+    """A helper warp's lanes read a block's values in turns of their own number and copy the next rows over them, other lanes' columns
+    too: the warp meets in between."""
+    kernel = next(d for d in _definitions((CSRC / "gated_scan.cu").read_text()) if "\ngated_scan_kernel(" in d)
+    read, copy = kernel.index("put(st - AHEAD);"), kernel.index("stage(st - AHEAD + BUFS);")
+    between = kernel[read:copy]
+    assert read < copy and "__syncwarp();" in between and between.index("__syncwarp();") < between.index("if (")
