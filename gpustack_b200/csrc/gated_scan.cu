@@ -16,10 +16,10 @@
 //   u_j = beta_j v_j - beta_j G_j S^T k_j - sum_(i < j) beta_j D_ij (k_i . k_j) u_i       (state space: beta_j v_j)
 //   o_j = G_j S^T q_j + sum_(i <= j) D_ij (k_i . q_j) u_i,      S <- G_3 S + sum_i D_i3 k_i u_i^T
 // so S^T k and S^T q of all four tokens come from the state before the block: their sums over the lanes travel together, and the
-// state is scaled once for four tokens.  Token by token, as this was, each token waits for a sum over the lanes: 680 us for the delta
-// rule over 4 x 2048 rows of 16 heads of 128 x 128 where blocks take 467 (fp32 pipe some 55 % busy), 453 -> 343 for the state space of
-// 32 heads of 128 x 64.  Errors against 64 bits are no larger (delta rule 4 x 600 rows: outputs 1.23e-7 -> 1.17e-7, states 1.61e-7 -> 1.50e-7;
-// state space 1.38e-7 -> 1.35e-7, 1.61e-7 -> 1.49e-7; rows of one sign 5.86e-8 -> 5.86e-8 and 1.43e-7 -> 1.45e-7, states 6 % less).
+// state is scaled once for four tokens.  Token by token, as this was, each token waits for a sum over the lanes: 676 us for the delta
+// rule over 4 x 2048 rows of 16 heads of 128 x 128 where blocks take 469 (fp32 pipe some 55 % busy), 450 -> 335 for the state space of
+// 32 heads of 128 x 64.  Errors against 64 bits are no larger (delta rule 4 x 600 rows: outputs 1.23e-7 -> 1.16e-7, states 1.61e-7 -> 1.51e-7;
+// state space 1.38e-7 -> 1.35e-7, 1.61e-7 -> 1.50e-7; rows of one sign 5.86e-8 -> 5.85e-8 and 1.43e-7 -> 1.42e-7, states 7 % less).
 // What bounds it is one warp's issue: the products of a token go column by column in turn so that four chains cover an FMA's latency,
 // and a token's sum over the lanes goes on a level per product that follows.  Of no use: eight warps of half the columns each (+6 %),
 // key rows held over the block instead of read twice, queries a block ahead (+10 %, registers).
@@ -134,12 +134,15 @@ constexpr int kGsSms = 148;
 constexpr int kGsTile = 4;                             // tokens of a block
 constexpr int kGsHelpers = 4;                          // warps that stage rows and form the factors of a block each: blocks of a stage
 constexpr int kGsStage = kGsHelpers * kGsTile;
-// A block's factors in shared memory, floats: beta_j | D_03 D_13 D_23 G_3 | G_j | what rounding left of G_j | D_ij k_i.k_j (i < j) |
-// D_ij k_i.q_j (row j, i <= j).  An error of theirs is one of every column and entry, which nothing averages out: decays and the last sums of
-// the products are formed in 64 bits and rounded once, and an output's last sum takes along what its rounding leaves (fp32 throughout:
-// outputs 3 to 8 % further off than token by token, 19 % over rows of one sign; all of it in 64 bits: the walk waits for it, 328 -> 379 us
-// for the state space of 4 x 2048 rows).
-constexpr int kGsBeta = 0, kGsD3 = 4, kGsG = 8, kGsGl = 12, kGsA = 16, kGsB = 24, kGsFactors = 40;
+// A block's factors in shared memory, floats: beta_j | D_j3 | G_j | what rounding left of G_j | D_ij k_i.k_j (i < j) | D_ij k_i.q_j (row j,
+// i <= j) | the state's factor | c - 1 behind the block.  An error of theirs is one of every column and entry, which nothing averages
+// out: decays and the last sums of the products are formed in 64 bits and rounded once, and an output's last sum takes along what its
+// rounding leaves (fp32 throughout: outputs 3 to 8 % further off than token by token, 19 % over rows of one sign; all of it in 64 bits: the
+// walk waits for it, 328 -> 379 us for the state space of 4 x 2048 rows).  The state is scaled by G_3 rounded to fp32.  What that
+// leaves would be an error of all its entries alike, and one of decays that do not change adds up (a state left alone for 2048 tokens: 1e-5
+// off, token by token 1e-6).  So the state is held as itself over a number c close to 1: the helpers, which know what was left,
+// keep c, G_j is times c, D_j3 over it, and the walk multiplies by c at its end.  Multiplied by both parts of G_3 instead: the walk 468 -> 496 us.
+constexpr int kGsBeta = 0, kGsD3 = 4, kGsG = 8, kGsGl = 12, kGsA = 16, kGsB = 24, kGsScale = 40, kGsRest = 41, kGsFactors = 44;
 
 template <int L, int R4, int C>
 struct GsShape {
@@ -230,8 +233,8 @@ gated_scan_kernel(GatedScanArgs a) {
       }
     };
     float ra = 0.f, rb = 0.f;
-    auto raw_gates = [&](int st) {
-      const int t = (st * BLOCKS + helper) * kGsTile + j;
+    auto raw_gates = [&](int st) {                    // lane n: token n of the stage
+      const int t = st * kGsStage + n;
       if (t < rows) {
         const float* g = a.gates + (size_t)(t0 + t) * a.ld_g;
         ra = DELTA ? g[a.H + h] : g[h];
@@ -284,19 +287,35 @@ gated_scan_kernel(GatedScanArgs a) {
             }
           }
           y = fmaf(skip, v[i * VW], y);
-          const float R = r[0][i] + r[1][i], left = gs_left(r[0][i], r[1][i], R), P = G[i] * R, sum = P + y;
-          low += gs_left(P, y, sum) + fmaf(Gl[i], R, fmaf(G[i], left, fmaf(G[i], R, -P)));
-          y = fabsf(sum) < INFINITY ? sum + low : sum;
+          const float R = r[0][i] + r[1][i], left = gs_left(r[0][i], r[1][i], R);
+          if (DELTA) {
+            const float P = G[i] * R, sum = P + y;
+            low += gs_left(P, y, sum) + fmaf(Gl[i], R, fmaf(G[i], left, fmaf(G[i], R, -P)));
+            y = fabsf(sum) < INFINITY ? sum + low : sum;
+          } else {                                     // (a third of the instructions, and as close where the steps are not the state's)
+            y = fmaf(G[i], R, fabsf(R) < INFINITY ? fmaf(Gl[i], R, fmaf(G[i], left, y)) : y);
+          }
           if (b * kGsTile + i < rows) out[(size_t)i * a.H * a.dv] = y;
         }
       }
     };
+    double carry = 0.0;                               // c - 1 before the stage
     auto factors = [&](int st) {
-      const int b = st * BLOCKS + helper, at = st % BUFS * BLOCKS + helper;
-      const float2 gb = b * kGsTile + j < rows ? gs_gate<DELTA>(ra, rb, rate, bias) : make_float2(1.f, 0.f);   // (behind the portion the state stays)
+      const int at = st % BUFS * BLOCKS + helper, from = helper * kGsTile;
+      const float2 gb = st * kGsStage + n < rows ? gs_gate<DELTA>(ra, rb, rate, bias) : make_float2(1.f, 0.f);   // (behind the portion the state stays)
       if (st + 1 < stages) raw_gates(st + 1);
-      const float g0 = __shfl_sync(0xffffffffu, gb.x, 0), g1 = __shfl_sync(0xffffffffu, gb.x, 1), g2 = __shfl_sync(0xffffffffu, gb.x, 2),
-                  g3 = __shfl_sync(0xffffffffu, gb.x, 3);
+      // lane n: the product of the four decays of its block of the stage, rounded, and what that leaves, over the product
+      float g = __shfl_xor_sync(0xffffffffu, gb.x, 1), scale = gb.x * g, rest = fmaf(gb.x, g, -scale);
+      g = __shfl_xor_sync(0xffffffffu, scale, 2);
+      rest = fmaf(scale, __shfl_xor_sync(0xffffffffu, rest, 2), rest * g);
+      rest += fmaf(scale, g, -scale * g);
+      scale *= g;
+      rest = scale > 1e-30f && scale < 1e30f ? rest * rcp_approx(scale) : 0.f;
+      const float beside = __shfl_xor_sync(0xffffffffu, rest, 4), pair = rest + beside, others = __shfl_xor_sync(0xffffffffu, pair, 8);
+      const float c = (float)carry + ((n & 4 ? beside : 0.f) + (n & 8 ? others : 0.f)), behind = c + fmaf(c, rest, rest);      // - 1
+      carry = fma(carry, (double)(pair + others), carry + (double)(pair + others));
+      const float g0 = __shfl_sync(0xffffffffu, gb.x, from), g1 = __shfl_sync(0xffffffffu, gb.x, from + 1),
+                  g2 = __shfl_sync(0xffffffffu, gb.x, from + 2), g3 = __shfl_sync(0xffffffffu, gb.x, from + 3);
       double decay = 1.0;                             // from token lo to token hi
       if (lo < 1 && hi >= 1) decay = g1;
       if (lo < 2 && hi >= 2) decay *= g2;
@@ -352,26 +371,32 @@ gated_scan_kernel(GatedScanArgs a) {
       float* f = fs + at * kGsFactors;
       if (lane < 16) {
         f[upper ? kGsA + hi * (hi - 1) / 2 + lo : kGsB + n] = (float)(decay * sum[0]);
-      } else if (lane < 20) {
+      } else if (n >> 2 == helper) {
         double G = g0, D3 = 1.0;
-        if (n >= 1) G *= g1;
-        if (n >= 2) G *= g2;
-        if (n >= 3) G *= g3;
-        if (n < 1) D3 = g1;
-        if (n < 2) D3 *= g2;
-        if (n < 3) D3 *= g3;
+        if (j >= 1) G *= g1;
+        if (j >= 2) G *= g2;
+        if (j >= 3) G *= g3;
+        if (j < 1) D3 = g1;
+        if (j < 2) D3 *= g2;
+        if (j < 3) D3 *= g3;
+        G = fma(G, (double)c, G);
+        D3 = fma(D3, (double)(behind * fmaf(behind, 1.f - behind, -1.f)), D3);      // over 1 + behind
         const float high = (float)G;
-        f[kGsBeta + n] = gb.y;
-        f[kGsG + n] = high;
-        f[kGsGl + n] = (float)(G - high);
-        f[kGsD3 + n] = n == 3 ? high : (float)D3;
+        f[kGsBeta + j] = gb.y;
+        f[kGsG + j] = high;
+        f[kGsGl + j] = (float)(G - high);
+        f[kGsD3 + j] = (float)D3;
+        if (j == 0) {
+          f[kGsScale] = scale;
+          f[kGsRest] = behind;
+        }
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&factors_full[st % BUFS]);
     };
     raw_gates(0);
     // a stage's factors, the outputs of the one AHEAD before it, then the rows of the next one for its buffer: none of the walk's
-    // stages waits for outputs or copies.  A warp copies, reads and writes out its own block only.
+    // stages waits for copies, or for the outputs of less than AHEAD + 1 stages before.  A warp copies, reads and writes out its own block only.
     for (int st = AHEAD - BUFS; st < stages + AHEAD; ++st) {
       if (st >= 0 && st < stages) factors(st);
       if (st >= AHEAD) put(st - AHEAD);
@@ -391,7 +416,7 @@ gated_scan_kernel(GatedScanArgs a) {
     const float* vr = vs + at * kGsTile * VW + mine;
     const float* f = fs + at * kGsFactors;
     float* ob = os + b % ((AHEAD + 1) * BLOCKS) * VW * Sh::OUT;
-    if ((b + 1) % BLOCKS == 0 && b + 1 < blocks) {
+    if ((b + 1) % BLOCKS == 0 && b + 1 < blocks) {    // the next stage's, a block early: at its own start 474 us of 469, delta rule of 4 x 2048 rows
       const int st = (b + 1) / BLOCKS;
       mbar_wait_guarded(&factors_full[st % BUFS], (st / BUFS) & 1);
     }
@@ -399,8 +424,7 @@ gated_scan_kernel(GatedScanArgs a) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) v[j] = vr[j * VW];
     const float4 beta = *reinterpret_cast<const float4*>(f + kGsBeta), d3 = *reinterpret_cast<const float4*>(f + kGsD3);
-    // S^T k of the block's tokens, then S^T q; a token's sum over the lanes goes on a level for each product that follows.  A row's
-    // successor in the next block is on its way as soon as the row is used (behind the last block: read, not used).
+    // S^T k of the block's tokens, then S^T q; a token's sum over the lanes goes on a level for each product that follows
     constexpr int FIRST = DELTA ? 0 : 4;
 #pragma unroll
     for (int t = FIRST; t < 8 || (DELTA && t < 4 + LV); ++t) {
@@ -418,7 +442,8 @@ gated_scan_kernel(GatedScanArgs a) {
           if (t - 1 - lv >= 0 && t - 1 - lv < 4) gs_level<C>(p, t - 1 - lv, lv);
       }
     }
-    const f32x2 g4 = pack2(d3.w, d3.w);
+    const float scale = f[kGsScale];
+    const f32x2 g4 = pack2(scale, scale);
 #pragma unroll
     for (int c = 0; c < C; ++c)
 #pragma unroll
@@ -438,7 +463,7 @@ gated_scan_kernel(GatedScanArgs a) {
       u[2] = beta.z * v[2];
       u[3] = beta.w * v[3];
     }
-    const float w[4] = {d3.x * u[0], d3.y * u[1], d3.z * u[2], u[3]};
+    const float w[4] = {d3.x * u[0], d3.y * u[1], d3.z * u[2], d3.w * u[3]};
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       f32x2 k[R2];
@@ -462,6 +487,14 @@ gated_scan_kernel(GatedScanArgs a) {
       if (lane == 0) mbar_arrive(&empty[b / BLOCKS % BUFS]);
     }
   }
+  const float rest = fs[(blocks - 1) % (BUFS * BLOCKS) * kGsFactors + kGsRest];
+#pragma unroll
+  for (int c = 0; c < C; ++c)
+#pragma unroll
+    for (int i = 0; i < R2; ++i) {
+      const float2 v = unpack2(S[c][i]);
+      S[c][i] = pack2(fabsf(v.x) < INFINITY ? fmaf(v.x, rest, v.x) : v.x, fabsf(v.y) < INFINITY ? fmaf(v.y, rest, v.y) : v.y);
+    }
 #pragma unroll
   for (int c = 0; c < C; ++c)
 #pragma unroll

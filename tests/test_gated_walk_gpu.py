@@ -93,3 +93,30 @@ def test_what_is_no_number_stays_behind_its_row(row, delta):
     out = _scan(bad, gates, rate, bias, None, lens, [5], S, H, G, dk, dv, delta)
     assert torch.equal(out[:row], clean[:row])
     assert bool(torch.isnan(out[row:]).all()) and bool(torch.isnan(S).all())
+
+
+@pytest.mark.parametrize("H,G,dk,dv", [(16, 16, 120, 64), (16, 16, 24, 16), (16, 8, 60, 32), (4, 4, 256, 16)])   # (128 and 64 keys: chunks)
+@pytest.mark.parametrize("delta", [True, False])
+def test_a_state_left_alone_decays_as_exactly_as_its_entries_are_rounded(H, G, dk, dv, delta):
+    """Keys of zero: after T tokens the state is its start times the decay to the power of T, whatever four decays' product rounds to."""
+    T, n = 2048, 2
+    x, q, k, v, gates, S, rate, bias = _inputs([T] * n, H, G, dk, dv, 8)
+    x[:, G * dk:2 * G * dk] = 0
+    gates[:] = torch.randn(2 * H, generator=torch.Generator().manual_seed(5)).cuda()
+    bias -= 4.0                                         # a state keeps a fifth of itself or more over the rows
+    one = torch.ones(1, H, dv, dk, device="cuda")       # the decays as the kernels form them
+    zero, skip = torch.zeros(1, x.shape[1], device="cuda"), torch.zeros(H, device="cuda")
+    from gpustack_b200 import ops
+    ops.gated_scan(zero, 0, G * dk, 2 * G * dk, gates[:1] if delta else gates[:1, :H].contiguous(), rate, bias, skip, _i32([0, 1]), _i32([1]), _i32([0]),
+                   one, torch.empty(1, H * dv, device="cuda"), H, G, dk, dv, delta, max_len=1)
+    g, S0 = one[0, :, 0, 0].to(F64), S.to(F64)
+    out = _scan(x, gates, rate, bias, None, [T] * n, [9] * n, S, H, G, dk, dv, delta)
+    want = S0 * (g ** T)[:, None, None]
+    rows = torch.arange(T - 64, T, device="cuda", dtype=F64) + 1
+    Q = q.to(F64).repeat_interleave(H // G, 1).view(n, T, H, dk)[:, -64:]
+    read = torch.einsum("nthk,nhvk->nthv", Q, S0.flip(0)) * (g ** rows[:, None])[..., None]
+    out = out.view(n, T, H, dv)[:, -64:].to(F64)
+    for h in range(H):
+        # T / 4 roundings of every entry by itself, 0.29 units of 2^-23 each and independent of one another: 8e-7; three times that
+        assert float((S[:, h].to(F64) - want[:, h]).norm() / want[:, h].norm()) < 2.4e-6, h
+        assert float((out[:, :, h] - read[:, :, h]).norm() / read[:, :, h].norm()) < 2.4e-6, h
