@@ -211,8 +211,11 @@ gated_scan_kernel(GatedScanArgs a) {
 
   if (warp >= kGsWarps) {
     // ------------------------------------------------------------------ staging, and a block's factors per warp and stage
-    const int helper = warp - kGsWarps, n = lane & 15, j = n & 3, lo = min(n >> 2, j), hi = max(n >> 2, j);
-    const bool upper = j > n >> 2;                    // lane n: the pair (row n / 4, column n % 4); above the diagonal keys with keys
+    const int helper = warp - kGsWarps, n = lane & 15, j = n & 3;
+    // the lane's pair of rows (above the diagonal keys with keys): place n of a 4 x 4 table, of few keys place lane / 2
+    constexpr bool FEW = DKP <= 32;
+    const int pair_row = FEW ? lane >> 3 : n >> 2, pair_col = FEW ? lane >> 1 & 3 : j, lo = min(pair_row, pair_col), hi = max(pair_row, pair_col);
+    const bool upper = pair_col > pair_row;
     const int hk = h / (a.H / a.G), v4 = min(VW, a.dvp - col0) >> 2;
     const float rate = a.rate[h], bias = a.dt_bias[h];
     const float* x = a.x + (size_t)t0 * a.ld + lane * 4;
@@ -322,56 +325,80 @@ gated_scan_kernel(GatedScanArgs a) {
       if (lo < 3 && hi >= 3) decay *= g3;
       asm volatile("cp.async.wait_group %0;" ::"n"(BUFS - AHEAD - 1) : "memory");
       __syncwarp();
-      float dot[16];
-      {
-        f32x2 d2[16];
+      double product;
+      const float* kb = ks + at * kGsTile * DKP;
+      const float* qb = qs + at * kGsTile * DKP;
+      if constexpr (FEW) {                             // eight lanes per row, each four keys of its products (lanes without keys: 202 -> 191 us, 16 keys)
+        float dot[4] = {0.f, 0.f, 0.f, 0.f};
+        const int d = (lane & 7) * 4;
+        if (d < DKP) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) d2[i] = 0;
-        const float* kb = ks + at * kGsTile * DKP;
-        const float* qb = qs + at * kGsTile * DKP;
+          for (int c = 0; c < 4; ++c) {
+            const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(kb + c * DKP + d),
+                             x = *reinterpret_cast<const ulonglong2*>((DELTA && c > pair_row ? kb : qb) + pair_row * DKP + d);
+            dot[c] = sum2(fma2(k.y, x.y, mul2(k.x, x.x)));
+          }
+        }
+        const bool up = lane & 4;
+        double sum[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const float own = up ? dot[i + 2] : dot[i], other = up ? dot[i] : dot[i + 2];
+          sum[i] = own + __shfl_xor_sync(0xffffffffu, other, 4);
+        }
+        const double own = lane & 2 ? sum[1] : sum[0], other = lane & 2 ? sum[0] : sum[1];
+        product = own + __shfl_xor_sync(0xffffffffu, other, 2);
+        product += __shfl_xor_sync(0xffffffffu, product, 1);
+      } else {
+        float dot[16];
+        {
+          f32x2 d2[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) d2[i] = 0;
 #pragma unroll 1
-        for (int d = lane * 4; d < DKP; d += 128) {
-          ulonglong2 k[4], q[4];
+          for (int d = lane * 4; d < DKP; d += 128) {
+            ulonglong2 k[4], q[4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            k[i] = *reinterpret_cast<const ulonglong2*>(kb + i * DKP + d);
-            q[i] = *reinterpret_cast<const ulonglong2*>(qb + i * DKP + d);
+            for (int i = 0; i < 4; ++i) {
+              k[i] = *reinterpret_cast<const ulonglong2*>(kb + i * DKP + d);
+              q[i] = *reinterpret_cast<const ulonglong2*>(qb + i * DKP + d);
+            }
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+              for (int c = 0; c < 4; ++c) {
+                if (c <= r) d2[r * 4 + c] = fma2(k[c].y, q[r].y, fma2(k[c].x, q[r].x, d2[r * 4 + c]));
+                else if (DELTA) d2[r * 4 + c] = fma2(k[c].y, k[r].y, fma2(k[c].x, k[r].x, d2[r * 4 + c]));
+              }
           }
 #pragma unroll
-          for (int r = 0; r < 4; ++r)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              if (c <= r) d2[r * 4 + c] = fma2(k[c].y, q[r].y, fma2(k[c].x, q[r].x, d2[r * 4 + c]));
-              else if (DELTA) d2[r * 4 + c] = fma2(k[c].y, k[r].y, fma2(k[c].x, k[r].x, d2[r * 4 + c]));
-            }
+          for (int i = 0; i < 16; ++i) dot[i] = sum2(d2[i]);
         }
 #pragma unroll
-        for (int i = 0; i < 16; ++i) dot[i] = sum2(d2[i]);
-      }
+        for (int w = 8; w > 2; w >>= 1) {                // lanes n and n + 16 end with pair n
+          const bool up = n & w;
 #pragma unroll
-      for (int w = 8; w > 2; w >>= 1) {                // lanes n and n + 16 end with pair n
-        const bool up = n & w;
-#pragma unroll
-        for (int i = 0; i < w; ++i) {
-          const float own = up ? dot[i + w] : dot[i], other = up ? dot[i] : dot[i + w];
-          dot[i] = own + __shfl_xor_sync(0xffffffffu, other, w);
+          for (int i = 0; i < w; ++i) {
+            const float own = up ? dot[i + w] : dot[i], other = up ? dot[i] : dot[i + w];
+            dot[i] = own + __shfl_xor_sync(0xffffffffu, other, w);
+          }
         }
-      }
-      double sum[4] = {dot[0], dot[1], dot[2], dot[3]};
+        double sum[4] = {dot[0], dot[1], dot[2], dot[3]};
 #pragma unroll
-      for (int w = 2; w > 0; w >>= 1) {
-        const bool up = n & w;
+        for (int w = 2; w > 0; w >>= 1) {
+          const bool up = n & w;
 #pragma unroll
-        for (int i = 0; i < w; ++i) {
-          const double own = up ? sum[i + w] : sum[i], other = up ? sum[i] : sum[i + w];
-          sum[i] = own + __shfl_xor_sync(0xffffffffu, other, w);
+          for (int i = 0; i < w; ++i) {
+            const double own = up ? sum[i + w] : sum[i], other = up ? sum[i] : sum[i + w];
+            sum[i] = own + __shfl_xor_sync(0xffffffffu, other, w);
+          }
         }
+        sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], 16);
+        product = sum[0];
       }
-      sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], 16);
       float* f = fs + at * kGsFactors;
-      if (lane < 16) {
-        f[upper ? kGsA + hi * (hi - 1) / 2 + lo : kGsB + n] = (float)(decay * sum[0]);
-      } else if (n >> 2 == helper) {
+      if (FEW ? !(lane & 1) : lane < 16) f[upper ? kGsA + hi * (hi - 1) / 2 + lo : kGsB + 4 * pair_row + pair_col] = (float)(decay * product);
+      if (lane >= 16 && n >> 2 == helper) {
         double G = g0, D3 = 1.0;
         if (j >= 1) G *= g1;
         if (j >= 2) G *= g2;
@@ -579,9 +606,12 @@ int gated_step_launch(const GatedScanArgs& a, int n_seqs, cudaStream_t s) {
 // of 16 columns 283, 225, 348, 860.  CTAs of 32 columns share an SM in pairs, which covers the start and the end of short portions: 16
 // of 16 rows 34.5 in CTAs of 64 columns, 31.0 of 32, but 8 of 1024 rows 476 and 551.  A bound on the rows per portion is often that of all
 // of them, so pairs are for sequences enough to fill the GPU three times (16 of 512 rows: 480 either way) or a bound that is short.
-template <int L, int R4>
+// Few keys: a lane of two columns walks faster than one of four, whose sums over lanes and columns take longer than its products.  State
+// space of 32 heads of 64 values, us token by token, in four columns a lane, in two: 16 keys, one sequence of 2048 rows 203, 221, 192, 64 of 33
+// rows 59, 55, 49; 32 keys 205, 187, 152 and 59, 55, 86: of 17 to 32 keys two only where CTAs of 32 columns find an SM each.
+template <int L, int R4, int C = 4>
 bool gs_fits(const GatedScanArgs& a, int n_seqs) {
-  constexpr int cols = GsShape<L, R4, 4>::VW;
+  constexpr int cols = GsShape<L, R4, C>::VW;
   return (int64_t)n_seqs * a.H * ((a.dv + cols - 1) / cols) <= kGsSms;
 }
 template <bool DELTA>
@@ -594,8 +624,8 @@ int gated_scan_pick(const GatedScanArgs& a, int n_seqs, int max_len, cudaStream_
     if (a.dkp <= 256) return gated_step_launch<16, 4, DELTA>(a, n_seqs, s);
     return gated_step_launch<32, 4, DELTA>(a, n_seqs, s);
   }
-  if (a.dkp <= 16) return gated_scan_launch<4, 1, 4, DELTA>(a, n_seqs, s);
-  if (a.dkp <= 32) return gated_scan_launch<8, 1, 4, DELTA>(a, n_seqs, s);
+  if (a.dkp <= 16) return gated_scan_launch<4, 1, 2, DELTA>(a, n_seqs, s);
+  if (a.dkp <= 32) return gs_fits<8, 1, 2>(a, n_seqs) ? gated_scan_launch<8, 1, 2, DELTA>(a, n_seqs, s) : gated_scan_launch<8, 1, 4, DELTA>(a, n_seqs, s);
   if (a.dkp <= 64) return gs_fits<16, 1>(a, n_seqs) ? gated_scan_launch<16, 1, 4, DELTA>(a, n_seqs, s) : gated_scan_launch<8, 2, 4, DELTA>(a, n_seqs, s);
   if (a.dkp <= 96) return gated_scan_launch<8, 3, 4, DELTA>(a, n_seqs, s);
   if (a.dkp <= 128) {

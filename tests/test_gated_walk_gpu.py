@@ -64,7 +64,8 @@ def _rel(a, b):
 # heads and copies of the portions so that each of the widths that a number of CTAs chooses runs: (16, 64), (32, 128), (32, 256)
 @pytest.mark.parametrize("H,G,dk,dv,copies", [(2, 1, 14, 17, 1), (2, 2, 32, 64, 1), (2, 1, 64, 33, 1), (4, 2, 52, 64, 6), (2, 1, 90, 70, 1),
                                               (1, 1, 128, 64, 1), (4, 2, 128, 60, 1), (8, 4, 124, 64, 2), (8, 4, 128, 128, 2), (1, 1, 256, 20, 1),
-                                              (4, 4, 200, 128, 2), (1, 1, 400, 40, 1), (2, 1, 24, 33, 1), (2, 1, 12, 101, 1)])
+                                              (4, 4, 200, 128, 2), (1, 1, 400, 40, 1), (2, 1, 24, 33, 1), (2, 1, 12, 101, 1),
+                                              (8, 4, 30, 64, 1)])
 @pytest.mark.parametrize("delta", [True, False])
 def test_blocks_of_four(H, G, dk, dv, copies, delta):
     lens = LENS * copies
