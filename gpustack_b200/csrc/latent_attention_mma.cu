@@ -316,7 +316,7 @@ constexpr int kLdHalf = 16, kLdBufs = 5, kLdMaxW = 576, kLdSteps = kLdMaxW / 16 
 // the largest of a warp's values, in one instruction
 __device__ __forceinline__ float warp_max_redux(float v) {
   float r;
-  asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));      // (every lane takes part: it stays where it is)
   return r;
 }
 // a page's 16 rows of all slabs

@@ -19,6 +19,15 @@ def test_bulk_copies_go_to_one_cta(path):
     assert not [i for i in _instructions(path.read_text()) if "multi" + "cast" in i]
 
 
+@pytest.mark.parametrize("path", SOURCES, ids=lambda p: p.name)
+def test_instructions_of_whole_warps_stay_in_place(path):
+    """An instruction that waits for other lanes is volatile: the compiler neither moves it into a branch nor makes two of it."""
+    text = path.read_text()
+    for m in re.finditer(r"\basm\b(?P<v>\s*volatile\b)?\s*\((?P<code>(?:\s*\"[^\"]*\")+)", text):
+        if re.search(r"\.sync\b", m["code"]):
+            assert m["v"], m["code"]
+
+
 def _definitions(text):
     """The source cut at every definition that begins a line."""
     return re.split(r"\n(?=template |__global__|__device__|static |extern )", text)
