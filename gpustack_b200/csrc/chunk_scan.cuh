@@ -331,7 +331,7 @@ chunk_carry_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   const bool fresh = a.ctx_lens[s] == 0;
   for (int i = tid; i < 128 * kCsCarryKeys; i += kCsThreads) {
     const int v = i / kCsCarryKeys, k = i % kCsCarryKeys;     // k fastest: the slot's layout, whole 32-byte sectors
-    tile[v][k] = (!fresh && v0 + v < a.dv) ? Sp[(size_t)(v0 + v) * DK + k0 + k] : 0.f;
+    tile[v][k] = (!fresh && v0 + v < a.dv) ? __ldcg(Sp + (size_t)(v0 + v) * DK + k0 + k) : 0.f;
   }
   cs_wait_before();
   cs_release_next();                                  // (behind the wait: an output's CTA finds the chunks' states complete)
@@ -347,7 +347,7 @@ chunk_carry_kernel(const ChunkScanArgs a, const typename Form::Params p) {
     float4 in[U];
 #pragma unroll
     for (int u = 0; u < U; ++u)
-      if (live && c0 + u < nc) in[u] = *reinterpret_cast<const float4*>(C + (size_t)(c0 + u) * step);
+      if (live && c0 + u < nc) in[u] = __ldcg(reinterpret_cast<const float4*>(C + (size_t)(c0 + u) * step));
     carry.fetch(c0, nc);
 #pragma unroll
     for (int u = 0; u < U; ++u) {

@@ -110,8 +110,7 @@ conv_rec_prep_vec_kernel(CrpArgs a, int lph, int rows) {
   }
   if (act) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if (i < m.n) raw[i] = *reinterpret_cast<const uint4*>(at + (int64_t)i * a.ld);
+    for (int i = 0; i < 4; ++i) raw[i] = ld_cg_if(reinterpret_cast<const uint4*>(at + (int64_t)i * a.ld), i < m.n);
     uint4 old[R > 0 ? R : 1];
     conv_before<TA, TAPS>(old, m, src, a.ld, a.ring, c, a.C);
 #pragma unroll
@@ -139,7 +138,7 @@ conv_rec_prep_vec_kernel(CrpArgs a, int lph, int rows) {
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
         crp_pairs(raw[i + k], x[i + k], TA());
-        if (act && r + k + 4 < m.n) raw[i + k] = *reinterpret_cast<const uint4*>(at + (int64_t)(r + k + 4) * a.ld);
+        if (act && r + k + 4 < m.n) raw[i + k] = __ldcg(reinterpret_cast<const uint4*>(at + (int64_t)(r + k + 4) * a.ld));
 #pragma unroll
         for (int e = 0; e < P; ++e) {
           f32x2 s = bias[e];

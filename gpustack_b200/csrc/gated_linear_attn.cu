@@ -75,18 +75,16 @@ gla_scan_kernel(const float* __restrict__ x, int64_t ld, int q_col, int k_col, i
 #pragma unroll
     for (int e = 0; e < PF; ++e) {
       const int i = threadIdx.x + e * kGlWarps * 32, tt = i / DKP, dd = i - tt * DKP;
-      pq[e] = pk[e] = pz[e] = 0.f;
-      if (i < nt * DKP && dd < dk) {
-        const float* row = x + (size_t)(ch + tt) * ld;
-        pq[e] = row[q_col + h * dk + dd];
-        pk[e] = row[k_col + h * dk + dd];
-        pz[e] = z[(size_t)(ch + tt) * ldz + h * dk + dd];
-      }
+      const bool there = i < nt * DKP && dd < dk;
+      const float* row = x + (size_t)(ch + tt) * ld;
+      pq[e] = ld_cg_if(row + q_col + h * dk + dd, there);
+      pk[e] = ld_cg_if(row + k_col + h * dk + dd, there);
+      pz[e] = ld_cg_if(z + (size_t)(ch + tt) * ldz + h * dk + dd, there);
     }
 #pragma unroll
     for (int e = 0; e < PV; ++e) {
       const int i = threadIdx.x + e * kGlWarps * 32, tt = i / kGlCols, cc = zc * kGlCols + (i % kGlCols);
-      pv[e] = (i < nt * kGlCols && cc < dv) ? x[(size_t)(ch + tt) * ld + v_col + h * dv + cc] : 0.f;
+      pv[e] = ld_cg_if(x + (size_t)(ch + tt) * ld + v_col + h * dv + cc, i < nt * kGlCols && cc < dv);
     }
   };
   fetch(t0);
@@ -160,7 +158,7 @@ struct GatedLinearForm {
     for (int b = 0; b < N; b += AHEAD) {
       float v[AHEAD];
 #pragma unroll
-      for (int i = 0; i < AHEAD; ++i) v[i] = r0 + (b + i) * STEP < at.rows ? z[(size_t)(b + i) * STEP * p.ldz] : 0.f;
+      for (int i = 0; i < AHEAD; ++i) v[i] = r0 + (b + i) * STEP < at.rows ? __ldcg(z + (size_t)(b + i) * STEP * p.ldz) : 0.f;
 #pragma unroll
       for (int i = 0; i < AHEAD; ++i) {
         const int t = r0 + (b + i) * STEP;
@@ -181,7 +179,7 @@ struct GatedLinearForm {
     __device__ __forceinline__ void fetch(int c0, int nc) {
 #pragma unroll
       for (int u = 0; u < kCsCarryDepth; ++u)
-        if (c0 + u < nc) f[u] = row[(c0 + u) * step];
+        if (c0 + u < nc) f[u] = __ldcg(row + (c0 + u) * step);
     }
   };
   static __device__ __forceinline__ float aq(const Scratch&, int) { return 1.0f; }
@@ -226,13 +224,13 @@ gla_step_kernel(const float* __restrict__ x, int64_t ld, int q_col, int k_col, i
     for (int i = threadIdx.x; i < nt * dk; i += blockDim.x) {
       const int tt = i / dk, dd = i - tt * dk;
       const float* row = x + (size_t)(ch + tt) * ld;
-      qs[i] = row[q_col + h * dk + dd];
-      ks[i] = row[k_col + h * dk + dd];
-      as[i] = gl_alpha(z[(size_t)(ch + tt) * ldz + h * dk + dd], inv_tau);
+      qs[i] = __ldcg(row + q_col + h * dk + dd);
+      ks[i] = __ldcg(row + k_col + h * dk + dd);
+      as[i] = gl_alpha(__ldcg(z + (size_t)(ch + tt) * ldz + h * dk + dd), inv_tau);
     }
     for (int i = threadIdx.x; i < nt * kGlCols; i += blockDim.x) {
       const int tt = i / kGlCols, c = zc * kGlCols + (i % kGlCols);
-      vs[i] = c < dv ? x[(size_t)(ch + tt) * ld + v_col + h * dv + c] : 0.f;
+      vs[i] = c < dv ? __ldcg(x + (size_t)(ch + tt) * ld + v_col + h * dv + c) : 0.f;
     }
     __syncthreads();
     for (int tt = 0; tt < nt; ++tt) {

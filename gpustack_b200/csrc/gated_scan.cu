@@ -240,8 +240,8 @@ gated_scan_kernel(GatedScanArgs a) {
       const int t = st * kGsStage + n;
       if (t < rows) {
         const float* g = a.gates + (size_t)(t0 + t) * a.ld_g;
-        ra = DELTA ? g[a.H + h] : g[h];
-        if (DELTA) rb = g[h];
+        ra = __ldcg(g + (DELTA ? a.H + h : h));
+        if (DELTA) rb = __ldcg(g + h);
       }
     };
     // outputs of this warp's block: the read-out of the state before it and what its own tokens add
@@ -553,16 +553,16 @@ gated_step_kernel(GatedScanArgs a) {
     ulonglong2 ts = make_ulonglong2(0, 0), tk = ts, tq = ts;
     if (d < dkp) {
       if (live && !fresh) ts = *reinterpret_cast<const ulonglong2*>(Sp + d);
-      tk = *reinterpret_cast<const ulonglong2*>(row + a.k_col + hk * dkp + d);
-      tq = *reinterpret_cast<const ulonglong2*>(row + a.q_col + hk * dkp + d);
+      tk = __ldcg(reinterpret_cast<const ulonglong2*>(row + a.k_col + hk * dkp + d));
+      tq = __ldcg(reinterpret_cast<const ulonglong2*>(row + a.q_col + hk * dkp + d));
     }
     S[2 * i] = ts.x; S[2 * i + 1] = ts.y;
     k[2 * i] = tk.x; k[2 * i + 1] = tk.y;
     q[2 * i] = tq.x; q[2 * i + 1] = tq.y;
   }
-  const float v = live ? row[a.v_col + h * a.dvp + col] : 0.f;
+  const float v = live ? __ldcg(row + a.v_col + h * a.dvp + col) : 0.f;
   const float* g = a.gates + (size_t)t * a.ld_g;
-  const float2 gb = gs_gate<DELTA>(DELTA ? g[a.H + h] : g[h], DELTA ? g[h] : 0.f, a.rate[h], a.dt_bias[h]);
+  const float2 gb = gs_gate<DELTA>(__ldcg(g + (DELTA ? a.H + h : h)), DELTA ? __ldcg(g + h) : 0.f, a.rate[h], a.dt_bias[h]);
   float u = gb.y * v;
   if (DELTA) u = gb.y * (v - gb.x * lanes_sum<L>(gs_dot1<R2>(S, k)));
   const f32x2 g2 = pack2(gb.x, gb.x), u2 = pack2(u, u);
@@ -665,7 +665,7 @@ struct StateSpaceForm {
       f[e] = 0.0;
       beta[e] = 0.f;
       if (t < at.rows) {
-        beta[e] = gs_softplus(p.gates[(size_t)(at.first + t) * p.ld_g + h] + bias);
+        beta[e] = gs_softplus(__ldcg(p.gates + (size_t)(at.first + t) * p.ld_g + h) + bias);
         const float lg = -rate * beta[e];
         f[e] = lg < -1.0e4f ? -1.0e4 : (double)lg;
       }
@@ -705,7 +705,7 @@ struct StateSpaceForm {
     __device__ __forceinline__ void fetch(int c0, int nc) {
 #pragma unroll
       for (int u = 0; u < kCsCarryDepth; ++u)
-        if (c0 + u < nc) f[u] = row[(c0 + u) * step];
+        if (c0 + u < nc) f[u] = __ldcg(row + (c0 + u) * step);
     }
   };
   static __device__ __forceinline__ void output_weights(const Params& p, const ChunkScanArgs&, Scratch& sc, int h, const ChunkPlace& at) {
@@ -734,17 +734,18 @@ struct StateSpaceForm {
 // out = RMSnorm over `parts` equal pieces of (y * silu(z)), times w[channel] -- the gate BEFORE the norm -- or, with the gate
 // AFTER it, RMSnorm of the pieces of y times w[place in the piece] (one weight vector for all pieces) times silu(z).  One CTA
 // per row; the row is staged in shared memory between the statistic and the product.
-template <typename TA>
-__device__ __forceinline__ float4 gs_ld4(const TA* p);
-template <>
-__device__ __forceinline__ float4 gs_ld4<float>(const float* p) { return *reinterpret_cast<const float4*>(p); }
-template <>
-__device__ __forceinline__ float4 gs_ld4<bf16>(const bf16* p) {
+// four or one value(s) of the rows that kernels before this one wrote, and of weights
+__device__ __forceinline__ float4 gs_cg4(const float* p) { return __ldcg(reinterpret_cast<const float4*>(p)); }
+__device__ __forceinline__ float4 gs_cg4(const bf16* p) {
+  const uint2 r = __ldcg(reinterpret_cast<const uint2*>(p));
+  return make_float4(bf16_lo(r.x), bf16_hi(r.x), bf16_lo(r.y), bf16_hi(r.y));
+}
+__device__ __forceinline__ float gs_cg1(const float* p) { return __ldcg(p); }
+__device__ __forceinline__ float gs_cg1(const bf16* p) { return __bfloat162float(__ldcg(p)); }
+__device__ __forceinline__ float4 gs_w4(const bf16* p) {
   const uint2 r = *reinterpret_cast<const uint2*>(p);
   return make_float4(bf16_lo(r.x), bf16_hi(r.x), bf16_lo(r.y), bf16_hi(r.y));
 }
-__device__ __forceinline__ float gs_ld1(const float* p) { return *p; }
-__device__ __forceinline__ float gs_ld1(const bf16* p) { return __bfloat162float(*p); }
 __device__ __forceinline__ void gs_st1(float* p, float v) { *p = v; }
 __device__ __forceinline__ void gs_st1(bf16* p, float v) { *p = __float2bfloat16_rn(v); }
 __device__ __forceinline__ void gs_st4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
@@ -774,15 +775,15 @@ gate_norm_kernel(const float* __restrict__ y, const TA* __restrict__ proj, int64
       for (int i = (sub * 32 + lane) * V; i < W; i += per * 32 * V) {
         const int c = p * W + i;
         if (VEC) {
-          float4 v = *reinterpret_cast<const float4*>(yr + c);
+          float4 v = gs_cg4(yr + c);
           if (!AFTER) {
-            const float4 g = gs_ld4<TA>(zr + c);
+            const float4 g = gs_cg4(zr + c);
             v.x *= gs_silu(g.x); v.y *= gs_silu(g.y); v.z *= gs_silu(g.z); v.w *= gs_silu(g.w);
           }
           *reinterpret_cast<float4*>(row + c) = v;
           ss = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, ss))));
         } else {
-          const float v = AFTER ? yr[c] : yr[c] * gs_silu(gs_ld1(zr + c));
+          const float v = AFTER ? gs_cg1(yr + c) : gs_cg1(yr + c) * gs_silu(gs_cg1(zr + c));
           row[c] = v;
           ss = fmaf(v, v, ss);
         }
@@ -802,14 +803,14 @@ gate_norm_kernel(const float* __restrict__ y, const TA* __restrict__ proj, int64
       const int c = p * W + i;
       if (VEC) {
         float4 v = *reinterpret_cast<const float4*>(row + c);
-        const float4 g = gs_ld4<bf16>(w + (AFTER ? i : c));
+        const float4 g = gs_w4(w + (AFTER ? i : c));
         if (AFTER) {
-          const float4 t = gs_ld4<TA>(zr + c);
+          const float4 t = gs_cg4(zr + c);
           v.x *= gs_silu(t.x); v.y *= gs_silu(t.y); v.z *= gs_silu(t.z); v.w *= gs_silu(t.w);
         }
         gs_st4(o + c, make_float4(v.x * rstd * g.x, v.y * rstd * g.y, v.z * rstd * g.z, v.w * rstd * g.w));
       } else {
-        gs_st1(o + c, row[c] * rstd * gs_ld1(w + (AFTER ? i : c)) * (AFTER ? gs_silu(gs_ld1(zr + c)) : 1.0f));
+        gs_st1(o + c, row[c] * rstd * __bfloat162float(w[AFTER ? i : c]) * (AFTER ? gs_silu(gs_cg1(zr + c)) : 1.0f));
       }
     }
   }
@@ -836,8 +837,8 @@ gate_norm_heads_kernel(const float* __restrict__ y, const TA* __restrict__ proj,
     if (n * step >= C) break;
     v[n] = g[n] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (i < C) {
-      v[n] = *reinterpret_cast<const float4*>(yr + i);
-      g[n] = gs_ld4<TA>(zr + i);
+      v[n] = gs_cg4(yr + i);
+      g[n] = gs_cg4(zr + i);
     }
   }
 #pragma unroll
@@ -857,7 +858,7 @@ gate_norm_heads_kernel(const float* __restrict__ y, const TA* __restrict__ proj,
       if (s < lanes) ss += __shfl_xor_sync(0xffffffffu, ss, s);
     if (i >= C) continue;
     const float rstd = inv_sqrt(ss * over + eps);
-    const float4 c = gs_ld4<bf16>(w + (AFTER ? i & (W - 1) : i));
+    const float4 c = gs_w4(w + (AFTER ? i & (W - 1) : i));
     x = make_float4(x.x * rstd * c.x, x.y * rstd * c.y, x.z * rstd * c.z, x.w * rstd * c.w);
     if (AFTER) { x.x *= g[n].x; x.y *= g[n].y; x.z *= g[n].z; x.w *= g[n].w; }
     gs_st4(o + i, x);
@@ -884,8 +885,8 @@ gate_norm_parts_kernel(const float* __restrict__ y, const TA* __restrict__ proj,
   for (int n = 0; n < N; ++n) {
     const int i = i0 + n * step;
     if (i >= C) break;
-    v[n] = *reinterpret_cast<const float4*>(yr + i);
-    g[n] = gs_ld4<TA>(zr + i);
+    v[n] = gs_cg4(yr + i);
+    g[n] = gs_cg4(zr + i);
   }
 #pragma unroll
   for (int n = 0; n < N; ++n) {
@@ -907,7 +908,7 @@ gate_norm_parts_kernel(const float* __restrict__ y, const TA* __restrict__ proj,
     float ss = 0.f;
     for (int j = 0; j < per; ++j) ss += sums[piece * per + j];
     const float rstd = inv_sqrt(ss / (float)W + eps);
-    const float4 c = gs_ld4<bf16>(w + (AFTER ? i - piece * W : i));
+    const float4 c = gs_w4(w + (AFTER ? i - piece * W : i));
     float4 x = v[n];
     x = make_float4(x.x * rstd * c.x, x.y * rstd * c.y, x.z * rstd * c.z, x.w * rstd * c.w);
     if (AFTER) { x.x *= g[n].x; x.y *= g[n].y; x.z *= g[n].z; x.w *= g[n].w; }

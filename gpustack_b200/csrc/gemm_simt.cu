@@ -23,9 +23,10 @@ __device__ __forceinline__ void from_f32x4(bf16* p, const float (&v)[4]) {
 
 // Bound by shared-memory reads and, where K is short, by the stores: a k's eight operands are two 16-byte reads, four neighbouring
 // results one store where Y's rows allow it, and a block of k is on its way while the one before is multiplied (6007 x 16 -> 512, fp32
-// results, 14.2 -> 8.4 us; 64 x 4096 -> 4096 in fp32 678 -> 257; 8192 x 512 -> 2048 794 -> 521).
+// results, 14.2 -> 8.4 us; 64 x 4096 -> 4096 in fp32 678 -> 257; 8192 x 512 -> 2048 794 -> 521).  CTAs per SM: left to
+// itself the compiler takes 71 registers for fp32 rows' loads past L1 (4100 x 16 -> 512 7.3 -> 5.6 us); of bf16 rows 44
 template <typename TX, typename TY>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, sizeof(TX) == 4 ? 4 : 0)
 gemm_simt_kernel(const TX* __restrict__ X, const bf16* __restrict__ W, const bf16* __restrict__ bias,
                  TY* __restrict__ Y, int M, int N, int K, int64_t ldx, int64_t ldw, int64_t ldy) {
   pdl_wait();
@@ -47,7 +48,7 @@ gemm_simt_kernel(const TX* __restrict__ X, const bf16* __restrict__ W, const bf1
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int r = lr + 16 * i;
-      xv[i] = k < K && m0 + r < M ? to_f32(X[(int64_t)(m0 + r) * ldx + k]) : 0.f;
+      xv[i] = k < K && m0 + r < M ? to_f32(__ldcg(X + (int64_t)(m0 + r) * ldx + k)) : 0.f;
       wv[i] = k < K && n0 + r < N ? to_f32(W[(int64_t)(n0 + r) * ldw + k]) : 0.f;
     }
   };

@@ -127,12 +127,12 @@ latent_prep_rows_kernel(const bf16* __restrict__ proj, int64_t ld, int kv_col, c
   uint32_t part[kLpHeads + 1];
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
-    lat[i] = ld_v4(kv + i * 256 + lane * 8);
+    lat[i] = __ldcg(reinterpret_cast<const uint4*>(kv + i * 256 + lane * 8));
     wn[i] = ld_v4(kv_norm_w + i * 256 + lane * 8);
   }
-  part[kLpHeads] = *reinterpret_cast<const uint32_t*>(kv + R + 2 * lane);
+  part[kLpHeads] = __ldcg(reinterpret_cast<const uint32_t*>(kv + R + 2 * lane));
 #pragma unroll
-  for (int h = 0; h < kLpHeads; ++h) part[h] = h < H ? *reinterpret_cast<const uint32_t*>(qr + (size_t)h * (dn + DR)) : 0u;
+  for (int h = 0; h < kLpHeads; ++h) part[h] = __float_as_uint(ld_cg_if(reinterpret_cast<const float*>(qr + (size_t)h * (dn + DR)), h < H));
   // lane l: the angle of pair l, formed and reduced in fp64 as above
   const double ang = (double)pos * freq[lane];
   const double turns = rint(ang * 0.15915494309189535);
@@ -184,7 +184,7 @@ latent_prep_rows_kernel(const bf16* __restrict__ proj, int64_t ld, int kv_col, c
 #pragma unroll
     for (int h = 0; h < kLpHeads; ++h) {
       const int n = h0 + kLpHeads + h;
-      next[h] = n < H ? *reinterpret_cast<const uint32_t*>(qr + (size_t)n * (dn + DR)) : 0u;
+      next[h] = __float_as_uint(ld_cg_if(reinterpret_cast<const float*>(qr + (size_t)n * (dn + DR)), n < H));
     }
 #pragma unroll
     for (int h = 0; h < kLpHeads; ++h) {

@@ -405,7 +405,7 @@ latent_attn_step_kernel(const __grid_constant__ CUtensorMap rows_map, LaArgs a) 
     for (int ci = threadIdx.x; ci < 16 * cpr; ci += blockDim.x) {
       const int i = ci / cpr, c = ci - i * cpr;
       uint4 v = make_uint4(0, 0, 0, 0);
-      if (i < HB && h0 + i < a.H) v = ld_v4(a.qa + (size_t)s * a.ldq + (size_t)(h0 + i) * W + c * 8);
+      if (i < HB && h0 + i < a.H) v = ld_cg_v4(a.qa + (size_t)s * a.ldq + (size_t)(h0 + i) * W + c * 8);
       *reinterpret_cast<uint4*>(q_s + i * pitch + c * 16) = v;
     }
     __syncthreads();
@@ -555,7 +555,7 @@ latent_attn_merge_kernel(const float* __restrict__ ws, const float* __restrict__
   const int b = blockIdx.x, h = blockIdx.y, lane = threadIdx.x & 31;
   const float* p = ws + ((size_t)b * H + h) * nsplit * (R + 2);
   float2 ml = make_float2(-INFINITY, 0.f);
-  if (lane < nsplit) ml = make_float2(p[(size_t)lane * (R + 2) + R], p[(size_t)lane * (R + 2) + R + 1]);
+  if (lane < nsplit) ml = make_float2(__ldcg(p + (size_t)lane * (R + 2) + R), __ldcg(p + (size_t)lane * (R + 2) + R + 1));
   float M = ml.x;
 #pragma unroll
   for (int w = 16; w > 0; w >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, w));
@@ -574,7 +574,7 @@ latent_attn_merge_kernel(const float* __restrict__ ws, const float* __restrict__
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int d = threadIdx.x + 128 * i;
-      if (d < R) acc[i] = fmaf(p[(size_t)s * (R + 2) + d], f, acc[i]);
+      acc[i] = fmaf(ld_cg_if(p + (size_t)s * (R + 2) + d, d < R), f, acc[i]);
     }
   }
 #pragma unroll

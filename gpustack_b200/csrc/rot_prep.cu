@@ -152,7 +152,8 @@ rot_prep_kernel(RotPrepArgs a) {
 // 45.4 -> 28.2); the unrotated rest are plain items.  LPH lanes (a power of two >= items per head) share a head, a warp covers
 // 32 / LPH head slots at a time, the sum of squares is reduced inside the group.
 // SILU is an instance of its own: its code, unused, cost the others 2 to 14 %.  Resident CTAs: five of bf16 rows (48 registers; without
-// the bound 58, 2048 rows 12.2 -> 14.1 us), fp32 rows as they compile.
+// the bound 58, 2048 rows 12.2 -> 14.1 us), fp32 rows as they compile.  Plain loads: past L1 fp32 rows take 5 to 14 % longer (8192 rows 52 -> 56,
+// 61 without a bound of six CTAs), and this kernel releases nothing early.
 constexpr int kRvThreads = 256;
 
 template <typename TA, typename TD, int TOK, bool SILU>
@@ -320,7 +321,7 @@ rot_plain_kernel(RotPrepArgs a, int T) {
   uint4 raw[ROWS];
 #pragma unroll
   for (int r = 0; r < ROWS; ++r)
-    if (t0 + r < T) raw[r] = *reinterpret_cast<const uint4*>(src + (size_t)r * a.ld);
+    if (t0 + r < T) raw[r] = __ldcg(reinterpret_cast<const uint4*>(src + (size_t)r * a.ld));
 #pragma unroll
   for (int r = 0; r < ROWS; ++r) {
     if (t0 + r >= T) break;
