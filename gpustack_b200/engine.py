@@ -404,8 +404,9 @@ class LLMEngine:
         for j, e in enumerate(singles):
             bt[j, :len(e[1].blocks)] = e[1].blocks
         dslots = np.asarray([e[1].state_slot for e in singles], dtype=np.int32)
-        # nothing reads the sampled tokens, and the copy of the logits waits for the stream: a wait of the step's own and the
-        # bookkeeping behind it would only keep that copy from following at once (3 rows, graph of 132 us: a step 252 -> 214 us)
+        # nothing reads the sampled tokens, and the copy of the logits waits for the stream: a wait of the step's own would only keep
+        # that copy from following at once (3 rows, graph of 132 us: a step 252 -> 214 us).  It comes before the requests move on, so that
+        # a step that failed on the device leaves them, and what `end` would give back, as they were
         wait = not any(want for _, _, _, want in chunks + singles)
         if chunks:
             self.runner.prefill([e[2] for e in chunks], [e[1].num_computed for e in chunks], [e[1].blocks for e in chunks],
@@ -422,6 +423,7 @@ class LLMEngine:
         else:
             self.runner.decode(B, last, comp, bt, state_slots=dslots if self.state_slots else None, wait=wait)
             parts = {e[0]: range(j, j + (1 if e[3] else 0)) for j, e in enumerate(singles)}
+        logits = self.runner.host_logits([row for i in range(len(entries)) for row in parts[i]])
         for _, r, toks, _ in chunks + singles:
             r.prompt_ids.extend(toks)
             r.num_computed += len(toks)
@@ -430,7 +432,7 @@ class LLMEngine:
             if r is not None:
                 s.replay_finish(r)
         self.counters["steps"] += 1
-        return self.runner.host_logits([row for i in range(len(entries)) for row in parts[i]])
+        return logits
 
     def _apply_sampling(self, reqs, toks):
         """Plain temperature sampling happens in the sampler kernel (Gumbel-max, runner._sample); only

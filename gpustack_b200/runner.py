@@ -38,6 +38,7 @@ def _align(n: int, a: int = 4) -> int:
 
 class ModelRunner:
     SUPPORTS_FP32 = False
+    t_decode: Optional[float] = None          # start of a decode step whose end host_logits() waits for
 
     def __init__(self, mcfg: ModelConfig, ecfg: EngineConfig, weights: ModelWeights, device: str = "cuda",
                  tp_group=None, tp_ctx=None):
@@ -526,7 +527,8 @@ class ModelRunner:
                state_slots: Optional[np.ndarray] = None, wait: bool = True) -> Optional[np.ndarray]:
         """One decode step for rows 0..B-1 of the scheduler's persistent batch.  temps (fp32) / seeds
         (uint32, already mixed with the position) per row drive the in-kernel sampler; None = greedy.
-        wait=False: the tokens stay on the device and the caller waits for the stream before it stages another step."""
+        wait=False: the tokens stay on the device and the caller takes the logits by host_logits(), which waits for the stream and
+        closes the step's time, before it stages another step."""
         S, bs = self.max_seqs, self.block_size
         Bp = B
         if self.graphs:
@@ -566,14 +568,18 @@ class ModelRunner:
         if wait:
             self.out_host[:B].copy_(self.out_ids[:B], non_blocking=True)
             torch.cuda.current_stream().synchronize()
-            self.stats["decode_gpu_s"] = self.stats.get("decode_gpu_s", 0.0) + time.perf_counter() - t_gpu
+            self._add_decode_time(t_gpu)
             self.stats["d2h_bytes"] += B * 4
         self.stats["decode_steps"] += 1
         self.stats["h2d_bytes"] += n * 4
         self.stats["decode_kv_tokens"] += int(pos.sum()) + B
         if not wait:
+            self.t_decode = t_gpu
             return None
         return self.out_host[:B].numpy()
+
+    def _add_decode_time(self, since: float) -> None:
+        self.stats["decode_gpu_s"] = self.stats.get("decode_gpu_s", 0.0) + time.perf_counter() - since
 
     # ------------------------------------------------------------------------------ prefill
     def prefill(self, token_chunks: Sequence[Sequence[int]], starts: Sequence[int], block_tables: Sequence[Sequence[int]],
@@ -759,7 +765,16 @@ class ModelRunner:
     # -------------------------------------------------------------------- test / debug hooks
     def host_logits(self, rows: Sequence[int]) -> np.ndarray:
         """fp32 logits [len(rows), V] of the given rows of the last _sample() call (local vocab shard).  Up to a few megabytes
-        pass a pinned buffer; neighbouring rows in order leave without a gather on the device."""
+        pass a pinned buffer; neighbouring rows in order leave without a gather on the device.  Ends a decode step that did not
+        wait (decode(wait=False))."""
+        out = self._host_logits(rows)
+        self.stats["d2h_bytes"] += out.nbytes
+        if self.t_decode is not None:
+            self._add_decode_time(self.t_decode)
+            self.t_decode = None
+        return out
+
+    def _host_logits(self, rows: Sequence[int]) -> np.ndarray:
         n = len(rows)
         if n and rows[-1] - rows[0] == n - 1 and all(b == a + 1 for a, b in zip(rows, rows[1:])):
             lg = self.logits[rows[0]:rows[0] + n]
