@@ -1,8 +1,8 @@
 // A recurrent mixer's closing step per (token, head): the head's fp32 output over its root mean square, times a weight, times the
 // gate's activation, rounded once.  A head of dv = 4 LPH values is held by LPH lanes as one 16-byte piece each, one head per group of
-// lanes; a group goes through the heads of one number (its weight stays in registers, a step is an addition per pointer), the next
-// head's loads in flight.  Bound: launch and latency up to 1000 rows, then instructions.  8 heads of 128, bf16 gates, 8192 rows:
-// a head per group, its place divided out, 18.9 us (205 instructions a thread), 17.1 now (155 a head).
+// lanes.  Of many rows (MORE) a group goes through the heads of one number (its weight stays in registers, a step is an addition per
+// pointer), the next head's loads in flight.  Bound: launch and latency up to 1000 rows, then instructions.  8 heads of 128, bf16 gates,
+// 8192 rows: a head per group, its place divided out, 20.7 us (205 instructions a thread), 18.4 of many (155 a head).
 #pragma once
 #include "common.cuh"
 
@@ -18,15 +18,15 @@ __device__ __forceinline__ float4 ho_ld4(const bf16* p) {
 __device__ __forceinline__ void ho_st4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
 __device__ __forceinline__ void ho_st4(bf16* p, float4 v) { *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w)); }
 
-template <typename TA, int LPH>
-__global__ void __launch_bounds__(kHoThreads, kHoCtas)
+template <typename TA, int LPH, bool MORE>
+__global__ void __launch_bounds__(kHoThreads, MORE ? kHoCtas : 0)
 head_out_kernel(const float* __restrict__ o, const TA* __restrict__ proj, int64_t ld, int gate_col, const bf16* __restrict__ w, int w_head,
                 TA* out, int64_t ldo, int items, int H, int step, int silu, float eps) {
   constexpr int DV = 4 * LPH;
   const int lane = threadIdx.x & 31, d = (lane % LPH) * 4;
   const int first = (blockIdx.x * (kHoThreads / 32) + (threadIdx.x >> 5)) * (32 / LPH), i0 = first + lane / LPH;
   if (first >= step) return;                           // (step: a multiple of H)
-  const int t0 = i0 / H, h = i0 - t0 * H, rows = step / H;
+  const int t0 = i0 / H, h = i0 - t0 * H, rows = MORE ? step / H : 0;
   const bool mine = i0 < step;
   const float* op = o + (size_t)i0 * DV + d;
   const TA* gp = gate_col >= 0 ? proj + (size_t)t0 * ld + gate_col + h * DV + d : nullptr;
@@ -42,10 +42,12 @@ head_out_kernel(const float* __restrict__ o, const TA* __restrict__ proj, int64_
   for (int at = first, i = i0; at < items; at += step, i += step) {
     const bool live = mine && i < items;
     float4 xn = zero, gn = zero;
-    op += (size_t)step * DV;
-    if (mine && i < items - step) {
-      xn = ho_ld4(op);
-      if (gate_col >= 0) gn = ho_ld4(gp += (size_t)rows * ld);
+    if constexpr (MORE) {
+      op += (size_t)step * DV;
+      if (mine && i < items - step) {
+        xn = ho_ld4(op);
+        if (gate_col >= 0) gn = ho_ld4(gp += (size_t)rows * ld);
+      }
     }
     float ss = fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, x.w * x.w)));
 #pragma unroll
@@ -61,6 +63,7 @@ head_out_kernel(const float* __restrict__ o, const TA* __restrict__ proj, int64_
       for (int e = 0; e < 4; ++e) v[e] *= silu ? gv[e] * sg[e] : sg[e];
     }
     if (live) ho_st4(to, make_float4(v[0], v[1], v[2], v[3]));
+    if constexpr (!MORE) break;
     to += (size_t)rows * ldo;
     x = xn;
     g = gn;
@@ -77,13 +80,22 @@ bool head_out_launch(const float* o, const void* proj, int64_t ld, int gate_col,
     return false;
   if (gate_col >= 0 && (ld % 4 != 0 || gate_col % 4 != 0 || ((uintptr_t)proj & al))) return false;
   const int items = T * H, per = kHoThreads / 32 * (128 / dv);      // groups per CTA
-  // groups in whole multiples of the heads; no more CTAs than are resident
+  // groups in whole multiples of the heads; no more CTAs than are resident.  Fewer registers and more CTAs serve less than five rounds
+  // better: 16 heads of 64 in bf16, a head per group and resident CTAs, 1000 rows 4.5 and 5.0 us, 2048 6.7 and 7.3, 3000 8.7 and 9.0,
+  // 4100 10.7 and 10.9; 32 heads of 32, 4100 rows, 10.8 and 10.4
+  constexpr int kRounds = 5;
   int step = items;
-  if (items > kHoCtas * 148 * per && H <= kHoCtas * 148 * per) step = kHoCtas * 148 * per / H * H;
+  if (items > kRounds * kHoCtas * 148 * per && H <= kHoCtas * 148 * per) step = kHoCtas * 148 * per / H * H;
   const int grid = (step + per - 1) / per;
 #define B200_HO(L)                                                                                                                 \
-  head_out_kernel<TA, L><<<grid, kHoThreads, 0, s>>>(o, (const TA*)proj, ld, gate_col, (const bf16*)w, w_head, (TA*)out, ldo, items, H, step, \
-                                                     silu, eps)
+  do {                                                                                                                             \
+    if (step < items)                                                                                                              \
+      head_out_kernel<TA, L, true><<<grid, kHoThreads, 0, s>>>(o, (const TA*)proj, ld, gate_col, (const bf16*)w, w_head, (TA*)out, ldo, \
+                                                               items, H, step, silu, eps);                                         \
+    else                                                                                                                           \
+      head_out_kernel<TA, L, false><<<grid, kHoThreads, 0, s>>>(o, (const TA*)proj, ld, gate_col, (const bf16*)w, w_head, (TA*)out, ldo, \
+                                                                items, H, step, silu, eps);                                        \
+  } while (0)
   if (dv == 32) B200_HO(8);
   else if (dv == 64) B200_HO(16);
   else B200_HO(32);

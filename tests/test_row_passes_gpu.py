@@ -82,7 +82,9 @@ def test_rows_without_a_rotation_and_values_in_pairs(T, src, dst, H, G, dk, dv):
     assert not any(o[:, n:].any() for o, n in zip(outs, (nq, nk, nv)))
 
 
-@pytest.mark.parametrize("T,H,dv", [(1, 1, 32), (5, 7, 64), (2601, 9, 32), (1201, 24, 128)])
+# a head per group of lanes; then several, from 5 * 740 CTAs on: of 4, 2 and 1 groups to a warp, rounds that end inside a warp and in the middle
+# of a row
+@pytest.mark.parametrize("T,H,dv", [(1, 1, 32), (5, 7, 64), (2601, 9, 32), (1201, 24, 128), (13200, 9, 32), (8600, 7, 64), (9867, 3, 128), (1235, 24, 128)])
 @pytest.mark.parametrize("dtype", [F32, BF])
 def test_closing_step_over_many_heads(T, H, dv, dtype):
     from gpustack_b200 import ops
