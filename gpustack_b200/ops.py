@@ -630,9 +630,10 @@ def mlstm_state_slices(dv: int) -> int:
 # taken was at most 11 % slower than the other in any of them.  One-pass -> chunks, 8 heads: gated linear attention of 256 rows 47 -> 50,
 # of 512 84 -> 52, 16 of 128 rows 70 -> 83, of 1024 rows 433 -> 390, one of 2048 beside thirty of 16 449 -> 108; state space of 32
 # heads: 1024 rows 109 -> 87, 2048 rows 207 -> 140, 16 of 512 rows 399 -> 532, one of 2048 beside thirty of 16 477 -> 195.
-# (Those are the times of the fit.  Since then gated linear attention's chunks take a fifth less and state space's one-pass form a tenth:
-# 1024 rows 98 -> 38, 2048 rows 187 -> 66 us of 8 heads; of 288 steps measured again 20 lie on the side that is now slower by more
-# than 5 %, most of them gated linear portions of 256 to 512 rows that stay one-pass, at worst 223 against 165.)
+# (Those are the times of the fit, and so is the 11 %.  Since then gated linear attention's chunks take a fifth less and state space's one-pass
+# form a tenth: 1024 rows 98 -> 38, 2048 rows 187 -> 66 us of 8 heads; of 288 steps measured again 20 lie on the side that is now slower
+# by more than 5 %, most of them gated linear portions of 256 to 512 rows that stay one-pass, at worst 223 against 165.  The line was
+# not fitted anew.)
 # Linear attention's and mLSTM's lines lie where their chunks of 64 rows by FMAs crossed the one-pass form.  Of 128 rows on the tensor
 # cores, measured at 432 steps of 1 to 201 sequences of 33 to 2048 rows and 4 to 32 heads: the 294 that go to chunks are faster than
 # one-pass, all of them, and no slower than by FMAs (one by 2 %); of the 138 that stay one-pass 68 would be more than 11 % faster over
@@ -652,7 +653,7 @@ def chunk_scan_pays(kind: str, rows: int, n_seqs: int, H: int, dk: int, dv: int,
         return False
     c = CHUNK_COSTS[kind]
     longest = -(-rows // n_seqs) if max_len == rows and n_seqs > 1 else max_len
-    if longest <= 32:                                   # half a chunk of 64 rows at most: over those one-pass was always the better
+    if longest <= 32:                                   # half a chunk of 64 rows at most: one-pass was the better or, 16 portions of 32 rows, 7 us off
         return False
     heads = H * dk * dv / c.width / 1000.0
     one = c.one_fixed + max(c.one_row * longest, c.one_work * (rows - n_seqs) * heads)

@@ -5,8 +5,8 @@ import torch
 pytestmark = pytest.mark.gpu
 
 F64 = torch.float64
-# as for the recurrences as a whole: sums of at most 300 terms of one size, each rounded, without cancellation beyond a factor of 2
-TOL = 2 * 300 * 2.0 ** -24
+# sums of at most 300 terms of one size without cancellation, each rounding by itself and by at most 2^-24 of the sum
+TOL = 300 ** 0.5 * 2.0 ** -24
 
 
 @pytest.mark.parametrize("rows", [61, 66, 131])
