@@ -33,38 +33,6 @@ namespace b200 {
 
 constexpr int kCsRows = 64, kCsThreads = 256, kCsShort = 16, kCsAPitch = kCsRows + 4;
 
-typedef unsigned long long cs_f2;
-__device__ __forceinline__ cs_f2 cs_dup(float a) {
-  cs_f2 r;
-  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
-  return r;
-}
-__device__ __forceinline__ cs_f2 cs_pack(float a, float b) {
-  cs_f2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ float2 cs_split(cs_f2 v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ cs_f2 cs_fma(cs_f2 a, cs_f2 b, cs_f2 c) {
-  cs_f2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ cs_f2 cs_sub(cs_f2 a, cs_f2 b) {
-  cs_f2 r;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ cs_f2 cs_mul(cs_f2 a, cs_f2 b) {
-  cs_f2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-
 // What every recurrence shares: rows, sequences, state, outputs, workspace.
 struct ChunkScanArgs {
   const void* x;                   // rows of TA
@@ -243,7 +211,7 @@ chunk_state_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   // a thread: KR keys (in pairs) x 4 values; the lanes of a group share the keys
   constexpr int LANES = VT / 4, KR = DK / (kCsThreads / LANES);
   const int vl = tid % LANES, kg = tid / LANES;
-  cs_f2 acc[KR / 2][4];
+  f32x2 acc[KR / 2][4];
 #pragma unroll
   for (int i = 0; i < KR / 2; ++i)
 #pragma unroll
@@ -270,14 +238,14 @@ chunk_state_kernel(const ChunkScanArgs a, const typename Form::Params p) {
         const float w = scratch.w[s];
         v = make_float4(v.x * w, v.y * w, v.z * w, v.w * w);
       }
-      const cs_f2 d[4] = {cs_dup(v.x), cs_dup(v.y), cs_dup(v.z), cs_dup(v.w)};
+      const f32x2 d[4] = {dup2(v.x), dup2(v.y), dup2(v.z), dup2(v.w)};
 #pragma unroll
       for (int i = 0; i < KR / 4; ++i) {
         const ulonglong2 kk = *reinterpret_cast<const ulonglong2*>(ks + s * DK + KR * kg + 4 * i);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          acc[2 * i][j] = cs_fma(kk.x, d[j], acc[2 * i][j]);
-          acc[2 * i + 1][j] = cs_fma(kk.y, d[j], acc[2 * i + 1][j]);
+          acc[2 * i][j] = fma2(kk.x, d[j], acc[2 * i][j]);
+          acc[2 * i + 1][j] = fma2(kk.y, d[j], acc[2 * i + 1][j]);
         }
       }
     }
@@ -286,7 +254,7 @@ chunk_state_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   if (v0 + 4 * vl < a.dv) {
 #pragma unroll
     for (int i = 0; i < KR / 2; ++i) {
-      const float2 u[4] = {cs_split(acc[i][0]), cs_split(acc[i][1]), cs_split(acc[i][2]), cs_split(acc[i][3])};
+      const float2 u[4] = {unpack2(acc[i][0]), unpack2(acc[i][1]), unpack2(acc[i][2]), unpack2(acc[i][3])};
       *reinterpret_cast<float4*>(out + (size_t)(2 * i) * a.dv) = make_float4(u[0].x, u[1].x, u[2].x, u[3].x);
       *reinterpret_cast<float4*>(out + (size_t)(2 * i + 1) * a.dv) = make_float4(u[0].y, u[1].y, u[2].y, u[3].y);
     }
@@ -380,7 +348,7 @@ struct CsRows {
 
 // a group's rows of one key or row: its pairs
 template <int VT>
-__device__ __forceinline__ void cs_pairs(const float* p, cs_f2 (&out)[CsRows<VT>::kPairs]) {
+__device__ __forceinline__ void cs_pairs(const float* p, f32x2 (&out)[CsRows<VT>::kPairs]) {
 #pragma unroll
   for (int i = 0; i < CsRows<VT>::kPairs; i += 2) {
     const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p + 2 * i);
@@ -392,30 +360,30 @@ __device__ __forceinline__ void cs_pairs(const float* p, cs_f2 (&out)[CsRows<VT>
 // acc += weights^T V over the chunk's own rows of block I0.  A row sees those up to itself -- the rest is left out, not multiplied by
 // zero, so that a value that is no number reaches no earlier row.
 template <int VT, int I0>
-__device__ __forceinline__ void cs_own_rows(cs_f2 (&acc)[CsRows<VT>::kPairs][4], const float* A, const float* V, int g, int vl) {
+__device__ __forceinline__ void cs_own_rows(f32x2 (&acc)[CsRows<VT>::kPairs][4], const float* A, const float* V, int g, int vl) {
   using R = CsRows<VT>;
 #pragma unroll 4
   for (int r = 0; r < R::kBlock; ++r) {
     const int s = R::kBlock * I0 + r;
     const float4 v = *reinterpret_cast<const float4*>(V + s * VT + 4 * vl);
-    const cs_f2 d[4] = {cs_dup(v.x), cs_dup(v.y), cs_dup(v.z), cs_dup(v.w)};
-    cs_f2 w[R::kPairs];
+    const f32x2 d[4] = {dup2(v.x), dup2(v.y), dup2(v.z), dup2(v.w)};
+    f32x2 w[R::kPairs];
     cs_pairs<VT>(A + s * kCsAPitch + R::kRows * g, w);
     if (r <= 2 * g) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[I0][j] = cs_fma(w[I0], d[j], acc[I0][j]);
+      for (int j = 0; j < 4; ++j) acc[I0][j] = fma2(w[I0], d[j], acc[I0][j]);
     } else if (r == 2 * g + 1) {
-      const float u = cs_split(w[I0]).y, vv[4] = {v.x, v.y, v.z, v.w};
+      const float u = unpack2(w[I0]).y, vv[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const float2 o = cs_split(acc[I0][j]);
-        acc[I0][j] = cs_pack(o.x, fmaf(u, vv[j], o.y));
+        const float2 o = unpack2(acc[I0][j]);
+        acc[I0][j] = pack2(o.x, fmaf(u, vv[j], o.y));
       }
     }
 #pragma unroll
     for (int i = I0 + 1; i < R::kPairs; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = cs_fma(w[i], d[j], acc[i][j]);
+      for (int j = 0; j < 4; ++j) acc[i][j] = fma2(w[i], d[j], acc[i][j]);
   }
 }
 
@@ -532,7 +500,7 @@ __device__ __forceinline__ void cs_vector_weights(float* qs, float* B, float* hi
     int bt = 1;
     while (bt * (bt + 1) / 2 <= u) ++bt;
     const int bs = u - bt * (bt - 1) / 2;
-    cs_f2 acc[4][4];
+    f32x2 acc[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -542,18 +510,18 @@ __device__ __forceinline__ void cs_vector_weights(float* qs, float* B, float* hi
       const int c = 4 * (2 * ((d + (bs >> 1)) & (QUADS / 2 - 1)) + half);
       const float4 sh = *reinterpret_cast<const float4*>(Eh + (bt - 1) * P + c), sl = *reinterpret_cast<const float4*>(El + (bt - 1) * P + c),
                    eh = *reinterpret_cast<const float4*>(Eh + bs * P + c), el = *reinterpret_cast<const float4*>(El + bs * P + c);
-      const cs_f2 m0 = cs_pack(ex2_approx((sh.x - eh.x) + (sl.x - el.x)), ex2_approx((sh.y - eh.y) + (sl.y - el.y))),
-                  m1 = cs_pack(ex2_approx((sh.z - eh.z) + (sl.z - el.z)), ex2_approx((sh.w - eh.w) + (sl.w - el.w)));
+      const f32x2 m0 = pack2(ex2_approx((sh.x - eh.x) + (sl.x - el.x)), ex2_approx((sh.y - eh.y) + (sl.y - el.y))),
+                  m1 = pack2(ex2_approx((sh.z - eh.z) + (sl.z - el.z)), ex2_approx((sh.w - eh.w) + (sl.w - el.w)));
       ulonglong2 k[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) k[j] = *reinterpret_cast<const ulonglong2*>(B + (4 * bs + j) * P + c);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         ulonglong2 q = *reinterpret_cast<const ulonglong2*>(hi + (4 * bt + i) * P + c);
-        q.x = cs_mul(q.x, m0);
-        q.y = cs_mul(q.y, m1);
+        q.x = mul2(q.x, m0);
+        q.y = mul2(q.y, m1);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = cs_fma(q.y, k[j].y, cs_fma(q.x, k[j].x, acc[i][j]));
+        for (int j = 0; j < 4; ++j) acc[i][j] = fma2(q.y, k[j].y, fma2(q.x, k[j].x, acc[i][j]));
       }
     }
 #pragma unroll
@@ -561,7 +529,7 @@ __device__ __forceinline__ void cs_vector_weights(float* qs, float* B, float* hi
       float v[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const float2 z = cs_split(acc[i][j]);
+        const float2 z = unpack2(acc[i][j]);
         v[i] = z.x + z.y;
       }
       const float a0 = __shfl_xor_sync(0xffffffffu, half ? v[0] : v[2], 1), a1 = __shfl_xor_sync(0xffffffffu, half ? v[1] : v[3], 1);
@@ -626,7 +594,7 @@ chunk_output_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   } else {
     const int tg = tid >> 4, vg = tid & 15;
     // k_s . q_t: rows t = tg + 16 i, columns s = vg + 16 j, j <= i; even and odd entries summed apart
-    cs_f2 acc[4][4];
+    f32x2 acc[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -642,14 +610,14 @@ chunk_output_kernel(const ChunkScanArgs a, const typename Form::Params p) {
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j <= i; ++j) acc[i][j] = cs_fma(q[i].y, k[j].y, cs_fma(q[i].x, k[j].x, acc[i][j]));
+        for (int j = 0; j <= i; ++j) acc[i][j] = fma2(q[i].y, k[j].y, fma2(q[i].x, k[j].x, acc[i][j]));
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = 0; j <= i; ++j) {
         const int t = tg + 16 * i, s = vg + 16 * j;
-        const float2 z = cs_split(acc[i][j]);
+        const float2 z = unpack2(acc[i][j]);
         A[s * kCsAPitch + R::place(t)] = (s <= t && t < n) ? Form::D(p, scratch, t, s) * (z.x + z.y) : 0.f;
       }
     if (!zero_start) {                               // the queries, [key][64]
@@ -670,7 +638,7 @@ chunk_output_kernel(const ChunkScanArgs a, const typename Form::Params p) {
     }
   }
   const int g = tid / R::kLanes, vl = tid % R::kLanes;
-  cs_f2 acc[R::kPairs][4];
+  f32x2 acc[R::kPairs][4];
 #pragma unroll
   for (int i = 0; i < R::kPairs; ++i)
 #pragma unroll
@@ -690,23 +658,23 @@ chunk_output_kernel(const ChunkScanArgs a, const typename Form::Params p) {
     const float* T = next_tile(i);
 #pragma unroll 4
     for (int d = 0; d < 32; ++d) {
-      cs_f2 q[R::kPairs];
+      f32x2 q[R::kPairs];
       cs_pairs<VT>(qs + (32 * i + d) * kCsRows + R::kRows * g, q);
       const float4 v = *reinterpret_cast<const float4*>(T + d * VT + 4 * vl);
-      const cs_f2 b[4] = {cs_dup(v.x), cs_dup(v.y), cs_dup(v.z), cs_dup(v.w)};
+      const f32x2 b[4] = {dup2(v.x), dup2(v.y), dup2(v.z), dup2(v.w)};
 #pragma unroll
       for (int u = 0; u < R::kPairs; ++u)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[u][j] = cs_fma(q[u], b[j], acc[u][j]);
+        for (int j = 0; j < 4; ++j) acc[u][j] = fma2(q[u], b[j], acc[u][j]);
     }
   }
   if (!zero_start) {
 #pragma unroll
     for (int i = 0; i < R::kPairs; ++i) {
       const int t = R::kBlock * i + 2 * g;
-      const cs_f2 f = cs_pack(Form::aq(scratch, t), Form::aq(scratch, t + 1));
+      const f32x2 f = pack2(Form::aq(scratch, t), Form::aq(scratch, t + 1));
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = cs_mul(acc[i][j], f);
+      for (int j = 0; j < 4; ++j) acc[i][j] = mul2(acc[i][j], f);
     }
   }
   constexpr int HALF = R::kPairs / 2;                // blocks in each half of the rows
@@ -720,7 +688,7 @@ chunk_output_kernel(const ChunkScanArgs a, const typename Form::Params p) {
   if (v >= a.dv) return;
 #pragma unroll
   for (int i = 0; i < R::kPairs; ++i) {
-    const float2 u[4] = {cs_split(acc[i][0]), cs_split(acc[i][1]), cs_split(acc[i][2]), cs_split(acc[i][3])};
+    const float2 u[4] = {unpack2(acc[i][0]), unpack2(acc[i][1]), unpack2(acc[i][2]), unpack2(acc[i][3])};
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const int t = R::kBlock * i + 2 * g + e;

@@ -41,7 +41,7 @@ constexpr int kCtCarryThreads = 256, kCtDepth = 8, kCtTable = 32;      // chunks
 // Two fp32 numbers -> the next bf16 term of each (packed) and what is left of them.
 __device__ __forceinline__ uint32_t ct_term(float& a, float& b) {
   const uint32_t h = pack_bf16(a, b);
-  const float2 r = cs_split(cs_sub(cs_pack(a, b), cs_pack(bf16_lo(h), bf16_hi(h))));
+  const float2 r = unpack2(sub2(pack2(a, b), pack2(bf16_lo(h), bf16_hi(h))));
   a = r.x;
   b = r.y;
   return h;
@@ -131,10 +131,10 @@ __device__ __forceinline__ void ct_store(const CtBlocks<TA>& b, int blocks, uint
 // zero times the results, which is zero for finite ones alone.  (With every value of 4 x 2048 rows
 // infinite, 8 heads of 128 x 128: 51 ms; with every key no number, which ends a sum, 4 ms.)
 struct CtFinite {
-  cs_f2 sum = 0ull;
-  __device__ __forceinline__ void add(float a, float b) { sum = cs_fma(cs_pack(a, b), 0ull, sum); }
+  f32x2 sum = 0ull;
+  __device__ __forceinline__ void add(float a, float b) { sum = fma2(pack2(a, b), 0ull, sum); }
   __device__ __forceinline__ bool all() const {
-    const float2 v = cs_split(sum);
+    const float2 v = unpack2(sum);
     return v.x + v.y == 0.f;
   }
 };
