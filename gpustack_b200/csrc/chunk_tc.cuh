@@ -1097,7 +1097,6 @@ inline int ct_allow(K kernel, int bytes) {
   b200_set_error("chunk scan: %d bytes of shared memory: %s", bytes, cudaGetErrorString(e));
   return B200_ERR_CUDA;
 }
-inline int ct_sms() { return device_info().sm_count > 0 ? device_info().sm_count : 148; }
 
 template <int DK, int VT, typename TA, typename Form>
 int ct_launch_shape(const ChunkScanArgs& a, const typename Form::Params& p, int64_t rows, bool beside, cudaStream_t s) {
@@ -1107,11 +1106,11 @@ int ct_launch_shape(const ChunkScanArgs& a, const typename Form::Params& p, int6
   int rc = ct_allow(ct_state_kernel<DK, VT, TA, Form>, sb);
   if (rc == B200_OK) rc = ct_allow(ct_output_kernel<DK, VT, TA, Form>, ob);
   if (rc != B200_OK) return rc;
-  const int grid = (int)(items < ct_sms() ? items : ct_sms());
+  const int grid = (int)(items < sm_count() ? items : sm_count());
   if (beside) (void)launch_pdl(ct_state_kernel<DK, VT, TA, Form>, dim3(grid), dim3(kCtThreads), (size_t)sb, s, 1, a, p, (int)items);
   else ct_state_kernel<DK, VT, TA, Form><<<grid, kCtThreads, sb, s>>>(a, p, (int)items);
   const dim3 carry((DK * a.dv / 8 + kCtCarryThreads - 1) / kCtCarryThreads, a.H, a.n_seqs);
-  const bool early = !Form::kNorm || items <= ct_sms();
+  const bool early = !Form::kNorm || items <= sm_count();
   (void)launch_pdl(ct_carry_kernel<DK, Form>, carry, dim3(kCtCarryThreads), 0, s, 1, a, p, early);
   (void)launch_pdl(ct_output_kernel<DK, VT, TA, Form>, dim3(grid), dim3(kCtThreads), (size_t)ob, s, 1, a, p, (int)items);
   return b200_check_launch(Form::kName);

@@ -257,7 +257,7 @@ extern "C" int b200_conv_rec_prep(const void* proj, int f32, int64_t ld, const f
   // three of fp32 rows) four times; tiles are whole multiples
   int rows = fast ? 4 : kCapRows;
   if (fast)
-    while (rows < 32 && tile_rows % (2 * rows) == 0 && (int64_t)n_tiles * (tile_rows / (2 * rows)) * ((a.C / vec + kCapWarps * 32 - 1) / (kCapWarps * 32)) >= 4 * (f32 ? 3 : 2) * 148)
+    while (rows < 32 && tile_rows % (2 * rows) == 0 && (int64_t)n_tiles * (tile_rows / (2 * rows)) * ((a.C / vec + kCapWarps * 32 - 1) / (kCapWarps * 32)) >= 4 * (f32 ? 3 : 2) * sm_count())
       rows *= 2;
   a.per_tile = n_tiles > 0 ? tile_rows / rows : 1;
   a.n_pieces = n_tiles * a.per_tile;

@@ -130,7 +130,6 @@ constexpr int gs_log2(int n) { return n <= 1 ? 0 : 1 + gs_log2(n / 2); }
 
 constexpr int kGsWarps = 4;                            // warps that walk columns
 constexpr int kGsStepWarps = 8;                        // of the single rows' kernel
-constexpr int kGsSms = 148;
 constexpr int kGsTile = 4;                             // tokens of a block
 constexpr int kGsHelpers = 4;                          // warps that stage rows and form the factors of a block each: blocks of a stage
 constexpr int kGsStage = kGsHelpers * kGsTile;
@@ -612,7 +611,7 @@ int gated_step_launch(const GatedScanArgs& a, int n_seqs, cudaStream_t s) {
 template <int L, int R4, int C = 4>
 bool gs_fits(const GatedScanArgs& a, int n_seqs) {
   constexpr int cols = GsShape<L, R4, C>::VW;
-  return (int64_t)n_seqs * a.H * ((a.dv + cols - 1) / cols) <= kGsSms;
+  return (int64_t)n_seqs * a.H * ((a.dv + cols - 1) / cols) <= sm_count();
 }
 template <bool DELTA>
 int gated_scan_pick(const GatedScanArgs& a, int n_seqs, int max_len, cudaStream_t s) {

@@ -5,6 +5,7 @@
 // 8192 rows: a head per group, its place divided out, 20.7 us (205 instructions a thread), 18.4 of many (155 a head).
 #pragma once
 #include "common.cuh"
+#include "runtime.h"
 
 namespace b200 {
 
@@ -84,8 +85,9 @@ bool head_out_launch(const float* o, const void* proj, int64_t ld, int gate_col,
   // better: 16 heads of 64 in bf16, a head per group and resident CTAs, 1000 rows 4.5 and 5.0 us, 2048 6.7 and 7.3, 3000 8.7 and 9.0,
   // 4100 10.7 and 10.9; 32 heads of 32, 4100 rows, 10.8 and 10.4
   constexpr int kRounds = 5;
+  const int resident = kHoCtas * sm_count() * per;
   int step = items;
-  if (items > kRounds * kHoCtas * 148 * per && H <= kHoCtas * 148 * per) step = kHoCtas * 148 * per / H * H;
+  if (items > kRounds * resident && H <= resident) step = resident / H * H;
   const int grid = (step + per - 1) / per;
 #define B200_HO(L)                                                                                                                 \
   do {                                                                                                                             \

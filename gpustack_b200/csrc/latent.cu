@@ -223,7 +223,7 @@ extern "C" int b200_latent_prep(const void* proj, int f32, int64_t ld, int kv_co
   auto al = [](const void* p, int n) { return (reinterpret_cast<uintptr_t>(p) & (n - 1)) == 0; };
   if (!f32 && R == 512 && dr == 64 && dims == 64 && ld % 8 == 0 && kv_col % 8 == 0 && ldq % 2 == 0 && dn % 2 == 0 && ldqa % 2 == 0 &&
       al(proj, 16) && al(kv_norm_w, 16) && al(cache, 16) && al(q, 4) && al(qa, 4)) {
-    const int warps = T >= 4 * 148 ? kLtWarps : 1;     // few rows: a CTA each, over as many SMs
+    const int warps = T >= 4 * sm_count() ? kLtWarps : 1;     // few rows: a CTA each, over as many SMs
     (void)launch_pdl(latent_prep_rows_kernel, dim3((T + warps - 1) / warps), dim3(warps * 32), 0, s, 1, (const bf16*)proj, ld, kv_col,
                      (const bf16*)q, ldq, (const bf16*)kv_norm_w, positions, slots, (bf16*)cache, (bf16*)qa, ldqa, T, H, dn, half_layout, freq, mag, eps);
     return b200_check_launch("b200_latent_prep");

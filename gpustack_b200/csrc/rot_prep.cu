@@ -389,7 +389,7 @@ extern "C" int b200_rot_prep_hm(const void* proj, int src_f32, int64_t ld, int q
               (size_t)(dims / 2) * sizeof(float2) <= 40 * 1024 && !(src_f32 && !dst_f32);
     if (ok && dims == 0 && !unit_norm && feature == 0 && !paged && has_v && k_out != nullptr && q_head_mul == nullptr && q_out != proj) {
       const int cols = H * dk + G * dk + G * dv, nx = (cols / vec + kRvThreads - 1) / kRvThreads;
-      const bool four = (int64_t)T * nx >= 4 * 4 * 148 && T <= 65535 * 4;
+      const bool four = (int64_t)T * nx >= 4 * 4 * sm_count() && T <= 65535 * 4;
 #define B200_RP(TA, TD)                                                                                          \
   do {                                                                                                           \
     if (four) (void)launch_pdl(rot_plain_kernel<TA, TD, 4>, dim3(nx, (T + 3) / 4), dim3(kRvThreads), 0, s, 1, a, T); \
@@ -411,7 +411,7 @@ extern "C" int b200_rot_prep_hm(const void* proj, int src_f32, int64_t ld, int q
       // 41.6; 16 + 4 + 4 heads into pages 31.1 -> 31.4 and 56.8 -> 50.7.  fp32 rows lose by it: 4800 rows 32.2 -> 38.0, 8192 rows 52.2 ->
       // 57.0 (all before values went in pairs of pieces)
       const size_t smem = (size_t)(dims / 2) * sizeof(float2);
-      const bool four = !src_f32 && dims > 0 && T >= 4 * 8 * 148 && 4 * smem <= 40 * 1024;
+      const bool four = !src_f32 && dims > 0 && T >= 4 * 8 * sm_count() && 4 * smem <= 40 * 1024;
 #define B200_RVS(TA, TD, TOK, S)                                                                                                  \
   (void)launch_pdl(rot_prep_vec_kernel<TA, TD, TOK, S>, dim3((unsigned)((T + TOK - 1) / TOK)), dim3(kRvThreads), TOK * smem, s, 1, a, T, lph, \
                    items_q, items_v, v_half)

@@ -14,6 +14,7 @@ struct DeviceInfo {
   int smem_optin;
 };
 const DeviceInfo& device_info();
+inline int sm_count() { return device_info().sm_count > 0 ? device_info().sm_count : 148; }
 
 // 2-D bf16 tensor map over a row-major [rows, cols] matrix with leading dimension ld_elems,
 // box = box_rows x box_cols elements, 128-byte swizzle (box_cols * 2 bytes must be 128).
