@@ -16,8 +16,8 @@
 //   u_j = beta_j v_j - beta_j G_j S^T k_j - sum_(i < j) beta_j D_ij (k_i . k_j) u_i       (state space: beta_j v_j)
 //   o_j = G_j S^T q_j + sum_(i <= j) D_ij (k_i . q_j) u_i,      S <- G_3 S + sum_i D_i3 k_i u_i^T
 // so S^T k and S^T q of all four tokens come from the state before the block: their sums over the lanes travel together, and the
-// state is scaled once for four tokens.  Token by token, as this was, each token waits for a sum over the lanes: 676 us for the delta
-// rule over 4 x 2048 rows of 16 heads of 128 x 128 where blocks take 469 (fp32 pipe some 55 % busy), 450 -> 335 for the state space of
+// state is scaled once for four tokens.  Token by token, as this was, each token waits for a sum over the lanes: 675 us for the delta
+// rule over 4 x 2048 rows of 16 heads of 128 x 128 where blocks take 471 (fp32 pipe some 55 % busy), 450 -> 334 for the state space of
 // 32 heads of 128 x 64.  Errors against 64 bits are no larger (delta rule 4 x 600 rows: outputs 1.23e-7 -> 1.16e-7, states 1.61e-7 -> 1.51e-7;
 // state space 1.38e-7 -> 1.35e-7, 1.61e-7 -> 1.50e-7; rows of one sign 5.86e-8 -> 5.85e-8 and 1.43e-7 -> 1.42e-7, states 7 % less).
 // What bounds it is one warp's issue: the products of a token go column by column in turn so that four chains cover an FMA's latency,
@@ -140,14 +140,14 @@ constexpr int kGsStage = kGsHelpers * kGsTile;
 // walk waits for it, 328 -> 379 us for the state space of 4 x 2048 rows).  The state is scaled by G_3 rounded to fp32.  What that
 // leaves would be an error of all its entries alike, and one of decays that do not change adds up (a state left alone for 2048 tokens: 1e-5
 // off, token by token 1e-6).  So the state is held as itself over a number c close to 1: the helpers, which know what was left,
-// keep c, G_j is times c, D_j3 over it, and the walk multiplies by c at its end.  Multiplied by both parts of G_3 instead: the walk 468 -> 496 us.
+// keep c, G_j is times c, D_j3 over it, and the walk multiplies by c at its end.  Multiplied by both parts of G_3 instead: the walk 471 -> 496 us.
 constexpr int kGsBeta = 0, kGsD3 = 4, kGsG = 8, kGsGl = 12, kGsA = 16, kGsB = 24, kGsScale = 40, kGsRest = 41, kGsFactors = 44;
 
 template <int L, int R4, int C>
 struct GsShape {
   static constexpr int DKP = 4 * R4 * L, CPW = C * 32 / L, BUFS = DKP <= 256 ? 4 : 2;
-  // stages that factors are ahead of outputs: one holds up a walk of few entries per lane (state space, one sequence of 2048 rows: 207 us,
-  // with two 184), with two a short portion of many takes longer (8 of 8 rows 12.2 and 14.3)
+  // stages that factors are ahead of outputs: one holds up a walk of few entries per lane (state space of 124 keys, one sequence of 2048 rows:
+  // 217 us, with two 197), with two a portion of many takes longer (8 of 8 rows 11.6 and 12.3)
   static constexpr int AHEAD = C * R4 <= 4 ? 2 : 1;
   static constexpr int VW = kGsWarps * CPW;
   static constexpr int OUT = 4 * (L / C + 1);         // of a column and block: what the steps u are, and its lanes' shares of the read-outs
@@ -442,7 +442,7 @@ gated_scan_kernel(GatedScanArgs a) {
     const float* vr = vs + at * kGsTile * VW + mine;
     const float* f = fs + at * kGsFactors;
     float* ob = os + b % ((AHEAD + 1) * BLOCKS) * VW * Sh::OUT;
-    if ((b + 1) % BLOCKS == 0 && b + 1 < blocks) {    // the next stage's, a block early: at its own start 474 us of 469, delta rule of 4 x 2048 rows
+    if ((b + 1) % BLOCKS == 0 && b + 1 < blocks) {    // the next stage's, a block early: at its own start 474 us, delta rule of 4 x 2048 rows
       const int st = (b + 1) / BLOCKS;
       mbar_wait_guarded(&factors_full[st % BUFS], (st / BUFS) & 1);
     }
@@ -601,10 +601,10 @@ int gated_step_launch(const GatedScanArgs& a, int n_seqs, cudaStream_t s) {
 
 // Single rows have a kernel of their own.  Portions: the more columns a warp walks the fewer instructions a column costs, the fewer
 // it walks the shorter a block takes, so the widest form whose CTAs still find an SM each: us for 1, 2, 3 and 4 sequences of the delta
-// rule with 16 heads of 128 x 128 (2048, 1024, 1024 and 2048 rows), in CTAs of 64 columns 471, 241, 242, 472, of 32 columns 336, 174, 285, 558,
-// of 16 columns 283, 225, 348, 860.  CTAs of 32 columns share an SM in pairs, which covers the start and the end of short portions: 16
-// of 16 rows 34.5 in CTAs of 64 columns, 31.0 of 32, but 8 of 1024 rows 476 and 551.  A bound on the rows per portion is often that of all
-// of them, so pairs are for sequences enough to fill the GPU three times (16 of 512 rows: 480 either way) or a bound that is short.
+// rule with 16 heads of 128 x 128 (2048, 1024, 1024 and 2048 rows), in CTAs of 64 columns 467, 236, 236, 468, of 32 columns 332, 169, 286, 566,
+// of 16 columns 264, 219, 339, 853.  CTAs of 32 columns share an SM in pairs, which covers the start and the end of short portions: 16
+// of 16 rows 28.7 in CTAs of 64 columns, 26.6 of 32, but 8 of 1024 rows 473 and 558.  A bound on the rows per portion is often that of all
+// of them, so pairs are for sequences enough to fill the GPU three times (16 of 512 rows: 477 and 489) or a bound that is short.
 // Few keys: a lane of two columns walks faster than one of four, whose sums over lanes and columns take longer than its products.  State
 // space of 32 heads of 64 values, us token by token, in four columns a lane, in two: 16 keys, one sequence of 2048 rows 203, 221, 192, 64 of 33
 // rows 59, 55, 49; 32 keys 205, 187, 152 and 59, 55, 86: of 17 to 32 keys two only where CTAs of 32 columns find an SM each.
