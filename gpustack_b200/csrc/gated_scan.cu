@@ -406,7 +406,7 @@ gated_scan_kernel(GatedScanArgs a) {
         if (j < 2) D3 *= g2;
         if (j < 3) D3 *= g3;
         G = fma(G, (double)c, G);
-        D3 = fma(D3, (double)(behind * fmaf(behind, 1.f - behind, -1.f)), D3);      // over 1 + behind
+        D3 = fma(D3, (double)(-behind * rcp_approx(1.f + behind)), D3);      // over 1 + behind
         const float high = (float)G;
         f[kGsBeta + j] = gb.y;
         f[kGsG + j] = high;
